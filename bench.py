@@ -166,6 +166,28 @@ class CallTimer:
         setattr(owner, name, wrapped)
         self._undo.append((owner, name, inner))
 
+    def wrap_op(self, owner, name, fwd, bwd):
+        """Time an operator's forward call and, through hooks on its autograd node, its backward pass."""
+        inner = getattr(owner, name)
+        timer = self
+
+        def wrapped(*a, **k):
+            if not timer.enabled:
+                return inner(*a, **k)
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
+            e[0].record()
+            out = inner(*a, **k)
+            e[1].record()
+            timer.events.setdefault(fwd, []).append((e[0], e[1]))
+            node = (out[0] if isinstance(out, tuple) else out).grad_fn
+            if node is not None:
+                node.register_prehook(lambda *_: e[2].record())
+                node.register_hook(lambda *_: (e[3].record(), timer.events.setdefault(bwd, []).append((e[2], e[3])))[0])
+            return out
+
+        setattr(owner, name, wrapped)
+        self._undo.append((owner, name, inner))
+
     def restore(self):
         for owner, name, inner in self._undo:
             setattr(owner, name, inner)
@@ -179,30 +201,11 @@ class CallTimer:
         return sum(a.elapsed_time(b) for a, b in self.events.get(tag, []))
 
 
-# kernels launched by one call of a C-ABI entry point (ssm_ssd_fwd: by phase)
-KERNELS_PER_CALL = {"ssm_selective_scan_fwd": 1, "ssm_selective_scan_bwd": 1, "ssm_selective_state_step": 1, "ssm_dw_causal_conv_fwd": 1,
-                    "ssm_dw_causal_conv_bwd": 1, "ssm_dw_causal_conv_update": 1, "ssm_fused_add_norm_fwd": 1, "ssm_fused_add_norm_bwd": 2,
-                    "ssm_chunk_scan_fwd": 3, "ssm_chunk_scan_bwd": 1, "ssm_ssd_fwd": 3, "ssm_ssd_fold_shards": 1, "ssm_mamba1_decode": 1}
+def launches() -> int:
+    """Kernels this package's library has launched in this process (counted by the library)."""
+    from ssm_b200 import _lib
 
-
-def count_launches(timer: CallTimer) -> int:
-    return sum(KERNELS_PER_CALL.get(k, 1) * v for k, v in timer.calls.items() if k.startswith("ssm_"))
-
-
-def wrap_abi_calls(timer: CallTimer):
-    """Count every C-ABI call made through `ssm_b200.ops` (each launches the kernels listed in KERNELS_PER_CALL)."""
-    from ssm_b200 import ops
-
-    inner = ops._call
-
-    def counted(fn, args):
-        if timer.enabled:
-            name = getattr(fn, "__name__", None) or getattr(fn, "name", "ssm_call")
-            timer.calls[name] = timer.calls.get(name, 0) + 1
-        return inner(fn, args)
-
-    ops._call = counted
-    timer._undo.append((ops, "_call", inner))
+    return int(_lib.load().ssm_b200_launch_count())
 
 
 # --------------------------------------------------------------------------------------
@@ -259,8 +262,8 @@ def run_prefill(args):
         print(f"[prefill] {cfg['n_layer']} layers ready: shard length {Lq}", file=sys.stderr, flush=True)
 
     timer = CallTimer()
-    timer.wrap(ops._SsdWorkspace, "run", lambda self, phase, *a, **k: f"ssd_phase{phase}")
-    wrap_abi_calls(timer)
+    timer.wrap(ops._SsdWorkspace, "run", lambda self, phase, *a, **k: f"ssd_phase{phase}")  # the phases of a sequence shard
+    timer.wrap(ops, "ssd_scan", "ssd_phase0")
 
     @torch.no_grad()
     def forward(ids):
@@ -294,7 +297,9 @@ def run_prefill(args):
 
     sampler = ClockSampler(local).start() if rank == 0 else None
     timer.enabled = True
+    launched = launches()
     ms = timed(lambda: forward(ids_dev))
+    launched = launches() - launched
     timer.enabled = False
     out_host = torch.empty(B, model.lm_head.weight.shape[0], dtype=torch.bfloat16).pin_memory()
 
@@ -341,7 +346,7 @@ def run_prefill(args):
                        "l2": "per-layer activations (GBs) exceed the 126 MB L2"},
             "e2e": {"value": tokens / (ms_e2e * 1e-3), "unit": "tokens/s", "ms_per_step": ms_e2e, "h2d_bytes_per_step": ids_host.numel() * 8,
                     "d2h_bytes_per_step": out_host.numel() * 2},
-            "gpu_launches": count_launches(timer),
+            "gpu_launches": launched,
             "roofline": roof, "clocks": clocks,
         }
         if not args.no_cpu and world == 1:
@@ -467,12 +472,9 @@ def bench_mamba1_block(batch=8, steps=10, warmup=3, timer=None):
     w = make_block_weights(cfg, dev, torch.bfloat16, seed=0)
     own = timer is None
     timer = timer or CallTimer()
-    timer.wrap(ops, "_scan_forward", "scan_fwd")
-    timer.wrap(ops, "_scan_backward", "scan_bwd")
-    timer.wrap(ops._ConvFn, "forward", "conv_fwd")
-    timer.wrap(ops._ConvFn, "backward", "conv_bwd")
-    timer.wrap(ops._NormFn, "forward", "norm_fwd")
-    timer.wrap(ops._NormFn, "backward", "norm_bwd")
+    timer.wrap_op(ops, "selective_scan", "scan_fwd", "scan_bwd")
+    timer.wrap_op(ops, "dw_causal_conv", "conv_fwd", "conv_bwd")
+    timer.wrap_op(ops, "fused_layer_norm", "norm_fwd", "norm_bwd")
     g = torch.Generator().manual_seed(1234)
     xs = [torch.randn(B, Lq, dm, generator=g).to(torch.bfloat16).to(dev) for _ in range(2)]
     rs = [torch.randn(B, Lq, dm, generator=g).to(dev) for _ in range(2)]
@@ -866,7 +868,7 @@ def run_single(args):
     roof, extra = {}, {}
     if wl == "mamba1_block":
         timer = CallTimer()
-        wrap_abi_calls(timer)
+        before = launches()
         r = bench_mamba1_block(batch=args.batch or 8, steps=steps, warmup=args.warmup, timer=timer)
         ms, value, unit, metric, hib = r["step_ms"], r["tokens"] / (r["step_ms"] * 1e-3), "tokens/s", "tokens_per_s", True
         ach = r["scan_bwd_bytes"] / (r["scan_bwd_ms"] * 1e-3) / 1e9
@@ -875,7 +877,7 @@ def run_single(args):
         for tag in ("scan_fwd", "conv_fwd", "conv_bwd", "norm_fwd", "norm_bwd"):
             roof[tag + "_ms"] = r[tag + "_ms"]
             roof[tag + "_frac"] = r[tag + "_bytes"] / (r[tag + "_ms"] * 1e-3) / 1e9 / peak
-        extra["gpu_launches"] = count_launches(timer)
+        extra["gpu_launches"] = launches() - before  # warm-up steps included
         timer.restore()
         work = f"mamba1_block fwd+bwd: batch {args.batch or 8}, seqlen 4096, d_model 768, d_inner 1536, d_state 16, d_conv 4, dt_rank 48, RMSNorm eps 1e-5"
     elif wl == "ssd":

@@ -51,6 +51,8 @@ typedef void* ssm_stream_t;
 
 int ssm_b200_abi_version(void);
 const char* ssm_b200_last_error(void);
+/* kernels launched by this library since the process started, over all devices and threads */
+int64_t ssm_b200_launch_count(void);
 
 /* ---------------------------------------------------------------------------------------
  * Selective scan (Mamba-1), forward.   Replaces selective_scan_cuda

@@ -147,6 +147,7 @@ class SsdBwdArgs(C.Structure):
 ENTRY_POINTS = {
     "ssm_b200_abi_version": (C.c_int, []),
     "ssm_b200_last_error": (C.c_char_p, []),
+    "ssm_b200_launch_count": (C.c_int64, []),
     "ssm_scan_checkpoint_interval": (C.c_int, []),
     "ssm_scan_split_segments": (C.c_int, [i32, i32, i32, i32]),
     "ssm_selective_scan_fwd": (C.c_int, [C.POINTER(ScanFwdArgs), vp]),

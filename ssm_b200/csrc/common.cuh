@@ -33,7 +33,10 @@ int f64_chunk(const ssm_chunk_bwd_args& g, bool backward, cudaStream_t st);
 int f64_conv(const ssm_conv_bwd_args& g, bool backward, cudaStream_t st);
 int f64_norm(const ssm_norm_bwd_args& g, bool backward, cudaStream_t st);
 
+void count_launch();
+// called once after every kernel launch
 inline int launch_status(const char* kernel) {
+  count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("%s: %s", kernel, cudaGetErrorString(e));

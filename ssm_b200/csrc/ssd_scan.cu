@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
     }
   }
   }  // compute warps
-  if (fail && lane == 0 && a.status) atomicExch(a.status, 1);
+  if (fail && lane == 0 && a.status) *(volatile int32_t*)a.status = 1;
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, kCols);
@@ -904,7 +904,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     }
   }
   if (tid == kCopyThread) tc::bulk_wait_all();  // the staging tile must outlive the stores that read it
-  if (fail && tid == 0 && a.status) atomicExch(a.status, 2);
+  if (fail && tid == 0 && a.status) *(volatile int32_t*)a.status = 2;
 }
 
 template <typename T, bool XSKIP>
@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(32) ssd_wait_selftest_kernel(int32_t* status, 
   if (threadIdx.x == 0) tc::mbar_init(tc::smem_u32(&mbar), 1);
   __syncwarp();
   const bool ok = tc::mbar_wait(tc::smem_u32(&mbar), 0, probes);
-  if (!ok && threadIdx.x == 0 && status) atomicExch(status, 3);
+  if (!ok && threadIdx.x == 0 && status) *(volatile int32_t*)status = 3;
 }
 
 template <typename T>

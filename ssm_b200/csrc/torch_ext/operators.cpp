@@ -1,0 +1,531 @@
+// The package's own operator surface (ssm_b200.ops) over the C ABI: forward passes, and the autograd nodes whose backward
+// passes call the backward entry points.  Everything between a Python call and its kernel launches happens here, once per
+// call and without Python: a small operator is bound by exactly this work (a Python implementation of the same steps, with
+// a ctypes struct per call and torch.autograd.Function, took 40 to 90 us a call; these take 6 to 15 us).
+#include <torch/csrc/autograd/custom_function.h>
+
+#include <utility>
+
+#include "operands.h"
+
+namespace ssm_ext {
+namespace {
+
+namespace py = pybind11;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+// ---------------------------------------------------------------------------------------------
+// one differentiable call
+// ---------------------------------------------------------------------------------------------
+// The operands of a call, kept by its autograd node.  `guarded` holds the tensors that the backward pass reads again with
+// their version counters at the time of the forward pass: an in-place edit in between is an error, as for any saved tensor.
+struct Call : torch::CustomClassHolder {
+  std::vector<std::pair<Tensor, uint32_t>> guarded;
+  variable_list inputs;  // the defined tensor arguments, in the order backward() answers for them
+  void input(const Tensor& t) { inputs.push_back(t); }
+  void input(const OptTensor& t) {
+    if (t.has_value() && t->defined()) inputs.push_back(*t);
+  }
+  bool needs_grad() const {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor& t : inputs)
+      if (t.requires_grad()) return true;
+    return false;
+  }
+  virtual variable_list forward(bool train) = 0;
+  virtual variable_list backward(const variable_list& grads) = 0;  // one gradient (or an undefined tensor) per input
+};
+
+struct CallFn : torch::autograd::Function<CallFn> {
+  static variable_list forward(AutogradContext* ctx, const c10::intrusive_ptr<Call>& call, at::TensorList inputs) {
+    for (const Tensor& t : inputs)
+      if (!t.is_inference()) call->guarded.emplace_back(t, t._version());
+    ctx->saved_data["call"] = c10::IValue::make_capsule(call);
+    ctx->set_materialize_grads(false);
+    return call->forward(true);
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    auto holder = ctx->saved_data["call"].toCapsule();
+    Call* call = static_cast<Call*>(holder.get());
+    for (const auto& kept : call->guarded) {
+      if (kept.first._version() == kept.second) continue;
+      std::string shape;
+      for (int64_t d : kept.first.sizes()) shape += (shape.empty() ? "" : ", ") + std::to_string(d);
+      TORCH_CHECK(false, "one of the tensors needed for the backward pass of an ssm_b200 operator has been modified in place (shape (" + shape + "), version " +
+                             std::to_string(kept.first._version()) + ", expected " + std::to_string(kept.second) + ")");
+    }
+    ValueErrors scope;
+    variable_list res = call->backward(grads);
+    res.insert(res.begin(), Tensor());  // the slot of `call`
+    return res;
+  }
+};
+
+variable_list invoke_call(const c10::intrusive_ptr<Call>& call) {
+  if (!call->needs_grad()) return call->forward(false);
+  const variable_list inputs = call->inputs;
+  call->inputs.clear();
+  return CallFn::apply(call, at::TensorList(inputs));
+}
+
+Tensor cast(const Tensor& grad, at::ScalarType t) { return grad.scalar_type() == t ? grad : grad.to(t); }
+
+// Several fp32 buffers that the kernels add into, zeroed by one launch; each starts on a 256-byte line.
+struct ZeroPool {
+  std::vector<std::pair<Tensor*, std::vector<int64_t>>> want;
+  int64_t total = 0;
+  void add(Tensor& t, at::IntArrayRef shape) { want.emplace_back(&t, shape.vec()), total += padded(shape); }
+  static int64_t padded(at::IntArrayRef shape) { return (c10::multiply_integers(shape) + 63) / 64 * 64; }
+  void make(const at::TensorOptions& f32) {
+    if (want.empty()) return;
+    Tensor all = at::zeros({total}, f32);
+    int64_t at = 0;
+    for (auto& [t, shape] : want) {
+      *t = all.narrow(0, at, c10::multiply_integers(shape)).view(shape);
+      at += padded(shape);
+    }
+  }
+};
+
+float* out_ptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
+
+// ---------------------------------------------------------------------------------------------
+// selective scan
+// ---------------------------------------------------------------------------------------------
+struct ScanCall final : Call {
+  ScanCtx c;
+  bool want_last, has_init, init_grad;
+  at::ScalarType last_type, t_delta, t_A, t_B, t_C, t_D{}, t_z{}, t_bias{}, t_init{};
+  std::vector<int64_t> shape_B, shape_C;
+  Tensor ck;
+
+  ScanCall(const Tensor& u, const Tensor& delta, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D, const OptTensor& z,
+           const OptTensor& dt_bias, bool softplus, bool return_last, const OptTensor& init, bool keep_fp32)
+      : c(u, delta, A, B, C, D, z, dt_bias, softplus, init, true), want_last(return_last), has_init(init.has_value()) {
+    for (const Tensor* t : {&u, &delta, &A, &B, &C}) input(*t);
+    input(D), input(z), input(dt_bias), input(init);
+    last_type = keep_fp32 ? at::kFloat : u.scalar_type();
+    t_delta = delta.scalar_type(), t_A = A.scalar_type(), t_B = B.scalar_type(), t_C = C.scalar_type();
+    if (D.has_value()) t_D = D->scalar_type();
+    if (z.has_value()) t_z = z->scalar_type();
+    if (dt_bias.has_value()) t_bias = dt_bias->scalar_type();
+    if (has_init) t_init = init->scalar_type();
+    init_grad = has_init && init->requires_grad();
+    shape_B = B.sizes().vec(), shape_C = C.sizes().vec();
+  }
+
+  variable_list forward(bool train) override {
+    c10::cuda::CUDAGuard guard(c.u.device());
+    Tensor out = at::empty_like(c.u), last, split;
+    ssm_scan_fwd_args a{};
+    c.fill(a);
+    a.out = out.data_ptr();
+    if (want_last) {
+      last = at::empty({c.nb, c.nd, c.nn}, c.u.options().dtype(last_type));
+      a.last_state = last.data_ptr(), a.last_dtype = dtype_code(last, "selective_scan");
+    }
+    if (train) ck = scan_checkpoints(c), a.checkpoints = ck.data_ptr<float>();
+    const int nseg = ssm_scan_split_segments((int)c.nb, (int)c.nd, (int)c.nl, (int)c.nn);  // > 1: the sequence is cut into parallel segments
+    if (nseg > 1) {
+      split = at::empty({2 * c.nb * c.nd * nseg * c.nn}, c.u.options().dtype(at::kFloat));
+      a.split_scratch = split.data_ptr<float>(), a.split_segments = nseg;
+    }
+    run(ssm_selective_scan_fwd(&a, stream_of(c.u)));
+    if (want_last) return {out, last};
+    return {out};
+  }
+
+  variable_list backward(const variable_list& grads) override {
+    c10::cuda::CUDAGuard guard(c.u.device());
+    const auto f32 = c.u.options().dtype(at::kFloat);
+    Tensor go = grads[0].defined() ? rows_like(grads[0], c.u) : at::zeros_like(c.u);
+    OptTensor gl;
+    if (grads.size() > 1 && grads[1].defined()) gl = f32c(grads[1]);
+    Tensor du = at::empty_like(c.u), dd = at::empty_like(c.u), dz, dA, dB, dC, dD, db, dinit;
+    if (c.z.has_value()) dz = at::empty_like(c.u);
+    ZeroPool params, coeffs;
+    params.add(dA, {c.nd, c.nn});
+    if (c.D.has_value()) params.add(dD, {c.nd});
+    if (c.bias.has_value()) params.add(db, {c.nd});
+    coeffs.add(dB, c.B.t.sizes()), coeffs.add(dC, c.C.t.sizes());
+    params.make(f32), coeffs.make(f32);
+    if (init_grad) {  // an empty sequence hands the gradient of the last state straight to the initial state
+      if (c.nl == 0) dinit = gl.has_value() ? gl->clone() : at::zeros({c.nb, c.nd, c.nn}, f32);
+      else dinit = at::empty({c.nb, c.nd, c.nn}, f32);
+    }
+    ssm_scan_bwd_args g{};
+    c.fill(g.fwd);
+    g.fwd.checkpoints = ck.data_ptr<float>();
+    g.dout = go.data_ptr(), g.dlast_state = fptr(gl);
+    g.du = du.data_ptr(), g.ddelta = dd.data_ptr(), g.dz = dz.defined() ? dz.data_ptr() : nullptr;
+    g.dA = out_ptr(dA), g.dB = out_ptr(dB), g.dC = out_ptr(dC), g.dD = out_ptr(dD), g.ddt_bias = out_ptr(db);
+    g.db_sb = c.B.sb, g.db_sg = c.B.sg, g.db_sn = c.B.sn, g.db_st = c.B.st;
+    g.dc_sb = c.C.sb, g.dc_sg = c.C.sg, g.dc_sn = c.C.sn, g.dc_st = c.C.st;
+    g.dinitial_state = out_ptr(dinit);
+    run(ssm_selective_scan_bwd(&g, stream_of(c.u)));
+    auto fold = [](Tensor grad, at::IntArrayRef shape, at::ScalarType t) {
+      if (grad.sizes() != shape)  // the coefficient had been regrouped: sum the repeats back
+        grad = grad.view({shape[0], shape[1], grad.size(1) / shape[1], shape[2], shape[3]}).sum(2);
+      return cast(grad, t);
+    };
+    variable_list res = {du, cast(dd, t_delta), cast(dA, t_A), fold(dB, shape_B, t_B), fold(dC, shape_C, t_C)};
+    if (c.D.has_value()) res.push_back(cast(dD, t_D));
+    if (c.z.has_value()) res.push_back(cast(dz, t_z));
+    if (c.bias.has_value()) res.push_back(cast(db, t_bias));
+    if (has_init) res.push_back(init_grad ? cast(dinit, t_init) : Tensor());
+    return res;
+  }
+};
+
+py::object selective_scan(const Tensor& u, const Tensor& delta, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D, const OptTensor& z,
+                          const OptTensor& dt_bias, bool softplus, bool return_last, const OptTensor& init, bool keep_fp32) {
+  ValueErrors scope;
+  variable_list r = invoke_call(c10::make_intrusive<ScanCall>(u, delta, A, B, C, D, z, dt_bias, softplus, return_last, init, keep_fp32));
+  if (return_last) return py::make_tuple(r[0], r[1]);
+  return py::cast(r[0]);
+}
+
+// ---------------------------------------------------------------------------------------------
+// single-token state steps (no gradients)
+// ---------------------------------------------------------------------------------------------
+Tensor state_step(const Tensor& state, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
+                  const OptTensor& z, const OptTensor& dt_bias, bool softplus) {
+  ValueErrors scope;
+  StepCtx c(state, x, dt, A, B, C, D, z, dt_bias, softplus);
+  c10::cuda::CUDAGuard guard(state.device());
+  const bool direct = state.scalar_type() == at::kFloat && state.is_contiguous();
+  Tensor work = direct ? state.detach() : f32c(state);
+  Tensor out = at::empty_like(c.x);
+  ssm_step_args a{};
+  c.fill(a, work);
+  a.out = out.data_ptr();
+  run(ssm_selective_state_step(&a, stream_of(state)));
+  if (!direct) state.detach().copy_(work);
+  return out;
+}
+
+Tensor state_step_heads(const Tensor& state, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
+                        const OptTensor& z, const OptTensor& dt_bias, bool softplus) {
+  ValueErrors scope;
+  SSM_ARG(state.dim() == 4 && x.dim() == 3, "state must be (B, H, P, N) and x (B, H, P).");
+  const int64_t nb = state.size(0), nh = state.size(1), np = state.size(2), nn = state.size(3);
+  SSM_ARG(x.size(0) == nb && x.size(1) == nh && x.size(2) == np && dt.dim() == 2 && dt.size(0) == nb && dt.size(1) == nh && A.dim() == 1 && A.size(0) == nh,
+          "x must be (B, H, P), dt (B, H) and A (H,).");
+  SSM_ARG(B.dim() == 3 && B.sizes() == C.sizes() && B.size(0) == nb && B.size(2) == nn && B.size(1) > 0 && nh % B.size(1) == 0,
+          "B and C must have shape (B, G, N) with G dividing H.");
+  same_device(state, {&x, &dt, &A, &B, &C});
+  need_cuda(state, {&D, &z, &dt_bias});
+  SSM_ARG(state.scalar_type() == at::kFloat && state.is_contiguous(), "state must be a contiguous float32 tensor.");
+  c10::cuda::CUDAGuard guard(state.device());
+  Tensor xs = x.detach().contiguous(), dts = like(dt, xs), Bt = B.detach().contiguous(), Ct = C.detach().contiguous();
+  OptTensor zs;
+  if (z.has_value()) zs = like(*z, xs);
+  if (Bt.scalar_type() != Ct.scalar_type() || !io_dtype_ok(Bt)) Bt = f32c(Bt), Ct = f32c(Ct);
+  Tensor A32 = f32c(A), out = at::empty_like(xs);
+  OptTensor D32 = f32c(D), b32 = f32c(dt_bias);
+  const int64_t g = Bt.size(1);
+  ssm_step_args a{};
+  a.batch = (int)nb, a.dim = (int)(nh * np), a.nstate = (int)nn, a.io_dtype = dtype_code(xs, "selective_state_step_heads");
+  a.bc_dtype = dtype_code(Bt, "selective_state_step_heads B/C"), a.bc_groups = (int)g, a.dt_softplus = softplus, a.param_heads = (int)nh;
+  a.state = state.data_ptr<float>(), a.x = xs.data_ptr(), a.dt = dts.data_ptr(), a.z = ptr(zs), a.A = A32.data_ptr<float>();
+  a.Bm = Bt.data_ptr(), a.Cm = Ct.data_ptr();
+  a.b_sb = a.c_sb = g * nn, a.b_sg = a.c_sg = nn, a.b_sn = a.c_sn = 1;
+  a.D = fptr(D32), a.dt_bias = fptr(b32), a.out = out.data_ptr();
+  run(ssm_selective_state_step(&a, stream_of(state)));
+  return out;
+}
+
+// ---------------------------------------------------------------------------------------------
+// element-wise chunked recurrence
+// ---------------------------------------------------------------------------------------------
+struct ChunkCall final : Call {
+  ChunkCtx c;
+  at::ScalarType t_dt, t_A, t_B, t_C, t_D{}, t_z{}, t_init{};
+
+  ChunkCall(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk, const OptTensor& D, const OptTensor& z,
+            const OptTensor& seq_lens, const OptTensor& cu_seqlens, const OptTensor& init)
+      : c(X, dt, A, B, C, chunk, D, z, seq_lens, cu_seqlens, init) {
+    for (const Tensor* t : {&X, &dt, &A, &B, &C}) input(*t);
+    input(D), input(z), input(init);
+    t_dt = dt.scalar_type(), t_A = A.scalar_type(), t_B = B.scalar_type(), t_C = C.scalar_type();
+    if (D.has_value()) t_D = D->scalar_type();
+    if (z.has_value()) t_z = z->scalar_type();
+    if (init.has_value()) t_init = init->scalar_type();
+  }
+
+  variable_list forward(bool) override {
+    c10::cuda::CUDAGuard guard(c.X.device());
+    Tensor Y = at::empty_like(c.X);
+    const int64_t n = ssm_chunk_scan_scratch_floats((int)c.nb, (int)c.nl, (int)c.nh, (int)c.np, c.chunk);
+    Tensor scratch = at::empty({std::max<int64_t>(n, 1)}, c.X.options().dtype(at::kFloat));
+    ssm_chunk_args a{};
+    c.fill(a);
+    a.Y = Y.data_ptr(), a.scratch = scratch.data_ptr<float>();
+    run(ssm_chunk_scan_fwd(&a, stream_of(c.X)));
+    return {Y};
+  }
+
+  variable_list backward(const variable_list& grads) override {
+    c10::cuda::CUDAGuard guard(c.X.device());
+    const auto f32 = c.X.options().dtype(at::kFloat);
+    Tensor gy = like(grads[0], c.X);
+    Tensor dX = at::empty_like(c.X), ddt, dA, dB, dC, dD, dz, dI;
+    ZeroPool pool;
+    int typed = 0;
+    // per-token B / C / z: their gradients are written by the kernel in the tensor's own type (no zero-fill, no fp32 copy)
+    auto own = [&](Tensor& grad, const OptTensor& t, Kind k, int bit) {
+      if (!t.has_value()) return;
+      if (k == Kind::BLHP) grad = at::empty_like(*t), typed |= bit;
+      else pool.add(grad, t->sizes());
+    };
+    pool.add(ddt, {c.nb, c.nl, c.nh}), pool.add(dA, c.A->sizes());
+    own(dB, c.B, c.kB, 1), own(dC, c.C, c.kC, 2), own(dz, c.z, c.kz, 4);
+    if (c.D.has_value()) pool.add(dD, c.D->sizes());
+    if (c.init.has_value()) pool.add(dI, c.init->sizes());
+    pool.make(f32);
+    Tensor hist = at::empty({c.nb, std::max<int64_t>(c.nl, 1), c.nh, c.np}, f32);
+    Tensor scratch = at::empty({std::max<int64_t>(1, ssm_chunk_scan_bwd_scratch_floats((int)c.nb, (int)c.nl, (int)c.nh, (int)c.np, c.chunk))}, f32);
+    ssm_chunk_bwd_args g{};
+    c.fill(g.fwd);
+    g.fwd.typed_grads = typed;
+    g.dY = gy.data_ptr(), g.dX = dX.data_ptr(), g.ddt = ddt.data_ptr<float>(), g.history = hist.data_ptr<float>(), g.scratch = scratch.data_ptr<float>();
+    auto grad_of = [](const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };
+    set_bc4(g.dA, grad_of(dA), c.kA), set_bc4(g.dB, grad_of(dB), c.kB), set_bc4(g.dC, grad_of(dC), c.kC), set_bc4(g.dD, grad_of(dD), c.kD),
+        set_bc4(g.dz, grad_of(dz), c.kz), set_bc4(g.dinitial, grad_of(dI), Kind::BHP);
+    run(ssm_chunk_scan_bwd(&g, stream_of(c.X)));
+    variable_list res = {dX, cast(ddt, t_dt), cast(dA, t_A), cast(dB, t_B), cast(dC, t_C)};
+    if (c.D.has_value()) res.push_back(cast(dD, t_D));
+    if (c.z.has_value()) res.push_back(cast(dz, t_z));
+    if (c.init.has_value()) res.push_back(cast(dI, t_init));
+    return res;
+  }
+};
+
+Tensor ssd_chunk_scan(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk, const OptTensor& D,
+                      const OptTensor& z, const OptTensor& seq_lens, const OptTensor& cu_seqlens, const OptTensor& init) {
+  ValueErrors scope;
+  return invoke_call(c10::make_intrusive<ChunkCall>(X, dt, A, B, C, chunk, D, z, seq_lens, cu_seqlens, init))[0];
+}
+
+// ---------------------------------------------------------------------------------------------
+// depthwise causal conv
+// ---------------------------------------------------------------------------------------------
+struct ConvCall final : Call {
+  ConvCtx c;
+  at::ScalarType t_w, t_b{};
+  std::vector<int64_t> shape_w;
+
+  ConvCall(const Tensor& x, const Tensor& weight, const OptTensor& bias, const std::string& activation, const OptTensor& halo)
+      : c(x, weight, bias, activation, halo, true) {
+    input(x), input(weight), input(bias);
+    t_w = weight.scalar_type(), shape_w = weight.sizes().vec();
+    if (bias.has_value()) t_b = bias->scalar_type();
+  }
+  variable_list forward(bool) override {
+    c10::cuda::CUDAGuard guard(c.x.device());
+    Tensor y = at::empty_like(c.x);
+    ssm_conv_args a{};
+    c.fill(a);
+    a.y = y.data_ptr();
+    run(ssm_dw_causal_conv_fwd(&a, stream_of(c.x)));
+    return {y};
+  }
+  variable_list backward(const variable_list& grads) override {
+    c10::cuda::CUDAGuard guard(c.x.device());
+    Tensor go = rows_like(grads[0], c.x), dx = at::empty_like(c.x), dw, db;
+    ZeroPool pool;
+    pool.add(dw, {c.nc, c.k});
+    if (c.b.has_value()) pool.add(db, {c.nc});
+    pool.make(c.x.options().dtype(at::kFloat));
+    ssm_conv_bwd_args g{};
+    c.fill(g.fwd);
+    g.dy = go.data_ptr(), g.dx = dx.data_ptr(), g.dweight = out_ptr(dw), g.dbias = out_ptr(db);
+    run(ssm_dw_causal_conv_bwd(&g, stream_of(c.x)));
+    variable_list res = {dx, cast(dw.view(shape_w), t_w)};
+    if (c.b.has_value()) res.push_back(cast(db, t_b));
+    return res;
+  }
+};
+
+Tensor dw_causal_conv(const Tensor& x, const Tensor& weight, const OptTensor& bias, const std::string& activation, const OptTensor& halo) {
+  ValueErrors scope;
+  return invoke_call(c10::make_intrusive<ConvCall>(x, weight, bias, activation, halo))[0];
+}
+
+Tensor dw_causal_conv_update(const Tensor& conv_state, const Tensor& x, const Tensor& weight, const OptTensor& bias, const std::string& activation) {
+  ValueErrors scope;
+  SSM_ARG(conv_state.dim() == 3 && x.dim() == 2 && conv_state.size(0) == x.size(0) && conv_state.size(1) == x.size(1),
+          "conv_state must be (B, C, K) and x (B, C).");
+  Tensor w2 = weight.dim() == 3 ? weight.select(1, 0) : weight;
+  SSM_ARG(w2.dim() == 2 && w2.size(0) == x.size(1) && w2.size(1) == conv_state.size(2), "weight must have shape (C, K).");
+  same_device(conv_state, {&x, &weight});
+  need_cuda(conv_state, {&bias});
+  SSM_ARG(conv_state.scalar_type() == at::kFloat && conv_state.is_contiguous(), "conv_state must be a contiguous float32 tensor.");
+  const bool silu = is_silu(activation);
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor xs = x.detach().contiguous(), w32 = f32c(w2), out = at::empty_like(xs);
+  OptTensor b32 = f32c(bias);
+  ssm_conv_update_args a{};
+  a.batch = (int)x.size(0), a.channels = (int)x.size(1), a.width = (int)conv_state.size(2), a.io_dtype = dtype_code(xs, "dw_causal_conv_update");
+  a.silu = silu;
+  a.conv_state = conv_state.data_ptr<float>(), a.x = xs.data_ptr(), a.weight = w32.data_ptr<float>(), a.bias = fptr(b32), a.out = out.data_ptr();
+  run(ssm_dw_causal_conv_update(&a, stream_of(xs)));
+  return out;
+}
+
+// ---------------------------------------------------------------------------------------------
+// fused residual add + LayerNorm / RMSNorm
+// ---------------------------------------------------------------------------------------------
+struct NormCall final : Call {
+  NormCtx c;
+  bool want_res;
+  at::ScalarType res_type, t_w, t_b{}, t_r{};
+
+  NormCall(const Tensor& x, const Tensor& weight, const OptTensor& bias, const OptTensor& residual, bool is_rms, double eps, bool prenorm, bool return_residual,
+           bool residual_in_fp32)
+      : c(x, weight, bias, residual, is_rms, eps, prenorm), want_res(return_residual) {
+    input(x), input(weight), input(bias), input(residual);
+    res_type = residual_in_fp32 ? at::kFloat : x.scalar_type();
+    t_w = weight.scalar_type();
+    if (bias.has_value()) t_b = bias->scalar_type();
+    if (residual.has_value()) t_r = residual->scalar_type();
+  }
+  variable_list forward(bool) override {
+    c10::cuda::CUDAGuard guard(c.x.device());
+    Tensor y = at::empty_like(c.x), ro;
+    ssm_norm_args a{};
+    c.fill(a);
+    a.y = y.data_ptr();
+    if (want_res) {
+      ro = at::empty(c.x.sizes(), c.x.options().dtype(res_type));
+      a.residual_out = ro.data_ptr(), a.resout_dtype = dtype_code(ro, "fused_layer_norm");
+    }
+    run(ssm_fused_add_norm_fwd(&a, stream_of(c.x)));
+    if (want_res) return {y, ro};
+    return {y};
+  }
+  variable_list backward(const variable_list& grads) override {
+    c10::cuda::CUDAGuard guard(c.x.device());
+    const auto f32 = c.x.options().dtype(at::kFloat);
+    const int64_t rows = c.x.size(0) * c.x.size(1), hidden = c.x.size(2);
+    Tensor go = grads[0].defined() ? like(grads[0], c.x) : at::zeros_like(c.x), gr;
+    Tensor dx = at::empty_like(c.x), dres, dw = at::empty({hidden}, f32), db;
+    if (c.res.has_value()) dres = at::empty_like(*c.res);
+    if (c.b.has_value()) db = at::empty({hidden}, f32);
+    Tensor partial = at::empty({ssm_norm_bwd_scratch_floats(rows, (int)hidden)}, f32);
+    ssm_norm_bwd_args g{};
+    c.fill(g.fwd);
+    g.dy = go.data_ptr(), g.dx = dx.data_ptr(), g.dresidual = dres.defined() ? dres.data_ptr() : nullptr;
+    g.dweight = dw.data_ptr<float>(), g.dbias = out_ptr(db), g.partial = partial.data_ptr<float>();
+    if (grads.size() > 1 && grads[1].defined()) {  // the gradient arriving through x + residual: added to dx and dresidual inside the kernel
+      gr = grads[1].detach().to(res_type).contiguous();
+      g.fwd.resout_dtype = dtype_code(gr, "fused_layer_norm"), g.dresidual_out = gr.data_ptr();
+    }
+    run(ssm_fused_add_norm_bwd(&g, stream_of(c.x)));
+    variable_list res = {dx, cast(dw, t_w)};
+    if (c.b.has_value()) res.push_back(cast(db, t_b));
+    if (c.res.has_value()) res.push_back(cast(dres, t_r));
+    return res;
+  }
+};
+
+py::object fused_layer_norm(const Tensor& x, const Tensor& weight, const OptTensor& bias, const OptTensor& residual, bool is_rms, double eps, bool prenorm,
+                            bool residual_in_fp32, bool return_residual) {
+  ValueErrors scope;
+  variable_list r = invoke_call(c10::make_intrusive<NormCall>(x, weight, bias, residual, is_rms, eps, prenorm, return_residual, residual_in_fp32));
+  if (return_residual) return py::make_tuple(r[0], r[1]);
+  return py::cast(r[0]);
+}
+
+// ---------------------------------------------------------------------------------------------
+// state-space-dual scan, forward on the tensor cores
+// ---------------------------------------------------------------------------------------------
+// The word a kernel sets when one of its bounded waits runs out, one per device, in pinned host memory that the kernels write
+// directly: a failure is visible to the next call without a copy, an event or a synchronisation per launch.
+Tensor ssd_status(int64_t device) {
+  static std::mutex lock;
+  static std::vector<Tensor> words(64);
+  TORCH_CHECK(device >= 0 && device < (int64_t)words.size(), "ssd_scan: device index out of range");
+  std::lock_guard<std::mutex> hold(lock);
+  Tensor& w = words[device];
+  if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt)).pin_memory();
+  return w;
+}
+// Raise if a launch since the last report ran out of a wait.
+void ssd_poll(int64_t device) {
+  volatile int32_t* word = ssd_status(device).data_ptr<int32_t>();
+  const int32_t code = *word;
+  if (code == 0) return;
+  *word = 0;
+  TORCH_CHECK(false, std::string() + "ssd_scan: a bounded device-side wait ran out in an earlier launch (status " + std::to_string(code) + "); its outputs are invalid");
+}
+
+struct SsdShape {
+  int64_t nb, nl, nh, np, ng, nn;
+};
+SsdShape ssd_check(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D, const OptTensor& z,
+                   const OptTensor& dt_bias, const OptTensor& init) {
+  SSM_ARG(X.dim() == 4 && dt.dim() == 3, "X must be (B, L, H, P) and dt (B, L, H).");
+  SsdShape s{X.size(0), X.size(1), X.size(2), X.size(3), 0, 0};
+  SSM_ARG(dt.size(0) == s.nb && dt.size(1) == s.nl && dt.size(2) == s.nh, "dt must align with (B, L, H).");
+  SSM_ARG(A.dim() == 1 && A.size(0) == s.nh, "A must have shape (H,).");
+  SSM_ARG(B.dim() == 4 && B.size(0) == s.nb && B.size(1) == s.nl && B.sizes() == C.sizes(), "B and C must have shape (B, L, G, N).");
+  s.ng = B.size(2), s.nn = B.size(3);
+  SSM_ARG(s.ng > 0 && s.nh % s.ng == 0, "Group dimension must divide H.");
+  if (D.has_value())
+    SSM_ARG((D->dim() == 1 && D->size(0) == s.nh) || (D->dim() == 2 && D->size(0) == s.nh && D->size(1) == s.np), "D must have shape (H,) or (H, P).");
+  if (z.has_value()) SSM_ARG(z->sizes() == X.sizes(), "z must have shape (B, L, H, P).");
+  if (dt_bias.has_value()) SSM_ARG(dt_bias->dim() == 1 && dt_bias->size(0) == s.nh, "dt_bias must have shape (H,).");
+  if (init.has_value())
+    SSM_ARG(init->dim() == 4 && init->size(0) == s.nb && init->size(1) == s.nh && init->size(2) == s.np && init->size(3) == s.nn,
+            "initial_states must have shape (B, H, P, N).");
+  same_device(X, {&dt, &A, &B, &C});
+  need_cuda(X, {&D, &z, &dt_bias, &init});
+  return s;
+}
+
+// (Y, final states fp32); the caller has checked ssm_ssd_supported().
+std::tuple<Tensor, Tensor> ssd_forward(const Tensor& X_, const Tensor& dt_, const Tensor& A_, const Tensor& B_, const Tensor& C_, const OptTensor& D_,
+                                       const OptTensor& z_, const OptTensor& bias_, bool softplus, const OptTensor& init_, int64_t chunk) {
+  ValueErrors scope;
+  const SsdShape s = ssd_check(X_, dt_, A_, B_, C_, D_, z_, bias_, init_);
+  c10::cuda::CUDAGuard guard(X_.device());
+  ssd_poll(X_.get_device());
+  Tensor X = X_.detach().contiguous(), dt = like(dt_, X), B = like(B_, X), C = like(C_, X), A = f32c(A_);
+  OptTensor D = f32c(D_), bias = f32c(bias_), init = f32c(init_), z;
+  if (z_.has_value()) z = like(*z_, X);
+  const auto f32 = X.options().dtype(at::kFloat);
+  Tensor Y = at::empty_like(X), fin = at::empty({s.nb, s.nh, s.np, s.nn}, f32);
+  Tensor ws = at::empty({ssm_ssd_scratch_bytes((int)s.nb, (int)s.nl, (int)s.nh)}, X.options().dtype(at::kByte));
+  const int64_t vec = s.nb * s.nh * ((s.nl + chunk - 1) / chunk) * chunk * 4;
+  char* base = reinterpret_cast<char*>(ws.data_ptr());
+  ssm_ssd_args a{};
+  a.batch = (int)s.nb, a.len = (int)s.nl, a.heads = (int)s.nh, a.headdim = (int)s.np, a.nstate = (int)s.nn, a.groups = (int)s.ng;
+  a.chunk_size = (int)chunk, a.io_dtype = dtype_code(X, "ssd_scan"), a.dt_softplus = softplus, a.d_has_p = D.has_value() && D->dim() == 2;
+  a.X = X.data_ptr(), a.dt = dt.data_ptr(), a.A = A.data_ptr<float>(), a.Bm = B.data_ptr(), a.Cm = C.data_ptr();
+  a.D = fptr(D), a.z = ptr(z), a.dt_bias = fptr(bias), a.initial_states = fptr(init), a.Y = Y.data_ptr(), a.final_states = fin.data_ptr<float>();
+  a.ws_dt = reinterpret_cast<float*>(base), a.ws_cum = reinterpret_cast<float*>(base + vec), a.ws_state = reinterpret_cast<float*>(base + 2 * vec);
+  a.ws_state_in = base + 2 * vec + ssm_ssd_state_scratch_bytes((int)s.nb, (int)s.nl, (int)s.nh);
+  a.status = ssd_status(X.get_device()).data_ptr<int32_t>();
+  run(ssm_ssd_fwd(&a, stream_of(X)));
+  return {Y, fin};
+}
+
+}  // namespace
+
+void bind_operators(py::module& m) {
+  auto ops = m.def_submodule("operators", "the operator surface of ssm_b200.ops");
+  ops.def("selective_scan", &selective_scan);
+  ops.def("state_step", &state_step);
+  ops.def("state_step_heads", &state_step_heads);
+  ops.def("ssd_chunk_scan", &ssd_chunk_scan);
+  ops.def("dw_causal_conv", &dw_causal_conv);
+  ops.def("dw_causal_conv_update", &dw_causal_conv_update);
+  ops.def("fused_layer_norm", &fused_layer_norm);
+  ops.def("ssd_forward", &ssd_forward);
+  ops.def("ssd_status", &ssd_status);
+  ops.def("ssd_poll", &ssd_poll);
+}
+
+}  // namespace ssm_ext

@@ -3,10 +3,11 @@
 ``selective_scan``, ``selective_state_step``, ``ssd_chunk_scan``, ``dw_causal_conv`` and
 ``fused_layer_norm`` take the arguments of ``ssm.ops`` in b-vitamins/ssm
 (src/ssm/ops/__init__.py:1255-1690; semantics src/ssm/ops/python/reference.py), accept CUDA
-tensors only, and are differentiable through ``torch.autograd.Function`` wrappers whose
-forward and backward both run hand-written sm_100a kernels behind the C ABI of
-``include/ssm_b200.h``.  Contract violations raise ``ValueError`` as upstream does.  There is
-no CPU path and no PyTorch fallback: a missing library or a CPU tensor is an error.
+tensors only, and are differentiable: forward and backward both run hand-written sm_100a
+kernels behind the C ABI of ``include/ssm_b200.h``.  What lies between a call and its launches
+(checks, layout and dtype normalisation, allocation, the autograd node) is C++
+(``csrc/torch_ext/operators.cpp``).  Contract violations raise ``ValueError`` as upstream does.
+There is no CPU path and no PyTorch fallback: a missing library or a CPU tensor is an error.
 
 Additive keyword arguments that upstream does not have are marked "extension" below; their
 defaults reproduce upstream behaviour.
@@ -26,6 +27,19 @@ from . import _lib as L
 Tensor = torch.Tensor
 
 _CODES = {torch.float32: L.F32, torch.bfloat16: L.BF16, torch.float16: L.F16}
+
+
+_ops = None
+
+
+def _native():
+    """The compiled operator surface (loaded once; raises if it has not been built)."""
+    global _ops
+    if _ops is None:
+        from .backend import load_extension
+
+        _ops = load_extension().operators
+    return _ops
 
 
 def _code(t: Tensor, what: str) -> int:
@@ -71,27 +85,6 @@ def _c(t: Optional[Tensor]) -> Optional[Tensor]:
     return t if t.is_contiguous() else t.contiguous()
 
 
-def _rows(t: Tensor) -> Tensor:
-    """A (B, D, L) activation in one of the two row layouts the kernels address directly: dense
-    (B, D, L), or a dense (D, B, L) buffer viewed as (B, D, L).  Anything else is copied to dense."""
-    t = t.detach()
-    if t.is_contiguous() or (t.dim() == 3 and t.stride(2) == 1 and t.permute(1, 0, 2).is_contiguous()):
-        return t
-    return t.contiguous()
-
-
-def _rows_like(t: Optional[Tensor], ref: Tensor) -> Optional[Tensor]:
-    """``t`` with the dtype and exactly the strides of ``ref`` (copied only when it differs)."""
-    if t is None:
-        return None
-    t = t.detach()
-    if t.dtype == ref.dtype and t.stride() == ref.stride():
-        return t
-    out = torch.empty_like(ref)
-    out.copy_(t)
-    return out
-
-
 def _guard(ctx, *tensors: Optional[Tensor]) -> None:
     """Remember the version counters of the tensors a backward pass will read again; `_check_guard`
     raises if one of them was modified in place in between (what autograd does for saved tensors)."""
@@ -106,50 +99,32 @@ def _check_guard(ctx) -> None:
 
 
 class _DeviceStatus:
-    """The device word that the tensor-core kernels set when one of their bounded waits runs out, with a pinned host
-    mirror.  After every launch the word is copied to the mirror asynchronously on the launching stream; `poll` reads
-    the mirror once that copy has finished, so a timed-out wait surfaces at the next call without the hot path ever
-    synchronising.  `poll(sync=True)` waits for the last launch first."""
+    """The word that the tensor-core kernels set when one of their bounded waits runs out: one per device, in pinned host
+    memory that the kernels write directly.  `poll` reads it, so a timed-out wait surfaces at the next call without the hot
+    path ever copying or synchronising.  `poll(sync=True)` waits for the device first."""
 
     _per_device: dict[int, "_DeviceStatus"] = {}
 
-    def __init__(self, device: torch.device):
-        self.word = torch.zeros(1, dtype=torch.int32, device=device)
-        self.host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        self.event: Optional[torch.cuda.Event] = None
+    def __init__(self, index: int):
+        self.index = index
+        self.word = _native().ssd_status(index)
 
     @classmethod
     def of(cls, device: torch.device) -> "_DeviceStatus":
         idx = device.index if device.index is not None else torch.cuda.current_device()
         st = cls._per_device.get(idx)
         if st is None:
-            st = cls._per_device[idx] = cls(torch.device("cuda", idx))
+            st = cls._per_device[idx] = cls(idx)
         return st
 
-    def after_launch(self) -> None:
-        if torch.cuda.is_current_stream_capturing():
-            return
-        self.host.copy_(self.word, non_blocking=True)
-        self.event = torch.cuda.Event()
-        self.event.record()
-
     def poll(self, sync: bool = False) -> None:
-        if self.event is None or torch.cuda.is_current_stream_capturing():
-            return
-        if sync:
-            self.event.synchronize()
-        elif not self.event.query():
-            return
-        code = int(self.host[0])
-        if code:
-            self.host.zero_()
-            self.word.zero_()
-            self.event = None
-            raise RuntimeError(f"ssd_scan: a bounded device-side wait ran out in an earlier launch (status {code}); its outputs are invalid")
+        if sync and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.synchronize(self.index)
+        _native().ssd_poll(self.index)
 
 
 def ssd_check_status(device: Optional[torch.device] = None) -> None:
-    """Wait for the last tensor-core SSD launch on ``device`` and raise if one of its bounded waits ran out."""
+    """Wait for ``device`` and raise if a bounded wait of a tensor-core SSD launch ran out."""
     _DeviceStatus.of(torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)).poll(sync=True)
 
 
@@ -158,9 +133,8 @@ def ssd_wait_selftest(probes: int = 100, device: Optional[torch.device] = None) 
     probes, recording status 3 like a tensor-core kernel whose copy never landed.  The next ``ssd_scan`` call (or
     :func:`ssd_check_status`) then raises; the device and the context stay usable."""
     st = _DeviceStatus.of(torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device))
-    with torch.cuda.device(st.word.device):
+    with torch.cuda.device(st.index):
         L.check(L.load().ssm_ssd_wait_selftest(st.word.data_ptr(), int(probes), _stream()))
-        st.after_launch()
 
 
 def _call(fn, args) -> None:
@@ -175,203 +149,6 @@ def _call(fn, args) -> None:
 # =========================================================================================
 # selective_scan
 # =========================================================================================
-
-
-def _scan_coeff(name: str, p: Tensor, nb: int, nd: int, nn: int, nl: int):
-    """Return (tensor, groups, (sb, sg, sn, st)) for the B / C layouts of reference.py:22-56."""
-    if p.dim() == 2:
-        if tuple(p.shape) != (nd, nn):
-            raise ValueError(f"{name} must have shape (D, N).")
-        return _f32(p), nd, (0, nn, 1, 0)
-    if p.dim() == 3:
-        if tuple(p.shape) != (nb, nd, nn):
-            raise ValueError(f"{name} must have shape (B, D, N) when 3-D.")
-        return _f32(p), nd, (nd * nn, nn, 1, 0)
-    if p.dim() == 4:
-        if p.shape[0] != nb or p.shape[-1] != nl:
-            raise ValueError(f"{name} must have shape (B, G, N, L) when 4-D.")
-        g = p.shape[1]
-        if g == 0 or nd % g != 0:
-            raise ValueError("Group dimension must divide D.")
-        if p.shape[2] != nn:
-            raise ValueError(f"{name} has mismatched state dimension.")
-        return _c(p), g, (g * nn * nl, nn * nl, nl, 1)
-    raise ValueError(f"Unsupported rank for {name}.")
-
-
-class _ScanCtx:
-    """Validated, contiguous inputs of one selective-scan call."""
-
-    def __init__(self, u, delta, A, B, C_, D, z, dt_bias, softplus, initial_state):
-        if u.ndim != 3 or delta.ndim != 3:
-            raise ValueError("u and delta must have shape (B, D, L).")
-        nb, nd, nl = u.shape
-        if tuple(delta.shape) != (nb, nd, nl):
-            raise ValueError("delta must match the shape of u.")
-        if A.ndim != 2 or tuple(A.shape) != (nd, A.shape[-1]):
-            raise ValueError("A must have shape (D, N).")
-        nn = A.shape[-1]
-        if nn < 1 or nn > 256:
-            raise ValueError("selective_scan: the state dimension must be in [1, 256].")
-        if A.is_complex():
-            raise ValueError("selective_scan: complex A is not built")
-        _need_cuda(u, delta, A, B, C_, D, z, dt_bias, initial_state)
-        self.io = _code(u, "selective_scan")
-        self.shape = (nb, nd, nl, nn)
-        self.u = _rows(u)
-        self.delta = _rows_like(delta, self.u)
-        self.A = _f32(A)
-        Bt, gb, sB = _scan_coeff("B", B, nb, nd, nn, nl)
-        Ct, gc, sC = _scan_coeff("C", C_, nb, nd, nn, nl)
-        if gb != gc:
-            # differing group counts: expand the coarser one so that one group map serves both
-            g = max(gb, gc)
-            if g % min(gb, gc) != 0:
-                raise ValueError("B and C group dimensions must nest.")
-            if gb < g:
-                Bt, sB = _regroup(Bt, sB, gb, g, nb, nn, nl)
-            else:
-                Ct, sC = _regroup(Ct, sC, gc, g, nb, nn, nl)
-            gb = g
-        if Bt.dtype != Ct.dtype:
-            Bt, Ct = Bt.float(), Ct.float()
-        _code(Bt, "selective_scan B/C")
-        self.B, self.C, self.groups, self.sB, self.sC = Bt, Ct, gb, sB, sC
-        if D is not None and tuple(D.shape) != (nd,):
-            raise ValueError("D must have shape (D,).")
-        if z is not None and tuple(z.shape) != (nb, nd, nl):
-            raise ValueError("z must have shape (B, D, L).")
-        if dt_bias is not None and tuple(dt_bias.shape) != (nd,):
-            raise ValueError("dt_bias must have shape (D,).")
-        if initial_state is not None and tuple(initial_state.shape) != (nb, nd, nn):
-            raise ValueError("initial_state must have shape (B, D, N).")
-        self.D = _f32(D)
-        self.z = _rows_like(z, self.u)
-        self.dt_bias = _f32(dt_bias)
-        self.init = _f32(initial_state)
-        self.softplus = bool(softplus)
-
-    def fill(self, a: L.ScanFwdArgs) -> None:
-        nb, nd, nl, nn = self.shape
-        a.batch, a.dim, a.len, a.nstate = nb, nd, nl, nn
-        a.io_dtype, a.bc_dtype = self.io, _CODES[self.B.dtype]
-        a.delta_softplus = int(self.softplus)
-        a.u, a.delta, a.z, a.A = _p(self.u), _p(self.delta), _p(self.z), _p(self.A)
-        a.Bm, a.Cm, a.bc_groups = _p(self.B), _p(self.C), self.groups
-        a.b_sb, a.b_sg, a.b_sn, a.b_st = self.sB
-        a.c_sb, a.c_sg, a.c_sn, a.c_st = self.sC
-        a.D, a.dt_bias, a.initial_state = _p(self.D), _p(self.dt_bias), _p(self.init)
-        a.row_sb, a.row_sd = (self.u.stride(0), self.u.stride(1)) if self.u.numel() else (nd * nl, nl)
-
-
-def _regroup(t: Tensor, strides, g_old: int, g_new: int, nb: int, nn: int, nl: int):
-    """Repeat a coarser-grouped (B, G, N, L) coefficient so that it has ``g_new`` groups."""
-    if strides[3] == 0:  # (D, N) / (B, D, N) are always per channel; cannot be coarser
-        raise ValueError("B and C group dimensions must nest.")
-    t = t.repeat_interleave(g_new // g_old, dim=1).contiguous()
-    return t, (g_new * nn * nl, nn * nl, nl, 1)
-
-
-def _scan_forward(ctx: _ScanCtx, want_last: bool, want_ckpt: bool, last_dtype: torch.dtype):
-    nb, nd, nl, nn = ctx.shape
-    lib = L.load()
-    out = torch.empty_like(ctx.u)
-    last = torch.empty(nb, nd, nn, dtype=last_dtype, device=ctx.u.device) if want_last else None
-    ck = None
-    if want_ckpt:
-        iv = lib.ssm_scan_checkpoint_interval()
-        ck = torch.empty(nb, nd, max(1, (nl + iv - 1) // iv), nn, dtype=torch.float32, device=ctx.u.device)
-    a = L.ScanFwdArgs()
-    ctx.fill(a)
-    a.out, a.last_state, a.checkpoints = _p(out), _p(last), _p(ck)
-    nseg = int(lib.ssm_scan_split_segments(nb, nd, nl, nn))  # > 1: too few rows to fill the GPU, the sequence is cut into parallel segments
-    split = None
-    if nseg > 1:
-        split = torch.empty(2 * nb * nd * nseg * nn, dtype=torch.float32, device=ctx.u.device)
-        a.split_scratch, a.split_segments = _p(split), nseg
-    a.last_dtype = _CODES[last_dtype] if want_last else 0
-    _call(lib.ssm_selective_scan_fwd, a)
-    return out, last, ck
-
-
-def _scan_backward(ctx: _ScanCtx, ck: Tensor, grad_out: Tensor, grad_last: Optional[Tensor], B_like: Tensor, C_like: Tensor,
-                   want_dinit: bool = False):
-    nb, nd, nl, nn = ctx.shape
-    lib = L.load()
-    dev = ctx.u.device
-    dinit = None
-    if want_dinit:
-        # an empty sequence hands the gradient of the last state straight to the initial state
-        dinit = torch.zeros(nb, nd, nn, dtype=torch.float32, device=dev) if (nl == 0 and grad_last is None) else \
-            (grad_last.detach().float().clone() if nl == 0 else torch.empty(nb, nd, nn, dtype=torch.float32, device=dev))
-    du = torch.empty_like(ctx.u)
-    ddelta = torch.empty_like(ctx.u)
-    dz = torch.empty_like(ctx.u) if ctx.z is not None else None
-    dA = torch.zeros(nd, nn, dtype=torch.float32, device=dev)
-    # gradient buffers in the layout of the (contiguous) coefficients the kernel read
-    dB = torch.zeros(ctx.B.shape, dtype=torch.float32, device=dev)
-    dC = torch.zeros(ctx.C.shape, dtype=torch.float32, device=dev)
-    dD = torch.zeros(nd, dtype=torch.float32, device=dev) if ctx.D is not None else None
-    dbias = torch.zeros(nd, dtype=torch.float32, device=dev) if ctx.dt_bias is not None else None
-    g = L.ScanBwdArgs()
-    ctx.fill(g.fwd)
-    g.fwd.checkpoints = _p(ck)
-    go = _rows_like(grad_out, ctx.u)
-    gl = _f32(grad_last)
-    g.dout, g.dlast_state = _p(go), _p(gl)
-    g.du, g.ddelta, g.dz = _p(du), _p(ddelta), _p(dz)
-    g.dA, g.dB, g.dC, g.dD, g.ddt_bias = _p(dA), _p(dB), _p(dC), _p(dD), _p(dbias)
-    g.db_sb, g.db_sg, g.db_sn, g.db_st = ctx.sB
-    g.dc_sb, g.dc_sg, g.dc_sn, g.dc_st = ctx.sC
-    g.dinitial_state = _p(dinit)
-    _call(lib.ssm_selective_scan_bwd, g)
-
-    def fold(grad: Tensor, like: Tensor) -> Tensor:
-        if grad.shape != like.shape:  # the coefficient had been regrouped: sum the repeats back
-            rep = grad.shape[1] // like.shape[1]
-            grad = grad.view(like.shape[0], like.shape[1], rep, *like.shape[2:]).sum(2)
-        return grad.to(like.dtype)
-
-    if want_dinit:
-        return du, ddelta, dA, fold(dB, B_like), fold(dC, C_like), dD, dz, dbias, dinit
-    return du, ddelta, dA, fold(dB, B_like), fold(dC, C_like), dD, dz, dbias
-
-
-class _SelectiveScanFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, u, delta, A, B, C_, D, z, dt_bias, softplus, return_last_state, initial_state, keep_state_fp32):
-        sc = _ScanCtx(u, delta, A, B, C_, D, z, dt_bias, softplus, initial_state)
-        needs = any(t is not None and t.requires_grad for t in (u, delta, A, B, C_, D, z, dt_bias, initial_state))
-        last_dtype = torch.float32 if keep_state_fp32 else u.dtype
-        out, last, ck = _scan_forward(sc, return_last_state, needs, last_dtype)
-        ctx.sc, ctx.ck = sc, ck
-        ctx.like = (B, C_, A, D, z, dt_bias, delta, initial_state)
-        _guard(ctx, u, delta, A, B, C_, D, z, dt_bias, initial_state)
-        if return_last_state:
-            return out, last
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_out, grad_last=None):
-        _check_guard(ctx)
-        sc: _ScanCtx = ctx.sc
-        B, C_, A, D, z, dt_bias, delta, init = ctx.like
-        if grad_out is None:
-            grad_out = torch.zeros_like(sc.u)
-        want_dinit = init is not None and init.requires_grad
-        res = _scan_backward(sc, ctx.ck, grad_out, grad_last, B, C_, want_dinit)
-        du, ddelta, dA, dB, dC, dD, dz, dbias = res[:8]
-        return (
-            du,
-            ddelta.to(delta.dtype),
-            dA.to(A.dtype),
-            dB,
-            dC,
-            None if D is None else dD.to(D.dtype),
-            None if z is None else dz.to(z.dtype),
-            None if dt_bias is None else dbias.to(dt_bias.dtype),
-            None, None, res[8].to(init.dtype) if want_dinit else None, None,
-        )
 
 
 def selective_scan(
@@ -397,8 +174,7 @@ def selective_scan(
     if u.dtype == torch.float64:  # double-precision kernels, meant for gradient checks (ops_f64.py)
         from . import ops_f64
         return ops_f64.selective_scan(u, delta, A, B, C, D, z, dt_bias, softplus, return_last_state, initial_state)
-    res = _SelectiveScanFn.apply(u, delta, A, B, C, D, z, dt_bias, softplus, return_last_state, initial_state, keep_state_fp32)
-    return res
+    return _native().selective_scan(u, delta, A, B, C, D, z, dt_bias, softplus, return_last_state, initial_state, keep_state_fp32)
 
 
 # =========================================================================================
@@ -564,8 +340,7 @@ def selective_state_step(
         with torch.no_grad():
             state.copy_(new)
         return y
-    sc = _StepCtx(state, x, dt, A, B, C, D, z, dt_bias, softplus)
-    return _step_forward(sc, state)
+    return _native().state_step(state, x, dt, A, B, C, D, z, dt_bias, softplus)
 
 
 def selective_state_step_heads(
@@ -575,226 +350,12 @@ def selective_state_step_heads(
     """Extension: Mamba-2 decode step.  ``state (B, H, P, N)`` fp32 in place, ``x, z (B, H, P)``,
     ``dt (B, H)``, ``A, D, dt_bias (H,)``, ``B, C (B, G, N)``; returns ``(B, H, P)``.  Equivalent to
     the upstream step on ``H*P`` flattened channels with per-head parameters broadcast."""
-    if state.ndim != 4 or x.ndim != 3:
-        raise ValueError("state must be (B, H, P, N) and x (B, H, P).")
-    nb, nh, npj, nn = state.shape
-    if tuple(x.shape) != (nb, nh, npj) or tuple(dt.shape) != (nb, nh) or tuple(A.shape) != (nh,):
-        raise ValueError("x must be (B, H, P), dt (B, H) and A (H,).")
-    if B.ndim != 3 or B.shape != C.shape or B.shape[0] != nb or B.shape[2] != nn or nh % B.shape[1] != 0:
-        raise ValueError("B and C must have shape (B, G, N) with G dividing H.")
-    _need_cuda(state, x, dt, A, B, C, D, z, dt_bias)
-    if state.dtype != torch.float32 or not state.is_contiguous():
-        raise ValueError("state must be a contiguous float32 tensor.")
-    lib = L.load()
-    xs, dts = _c(x), _c(dt.to(x.dtype))
-    zs = None if z is None else _c(z.to(x.dtype))
-    Bt, Ct = _c(B), _c(C)
-    if Bt.dtype != Ct.dtype or Bt.dtype not in _CODES:
-        Bt, Ct = Bt.float(), Ct.float()
-    A32, D32, b32 = _f32(A), _f32(D), _f32(dt_bias)
-    out = torch.empty_like(xs)
-    g = Bt.shape[1]
-    a = L.StepArgs()
-    a.batch, a.dim, a.nstate, a.io_dtype = nb, nh * npj, nn, _code(x, "selective_state_step_heads")
-    a.bc_dtype, a.bc_groups, a.dt_softplus, a.param_heads = _CODES[Bt.dtype], g, int(softplus), nh
-    a.state, a.x, a.dt, a.z, a.A = _p(state), _p(xs), _p(dts), _p(zs), _p(A32)
-    a.Bm, a.Cm = _p(Bt), _p(Ct)
-    a.b_sb, a.b_sg, a.b_sn = g * nn, nn, 1
-    a.c_sb, a.c_sg, a.c_sn = g * nn, nn, 1
-    a.D, a.dt_bias, a.out = _p(D32), _p(b32), _p(out)
-    _call(lib.ssm_selective_state_step, a)
-    return out
+    return _native().state_step_heads(state, x, dt, A, B, C, D, z, dt_bias, softplus)
 
 
 # =========================================================================================
 # ssd_chunk_scan (element-wise chunked recurrence)
 # =========================================================================================
-
-
-def _seq_lens(seq_meta: Optional[dict[str, Any]], nb: int, nl: int, device) -> Optional[Tensor]:
-    """Per-row valid lengths as an int64 device tensor (reference.py:413-428)."""
-    if not seq_meta:
-        return None
-    if seq_meta.get("cu_seqlens") is not None:
-        cu = torch.as_tensor(seq_meta["cu_seqlens"]).to(device=device, dtype=torch.long)
-        if cu.numel() != nb + 1:
-            raise ValueError("cu_seqlens must have length B + 1.")
-        return (cu[1:] - cu[:-1]).contiguous()
-    if seq_meta.get("seq_lens") is not None:
-        sl = torch.as_tensor(seq_meta["seq_lens"]).to(device=device, dtype=torch.long)
-        if sl.numel() != nb:
-            raise ValueError("seq_lens must have length B.")
-        return sl.contiguous()
-    raise ValueError("seq_meta must provide cu_seqlens or seq_lens.")
-
-
-def _bc4(t: Optional[Tensor], kind: str) -> tuple[Optional[int], tuple[int, int, int, int]]:
-    """Pointer and (sb, st, sh, sq) strides of a contiguous parameter of layout ``kind``."""
-    if t is None:
-        return None, (0, 0, 0, 0)
-    if kind == "h":
-        return t.data_ptr(), (0, 0, 1, 0)
-    if kind == "hp":
-        return t.data_ptr(), (0, 0, t.shape[1], 1)
-    if kind == "bhp":
-        return t.data_ptr(), (t.shape[1] * t.shape[2], 0, t.shape[2], 1)
-    if kind == "blh":
-        return t.data_ptr(), (t.shape[1] * t.shape[2], t.shape[2], 1, 0)
-    if kind == "blhp":
-        return t.data_ptr(), (t.shape[1] * t.shape[2] * t.shape[3], t.shape[2] * t.shape[3], t.shape[3], 1)
-    raise AssertionError(kind)
-
-
-def _set_bc4(dst: L.Bcast4, ptr: Optional[int], strides) -> None:
-    dst.ptr = ptr
-    dst.sb, dst.st, dst.sh, dst.sq = strides
-
-
-class _ChunkCtx:
-    def __init__(self, X, dt, A, B, C_, chunk_size, D, z, seq_meta, initial_states):
-        if X.ndim != 4:
-            raise ValueError("X must have shape (B, L, H, P).")
-        if dt.ndim != 3:
-            raise ValueError("dt must have shape (B, L, H).")
-        nb, nl, nh, npj = X.shape
-        if tuple(dt.shape) != (nb, nl, nh):
-            raise ValueError("dt must align with (B, L, H).")
-        if int(chunk_size) <= 0:
-            raise ValueError("chunk_size must be positive.")
-        _need_cuda(X, dt, A, B, C_, D, z, initial_states)
-        self.shape = (nb, nl, nh, npj)
-        self.chunk = int(chunk_size)
-        self.io = _code(X, "ssd_chunk_scan")
-        self.X, self.dt = _c(X), _c(dt.to(X.dtype))
-        if A.ndim == 1:
-            if A.shape[0] != nh:
-                raise ValueError("A must have shape (H,) when 1-D.")
-            self.A, self.kA = _f32(A), "h"
-        elif A.ndim == 2:
-            if tuple(A.shape) != (nh, npj):
-                raise ValueError("A must have shape (H, P) when 2-D.")
-            self.A, self.kA = _f32(A), "hp"
-        else:
-            raise ValueError("A must be 1-D or 2-D.")
-
-        def coeff(name, p):
-            if p.dim() == 2:
-                if tuple(p.shape) != (nh, npj):
-                    raise ValueError(f"{name} must have shape (H, P).")
-                return "hp"
-            if p.dim() == 3:
-                if tuple(p.shape) != (nb, nh, npj):
-                    raise ValueError(f"{name} must be (B, H, P) when 3-D.")
-                return "bhp"
-            if p.dim() == 4:
-                if tuple(p.shape) != (nb, nl, nh, npj):
-                    raise ValueError(f"{name} must have shape (B, L, H, P) when 4-D.")
-                return "blhp"
-            raise ValueError(f"Unsupported rank for {name}.")
-
-        self.kB, self.kC = coeff("B", B), coeff("C", C_)
-        self.kD = None
-        if D is not None:
-            if D.ndim == 1 and D.shape[0] == nh:
-                self.kD = "h"
-            elif D.ndim == 2 and tuple(D.shape) == (nh, npj):
-                self.kD = "hp"
-            else:
-                raise ValueError("D must have shape (H,) or (H, P).")
-        self.kz = None
-        if z is not None:
-            if z.ndim == 3 and tuple(z.shape) == (nb, nl, nh):
-                self.kz = "blh"
-            elif z.ndim == 4 and tuple(z.shape) == (nb, nl, nh, npj):
-                self.kz = "blhp"
-            else:
-                raise ValueError("z must have shape (B, L, H) or (B, L, H, P).")
-        if initial_states is not None and tuple(initial_states.shape) != (nb, nh, npj):
-            raise ValueError("initial_states must have shape (B, H, P).")
-        # B, C and z share one run-time dtype in the kernel
-        par = [t for t in (B, C_, z) if t is not None]
-        pd = X.dtype if all(t.dtype == X.dtype for t in par) else torch.float32  # the kernels take X's element type or fp32
-        self.par = _CODES[pd]
-        self.B, self.C = _c(B.to(pd)), _c(C_.to(pd))
-        self.z = None if z is None else _c(z.to(pd))
-        self.D = _f32(D)
-        self.init = _f32(initial_states)
-        self.lens = _seq_lens(seq_meta, nb, nl, X.device)
-
-    def fill(self, a: L.ChunkArgs) -> None:
-        nb, nl, nh, npj = self.shape
-        a.batch, a.len, a.heads, a.proj = nb, nl, nh, npj
-        a.io_dtype, a.par_dtype, a.chunk_size = self.io, self.par, self.chunk
-        a.X, a.dt = _p(self.X), _p(self.dt)
-        _set_bc4(a.A, *_bc4(self.A, self.kA))
-        _set_bc4(a.Bm, *_bc4(self.B, self.kB))
-        _set_bc4(a.Cm, *_bc4(self.C, self.kC))
-        _set_bc4(a.D, *_bc4(self.D, self.kD or "h"))
-        _set_bc4(a.z, *_bc4(self.z, self.kz or "blh"))
-        _set_bc4(a.initial, *_bc4(self.init, "bhp"))
-        a.seq_lens = _p(self.lens)
-
-
-def _chunk_forward(cc: _ChunkCtx, want_final: bool = False):
-    nb, nl, nh, npj = cc.shape
-    lib = L.load()
-    Y = torch.empty_like(cc.X)
-    final = torch.empty(nb, nh, npj, dtype=torch.float32, device=cc.X.device) if want_final else None
-    n = lib.ssm_chunk_scan_scratch_floats(nb, nl, nh, npj, cc.chunk)
-    scratch = torch.empty(max(int(n), 1), dtype=torch.float32, device=cc.X.device)
-    a = L.ChunkArgs()
-    cc.fill(a)
-    a.Y, a.final_state, a.scratch = _p(Y), _p(final), _p(scratch)
-    _call(lib.ssm_chunk_scan_fwd, a)
-    return Y, final
-
-
-class _ChunkScanFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, X, dt, A, B, C_, chunk_size, D, z, seq_meta, initial_states):
-        cc = _ChunkCtx(X, dt, A, B, C_, chunk_size, D, z, seq_meta, initial_states)
-        Y, _ = _chunk_forward(cc)
-        ctx.cc = cc
-        ctx.like = (dt, A, B, C_, D, z, initial_states)
-        _guard(ctx, X, dt, A, B, C_, D, z, initial_states)
-        return Y
-
-    @staticmethod
-    def backward(ctx, gY):
-        _check_guard(ctx)
-        cc: _ChunkCtx = ctx.cc
-        dt, A, B, C_, D, z, init = ctx.like
-        nb, nl, nh, npj = cc.shape
-        lib = L.load()
-        dev = cc.X.device
-        zeros = lambda t: None if t is None else torch.zeros(t.shape, dtype=torch.float32, device=dev)  # noqa: E731
-        dX = torch.empty_like(cc.X)
-        ddt = torch.zeros(nb, nl, nh, dtype=torch.float32, device=dev)
-        # per-token B / C / z: their gradients are written by the kernel in the tensor's own type (no zero-fill, no fp32 copy)
-        typed = [t is not None and k == "blhp" for t, k in ((cc.B, cc.kB), (cc.C, cc.kC), (cc.z, cc.kz))]
-        own = lambda t, ty: torch.empty_like(t) if ty else zeros(t)  # noqa: E731
-        dA, dB, dC, dD, dz, dI = zeros(cc.A), own(cc.B, typed[0]), own(cc.C, typed[1]), zeros(cc.D), own(cc.z, typed[2]), zeros(cc.init)
-        hist = torch.empty(nb, max(nl, 1), nh, npj, dtype=torch.float32, device=dev)
-        g = L.ChunkBwdArgs()
-        cc.fill(g.fwd)
-        g.fwd.typed_grads = sum(1 << i for i, ty in enumerate(typed) if ty)
-        gy = _c(gY.to(cc.X.dtype))
-        scratch = torch.empty(max(1, int(lib.ssm_chunk_scan_bwd_scratch_floats(nb, nl, nh, npj, cc.chunk))), dtype=torch.float32, device=dev)
-        g.dY, g.dX, g.ddt, g.history, g.scratch = _p(gy), _p(dX), _p(ddt), _p(hist), _p(scratch)
-        _set_bc4(g.dA, *_bc4(dA, cc.kA))
-        _set_bc4(g.dB, *_bc4(dB, cc.kB))
-        _set_bc4(g.dC, *_bc4(dC, cc.kC))
-        _set_bc4(g.dD, *_bc4(dD, cc.kD or "h"))
-        _set_bc4(g.dz, *_bc4(dz, cc.kz or "blh"))
-        _set_bc4(g.dinitial, *_bc4(dI, "bhp"))
-        _call(lib.ssm_chunk_scan_bwd, g)
-        return (
-            dX, ddt.to(dt.dtype), dA.to(A.dtype), dB.to(B.dtype), dC.to(C_.dtype), None,
-            None if D is None else dD.to(D.dtype),
-            None if z is None else dz.to(z.dtype),
-            None,
-            None if init is None else dI.to(init.dtype),
-        )
 
 
 def ssd_chunk_scan(
@@ -814,90 +375,19 @@ def ssd_chunk_scan(
     if X.dtype == torch.float64:
         from . import ops_f64
         return ops_f64.ssd_chunk_scan(X, dt, A, B, C, chunk_size, D, z, seq_meta, initial_states)
-    return _ChunkScanFn.apply(X, dt, A, B, C, chunk_size, D, z, seq_meta, initial_states)
+    lens = cu = None
+    if seq_meta:  # valid lengths per row (reference.py:413-428)
+        lens, cu = seq_meta.get("seq_lens"), seq_meta.get("cu_seqlens")
+        if cu is None and lens is None:
+            raise ValueError("seq_meta must provide cu_seqlens or seq_lens.")
+        cu = None if cu is None else torch.as_tensor(cu)
+        lens = None if lens is None or cu is not None else torch.as_tensor(lens)
+    return _native().ssd_chunk_scan(X, dt, A, B, C, int(chunk_size), D, z, lens, cu, initial_states)
 
 
 # =========================================================================================
 # dw_causal_conv
 # =========================================================================================
-
-
-class _ConvCtx:
-    def __init__(self, x, weight, bias, activation, halo=None):
-        if x.ndim != 3:
-            raise ValueError("x must have shape (B, C, L) or (B, L, C).")
-        nc = weight.shape[0]
-        if x.shape[1] == nc:
-            self.first = True
-        elif x.shape[2] == nc:
-            self.first = False
-        else:
-            raise ValueError("weight channel dimension must match x.")
-        if weight.ndim == 3:
-            if weight.shape[1] != 1:
-                raise ValueError("Expected depthwise weights with shape (C, 1, K).")
-            w2 = weight[:, 0, :]
-        elif weight.ndim == 2:
-            w2 = weight
-        else:
-            raise ValueError("weight must have 2 or 3 dimensions.")
-        if bias is not None and tuple(bias.shape) != (nc,):
-            raise ValueError("bias must have shape (C,).")
-        act = str(activation).lower()
-        if act not in ("silu", "swish", "identity", "none"):
-            raise ValueError(f"Unsupported activation '{activation}'.")
-        k = w2.shape[1]
-        if k < 1 or k > 8:
-            raise ValueError("dw_causal_conv: kernel width must be in [1, 8].")
-        _need_cuda(x, weight, bias, halo)
-        self.silu = act in ("silu", "swish")
-        self.io = _code(x, "dw_causal_conv")
-        self.x, self.w, self.b = (_rows(x) if self.first else _c(x)), _f32(w2), _f32(bias)
-        self.nb = x.shape[0]
-        self.nc, self.k = nc, k
-        self.nl = x.shape[2] if self.first else x.shape[1]
-        if halo is not None and tuple(halo.shape) != (self.nb, nc, k - 1):
-            raise ValueError("halo must have shape (B, C, K-1).")
-        self.halo = _f32(halo)
-
-    def fill(self, a: L.ConvArgs) -> None:
-        a.batch, a.channels, a.len, a.width = self.nb, self.nc, self.nl, self.k
-        a.io_dtype, a.channels_first, a.silu = self.io, int(self.first), int(self.silu)
-        a.x, a.weight, a.bias, a.halo = _p(self.x), _p(self.w), _p(self.b), _p(self.halo)
-        if self.first and self.x.numel():
-            a.row_sb, a.row_sc = self.x.stride(0), self.x.stride(1)
-        else:
-            a.row_sb, a.row_sc = self.nc * self.nl, self.nl
-
-
-class _ConvFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, activation, halo):
-        cc = _ConvCtx(x, weight, bias, activation, halo)
-        y = torch.empty_like(cc.x)
-        a = L.ConvArgs()
-        cc.fill(a)
-        a.y = _p(y)
-        _call(L.load().ssm_dw_causal_conv_fwd, a)
-        ctx.cc, ctx.like = cc, (weight, bias)
-        _guard(ctx, x, weight, bias)
-        return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        _check_guard(ctx)
-        cc: _ConvCtx = ctx.cc
-        weight, bias = ctx.like
-        dev = cc.x.device
-        dx = torch.empty_like(cc.x)
-        dw = torch.zeros(cc.nc, cc.k, dtype=torch.float32, device=dev)
-        db = torch.zeros(cc.nc, dtype=torch.float32, device=dev) if bias is not None else None
-        g = L.ConvBwdArgs()
-        cc.fill(g.fwd)
-        go = _rows_like(gy, cc.x)
-        g.dy, g.dx, g.dweight, g.dbias = _p(go), _p(dx), _p(dw), _p(db)
-        _call(L.load().ssm_dw_causal_conv_bwd, g)
-        return dx, dw.view(weight.shape).to(weight.dtype), None if bias is None else db.to(bias.dtype), None, None
 
 
 def dw_causal_conv(x: Tensor, weight: Tensor, bias: Optional[Tensor] = None, activation: str = "silu",
@@ -910,7 +400,7 @@ def dw_causal_conv(x: Tensor, weight: Tensor, bias: Optional[Tensor] = None, act
             raise ValueError("dw_causal_conv in float64 takes no halo.")
         from . import ops_f64
         return ops_f64.dw_causal_conv(x, weight, bias, activation)
-    return _ConvFn.apply(x, weight, bias, activation, halo)
+    return _native().dw_causal_conv(x, weight, bias, str(activation), halo)
 
 
 def dw_causal_conv_update(conv_state: Tensor, x: Tensor, weight: Tensor, bias: Optional[Tensor] = None,
@@ -918,25 +408,7 @@ def dw_causal_conv_update(conv_state: Tensor, x: Tensor, weight: Tensor, bias: O
     """Extension: decode-time conv.  Rolls ``conv_state (B, C, K)`` (fp32, in place) left by one,
     appends ``x (B, C)`` and returns ``act(bias + <conv_state, weight>)`` (what upstream's
     ``Mamba1.step`` does with ``torch.roll``, modules/mamba1.py:345-353)."""
-    if conv_state.ndim != 3 or x.ndim != 2 or conv_state.shape[:2] != x.shape:
-        raise ValueError("conv_state must be (B, C, K) and x (B, C).")
-    w2 = weight[:, 0, :] if weight.ndim == 3 else weight
-    if tuple(w2.shape) != (x.shape[1], conv_state.shape[2]):
-        raise ValueError("weight must have shape (C, K).")
-    _need_cuda(conv_state, x, weight, bias)
-    if conv_state.dtype != torch.float32 or not conv_state.is_contiguous():
-        raise ValueError("conv_state must be a contiguous float32 tensor.")
-    act = str(activation).lower()
-    if act not in ("silu", "swish", "identity", "none"):
-        raise ValueError(f"Unsupported activation '{activation}'.")
-    xs, w32, b32 = _c(x), _f32(w2), _f32(bias)
-    out = torch.empty_like(xs)
-    a = L.ConvUpdateArgs()
-    a.batch, a.channels, a.width, a.io_dtype = x.shape[0], x.shape[1], conv_state.shape[2], _code(x, "dw_causal_conv_update")
-    a.silu = int(act in ("silu", "swish"))
-    a.conv_state, a.x, a.weight, a.bias, a.out = _p(conv_state), _p(xs), _p(w32), _p(b32), _p(out)
-    _call(L.load().ssm_dw_causal_conv_update, a)
-    return out
+    return _native().dw_causal_conv_update(conv_state, x, weight, bias, str(activation))
 
 
 # =========================================================================================
@@ -970,57 +442,6 @@ class _NormCtx:
         a.x, a.residual, a.weight, a.bias = _p(self.x), _p(self.res), _p(self.w), _p(self.b)
 
 
-class _NormFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, residual, is_rms, eps, prenorm, return_residual, residual_dtype):
-        nc = _NormCtx(x, weight, bias, residual, is_rms, eps, prenorm)
-        y = torch.empty_like(nc.x)
-        ro = torch.empty(nc.x.shape, dtype=residual_dtype, device=nc.x.device) if return_residual else None
-        a = L.NormArgs()
-        nc.fill(a)
-        a.y, a.residual_out = _p(y), _p(ro)
-        a.resout_dtype = _CODES[residual_dtype] if return_residual else 0
-        _call(L.load().ssm_fused_add_norm_fwd, a)
-        ctx.nc, ctx.like = nc, (weight, bias, residual)
-        ctx.res_dtype = residual_dtype
-        _guard(ctx, x, weight, bias, residual)
-        if return_residual:
-            return y, ro
-        return y
-
-    @staticmethod
-    def backward(ctx, gy, gro=None):
-        _check_guard(ctx)
-        nc: _NormCtx = ctx.nc
-        weight, bias, residual = ctx.like
-        if gy is None:
-            gy = torch.zeros_like(nc.x)
-        lib = L.load()
-        dev = nc.x.device
-        hidden = nc.x.shape[2]
-        rows = nc.x.shape[0] * nc.x.shape[1]
-        dx = torch.empty_like(nc.x)
-        dres = torch.empty_like(nc.res) if nc.res is not None else None
-        dw = torch.empty(hidden, dtype=torch.float32, device=dev)
-        db = torch.empty(hidden, dtype=torch.float32, device=dev) if bias is not None else None
-        partial = torch.empty(int(lib.ssm_norm_bwd_scratch_floats(rows, hidden)), dtype=torch.float32, device=dev)
-        g = L.NormBwdArgs()
-        nc.fill(g.fwd)
-        go = _c(gy.to(nc.x.dtype))
-        g.dy, g.dx, g.dresidual, g.dweight, g.dbias, g.partial = _p(go), _p(dx), _p(dres), _p(dw), _p(db), _p(partial)
-        gr = None
-        if gro is not None:  # gradient arriving through the x + residual output: added to dx and dresidual inside the kernel
-            gr = _c(gro.to(ctx.res_dtype))
-            g.fwd.resout_dtype = _CODES[ctx.res_dtype]
-            g.dresidual_out = _p(gr)
-        _call(lib.ssm_fused_add_norm_bwd, g)
-        return (
-            dx, dw.to(weight.dtype), None if bias is None else db.to(bias.dtype),
-            None if residual is None else dres.to(residual.dtype),
-            None, None, None, None, None,
-        )
-
-
 def fused_layer_norm(
     x: Tensor,
     weight: Tensor,
@@ -1040,8 +461,7 @@ def fused_layer_norm(
     if x.dtype == torch.float64:
         from . import ops_f64
         return ops_f64.fused_layer_norm(x, weight, bias, residual, is_rms, eps, prenorm, residual_in_fp32, return_residual)
-    rd = torch.float32 if residual_in_fp32 else x.dtype
-    return _NormFn.apply(x, weight, bias, residual, is_rms, eps, prenorm, return_residual, rd)
+    return _native().fused_layer_norm(x, weight, bias, residual, is_rms, float(eps), prenorm, residual_in_fp32, return_residual)
 
 
 # =========================================================================================
@@ -1149,7 +569,6 @@ class _SsdWorkspace:
             self.states_f32 = torch.empty(nb, self.nchunks, nh, npj * nn, dtype=torch.float32, device=dev)
         a.ws_state_in_f32 = _p(self.states_f32)
         _call(L.load().ssm_ssd_fwd, a)
-        self._status.after_launch()
         return Y, final
 
     def states_before_chunks(self) -> Tensor:
@@ -1173,12 +592,6 @@ class _SsdWorkspace:
         vec = nb * nh * self.nchunks * self.chunk
         cum = self.ws[vec * 4: 2 * vec * 4].view(torch.float32).view(nb, nh, self.nchunks, self.chunk)
         return cum[..., -1].sum(-1) * math.log(2.0)  # the scratch holds base-2 exponents
-
-
-def _ssd_tensor_core(X, dt, A, B, C_, D, z, dt_bias, dt_softplus, initial_states, chunk_size):
-    w = _SsdWorkspace(X, dt, A, B, C_, D, z, dt_bias, dt_softplus, chunk_size)
-    Y, final = w.run(0, initial_states, True)
-    return Y, final, w.status
 
 
 def ssd_tensor_core_supported(X: Tensor, B: Tensor, chunk_size: int) -> bool:
@@ -1329,7 +742,7 @@ class _SsdFn(torch.autograd.Function):
         ctx.chunk = int(chunk_size)
         ctx.dual = bool(dual_backward) and ssd_tensor_core_supported(X, B, chunk_size)
         if ssd_tensor_core_supported(X, B, chunk_size):
-            Y, final, _ = _ssd_tensor_core(X, dt, A, B, C_, D, z, dt_bias, dt_softplus, initial_states, int(chunk_size))
+            Y, final = _native().ssd_forward(X, dt, A, B, C_, D, z, dt_bias, dt_softplus, initial_states, int(chunk_size))
             if check_status:
                 ssd_check_status(X.device)
             return Y, final

@@ -163,6 +163,7 @@ typedef struct {
   const float* D;       /* nullable */
   const float* dt_bias; /* nullable */
   void* out;
+  int32_t a_log, reserved0; /* a_log: A holds log(-A) (forward only) */
 } ssm_step_args;
 
 int ssm_selective_state_step(const ssm_step_args* args, ssm_stream_t stream);
@@ -287,11 +288,11 @@ int ssm_dw_causal_conv_bwd(const ssm_conv_bwd_args* args, ssm_stream_t stream);
  * out = silu?(bias + <conv_state, weight>). */
 typedef struct {
   int32_t batch, channels, width, io_dtype;
-  int32_t silu, reserved0;
+  int32_t silu, param_dtype; /* param_dtype: element type of weight and bias (0: fp32) */
   float* conv_state;
   const void* x;
-  const float* weight;
-  const float* bias; /* nullable */
+  const void* weight;
+  const void* bias; /* nullable */
   void* out;
 } ssm_conv_update_args;
 
@@ -302,24 +303,26 @@ int ssm_dw_causal_conv_update(const ssm_conv_update_args* args, ssm_stream_t str
  * fused_layer_norm_backward_cuda (src/ssm/ops/cuda/layer_norm.cu:372-496, 498-676; spec
  * reference.py:540-609).
  *
- * x, y: (rows, hidden) io_dtype.  residual: res_dtype or NULL.  weight, bias fp32.
+ * x, y: (rows, hidden) io_dtype.  residual: res_dtype or NULL.  weight, bias: param_dtype.
  * prenorm: y = norm(x + residual)*w + b, else y = norm(x)*w + b + residual.
  * All arithmetic is fp32 (upstream's residual_in_fp32 only matters for fp64 inputs, which
  * are not built).  hidden <= 16384 (16-bit) / 8192 (fp32).  residual_out: optional
  * (rows, hidden) of resout_dtype receiving x + residual (additive extension).
- * Backward: dx io_dtype, dresidual res_dtype (NULL iff residual NULL); dweight, dbias fp32
- * (hidden) written (not accumulated); partial: scratch fp32 of
+ * Backward: dx io_dtype, dresidual res_dtype (NULL iff residual NULL); dweight, dbias
+ * (hidden), dparam_dtype, written (not accumulated); partial: scratch fp32 of
  * ssm_norm_bwd_scratch_floats(rows, hidden) floats.
  * ------------------------------------------------------------------------------------- */
 typedef struct {
   int64_t rows;
   int32_t hidden, io_dtype, res_dtype, resout_dtype;
-  int32_t is_rms, prenorm, reserved0, reserved2;
+  int32_t is_rms, prenorm;
+  int32_t param_dtype; /* element type of weight and bias (0: fp32) */
+  int32_t dparam_dtype; /* backward: element type of dweight and dbias as written (0: fp32) */
   float eps, reserved1;
   const void* x;
   const void* residual; /* nullable */
-  const float* weight;
-  const float* bias; /* nullable */
+  const void* weight; /* param_dtype */
+  const void* bias;   /* param_dtype, nullable */
   void* y;
   void* residual_out; /* nullable */
 } ssm_norm_args;
@@ -331,8 +334,8 @@ typedef struct {
   const void* dy;
   void* dx;
   void* dresidual; /* nullable */
-  float* dweight;
-  float* dbias; /* nullable */
+  void* dweight; /* fwd.dparam_dtype */
+  void* dbias;   /* fwd.dparam_dtype, nullable */
   float* partial;
   const void* dresidual_out; /* nullable: gradient arriving through residual_out, (rows, hidden) of fwd.resout_dtype; added to dx and dresidual */
 } ssm_norm_bwd_args;
@@ -500,6 +503,83 @@ int ssm_ssd_bwd_group_sum(const void* y, const float* weight, void* out, int32_t
 int ssm_ssd_bwd_spread(const void* src, void* dst, int64_t rows, int32_t heads, int32_t groups, int64_t row_bytes, ssm_stream_t stream);
 int ssm_ssd_state_dot(const void* fwd_states, const void* adj_states, float* out, int32_t batch, int32_t nchunks, int32_t heads, int32_t elems,
                       int32_t io_dtype, ssm_stream_t stream);
+
+/* ---------------------------------------------------------------------------------------
+ * One decode token through a whole mixer in one launch (no counterpart upstream, whose step methods are sequences of
+ * operator calls: src/ssm/modules/mamba1.py:324-385).  For up to 16 sequences, bf16 / fp16 activations and projection
+ * weights (io_dtype), conv width 4; ssm_mamba*_decode_supported() says whether a shape is built.  hidden (batch, d_model).
+ * Weights as in ssm_b200/mixer.py, row-major (out, in): io_dtype; dt_bias, A, D fp32.  a_log: A holds log(-A).  States fp32,
+ * updated in place.  scratch: ssm_mamba*_decode_scratch_bytes() bytes.
+ * Mamba-1: out is the mixer's output (batch, d_model), or, with norm_w, RMSNorm(residual + mixer output) * norm_w with the
+ * sum written to residual_out (residual nullable).  The state is (batch, d_inner, 16).
+ * Mamba-2: out is the mixer's output; norm_w (d_inner) is the gated norm in front of the out projection.  The state is
+ * (batch, heads, 64, 128).
+ * ------------------------------------------------------------------------------------- */
+typedef struct {
+  int32_t batch, d_model, d_inner, nstate;
+  int32_t dt_rank, width, io_dtype, a_log;
+  int32_t res_dtype, resout_dtype;
+  float eps;
+  int32_t reserved0;
+  const void* hidden;
+  const void* in_x;
+  const void* in_z;
+  const void* conv_w;
+  const void* conv_b; /* nullable */
+  const void* x_proj;
+  const void* dt_proj;
+  const float* dt_bias;
+  const float* A;
+  const float* D;
+  const void* out_proj;
+  const void* norm_w;   /* nullable */
+  const void* residual; /* nullable */
+  float* conv_state;
+  float* ssm_state;
+  void* out;
+  void* residual_out; /* with norm_w */
+  void* scratch;
+} ssm_mamba1_decode_args;
+
+int ssm_mamba1_decode_supported(int32_t batch, int32_t d_model, int32_t d_inner, int32_t nstate, int32_t dt_rank, int32_t width, int32_t io_dtype);
+int64_t ssm_mamba1_decode_scratch_bytes(int32_t batch, int32_t d_model, int32_t d_inner, int32_t nstate, int32_t dt_rank);
+int ssm_mamba1_decode(const ssm_mamba1_decode_args* args, ssm_stream_t stream);
+
+typedef struct {
+  int32_t batch, d_model, heads, headdim;
+  int32_t nstate, groups, width, io_dtype;
+  int32_t a_log, reserved0;
+  float eps;
+  int32_t reserved1;
+  const void* hidden;
+  const void* in_z;
+  const void* in_x;
+  const void* in_B;
+  const void* in_C;
+  const void* in_dt;
+  const void* conv_x_w;
+  const void* conv_x_b; /* nullable, as the other two biases */
+  const void* conv_B_w;
+  const void* conv_B_b;
+  const void* conv_C_w;
+  const void* conv_C_b;
+  const float* dt_bias;
+  const float* A;
+  const float* D;
+  const void* norm_w;
+  const void* out_proj;
+  float* conv_state_x;
+  float* conv_state_B;
+  float* conv_state_C;
+  float* ssm_state;
+  void* out;
+  void* scratch;
+} ssm_mamba2_decode_args;
+
+int ssm_mamba2_decode_supported(int32_t batch, int32_t d_model, int32_t heads, int32_t headdim, int32_t nstate, int32_t groups, int32_t width,
+                                int32_t io_dtype);
+int64_t ssm_mamba2_decode_scratch_bytes(int32_t batch, int32_t heads, int32_t groups);
+int ssm_mamba2_decode(const ssm_mamba2_decode_args* args, ssm_stream_t stream);
 
 #ifdef __cplusplus
 }

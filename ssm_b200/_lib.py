@@ -50,7 +50,7 @@ class StepArgs(C.Structure):
         ("state", fp), ("x", vp), ("dt", vp), ("z", vp), ("A", fp), ("Bm", vp), ("Cm", vp),
         ("b_sb", i64), ("b_sg", i64), ("b_sn", i64),
         ("c_sb", i64), ("c_sg", i64), ("c_sn", i64),
-        ("D", fp), ("dt_bias", fp), ("out", vp),
+        ("D", fp), ("dt_bias", fp), ("out", vp), ("a_log", i32), ("reserved0", i32),
     ]
 
 
@@ -102,7 +102,7 @@ class ConvBwdArgs(C.Structure):
 class ConvUpdateArgs(C.Structure):
     _fields_ = [
         ("batch", i32), ("channels", i32), ("width", i32), ("io_dtype", i32),
-        ("silu", i32), ("reserved0", i32),
+        ("silu", i32), ("param_dtype", i32),
         ("conv_state", fp), ("x", vp), ("weight", fp), ("bias", fp), ("out", vp),
     ]
 
@@ -111,7 +111,7 @@ class NormArgs(C.Structure):
     _fields_ = [
         ("rows", i64),
         ("hidden", i32), ("io_dtype", i32), ("res_dtype", i32), ("resout_dtype", i32),
-        ("is_rms", i32), ("prenorm", i32), ("reserved0", i32), ("reserved2", i32),
+        ("is_rms", i32), ("prenorm", i32), ("param_dtype", i32), ("dparam_dtype", i32),
         ("eps", C.c_float), ("reserved1", C.c_float),
         ("x", vp), ("residual", vp), ("weight", fp), ("bias", fp), ("y", vp), ("residual_out", vp),
     ]
@@ -152,6 +152,12 @@ ENTRY_POINTS = {
     "ssm_scan_split_segments": (C.c_int, [i32, i32, i32, i32]),
     "ssm_selective_scan_fwd": (C.c_int, [C.POINTER(ScanFwdArgs), vp]),
     "ssm_selective_scan_bwd": (C.c_int, [C.POINTER(ScanBwdArgs), vp]),
+    "ssm_mamba1_decode_supported": (C.c_int, [i32] * 7),
+    "ssm_mamba1_decode_scratch_bytes": (C.c_int64, [i32] * 5),
+    "ssm_mamba1_decode": (C.c_int, [vp, vp]),
+    "ssm_mamba2_decode_supported": (C.c_int, [i32] * 8),
+    "ssm_mamba2_decode_scratch_bytes": (C.c_int64, [i32] * 3),
+    "ssm_mamba2_decode": (C.c_int, [vp, vp]),
     "ssm_selective_state_step": (C.c_int, [C.POINTER(StepArgs), vp]),
     "ssm_selective_state_step_bwd": (C.c_int, [C.POINTER(StepBwdArgs), vp]),
     "ssm_chunk_scan_scratch_floats": (C.c_int64, [i32, i32, i32, i32, i32]),

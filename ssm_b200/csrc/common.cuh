@@ -85,6 +85,30 @@ __device__ __forceinline__ void store_dyn(void* base, int64_t i, int dtype, floa
   else reinterpret_cast<__half*>(base)[i] = __float2half_rn(v);
 }
 
+// V consecutive parameter values (weights, biases) of run-time type -> fp32; aligned to the vector, read through L1
+template <int V>
+__device__ __forceinline__ void load_param_vec(const void* base, int64_t i, int dtype, float (&f)[V]) {
+  if (dtype == SSM_F32) {
+#pragma unroll
+    for (int k = 0; k < V; k += 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i + k));
+      f[k] = v.x, f[k + 1] = v.y, f[k + 2] = v.z, f[k + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < V; k += 4) {
+      const uint2 raw = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(base) + i + k));
+      if (dtype == SSM_BF16) {
+        f[k] = __uint_as_float(raw.x << 16), f[k + 1] = __uint_as_float(raw.x & 0xffff0000u);
+        f[k + 2] = __uint_as_float(raw.y << 16), f[k + 3] = __uint_as_float(raw.y & 0xffff0000u);
+      } else {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+        f[k] = a.x, f[k + 1] = a.y, f[k + 2] = b.x, f[k + 3] = b.y;
+      }
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------
 // device: 16-byte vectors of T  (4 x fp32 or 8 x 16-bit)
 // ---------------------------------------------------------------------------------------

@@ -629,18 +629,19 @@ __global__ void __launch_bounds__(256) conv_update_kernel(const ssm_conv_update_
   const int c = (int)(i % a.channels), K = a.width;
   float* cs = a.conv_state + i * K;
   const float xn = to_f<T>(reinterpret_cast<const T*>(a.x)[i]);
-  float acc = a.bias ? __ldg(a.bias + c) : 0.f;
+  float acc = a.bias ? load_dyn(a.bias, c, a.param_dtype) : 0.f;
   if (K == 4 && aligned_to_dev(cs)) {
     float4 v = *reinterpret_cast<float4*>(cs);
     v = make_float4(v.y, v.z, v.w, xn);
     *reinterpret_cast<float4*>(cs) = v;
-    const float4 w = __ldg(reinterpret_cast<const float4*>(a.weight + (int64_t)c * 4));
-    acc = fmaf(v.x, w.x, fmaf(v.y, w.y, fmaf(v.z, w.z, fmaf(v.w, w.w, acc))));
+    float w[4];
+    load_param_vec<4>(a.weight, (int64_t)c * 4, a.param_dtype, w);
+    acc = fmaf(v.x, w[0], fmaf(v.y, w[1], fmaf(v.z, w[2], fmaf(v.w, w[3], acc))));
   } else {
     for (int j = 0; j < K; ++j) {
       const float v = j + 1 < K ? cs[j + 1] : xn;
       cs[j] = v;
-      acc = fmaf(v, __ldg(a.weight + (int64_t)c * K + j), acc);
+      acc = fmaf(v, load_dyn(a.weight, (int64_t)c * K + j, a.param_dtype), acc);
     }
   }
   reinterpret_cast<T*>(a.out)[i] = from_f<T>(a.silu ? silu_fast(acc) : acc);
@@ -757,7 +758,8 @@ extern "C" int ssm_dw_causal_conv_update(const ssm_conv_update_args* a, ssm_stre
   const int64_t n = (int64_t)a->batch * a->channels;
   if (n == 0) return SSM_OK;
   SSM_REQUIRE(a->conv_state && a->x && a->weight && a->out, SSM_ERR_NULL, "dw_causal_conv_update: missing pointer");
-  SSM_REQUIRE(a->width != 4 || aligned_to(a->weight, 16), SSM_ERR_ALIGN, "dw_causal_conv_update: weight must be 16-byte aligned");
+  SSM_REQUIRE(valid_dtype(a->param_dtype), SSM_ERR_DTYPE, "dw_causal_conv_update: unknown parameter dtype");
+  SSM_REQUIRE(a->width != 4 || aligned_to(a->weight, 4 * dtype_size(a->param_dtype)), SSM_ERR_ALIGN, "dw_causal_conv_update: weight must be aligned to four elements");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const unsigned grid = (unsigned)((n + 255) / 256);
   switch (a->io_dtype) {

@@ -270,12 +270,12 @@ __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK) norm_fwd_kernel(const ss
     const int ch = c * G + gt;
     if (ch < nchunk) {
       float o[V], wv[V], bv[V];
+load_param_vec<V>(a.weight, ch * V, a.param_dtype, wv);
+      if (a.bias) {
+        load_param_vec<V>(a.bias, ch * V, a.param_dtype, bv);
+      } else {
 #pragma unroll
-      for (int i = 0; i < V; i += 4) {  // weight / bias are fp32 and 16-byte aligned at every chunk (hidden % V == 0, V >= 4)
-        const float4 w4 = __ldg(reinterpret_cast<const float4*>(a.weight + ch * V + i));
-        wv[i] = w4.x, wv[i + 1] = w4.y, wv[i + 2] = w4.z, wv[i + 3] = w4.w;
-        const float4 b4 = a.bias ? __ldg(reinterpret_cast<const float4*>(a.bias + ch * V + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        bv[i] = b4.x, bv[i + 1] = b4.y, bv[i + 2] = b4.z, bv[i + 3] = b4.w;
+        for (int i = 0; i < V; ++i) bv[i] = 0.f;
       }
 #pragma unroll
       for (int i = 0; i < V; ++i) {
@@ -325,12 +325,7 @@ __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_min_ctas<G, MC>
     }
   // the weights of this thread's columns are re-read from L1 for every row (16-byte loads) instead of occupying registers
   auto load_w = [&](int c, float (&wv)[V]) {
-    const int ch = c * G + gt;
-#pragma unroll
-    for (int i = 0; i < V; i += 4) {
-      const float4 w4 = ch < nchunk ? __ldg(reinterpret_cast<const float4*>(a.weight + ch * V + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      wv[i] = w4.x, wv[i + 1] = w4.y, wv[i + 2] = w4.z, wv[i + 3] = w4.w;
-    }
+    load_param_vec<V>(a.weight, min(c * G + gt, nchunk - 1) * V, a.param_dtype, wv);  // beyond the row: dropped (dy is zero there)
   };
   const int64_t npass = (a.rows + Cfg::RPC - 1) / Cfg::RPC;
   for (int64_t pass = blockIdx.x; pass < npass; pass += gridDim.x) {
@@ -450,7 +445,7 @@ __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_min_ctas<G, MC>
 // so the loads of a column are spread over many threads instead of one serial chain.
 constexpr int kFoldLanes = 16;
 __global__ void __launch_bounds__(32 * kFoldLanes) norm_fold_kernel(const float* __restrict__ partial, int nctas, int hidden,
-                                                                   float* __restrict__ dweight, float* __restrict__ dbias) {
+                                                                   void* __restrict__ dweight, void* __restrict__ dbias, int dtype) {
   __shared__ float sw[kFoldLanes][33], sb[kFoldLanes][33];
   const int cx = threadIdx.x & 31, ky = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + cx;
@@ -467,8 +462,8 @@ __global__ void __launch_bounds__(32 * kFoldLanes) norm_fold_kernel(const float*
   if (ky == 0 && col < hidden) {
 #pragma unroll
     for (int k = 1; k < kFoldLanes; ++k) tw += sw[k][cx], tb += sb[k][cx];
-    dweight[col] = tw;
-    if (dbias) dbias[col] = tb;
+    store_dyn(dweight, col, dtype, tw);
+    if (dbias) store_dyn(dbias, col, dtype, tb);
   }
 }
 
@@ -509,8 +504,8 @@ __global__ void __launch_bounds__(128) norm_scalar_kernel(const ssm_norm_bwd_arg
   if (!BWD) {
     for (int c = threadIdx.x; c < a.hidden; c += 128) {
       const float sv = norm_s_at<T>(a, base + c);
-      float y = (sv - mean) * rstd * __ldg(a.weight + c);
-      if (a.bias) y += __ldg(a.bias + c);
+      float y = (sv - mean) * rstd * load_dyn(a.weight, c, a.param_dtype);
+      if (a.bias) y += load_dyn(a.bias, c, a.param_dtype);
       if (a.residual && !a.prenorm) y += load_dyn(a.residual, base + c, a.res_dtype);
       reinterpret_cast<T*>(a.y)[base + c] = from_f<T>(y);
       if (a.residual_out) {
@@ -524,11 +519,11 @@ __global__ void __launch_bounds__(128) norm_scalar_kernel(const ssm_norm_bwd_arg
     for (int c = threadIdx.x; c < a.hidden; c += 128) {
       const float xh = (norm_s_at<T>(a, base + c) - mean) * rstd;
       const float dyv = to_f<T>(reinterpret_cast<const T*>(g.dy)[base + c]);
-      const float wdy = dyv * __ldg(a.weight + c);
+      const float wdy = dyv * load_dyn(a.weight, c, a.param_dtype);
       c1 = fmaf(wdy, xh, c1);
       c2 += wdy;
-      atomicAdd(g.dweight + c, dyv * xh);
-      if (g.dbias) atomicAdd(g.dbias + c, dyv);
+      atomicAdd(g.partial + c, dyv * xh);
+      if (g.dbias) atomicAdd(g.partial + a.hidden + c, dyv);
     }
     c1 = block_allsum128(c1, scratch) * inv;
     c2 = a.is_rms ? 0.f : block_allsum128(c2, scratch) * inv;
@@ -536,7 +531,7 @@ __global__ void __launch_bounds__(128) norm_scalar_kernel(const ssm_norm_bwd_arg
       const float xh = (norm_s_at<T>(a, base + c) - mean) * rstd;
       const float dyv = to_f<T>(reinterpret_cast<const T*>(g.dy)[base + c]);
       const float gro = g.dresidual_out ? load_dyn(g.dresidual_out, base + c, a.resout_dtype) : 0.f;
-      const float ds = (dyv * __ldg(a.weight + c) - xh * c1 - c2) * rstd + gro;
+      const float ds = (dyv * load_dyn(a.weight, c, a.param_dtype) - xh * c1 - c2) * rstd + gro;
       reinterpret_cast<T*>(g.dx)[base + c] = from_f<T>(ds);
       if (g.dresidual) store_dyn(g.dresidual, base + c, a.res_dtype, a.prenorm ? ds : dyv + gro);
     }
@@ -549,6 +544,7 @@ static int norm_validate(const ssm_norm_args* a) {
   SSM_REQUIRE(valid_dtype(a->io_dtype), SSM_ERR_DTYPE, "fused_layer_norm: unknown dtype");
   SSM_REQUIRE(!a->residual || valid_dtype(a->res_dtype), SSM_ERR_DTYPE, "fused_layer_norm: unknown residual dtype");
   SSM_REQUIRE(!a->residual_out || valid_dtype(a->resout_dtype), SSM_ERR_DTYPE, "fused_layer_norm: unknown residual_out dtype");
+  SSM_REQUIRE(valid_dtype(a->param_dtype) && valid_dtype(a->dparam_dtype), SSM_ERR_DTYPE, "fused_layer_norm: unknown parameter dtype");
   SSM_REQUIRE(a->rows < (1ll << 31), SSM_ERR_TOO_LARGE, "fused_layer_norm: too many rows");
   return SSM_OK;
 }
@@ -599,7 +595,7 @@ static int norm_bwd_launch(const ssm_norm_bwd_args& g, cudaStream_t st, int max_
   if (nctas > resident) nctas = resident;
   norm_bwd_kernel<T, G, MC><<<nctas, Cfg::BLOCK, 0, st>>>(g);
   if (int rc = launch_status("norm_bwd_kernel")) return rc;
-  norm_fold_kernel<<<(g.fwd.hidden + 31) / 32, 32 * kFoldLanes, 0, st>>>(g.partial, nctas, g.fwd.hidden, g.dweight, g.dbias);
+  norm_fold_kernel<<<(g.fwd.hidden + 31) / 32, 32 * kFoldLanes, 0, st>>>(g.partial, nctas, g.fwd.hidden, g.dweight, g.dbias, g.fwd.dparam_dtype);
   return launch_status("norm_fold_kernel");
 }
 
@@ -633,14 +629,21 @@ static int norm_fwd_t(const ssm_norm_args& a, cudaStream_t st) {
     default: return nchunk <= 128 * 6 ? norm_fwd_launch<T, 128, 6>(a, st) : norm_fwd_launch<T, 512>(a, st);
   }
 }
+// rows that cannot be vectorised: sums by atomics into one partial row, folded into the element type of the gradients
+template <typename T>
+static int norm_bwd_scalar(const ssm_norm_bwd_args& g, cudaStream_t st) {
+  const int hidden = g.fwd.hidden;
+  cudaMemsetAsync(g.partial, 0, sizeof(float) * 2 * hidden, st);
+  norm_scalar_kernel<T, true><<<(unsigned)g.fwd.rows, 128, 0, st>>>(g);
+  if (int rc = launch_status("norm_scalar_kernel")) return rc;
+  norm_fold_kernel<<<(hidden + 31) / 32, 32 * kFoldLanes, 0, st>>>(g.partial, 1, hidden, g.dweight, g.dbias, g.fwd.dparam_dtype);
+  return launch_status("norm_fold_kernel");
+}
 template <typename T>
 static int norm_bwd_t(const ssm_norm_bwd_args& g, cudaStream_t st) {
   const ssm_norm_args& a = g.fwd;
   if (!norm_vec_ok(a, kNormBwdChunks, g.dy, g.dx, g.dresidual) || !aligned_to(g.dresidual_out, 16)) {
-    cudaMemsetAsync(g.dweight, 0, sizeof(float) * a.hidden, st);
-    if (g.dbias) cudaMemsetAsync(g.dbias, 0, sizeof(float) * a.hidden, st);
-    norm_scalar_kernel<T, true><<<(unsigned)a.rows, 128, 0, st>>>(g);
-    return launch_status("norm_scalar_kernel");
+    return norm_bwd_scalar<T>(g, st);
   }
   return norm_bwd_dispatch<T>(g, st, kNormBwdMaxCtas);
 }
@@ -691,15 +694,11 @@ static int noalloc_scratch_address(float** out) {
 template <typename T>
 static int norm_bwd_noalloc_t(const ssm_norm_bwd_args& g, float* scratch, cudaStream_t st) {
   const ssm_norm_args& a = g.fwd;
-  if (!norm_vec_ok(a, kNormBwdChunks, g.dy, g.dx, g.dresidual) || !aligned_to(g.dresidual_out, 16)) {
-    // rows that cannot be vectorised take the scalar kernel, which needs no scratch at all
-    cudaMemsetAsync(g.dweight, 0, sizeof(float) * a.hidden, st);
-    if (g.dbias) cudaMemsetAsync(g.dbias, 0, sizeof(float) * a.hidden, st);
-    norm_scalar_kernel<T, true><<<(unsigned)a.rows, 128, 0, st>>>(g);
-    return launch_status("norm_scalar_kernel");
-  }
   ssm_norm_bwd_args h = g;
   h.partial = scratch;
+  if (!norm_vec_ok(a, kNormBwdChunks, g.dy, g.dx, g.dresidual) || !aligned_to(g.dresidual_out, 16)) {
+    return norm_bwd_scalar<T>(h, st);
+  }
   return norm_bwd_dispatch<T>(h, st, kNoAllocCtas);
 }
 
@@ -737,8 +736,8 @@ extern "C" int ssm_fused_add_norm_bwd(const ssm_norm_bwd_args* g, ssm_stream_t s
   SSM_REQUIRE(g->dweight, SSM_ERR_NULL, "fused_layer_norm_backward: dweight is required");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (a->rows == 0) {
-    cudaMemsetAsync(g->dweight, 0, sizeof(float) * a->hidden, st);
-    if (g->dbias) cudaMemsetAsync(g->dbias, 0, sizeof(float) * a->hidden, st);
+    cudaMemsetAsync(g->dweight, 0, (size_t)dtype_size(a->dparam_dtype) * a->hidden, st);
+    if (g->dbias) cudaMemsetAsync(g->dbias, 0, (size_t)dtype_size(a->dparam_dtype) * a->hidden, st);
     return SSM_OK;
   }
   SSM_REQUIRE(a->x && a->weight && g->dy && g->dx && g->partial, SSM_ERR_NULL, "fused_layer_norm_backward: missing pointer");
@@ -760,8 +759,8 @@ extern "C" int ssm_fused_add_norm_bwd_noalloc(const ssm_norm_bwd_args* g, ssm_st
   SSM_REQUIRE(g->dweight, SSM_ERR_NULL, "fused_layer_norm_backward_noalloc: dweight is required");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (a->rows == 0) {
-    cudaMemsetAsync(g->dweight, 0, sizeof(float) * a->hidden, st);
-    if (g->dbias) cudaMemsetAsync(g->dbias, 0, sizeof(float) * a->hidden, st);
+    cudaMemsetAsync(g->dweight, 0, (size_t)dtype_size(a->dparam_dtype) * a->hidden, st);
+    if (g->dbias) cudaMemsetAsync(g->dbias, 0, (size_t)dtype_size(a->dparam_dtype) * a->hidden, st);
     return SSM_OK;
   }
   SSM_REQUIRE(a->x && a->weight && g->dy && g->dx, SSM_ERR_NULL, "fused_layer_norm_backward_noalloc: missing pointer");

@@ -10,6 +10,9 @@ namespace ssmb {
 
 constexpr int kStepThreads = 128;
 
+// A as stored, or from log(-A): a decode step then needs no pass of its own to form it
+__device__ __forceinline__ float step_A(const ssm_step_args& a, float v) { return a.a_log ? -expf(v) : v; }
+
 template <typename T, int LPR>
 __global__ void __launch_bounds__(kStepThreads) step_fwd_kernel(const ssm_step_args a, int vec) {
   const int64_t gid = (int64_t)blockIdx.x * kStepThreads + threadIdx.x;
@@ -40,7 +43,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_kernel(const ssm_step_a
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int n = n0 + i;
-        const float An = a.param_heads > 0 ? __ldg(a.A + head) : __ldg(a.A + (int64_t)d * N + n);
+        const float An = step_A(a, a.param_heads > 0 ? __ldg(a.A + head) : __ldg(a.A + (int64_t)d * N + n));
         const float Bn = load_dyn(a.Bm, boff + (int64_t)n * a.b_sn, a.bc_dtype);
         const float Cn = load_dyn(a.Cm, coff + (int64_t)n * a.c_sn, a.bc_dtype);
         sv[i] = fmaf(ex2_approx(dt * An * kLog2e), sv[i], dtx * Bn);
@@ -50,7 +53,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_kernel(const ssm_step_a
     }
   } else {
     for (int n = sg; n < N; n += LPR) {
-      const float An = a.param_heads > 0 ? __ldg(a.A + head) : __ldg(a.A + (int64_t)d * N + n);
+      const float An = step_A(a, a.param_heads > 0 ? __ldg(a.A + head) : __ldg(a.A + (int64_t)d * N + n));
       const float Bn = load_dyn(a.Bm, boff + (int64_t)n * a.b_sn, a.bc_dtype);
       const float Cn = load_dyn(a.Cm, coff + (int64_t)n * a.c_sn, a.bc_dtype);
       const float s = fmaf(ex2_approx(dt * An * kLog2e), st[n], dtx * Bn);
@@ -93,7 +96,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_vec_kernel(const ssm_st
   const int g = d / (a.dim / a.bc_groups);
   const int64_t boff = (int64_t)b * a.b_sb + (int64_t)g * a.b_sg;
   const int64_t coff = (int64_t)b * a.c_sb + (int64_t)g * a.c_sg;
-  const float Ahead = a.param_heads > 0 ? __ldg(a.A + head) * kLog2e : 0.f;
+  const float Ahead = a.param_heads > 0 ? step_A(a, __ldg(a.A + head)) * kLog2e : 0.f;
   float y = 0.f;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
@@ -103,7 +106,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_vec_kernel(const ssm_st
       An[0] = An[1] = An[2] = An[3] = Ahead;
     } else {
       const float4 q = __ldg(reinterpret_cast<const float4*>(a.A + (int64_t)d * N + n0));
-      An[0] = q.x * kLog2e, An[1] = q.y * kLog2e, An[2] = q.z * kLog2e, An[3] = q.w * kLog2e;
+      An[0] = step_A(a, q.x) * kLog2e, An[1] = step_A(a, q.y) * kLog2e, An[2] = step_A(a, q.z) * kLog2e, An[3] = step_A(a, q.w) * kLog2e;
     }
     float sv[4] = {s[v].x, s[v].y, s[v].z, s[v].w};
 #pragma unroll
@@ -167,7 +170,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_fast_kernel(const ssm_s
     load_bc4<BT>(a.Cm, coff + n0, Cv[v]);
     if (a.param_heads == 0) {
       const float4 q = __ldg(reinterpret_cast<const float4*>(a.A + (int64_t)d * N + n0));
-      An[v][0] = q.x * kLog2e, An[v][1] = q.y * kLog2e, An[v][2] = q.z * kLog2e, An[v][3] = q.w * kLog2e;
+      An[v][0] = step_A(a, q.x) * kLog2e, An[v][1] = step_A(a, q.y) * kLog2e, An[v][2] = step_A(a, q.z) * kLog2e, An[v][3] = step_A(a, q.w) * kLog2e;
     }
   }
   const float x = to_f<T>(reinterpret_cast<const T*>(a.x)[row]);
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_fast_kernel(const ssm_s
   const float dtx = dt * x;
   float y = 0.f;
   if (a.param_heads > 0) {  // one decay for the whole head: a single ex2 per thread
-    const float da = ex2_approx(dt * __ldg(a.A + head) * kLog2e);
+    const float da = ex2_approx(dt * step_A(a, __ldg(a.A + head)) * kLog2e);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       float sv[4] = {s[v].x, s[v].y, s[v].z, s[v].w};
@@ -401,6 +404,7 @@ extern "C" int ssm_selective_state_step_bwd(const ssm_step_bwd_args* g, ssm_stre
   if (a->io_dtype == SSM_F64) return f64_step(*g, true, reinterpret_cast<cudaStream_t>(stream));
   if (int rc = step_validate(a)) return rc;
   SSM_REQUIRE(a->param_heads == 0, SSM_ERR_UNSUPPORTED, "selective_state_step_backward: per-head parameters have no backward");
+  SSM_REQUIRE(a->a_log == 0, SSM_ERR_UNSUPPORTED, "selective_state_step_backward: A must be given as it is");
   if (a->batch == 0 || a->dim == 0) return SSM_OK;
   SSM_REQUIRE(g->dout && g->dstate && g->dx && g->ddt && g->dA && g->dB && g->dC, SSM_ERR_NULL,
               "selective_state_step_backward: missing pointer");

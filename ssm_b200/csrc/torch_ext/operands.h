@@ -211,7 +211,8 @@ struct StepCtx {
   bool softplus;
 
   StepCtx(const Tensor& state, const Tensor& x_, const Tensor& dt_, const Tensor& A_, const Tensor& B_, const Tensor& C_, const OptTensor& D_,
-          const OptTensor& z_, const OptTensor& bias_, bool softplus_)
+          const OptTensor& z_, const OptTensor& bias_, bool softplus_,
+          bool keep_views = false)
       : softplus(softplus_) {
     SSM_ARG(state.dim() == 3, "state must have shape (B, D, N).");
     SSM_ARG(x_.dim() == 2 && dt_.dim() == 2, "x and dt must have shape (B, D).");
@@ -222,7 +223,17 @@ struct StepCtx {
     need_cuda(state, {&D_, &z_, &bias_});
     dtype_code(x_, "selective_state_step");
     cb = step_coeff("B", B_, nb, nd, nn), cc = step_coeff("C", C_, nb, nd, nn);
-    B = B_.detach().contiguous(), C = C_.detach().contiguous();
+    // keep_views: a (B, G, N) view with contiguous states (a slice of a wider projection) is addressed where it lies.  Not for
+    // the backward pass, whose gradient buffers share the strides of B and C.
+    auto states = [&](const Tensor& t, StepCoeff& sc) {
+      Tensor d = t.detach();
+      if (keep_views && d.dim() == 3 && d.stride(2) == 1) {
+        sc.sb = d.stride(0), sc.sg = d.stride(1);
+        return d;
+      }
+      return d.contiguous();
+    };
+    B = states(B_, cb), C = states(C_, cc);
     if (cb.groups != cc.groups || B.scalar_type() != C.scalar_type() || !io_dtype_ok(B)) {
       auto expand = [&](Tensor t, StepCoeff& sc) {  // bring to per-channel fp32 (B, D, N) / (D, N)
         t = t.to(at::kFloat);
@@ -230,7 +241,7 @@ struct StepCtx {
         sc = t.dim() == 2 ? StepCoeff{(int)nd, 0, nn, 1} : StepCoeff{(int)nd, nd * nn, nn, 1};
         return t.contiguous();
       };
-      B = expand(B, cb), C = expand(C, cc);
+      B = expand(B, cb), C = expand(C, cc);  // contiguous
     }
     if (D_.has_value()) SSM_ARG(D_->dim() == 1 && D_->size(0) == nd, "D must have shape (D,).");
     if (z_.has_value()) SSM_ARG(z_->sizes() == x_.sizes(), "z must have shape (B, D).");
@@ -419,7 +430,14 @@ struct NormCtx {
     same_device(x_, {&weight});
     need_cuda(x_, {&bias, &residual});
     dtype_code(x_, "fused_layer_norm");
-    x = x_.detach().contiguous(), w = f32c(weight), b = f32c(bias);
+    x = x_.detach().contiguous();
+    // weight and bias go in as they are when they share a type that the kernels read
+    if (io_dtype_ok(weight) && (!bias.has_value() || bias->scalar_type() == weight.scalar_type())) {
+      w = weight.detach().contiguous();
+      if (bias.has_value()) b = bias->detach().contiguous();
+    } else {
+      w = f32c(weight), b = f32c(bias);
+    }
     if (residual.has_value()) {
       dtype_code(*residual, "fused_layer_norm residual");
       res = residual->detach().contiguous();
@@ -429,7 +447,8 @@ struct NormCtx {
     a.rows = x.size(0) * x.size(1), a.hidden = (int)x.size(2);
     a.io_dtype = dtype_code(x, "fused_layer_norm"), a.res_dtype = res.has_value() ? dtype_code(*res, "fused_layer_norm residual") : 0;
     a.is_rms = is_rms, a.prenorm = prenorm, a.eps = (float)eps;
-    a.x = x.data_ptr(), a.residual = ptr(res), a.weight = w.data_ptr<float>(), a.bias = fptr(b);
+    a.x = x.data_ptr(), a.residual = ptr(res), a.weight = w.data_ptr(), a.bias = ptr(b);
+    a.param_dtype = dtype_code(w, "fused_layer_norm");
   }
 };
 

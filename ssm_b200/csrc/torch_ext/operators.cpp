@@ -190,23 +190,23 @@ py::object selective_scan(const Tensor& u, const Tensor& delta, const Tensor& A,
 // single-token state steps (no gradients)
 // ---------------------------------------------------------------------------------------------
 Tensor state_step(const Tensor& state, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
-                  const OptTensor& z, const OptTensor& dt_bias, bool softplus) {
+                  const OptTensor& z, const OptTensor& dt_bias, bool softplus, bool a_log) {
   ValueErrors scope;
-  StepCtx c(state, x, dt, A, B, C, D, z, dt_bias, softplus);
+  StepCtx c(state, x, dt, A, B, C, D, z, dt_bias, softplus, true);
   c10::cuda::CUDAGuard guard(state.device());
   const bool direct = state.scalar_type() == at::kFloat && state.is_contiguous();
   Tensor work = direct ? state.detach() : f32c(state);
   Tensor out = at::empty_like(c.x);
   ssm_step_args a{};
   c.fill(a, work);
-  a.out = out.data_ptr();
+  a.out = out.data_ptr(), a.a_log = a_log;
   run(ssm_selective_state_step(&a, stream_of(state)));
   if (!direct) state.detach().copy_(work);
   return out;
 }
 
 Tensor state_step_heads(const Tensor& state, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
-                        const OptTensor& z, const OptTensor& dt_bias, bool softplus) {
+                        const OptTensor& z, const OptTensor& dt_bias, bool softplus, bool a_log) {
   ValueErrors scope;
   SSM_ARG(state.dim() == 4 && x.dim() == 3, "state must be (B, H, P, N) and x (B, H, P).");
   const int64_t nb = state.size(0), nh = state.size(1), np = state.size(2), nn = state.size(3);
@@ -231,7 +231,7 @@ Tensor state_step_heads(const Tensor& state, const Tensor& x, const Tensor& dt, 
   a.state = state.data_ptr<float>(), a.x = xs.data_ptr(), a.dt = dts.data_ptr(), a.z = ptr(zs), a.A = A32.data_ptr<float>();
   a.Bm = Bt.data_ptr(), a.Cm = Ct.data_ptr();
   a.b_sb = a.c_sb = g * nn, a.b_sg = a.c_sg = nn, a.b_sn = a.c_sn = 1;
-  a.D = fptr(D32), a.dt_bias = fptr(b32), a.out = out.data_ptr();
+  a.D = fptr(D32), a.dt_bias = fptr(b32), a.out = out.data_ptr(), a.a_log = a_log;
   run(ssm_selective_state_step(&a, stream_of(state)));
   return out;
 }
@@ -364,12 +364,15 @@ Tensor dw_causal_conv_update(const Tensor& conv_state, const Tensor& x, const Te
   SSM_ARG(conv_state.scalar_type() == at::kFloat && conv_state.is_contiguous(), "conv_state must be a contiguous float32 tensor.");
   const bool silu = is_silu(activation);
   c10::cuda::CUDAGuard guard(x.device());
-  Tensor xs = x.detach().contiguous(), w32 = f32c(w2), out = at::empty_like(xs);
-  OptTensor b32 = f32c(bias);
+  Tensor xs = x.detach().contiguous(), w = w2.detach().contiguous(), out = at::empty_like(xs);
+  OptTensor b = bias.has_value() ? OptTensor(bias->detach().contiguous()) : OptTensor();
+  if (!io_dtype_ok(w) || (b.has_value() && b->scalar_type() != w.scalar_type())) w = f32c(w), b = f32c(b);
+  if (reinterpret_cast<uintptr_t>(w.data_ptr()) % 16) w = w.clone();  // a view into another tensor
   ssm_conv_update_args a{};
   a.batch = (int)x.size(0), a.channels = (int)x.size(1), a.width = (int)conv_state.size(2), a.io_dtype = dtype_code(xs, "dw_causal_conv_update");
   a.silu = silu;
-  a.conv_state = conv_state.data_ptr<float>(), a.x = xs.data_ptr(), a.weight = w32.data_ptr<float>(), a.bias = fptr(b32), a.out = out.data_ptr();
+  a.conv_state = conv_state.data_ptr<float>(), a.x = xs.data_ptr(), a.weight = w.data_ptr(), a.bias = ptr(b), a.out = out.data_ptr();
+  a.param_dtype = dtype_code(w, "dw_causal_conv_update");
   run(ssm_dw_causal_conv_update(&a, stream_of(xs)));
   return out;
 }
@@ -410,14 +413,15 @@ struct NormCall final : Call {
     const auto f32 = c.x.options().dtype(at::kFloat);
     const int64_t rows = c.x.size(0) * c.x.size(1), hidden = c.x.size(2);
     Tensor go = grads[0].defined() ? like(grads[0], c.x) : at::zeros_like(c.x), gr;
-    Tensor dx = at::empty_like(c.x), dres, dw = at::empty({hidden}, f32), db;
+    Tensor dx = at::empty_like(c.x), dres, dw = at::empty({hidden}, c.w.options()), db;
     if (c.res.has_value()) dres = at::empty_like(*c.res);
-    if (c.b.has_value()) db = at::empty({hidden}, f32);
+    if (c.b.has_value()) db = at::empty({hidden}, c.w.options());
     Tensor partial = at::empty({ssm_norm_bwd_scratch_floats(rows, (int)hidden)}, f32);
     ssm_norm_bwd_args g{};
     c.fill(g.fwd);
     g.dy = go.data_ptr(), g.dx = dx.data_ptr(), g.dresidual = dres.defined() ? dres.data_ptr() : nullptr;
-    g.dweight = dw.data_ptr<float>(), g.dbias = out_ptr(db), g.partial = partial.data_ptr<float>();
+    g.fwd.dparam_dtype = g.fwd.param_dtype;
+    g.dweight = dw.data_ptr(), g.dbias = db.defined() ? db.data_ptr() : nullptr, g.partial = partial.data_ptr<float>();
     if (grads.size() > 1 && grads[1].defined()) {  // the gradient arriving through x + residual: added to dx and dresidual inside the kernel
       gr = grads[1].detach().to(res_type).contiguous();
       g.fwd.resout_dtype = dtype_code(gr, "fused_layer_norm"), g.dresidual_out = gr.data_ptr();
@@ -436,6 +440,112 @@ py::object fused_layer_norm(const Tensor& x, const Tensor& weight, const OptTens
   variable_list r = invoke_call(c10::make_intrusive<NormCall>(x, weight, bias, residual, is_rms, eps, prenorm, return_residual, residual_in_fp32));
   if (return_residual) return py::make_tuple(r[0], r[1]);
   return py::cast(r[0]);
+}
+
+// ---------------------------------------------------------------------------------------------
+// one decode token through a whole mixer (no gradients)
+// ---------------------------------------------------------------------------------------------
+bool plain(const Tensor& t, at::ScalarType type) {
+  return t.scalar_type() == type && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+}
+bool plain(const OptTensor& t, at::ScalarType type) { return !t.has_value() || plain(*t, type); }
+
+// Up to 16 sequences: one launch (ssm_mamba1_decode).  More: library GEMMs around the conv and state kernels.  With norm_w the
+// residual add and RMSNorm behind the mixer are included and the result is (normed, residual stream in fp32).
+py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tensor& conv_state, const Tensor& ssm_state, const Tensor& in_x, const Tensor& in_z,
+                       const Tensor& conv_w, const OptTensor& conv_b, const Tensor& x_proj, const Tensor& dt_proj, const Tensor& dt_bias, const Tensor& A,
+                       bool a_log, const Tensor& D, const Tensor& out_proj, const OptTensor& norm_w, double eps) {
+  ValueErrors scope;
+  at::NoGradGuard no_grad;
+  SSM_ARG(tok.dim() == 2 && tok.is_cuda(), "mamba1_step: tok must be a (B, d_model) CUDA tensor.");
+  const int64_t nb = tok.size(0), dm = tok.size(1), di = in_x.size(0), n = ssm_state.size(-1), r = dt_proj.size(1), k = conv_w.size(-1);
+  const auto T = tok.scalar_type();
+  const bool half = T == at::kBFloat16 || T == at::kHalf;
+  bool fused = half && plain(tok, T) && plain(conv_state, at::kFloat) && plain(ssm_state, at::kFloat) && plain(A, at::kFloat) && plain(D, at::kFloat) &&
+               plain(dt_bias, at::kFloat) && plain(conv_b, T) && plain(norm_w, T) && (!residual.has_value() || (residual->is_contiguous() && io_dtype_ok(*residual)));
+  for (const Tensor* w : {&in_x, &in_z, &conv_w, &x_proj, &dt_proj, &out_proj}) fused = fused && plain(*w, T);
+  fused = fused && in_x.sizes() == in_z.sizes() && in_x.size(1) == dm && conv_w.size(0) == di && x_proj.size(0) == r + 2 * n && x_proj.size(1) == di &&
+          dt_proj.size(0) == di && out_proj.size(0) == dm && out_proj.size(1) == di && conv_state.dim() == 3 && conv_state.size(0) == nb && conv_state.size(1) == di &&
+          conv_state.size(2) == k && ssm_state.dim() == 3 && ssm_state.size(0) == nb && ssm_state.size(1) == di && A.dim() == 2 && A.size(0) == di && A.size(1) == n &&
+          D.numel() == di && dt_bias.numel() == di && (!residual.has_value() || residual->numel() == nb * dm) &&
+          ssm_mamba1_decode_supported((int)nb, (int)dm, (int)di, (int)n, (int)r, (int)k, dtype_code(tok, "mamba1_step"));
+  if (fused) {
+    c10::cuda::CUDAGuard guard(tok.device());
+    Tensor out = at::empty_like(tok), res;
+    Tensor scratch = at::empty({ssm_mamba1_decode_scratch_bytes((int)nb, (int)dm, (int)di, (int)n, (int)r)}, tok.options().dtype(at::kByte));
+    ssm_mamba1_decode_args a{};
+    a.batch = (int)nb, a.d_model = (int)dm, a.d_inner = (int)di, a.nstate = (int)n, a.dt_rank = (int)r, a.width = (int)k;
+    a.io_dtype = dtype_code(tok, "mamba1_step"), a.a_log = a_log, a.eps = (float)eps;
+    a.hidden = tok.data_ptr(), a.in_x = in_x.data_ptr(), a.in_z = in_z.data_ptr(), a.conv_w = conv_w.data_ptr(), a.conv_b = ptr(conv_b);
+    a.x_proj = x_proj.data_ptr(), a.dt_proj = dt_proj.data_ptr(), a.dt_bias = dt_bias.data_ptr<float>(), a.A = A.data_ptr<float>(), a.D = D.data_ptr<float>();
+    a.out_proj = out_proj.data_ptr(), a.norm_w = ptr(norm_w);
+    a.conv_state = conv_state.data_ptr<float>(), a.ssm_state = ssm_state.data_ptr<float>(), a.out = out.data_ptr(), a.scratch = scratch.data_ptr();
+    if (norm_w.has_value()) {
+      res = at::empty({nb, dm}, tok.options().dtype(at::kFloat));
+      a.residual_out = res.data_ptr(), a.resout_dtype = SSM_F32;
+      if (residual.has_value()) a.residual = residual->data_ptr(), a.res_dtype = dtype_code(*residual, "mamba1_step residual");
+    }
+    run(ssm_mamba1_decode(&a, stream_of(tok)));
+    if (norm_w.has_value()) return py::make_tuple(out, res);
+    return py::cast(out);
+  }
+  Tensor x = at::matmul(tok, in_x.t()), z = at::matmul(tok, in_z.t());
+  Tensor u = dw_causal_conv_update(conv_state, x, conv_w, conv_b, "silu");
+  Tensor xd = at::matmul(u, x_proj.t());
+  Tensor delta = at::matmul(xd.narrow(1, 0, r), dt_proj.t());
+  Tensor y = state_step(ssm_state, u, delta, A, xd.narrow(1, r, n).unsqueeze(1), xd.narrow(1, r + n, n).unsqueeze(1), D, z, dt_bias, true, a_log);
+  Tensor out = at::matmul(y, out_proj.t());
+  if (!norm_w.has_value()) return py::cast(out);
+  OptTensor res = residual.has_value() ? OptTensor(residual->reshape({1, nb, dm})) : OptTensor();
+  variable_list rr = invoke_call(c10::make_intrusive<NormCall>(out.unsqueeze(0), *norm_w, OptTensor(), res, true, eps, true, true, true));
+  return py::make_tuple(rr[0].view({nb, dm}), rr[1].view({nb, dm}));
+}
+
+// The same for Mamba-2 (the gated norm is part of the mixer).
+Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B, const Tensor& conv_C, const Tensor& ssm_state, const Tensor& in_z,
+                   const Tensor& in_x, const Tensor& in_B, const Tensor& in_C, const Tensor& in_dt, const Tensor& wx, const OptTensor& bx, const Tensor& wB,
+                   const OptTensor& bB, const Tensor& wC, const OptTensor& bC, const Tensor& dt_bias, const Tensor& A, bool a_log, const Tensor& D,
+                   const Tensor& norm_w, const Tensor& out_proj, double eps) {
+  ValueErrors scope;
+  at::NoGradGuard no_grad;
+  SSM_ARG(tok.dim() == 2 && tok.is_cuda() && ssm_state.dim() == 4, "mamba2_step: tok must be a (B, d_model) CUDA tensor and the state (B, H, P, N).");
+  const int64_t nb = tok.size(0), dm = tok.size(1), nh = ssm_state.size(1), hp = ssm_state.size(2), n = ssm_state.size(3), di = nh * hp;
+  SSM_ARG(in_B.size(0) % n == 0, "mamba2_step: in_B must have groups * d_state rows.");
+  const int64_t g = in_B.size(0) / n, k = wx.size(-1);
+  const auto T = tok.scalar_type();
+  bool fused = (T == at::kBFloat16 || T == at::kHalf) && plain(tok, T) && plain(dt_bias, at::kFloat) && plain(A, at::kFloat) && plain(D, at::kFloat) &&
+               plain(bx, T) && plain(bB, T) && plain(bC, T);
+  for (const Tensor* t : {&conv_x, &conv_B, &conv_C, &ssm_state}) fused = fused && plain(*t, at::kFloat);
+  for (const Tensor* w : {&in_z, &in_x, &in_B, &in_C, &in_dt, &wx, &wB, &wC, &norm_w, &out_proj}) fused = fused && plain(*w, T);
+  for (const Tensor* w : {&in_z, &in_x, &in_B, &in_C, &in_dt}) fused = fused && w->dim() == 2 && w->size(1) == dm;
+  fused = fused && in_x.size(0) == di && in_z.size(0) == di && in_C.size(0) == g * n && in_dt.size(0) == nh && wx.numel() == di * k && wB.numel() == g * n * k &&
+          wC.numel() == g * n * k && conv_x.numel() == nb * di * k && conv_B.numel() == nb * g * n * k && conv_C.numel() == nb * g * n * k &&
+          ssm_state.size(0) == nb && dt_bias.numel() == nh && A.numel() == nh && D.numel() == nh && norm_w.numel() == di && out_proj.dim() == 2 &&
+          out_proj.size(0) == dm && out_proj.size(1) == di &&
+          ssm_mamba2_decode_supported((int)nb, (int)dm, (int)nh, (int)hp, (int)n, (int)g, (int)k, dtype_code(tok, "mamba2_step"));
+  if (fused) {
+    c10::cuda::CUDAGuard guard(tok.device());
+    Tensor out = at::empty_like(tok);
+    Tensor scratch = at::empty({ssm_mamba2_decode_scratch_bytes((int)nb, (int)nh, (int)g)}, tok.options().dtype(at::kByte));
+    ssm_mamba2_decode_args a{};
+    a.batch = (int)nb, a.d_model = (int)dm, a.heads = (int)nh, a.headdim = (int)hp, a.nstate = (int)n, a.groups = (int)g, a.width = (int)k;
+    a.io_dtype = dtype_code(tok, "mamba2_step"), a.a_log = a_log, a.eps = (float)eps;
+    a.hidden = tok.data_ptr(), a.in_z = in_z.data_ptr(), a.in_x = in_x.data_ptr(), a.in_B = in_B.data_ptr(), a.in_C = in_C.data_ptr(), a.in_dt = in_dt.data_ptr();
+    a.conv_x_w = wx.data_ptr(), a.conv_x_b = ptr(bx), a.conv_B_w = wB.data_ptr(), a.conv_B_b = ptr(bB), a.conv_C_w = wC.data_ptr(), a.conv_C_b = ptr(bC);
+    a.dt_bias = dt_bias.data_ptr<float>(), a.A = A.data_ptr<float>(), a.D = D.data_ptr<float>(), a.norm_w = norm_w.data_ptr(), a.out_proj = out_proj.data_ptr();
+    a.conv_state_x = conv_x.data_ptr<float>(), a.conv_state_B = conv_B.data_ptr<float>(), a.conv_state_C = conv_C.data_ptr<float>();
+    a.ssm_state = ssm_state.data_ptr<float>(), a.out = out.data_ptr(), a.scratch = scratch.data_ptr();
+    run(ssm_mamba2_decode(&a, stream_of(tok)));
+    return out;
+  }
+  Tensor z = at::matmul(tok, in_z.t());
+  Tensor x = dw_causal_conv_update(conv_x, at::matmul(tok, in_x.t()), wx, bx, "silu");
+  Tensor Bm = dw_causal_conv_update(conv_B, at::matmul(tok, in_B.t()), wB, bB, "silu").view({nb, g, n});
+  Tensor Cm = dw_causal_conv_update(conv_C, at::matmul(tok, in_C.t()), wC, bC, "silu").view({nb, g, n});
+  Tensor dt = at::matmul(tok, in_dt.t());
+  Tensor y = state_step_heads(ssm_state, x.view({nb, nh, hp}), dt, A, Bm, Cm, D, z.view({nb, nh, hp}), dt_bias, true, a_log);
+  variable_list rr = invoke_call(c10::make_intrusive<NormCall>(y.view({1, nb, di}), norm_w, OptTensor(), OptTensor(), true, eps, true, false, true));
+  return at::matmul(rr[0].view({nb, di}), out_proj.t());
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -523,6 +633,8 @@ void bind_operators(py::module& m) {
   ops.def("dw_causal_conv", &dw_causal_conv);
   ops.def("dw_causal_conv_update", &dw_causal_conv_update);
   ops.def("fused_layer_norm", &fused_layer_norm);
+  ops.def("mamba1_step", &mamba1_step);
+  ops.def("mamba2_step", &mamba2_step);
   ops.def("ssd_forward", &ssd_forward);
   ops.def("ssd_status", &ssd_status);
   ops.def("ssd_poll", &ssd_poll);

@@ -265,7 +265,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> fused_layer_norm_backward(const Tenso
   ssm_norm_bwd_args g{};
   c.fill(g.fwd);
   g.dy = go.data_ptr(), g.dx = dx.data_ptr(), g.dresidual = c.res.has_value() ? dres.data_ptr() : nullptr;
-  g.dweight = dw.data_ptr<float>(), g.dbias = c.b.has_value() ? db.data_ptr<float>() : nullptr, g.partial = partial.data_ptr<float>();
+  g.dweight = dw.data_ptr(), g.dbias = c.b.has_value() ? db.data_ptr() : nullptr, g.partial = partial.data_ptr<float>();
   g.dresidual_out = nullptr;
   run(ssm_fused_add_norm_bwd(&g, stream_of(c.x)));
   // absent inputs give empty tensors, as upstream's extension does

@@ -64,15 +64,23 @@ def mamba1_block_forward(ops: Any, w: dict, cfg: dict, hidden: Tensor, residual:
                                 residual_in_fp32=True, return_residual=True)
 
 
+def _native_step(ops: Any, tok: Tensor, name: str) -> bool:
+    """A whole-mixer step of the operator namespace can serve this call: it has one, and nothing is to be differentiated."""
+    return hasattr(ops, name) and tok.is_cuda and tok.dtype != torch.float64 and not torch.is_grad_enabled()
+
+
 def mamba1_mixer_step(ops: Any, w: dict, cfg: dict, tok: Tensor, conv_state: Tensor, ssm_state: Tensor) -> Tensor:
     """One decode token through the Mamba-1 mixer: tok (B, d_model) -> (B, d_model); ``conv_state (B, d_inner, K)`` and
     ``ssm_state (B, d_inner, N)`` (both fp32) are updated in place (reference step: modules/mamba1.py:324-385)."""
+    if _native_step(ops, tok, "mamba1_step"):
+        return ops.mamba1_step(tok, None, conv_state, ssm_state, w)
     n, r = cfg["d_state"], cfg["dt_rank"]
     x, z = tok @ w["in_x"].t(), tok @ w["in_z"].t()
     u = ops.dw_causal_conv_update(conv_state, x, w["conv_w"], w["conv_b"], "silu")
     xd = u @ w["x_proj"].t()
     delta = xd[:, :r] @ w["dt_proj"].t()
-    y = ops.selective_state_step(ssm_state, u, delta, w["A"], xd[:, r:r + n].unsqueeze(1), xd[:, r + n:].unsqueeze(1),
+    A = w["A"] if "A" in w else -torch.exp(w["A_log"])
+    y = ops.selective_state_step(ssm_state, u, delta, A, xd[:, r:r + n].unsqueeze(1), xd[:, r + n:].unsqueeze(1),
                                  D=w["D"], z=z, dt_bias=w["dt_bias"], softplus=True)
     return y @ w["out_proj"].t()
 
@@ -139,7 +147,7 @@ class Mamba1Block(nn.Module):
 
     def mixer_step(self, tok: Tensor, cache) -> Tensor:
         """The mixer alone on one token: tok (B, d_model) -> (B, d_model); ``cache`` from `allocate_inference_cache`."""
-        return mamba1_mixer_step(self._namespace(), self._weights(), dict(d_state=self.d_state, dt_rank=self.dt_rank), tok, cache[0], cache[1])
+        return mamba1_mixer_step(self._namespace(), self._parameters, dict(d_state=self.d_state, dt_rank=self.dt_rank), tok, cache[0], cache[1])
 
     def allocate_inference_cache(self, batch_size: int, dtype: Optional[torch.dtype] = None):
         """(conv_state (B, d_inner, K), ssm_state (B, d_inner, N)), both fp32 and zero-filled."""
@@ -153,8 +161,12 @@ class Mamba1Block(nn.Module):
         if hidden.ndim != 3 or hidden.shape[1] != 1:
             raise ValueError("step expects inputs of shape (B, 1, d_model)")
         ops = self._namespace()
+        if _native_step(ops, hidden, "mamba1_step"):
+            p = self._parameters
+            out, res = ops.mamba1_step(hidden[:, 0], residual, conv_state, ssm_state, p, p["norm_w"], self.eps)
+            return out.unsqueeze(1), res.unsqueeze(1)
         cfg = dict(d_state=self.d_state, dt_rank=self.dt_rank)
-        out = mamba1_mixer_step(ops, self._weights(), cfg, hidden[:, 0], conv_state, ssm_state).unsqueeze(1)
+        out = mamba1_mixer_step(ops, self._parameters, cfg, hidden[:, 0], conv_state, ssm_state).unsqueeze(1)
         res1 = None if residual is None else residual
         return ops.fused_layer_norm(out, self.norm_w, None, residual=res1, is_rms=True, eps=self.eps, prenorm=True,
                                     residual_in_fp32=True, return_residual=True)
@@ -225,9 +237,11 @@ def mamba2_mixer_forward(ops: Any, w: dict, cfg: dict, u: Tensor, group=None, sh
 def mamba2_mixer_step(ops: Any, w: dict, cfg: dict, tok: Tensor, conv_states: tuple, ssm_state: Tensor) -> Tensor:
     """One decode token through the Mamba-2 mixer: tok (B, d_model), normed -> (B, d_model).  ``conv_states``: the rolling
     windows of the x, B and C convolutions ((B, C_i, K) fp32 each); ``ssm_state (B, H, P, N)`` fp32; all updated in place."""
+    eps = cfg.get("eps", 1e-5)
+    if _native_step(ops, tok, "mamba2_step"):
+        return ops.mamba2_step(tok, conv_states, ssm_state, w, eps)
     nb = tok.shape[0]
     nh, hp, n, g = cfg["heads"], cfg["headdim"], cfg["d_state"], cfg["groups"]
-    eps = cfg.get("eps", 1e-5)
     z = tok @ w["in_z"].t()
     x = ops.dw_causal_conv_update(conv_states[0], tok @ w["in_x"].t(), w["conv_x"], w["conv_x_b"], "silu")
     Bm = ops.dw_causal_conv_update(conv_states[1], tok @ w["in_B"].t(), w["conv_B"], w["conv_B_b"], "silu").view(nb, g, n)
@@ -314,4 +328,4 @@ class Mamba2Block(nn.Module):
 
     def mixer_step(self, tok: Tensor, cache) -> Tensor:
         """The mixer alone on one normed token: tok (B, d_model) -> (B, d_model); ``cache`` from `allocate_inference_cache`."""
-        return mamba2_mixer_step(self._namespace(), {k: v for k, v in self.named_parameters()}, self._cfg(), tok, cache[0], cache[1])
+        return mamba2_mixer_step(self._namespace(), self._parameters, self._cfg(), tok, cache[0], cache[1])

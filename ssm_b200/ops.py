@@ -340,7 +340,7 @@ def selective_state_step(
         with torch.no_grad():
             state.copy_(new)
         return y
-    return _native().state_step(state, x, dt, A, B, C, D, z, dt_bias, softplus)
+    return _native().state_step(state, x, dt, A, B, C, D, z, dt_bias, softplus, False)
 
 
 def selective_state_step_heads(
@@ -350,7 +350,24 @@ def selective_state_step_heads(
     """Extension: Mamba-2 decode step.  ``state (B, H, P, N)`` fp32 in place, ``x, z (B, H, P)``,
     ``dt (B, H)``, ``A, D, dt_bias (H,)``, ``B, C (B, G, N)``; returns ``(B, H, P)``.  Equivalent to
     the upstream step on ``H*P`` flattened channels with per-head parameters broadcast."""
-    return _native().state_step_heads(state, x, dt, A, B, C, D, z, dt_bias, softplus)
+    return _native().state_step_heads(state, x, dt, A, B, C, D, z, dt_bias, softplus, False)
+
+
+def mamba1_step(tok: Tensor, residual: Optional[Tensor], conv_state: Tensor, ssm_state: Tensor, w: dict, norm_w: Optional[Tensor] = None,
+                eps: float = 1e-5):
+    """Extension: one decode token through a Mamba-1 mixer, and with ``norm_w`` the residual add and RMSNorm behind it
+    (then the result is ``(normed, residual)``).  ``tok (B, d_model)``; ``w`` as in `ssm_b200.mixer`, with ``A_log`` or ``A``;
+    states fp32, in place; no gradients.  Up to 16 sequences run as one launch."""
+    a_log = "A_log" in w
+    return _native().mamba1_step(tok, residual, conv_state, ssm_state, w["in_x"], w["in_z"], w["conv_w"], w["conv_b"], w["x_proj"], w["dt_proj"],
+                                 w["dt_bias"], w["A_log"] if a_log else w["A"], a_log, w["D"], w["out_proj"], norm_w, eps)
+
+
+def mamba2_step(tok: Tensor, conv_states: tuple, ssm_state: Tensor, w: dict, eps: float = 1e-5) -> Tensor:
+    """Extension: one decode token through a Mamba-2 mixer; the counterpart of :func:`mamba1_step`."""
+    return _native().mamba2_step(tok, *conv_states, ssm_state, w["in_z"], w["in_x"], w["in_B"], w["in_C"], w["in_dt"], w["conv_x"], w["conv_x_b"],
+                                 w["conv_B"], w["conv_B_b"], w["conv_C"], w["conv_C_b"], w["dt_bias"], w["A_log"], True, w["D"], w["norm_w"],
+                                 w["out_proj"], eps)
 
 
 # =========================================================================================
@@ -850,6 +867,8 @@ __all__ = [
     "selective_scan",
     "selective_state_step",
     "selective_state_step_heads",
+    "mamba1_step",
+    "mamba2_step",
     "ssd_chunk_scan",
     "dw_causal_conv",
     "dw_causal_conv_update",

@@ -211,6 +211,98 @@ __global__ void __launch_bounds__(kStepThreads) step_fwd_fast_kernel(const ssm_s
   }
 }
 
+// The same step for states that fill the GPU several times over: persistent warps, each with three 2 KB pieces of the state in
+// flight (cp.async; a piece is 512 floats = 512 / N rows).  The copies and the write-back run over a piece in memory order, whole
+// 128-byte lines per instruction whatever N is; the rows are picked out of shared memory.  The row-per-thread kernel above is
+// bound by what its short-lived threads keep in flight (64 bytes each, only until they use it) and, at N = 16, reads half
+// sectors.  (batch, heads x headdim, N) = (256, 80 x 64, 128), 1342 MB: 274 us with that kernel.
+constexpr int kStreamThreads = 256, kStreamStages = 3, kStreamCtasPerSm = 3;
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+template <typename T, typename BT, int N, bool HEADS>
+__global__ void __launch_bounds__(kStreamThreads, kStreamCtasPerSm) step_stream_kernel(const ssm_step_args a) {
+  constexpr int kPiece = 512, RPW = kPiece / N, LPR = N / 16;
+  __shared__ __align__(16) float buf[kStreamStages][kStreamThreads / 32][kPiece];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rows = a.batch * a.dim;
+  const int pieces = (rows + RPW - 1) / RPW, stride = gridDim.x * (kStreamThreads / 32);
+  const int64_t total = (int64_t)rows * N;
+  const int r = lane / LPR, sg = lane % LPR, rot = N == 16 ? r >> 1 : r;
+  auto issue = [&](int piece, int st) {
+    if (piece < pieces) {
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&buf[st][warp][lane * 4]);
+      const int64_t at = (int64_t)piece * kPiece + lane * 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (at + i * 128 < total) cp_async16(dst + i * 512, a.state + at + i * 128);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  int piece = blockIdx.x * (kStreamThreads / 32) + warp;
+  issue(piece, 0);
+  issue(piece + stride, 1);
+  int st = 0;
+  for (; piece < pieces; piece += stride) {
+    __syncwarp();  // every lane has read the piece before last, whose buffer is refilled now
+    issue(piece + 2 * stride, st >= 1 ? st - 1 : 2);
+    const int row_raw = piece * RPW + r;
+    const bool live = row_raw < rows;
+    const int row = live ? row_raw : rows - 1;
+    const int b = row / a.dim, d = row % a.dim;
+    const int head = HEADS ? d / (a.dim / a.param_heads) : d;
+    const float x = to_f<T>(reinterpret_cast<const T*>(a.x)[row]);
+    float dt = to_f<T>(reinterpret_cast<const T*>(a.dt)[HEADS ? (int64_t)b * a.param_heads + head : row]);
+    const float bias = a.dt_bias ? __ldg(a.dt_bias + head) : 0.f, Dv = a.D ? __ldg(a.D + head) : 0.f;
+    const float zv = a.z ? to_f<T>(reinterpret_cast<const T*>(a.z)[row]) : 0.f;
+    const float Ah = HEADS ? step_A(a, __ldg(a.A + head)) : 0.f;
+    const int g = d / (a.dim / a.bc_groups);
+    const int64_t boff = (int64_t)b * a.b_sb + (int64_t)g * a.b_sg, coff = (int64_t)b * a.c_sb + (int64_t)g * a.c_sg;
+    float Bv[4][4], Cv[4][4];
+    float4 Av[4];
+    int at[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      at[v] = (sg + LPR * ((v + rot) & 3)) * 4;  // rotated so that eight neighbouring lanes read 128 different bytes
+      load_bc4<BT>(a.Bm, boff + at[v], Bv[v]);
+      load_bc4<BT>(a.Cm, coff + at[v], Cv[v]);
+      if (!HEADS) Av[v] = __ldg(reinterpret_cast<const float4*>(a.A + (int64_t)d * N + at[v]));
+    }
+    dt += bias;
+    if (a.dt_softplus) dt = softplus_fast(dt);
+    const float dtx = dt * x, dah = HEADS ? ex2_approx(dt * Ah * kLog2e) : 0.f;
+    asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+    __syncwarp();
+    float* mine = &buf[st][warp][r * N];
+    float y = 0.f;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const float4 s4 = *reinterpret_cast<const float4*>(mine + at[v]);
+      float sv[4] = {s4.x, s4.y, s4.z, s4.w};
+      const float An[4] = {Av[v].x, Av[v].y, Av[v].z, Av[v].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float da = HEADS ? dah : ex2_approx(dt * (step_A(a, An[i]) * kLog2e));
+        sv[i] = fmaf(da, sv[i], dtx * Bv[v][i]);
+        y = fmaf(Cv[v][i], sv[i], y);
+      }
+      *reinterpret_cast<float4*>(mine + at[v]) = make_float4(sv[0], sv[1], sv[2], sv[3]);
+    }
+    __syncwarp();
+    const int64_t out_at = (int64_t)piece * kPiece + lane * 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (out_at + i * 128 < total) __stcs(reinterpret_cast<float4*>(a.state + out_at + i * 128), *reinterpret_cast<const float4*>(&buf[st][warp][lane * 4 + i * 128]));
+    y = group_sum<LPR, 1>(y);
+    if (sg == 0 && live) {
+      y = fmaf(Dv, x, y);
+      if (a.z) y *= silu_fast(zv);
+      reinterpret_cast<T*>(a.out)[row] = from_f<T>(y);
+    }
+    st = st == 2 ? 0 : st + 1;
+  }
+}
+
 // Backward of the plain step.  One group of LPR lanes per row, parameter gradients by atomics.
 template <typename T, int LPR>
 __global__ void __launch_bounds__(kStepThreads) step_bwd_kernel(const ssm_step_bwd_args g) {
@@ -317,8 +409,29 @@ static int step_fwd_fast_launch(const ssm_step_args& a, cudaStream_t st) {
   step_fwd_fast_kernel<T, BT, NV, LPR><<<(unsigned)((threads + kStepThreads - 1) / kStepThreads), kStepThreads, 0, st>>>(a);
   return launch_status("step_fwd_fast_kernel");
 }
+// Two pieces or more per warp of a full GPU, else the pipeline never gets going and one thread per row is the shorter path.
+template <typename T, typename BT, int N>
+static int step_stream_launch(const ssm_step_args& a, int sms, cudaStream_t st) {
+  const int grid = sms * kStreamCtasPerSm;
+  if (a.param_heads > 0) step_stream_kernel<T, BT, N, true><<<grid, kStreamThreads, 0, st>>>(a);
+  else step_stream_kernel<T, BT, N, false><<<grid, kStreamThreads, 0, st>>>(a);
+  return launch_status("step_stream_kernel");
+}
 template <typename T, typename BT>
 static int step_fwd_fast_n(const ssm_step_args& a, cudaStream_t st) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t rows = (int64_t)a.batch * a.dim;
+  if (rows * a.nstate / 512 >= (int64_t)2 * sms * kStreamCtasPerSm * (kStreamThreads / 32) && rows < (1ll << 30)) {
+    switch (a.nstate) {
+      case 16: return step_stream_launch<T, BT, 16>(a, sms, st);
+      case 32: return step_stream_launch<T, BT, 32>(a, sms, st);
+      case 64: return step_stream_launch<T, BT, 64>(a, sms, st);
+      case 128: return step_stream_launch<T, BT, 128>(a, sms, st);
+      default: return step_stream_launch<T, BT, 256>(a, sms, st);
+    }
+  }
   switch (a.nstate) {
     case 16: return step_fwd_fast_launch<T, BT, 4, 1>(a, st);
     case 32: return step_fwd_fast_launch<T, BT, 4, 2>(a, st);

@@ -61,3 +61,38 @@ def test_mamba2_step_matches_oracle(nb, dm, groups, dtype):
             close(out_g, out_c, **TOL, what="mixer output")
     for g, c in zip((*wg, sg), (*wc, sc)):
         close(g, c, **TOL, what="cache")
+
+
+# states of more than two pieces per resident warp (the streaming kernel), rows that do not fill the last piece, every state width
+@pytest.mark.parametrize("n,dtype", [(16, torch.bfloat16), (32, torch.float32), (64, torch.float16), (128, torch.bfloat16), (256, torch.float32)])
+def test_large_state_step_matches_oracle(n, dtype):
+    from ssm_b200 import ops
+
+    nb, nd = 3, 3_700_000 // n // 3 | 1
+    gen = torch.Generator().manual_seed(n)
+    rnd = lambda *s: torch.randn(*s, generator=gen)  # noqa: E731
+    state, x, dt, z = rnd(nb, nd, n), rnd(nb, nd).to(dtype), rnd(nb, nd).to(dtype), rnd(nb, nd).to(dtype)
+    A, B, C, D, bias = -torch.exp(rnd(nd, n) * 0.5), rnd(nb, 1, n).to(dtype), rnd(nb, 1, n).to(dtype), rnd(nd), rnd(nd)
+    sg = state.cuda()
+    c = lambda t: t.cuda()  # noqa: E731
+    y = ops.selective_state_step(sg, c(x), c(dt), c(A), c(B), c(C), D=c(D), z=c(z), dt_bias=c(bias), softplus=True)
+    yo = orc.selective_state_step(state, x, dt, A, B, C, D=D, z=z, dt_bias=bias, softplus=True)
+    tol = dict(rtol=1e-4, atol=1e-4) if dtype == torch.float32 else dict(rtol=2e-2, atol=1e-2)
+    close(y, yo, **tol, what="y"), close(sg, state, rtol=1e-4, atol=1e-4, what="state")
+
+
+def test_large_state_step_with_parameters_per_head_matches_oracle():
+    from ssm_b200 import ops
+
+    nb, nh, p, n = 5, 100, 60, 128
+    gen = torch.Generator().manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=gen)  # noqa: E731
+    state, x, dt, z = rnd(nb, nh, p, n), rnd(nb, nh, p).bfloat16(), rnd(nb, nh).bfloat16(), rnd(nb, nh, p).bfloat16()
+    A, B, C, D, bias = -torch.exp(rnd(nh) * 0.5), rnd(nb, 2, n).bfloat16(), rnd(nb, 2, n).bfloat16(), rnd(nh), rnd(nh)
+    sg = state.cuda()
+    y = ops.selective_state_step_heads(sg, x.cuda(), dt.cuda(), A.cuda(), B.cuda(), C.cuda(), D=D.cuda(), z=z.cuda(), dt_bias=bias.cuda(), softplus=True)
+    rep = lambda t: t[:, None].expand(nh, p).reshape(-1)  # noqa: E731
+    flat = state.view(nb, nh * p, n)
+    yo = orc.selective_state_step(flat, x.reshape(nb, -1), dt.repeat_interleave(p, 1), A[:, None, None].expand(nh, p, n).reshape(nh * p, n), B, C, D=rep(D),
+                                  z=z.reshape(nb, -1), dt_bias=rep(bias), softplus=True)
+    close(y.reshape(nb, -1), yo, rtol=2e-2, atol=1e-2, what="y"), close(sg.view_as(flat), flat, rtol=1e-4, atol=1e-4, what="state")

@@ -439,6 +439,12 @@ typedef struct {
   int32_t bc_width;       /* 0 (= nstate) or 64 */
   int32_t x_heads;        /* 0 (= heads) or a divisor of heads */
   float* ws_state_in_f32; /* nullable */
+  /* Packed sequences: num_seqs > 0 sequences lie end to end along len of a batch of one, each scanned from a zero state with
+   * chunks counted from its first step.  seq_table (device): num_chunks pairs {first step, end of the sequence}, sequence by
+   * sequence, then num_seqs + 1 chunk offsets.  final_states, and the state and shard-summary part of the scratch, are per
+   * sequence; scratch: ssm_ssd_packed_scratch_bytes().  phase 0 (states and Y) or 1 (states only), no initial_states. */
+  const int32_t* seq_table; /* nullable */
+  int32_t num_seqs, num_chunks;
 } ssm_ssd_args;
 
 int ssm_ssd_supported(int32_t headdim, int32_t nstate, int32_t chunk_size, int32_t io_dtype);
@@ -449,6 +455,9 @@ int ssm_ssd_supported(int32_t headdim, int32_t nstate, int32_t chunk_size, int32
 int ssm_ssd_wait_selftest(int32_t* status, int32_t probes, ssm_stream_t stream);
 int64_t ssm_ssd_scratch_bytes(int32_t batch, int32_t len, int32_t heads);
 int64_t ssm_ssd_state_scratch_bytes(int32_t batch, int32_t len, int32_t heads);
+/* scratch of a packed call: ws_dt, ws_cum (num_chunks * 256 * heads floats each), ws_state, ws_state_in as above; the offset of
+ * ws_state_in from ws_state is written to *state_bytes */
+int64_t ssm_ssd_packed_scratch_bytes(int32_t num_seqs, int32_t num_chunks, int32_t heads, int64_t* state_bytes);
 int ssm_ssd_fwd(const ssm_ssd_args* args, ssm_stream_t stream);
 
 /* Sequence shards (no reference counterpart: the reference is single-device).  After phase 1 every rank all-gathers its

@@ -130,7 +130,7 @@ class SsdArgs(C.Structure):
         ("initial_states", fp), ("Y", vp), ("final_states", fp),
         ("ws_dt", fp), ("ws_cum", fp), ("ws_state", fp), ("ws_state_in", vp), ("status", vp),
         ("row_dots", fp), ("row_scale", fp), ("bc_width", i32), ("x_heads", i32),
-        ("ws_state_in_f32", fp),
+        ("ws_state_in_f32", fp), ("seq_table", vp), ("num_seqs", i32), ("num_chunks", i32),
     ]
 
 
@@ -175,6 +175,7 @@ ENTRY_POINTS = {
     "ssm_ssd_wait_selftest": (C.c_int, [vp, i32, vp]),
     "ssm_ssd_scratch_bytes": (C.c_int64, [i32, i32, i32]),
     "ssm_ssd_state_scratch_bytes": (C.c_int64, [i32, i32, i32]),
+    "ssm_ssd_packed_scratch_bytes": (C.c_int64, [i32, i32, i32, C.POINTER(i64)]),
     "ssm_ssd_bwd_gate": (C.c_int, [C.POINTER(SsdBwdArgs), vp]),
     "ssm_ssd_bwd_finish": (C.c_int, [C.POINTER(SsdBwdArgs), vp]),
     "ssm_time_flip": (C.c_int, [vp, vp, i32, i32, i32, C.c_int64, vp]),

@@ -47,6 +47,10 @@ __host__ __device__ inline int64_t ssd_summary_floats_padded(int batch, int head
 constexpr int kCumHeads = 32;
 constexpr int kCumLd = kQ + 8;  // row pitch of the transposed tile (floats): rows stay 16-byte aligned, lanes 32 bytes apart
 
+// first step of a chunk, and the first step beyond its sequence: of packed sequences they come from the table
+__device__ __forceinline__ int chunk_begin(const ssm_ssd_args& a, int c) { return a.seq_table ? __ldg(a.seq_table + 2 * c) : c * kQ; }
+__device__ __forceinline__ int chunk_limit(const ssm_ssd_args& a, int c) { return a.seq_table ? __ldg(a.seq_table + 2 * c + 1) : a.len; }
+
 template <typename T>
 __global__ void __launch_bounds__(kQ) ssd_cumsum_kernel(const ssm_ssd_args a, int nchunks) {
   __shared__ __align__(16) float sD[kCumHeads * kCumLd];
@@ -54,8 +58,8 @@ __global__ void __launch_bounds__(kQ) ssd_cumsum_kernel(const ssm_ssd_args a, in
   const int h0 = blockIdx.x * kCumHeads, c = blockIdx.y, b = blockIdx.z;
   const int nh = min(kCumHeads, a.heads - h0);
   {
-    const int t = c * kQ + tid;
-    if (t < a.len) {
+    const int t = chunk_begin(a, c) + tid;
+    if (t < chunk_limit(a, c)) {
       const int64_t at = ((int64_t)b * a.len + t) * a.heads + h0;
       if (a.dt_mode & 1) {  // fp32 step sizes, already activated
         const float* p = reinterpret_cast<const float*>(a.dt) + at;
@@ -188,8 +192,17 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
   __shared__ uint32_t tmem_slot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wg = tid >> 7;
-  const int h0 = blockIdx.x * HPC, b = blockIdx.y;
+  const int h0 = blockIdx.x * HPC;
   const int g = h0 / (a.heads / a.groups);
+  // b: batch element of the operands; sb: whose state this is (the packed sequence, or b); the walk covers chunks c_off ..
+  // c_off + nwalk, whose first step is t_off
+  const bool packed = a.seq_table != nullptr;
+  const int sb = blockIdx.y, b = packed ? 0 : sb;
+  const int* seq_first = packed ? a.seq_table + 2 * a.num_chunks + sb : nullptr;
+  const int c_off = packed ? __ldg(seq_first) : 0;
+  const int nwalk = packed ? __ldg(seq_first + 1) - c_off : nchunks;
+  const int t_off = packed && nwalk > 0 ? __ldg(a.seq_table + 2 * c_off) : 0;
+  const int n_states = packed ? a.num_seqs : a.batch;  // batch extent of the states
   const int n = (warp & 3) * 32 + lane;  // this thread's state index = TMEM lane
   constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
   constexpr uint32_t kCols = HPC <= 1 ? 128 : (HPC == 2 ? 256 : 512);  // 2 accumulators of 64 columns per head, a power of two
@@ -209,8 +222,8 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const int role = __shfl_sync(0xffffffffu, warp, 0);  // the same in every lane, and visibly so
 
-  const int64_t vrow0 = ((int64_t)b * a.heads + h0) * nchunks * kQ;  // exponent vectors of head h0 (next head: + nchunks * kQ)
-  const int nst = SPC * nchunks;
+  const int64_t vrow0 = (((int64_t)b * a.heads + h0) * nchunks + c_off) * kQ;  // exponent vectors of head h0 (next head: + nchunks * kQ)
+  const int nst = SPC * nwalk;
   // stage s = steps [s * 64, s * 64 + 64), issued by one thread: two boxes of B, one box of x per head, and with a
   // chunk's first stage the exponent vectors of its heads.  Steps beyond the sequence read as zero.
   auto copy_stage = [&](int s) {
@@ -218,11 +231,11 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
     const uint32_t full = tc::smem_u32(&mbar_full[s % NS]);
     const bool first = s % SPC == 0;
     tc::mbar_expect_tx(full, M::STAGE + (first ? HPC * kQ * 4 + M::LAST_BYTES : 0));
-    tc::tma_load_4d(base, &maps.b, full, 0, g, s * kStep, b);
-    tc::tma_load_4d(base + M::BLK_BYTES, &maps.b, full, 64, g, s * kStep, b);
+    tc::tma_load_4d(base, &maps.b, full, 0, g, t_off + s * kStep, b);
+    tc::tma_load_4d(base + M::BLK_BYTES, &maps.b, full, 64, g, t_off + s * kStep, b);
 #pragma unroll
     for (int hh = 0; hh < HPC; ++hh)
-      tc::tma_load_4d(base + M::A_BYTES + hh * M::BLK_BYTES, &maps.x, full, 0, a.x_heads ? (h0 + hh) % a.x_heads : h0 + hh, s * kStep, b);
+      tc::tma_load_4d(base + M::A_BYTES + hh * M::BLK_BYTES, &maps.x, full, 0, a.x_heads ? (h0 + hh) % a.x_heads : h0 + hh, t_off + s * kStep, b);
     if (first) {
       const int c = s / SPC;
 #pragma unroll
@@ -277,7 +290,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
   float st[HPC][32];
 #pragma unroll
   for (int hh = 0; hh < HPC; ++hh) {
-    const float* init = a.initial_states ? a.initial_states + (((int64_t)b * a.heads + h0 + hh) * kP + wg * 32) * kN + n : nullptr;
+    const float* init = a.initial_states ? a.initial_states + (((int64_t)sb * a.heads + h0 + hh) * kP + wg * 32) * kN + n : nullptr;
 #pragma unroll
     for (int i = 0; i < 32; ++i) st[hh][i] = init ? __ldg(init + (int64_t)i * kN) : 0.f;
   }
@@ -286,7 +299,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
   auto emit_state_in = [&](int c) {
 #pragma unroll
     for (int hh = 0; hh < HPC; ++hh) {
-      T* blk = sin + (((int64_t)b * nchunks + c) * a.heads + h0 + hh) * (int64_t)(kP * kN);
+      T* blk = sin + (((int64_t)b * nchunks + c_off + c) * a.heads + h0 + hh) * (int64_t)(kP * kN);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         Vec16<T> o;
@@ -294,7 +307,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
         *reinterpret_cast<uint4*>(blk + ((size_t)(wg * 4 + q) * kN + n) * 8) = o.raw;
       }
       if (a.ws_state_in_f32) {  // the same tile unrounded (the backward pass forms <adjoint state, state> from it)
-        float* blk32 = a.ws_state_in_f32 + (((int64_t)b * nchunks + c) * a.heads + h0 + hh) * (int64_t)(kP * kN);
+        float* blk32 = a.ws_state_in_f32 + (((int64_t)b * nchunks + c_off + c) * a.heads + h0 + hh) * (int64_t)(kP * kN);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           float4* dst = reinterpret_cast<float4*>(blk32 + ((size_t)(wg * 4 + q) * kN + n) * 8);
@@ -343,7 +356,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
         clast[hh] = sLast[((c % M::NVEC) * HPC + hh) * 4 + 3];
         // exponent (base 2) of the decay from the start of the sequence to the start of this chunk: what a state
         // that arrives later (phase 2 of a sequence shard) is multiplied by before it joins this chunk's state
-        if (tid == 0) a.ws_state[ssd_summary_floats_padded(a.batch, a.heads) + ((int64_t)b * a.heads + h0 + hh) * nchunks + c] = ctot[hh];
+        if (tid == 0 && !packed) a.ws_state[ssd_summary_floats_padded(a.batch, a.heads) + ((int64_t)b * a.heads + h0 + hh) * nchunks + c] = ctot[hh];
         ctot[hh] += clast[hh];
       }
     }
@@ -357,7 +370,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
 #pragma unroll
       for (int k = 0; k < M::BLK_BYTES / 16 / 256; ++k) {
         const int u = tid + 256 * k;  // 16-byte unit of this head's tile; 8 units per step
-        const float w = ex2_approx(c_last - vcp[u >> 3]);
+        const float w = ex2_approx(c_last - vcp[u >> 3]);  // 0 for steps beyond the sequence
         unsigned char* px = base + M::A_BYTES + hh * M::BLK_BYTES + (size_t)u * 16;
         Vec16<T> v;
         v.raw = *reinterpret_cast<const uint4*>(px);
@@ -366,6 +379,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] *= w;
         v.pack(f);
+        if (packed && w == 0.f) v.raw = make_uint4(0, 0, 0, 0);  // what follows is another sequence
         *reinterpret_cast<uint4*>(px) = v.raw;
       }
     }
@@ -376,12 +390,12 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
     __syncwarp();
     if (lane == 0) tc::mbar_arrive(tc::smem_u32(&mbar_scaled[s % NS]));
   }
-  if (nchunks > 0 && !fail) fail = !fold_chunk(nchunks - 1, clast);
+  if (nwalk > 0 && !fail) fail = !fold_chunk(nwalk - 1, clast);
   // final states in fp32, (p, n) order: to the caller, and kept in scratch for a later phase 2
   if (!fail) {
 #pragma unroll
     for (int hh = 0; hh < HPC; ++hh) {
-      const int64_t off = (((int64_t)b * a.heads + h0 + hh) * kP + wg * 32) * kN + n;
+      const int64_t off = (((int64_t)sb * a.heads + h0 + hh) * kP + wg * 32) * kN + n;
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         if (a.final_states) a.final_states[off + (int64_t)i * kN] = st[hh][i];
@@ -389,7 +403,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
       }
       // the shard's total log-decay (natural log) follows the states in the scratch: together they are what a
       // sequence shard sends to the other ranks
-      if (tid == 0) a.ws_state[(int64_t)a.batch * a.heads * kP * kN + (int64_t)b * a.heads + h0 + hh] = ctot[hh] * kLn2;
+      if (tid == 0) a.ws_state[(int64_t)n_states * a.heads * kP * kN + (int64_t)sb * a.heads + h0 + hh] = ctot[hh] * kLn2;
     }
   }
   }  // compute warps
@@ -535,7 +549,12 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   const int h0 = part * hpc;
   const int nh = min(hpc, a.heads - h0);
   const int g = h0 / (a.heads / a.groups);
-  const int t0 = c * kQ;
+  const int t0 = chunk_begin(a, c);
+  // rows of this block that exist; a ragged block of a packed sequence stores its rows by hand (what follows them belongs to
+  // the next sequence), everything else leaves through TMA, which cuts at the end of the tensor
+  const int t_live = chunk_limit(a, c) - t0 - MB * kBlk;
+  const bool ragged = a.seq_table != nullptr && t_live < kBlk;
+  if (ragged && t_live <= 0) return;  // the whole CTA: nothing has been issued yet
   const int i_loc = (warp & 3) * 32 + lane;    // row within the block = TMEM lane
   const int i_chunk = MB * kBlk + i_loc;       // row within the chunk
   const int rc = MB * 4 + (warp & 3);          // this warp's rows as a 32-step chunk index
@@ -682,6 +701,11 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     tc::fence_async_smem();  // the staged rows leave through a bulk store
   };
   const int t_blk = t0 + MB * kBlk;  // first step of this block's rows
+  auto store_rows = [&](int h) {     // the staged rows of a ragged block, 16 bytes a thread
+    for (int u = tid; u < t_live * 8; u += kScanThreads)
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.Y) + (((int64_t)b * a.len + t_blk + (u >> 3)) * a.heads + h) * kP + (u & 7) * 8) =
+          *reinterpret_cast<const uint4*>(swz(sZ, u >> 3, u & 7));
+  };
 
   float ct_prev = 0.f;   // the previous head's row exponent and x row, carried into its (deferred) epilogue
   uint4 xr_prev[kXR];
@@ -751,7 +775,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
         tc::mbar_expect_tx(mb_z(buf), M::Z_BYTES);
         tc::tma_load_4d(tc::smem_u32(sZin(buf)), &maps.z, mb_z(buf), 0, h, t_blk, b);
       }
-      if (hi >= 2) {  // staged by the epilogue of the previous iteration; its reads are awaited after the mask, below
+      if (hi >= 2 && !ragged) {  // staged by the epilogue of the previous iteration; its reads are awaited after the mask, below
         tc::tma_store_4d(&maps.y, tc::smem_u32(sZ), 0, h - 2, t_blk, b);
         tc::bulk_commit();
       }
@@ -762,6 +786,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
       }
     }
 
+    if (ragged && hi >= 2) store_rows(h - 2);  // read before the mid-iteration barrier, overwritten after it
     // ---- decay mask: G (registers) x the factors formed above -> the A operand in tensor memory
     if (!reuse) {
 #pragma unroll
@@ -880,19 +905,21 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     tc::fence_after_sync();
     ok = __syncthreads_and(ok);
     if (ok) {
-      if (tid == kCopyThread) {
-        if (nh >= 2) {
-          tc::tma_store_4d(&maps.y, tc::smem_u32(sZ), 0, h0 + last - 1, t_blk, b);
-          tc::bulk_commit();
-          tc::bulk_wait_read();
-        }
+      if (ragged) {
+        if (nh >= 2) store_rows(h0 + last - 1);
+      } else if (tid == kCopyThread && nh >= 2) {
+        tc::tma_store_4d(&maps.y, tc::smem_u32(sZ), 0, h0 + last - 1, t_blk, b);
+        tc::bulk_commit();
+        tc::bulk_wait_read();
       }
       if (has_z) ok = tc::mbar_wait(mb_z(buf), (last >> 1) & 1);
       ok = __syncthreads_and(ok);  // also orders thread 0's wait on the store's reads before everyone's writes
       if (ok) {
         epilogue(h0 + last, buf, ct_prev, xr_prev);
         __syncthreads();
-        if (tid == kCopyThread) {
+        if (ragged) {
+          store_rows(h0 + last);
+        } else if (tid == kCopyThread) {
           tc::tma_store_4d(&maps.y, tc::smem_u32(sZ), 0, h0 + last, t_blk, b);
           tc::bulk_commit();
         }
@@ -964,7 +991,7 @@ static int ssd_state_launch(const ssm_ssd_args& a, int nchunks, cudaStream_t st)
   if (int rc = encode_rows_map(&maps.x, a.X, a, StateSmem<HPC>::kStep, kP, a.x_heads ? a.x_heads : a.heads)) return rc;
   const size_t smem = StateSmem<HPC>::ALLOC;
   cudaFuncSetAttribute(ssd_state_kernel<T, HPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  ssd_state_kernel<T, HPC><<<dim3(a.heads / HPC, a.batch), kStateThreads, smem, st>>>(a, maps, nchunks);
+  ssd_state_kernel<T, HPC><<<dim3(a.heads / HPC, a.num_seqs ? a.num_seqs : a.batch), kStateThreads, smem, st>>>(a, maps, nchunks);
   return launch_status("ssd_state_kernel");
 }
 
@@ -999,7 +1026,8 @@ __global__ void __launch_bounds__(32) ssd_wait_selftest_kernel(int32_t* status, 
 
 template <typename T>
 static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
-  const int nchunks = (a.len + kQ - 1) / kQ;
+  const int nchunks = a.num_seqs ? a.num_chunks : (a.len + kQ - 1) / kQ;
+  const int walks = a.num_seqs ? a.num_seqs : a.batch;  // sequences that the state kernel walks
   // heads per scan CTA (a divisor of the heads of one B / C group, so that a CTA's heads share their G): every CTA
   // pays a prologue (C / B tiles, G) of about two heads' worth of time, and the grid runs in whole waves of one CTA
   // per SM; take the divisor with the least (waves x (prologue + heads)).
@@ -1029,12 +1057,12 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
     // heads per CTA of the sequential state kernel: enough to bring the grid down to about one CTA per SM
     // (its CTAs all run for the whole sequence, so a second, partial wave would double the time), at most 4,
     // and a divisor of the heads of one B / C group
-    int shpc = (int)(((int64_t)a.batch * a.heads + sm_count - 1) / sm_count);
+    int shpc = (int)(((int64_t)walks * a.heads + sm_count - 1) / sm_count);
     shpc = shpc < 1 ? 1 : (shpc > 4 ? 4 : shpc);
     while (hpg % shpc != 0) --shpc;
     // between one and two (batch, head) pairs per SM: two heads per CTA would leave almost half of the SMs idle; one head per
     // CTA, two CTAs per SM (they fit) keeps every SM busy and halves what the longest SM has to walk
-    if ((int64_t)a.batch * a.heads > sm_count && (int64_t)a.batch * a.heads <= 2 * (int64_t)sm_count) shpc = 1;
+    if ((int64_t)walks * a.heads > sm_count && (int64_t)walks * a.heads <= 2 * (int64_t)sm_count) shpc = 1;
     int rc;
     switch (shpc) {
       case 1: rc = ssd_state_launch<T, 1>(a, nchunks, st); break;
@@ -1097,6 +1125,12 @@ extern "C" int64_t ssm_ssd_scratch_bytes(int32_t batch, int32_t len, int32_t hea
   return 2 * vec + fin + st;
 }
 
+extern "C" int64_t ssm_ssd_packed_scratch_bytes(int32_t num_seqs, int32_t num_chunks, int32_t heads, int64_t* state_bytes) {
+  const int64_t fin = (ssd_summary_floats_padded(num_seqs, heads) * 4 + 255) / 256 * 256;
+  if (state_bytes) *state_bytes = fin;
+  return 2 * (int64_t)heads * num_chunks * kQ * 4 + fin + (int64_t)num_chunks * heads * kP * kN * 2;
+}
+
 extern "C" int64_t ssm_ssd_shard_summary_floats(int32_t batch, int32_t heads) { return (int64_t)batch * heads * (kP * kN + 1); }
 
 extern "C" int ssm_ssd_fold_shards(const float* gathered, int32_t world, int32_t rank, int32_t batch, int32_t heads, const float* initial_states,
@@ -1133,7 +1167,13 @@ extern "C" int ssm_ssd_fwd(const ssm_ssd_args* a, ssm_stream_t stream) {
   SSM_REQUIRE(aligned_to(a->X, 16) && aligned_to(a->Bm, 16) && aligned_to(a->Cm, 16) && (!a->Y || aligned_to(a->Y, 16)) && aligned_to(a->ws_state_in, 16) &&
                   (!a->z || aligned_to(a->z, 16)),
               SSM_ERR_ALIGN, "ssd_scan: tensors must be 16-byte aligned");
-  const int64_t nchunks = (a->len + kQ - 1) / kQ;
+  if (a->num_seqs) {
+    SSM_REQUIRE(a->num_seqs > 0 && a->num_seqs <= 65535 && a->num_chunks > 0 && a->seq_table && a->batch == 1, SSM_ERR_SHAPE,
+                "ssd_scan: packed sequences need a batch of one and a table");
+    SSM_REQUIRE(a->phase != 2 && !a->initial_states && !a->row_dots && !a->row_scale, SSM_ERR_UNSUPPORTED, "ssd_scan: not built for packed sequences");
+  }
+  const int64_t nchunks = a->num_seqs ? a->num_chunks : (a->len + kQ - 1) / kQ;
+  SSM_REQUIRE((a->num_seqs == 0) == (a->seq_table == nullptr), SSM_ERR_NULL, "ssd_scan: num_seqs without a table");
   SSM_REQUIRE((int64_t)a->batch * nchunks <= 65535 && a->heads <= 65535 && (int64_t)a->batch * nchunks * a->heads * 2 < (1ll << 31), SSM_ERR_TOO_LARGE,
               "ssd_scan: grid too large");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);

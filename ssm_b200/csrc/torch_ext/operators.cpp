@@ -595,31 +595,83 @@ SsdShape ssd_check(const Tensor& X, const Tensor& dt, const Tensor& A, const Ten
   return s;
 }
 
-// (Y, final states fp32); the caller has checked ssm_ssd_supported().
-std::tuple<Tensor, Tensor> ssd_forward(const Tensor& X_, const Tensor& dt_, const Tensor& A_, const Tensor& B_, const Tensor& C_, const OptTensor& D_,
-                                       const OptTensor& z_, const OptTensor& bias_, bool softplus, const OptTensor& init_, int64_t chunk) {
-  ValueErrors scope;
+// Boundaries of packed sequences as host integers (one read of cu_seqlens), checked.
+std::vector<int64_t> seq_bounds(const Tensor& cu, int64_t len) {
+  Tensor host = cu.to(at::kCPU, at::kLong).contiguous();
+  std::vector<int64_t> v(host.data_ptr<int64_t>(), host.data_ptr<int64_t>() + host.numel());
+  bool ok = v.size() >= 2 && v.front() == 0 && v.back() == len;
+  for (size_t i = 1; i < v.size(); ++i) ok = ok && v[i] >= v[i - 1];
+  SSM_ARG(ok, "cu_seqlens must rise from 0 to L.");
+  return v;
+}
+
+// (Y, final states fp32); the caller has checked ssm_ssd_supported().  With `cu` the sequences packed along L of a batch of one are
+// scanned each from a zero state and the states are per sequence (S, H, P, N); want_y false: states only.
+std::tuple<Tensor, Tensor> ssd_run(const Tensor& X_, const Tensor& dt_, const Tensor& A_, const Tensor& B_, const Tensor& C_, const OptTensor& D_,
+                                   const OptTensor& z_, const OptTensor& bias_, bool softplus, const OptTensor& init_, int64_t chunk,
+                                   const std::vector<int64_t>* cu, bool want_y) {
   const SsdShape s = ssd_check(X_, dt_, A_, B_, C_, D_, z_, bias_, init_);
   c10::cuda::CUDAGuard guard(X_.device());
   ssd_poll(X_.get_device());
-  Tensor X = X_.detach().contiguous(), dt = like(dt_, X), B = like(B_, X), C = like(C_, X), A = f32c(A_);
+  Tensor X = X_.detach().contiguous(), dt = like(dt_, X), B = like(B_, X), C = like(C_, X), A = f32c(A_), table;
   OptTensor D = f32c(D_), bias = f32c(bias_), init = f32c(init_), z;
   if (z_.has_value()) z = like(*z_, X);
   const auto f32 = X.options().dtype(at::kFloat);
-  Tensor Y = at::empty_like(X), fin = at::empty({s.nb, s.nh, s.np, s.nn}, f32);
-  Tensor ws = at::empty({ssm_ssd_scratch_bytes((int)s.nb, (int)s.nl, (int)s.nh)}, X.options().dtype(at::kByte));
-  const int64_t vec = s.nb * s.nh * ((s.nl + chunk - 1) / chunk) * chunk * 4;
-  char* base = reinterpret_cast<char*>(ws.data_ptr());
+  int64_t walks = s.nb, nchunks = s.nb * ((s.nl + chunk - 1) / chunk), bytes, state_bytes;
   ssm_ssd_args a{};
+  if (cu) {
+    walks = (int64_t)cu->size() - 1;
+    std::vector<int32_t> t, first;
+    for (int64_t q = 0; q < walks; ++q) {
+      first.push_back((int32_t)(t.size() / 2));
+      for (int64_t c = (*cu)[q]; c < (*cu)[q + 1]; c += chunk) t.push_back((int32_t)c), t.push_back((int32_t)(*cu)[q + 1]);
+    }
+    nchunks = (int64_t)t.size() / 2;
+    first.push_back((int32_t)nchunks);
+    t.insert(t.end(), first.begin(), first.end());
+    table = at::empty({(int64_t)t.size()}, at::TensorOptions().dtype(at::kInt));
+    std::copy(t.begin(), t.end(), table.data_ptr<int32_t>());
+    table = table.to(X.device(), true);
+    a.seq_table = table.data_ptr<int32_t>(), a.num_seqs = (int)walks, a.num_chunks = (int)nchunks;
+    bytes = ssm_ssd_packed_scratch_bytes((int)walks, (int)nchunks, (int)s.nh, &state_bytes);
+  } else {
+    bytes = ssm_ssd_scratch_bytes((int)s.nb, (int)s.nl, (int)s.nh), state_bytes = ssm_ssd_state_scratch_bytes((int)s.nb, (int)s.nl, (int)s.nh);
+  }
+  Tensor Y, fin = at::empty({walks, s.nh, s.np, s.nn}, f32);
+  if (want_y) Y = at::empty_like(X);
+  Tensor ws = at::empty({bytes}, X.options().dtype(at::kByte));
+  const int64_t vec = s.nh * nchunks * chunk * 4;
+  char* base = reinterpret_cast<char*>(ws.data_ptr());
   a.batch = (int)s.nb, a.len = (int)s.nl, a.heads = (int)s.nh, a.headdim = (int)s.np, a.nstate = (int)s.nn, a.groups = (int)s.ng;
   a.chunk_size = (int)chunk, a.io_dtype = dtype_code(X, "ssd_scan"), a.dt_softplus = softplus, a.d_has_p = D.has_value() && D->dim() == 2;
+  a.phase = want_y ? 0 : 1;
   a.X = X.data_ptr(), a.dt = dt.data_ptr(), a.A = A.data_ptr<float>(), a.Bm = B.data_ptr(), a.Cm = C.data_ptr();
-  a.D = fptr(D), a.z = ptr(z), a.dt_bias = fptr(bias), a.initial_states = fptr(init), a.Y = Y.data_ptr(), a.final_states = fin.data_ptr<float>();
+  a.D = fptr(D), a.z = ptr(z), a.dt_bias = fptr(bias), a.initial_states = fptr(init), a.Y = want_y ? Y.data_ptr() : nullptr;
+  a.final_states = fin.data_ptr<float>();
   a.ws_dt = reinterpret_cast<float*>(base), a.ws_cum = reinterpret_cast<float*>(base + vec), a.ws_state = reinterpret_cast<float*>(base + 2 * vec);
-  a.ws_state_in = base + 2 * vec + ssm_ssd_state_scratch_bytes((int)s.nb, (int)s.nl, (int)s.nh);
+  a.ws_state_in = base + 2 * vec + state_bytes;
   a.status = ssd_status(X.get_device()).data_ptr<int32_t>();
   run(ssm_ssd_fwd(&a, stream_of(X)));
   return {Y, fin};
+}
+
+std::tuple<Tensor, Tensor> ssd_forward(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
+                                       const OptTensor& z, const OptTensor& dt_bias, bool softplus, const OptTensor& init, int64_t chunk) {
+  ValueErrors scope;
+  return ssd_run(X, dt, A, B, C, D, z, dt_bias, softplus, init, chunk, nullptr, true);
+}
+
+// Packed sequences.  reset: Y restarts at every boundary; without it Y is the scan through all of them.  -> (Y, last state, states)
+std::tuple<Tensor, Tensor, Tensor> ssd_packed(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
+                                              const OptTensor& z, const OptTensor& dt_bias, bool softplus, const OptTensor& init, int64_t chunk,
+                                              const Tensor& cu_seqlens, bool reset) {
+  ValueErrors scope;
+  const std::vector<int64_t> cu = seq_bounds(cu_seqlens, X.size(1));
+  auto [Y, states] = ssd_run(X, dt, A, B, C, D, z, dt_bias, softplus, c10::nullopt, chunk, &cu, reset);
+  Tensor last;
+  if (reset) last = states.slice(0, states.size(0) - 1).clone();
+  else std::tie(Y, last) = ssd_run(X, dt, A, B, C, D, z, dt_bias, softplus, init, chunk, nullptr, true);
+  return {Y, last, states};
 }
 
 }  // namespace
@@ -636,6 +688,7 @@ void bind_operators(py::module& m) {
   ops.def("mamba1_step", &mamba1_step);
   ops.def("mamba2_step", &mamba2_step);
   ops.def("ssd_forward", &ssd_forward);
+  ops.def("ssd_packed", &ssd_packed);
   ops.def("ssd_status", &ssd_status);
   ops.def("ssd_poll", &ssd_poll);
 }

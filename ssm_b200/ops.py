@@ -831,12 +831,21 @@ def ssd_scan(
             raise ValueError("return_varlen_states needs cu_seqlens.")
         Y, final = _SsdFn.apply(X, dt, A, B, C, D, z, dt_bias, dt_softplus, initial_states, chunk_size, check_status, dual)
         return (Y, final) if return_final_states else Y
-    # packed sequences: every sequence is its own scan from a zero state (chunks counted from its first token), so the
-    # kernels see plain dense problems; the boundaries are host integers (one read of cu_seqlens)
+    # packed sequences: every sequence is its own scan from a zero state (chunks counted from its first token); the boundaries are
+    # host integers (one read of cu_seqlens).  Without gradients the tensor-core kernels take them all at once, otherwise the
+    # scans are separate dense problems
     if X.ndim != 4 or X.shape[0] != 1:
         raise ValueError("cu_seqlens needs a batch of one (sequences packed along L).")
     if initial_states is not None and seq_reset:
         raise ValueError("initial_states cannot be combined with sequences that restart at cu_seqlens.")
+    grads = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (X, dt, A, B, C, D, z, dt_bias, initial_states))
+    if not grads and X.shape[1] > 0 and ssd_tensor_core_supported(X, B, chunk_size):  # all sequences in one set of launches
+        Y, final, varlen = _native().ssd_packed(X, dt, A, B, C, D, z, dt_bias, dt_softplus, initial_states, int(chunk_size), torch.as_tensor(cu_seqlens),
+                                                seq_reset)
+        if check_status:
+            ssd_check_status(X.device)
+        out = (Y,) + ((final,) if return_final_states else ()) + ((varlen,) if return_varlen_states else ())
+        return out[0] if len(out) == 1 else out
     cu = [int(v) for v in torch.as_tensor(cu_seqlens).tolist()]
     if len(cu) < 2 or cu[0] != 0 or cu[-1] != X.shape[1] or any(b < a for a, b in zip(cu, cu[1:])):
         raise ValueError("cu_seqlens must rise from 0 to L.")

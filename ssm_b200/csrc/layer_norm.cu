@@ -15,7 +15,7 @@
 namespace ssmb {
 
 constexpr int kNormFwdChunks = 4;  // 16-byte chunks of x per thread, forward
-constexpr int kNormBwdChunks = 2;  // widest backward configuration: 512 threads x 2 chunks
+constexpr int kNormBwdChunks = 4;  // widest backward configuration: 512 threads x 4 chunks
 constexpr int kNormBwdMaxCtas = 592;  // 4 per SM on a 148-SM part
 
 // V consecutive elements of run-time type -> fp32
@@ -290,125 +290,172 @@ load_param_vec<V>(a.weight, ch * V, a.param_dtype, wv);
   }
 }
 
-// MC = 16-byte chunks of a row per thread.  A row of up to 32 * MC chunks is owned by ONE warp (G = 32): every reduction is
-// a shuffle tree and four rows are in flight per CTA; wider rows take 128 or 512 threads with block-wide reductions.
-// The time of a row is a chain of latencies (loads, two reductions, stores), so what counts is how many loads an SM has in
-// flight: all loads of a row are issued before the first use, and with 128-thread CTAs the running weight / bias gradients
-// of a thread's columns live in shared-memory slots of its own (same additions in the same order) instead of 16 MC registers,
-// which leaves the registers to the loads in flight and lets more CTAs fit.
+// Sums of two values over the G threads of a row group.  Wide groups exchange them through one of two scratch rows used in turn,
+// so a reduction costs one barrier: whoever writes a row again has passed the barrier of the reduction in between.
+template <int G>
+__device__ __forceinline__ void group_allsum2(float& a, float& b, float2 (*scratch)[16], int& turn) {
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, off);
+    b += __shfl_xor_sync(0xffffffffu, b, off);
+  }
+  if constexpr (G > 32) {
+    if ((threadIdx.x & 31) == 0) scratch[turn][threadIdx.x >> 5] = make_float2(a, b);
+    __syncthreads();
+    a = 0.f, b = 0.f;
+#pragma unroll
+    for (int w = 0; w < G / 32; ++w) {
+      const float2 v = scratch[turn][w];
+      a += v.x, b += v.y;
+    }
+    turn ^= 1;
+  }
+}
+
+// A row's pieces of everything the backward pass reads, in flight: x, the residual, dy, and the gradient arriving through the
+// x + residual output.
+template <int MC>
+struct NormBwdRaw {
+  NormRowRaw<MC> in;
+  uint4 dy[MC], ga[MC], gb[MC];
+};
+
+// MC = 16-byte chunks of a row per thread.  A row of up to 32 * MC chunks is owned by ONE warp (G = 32); wider rows take 128 or
+// 512 threads.  The time of a row is a chain of latencies, so:
+//  * every load of a row is issued before the first use (requesting the next row ahead as well costs more CTAs per SM than it
+//    hides: 123 us against 107);
+//  * a row needs two rounds of sums, two values each: {sum s, sum w dy}, then {sum (s - mean)^2, sum w dy (s - mean)}, from which
+//    the standard deviation and both correction terms follow (one round for RMSNorm);
+//  * with 128-thread CTAs the running weight / bias gradients of a thread's columns live in shared-memory slots of its own, four
+//    to a 16-byte access (same additions in the same order), which leaves the registers to the loads in flight.
+// 16376 rows of 1600 bf16 columns, fp32 residual and its gradient, 471 MB: 157 us with one barrier pair per value and sum, now
+// 107 us (4.4 TB/s).
 template <int G, int MC>
 constexpr int norm_bwd_min_ctas() {
-  return G <= 128 ? (MC <= 2 ? 5 : (MC == 3 ? 3 : 2)) : 1;
+  return G <= 128 ? (MC <= 1 ? 5 : (MC == 2 ? 4 : (MC == 3 ? 3 : 2))) : 1;
 }
 template <typename T, int G, int MC>
 __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_min_ctas<G, MC>()) norm_bwd_kernel(const ssm_norm_bwd_args g) {
   using Cfg = NormCfg<T, G>;
   constexpr int V = Cfg::V;
-  constexpr int kNormBwdChunks = MC;
   constexpr bool kSmemAcc = G <= 128;
   constexpr int kAccRegs = kSmemAcc ? 1 : MC;
-  constexpr int kAccRow = MC * V * G + 1;
+  constexpr int kAccRow = MC * (V / 4) * G;  // float4 slots of one gradient: [chunk][quarter][thread]
   const ssm_norm_args& a = g.fwd;
-  __shared__ float scratch[32];
-  __shared__ float acc_all[kSmemAcc ? Cfg::RPC * 2 * kAccRow : 1];  // [row slot][weight | bias][chunk][element][thread]
+  __shared__ float2 scratch[2][16];
+  __shared__ float4 acc_all[kSmemAcc ? Cfg::RPC * 2 * kAccRow : 1];  // [row slot][weight | bias]
   const int gt = threadIdx.x % G, slot = threadIdx.x / G;
-  float* acc = acc_all + (kSmemAcc ? slot * 2 * kAccRow : 0);
+  float4* acc = acc_all + (kSmemAcc ? slot * 2 * kAccRow : 0);
   const int nchunk = a.hidden / V;
   const float inv = 1.f / (float)a.hidden;
   float dw[kAccRegs][V], db[kAccRegs][V];
 #pragma unroll
-  for (int c = 0; c < kNormBwdChunks; ++c)
+  for (int c = 0; c < MC; ++c) {
+    if constexpr (kSmemAcc) {
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      if constexpr (kSmemAcc) acc[(c * V + i) * G + gt] = 0.f, acc[kAccRow + (c * V + i) * G + gt] = 0.f;
-      else dw[c][i] = 0.f, db[c][i] = 0.f;
+      for (int q = 0; q < V / 4; ++q) acc[(c * (V / 4) + q) * G + gt] = acc[kAccRow + (c * (V / 4) + q) * G + gt] = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+#pragma unroll
+      for (int i = 0; i < V; ++i) dw[c][i] = 0.f, db[c][i] = 0.f;
     }
-  // the weights of this thread's columns are re-read from L1 for every row (16-byte loads) instead of occupying registers
+  }
+  // the weights of this thread's columns are re-read from L1 for every row instead of occupying registers
   auto load_w = [&](int c, float (&wv)[V]) {
     load_param_vec<V>(a.weight, min(c * G + gt, nchunk - 1) * V, a.param_dtype, wv);  // beyond the row: dropped (dy is zero there)
   };
+  auto issue = [&](int64_t row, NormBwdRaw<MC>& raw) {
+    norm_issue_row<T, G, MC>(a, row, gt, nchunk, raw.in);
+    io_issue_row<T, G, MC>(g.dy, row * a.hidden, gt, nchunk, raw.dy);
+    if (g.dresidual_out) dyn_issue_row<V, G, MC>(g.dresidual_out, row * a.hidden, gt, nchunk, a.resout_dtype, raw.ga, raw.gb);
+  };
   const int64_t npass = (a.rows + Cfg::RPC - 1) / Cfg::RPC;
+  int turn = 0;
   for (int64_t pass = blockIdx.x; pass < npass; pass += gridDim.x) {
     const int64_t row = pass * Cfg::RPC + slot;
-    const bool live = row < a.rows;  // G == 32: a dead warp still joins nothing but its own shuffles
-    float s[kNormBwdChunks][V], r[kNormBwdChunks][V], dy[kNormBwdChunks][V];
-    if (live) {
-      // every load of the row goes out before the first value is used: x, the residual, dy and the gradient arriving through
-      // the x + residual output (which takes the place of the residual values, dead once the row sum is formed)
-      NormRowRaw<kNormBwdChunks> raw;
-      uint4 dyr[kNormBwdChunks], ga[kNormBwdChunks], gb[kNormBwdChunks];
-      norm_issue_row<T, G, kNormBwdChunks>(a, row, gt, nchunk, raw);
-      io_issue_row<T, G, kNormBwdChunks>(g.dy, row * a.hidden, gt, nchunk, dyr);
-      if (g.dresidual_out) dyn_issue_row<V, G, kNormBwdChunks>(g.dresidual_out, row * a.hidden, gt, nchunk, a.resout_dtype, ga, gb);
-      norm_convert_row<T, G, kNormBwdChunks>(a, gt, nchunk, raw, s, r);
+    const bool live = row < a.rows;  // dead warps of the last pass (G == 32) work on the last row again and drop the result
+    float s[MC][V], r[MC][V], dy[MC][V];
+    NormBwdRaw<MC> raw;
+    issue(live ? row : a.rows - 1, raw);
+    norm_convert_row<T, G, MC>(a, gt, nchunk, raw.in, s, r);
 #pragma unroll
-      for (int c = 0; c < kNormBwdChunks; ++c) {
-        if (c * G + gt < nchunk) {
-          Vec16<T> v;
-          v.raw = dyr[c];
-          v.unpack(dy[c]);
-          if (g.dresidual_out) dyn_convert<V>(a.resout_dtype, ga[c], gb[c], r[c]);
-        } else {
+    for (int c = 0; c < MC; ++c) {
+      if (live && c * G + gt < nchunk) {
+        Vec16<T> v;
+        v.raw = raw.dy[c];
+        v.unpack(dy[c]);
+        // the gradient through x + residual takes the place of the residual values, dead once the row sum is formed
+        if (g.dresidual_out) dyn_convert<V>(a.resout_dtype, raw.ga[c], raw.gb[c], r[c]);
+      } else {
 #pragma unroll
-          for (int i = 0; i < V; ++i) dy[c][i] = 0.f;
-        }
+        for (int i = 0; i < V; ++i) dy[c][i] = 0.f;
       }
-    } else {
-#pragma unroll
-      for (int c = 0; c < kNormBwdChunks; ++c)
-#pragma unroll
-        for (int i = 0; i < V; ++i) s[c][i] = 0.f, r[c][i] = 0.f, dy[c][i] = 0.f;
     }
-    float mean, rstd;
-    norm_stats<T, G, kNormBwdChunks>(a, gt, nchunk, s, scratch, mean, rstd);
-    float c1 = 0.f, c2 = 0.f;
+    float mean = 0.f, c2 = 0.f;
+    if (!a.is_rms) {
 #pragma unroll
-    for (int c = 0; c < kNormBwdChunks; ++c) {
+      for (int c = 0; c < MC; ++c) {
+        float wv[V];
+        load_w(c, wv);
+#pragma unroll
+        for (int i = 0; i < V; ++i) mean += s[c][i], c2 = fmaf(dy[c][i], wv[i], c2);
+      }
+      group_allsum2<G>(mean, c2, scratch, turn);
+      mean *= inv, c2 *= inv;
+    }
+    float q = 0.f, c1 = 0.f;
+#pragma unroll
+    for (int c = 0; c < MC; ++c) {
       float wv[V];
       load_w(c, wv);
+      if (c * G + gt < nchunk) {
 #pragma unroll
-      for (int i = 0; i < V; ++i) {
-        const float xh = (s[c][i] - mean) * rstd;
-        const float wdy = dy[c][i] * wv[i];
-        s[c][i] = xh;  // keep xhat
-        c1 = fmaf(wdy, xh, c1);
-        c2 += wdy;
-        if (live && (c * G + gt) < nchunk) {
-          if constexpr (kSmemAcc) {
-            float* pw = acc + (c * V + i) * G + gt;
-            float* pb = acc + kAccRow + (c * V + i) * G + gt;
-            *pw = fmaf(dy[c][i], xh, *pw);
-            *pb += dy[c][i];
-          } else {
-            dw[c][i] = fmaf(dy[c][i], xh, dw[c][i]);
-            db[c][i] += dy[c][i];
-          }
+        for (int i = 0; i < V; ++i) {
+          s[c][i] -= mean;
+          q = fmaf(s[c][i], s[c][i], q);
+          c1 = fmaf(dy[c][i] * wv[i], s[c][i], c1);
         }
       }
     }
-    c1 = group_allsum<G>(c1, scratch) * inv;
-    c2 = a.is_rms ? 0.f : group_allsum<G>(c2, scratch) * inv;
-    if (live) {
+    group_allsum2<G>(q, c1, scratch, turn);
+    const float rstd = rsqrtf(q * inv + a.eps);
+    c1 *= inv * rstd;
 #pragma unroll
-      for (int c = 0; c < kNormBwdChunks; ++c) {
-        const int ch = c * G + gt;
-        if (ch < nchunk) {
-          float dsv[V], wv[V];
-          load_w(c, wv);
+    for (int c = 0; c < MC; ++c) {
+      const int ch = c * G + gt;
+      if (live && ch < nchunk) {
 #pragma unroll
-          for (int i = 0; i < V; ++i) dsv[i] = (dy[c][i] * wv[i] - s[c][i] * c1 - c2) * rstd;
-          const int64_t off = row * a.hidden + (int64_t)ch * V;
-          if (g.dresidual_out) {  // gradient arriving through the x + residual output reaches x and residual unchanged
+        for (int i = 0; i < V; ++i) s[c][i] *= rstd;  // xhat
+        if constexpr (kSmemAcc) {
 #pragma unroll
-            for (int i = 0; i < V; ++i) dsv[i] += r[c][i], dy[c][i] += r[c][i];
+          for (int k = 0; k < V / 4; ++k) {
+            float4* pw = acc + (c * (V / 4) + k) * G + gt;
+            float4* pb = pw + kAccRow;
+            float4 w4 = *pw, b4 = *pb;
+            const float *d = &dy[c][4 * k], *x = &s[c][4 * k];
+            w4.x = fmaf(d[0], x[0], w4.x), w4.y = fmaf(d[1], x[1], w4.y), w4.z = fmaf(d[2], x[2], w4.z), w4.w = fmaf(d[3], x[3], w4.w);
+            b4.x += d[0], b4.y += d[1], b4.z += d[2], b4.w += d[3];
+            *pw = w4;
+            if (g.dbias) *pb = b4;
           }
-          Vec16<T> v;
-          v.pack(dsv);
-          v.store_stream(reinterpret_cast<T*>(g.dx) + off);
-          if (g.dresidual) {
-            if (a.prenorm) store_dyn_vec<V>(g.dresidual, off, a.res_dtype, dsv);
-            else store_dyn_vec<V>(g.dresidual, off, a.res_dtype, dy[c]);
-          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < V; ++i) dw[c][i] = fmaf(dy[c][i], s[c][i], dw[c][i]), db[c][i] += dy[c][i];
+        }
+        float dsv[V], wv[V];
+        load_w(c, wv);
+#pragma unroll
+        for (int i = 0; i < V; ++i) dsv[i] = (dy[c][i] * wv[i] - s[c][i] * c1 - c2) * rstd;
+        const int64_t off = row * a.hidden + (int64_t)ch * V;
+        if (g.dresidual_out) {  // gradient arriving through the x + residual output reaches x and residual unchanged
+#pragma unroll
+          for (int i = 0; i < V; ++i) dsv[i] += r[c][i], dy[c][i] += r[c][i];
+        }
+        Vec16<T> v;
+        v.pack(dsv);
+        v.store_stream(reinterpret_cast<T*>(g.dx) + off);
+        if (g.dresidual) {
+          if (a.prenorm) store_dyn_vec<V>(g.dresidual, off, a.res_dtype, dsv);
+          else store_dyn_vec<V>(g.dresidual, off, a.res_dtype, dy[c]);
         }
       }
     }
@@ -419,22 +466,26 @@ __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_min_ctas<G, MC>
     float* pw = g.partial + (int64_t)blockIdx.x * 2 * a.hidden;
     float* pb = pw + a.hidden;
 #pragma unroll
-    for (int c = 0; c < kNormBwdChunks; ++c) {
+    for (int c = 0; c < MC; ++c) {
       const int ch = c * G + gt;
       if (ch < nchunk) {
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
+        for (int k = 0; k < V / 4; ++k) {
+          float4 tw, tb;
           if constexpr (kSmemAcc) {
-            float tw = 0.f, tb = 0.f;
+            tw = tb = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int q = 0; q < Cfg::RPC; ++q) {
-              tw += acc_all[q * 2 * kAccRow + (c * V + i) * G + gt];
-              tb += acc_all[q * 2 * kAccRow + kAccRow + (c * V + i) * G + gt];
+              const float4 x = acc_all[q * 2 * kAccRow + (c * (V / 4) + k) * G + gt], y = acc_all[(q * 2 + 1) * kAccRow + (c * (V / 4) + k) * G + gt];
+              tw.x += x.x, tw.y += x.y, tw.z += x.z, tw.w += x.w;
+              tb.x += y.x, tb.y += y.y, tb.z += y.z, tb.w += y.w;
             }
-            pw[ch * V + i] = tw, pb[ch * V + i] = tb;
           } else {
-            pw[ch * V + i] = dw[c][i], pb[ch * V + i] = db[c][i];
+            tw = make_float4(dw[c][4 * k], dw[c][4 * k + 1], dw[c][4 * k + 2], dw[c][4 * k + 3]);
+            tb = make_float4(db[c][4 * k], db[c][4 * k + 1], db[c][4 * k + 2], db[c][4 * k + 3]);
           }
+          *reinterpret_cast<float4*>(pw + ch * V + 4 * k) = tw;
+          *reinterpret_cast<float4*>(pb + ch * V + 4 * k) = tb;
         }
       }
     }
@@ -443,7 +494,7 @@ __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_min_ctas<G, MC>
 
 // Column sums of the per-CTA partial rows: 32 columns x kFoldLanes partial-row lanes per CTA,
 // so the loads of a column are spread over many threads instead of one serial chain.
-constexpr int kFoldLanes = 16;
+constexpr int kFoldLanes = 32;
 __global__ void __launch_bounds__(32 * kFoldLanes) norm_fold_kernel(const float* __restrict__ partial, int nctas, int hidden,
                                                                    void* __restrict__ dweight, void* __restrict__ dbias, int dtype) {
   __shared__ float sw[kFoldLanes][33], sb[kFoldLanes][33];
@@ -558,14 +609,6 @@ static bool norm_vec_ok(const ssm_norm_args& a, int maxchunks, const void* p1, c
   return ok(a.x) && ok(a.y) && ok(a.residual) && ok(a.residual_out) && ok(a.weight) && ok(a.bias) && ok(p1) && ok(p2) && ok(p3);
 }
 
-static int norm_group(const ssm_norm_args& a, int maxchunks) {
-  const int V = 16 / dtype_size(a.io_dtype);
-  const int nchunk = a.hidden / V;
-  if (nchunk <= 32 * maxchunks) return 32;
-  if (nchunk <= 128 * maxchunks) return 128;
-  return 512;
-}
-
 static int norm_bwd_ctas(const ssm_norm_args& a, int rpc) {
   const int64_t npass = (a.rows + rpc - 1) / rpc;
   return (int)(npass < kNormBwdMaxCtas ? npass : kNormBwdMaxCtas);
@@ -611,7 +654,8 @@ static int norm_bwd_dispatch(const ssm_norm_bwd_args& g, cudaStream_t st, int ma
   if (nchunk <= 256) return norm_bwd_launch<T, 128, 2>(g, st, max_ctas);
   if (nchunk <= 384) return norm_bwd_launch<T, 128, 3>(g, st, max_ctas);  // e.g. 2560 columns of 16 bits: three CTAs per SM, not two
   if (nchunk <= 512) return norm_bwd_launch<T, 128, 4>(g, st, max_ctas);
-  return norm_bwd_launch<T, 512, 2>(g, st, max_ctas);
+  if (nchunk <= 1024) return norm_bwd_launch<T, 512, 2>(g, st, max_ctas);
+  return norm_bwd_launch<T, 512, 4>(g, st, max_ctas);
 }
 
 template <typename T>
@@ -623,11 +667,16 @@ static int norm_fwd_t(const ssm_norm_args& a, cudaStream_t st) {
     return launch_status("norm_scalar_kernel");
   }
   const int nchunk = a.hidden / (16 / (int)sizeof(T));
-  switch (norm_group(a, kNormFwdChunks)) {
-    case 32: return norm_fwd_launch<T, 32>(a, st);
-    case 128: return norm_fwd_launch<T, 128>(a, st);
-    default: return nchunk <= 128 * 6 ? norm_fwd_launch<T, 128, 6>(a, st) : norm_fwd_launch<T, 512>(a, st);
-  }
+  // as few chunks per thread as the row needs: what a thread does not hold leaves room for more rows in flight
+  if (nchunk <= 32) return norm_fwd_launch<T, 32, 1>(a, st);
+  if (nchunk <= 64) return norm_fwd_launch<T, 32, 2>(a, st);
+  if (nchunk <= 96) return norm_fwd_launch<T, 32, 3>(a, st);
+  if (nchunk <= 128) return norm_fwd_launch<T, 32, 4>(a, st);
+  if (nchunk <= 256) return norm_fwd_launch<T, 128, 2>(a, st);
+  if (nchunk <= 384) return norm_fwd_launch<T, 128, 3>(a, st);
+  if (nchunk <= 512) return norm_fwd_launch<T, 128, 4>(a, st);
+  if (nchunk <= 768) return norm_fwd_launch<T, 128, 6>(a, st);
+  return norm_fwd_launch<T, 512>(a, st);
 }
 // rows that cannot be vectorised: sums by atomics into one partial row, folded into the element type of the gradients
 template <typename T>

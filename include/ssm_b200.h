@@ -251,17 +251,18 @@ int ssm_chunk_scan_bwd(const ssm_chunk_bwd_args* args, ssm_stream_t stream);
  * (src/ssm/ops/cuda/dw_causal_conv.cu:771-857, 859-965; spec reference.py:466-537).
  *
  * x, y: channels_first ? (batch, channels, len) : (batch, len, channels), io_dtype.
- * weight: (channels, width) fp32, tap j multiplies x[t - (width-1) + j].  bias fp32/NULL.
+ * weight: (channels, width), tap j multiplies x[t - (width-1) + j].  bias (channels) or NULL; both param_dtype.
  * 1 <= width <= 8.  Optional halo: (batch, channels, width-1) fp32 inputs that precede
  * t = 0 (sequence-sharded prefill; NULL means zeros, the upstream behaviour).
  * Backward: dx io_dtype; dweight (channels, width), dbias (channels) fp32 accumulated into.
  * ------------------------------------------------------------------------------------- */
 typedef struct {
   int32_t batch, channels, len, width;
-  int32_t io_dtype, channels_first, silu, reserved0;
+  int32_t io_dtype, channels_first, silu;
+  int32_t param_dtype; /* element type of weight and bias (0: fp32); their gradients are fp32 */
   const void* x;
-  const float* weight;
-  const float* bias; /* nullable */
+  const void* weight;
+  const void* bias;  /* nullable */
   const float* halo; /* nullable */
   void* y;
   /* channels_first only: element strides of the batch and channel axes of x, y (and dy, dx);

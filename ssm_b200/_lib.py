@@ -89,7 +89,7 @@ class ChunkBwdArgs(C.Structure):
 class ConvArgs(C.Structure):
     _fields_ = [
         ("batch", i32), ("channels", i32), ("len", i32), ("width", i32),
-        ("io_dtype", i32), ("channels_first", i32), ("silu", i32), ("reserved0", i32),
+        ("io_dtype", i32), ("channels_first", i32), ("silu", i32), ("param_dtype", i32),
         ("x", vp), ("weight", fp), ("bias", fp), ("halo", fp), ("y", vp),
         ("row_sb", i64), ("row_sc", i64),
     ]

@@ -45,6 +45,14 @@ inline int launch_status(const char* kernel) {
   return SSM_OK;
 }
 
+// SMs of the current device (148 on a B200)
+inline int sm_count() {
+  int dev = 0, n = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n;
+}
+
 inline bool valid_dtype(int d) { return d == SSM_F32 || d == SSM_BF16 || d == SSM_F16; }
 inline int dtype_size(int d) { return d == SSM_F32 ? 4 : 2; }
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }

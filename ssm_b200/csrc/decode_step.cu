@@ -424,12 +424,6 @@ __global__ void __launch_bounds__(kDecThreads, 1) mamba2_decode_kernel(const ssm
   }
 }
 
-static int dec_sms() {
-  int dev = 0, n = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n;
-}
 // Warps per tile: the split with the least rounds x (columns per warp + a round's fixed cost, which is worth about eight
 // 32-column pieces: two CTA barriers, the exchange of the partial sums, the epilogue).
 static int dec_split(int tiles, int k, int sms) {
@@ -483,7 +477,7 @@ extern "C" int ssm_mamba1_decode(const ssm_mamba1_decode_args* a, ssm_stream_t s
   SSM_REQUIRE(aligned_to(a->hidden, 16) && aligned_to(a->in_x, 16) && aligned_to(a->in_z, 16) && aligned_to(a->x_proj, 16) && aligned_to(a->dt_proj, 8) &&
                   aligned_to(a->out_proj, 16) && aligned_to(a->conv_state, 16) && aligned_to(a->ssm_state, 16) && aligned_to(a->A, 16) && aligned_to(a->scratch, 16),
               SSM_ERR_ALIGN, "mamba1_decode: tensors must be 16-byte aligned");
-  const int sms = dec_sms();
+  const int sms = sm_count();
   DecSplits sp{};
   sp.s[0] = dec_split(2 * tiles_of(a->d_inner), a->d_model, sms);
   sp.s[1] = dec_split(tiles_of(a->dt_rank + 2 * a->nstate), a->d_inner, sms);
@@ -515,7 +509,7 @@ extern "C" int ssm_mamba2_decode(const ssm_mamba2_decode_args* a, ssm_stream_t s
                   aligned_to(a->in_dt, 16) && aligned_to(a->out_proj, 16) && aligned_to(a->conv_state_x, 16) && aligned_to(a->conv_state_B, 16) &&
                   aligned_to(a->conv_state_C, 16) && aligned_to(a->ssm_state, 16) && aligned_to(a->scratch, 16),
               SSM_ERR_ALIGN, "mamba2_decode: tensors must be 16-byte aligned");
-  const int sms = dec_sms(), di = a->heads * 64;
+  const int sms = sm_count(), di = a->heads * 64;
   DecSplits sp{};
   sp.s[0] = dec_split(2 * tiles_of(di) + 2 * tiles_of(a->groups * 128) + tiles_of(a->heads), a->d_model, sms);
   sp.s[1] = dec_split(tiles_of(a->d_model), di, sms);

@@ -8,6 +8,8 @@
 //
 // Taps are held newest-first: wr[m] = weight[K-1-m] multiplies x[t-m], so that every
 // register-array index below is a compile-time constant for any run-time width K <= 8.
+#include <math.h>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -30,8 +32,12 @@ __device__ __forceinline__ float conv_x_at(const T* __restrict__ row, const floa
 // ---------------------------------------------------------------------------------------
 // channels-first forward
 // ---------------------------------------------------------------------------------------
-template <typename T, int KM>
-__global__ void __launch_bounds__(kConvThreads) conv_cf_fwd_kernel(const ssm_conv_args a, int vec) {
+// How the rows of a channels-first tensor can be read: element by element (the tensor itself is off a 16-byte boundary), as 16-byte
+// pieces from end to end, or as pieces with ragged ends.
+enum { kRowScalar = 0, kRowPieces = 1, kRowRagged = 2 };
+
+template <typename T, int KM, int ROW>
+__global__ void __launch_bounds__(kConvThreads) conv_cf_fwd_kernel(const ssm_conv_args a) {
   constexpr int KH = KM - 1;
   constexpr int V = 16 / sizeof(T);
   const int64_t rowi = blockIdx.x;  // b * C + c
@@ -43,62 +49,75 @@ __global__ void __launch_bounds__(kConvThreads) conv_cf_fwd_kernel(const ssm_con
   const float* halo = a.halo ? a.halo + rowi * (K - 1) : nullptr;
   float wr[KM];
 #pragma unroll
-  for (int m = 0; m < KM; ++m) wr[m] = m < K ? __ldg(a.weight + (int64_t)c * K + (K - 1 - m)) : 0.f;
-  const float bias = a.bias ? __ldg(a.bias + c) : 0.f;
+  for (int m = 0; m < KM; ++m) wr[m] = m < K ? load_dyn(a.weight, (int64_t)c * K + (K - 1 - m), a.param_dtype) : 0.f;
+  const float bias = a.bias ? load_dyn(a.bias, c, a.param_dtype) : 0.f;
+  int lo = 0, hi = 0;
 
-  if (vec) {
+  if constexpr (ROW != kRowScalar) {
+    // A row may start anywhere: its 16-byte pieces are cut where they lie in memory, so piece ch holds the steps ch * V - sh ..,
+    // sh = the row's offset from a 16-byte boundary (the same for x and y).  The loop below takes the pieces that lie inside the row
+    // and whose earlier inputs do too, or precede the row altogether (sh = 0); the steps at ragged ends are left to the scalar
+    // loop.
     // A thread takes UB vectors of 16 bytes per pass and issues their loads, and those of the vectors before them (the K - 1
     // earlier inputs: the neighbouring thread's vector, served by the L1), before the first value is used.  Vectors beyond the
     // end of the row are read at the last valid address and dropped.
-    constexpr int UB = 4;
-    const int nch = L / V;
-    for (int base = threadIdx.x; base < nch; base += kConvThreads * UB) {
-      uint4 curr[UB], prvr[UB];
+    constexpr int UB = 4, NB = (KH + V - 1) / V;
+    const int sh = ROW == kRowRagged ? (int)(roff % V) : 0, ch0 = sh ? NB + 1 : 0, nch = (L + sh) / V;
+    const T* xg = x - sh;
+    if (ch0 < nch) {
+      lo = ch0 * V - sh, hi = nch * V - sh;
+      for (int base = ch0 + threadIdx.x; base < nch; base += kConvThreads * UB) {
+        uint4 curr[UB], prvr[UB][NB];
 #pragma unroll
-      for (int j = 0; j < UB; ++j) {
-        const int ch = min(base + j * kConvThreads, nch - 1);
-        curr[j] = __ldcs(reinterpret_cast<const uint4*>(x + (int64_t)ch * V));
-        prvr[j] = __ldg(reinterpret_cast<const uint4*>(x + (int64_t)max(ch - 1, 0) * V));
-      }
+        for (int j = 0; j < UB; ++j) {
+          const int ch = min(base + j * kConvThreads, nch - 1);
+          curr[j] = __ldcs(reinterpret_cast<const uint4*>(xg + (int64_t)ch * V));
 #pragma unroll
-      for (int j = 0; j < UB; ++j) {
-        const int ch = base + j * kConvThreads;
-        if (ch >= nch) break;
-        const int t0 = ch * V;
-        Vec16<T> v;
-        float cur[V], prv[V], hist[KH > 0 ? KH : 1];  // hist[m] = x[t0 - 1 - m]
-        v.raw = curr[j];
-        v.unpack(cur);
-        v.raw = prvr[j];
-        v.unpack(prv);
-#pragma unroll
-        for (int m = 0; m < KH; ++m) {
-          float hv = 0.f;
-          if (m < K - 1) hv = (ch > 0 && m < V) ? prv[m < V ? V - 1 - m : 0] : conv_x_at<T>(x, halo, K, t0 - 1 - m, L);
-          hist[m] = hv;
+          for (int q = 0; q < NB; ++q) prvr[j][q] = __ldg(reinterpret_cast<const uint4*>(xg + (int64_t)max(ch - 1 - q, 0) * V));
         }
-        float out[V];
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          float acc = bias;
+        for (int j = 0; j < UB; ++j) {
+          const int ch = base + j * kConvThreads;
+          if (ch >= nch) break;
+          Vec16<T> v;
+          float cur[V], prv[NB][V];  // prv[q][i] = x[t0 - (q + 1) V + i]
+          v.raw = curr[j];
+          v.unpack(cur);
 #pragma unroll
-          for (int m = 0; m < KM; ++m) {
-            if (m < K) acc = fmaf(wr[m], (i - m >= 0) ? cur[(i - m >= 0) ? i - m : 0] : hist[(m - i - 1 >= 0) ? m - i - 1 : 0], acc);
+          for (int q = 0; q < NB; ++q) {
+            v.raw = prvr[j][q], v.unpack(prv[q]);
+            if (ch - 1 - q < 0) {
+#pragma unroll
+              for (int i = 0; i < V; ++i) prv[q][i] = conv_x_at<T>(x, halo, K, (ch - 1 - q) * V + i, L);
+            }
           }
-          out[i] = a.silu ? (sizeof(T) == 2 ? silu_half_io(acc) : silu_fast(acc)) : acc;
+          float out[V];
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            float acc = bias;
+#pragma unroll
+            for (int m = 0; m < KM; ++m) {
+              constexpr int kLast = V - 1;
+              const int back = m - i - 1;  // steps before the piece, when not inside it
+              if (m < K) acc = fmaf(wr[m], i >= m ? cur[i >= m ? i - m : 0] : prv[back >= 0 ? back / V : 0][back >= 0 ? kLast - back % V : 0], acc);
+            }
+            out[i] = a.silu ? (sizeof(T) == 2 ? silu_half_io(acc) : silu_fast(acc)) : acc;
+          }
+          v.pack(out);
+          v.store_stream(y - sh + (int64_t)ch * V);
         }
-        v.pack(out);
-        v.store_stream(y + t0);
       }
     }
-  } else {
-    for (int t = threadIdx.x; t < L; t += kConvThreads) {
-      float acc = bias;
+  }
+  if constexpr (ROW == kRowPieces) return;
+  // the steps outside [lo, hi): all of a row that cannot be read in pieces
+  for (int u = threadIdx.x; u < L - (hi - lo); u += kConvThreads) {
+    const int t = u < lo ? u : u + (hi - lo);
+    float acc = bias;
 #pragma unroll
-      for (int m = 0; m < KM; ++m)
-        if (m < K) acc = fmaf(wr[m], conv_x_at<T>(x, halo, K, t - m, L), acc);
-      y[t] = from_f<T>(a.silu ? silu_fast(acc) : acc);
-    }
+    for (int m = 0; m < KM; ++m)
+      if (m < K) acc = fmaf(wr[m], conv_x_at<T>(x, halo, K, t - m, L), acc);
+    y[t] = from_f<T>(a.silu ? (sizeof(T) == 2 ? silu_half_io(acc) : silu_fast(acc)) : acc);
   }
 }
 
@@ -106,8 +125,8 @@ __global__ void __launch_bounds__(kConvThreads) conv_cf_fwd_kernel(const ssm_con
 // channels-first backward.  pre[t] = bias + sum_m wr[m] x[t-m];  dpre = dy * act'(pre)
 //   dx[t] = sum_m wr[m] dpre[t+m];  dwr[m] += sum_t dpre[t] x[t-m];  dbias += sum_t dpre[t]
 // ---------------------------------------------------------------------------------------
-template <typename T, int KM>
-__global__ void __launch_bounds__(kConvThreads) conv_cf_bwd_kernel(const ssm_conv_bwd_args g, int vec) {
+template <typename T, int KM, int ROW>
+__global__ void __launch_bounds__(kConvThreads) conv_cf_bwd_kernel(const ssm_conv_bwd_args g) {
   constexpr int KH = KM - 1;
   const ssm_conv_args& a = g.fwd;
   const int64_t rowi = blockIdx.x;
@@ -120,86 +139,82 @@ __global__ void __launch_bounds__(kConvThreads) conv_cf_bwd_kernel(const ssm_con
   const float* halo = a.halo ? a.halo + rowi * (K - 1) : nullptr;
   float wr[KM], dwr[KM];
 #pragma unroll
-  for (int m = 0; m < KM; ++m) wr[m] = m < K ? __ldg(a.weight + (int64_t)c * K + (K - 1 - m)) : 0.f, dwr[m] = 0.f;
-  const float bias = a.bias ? __ldg(a.bias + c) : 0.f;
+  for (int m = 0; m < KM; ++m) wr[m] = m < K ? load_dyn(a.weight, (int64_t)c * K + (K - 1 - m), a.param_dtype) : 0.f, dwr[m] = 0.f;
+  const float bias = a.bias ? load_dyn(a.bias, c, a.param_dtype) : 0.f;
   float db = 0.f;
+  int lo = 0, hi = 0;
 
-  if (vec) {
-    // 16-byte accesses: a thread owns one vector of outputs and reads the neighbouring
-    // vectors of x (both sides) and dy (later side) through L1.
-    constexpr int V = 16 / sizeof(T);
-    constexpr int NB = (KH + V - 1) / V;  // neighbour vectors per side
-    const int last = L - V;  // start of the row's last vector: what out-of-range neighbours read (and drop)
-    for (int t0 = threadIdx.x * V; t0 < L; t0 += kConvThreads * V) {
-      // every load of the pass is issued before the first value is used
-      uint4 xr[2 * NB + 1], dyr[NB + 1];
+  if constexpr (ROW != kRowScalar) {
+    // 16-byte pieces cut where they lie in memory, as in the forward kernel; a ragged end of the row is left to the scalar loop.  A
+    // thread owns one piece of outputs and reads the neighbouring pieces of x (both sides) and dy (later side) through L1.
+    // (Taking the neighbours' x and dpre from the neighbouring lanes by shuffles instead of forming the K - 1 later dpre again
+    // needs fewer instructions but has fewer loads in flight: 101 us against 90 at (8, 1536, 4096) bf16.)
+    constexpr int V = 16 / sizeof(T), NB = (KH + V - 1) / V;  // NB: neighbour pieces per side
+    const int sh = ROW == kRowRagged ? (int)(roff % V) : 0, p1 = (L + sh) / V;
+    const int ch0 = sh ? NB + 1 : 0, ch1 = ROW == kRowRagged && (L + sh) % V ? p1 - NB : p1;  // the pieces whose outputs are formed here
+    if (ch0 < ch1) {
+      lo = ch0 * V - sh, hi = ch1 * V - sh;
+      const T *xg = x - sh, *dg = dy - sh;
+      for (int ch = ch0 + threadIdx.x; ch < ch1; ch += kConvThreads) {
+        // every load of the pass is issued before the first value is used
+        uint4 xr[2 * NB + 1], dyr[NB + 1];
 #pragma unroll
-      for (int j = 0; j <= 2 * NB; ++j) xr[j] = __ldg(reinterpret_cast<const uint4*>(x + min(max(t0 + (j - NB) * V, 0), last)));
+        for (int j = 0; j <= 2 * NB; ++j) xr[j] = __ldg(reinterpret_cast<const uint4*>(xg + (int64_t)min(max(ch + j - NB, 0), p1 - 1) * V));
 #pragma unroll
-      for (int j = 0; j <= NB; ++j) dyr[j] = __ldg(reinterpret_cast<const uint4*>(dy + min(t0 + j * V, last)));
-      float xa[(2 * NB + 1) * V];  // xa[q] = x[t0 - NB * V + q]
+        for (int j = 0; j <= NB; ++j) dyr[j] = __ldg(reinterpret_cast<const uint4*>(dg + (int64_t)min(ch + j, p1 - 1) * V));
+        float xa[(2 * NB + 1) * V];  // xa[q] = x[t0 - NB * V + q]
 #pragma unroll
-      for (int j = 0; j <= 2 * NB; ++j) {
-        const int tv = t0 + (j - NB) * V;
-        if (tv >= 0 && tv < L) {
+        for (int j = 0; j <= 2 * NB; ++j) {
+          const int cj = ch + j - NB;
           Vec16<T> v;
           v.raw = xr[j];
           float f[V];
           v.unpack(f);
+          if (cj < 0 || cj >= p1) {  // beyond an end on a boundary: the halo, or nothing
+#pragma unroll
+            for (int i = 0; i < V; ++i) f[i] = cj < 0 ? conv_x_at<T>(x, halo, K, cj * V + i, L) : 0.f;
+          }
 #pragma unroll
           for (int i = 0; i < V; ++i) xa[j * V + i] = f[i];
-        } else {
-#pragma unroll
-          for (int i = 0; i < V; ++i) xa[j * V + i] = tv < 0 ? conv_x_at<T>(x, halo, K, tv + i, L) : 0.f;
         }
-      }
-      float dya[(NB + 1) * V];  // dy[t0 + q], zero beyond the row
+        float dp[(NB + 1) * V];  // dpre[t0 + i], first dy
 #pragma unroll
-      for (int j = 0; j <= NB; ++j) {
-        const int tv = t0 + j * V;
-        float f[V];
-        if (tv < L) {
+        for (int j = 0; j <= NB; ++j) {
           Vec16<T> v;
-          v.raw = dyr[j];
-          v.unpack(f);
-        } else {
-#pragma unroll
-          for (int i = 0; i < V; ++i) f[i] = 0.f;
+          v.raw = ch + j < p1 ? dyr[j] : make_uint4(0, 0, 0, 0);
+          v.unpack(*reinterpret_cast<float(*)[V]>(dp + j * V));
         }
 #pragma unroll
-        for (int i = 0; i < V; ++i) dya[j * V + i] = f[i];
+        for (int i = 0; i < V + KH; ++i) {
+          float pre = bias;
+#pragma unroll
+          for (int m = 0; m < KM; ++m)
+            if (m < K) pre = fmaf(wr[m], xa[NB * V + i - m], pre);
+          if (a.silu) dp[i] *= sizeof(T) == 2 ? silu_grad_half_io(pre) : silu_grad_fast(pre);
+        }
+        float out[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          float acc = 0.f;
+#pragma unroll
+          for (int m = 0; m < KM; ++m)
+            if (m < K) {
+              acc = fmaf(wr[m], dp[i + m], acc);
+              dwr[m] = fmaf(dp[i], xa[NB * V + i - m], dwr[m]);
+            }
+          out[i] = acc;
+          db += dp[i];
+        }
+        Vec16<T> v;
+        v.pack(out);
+        v.store_stream(dx - sh + (int64_t)ch * V);
       }
-      float dp[V + KH];  // dpre[t0 + i]
-#pragma unroll
-      for (int i = 0; i < V + KH; ++i) {
-        float pre = bias;
-#pragma unroll
-        for (int m = 0; m < KM; ++m)
-          if (m < K) pre = fmaf(wr[m], xa[NB * V + i - m], pre);
-        float v = dya[i];
-        if (a.silu) v *= sizeof(T) == 2 ? silu_grad_half_io(pre) : silu_grad_fast(pre);
-        dp[i] = (i < V + K - 1) ? v : 0.f;
-      }
-      float out[V];
-#pragma unroll
-      for (int i = 0; i < V; ++i) {
-        float acc = 0.f;
-#pragma unroll
-        for (int m = 0; m < KM; ++m)
-          if (m < K) {
-            acc = fmaf(wr[m], dp[i + m], acc);
-            dwr[m] = fmaf(dp[i], xa[NB * V + i - m], dwr[m]);
-          }
-        out[i] = acc;
-        db += dp[i];
-      }
-      Vec16<T> v;
-      v.pack(out);
-      v.store_stream(dx + t0);
     }
   }
-  constexpr int S = 4;  // scalar path: outputs per thread per pass; x / dy re-reads hit L1
-  for (int t0 = vec ? L : threadIdx.x * S; t0 < L; t0 += kConvThreads * S) {
+  constexpr int S = 4;  // steps outside [lo, hi): outputs per thread per pass; x / dy re-reads hit L1
+  const int head = (lo + S - 1) / S * S;  // the groups before lo, then those from hi on
+  for (int u = ROW == kRowPieces ? L : threadIdx.x * S; u < head + L - hi; u += kConvThreads * S) {
+    const int t0 = u < head ? u : hi + u - head, t1 = u < head ? min(lo, u + S) : L;  // this thread's outputs: t0 .. min(t0 + S, t1)
     float xw[S + 2 * KH];  // xw[q] = x[t0 - KH + q]
 #pragma unroll
     for (int q = 0; q < S + 2 * KH; ++q) {
@@ -217,14 +232,14 @@ __global__ void __launch_bounds__(kConvThreads) conv_cf_bwd_kernel(const ssm_con
         for (int m = 0; m < KM; ++m)
           if (m < K) pre = fmaf(wr[m], xw[i - m + KH], pre);
         v = to_f<T>(dy[t]);
-        if (a.silu) v *= silu_grad_fast(pre);
+        if (a.silu) v *= sizeof(T) == 2 ? silu_grad_half_io(pre) : silu_grad_fast(pre);
       }
       dp[i] = v;
     }
 #pragma unroll
     for (int i = 0; i < S; ++i) {
       const int t = t0 + i;
-      if (t < L) {
+      if (t < t1) {
         float acc = 0.f;
 #pragma unroll
         for (int m = 0; m < KM; ++m)
@@ -345,21 +360,16 @@ __global__ void __launch_bounds__(kConvThreads, 3) conv_cl_fwd_kernel(const ssm_
   T* __restrict__ y = reinterpret_cast<T*>(a.y) + (int64_t)b * L * C + c0;
   // channel pairs as float2 for the packed-fp32 multiply-adds
   float2 wr[KM][V / 2], bias[V / 2];
-  if (K == KM && nvalid == V && (reinterpret_cast<uintptr_t>(a.weight) & 15) == 0 && (!a.bias || (reinterpret_cast<uintptr_t>(a.bias) & 15) == 0)) {
-    // the thread's V x K weights are one contiguous run: 16-byte loads (a scalar load per weight costs a sector request per lane,
+  if (K == KM && nvalid == V && (reinterpret_cast<uintptr_t>(a.weight) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.bias) & 15) == 0) {
+    // the thread's V x K weights are one contiguous run: vector loads (a scalar load per weight costs a sector request per lane,
     // more of them than the whole tile of x)
-    float wf[V * KM];
-    const float4* wp = reinterpret_cast<const float4*>(a.weight + (int64_t)c0 * KM);
+    float wf[V * KM], bf[V];
+    load_param_vec<V * KM>(a.weight, (int64_t)c0 * KM, a.param_dtype, wf);
+    if (a.bias) {
+      load_param_vec<V>(a.bias, c0, a.param_dtype, bf);
+    } else {
 #pragma unroll
-    for (int q = 0; q < V * KM / 4; ++q) {
-      const float4 w4 = __ldg(wp + q);
-      wf[4 * q] = w4.x, wf[4 * q + 1] = w4.y, wf[4 * q + 2] = w4.z, wf[4 * q + 3] = w4.w;
-    }
-    float bf[V];
-#pragma unroll
-    for (int q = 0; q < V / 4; ++q) {
-      const float4 b4 = a.bias ? __ldg(reinterpret_cast<const float4*>(a.bias + c0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-      bf[4 * q] = b4.x, bf[4 * q + 1] = b4.y, bf[4 * q + 2] = b4.z, bf[4 * q + 3] = b4.w;
+      for (int i = 0; i < V; ++i) bf[i] = 0.f;
     }
 #pragma unroll
     for (int i = 0; i < V; i += 2) {
@@ -368,13 +378,13 @@ __global__ void __launch_bounds__(kConvThreads, 3) conv_cl_fwd_kernel(const ssm_
       for (int m = 0; m < KM; ++m) wr[m][i / 2] = make_float2(wf[i * KM + (KM - 1 - m)], wf[(i + 1) * KM + (KM - 1 - m)]);
     }
   } else {
+    auto wat = [&](int ch, int m) { return load_dyn(a.weight, (int64_t)ch * K + (K - 1 - m), a.param_dtype); };
 #pragma unroll
     for (int i = 0; i < V; i += 2) {
       const int c1 = min(c0 + i, C - 1), c2 = min(c0 + i + 1, C - 1);
-      bias[i / 2] = a.bias ? make_float2(__ldg(a.bias + c1), __ldg(a.bias + c2)) : make_float2(0.f, 0.f);
+      bias[i / 2] = a.bias ? make_float2(load_dyn(a.bias, c1, a.param_dtype), load_dyn(a.bias, c2, a.param_dtype)) : make_float2(0.f, 0.f);
 #pragma unroll
-      for (int m = 0; m < KM; ++m)
-        wr[m][i / 2] = m < K ? make_float2(__ldg(a.weight + (int64_t)c1 * K + (K - 1 - m)), __ldg(a.weight + (int64_t)c2 * K + (K - 1 - m))) : make_float2(0.f, 0.f);
+      for (int m = 0; m < KM; ++m) wr[m][i / 2] = m < K ? make_float2(wat(c1, m), wat(c2, m)) : make_float2(0.f, 0.f);
     }
   }
   float2 hist[KH > 0 ? KH : 1][V / 2];  // hist[m] = x[t - 1 - m]
@@ -490,31 +500,14 @@ __global__ void __launch_bounds__(kConvThreads) conv_cl_bwd_kernel(const ssm_con
   const T* __restrict__ dy = reinterpret_cast<const T*>(g.dy) + (int64_t)b * L * C + c0;
   T* __restrict__ dx = reinterpret_cast<T*>(g.dx) + (int64_t)b * L * C + c0;
   float w[KM][V], wr[KM][V], bias[V];  // w[q] = weight[c][q];  wr[m] = weight[c][K-1-m]
-  if (K == KM && nvalid == V && (reinterpret_cast<uintptr_t>(a.weight) & 15) == 0 && (!a.bias || (reinterpret_cast<uintptr_t>(a.bias) & 15) == 0)) {
-    // the thread's V x K weights are one contiguous run: 16-byte loads instead of a sector request per lane and weight
-    float wf[V * KM];
-    const float4* wp = reinterpret_cast<const float4*>(a.weight + (int64_t)c0 * KM);
 #pragma unroll
-    for (int q = 0; q < V * KM / 4; ++q) {
-      const float4 w4 = __ldg(wp + q);
-      wf[4 * q] = w4.x, wf[4 * q + 1] = w4.y, wf[4 * q + 2] = w4.z, wf[4 * q + 3] = w4.w;
-    }
-    const float4 b4 = a.bias ? __ldg(reinterpret_cast<const float4*>(a.bias + c0)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    bias[0] = b4.x, bias[1] = b4.y, bias[2] = b4.z, bias[3] = b4.w;
+  for (int i = 0; i < V; ++i) {
+    const int cc = min(c0 + i, C - 1);
+    bias[i] = a.bias ? load_dyn(a.bias, cc, a.param_dtype) : 0.f;
 #pragma unroll
-    for (int i = 0; i < V; ++i)
-#pragma unroll
-      for (int q = 0; q < KM; ++q) w[q][i] = wf[i * KM + q], wr[q][i] = wf[i * KM + (KM - 1 - q)];
-  } else {
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const int cc = min(c0 + i, C - 1);
-      bias[i] = a.bias ? __ldg(a.bias + cc) : 0.f;
-#pragma unroll
-      for (int q = 0; q < KM; ++q) {
-        w[q][i] = q < K ? __ldg(a.weight + (int64_t)cc * K + q) : 0.f;
-        wr[q][i] = q < K ? __ldg(a.weight + (int64_t)cc * K + (K - 1 - q)) : 0.f;
-      }
+    for (int q = 0; q < KM; ++q) {
+      w[q][i] = q < K ? load_dyn(a.weight, (int64_t)cc * K + q, a.param_dtype) : 0.f;
+      wr[q][i] = q < K ? load_dyn(a.weight, (int64_t)cc * K + (K - 1 - q), a.param_dtype) : 0.f;
     }
   }
   float dwr[KM][V], db[V];
@@ -621,6 +614,158 @@ __global__ void __launch_bounds__(kConvThreads) conv_cl_bwd_kernel(const ssm_con
   }
 }
 
+// SiLU gradient of a pair of pre-activations
+template <bool HALF>
+__device__ __forceinline__ float2 silu_grad2(float2 p) {
+  float2 s;
+  if constexpr (HALF) {  // sigmoid(x) = 0.5 + 0.5 tanh(x / 2), one special-function instruction (see silu_grad_half_io)
+    const float2 h = __fmul2_rn(p, make_float2(0.5f, 0.5f));
+    float2 t;
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t.x) : "f"(h.x));
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t.y) : "f"(h.y));
+    s = __ffma2_rn(t, make_float2(0.5f, 0.5f), make_float2(0.5f, 0.5f));
+  } else {
+    s = make_float2(sigmoid_fast(p.x), sigmoid_fast(p.y));
+  }
+  const float2 r = __ffma2_rn(s, make_float2(-1.f, -1.f), make_float2(1.f, 1.f));
+  return __ffma2_rn(__fmul2_rn(p, s), r, s);
+}
+
+// The same walk for the width that state-space models use (4) and channels in whole groups of four: taps, windows and
+// accumulators are pairs of channels for the packed-fp32 instructions, the taps exist once, and the eight steps of a batch of loads run
+// without any check unless they touch an end of the tile.  Bound by instructions (about 13 per element; the kernel above
+// takes 31), hence four CTAs per SM and a tile length that fills whole waves (conv_cl_tile).
+// (4, 4093, 2560) bf16, 251 MB: 154 us with the kernel above, 76 us with this one (3.3 TB/s; two channels per thread and six CTAs
+// more per SM: 91).  Narrow tensors, NT = 512: (2, 16384, 128) bf16 72 -> 18 us.
+template <typename T, int V, int NT>
+__global__ void __launch_bounds__(NT, V == 4 ? 512 / NT : 768 / NT) conv_cl_bwd4_kernel(const ssm_conv_bwd_args g, int tile) {
+  const ssm_conv_args& a = g.fwd;
+  constexpr int U = 32 / (V * (int)sizeof(T) / 2);  // steps per batch of loads: 64 bytes of x and of dy a thread
+  constexpr int P = V / 2;
+  using Raw = typename std::conditional<V * sizeof(T) == 16, uint4, typename std::conditional<V * sizeof(T) == 8, uint2, uint32_t>::type>::type;
+  const int C = a.channels, L = a.len, nvec = C / V;
+  const int64_t item = (int64_t)blockIdx.x * NT + threadIdx.x;  // channel groups fastest, then time tiles
+  const int c0 = (int)(item % nvec) * V;
+  const int64_t ts64 = item / nvec * tile;
+  const bool live = ts64 < L;
+  const int ts = live ? (int)ts64 : 0, te = live ? min(L, ts + tile) : -3, b = blockIdx.z;
+  const T* __restrict__ x = reinterpret_cast<const T*>(a.x) + (int64_t)b * L * C + c0;
+  const T* __restrict__ dy = reinterpret_cast<const T*>(g.dy) + (int64_t)b * L * C + c0;
+  T* __restrict__ dx = reinterpret_cast<T*>(g.dx) + (int64_t)b * L * C + c0;
+  float2 w[4][P], bias[P], dw[4][P], db[P];  // w[m], dw[m]: the tap of x[t - m]
+  {
+    float wf[V * 4], bf[V];
+    load_param_vec<V * 4>(a.weight, (int64_t)c0 * 4, a.param_dtype, wf);
+#pragma unroll
+    for (int i = 0; i < V; ++i) bf[i] = a.bias ? load_dyn(a.bias, c0 + i, a.param_dtype) : 0.f;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      bias[p] = make_float2(bf[2 * p], bf[2 * p + 1]), db[p] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) w[m][p] = make_float2(wf[8 * p + 3 - m], wf[8 * p + 7 - m]), dw[m][p] = make_float2(0.f, 0.f);
+    }
+  }
+  float2 xh[3][P], dh[3][P];  // x[s - 1 - m], dpre[s - 1 - m]
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const int t = ts - 1 - m;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      float f[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        f[q] = 0.f;
+        if (t >= 0) f[q] = to_f<T>(x[(int64_t)t * C + 2 * p + q]);
+        else if (a.halo) f[q] = __ldg(a.halo + ((int64_t)b * C + c0 + 2 * p + q) * 3 + 3 + t);
+      }
+      xh[m][p] = make_float2(f[0], f[1]), dh[m][p] = make_float2(0.f, 0.f);
+    }
+  }
+  auto step = [&](auto inner, int s, const Raw& xr, const Raw& gr) {
+    constexpr bool kInner = decltype(inner)::value;
+    float xf[V], gf[V];
+    const T *ex = reinterpret_cast<const T*>(&xr), *eg = reinterpret_cast<const T*>(&gr);
+#pragma unroll
+    for (int i = 0; i < V; ++i) xf[i] = kInner || s < L ? to_f<T>(ex[i]) : 0.f, gf[i] = kInner || s < L ? to_f<T>(eg[i]) : 0.f;
+    Raw ow;
+    T* out = reinterpret_cast<T*>(&ow);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const float2 cur = make_float2(xf[2 * p], xf[2 * p + 1]);
+      float2 pre = __ffma2_rn(w[0][p], cur, bias[p]);
+#pragma unroll
+      for (int m = 1; m < 4; ++m) pre = __ffma2_rn(w[m][p], xh[m - 1][p], pre);
+      float2 dp = make_float2(gf[2 * p], gf[2 * p + 1]);
+      if (a.silu) dp = __fmul2_rn(dp, silu_grad2<sizeof(T) == 2>(pre));
+      if (kInner || s < te) {  // each position's parameter gradient is counted by the tile that owns it
+        db[p] = __fadd2_rn(db[p], dp);
+        dw[0][p] = __ffma2_rn(dp, cur, dw[0][p]);
+#pragma unroll
+        for (int m = 1; m < 4; ++m) dw[m][p] = __ffma2_rn(dp, xh[m - 1][p], dw[m][p]);
+      }
+      // dx[s - 3] = w[3] dpre[s] + w[2] dpre[s - 1] + w[1] dpre[s - 2] + w[0] dpre[s - 3]
+      float2 o = __fmul2_rn(w[3][p], dp);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) o = __ffma2_rn(w[2 - m][p], dh[m][p], o);
+      out[2 * p] = from_f<T>(o.x), out[2 * p + 1] = from_f<T>(o.y);
+      xh[2][p] = xh[1][p], xh[1][p] = xh[0][p], xh[0][p] = cur;
+      dh[2][p] = dh[1][p], dh[1][p] = dh[0][p], dh[0][p] = dp;
+    }
+    if (kInner || (s - 3 >= ts && s - 3 < te)) __stcs(reinterpret_cast<Raw*>(dx + (int64_t)(s - 3) * C), ow);
+  };
+  for (int s0 = ts; s0 < te + 3; s0 += U) {
+    Raw xr[U], gr[U];
+    if (s0 >= ts + 3 && s0 + U <= te) {
+      const T *px = x + (int64_t)s0 * C, *pg = dy + (int64_t)s0 * C;
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        xr[j] = __ldcs(reinterpret_cast<const Raw*>(px)), gr[j] = __ldcs(reinterpret_cast<const Raw*>(pg));
+        px += C, pg += C;
+      }
+#pragma unroll
+      for (int j = 0; j < U; ++j) step(std::true_type{}, s0 + j, xr[j], gr[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        const int sc = min(s0 + j, L - 1);  // beyond the sequence: its last row, dropped
+        xr[j] = __ldcs(reinterpret_cast<const Raw*>(x + (int64_t)sc * C));
+        gr[j] = __ldcs(reinterpret_cast<const Raw*>(dy + (int64_t)sc * C));
+      }
+#pragma unroll
+      for (int j = 0; j < U; ++j) step(std::false_type{}, s0 + j, xr[j], gr[j]);
+    }
+  }
+  auto comp = [](const float2 (&v)[P], int i) { return i & 1 ? v[i / 2].y : v[i / 2].x; };
+  // Narrow tensors: the threads of a CTA that share channels meet in shared memory, one global addition per CTA and gradient (an
+  // addition to a word that many CTAs want takes about 40 ns).
+  __shared__ float sums[NT > 128 ? NT * 5 : 1];
+  if constexpr (NT > 128) {
+    for (int i = threadIdx.x; i < C * 5; i += NT) sums[i] = 0.f;
+    __syncthreads();
+    if (live) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        atomicAdd(sums + (c0 + i) * 5 + 4, comp(db, i));
+#pragma unroll
+        for (int m = 0; m < 4; ++m) atomicAdd(sums + (c0 + i) * 5 + 3 - m, comp(dw[m], i));
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < C * 5; i += NT) {
+      const int c = i / 5, q = i % 5;
+      if (q < 4) atomicAdd(g.dweight + c * 4 + q, sums[i]);
+      else if (g.dbias) atomicAdd(g.dbias + c, sums[i]);
+    }
+  } else if (live) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      if (g.dbias) atomicAdd(g.dbias + c0 + i, comp(db, i));
+#pragma unroll
+      for (int m = 0; m < 4; ++m) atomicAdd(g.dweight + (int64_t)(c0 + i) * 4 + (3 - m), comp(dw[m], i));
+    }
+  }
+}
+
 // decode-time update: one thread per (batch, channel)
 template <typename T>
 __global__ void __launch_bounds__(256) conv_update_kernel(const ssm_conv_update_args a) {
@@ -651,7 +796,7 @@ static int conv_validate(const ssm_conv_args* a) {
   SSM_REQUIRE(a != nullptr, SSM_ERR_NULL, "dw_causal_conv: args is NULL");
   SSM_REQUIRE(a->batch >= 0 && a->channels >= 0 && a->len >= 0, SSM_ERR_SHAPE, "dw_causal_conv: negative size");
   SSM_REQUIRE(a->width >= 1 && a->width <= kConvMaxK, SSM_ERR_UNSUPPORTED, "dw_causal_conv: kernel width must be in [1, 8]");
-  SSM_REQUIRE(valid_dtype(a->io_dtype), SSM_ERR_DTYPE, "dw_causal_conv: unknown dtype");
+  SSM_REQUIRE(valid_dtype(a->io_dtype) && valid_dtype(a->param_dtype), SSM_ERR_DTYPE, "dw_causal_conv: unknown dtype");
   SSM_REQUIRE(a->batch <= 65535, SSM_ERR_TOO_LARGE, "dw_causal_conv: batch exceeds 65535");
   SSM_REQUIRE(!a->channels_first || (a->row_sb >= 0 && a->row_sc >= a->len), SSM_ERR_SHAPE, "dw_causal_conv: bad row strides");
   SSM_REQUIRE((int64_t)a->batch * a->channels < (1ll << 31), SSM_ERR_TOO_LARGE, "dw_causal_conv: batch*channels too large");
@@ -662,29 +807,42 @@ static dim3 conv_cl_grid(const ssm_conv_args& a, int V) {
   return dim3(((a.channels + V - 1) / V + kConvThreads - 1) / kConvThreads, (a.len + kConvTimeTile - 1) / kConvTimeTile, a.batch);
 }
 
-// Steps per thread of the channels-last forward: the full tile when that still gives the GPU eight or more waves of CTAs
-// (a ragged last wave then costs little), shorter walks otherwise, down to 8 steps (every walk re-reads K - 1 earlier inputs).
-static int64_t conv_cl_fwd_ctas(const ssm_conv_args& a, int V, int tile) {
+// Steps per thread of a channels-last walk: the tile length with the least (waves of resident CTAs) x (steps per CTA), where a
+// walk costs about `extra` steps more than its tile (the window and weight loads of its start, the sums at its end).
+static int64_t conv_cl_ctas(const ssm_conv_args& a, int V, int threads, int tile) {
   const int64_t items = (int64_t)((a.channels + V - 1) / V) * ((a.len + tile - 1) / tile);
-  return (items + kConvThreads - 1) / kConvThreads;
+  return (items + threads - 1) / threads;
 }
-static int conv_cl_fwd_tile(const ssm_conv_args& a, int V) {
-  int tile = kConvTimeTile;
-  while (tile > 8 && conv_cl_fwd_ctas(a, V, tile) * a.batch < 4 * 3 * 148) tile >>= 1;  // four waves of three CTAs per SM
-  while (conv_cl_fwd_ctas(a, V, tile) >= (1ll << 31)) tile <<= 1;
-  return tile;
+static int conv_cl_tile(const ssm_conv_args& a, int V, int threads, int ctas_per_sm, int extra, int longest) {
+  const int64_t slots = (int64_t)sm_count() * ctas_per_sm;
+  int best = 8;
+  double cost = 1e300;
+  for (int tile = 8; tile <= longest; tile += 8) {
+    const int64_t n = conv_cl_ctas(a, V, threads, tile) * a.batch;
+    if (n >= (1ll << 31)) continue;
+    // a last wave costs what it holds, but no less than half a wave: its CTAs run alone and cannot hide their latencies
+    const double waves = (double)(n / slots) + (n % slots ? fmax(0.5, (double)(n % slots) / slots) : 0.0);
+    const double c = fmax(1.0, waves) * (tile + extra);
+    if (c < cost) cost = c, best = tile;
+  }
+  return best;
 }
+
+// every row a whole number of 16-byte pieces, starting on a boundary
+static bool conv_rows_whole(const ssm_conv_args& a, int V) { return a.len % V == 0 && a.row_sb % V == 0 && a.row_sc % V == 0; }
 
 template <typename T, int KM>
 static int conv_fwd_launch(const ssm_conv_args& a, cudaStream_t st) {
   constexpr int V = 16 / sizeof(T);
   if (a.channels_first) {
-    const int vec = (a.len % V == 0) && (a.row_sb % V == 0) && (a.row_sc % V == 0) && aligned_to(a.x, 16) && aligned_to(a.y, 16);
-    conv_cf_fwd_kernel<T, KM><<<(unsigned)((int64_t)a.batch * a.channels), kConvThreads, 0, st>>>(a, vec);
+    const unsigned grid = (unsigned)((int64_t)a.batch * a.channels);
+    if (!(aligned_to(a.x, 16) && aligned_to(a.y, 16))) conv_cf_fwd_kernel<T, KM, kRowScalar><<<grid, kConvThreads, 0, st>>>(a);
+    else if (conv_rows_whole(a, V)) conv_cf_fwd_kernel<T, KM, kRowPieces><<<grid, kConvThreads, 0, st>>>(a);
+    else conv_cf_fwd_kernel<T, KM, kRowRagged><<<grid, kConvThreads, 0, st>>>(a);
   } else {
     const int vec = (a.channels % V == 0) && aligned_to(a.x, 16) && aligned_to(a.y, 16);
-    const int tile = conv_cl_fwd_tile(a, V);
-    conv_cl_fwd_kernel<T, KM><<<dim3((unsigned)conv_cl_fwd_ctas(a, V, tile), 1, a.batch), kConvThreads, 0, st>>>(a, vec, tile);
+    const int tile = conv_cl_tile(a, V, kConvThreads, 3, 12, 128);
+    conv_cl_fwd_kernel<T, KM><<<dim3((unsigned)conv_cl_ctas(a, V, kConvThreads, tile), 1, a.batch), kConvThreads, 0, st>>>(a, vec, tile);
   }
   return launch_status("dw_causal_conv_fwd");
 }
@@ -693,15 +851,28 @@ template <typename T, int KM>
 static int conv_bwd_launch(const ssm_conv_bwd_args& g, cudaStream_t st) {
   const ssm_conv_args& a = g.fwd;
   if (a.channels_first) {
-    constexpr int VT = 16 / sizeof(T);
-    const int vec = (a.len % VT == 0) && (a.row_sb % VT == 0) && (a.row_sc % VT == 0) && aligned_to(a.x, 16) && aligned_to(g.dy, 16) &&
-                    aligned_to(g.dx, 16);
-    conv_cf_bwd_kernel<T, KM><<<(unsigned)((int64_t)a.batch * a.channels), kConvThreads, 0, st>>>(g, vec);
+    const unsigned grid = (unsigned)((int64_t)a.batch * a.channels);
+    if (!(aligned_to(a.x, 16) && aligned_to(g.dy, 16) && aligned_to(g.dx, 16))) conv_cf_bwd_kernel<T, KM, kRowScalar><<<grid, kConvThreads, 0, st>>>(g);
+    else if (conv_rows_whole(a, 16 / sizeof(T))) conv_cf_bwd_kernel<T, KM, kRowPieces><<<grid, kConvThreads, 0, st>>>(g);
+    else conv_cf_bwd_kernel<T, KM, kRowRagged><<<grid, kConvThreads, 0, st>>>(g);
   } else {
     constexpr int V = 4;
     const size_t gb = V * sizeof(T);
     const int vec = (a.channels % V == 0) && aligned_to(a.x, gb) && aligned_to(g.dy, gb) && aligned_to(g.dx, gb);
-    conv_cl_bwd_kernel<T, KM><<<conv_cl_grid(a, V), kConvThreads, 0, st>>>(g, vec);
+    if (a.width == 4 && vec && aligned_to(a.weight, 16) && aligned_to(a.bias, 16)) {
+      constexpr int VB = 8 / sizeof(T), kPerSm = VB == 4 ? 512 : 768;  // channels and resident threads per SM
+      // up to 512 channels: CTAs of 512 threads, each holding all channels at several time tiles
+      constexpr int kWide = 512;
+      if (a.channels <= kWide) {
+        const int tile = conv_cl_tile(a, VB, kWide, kPerSm / kWide, 16, 256);
+        conv_cl_bwd4_kernel<T, VB, kWide><<<dim3((unsigned)conv_cl_ctas(a, VB, kWide, tile), 1, a.batch), kWide, 0, st>>>(g, tile);
+      } else {
+        const int tile = conv_cl_tile(a, VB, kConvThreads, kPerSm / kConvThreads, 16, 256);
+        conv_cl_bwd4_kernel<T, VB, kConvThreads><<<dim3((unsigned)conv_cl_ctas(a, VB, kConvThreads, tile), 1, a.batch), kConvThreads, 0, st>>>(g, tile);
+      }
+    } else {
+      conv_cl_bwd_kernel<T, KM><<<conv_cl_grid(a, V), kConvThreads, 0, st>>>(g, vec);
+    }
   }
   return launch_status("dw_causal_conv_bwd");
 }

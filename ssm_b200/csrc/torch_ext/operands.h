@@ -397,7 +397,13 @@ struct ConvCtx {
     same_device(x_, {&weight});
     need_cuda(x_, {&bias, &halo_});
     dtype_code(x_, "dw_causal_conv");
-    x = first && keep_rows ? rows(x_) : x_.detach().contiguous(), w = f32c(w2), b = f32c(bias);
+    x = first && keep_rows ? rows(x_) : x_.detach().contiguous();
+    if (io_dtype_ok(w2) && (!bias.has_value() || bias->scalar_type() == w2.scalar_type())) {  // as they are
+      w = w2.detach().contiguous();
+      if (bias.has_value()) b = bias->detach().contiguous();
+    } else {
+      w = f32c(w2), b = f32c(bias);
+    }
     nb = x_.size(0), nl = first ? x_.size(2) : x_.size(1);
     if (halo_.has_value())
       SSM_ARG(halo_->dim() == 3 && halo_->size(0) == nb && halo_->size(1) == nc && halo_->size(2) == k - 1, "halo must have shape (B, C, K-1).");
@@ -406,7 +412,8 @@ struct ConvCtx {
   void fill(ssm_conv_args& a) const {
     a.batch = (int)nb, a.channels = (int)nc, a.len = (int)nl, a.width = (int)k;
     a.io_dtype = dtype_code(x, "dw_causal_conv"), a.channels_first = first, a.silu = silu;
-    a.x = x.data_ptr(), a.weight = w.data_ptr<float>(), a.bias = fptr(b), a.halo = fptr(halo);
+    a.x = x.data_ptr(), a.weight = w.data_ptr(), a.bias = ptr(b), a.halo = fptr(halo);
+    a.param_dtype = dtype_code(w, "dw_causal_conv");
     const bool own = first && x.numel() > 0;
     a.row_sb = own ? x.stride(0) : nc * nl, a.row_sc = own ? x.stride(1) : nl;
   }

@@ -75,11 +75,20 @@ Tensor cast(const Tensor& grad, at::ScalarType t) { return grad.scalar_type() ==
 struct ZeroPool {
   std::vector<std::pair<Tensor*, std::vector<int64_t>>> want;
   int64_t total = 0;
+  Tensor all;
   void add(Tensor& t, at::IntArrayRef shape) { want.emplace_back(&t, shape.vec()), total += padded(shape); }
   static int64_t padded(at::IntArrayRef shape) { return (c10::multiply_integers(shape) + 63) / 64 * 64; }
   void make(const at::TensorOptions& f32) {
     if (want.empty()) return;
-    Tensor all = at::zeros({total}, f32);
+    all = at::zeros({total}, f32);
+    share();
+  }
+  // all of them in another type, by one conversion
+  void cast_all(at::ScalarType type) {
+    all = all.to(type);
+    share();
+  }
+  void share() {
     int64_t at = 0;
     for (auto& [t, shape] : want) {
       *t = all.narrow(0, at, c10::multiply_integers(shape)).view(shape);
@@ -342,6 +351,7 @@ struct ConvCall final : Call {
     c.fill(g.fwd);
     g.dy = go.data_ptr(), g.dx = dx.data_ptr(), g.dweight = out_ptr(dw), g.dbias = out_ptr(db);
     run(ssm_dw_causal_conv_bwd(&g, stream_of(c.x)));
+    if (t_w != at::kFloat && (!c.b.has_value() || t_b == t_w)) pool.cast_all(t_w);
     variable_list res = {dx, cast(dw.view(shape_w), t_w)};
     if (c.b.has_value()) res.push_back(cast(db, t_b));
     return res;

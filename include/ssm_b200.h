@@ -231,19 +231,24 @@ int ssm_chunk_scan_fwd(const ssm_chunk_args* args, ssm_stream_t stream);
  * accumulated into (caller zero-fills).  history: scratch (batch, len, heads, proj) fp32.
  * fwd.typed_grads, bits 0 / 1 / 2: dB / dC / dz is instead a buffer of par_dtype elements with no broadcast axis (every
  * (b, t, h, q) a distinct element) that the call WRITES, every element of it, zeros beyond a row's length included: no zero-fill
- * by the caller, no fp32 copy to convert afterwards. */
+ * by the caller, no fp32 copy to convert afterwards.
+ * ssm_chunk_scan_bwd_fused(args) tells whether a call with these arguments (typed_grads bits 0 - 2, layouts, pointers of the
+ * gradients of B, C, z) keeps its states in registers: it then needs no history, and bit 3 may be set. */
 typedef struct {
   ssm_chunk_args fwd;
   const void* dY;
   void* dX;
-  float* ddt;
+  void* ddt; /* fp32, accumulated into; with bit 3 of typed_grads io_dtype, written */
   ssm_bcast4 dA, dB, dC, dD, dz, dinitial; /* ptr as float*; NULL to skip where fwd's is NULL */
   float* history;
   float* scratch; /* nullable: ssm_chunk_scan_bwd_scratch_floats() floats; with it the chunks run in parallel, without it one thread
                      per (batch, head, proj) walks the whole sequence */
+  float* fwd_scratch; /* nullable: the scratch that the forward call with the same arguments left behind */
+  float* scratch_fwd; /* set inside the call */
 } ssm_chunk_bwd_args;
 
 int64_t ssm_chunk_scan_bwd_scratch_floats(int32_t batch, int32_t len, int32_t heads, int32_t proj, int32_t chunk_size);
+int ssm_chunk_scan_bwd_fused(const ssm_chunk_bwd_args* args);
 int ssm_chunk_scan_bwd(const ssm_chunk_bwd_args* args, ssm_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------

@@ -9,11 +9,13 @@
 //   forward   (1) every chunk integrates from a zero state and records its decay product,
 //             (2) a short serial pass over chunks turns those into each chunk's incoming state,
 //             (3) every chunk is replayed from its true incoming state and writes Y;
-//   backward  the same three phases give every chunk its incoming state, their mirror image
-//             gives every chunk the adjoint that enters it from the right
+//   backward  the incoming states come from the forward call (or the same three phases), their
+//             mirror image gives every chunk the adjoint that enters it from the right
 //             (g_t = C_t dy_t + exp(dt_{t+1} A) g_{t+1} is a linear recurrence too), and one
-//             final pass per chunk replays the states into the history scratch and walks back
-//             through them producing every gradient.
+//             final pass per chunk replays the states and walks back through them producing every
+//             gradient.
+// The usual layouts run on lanes of four projections (chunk_scan_vec.cuh); the kernels of this
+// file take any broadcast.
 // Every thread keeps raw pointers that advance by one time stride per step, and the loads of
 // eight steps are issued before the first of them is used, so that enough bytes are in flight.
 // Without scratch memory a single serial pass is used instead.
@@ -57,7 +59,11 @@ __device__ __forceinline__ Stream<PT> par_stream(const ssm_bcast4& c, int b, int
   return {reinterpret_cast<const PT*>(c.ptr) + bc4_off(c, b, t, h, q), c.st};
 }
 
-// per-lane context shared by all kernels
+}  // namespace ssmb
+#include "chunk_scan_vec.cuh"
+namespace ssmb {
+
+// per-lane context shared by all scalar kernels
 template <typename T>
 struct Lane {
   int b, h, q, hp, HP, valid;
@@ -148,118 +154,6 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_fwd_kernel(const ssm_chun
   for (; k < n; ++k) Y[(int64_t)k * ln.HP] = from_f<T>(step(sx.at(k), sdt.at(k), sB.at(k), sC.at(k), has_z ? sz.at(k) : 0.f));
   for (int t = te; t < t1; ++t) Y[(int64_t)(t - t0) * ln.HP] = from_f<T>(0.f);
   if (MODE == 0 && a.final_state) a.final_state[(int64_t)ln.b * ln.HP + ln.hp] = s;
-}
-
-// 16-bit rows with the projection axis contiguous and a multiple of 8: a thread takes 8 neighbouring lanes of one head, so every
-// load and store is 16 bytes (a scalar lane moves 2 bytes per instruction and the kernels above are bound by instruction issue,
-// not by bytes), and the loads of kVecUnroll steps go out before the first is used.  MODE 1: local state and decay product of a
-// chunk.  MODE 3: the chunk replayed from its incoming state, Y written.
-constexpr int kVecUnroll = 4;
-template <typename T, int MODE>
-__global__ void __launch_bounds__(kChunkThreads) chunk_fwd_vec_kernel(const ssm_chunk_args a, int nchunks, int chunk_len) {
-  constexpr int V = 8;
-  const int HP = a.heads * a.proj;
-  const int hp = (blockIdx.x * kChunkThreads + threadIdx.x) * V;
-  if (hp >= HP) return;
-  const int h = hp / a.proj, q = hp % a.proj;
-  const int b = blockIdx.z, c = blockIdx.y;
-  const int valid = chunk_valid_len(a, b);
-  const int t0 = c * chunk_len, t1 = min(a.len, t0 + chunk_len);
-  const int n = max(t0, min(t1, valid)) - t0;
-  float Av[V], Dv[V];
-#pragma unroll
-  for (int e = 0; e < V; ++e) {
-    Av[e] = bc4_load_f32(a.A, 0, 0, h, q + e) * kLog2e;
-    Dv[e] = (MODE == 3 && a.D.ptr) ? bc4_load_f32(a.D, 0, 0, h, q + e) : 0.f;
-  }
-  float* P = a.scratch;                                            // [batch][nchunks][HP] decay products
-  float* S = a.scratch + (int64_t)a.batch * nchunks * HP;          // local end state, then incoming state
-  const int64_t slot = ((int64_t)b * nchunks + c) * HP + hp;
-  const T* px = reinterpret_cast<const T*>(a.X) + ((int64_t)b * a.len + t0) * HP + hp;
-  const T* pdt = reinterpret_cast<const T*>(a.dt) + ((int64_t)b * a.len + t0) * a.heads + h;
-  const T* pB = reinterpret_cast<const T*>(a.Bm.ptr) + bc4_off(a.Bm, b, t0, h, q);
-  auto unpack8 = [](const uint4& r, float (&f)[V]) {
-    Vec16<T> v;
-    v.raw = r;
-    v.unpack(f);
-  };
-  float s[V];
-  if (MODE == 1) {
-#pragma unroll
-    for (int e = 0; e < V; ++e) s[e] = 0.f;
-    float sumdt = 0.f;
-    for (int k = 0; k < n; k += kVecUnroll) {
-      uint4 xr[kVecUnroll], br[kVecUnroll];
-      float d[kVecUnroll];
-#pragma unroll
-      for (int i = 0; i < kVecUnroll; ++i) {
-        const int kk = min(k + i, n - 1);  // beyond the chunk: a valid address, dropped below
-        xr[i] = __ldg(reinterpret_cast<const uint4*>(px + (int64_t)kk * HP));
-        br[i] = __ldg(reinterpret_cast<const uint4*>(pB + (int64_t)kk * a.Bm.st));
-        d[i] = to_f<T>(__ldg(pdt + (int64_t)kk * a.heads));
-      }
-#pragma unroll
-      for (int i = 0; i < kVecUnroll; ++i) {
-        if (k + i < n) {
-          float x[V], bv[V];
-          unpack8(xr[i], x);
-          unpack8(br[i], bv);
-#pragma unroll
-          for (int e = 0; e < V; ++e) s[e] = fmaf(ex2_approx(d[i] * Av[e]), s[e], d[i] * bv[e] * x[e]);
-          sumdt += d[i];
-        }
-      }
-    }
-    float pr[V];
-#pragma unroll
-    for (int e = 0; e < V; ++e) pr[e] = ex2_approx(sumdt * Av[e]);
-    reinterpret_cast<float4*>(P + slot)[0] = make_float4(pr[0], pr[1], pr[2], pr[3]);
-    reinterpret_cast<float4*>(P + slot)[1] = make_float4(pr[4], pr[5], pr[6], pr[7]);
-    reinterpret_cast<float4*>(S + slot)[0] = make_float4(s[0], s[1], s[2], s[3]);
-    reinterpret_cast<float4*>(S + slot)[1] = make_float4(s[4], s[5], s[6], s[7]);
-    return;
-  }
-  const T* pC = reinterpret_cast<const T*>(a.Cm.ptr) + bc4_off(a.Cm, b, t0, h, q);
-  const bool has_z = a.z.ptr != nullptr;
-  const T* pz = has_z ? reinterpret_cast<const T*>(a.z.ptr) + bc4_off(a.z, b, t0, h, q) : nullptr;
-  T* Y = reinterpret_cast<T*>(a.Y) + ((int64_t)b * a.len + t0) * HP + hp;
-  {
-    const float4 s0 = reinterpret_cast<const float4*>(S + slot)[0], s1 = reinterpret_cast<const float4*>(S + slot)[1];
-    s[0] = s0.x, s[1] = s0.y, s[2] = s0.z, s[3] = s0.w, s[4] = s1.x, s[5] = s1.y, s[6] = s1.z, s[7] = s1.w;
-  }
-  for (int k = 0; k < n; k += kVecUnroll) {
-    uint4 xr[kVecUnroll], br[kVecUnroll], cr[kVecUnroll], zr[kVecUnroll];
-    float d[kVecUnroll];
-#pragma unroll
-    for (int i = 0; i < kVecUnroll; ++i) {
-      const int kk = min(k + i, n - 1);
-      xr[i] = __ldg(reinterpret_cast<const uint4*>(px + (int64_t)kk * HP));
-      br[i] = __ldg(reinterpret_cast<const uint4*>(pB + (int64_t)kk * a.Bm.st));
-      cr[i] = __ldg(reinterpret_cast<const uint4*>(pC + (int64_t)kk * a.Cm.st));
-      zr[i] = has_z ? __ldg(reinterpret_cast<const uint4*>(pz + (int64_t)kk * a.z.st)) : make_uint4(0, 0, 0, 0);
-      d[i] = to_f<T>(__ldg(pdt + (int64_t)kk * a.heads));
-    }
-#pragma unroll
-    for (int i = 0; i < kVecUnroll; ++i) {
-      if (k + i < n) {
-        float x[V], bv[V], cv[V], zv[V], y[V];
-        unpack8(xr[i], x);
-        unpack8(br[i], bv);
-        unpack8(cr[i], cv);
-        unpack8(zr[i], zv);
-#pragma unroll
-        for (int e = 0; e < V; ++e) {
-          s[e] = fmaf(ex2_approx(d[i] * Av[e]), s[e], d[i] * bv[e] * x[e]);
-          y[e] = fmaf(Dv[e], x[e], s[e] * cv[e]);
-          if (has_z) y[e] *= silu_fast(zv[e]);
-        }
-        Vec16<T> o;
-        o.pack(y);
-        *reinterpret_cast<uint4*>(Y + (int64_t)(k + i) * HP) = o.raw;
-      }
-    }
-  }
-  for (int t = t0 + n; t < t1; ++t) *reinterpret_cast<uint4*>(Y + (int64_t)(t - t0) * HP) = make_uint4(0, 0, 0, 0);
 }
 
 // The carry over the pieces: v_{c+1} = P[c] v_c + L[c], and L[c] is replaced by v_c (what enters piece c).  One lane per hp,
@@ -367,54 +261,6 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_local_kernel(const ss
   R[slot] = carry;
 }
 
-// the same on 16-byte lanes (8 neighbouring projections of one head per thread; 16-bit per-token C / z, see chunk_vec_ok)
-template <typename T>
-__global__ void __launch_bounds__(kChunkThreads) chunk_bwd_local_vec_kernel(const ssm_chunk_bwd_args g, int nchunks) {
-  constexpr int V = 8, U = 4;
-  const ssm_chunk_args& a = g.fwd;
-  const int HP = a.heads * a.proj;
-  const int hp = (blockIdx.x * kChunkThreads + threadIdx.x) * V;
-  if (hp >= HP) return;
-  const int h = hp / a.proj, q = hp % a.proj;
-  const int b = blockIdx.z, c = blockIdx.y;
-  const int t0 = c * a.chunk_size, t1 = min(a.len, t0 + a.chunk_size);
-  const int n = max(t0, min(t1, chunk_valid_len(a, b))) - t0;
-  float* R = g.scratch + 2 * (int64_t)a.batch * nchunks * HP + ((int64_t)b * nchunks + c) * HP + hp;
-  float Av[V], carry[V];
-#pragma unroll
-  for (int e = 0; e < V; ++e) Av[e] = bc4_load_f32(a.A, 0, 0, h, q + e) * kLog2e, carry[e] = 0.f;
-  const T* pdy = reinterpret_cast<const T*>(g.dY) + ((int64_t)b * a.len + t0) * HP + hp;
-  const T* pdt = reinterpret_cast<const T*>(a.dt) + ((int64_t)b * a.len + t0) * a.heads + h;
-  const T* pC = reinterpret_cast<const T*>(a.Cm.ptr) + bc4_off(a.Cm, b, t0, h, q);
-  const bool has_z = a.z.ptr != nullptr;
-  const T* pz = has_z ? reinterpret_cast<const T*>(a.z.ptr) + bc4_off(a.z, b, t0, h, q) : nullptr;
-  for (int k = n; k > 0; k -= U) {
-    uint4 gr[U], cr[U], zr[U];
-    float d[U];
-#pragma unroll
-    for (int i = 0; i < U; ++i) {
-      const int kk = max(k - 1 - i, 0);
-      gr[i] = __ldg(reinterpret_cast<const uint4*>(pdy + (int64_t)kk * HP));
-      cr[i] = __ldg(reinterpret_cast<const uint4*>(pC + (int64_t)kk * a.Cm.st));
-      zr[i] = has_z ? __ldg(reinterpret_cast<const uint4*>(pz + (int64_t)kk * a.z.st)) : make_uint4(0, 0, 0, 0);
-      d[i] = to_f<T>(__ldg(pdt + (int64_t)kk * a.heads));
-    }
-#pragma unroll
-    for (int i = 0; i < U; ++i) {
-      if (k - 1 - i < 0) break;
-      float dout[V], cv[V], zv[V];
-      Vec16<T> v;
-      v.raw = gr[i], v.unpack(dout);
-      v.raw = cr[i], v.unpack(cv);
-      v.raw = zr[i], v.unpack(zv);
-#pragma unroll
-      for (int e = 0; e < V; ++e) carry[e] = ex2_approx(d[i] * Av[e]) * fmaf(cv[e], gated_dy(dout[e], has_z, zv[e]), carry[e]);
-    }
-  }
-  reinterpret_cast<float4*>(R)[0] = make_float4(carry[0], carry[1], carry[2], carry[3]);
-  reinterpret_cast<float4*>(R)[1] = make_float4(carry[4], carry[5], carry[6], carry[7]);
-}
-
 // reverse phase 2: over the pieces from the right; R[c] <- adjoint entering piece c from piece c + 1
 __global__ void __launch_bounds__(kCarryLanes * kCarryGroups) chunk_bwd_carry_kernel(const ssm_chunk_bwd_args g, int nchunks) {
   const ssm_chunk_args& a = g.fwd;
@@ -423,7 +269,7 @@ __global__ void __launch_bounds__(kCarryLanes * kCarryGroups) chunk_bwd_carry_ke
   const bool live = hp_raw < HP;
   const int hp = live ? hp_raw : HP - 1;
   const int b = blockIdx.z;
-  const float* P = g.scratch + (int64_t)b * nchunks * HP + hp;
+  const float* P = g.scratch_fwd + (int64_t)b * nchunks * HP + hp;
   float* R = g.scratch + 2 * (int64_t)a.batch * nchunks * HP + (int64_t)b * nchunks * HP + hp;
   const float carry = carry_pieces<true>(P, R, nchunks, HP, 0.f, live);
   if (live && threadIdx.x < kCarryLanes && g.dinitial.ptr) {
@@ -460,7 +306,7 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_kernel(const ssm_chun
     s0 = a.initial.ptr ? bc4_load_f32(a.initial, ln.b, 0, ln.h, ln.q) : 0.f;
     carry = 0.f;
   } else {
-    s0 = g.scratch[(int64_t)a.batch * nchunks * ln.HP + slot];
+    s0 = g.scratch_fwd[(int64_t)a.batch * nchunks * ln.HP + slot];
     carry = g.scratch[2 * (int64_t)a.batch * nchunks * ln.HP + slot];
   }
   const Stream<T> sx = ln.x(a, t0), sdt = ln.dt(a, t0);
@@ -531,7 +377,7 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_kernel(const ssm_chun
     else atomicAdd(bc4_ptr(g.dB, ln.b, t, ln.h, ln.q), G * d * x);
     dX[(int64_t)k * ln.HP] = from_f<T>(fmaf(dyv, ln.Dv, G * d * bv));
     const float gsa = G * sp * da;
-    add_reduced(g.ddt + ((int64_t)ln.b * a.len + t) * a.heads + ln.h, fmaf(G, bv * x, gsa * A_nat), warp_heads);
+    add_reduced(reinterpret_cast<float*>(g.ddt) + ((int64_t)ln.b * a.len + t) * a.heads + ln.h, fmaf(G, bv * x, gsa * A_nat), warp_heads);
     dA_acc = fmaf(gsa, d, dA_acc);
     dD_acc = fmaf(dyv, x, dD_acc);
     carry = G * da;
@@ -564,197 +410,6 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_kernel(const ssm_chun
 }
 
 
-// Final backward pass on 16-byte lanes: a thread takes 8 neighbouring projections of one head and one chunk (states and
-// adjoints entering the chunk from the scratch).  Same arithmetic as chunk_bwd_kernel<.., 1>; every stream is read and
-// written as 16-byte pieces, the per-(b, t, h) sum for ddt is formed over the thread's 8 lanes and, where the threads of a
-// head are neighbouring lanes of one warp, over those by shuffles before one atomic add.
-template <typename T>
-__global__ void __launch_bounds__(kChunkThreads) chunk_bwd_vec_kernel(const ssm_chunk_bwd_args g, int nchunks) {
-  constexpr int V = 8, U = 2;
-  const ssm_chunk_args& a = g.fwd;
-  const int HP = a.heads * a.proj;
-  const int hp_raw = (blockIdx.x * kChunkThreads + threadIdx.x) * V;
-  const bool active = hp_raw < HP;
-  const int hp = active ? hp_raw : HP - V;  // idle threads of the last CTA shadow a valid lane group and write nothing
-  const int h = hp / a.proj, q = hp % a.proj;
-  const int b = blockIdx.z, c = blockIdx.y;
-  const int valid = chunk_valid_len(a, b);
-  const int t0 = c * a.chunk_size, t1 = min(a.len, t0 + a.chunk_size);
-  const int n = max(t0, min(t1, valid)) - t0;
-  const int64_t slot = ((int64_t)b * nchunks + c) * HP + hp;
-  float Av[V], Dv[V], s0[V], carry[V];
-  {
-    const float* ps = g.scratch + (int64_t)a.batch * nchunks * HP + slot;
-    const float* pr = g.scratch + 2 * (int64_t)a.batch * nchunks * HP + slot;
-    const float4 a0 = reinterpret_cast<const float4*>(ps)[0], a1 = reinterpret_cast<const float4*>(ps)[1];
-    const float4 r0 = reinterpret_cast<const float4*>(pr)[0], r1 = reinterpret_cast<const float4*>(pr)[1];
-    s0[0] = a0.x, s0[1] = a0.y, s0[2] = a0.z, s0[3] = a0.w, s0[4] = a1.x, s0[5] = a1.y, s0[6] = a1.z, s0[7] = a1.w;
-    carry[0] = r0.x, carry[1] = r0.y, carry[2] = r0.z, carry[3] = r0.w, carry[4] = r1.x, carry[5] = r1.y, carry[6] = r1.z, carry[7] = r1.w;
-  }
-#pragma unroll
-  for (int e = 0; e < V; ++e) {
-    Av[e] = bc4_load_f32(a.A, 0, 0, h, q + e) * kLog2e;
-    Dv[e] = a.D.ptr ? bc4_load_f32(a.D, 0, 0, h, q + e) : 0.f;
-  }
-  const int64_t row0 = ((int64_t)b * a.len + t0) * HP + hp;
-  const T* px = reinterpret_cast<const T*>(a.X) + row0;
-  const T* pdy = reinterpret_cast<const T*>(g.dY) + row0;
-  const T* pdt = reinterpret_cast<const T*>(a.dt) + ((int64_t)b * a.len + t0) * a.heads + h;
-  const T* pB = reinterpret_cast<const T*>(a.Bm.ptr) + bc4_off(a.Bm, b, t0, h, q);
-  const T* pC = reinterpret_cast<const T*>(a.Cm.ptr) + bc4_off(a.Cm, b, t0, h, q);
-  const bool has_z = a.z.ptr != nullptr;
-  const T* pz = has_z ? reinterpret_cast<const T*>(a.z.ptr) + bc4_off(a.z, b, t0, h, q) : nullptr;
-  float* hist = g.history + row0;
-  T* dX = reinterpret_cast<T*>(g.dX) + row0;
-  // element offsets of this thread's first step in the gradient buffers of B, C, z (fp32, or the io type: a.typed_grads)
-  const int64_t oB = bc4_off(g.dB, b, t0, h, q), oC = bc4_off(g.dC, b, t0, h, q), oZ = has_z ? bc4_off(g.dz, b, t0, h, q) : 0;
-  const bool typed_b = a.typed_grads & 1, typed_c = a.typed_grads & 2, typed_z = a.typed_grads & 4;
-  auto unpack8 = [](const uint4& r, float (&f)[V]) {
-    Vec16<T> v;
-    v.raw = r;
-    v.unpack(f);
-  };
-  auto ld8 = [](const float* p, float (&f)[V]) {
-    const float4 u0 = reinterpret_cast<const float4*>(p)[0], u1 = reinterpret_cast<const float4*>(p)[1];
-    f[0] = u0.x, f[1] = u0.y, f[2] = u0.z, f[3] = u0.w, f[4] = u1.x, f[5] = u1.y, f[6] = u1.z, f[7] = u1.w;
-  };
-  auto st8 = [](float* p, const float (&f)[V]) {
-    reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
-    reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
-  };
-  auto put8 = [&](const ssm_bcast4& p, bool typed, int64_t off, const float (&f)[V]) {
-    if (typed) {
-      Vec16<T> o;
-      o.pack(f);
-      *reinterpret_cast<uint4*>(const_cast<T*>(reinterpret_cast<const T*>(p.ptr)) + off) = o.raw;
-    } else {
-      st8(const_cast<float*>(reinterpret_cast<const float*>(p.ptr)) + off, f);
-    }
-  };
-
-  // ---- states of the chunk, into the history ---------------------------------------------------------------
-  {
-    constexpr int UF = 4;
-    float s[V];
-#pragma unroll
-    for (int e = 0; e < V; ++e) s[e] = s0[e];
-    for (int k = 0; k < n; k += UF) {
-      uint4 xr[UF], br[UF];
-      float d[UF];
-#pragma unroll
-      for (int i = 0; i < UF; ++i) {
-        const int kk = min(k + i, n - 1);
-        xr[i] = __ldg(reinterpret_cast<const uint4*>(px + (int64_t)kk * HP));
-        br[i] = __ldg(reinterpret_cast<const uint4*>(pB + (int64_t)kk * a.Bm.st));
-        d[i] = to_f<T>(__ldg(pdt + (int64_t)kk * a.heads));
-      }
-#pragma unroll
-      for (int i = 0; i < UF; ++i) {
-        if (k + i < n) {
-          float x[V], bv[V];
-          unpack8(xr[i], x);
-          unpack8(br[i], bv);
-#pragma unroll
-          for (int e = 0; e < V; ++e) s[e] = fmaf(ex2_approx(d[i] * Av[e]), s[e], d[i] * bv[e] * x[e]);
-          if (active) st8(hist + (int64_t)(k + i) * HP, s);
-        }
-      }
-    }
-  }
-  if (active) {
-    const float zero8[V] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int t = t0 + n; t < t1; ++t) {  // beyond the sequence: zeros in what this call writes in full
-      *reinterpret_cast<uint4*>(dX + (int64_t)(t - t0) * HP) = make_uint4(0, 0, 0, 0);
-      if (typed_b) put8(g.dB, true, oB + (int64_t)(t - t0) * g.dB.st, zero8);
-      if (typed_c) put8(g.dC, true, oC + (int64_t)(t - t0) * g.dC.st, zero8);
-      if (has_z && typed_z) put8(g.dz, true, oZ + (int64_t)(t - t0) * g.dz.st, zero8);
-    }
-  }
-
-  // ---- reverse recurrence  g_t = C_t dy_t + exp(dt_{t+1} A) g_{t+1} -------------------------------------------
-  // threads of one head: proj / 8 neighbouring threads; reduced by shuffles when that is a power of two within a warp
-  const int group = a.proj / V;
-  const bool shuffle_heads = (group & (group - 1)) == 0 && group <= 32;
-  float dA_acc[V], dD_acc = 0.f;
-#pragma unroll
-  for (int e = 0; e < V; ++e) dA_acc[e] = 0.f;
-  for (int k = n; k > 0; k -= U) {
-    uint4 xr[U], br[U], cr[U], zr[U], gr[U];
-    float d[U], st[U + 1][V];
-#pragma unroll
-    for (int i = 0; i < U; ++i) {
-      const int kk = max(k - 1 - i, 0);
-      xr[i] = __ldg(reinterpret_cast<const uint4*>(px + (int64_t)kk * HP));
-      br[i] = __ldg(reinterpret_cast<const uint4*>(pB + (int64_t)kk * a.Bm.st));
-      cr[i] = __ldg(reinterpret_cast<const uint4*>(pC + (int64_t)kk * a.Cm.st));
-      zr[i] = has_z ? __ldg(reinterpret_cast<const uint4*>(pz + (int64_t)kk * a.z.st)) : make_uint4(0, 0, 0, 0);
-      gr[i] = __ldg(reinterpret_cast<const uint4*>(pdy + (int64_t)kk * HP));
-      d[i] = to_f<T>(__ldg(pdt + (int64_t)kk * a.heads));
-    }
-#pragma unroll
-    for (int i = 0; i <= U; ++i) {
-      const int kk = k - 1 - i;  // the state after step kk; before the chunk's first step: the incoming state
-      if (kk >= 0) {
-        ld8(hist + (int64_t)kk * HP, st[i]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < V; ++e) st[i][e] = s0[e];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < U; ++i) {
-      const int kk = k - 1 - i;
-      if (kk < 0) break;
-      float x[V], bv[V], cv[V], zv[V], dout[V], dxo[V], dbo[V], dco[V], dzo[V];
-      unpack8(xr[i], x);
-      unpack8(br[i], bv);
-      unpack8(cr[i], cv);
-      unpack8(zr[i], zv);
-      unpack8(gr[i], dout);
-      float ddt_sum = 0.f;
-#pragma unroll
-      for (int e = 0; e < V; ++e) {
-        float dyv = dout[e];
-        if (has_z) {
-          const float sg = sigmoid_fast(zv[e]);
-          const float yfull = fmaf(Dv[e], x[e], st[i][e] * cv[e]);
-          dzo[e] = dout[e] * yfull * sg * (1.f + zv[e] * (1.f - sg));
-          dyv = dout[e] * zv[e] * sg;
-        }
-        const float da = ex2_approx(d[i] * Av[e]);
-        const float G = fmaf(cv[e], dyv, carry[e]);
-        dco[e] = dyv * st[i][e];
-        dbo[e] = G * d[i] * x[e];
-        dxo[e] = fmaf(dyv, Dv[e], G * d[i] * bv[e]);
-        const float gsa = G * st[i + 1][e] * da;
-        ddt_sum += fmaf(G, bv[e] * x[e], gsa * (Av[e] * kLn2));
-        dA_acc[e] = fmaf(gsa, d[i], dA_acc[e]);
-        dD_acc = fmaf(dyv, x[e], dD_acc);
-        carry[e] = G * da;
-      }
-      if (!active) ddt_sum = 0.f;
-      if (shuffle_heads) {
-        for (int m = 1; m < group; m <<= 1) ddt_sum += __shfl_xor_sync(0xffffffffu, ddt_sum, m);
-        if (active && (threadIdx.x & (group - 1)) == 0) atomicAdd(g.ddt + ((int64_t)b * a.len + t0 + kk) * a.heads + h, ddt_sum);
-      } else if (active) {
-        atomicAdd(g.ddt + ((int64_t)b * a.len + t0 + kk) * a.heads + h, ddt_sum);
-      }
-      if (active) {
-        put8(g.dC, typed_c, oC + (int64_t)kk * g.dC.st, dco);
-        put8(g.dB, typed_b, oB + (int64_t)kk * g.dB.st, dbo);
-        if (has_z) put8(g.dz, typed_z, oZ + (int64_t)kk * g.dz.st, dzo);
-        Vec16<T> o;
-        o.pack(dxo);
-        *reinterpret_cast<uint4*>(dX + (int64_t)kk * HP) = o.raw;
-      }
-    }
-  }
-  if (!active) return;
-#pragma unroll
-  for (int e = 0; e < V; ++e) atomicAdd(bc4_ptr(g.dA, 0, 0, h, q + e), dA_acc[e]);
-  if (g.dD.ptr) atomicAdd(bc4_ptr(g.dD, 0, 0, h, 0), dD_acc);  // one skip weight per head (the launcher checks)
-}
-
 static bool bc4_dense_host(const ssm_bcast4& p) { return p.ptr && p.sb != 0 && p.st != 0 && p.sh != 0 && p.sq != 0; }
 
 static int chunk_validate(const ssm_chunk_args* a) {
@@ -776,13 +431,14 @@ static int chunk_fwd_len(int chunk_size, int len) {
   return piece < chunk_size ? piece : chunk_size;
 }
 
-// 16-byte rows for the vector kernels: the projection axis contiguous and a multiple of 8, every other stride a multiple of 8
-template <typename T>
-static bool chunk_vec_ok(const ssm_chunk_args& a) {
-  if (sizeof(T) != 2 || a.proj % 8 != 0 || a.scratch == nullptr) return false;
-  auto dense8 = [](const ssm_bcast4& p) { return p.sq == 1 && p.sb % 8 == 0 && p.st % 8 == 0 && p.sh % 8 == 0 && aligned_to(p.ptr, 16); };
-  if (!dense8(a.Bm) || !dense8(a.Cm) || (a.z.ptr && !dense8(a.z))) return false;
-  return aligned_to(a.X, 16) && aligned_to(a.Y, 16) && aligned_to(a.scratch, 16);
+// The layouts that the four-projection kernels read: the projection axis contiguous, every row a multiple of four elements and
+// aligned to them; B, C, z of X's element type.
+static bool chunk_vec_ok(const ssm_chunk_args& a, int piece) {
+  if (a.proj % 4 != 0 || a.scratch == nullptr || a.par_dtype != a.io_dtype || piece > kPiece) return false;
+  const size_t al = 4 * dtype_size(a.io_dtype);
+  auto rows4 = [&](const ssm_bcast4& p) { return p.sq == 1 && p.sb % 4 == 0 && p.st % 4 == 0 && p.sh % 4 == 0 && aligned_to(p.ptr, al); };
+  if (!rows4(a.Bm) || !rows4(a.Cm) || (a.z.ptr && !rows4(a.z))) return false;
+  return aligned_to(a.X, al) && aligned_to(a.Y, al) && aligned_to(a.scratch, 16);
 }
 
 // chunk_len: steps per piece (the backward passes the caller's chunk size, which its own scratch and history are sized by)
@@ -796,20 +452,16 @@ static int chunk_fwd_t(const ssm_chunk_args& a, cudaStream_t st, int chunk_len, 
     return launch_status("chunk_fwd_kernel<serial>");
   }
   SSM_REQUIRE(nchunks <= 65535, SSM_ERR_TOO_LARGE, "ssd_chunk_scan: more than 65535 chunks");
-  const bool vec = std::is_same<T, PT>::value && chunk_vec_ok<T>(a);
-  const unsigned gv = (HP / 8 + kChunkThreads - 1) / kChunkThreads;
-  if constexpr (sizeof(T) == 2) {
-    if (vec) chunk_fwd_vec_kernel<T, 1><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  }
-  if (!vec) chunk_fwd_kernel<T, PT, 1><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  const bool vec = std::is_same<T, PT>::value && chunk_vec_ok(a, chunk_len);
+  const unsigned gv = (HP / 4 + kChunkThreads - 1) / kChunkThreads;
+  if (vec) chunk_fwd4_kernel<T, false><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  else chunk_fwd_kernel<T, PT, 1><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
   if (int rc = launch_status("chunk_fwd_kernel<local>")) return rc;
   chunk_carry_kernel<<<dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), kCarryLanes * kCarryGroups, 0, st>>>(a, nchunks);
   if (int rc = launch_status("chunk_carry_kernel")) return rc;
   if (through_phase2_only) return SSM_OK;
-  if constexpr (sizeof(T) == 2) {
-    if (vec) chunk_fwd_vec_kernel<T, 3><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  }
-  if (!vec) chunk_fwd_kernel<T, PT, 3><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  if (vec) chunk_fwd4_kernel<T, true><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  else chunk_fwd_kernel<T, PT, 3><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
   return launch_status("chunk_fwd_kernel<apply>");
 }
 
@@ -822,6 +474,19 @@ static int chunk_bwd_len(int chunk_size, int len) {
   return piece < chunk_size ? piece : chunk_size;
 }
 
+// The call runs on the four-projection kernels: readable layouts, gradients of B, C, z written in full in their own type, and heads
+// whose projections are a power of two of at most a warp's lanes (their sums for ddt then stay inside a warp).
+static bool chunk_bwd_vec_ok(const ssm_chunk_bwd_args& g, int piece, int nchunks) {
+  const ssm_chunk_args& a = g.fwd;
+  const size_t al = 4 * dtype_size(a.io_dtype);
+  const int share = a.proj / 4, need = 3 | (a.z.ptr ? 4 : 0);
+  ssm_chunk_args f = a;
+  f.scratch = g.scratch, f.Y = g.dX;  // only their alignment is looked at
+  if (!chunk_vec_ok(f, piece) || nchunks <= 1 || nchunks > 65535 || (a.typed_grads & need) != need || share > 32 || (share & (share - 1)) != 0) return false;
+  auto rows4 = [&](const ssm_bcast4& p) { return p.sq == 1 && p.sb % 4 == 0 && p.st % 4 == 0 && p.sh % 4 == 0 && aligned_to(p.ptr, al); };
+  return rows4(g.dB) && rows4(g.dC) && (!a.z.ptr || rows4(g.dz)) && aligned_to(g.dY, al);
+}
+
 template <typename T, typename PT>
 static int chunk_bwd_t(const ssm_chunk_bwd_args& g_in, cudaStream_t st) {
   ssm_chunk_bwd_args g = g_in;
@@ -830,46 +495,35 @@ static int chunk_bwd_t(const ssm_chunk_bwd_args& g_in, cudaStream_t st) {
   const int HP = a.heads * a.proj;
   const unsigned gx = (HP + kChunkThreads - 1) / kChunkThreads;
   const int nchunks = (a.len + a.chunk_size - 1) / a.chunk_size;
+  const bool vec = std::is_same<T, PT>::value && chunk_bwd_vec_ok(g, a.chunk_size, nchunks);
+  SSM_REQUIRE(vec || (g.history && !(a.typed_grads & 8)), SSM_ERR_UNSUPPORTED, "ssd_chunk_scan_backward: this call needs a history and an fp32 ddt");
   if (!g.scratch || nchunks <= 1 || nchunks > 65535) {
     chunk_bwd_kernel<T, PT, 0><<<dim3(gx, 1, a.batch), kChunkThreads, 0, st>>>(g, 1);
     return launch_status("chunk_bwd_kernel<serial>");
   }
-  // states entering every chunk (forward phases 1 and 2 on the backward call's scratch; no final state, no Y)
-  ssm_chunk_args f = a;
-  f.scratch = g.scratch, f.final_state = nullptr;
-  if (int rc = chunk_fwd_t<T, PT>(f, st, a.chunk_size, true)) return rc;
-  bool local_vec = false;
-  if constexpr (sizeof(T) == 2 && std::is_same<T, PT>::value) {
-    ssm_chunk_args f2 = a;
-    f2.scratch = g.scratch;
-    f2.Y = g.dX;  // only its alignment is looked at
-    local_vec = chunk_vec_ok<T>(f2) && aligned_to(g.dY, 16);
-    if (local_vec) {
-      const unsigned gv = (HP / 8 + kChunkThreads - 1) / kChunkThreads;
-      chunk_bwd_local_vec_kernel<T><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
-    }
+  // states entering every piece and the pieces' decay products: left by the forward call, or formed again (its phases 1 and 2 on
+  // this call's scratch; no final state, no Y)
+  if (g.fwd_scratch && chunk_fwd_len(g_in.fwd.chunk_size, a.len) == a.chunk_size) {
+    g.scratch_fwd = g.fwd_scratch;
+  } else {
+    ssm_chunk_args f = a;
+    f.scratch = g.scratch, f.final_state = nullptr;
+    if (int rc = chunk_fwd_t<T, PT>(f, st, a.chunk_size, true)) return rc;
+    g.scratch_fwd = g.scratch;
   }
-  if (!local_vec) chunk_bwd_local_kernel<T, PT><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
+  float* R = g.scratch + 2 * (int64_t)a.batch * nchunks * HP;
+  const unsigned gv = (HP / 4 + kChunkThreads - 1) / kChunkThreads;
+  if (vec) chunk_bwd_local4_kernel<T><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(g, R, nchunks, a.chunk_size);
+  else chunk_bwd_local_kernel<T, PT><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
   if (int rc = launch_status("chunk_bwd_local_kernel")) return rc;
   chunk_bwd_carry_kernel<<<dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), kCarryLanes * kCarryGroups, 0, st>>>(g, nchunks);
   if (int rc = launch_status("chunk_bwd_carry_kernel")) return rc;
-  if constexpr (sizeof(T) == 2 && std::is_same<T, PT>::value) {
-    // 16-byte lanes: dense 16-bit B, C, z (see chunk_vec_ok), dense fp32 gradient buffers for them with 16-byte rows, and a
-    // skip weight per head (or none), whose gradient is then one sum per thread
-    // (a broadcast axis, stride 0, would make several steps write one element: those buffers keep the atomic path)
-    auto dense4 = [](const ssm_bcast4& p) {  // multiples of 8 elements: 16-byte rows whether the buffer is fp32 or 16-bit
-      return p.ptr && p.sq == 1 && p.sb != 0 && p.st != 0 && p.sh != 0 && p.sb % 8 == 0 && p.st % 8 == 0 && p.sh % 8 == 0 && aligned_to(p.ptr, 16);
-    };
-    ssm_chunk_args f2 = a;
-    f2.scratch = g.scratch;
-    f2.Y = g.dX;  // only its alignment is looked at
-    const bool vec = chunk_vec_ok<T>(f2) && dense4(g.dB) && dense4(g.dC) && (!a.z.ptr || dense4(g.dz)) && (!a.D.ptr || !g.dD.ptr || a.D.sq == 0) &&
-                     aligned_to(g.dY, 16) && aligned_to(g.history, 16) && (a.heads * a.proj) % 8 == 0;
-    if (vec) {
-      const unsigned gv = (a.heads * a.proj / 8 + kChunkThreads - 1) / kChunkThreads;
-      chunk_bwd_vec_kernel<T><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
-      return launch_status("chunk_bwd_vec_kernel");
-    }
+  if (vec) {
+    const int64_t items = (int64_t)a.batch * nchunks, slots = (int64_t)bwd4_ctas<T>() * sm_count() / gv;  // one wave of CTAs, each looping over pieces
+    const int64_t rounds = (items + (slots < 1 ? 1 : slots) - 1) / (slots < 1 ? 1 : slots);
+    const unsigned gy = (unsigned)((items + rounds - 1) / rounds);  // as many CTAs as the longest of them makes worthwhile
+    chunk_bwd4_kernel<T><<<dim3(gv, gy), kChunkThreads, 0, st>>>(g, g.scratch_fwd + items * HP, R, nchunks, a.chunk_size, (a.typed_grads & 8) != 0);
+    return launch_status("chunk_bwd4_kernel");
   }
   chunk_bwd_kernel<T, PT, 1><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
   return launch_status("chunk_bwd_kernel");
@@ -891,6 +545,12 @@ extern "C" int64_t ssm_chunk_scan_bwd_scratch_floats(int32_t batch, int32_t len,
   const int64_t piece = chunk_bwd_len(chunk_size, len);
   const int64_t nchunks = (len + piece - 1) / piece;
   return 3 * (int64_t)batch * nchunks * heads * proj;  // decay products, states entering, adjoints entering every chunk
+}
+
+extern "C" int ssm_chunk_scan_bwd_fused(const ssm_chunk_bwd_args* g) {
+  if (!g || g->fwd.io_dtype == SSM_F64 || chunk_validate(&g->fwd) || g->fwd.len == 0) return 0;
+  const int piece = chunk_bwd_len(g->fwd.chunk_size, g->fwd.len);
+  return chunk_bwd_vec_ok(*g, piece, (g->fwd.len + piece - 1) / piece);
 }
 
 extern "C" int ssm_chunk_scan_fwd(const ssm_chunk_args* a, ssm_stream_t stream) {
@@ -922,10 +582,10 @@ extern "C" int ssm_chunk_scan_bwd(const ssm_chunk_bwd_args* g, ssm_stream_t stre
   if (int rc = chunk_validate(a)) return rc;
   if (a->batch == 0 || a->heads == 0 || a->proj == 0 || a->len == 0) return SSM_OK;
   SSM_REQUIRE(a->A.ptr && a->Bm.ptr && a->Cm.ptr && a->X && a->dt, SSM_ERR_NULL, "ssd_chunk_scan_backward: missing input");
-  SSM_REQUIRE(g->dY && g->dX && g->ddt && g->dA.ptr && g->dB.ptr && g->dC.ptr && g->history, SSM_ERR_NULL,
+  SSM_REQUIRE(g->dY && g->dX && g->ddt && g->dA.ptr && g->dB.ptr && g->dC.ptr, SSM_ERR_NULL,
               "ssd_chunk_scan_backward: missing gradient buffer");
   SSM_REQUIRE(!a->z.ptr || g->dz.ptr, SSM_ERR_NULL, "ssd_chunk_scan_backward: dz is required when z is given");
-  SSM_REQUIRE((a->typed_grads & ~7) == 0 && (!(a->typed_grads & 1) || bc4_dense_host(g->dB)) && (!(a->typed_grads & 2) || bc4_dense_host(g->dC)) &&
+  SSM_REQUIRE((a->typed_grads & ~15) == 0 && (!(a->typed_grads & 1) || bc4_dense_host(g->dB)) && (!(a->typed_grads & 2) || bc4_dense_host(g->dC)) &&
                   (!(a->typed_grads & 4) || (a->z.ptr && bc4_dense_host(g->dz))),
               SSM_ERR_SHAPE, "ssd_chunk_scan_backward: a typed gradient buffer must have no broadcast axis");
   SSM_REQUIRE(a->par_dtype == a->io_dtype || a->par_dtype == SSM_F32, SSM_ERR_UNSUPPORTED,

@@ -263,7 +263,9 @@ struct ChunkCall final : Call {
     if (init.has_value()) t_init = init->scalar_type();
   }
 
-  variable_list forward(bool) override {
+  Tensor kept;  // the forward call's scratch: the states entering every piece
+
+  variable_list forward(bool train) override {
     c10::cuda::CUDAGuard guard(c.X.device());
     Tensor Y = at::empty_like(c.X);
     const int64_t n = ssm_chunk_scan_scratch_floats((int)c.nb, (int)c.nl, (int)c.nh, (int)c.np, c.chunk);
@@ -272,6 +274,7 @@ struct ChunkCall final : Call {
     c.fill(a);
     a.Y = Y.data_ptr(), a.scratch = scratch.data_ptr<float>();
     run(ssm_chunk_scan_fwd(&a, stream_of(c.X)));
+    if (train) kept = scratch;
     return {Y};
   }
 
@@ -279,7 +282,7 @@ struct ChunkCall final : Call {
     c10::cuda::CUDAGuard guard(c.X.device());
     const auto f32 = c.X.options().dtype(at::kFloat);
     Tensor gy = like(grads[0], c.X);
-    Tensor dX = at::empty_like(c.X), ddt, dA, dB, dC, dD, dz, dI;
+    Tensor dX = at::empty_like(c.X), ddt, dA, dB, dC, dD, dz, dI, hist;
     ZeroPool pool;
     int typed = 0;
     // per-token B / C / z: their gradients are written by the kernel in the tensor's own type (no zero-fill, no fp32 copy)
@@ -288,20 +291,28 @@ struct ChunkCall final : Call {
       if (k == Kind::BLHP) grad = at::empty_like(*t), typed |= bit;
       else pool.add(grad, t->sizes());
     };
-    pool.add(ddt, {c.nb, c.nl, c.nh}), pool.add(dA, c.A->sizes());
     own(dB, c.B, c.kB, 1), own(dC, c.C, c.kC, 2), own(dz, c.z, c.kz, 4);
-    if (c.D.has_value()) pool.add(dD, c.D->sizes());
-    if (c.init.has_value()) pool.add(dI, c.init->sizes());
-    pool.make(f32);
-    Tensor hist = at::empty({c.nb, std::max<int64_t>(c.nl, 1), c.nh, c.np}, f32);
     Tensor scratch = at::empty({std::max<int64_t>(1, ssm_chunk_scan_bwd_scratch_floats((int)c.nb, (int)c.nl, (int)c.nh, (int)c.np, c.chunk))}, f32);
     ssm_chunk_bwd_args g{};
     c.fill(g.fwd);
-    g.fwd.typed_grads = typed;
-    g.dY = gy.data_ptr(), g.dX = dX.data_ptr(), g.ddt = ddt.data_ptr<float>(), g.history = hist.data_ptr<float>(), g.scratch = scratch.data_ptr<float>();
+    g.dY = gy.data_ptr(), g.dX = dX.data_ptr(), g.scratch = scratch.data_ptr<float>(), g.fwd_scratch = kept.data_ptr<float>();
     auto grad_of = [](const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };
-    set_bc4(g.dA, grad_of(dA), c.kA), set_bc4(g.dB, grad_of(dB), c.kB), set_bc4(g.dC, grad_of(dC), c.kC), set_bc4(g.dD, grad_of(dD), c.kD),
-        set_bc4(g.dz, grad_of(dz), c.kz), set_bc4(g.dinitial, grad_of(dI), Kind::BHP);
+    auto set_bcz = [&]() { set_bc4(g.dB, grad_of(dB), c.kB), set_bc4(g.dC, grad_of(dC), c.kC), set_bc4(g.dz, grad_of(dz), c.kz); };
+    bool fused = typed == (3 | (c.z.has_value() ? 4 : 0));
+    if (fused) {
+      set_bcz();
+      g.fwd.typed_grads = typed;
+      fused = ssm_chunk_scan_bwd_fused(&g) != 0;
+    }
+    if (fused) ddt = at::empty({c.nb, c.nl, c.nh}, c.X.options()), typed |= 8;
+    else pool.add(ddt, {c.nb, c.nl, c.nh}), hist = at::empty({c.nb, std::max<int64_t>(c.nl, 1), c.nh, c.np}, f32);
+    pool.add(dA, c.A->sizes());
+    if (c.D.has_value()) pool.add(dD, c.D->sizes());
+    if (c.init.has_value()) pool.add(dI, c.init->sizes());
+    pool.make(f32);
+    set_bcz();
+    g.fwd.typed_grads = typed, g.ddt = ddt.data_ptr(), g.history = out_ptr(hist);
+    set_bc4(g.dA, grad_of(dA), c.kA), set_bc4(g.dD, grad_of(dD), c.kD), set_bc4(g.dinitial, grad_of(dI), Kind::BHP);
     run(ssm_chunk_scan_bwd(&g, stream_of(c.X)));
     variable_list res = {dX, cast(ddt, t_dt), cast(dA, t_A), cast(dB, t_B), cast(dC, t_C)};
     if (c.D.has_value()) res.push_back(cast(dD, t_D));

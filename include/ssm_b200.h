@@ -401,29 +401,19 @@ int ssm_fused_add_norm_bwd_noalloc(const ssm_norm_bwd_args* args, ssm_stream_t s
  * given initial_states on top of what phase 1 left in the scratch (by linearity), writes
  * the corrected final_states and produces Y.  A sequence shard uses 1, exchanges final
  * states with its neighbours, then 2.
- * dt_mode: 0 = dt is (batch, len, heads) in io_dtype and goes through dt_bias / dt_softplus.  1 = dt is fp32 and holds
- * the step sizes as they are used (dt_bias and dt_softplus are ignored).  3 = as 1, and the step size enters the
- * decay exp(dt A) only: the inputs are added with unit weight, S_t = exp(dt_t A) S_{t-1} + x_t B_t^T.  Modes 1 and 3
- * are what the backward pass uses to run the adjoint recurrence through the same kernels.  + 4 (to any mode): the caller
- * promises that heads 2 i and 2 i + 1 have equal step sizes and decay; the decay mask is then formed once per pair.
+ * reverse: the adjoint pass of the backward.  X, Bm and Cm hold dy, C and B; ws_dt and ws_cum are those of the forward call on
+ * the same step sizes (nothing is recomputed), initial_states the gradient of the final state.  Y receives
+ * dx_j = dt_j (G_j B_j) without the skip term, G_j the adjoint state of step j; ws_state_in, for every chunk, the adjoint that enters it from
+ * the right (that of the next chunk's first step); final_states the adjoint state of step 0.
  * row_dots: (batch, len, heads) fp32, zero-filled by the caller.  When given, z is not a gate: Y is written ungated and
  * row_dots[b, t, h] receives sum_p y[p] z[p], with y taken before the D x term and before rounding to io_dtype (the
  * backward pass forms dy . y and d(dt x) . x this way).
- * row_scale: (batch, len, heads) fp32 positive weights: output row t of head h is multiplied by row_scale[b, t, h],
- * applied to the decay mask before it is rounded to the operand dtype (so a pass weighted this way rounds the same
- * masked tile as the forward pass, whose mask carries dt of the source step).
  * ws_state_in_f32: optional (batch, nchunks, heads, headdim * nstate) fp32: ws_state_in before rounding, same element order.
- * bc_width: stored width of the rows of Bm and Cm.  0 or nstate: (batch, len, groups, nstate).  64: (batch, len, groups, 64),
- * read as nstate-wide rows whose upper part is zero (the tensor-map copies fill what lies outside the tensor with
- * zeros) -- how the backward pass feeds x and dy in the places of B and C.
- * x_heads: 0, or the number of distinct input heads: X is then (batch, len, x_heads, headdim) and head h reads input head
- * h % x_heads (heads % x_heads == 0) -- how the backward pass feeds the two halves of a single group's B (or C) row to every
- * head without writing them out per head.  dt, z, Y and the states keep `heads` heads.
  * ------------------------------------------------------------------------------------- */
 typedef struct {
   int32_t batch, len, heads, headdim;
   int32_t nstate, groups, chunk_size, io_dtype;
-  int32_t dt_softplus, d_has_p, phase, dt_mode;
+  int32_t dt_softplus, d_has_p, phase, reverse;
   const void* X;
   const void* dt;
   const float* A;
@@ -441,9 +431,6 @@ typedef struct {
   void* ws_state_in;
   int32_t* status; /* nullable */
   float* row_dots; /* nullable */
-  const float* row_scale; /* nullable */
-  int32_t bc_width;       /* 0 (= nstate) or 64 */
-  int32_t x_heads;        /* 0 (= heads) or a divisor of heads */
   float* ws_state_in_f32; /* nullable */
   /* Packed sequences: num_seqs > 0 sequences lie end to end along len of a batch of one, each scanned from a zero state with
    * chunks counted from its first step.  seq_table (device): num_chunks pairs {first step, end of the sequence}, sequence by
@@ -477,34 +464,27 @@ int ssm_ssd_fold_shards(const float* gathered, int32_t world, int32_t rank, int3
 
 /* ---------------------------------------------------------------------------------------
  * Backward of the state-space-dual scan in the dual form (no counterpart upstream, whose Mamba-2 scan has no d_state
- * axis).  Its contractions are four more runs of ssm_ssd_fwd (dt_mode 1 / 3, row_dots, row_scale, bc_width above) on
- * transformed operands; the entry points below are the bandwidth passes around them.  `len` is the sequence length
- * rounded up to whole chunks (the length of the work tensors dy, dy_rev, y_plain, dx_rev), `len_valid` the length
- * of the caller's tensors (gY, z, X, dX, dz); work rows beyond len_valid are written as zeros.
- *   ssm_ssd_bwd_gate    dy = gY * silu(z) (gY when z is NULL), in time order and time-reversed (dy_rev)
- *   ssm_ssd_bwd_finish  dz = gY (y_plain + D x) silu'(z);  dX = reversed(dx_rev) + D dy;  dD (heads) or (heads, headdim)
- *                       += sum dy x (zero-filled by the caller; NULL when D is NULL)
- *   ssm_time_flip       dst[b, len - 1 - t] = src[b, t] for rows of row_bytes bytes (a multiple of 16); src has len_valid rows
- *   ssm_ssd_bwd_group_sum  out[b, t, g, :] = sum over the heads h of group g of weight[b, t, h] * y[b, ts, h, :]
- *                       (ts = len - 1 - t when reversed, else t; weight nullable; y (batch, len, heads, nstate);
- *                       out (batch, len_out, groups, nstate) in out_dtype = io_dtype or SSM_F32)
- *   ssm_ssd_bwd_spread  dst[r, h, :] = src[r, h / (heads / groups), :] for `rows` rows r: (rows, groups, row_bytes) ->
- *                       (rows, heads, row_bytes), the row of a B / C group handed to each of its heads
- *   ssm_ssd_state_dot   out[b, c, h] = <fwd_states[b, c, h, :], adj_states[b, nchunks - c, h, :]> for c >= 1, 0 for c = 0;
- *                       both (batch, nchunks, heads, elems) in io_dtype or SSM_F32 (ws_state_in / ws_state_in_f32 of two
- *                       ssm_ssd_fwd runs)
+ * axis), in this order:
+ *   ssm_ssd_bwd_gate    dy = gY * silu(z) (needed only with a gate)
+ *   ssm_ssd_fwd         again, without skip and gate: y, row_dots u = dy . y (z = dy), states before the chunks, also in fp32
+ *   ssm_ssd_fwd         reverse = 1: dx without the skip term, row_dots qd = delta d(delta x) . x (z = X), adjoints, also in fp32
+ *   ssm_ssd_bwd_bc      dB, dC (fp32, zero-filled by the caller) from dy, X, B, C, the exponents and both sets of states
+ *   ssm_ssd_bwd_finish  dz = gY (y + D x) silu'(z);  dX = dx + D dy;  dD (heads) or (heads, headdim) += sum dy x (zero-filled
+ *                       by the caller; NULL when D is NULL)
+ *   ssm_ssd_bwd_steps   ddt in dt's type, and dA (heads), ddt_bias (heads) += (fp32, zero-filled by the caller), from u, qd and the
+ *                       products <state, adjoint> at the chunk boundaries: the gradient of the decay exponent obeys
+ *                       da_{t+1} = da_t + qd_t - u_t
  * --------------------------------------------------------------------------------------- */
 typedef struct {
-  int32_t batch, len, len_valid, heads;
-  int32_t headdim, io_dtype, d_has_p, reserved0;
-  const void* gY;      /* (batch, len_valid, heads, headdim); nullable in finish when z is NULL */
+  int32_t batch, len, heads, headdim;
+  int32_t io_dtype, d_has_p;
+  const void* gY;      /* (batch, len, heads, headdim) */
   const void* z;       /* nullable */
   const void* X;       /* finish */
-  const void* y_plain; /* finish, with z: output of the forward pass without skip and gate, (batch, len, ...) */
-  const void* dx_rev;  /* finish: output of the adjoint pass, time-reversed, (batch, len, ...) */
+  const void* y_plain; /* finish, with z */
+  const void* dx;      /* finish: output of the adjoint pass */
   const float* D;      /* nullable */
   void* dy;            /* gate: out; finish: in */
-  void* dy_rev;        /* gate: out */
   void* dX;            /* finish: out */
   void* dz;            /* finish: out, with z */
   float* dD;           /* finish: accumulated, nullable */
@@ -512,12 +492,41 @@ typedef struct {
 
 int ssm_ssd_bwd_gate(const ssm_ssd_bwd_args* args, ssm_stream_t stream);
 int ssm_ssd_bwd_finish(const ssm_ssd_bwd_args* args, ssm_stream_t stream);
-int ssm_time_flip(const void* src, void* dst, int32_t batch, int32_t len, int32_t len_valid, int64_t row_bytes, ssm_stream_t stream);
-int ssm_ssd_bwd_group_sum(const void* y, const float* weight, void* out, int32_t batch, int32_t len, int32_t len_out, int32_t heads, int32_t groups,
-                          int32_t nstate, int32_t reversed, int32_t io_dtype, int32_t out_dtype, ssm_stream_t stream);
-int ssm_ssd_bwd_spread(const void* src, void* dst, int64_t rows, int32_t heads, int32_t groups, int64_t row_bytes, ssm_stream_t stream);
-int ssm_ssd_state_dot(const void* fwd_states, const void* adj_states, float* out, int32_t batch, int32_t nchunks, int32_t heads, int32_t elems,
-                      int32_t io_dtype, ssm_stream_t stream);
+
+typedef struct {
+  int32_t batch, len, heads, groups;
+  int32_t io_dtype, reserved0;
+  const void* X;  /* (batch, len, heads, 64) */
+  const void* dy; /* (batch, len, heads, 64) */
+  const void* Bm; /* (batch, len, groups, 128) */
+  const void* Cm;
+  const float* ws_dt; /* exponents and states as the two runs of ssm_ssd_fwd left them */
+  const float* ws_cum;
+  const void* state_in;
+  const void* adjoint_in;
+  float* dB; /* (batch, len, groups, 128), accumulated */
+  float* dC;
+  int32_t* status; /* nullable */
+} ssm_ssd_bc_args;
+int ssm_ssd_bwd_bc(const ssm_ssd_bc_args* args, ssm_stream_t stream);
+
+typedef struct {
+  int32_t batch, len, heads, io_dtype;
+  int32_t dt_softplus, reserved0;
+  const void* dt;       /* (batch, len, heads) io_dtype */
+  const float* dt_bias; /* nullable */
+  const float* A;
+  const float* u;  /* (batch, len, heads) */
+  const float* qd;
+  const float* ws_cum;
+  const float* state_f32;   /* (batch, nchunks, heads, 64 * 128): states before the chunks */
+  const float* adjoint_f32; /* likewise: adjoints entering them from the right */
+  const float* start0;      /* (batch, heads): <d initial state, initial state>; nullable */
+  void* ddt;                /* (batch, len, heads) io_dtype, written */
+  float* dA;
+  float* ddt_bias; /* nullable */
+} ssm_ssd_steps_args;
+int ssm_ssd_bwd_steps(const ssm_ssd_steps_args* args, ssm_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------
  * One decode token through a whole mixer in one launch (no counterpart upstream, whose step methods are sequences of

@@ -125,21 +125,19 @@ class SsdArgs(C.Structure):
     _fields_ = [
         ("batch", i32), ("len", i32), ("heads", i32), ("headdim", i32),
         ("nstate", i32), ("groups", i32), ("chunk_size", i32), ("io_dtype", i32),
-        ("dt_softplus", i32), ("d_has_p", i32), ("phase", i32), ("dt_mode", i32),
+        ("dt_softplus", i32), ("d_has_p", i32), ("phase", i32), ("reverse", i32),
         ("X", vp), ("dt", vp), ("A", fp), ("Bm", vp), ("Cm", vp), ("D", fp), ("z", vp), ("dt_bias", fp),
         ("initial_states", fp), ("Y", vp), ("final_states", fp),
         ("ws_dt", fp), ("ws_cum", fp), ("ws_state", fp), ("ws_state_in", vp), ("status", vp),
-        ("row_dots", fp), ("row_scale", fp), ("bc_width", i32), ("x_heads", i32),
+        ("row_dots", fp),
         ("ws_state_in_f32", fp), ("seq_table", vp), ("num_seqs", i32), ("num_chunks", i32),
     ]
 
 
 class SsdBwdArgs(C.Structure):
     _fields_ = [
-        ("batch", i32), ("len", i32), ("len_valid", i32), ("heads", i32),
-        ("headdim", i32), ("io_dtype", i32), ("d_has_p", i32), ("reserved0", i32),
-        ("gY", vp), ("z", vp), ("X", vp), ("y_plain", vp), ("dx_rev", vp), ("D", fp),
-        ("dy", vp), ("dy_rev", vp), ("dX", vp), ("dz", vp), ("dD", fp),
+        ("batch", i32), ("len", i32), ("heads", i32), ("headdim", i32), ("io_dtype", i32), ("d_has_p", i32),
+        ("gY", vp), ("z", vp), ("X", vp), ("y_plain", vp), ("dx", vp), ("D", fp), ("dy", vp), ("dX", vp), ("dz", vp), ("dD", fp),
     ]
 
 
@@ -179,10 +177,8 @@ ENTRY_POINTS = {
     "ssm_ssd_packed_scratch_bytes": (C.c_int64, [i32, i32, i32, C.POINTER(i64)]),
     "ssm_ssd_bwd_gate": (C.c_int, [C.POINTER(SsdBwdArgs), vp]),
     "ssm_ssd_bwd_finish": (C.c_int, [C.POINTER(SsdBwdArgs), vp]),
-    "ssm_time_flip": (C.c_int, [vp, vp, i32, i32, i32, C.c_int64, vp]),
-    "ssm_ssd_bwd_group_sum": (C.c_int, [vp, fp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp]),
-    "ssm_ssd_bwd_spread": (C.c_int, [vp, vp, C.c_int64, i32, i32, C.c_int64, vp]),
-    "ssm_ssd_state_dot": (C.c_int, [vp, vp, fp, i32, i32, i32, i32, i32, vp]),
+    "ssm_ssd_bwd_bc": (C.c_int, [vp, vp]),
+    "ssm_ssd_bwd_steps": (C.c_int, [vp, vp]),
     "ssm_ssd_fwd": (C.c_int, [C.POINTER(SsdArgs), vp]),
     "ssm_ssd_shard_summary_floats": (C.c_int64, [i32, i32]),
     "ssm_ssd_fold_shards": (C.c_int, [vp, i32, i32, i32, i32, vp, vp, vp]),

@@ -1,385 +1,249 @@
-// Element-wise and reduction kernels around the dual-form backward of the state-space-dual scan.
+// Element-wise passes and step-size bookkeeping of the dual-form backward of the state-space-dual scan.  The contractions run on
+// the tensor cores: the forward kernels, their mirror image in time (ssd_scan.cu) and the B / C gradients (ssd_bwd_bc.cu).
 //
-// The contractions of that backward pass run on the forward pass's tensor-core kernels (ssd_scan.cu) applied to
-// transformed operands: the time-reversed sequence for the adjoint recurrence, and the head / state axes exchanged for
-// dB and dC.  What is left is bandwidth work over (batch, len, heads, headdim) tensors, done here in as few passes as
-// the data flow allows:
+//   ssd_bwd_gate_kernel    dy = gY * silu(z)
+//   ssd_bwd_finish_kernel  dz = gY * (y + D x) * silu'(z);  dX = dx + D dy;  dD = sum dy x
+//   ssd_bwd_steps_kernel   ddt, dA, d dt_bias from the per-step dot products of the two scan passes
 //
-//   ssd_bwd_gate_kernel     dy = gY * silu(z)  (or gY), written in time order and time-reversed
-//   time_flip_kernel        rows of one (batch, len, row) tensor in reverse time order
-//   ssd_bwd_finish_kernel   dz = gY * (y + D x) * silu'(z);  dX = reversed(dX_adj) + D dy;  dD = sum dy x
-//   ssd_bwd_group_sum_kernel  per-head rows (batch, len, heads, 128) summed over the heads of a B / C group, optionally
-//                           read in reverse time order and weighted per (step, head)
-//   ssd_state_dot_kernel    <state before chunk c of one pass, state before chunk nchunks - c of the other>
-//
-// Every thread moves 16-byte units; rows are contiguous.
+// The first two move 16-byte units of (batch, len, heads * 64) rows, several steps' loads in flight per thread.
 #include <type_traits>
 
-#include "common.cuh"
+#include "ssd_common.cuh"
 
 namespace ssmb {
 
 constexpr int kUnit = 8;  // 16-bit elements per 16-byte unit
 
-// thread = one unit column of the (heads * headdim) row; grid.y = slices of the time axis; grid.z = batch
+// thread = one unit of a row, four units apart by the grid
 template <typename T>
-__global__ void __launch_bounds__(256) ssd_bwd_gate_kernel(const ssm_ssd_bwd_args a, int steps_per_block) {
-  const int units = a.heads * a.headdim / kUnit;
-  const int u = blockIdx.x * 256 + threadIdx.x;
-  if (u >= units) return;
-  const int b = blockIdx.z;
-  const int t_begin = blockIdx.y * steps_per_block;
-  const int t_end = min(t_begin + steps_per_block, a.len);
-  const int64_t row = (int64_t)a.heads * a.headdim;
-  const T* gy = reinterpret_cast<const T*>(a.gY);
-  const T* z = reinterpret_cast<const T*>(a.z);
-  T* dy = reinterpret_cast<T*>(a.dy);
-  T* dyr = reinterpret_cast<T*>(a.dy_rev);
-#pragma unroll 4
-  for (int t = t_begin; t < t_end; ++t) {
-    const int64_t at = ((int64_t)b * a.len + t) * row + (int64_t)u * kUnit;
-    const int64_t rt = ((int64_t)b * a.len + (a.len - 1 - t)) * row + (int64_t)u * kUnit;
-    Vec16<T> g;
-    float f[8];
-    if (t < a.len_valid) {
-      g.load_stream(gy + ((int64_t)b * a.len_valid + t) * row + (int64_t)u * kUnit);
-      if (z) {
-        Vec16<T> zz;
-        float zv[8];
-        zz.load(z + ((int64_t)b * a.len_valid + t) * row + (int64_t)u * kUnit);
-        g.unpack(f);
-        zz.unpack(zv);
+__global__ void __launch_bounds__(256) ssd_bwd_gate_kernel(const ssm_ssd_bwd_args a, int64_t units) {
+  constexpr int U = 4;
+  const uint4* gy = reinterpret_cast<const uint4*>(a.gY);
+  const uint4* z = reinterpret_cast<const uint4*>(a.z);
+  const int64_t i0 = (int64_t)blockIdx.x * (256 * U) + threadIdx.x;
+  uint4 gr[U], zr[U];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] *= silu_fast(zv[e]);
-        g.pack(f);
-      }
-    } else {
-      g.raw = make_uint4(0, 0, 0, 0);  // padding up to whole chunks
-    }
-    g.store(dy + at);
-    g.store(dyr + rt);
+  for (int k = 0; k < U; ++k) {
+    const int64_t i = i0 + k * 256 < units ? i0 + k * 256 : units - 1;
+    gr[k] = __ldg(gy + i), zr[k] = __ldg(z + i);
+  }
+#pragma unroll
+  for (int k = 0; k < U; ++k) {
+    Vec16<T> g, zz;
+    float f[8], zv[8];
+    g.raw = gr[k], zz.raw = zr[k];
+    g.unpack(f), zz.unpack(zv);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] *= silu_fast(zv[e]);
+    g.pack(f);
+    if (i0 + k * 256 < units) reinterpret_cast<uint4*>(a.dy)[i0 + k * 256] = g.raw;
   }
 }
 
-// dst[b, len - 1 - t, :] = src[b, t, :]; src has len_valid rows per batch element, the rest of dst's rows are zero
-__global__ void __launch_bounds__(256) time_flip_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int len, int len_valid, int row_units,
-                                                        int steps_per_block) {
-  const int u = blockIdx.x * 256 + threadIdx.x;
-  if (u >= row_units) return;
-  const int b = blockIdx.z;
-  const int t_begin = blockIdx.y * steps_per_block;
-  const int t_end = min(t_begin + steps_per_block, len);
-#pragma unroll 4
-  for (int t = t_begin; t < t_end; ++t) {
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (t < len_valid) v = __ldcs(src + ((int64_t)b * len_valid + t) * row_units + u);
-    dst[((int64_t)b * len + (len - 1 - t)) * row_units + u] = v;
-  }
-}
-
+// thread = one unit column of the (heads * 64) row, walking steps_per_block steps two at a time; grid.y = slices of the time axis
 template <typename T>
 __global__ void __launch_bounds__(256) ssd_bwd_finish_kernel(const ssm_ssd_bwd_args a, int steps_per_block) {
-  const int units = a.heads * a.headdim / kUnit;
-  const int u = blockIdx.x * 256 + threadIdx.x;
-  const bool live = u < units;
+  constexpr int U = 2;
+  const int units = a.heads * kP / kUnit;
+  const int u_raw = blockIdx.x * 256 + threadIdx.x;
+  const bool live = u_raw < units;
+  const int u = live ? u_raw : units - 1;
   const int b = blockIdx.z;
-  const int t_begin = blockIdx.y * steps_per_block;
-  const int t_end = min(t_begin + steps_per_block, a.len_valid);
-  const int64_t row = (int64_t)a.heads * a.headdim;
-  const int upr = a.headdim / kUnit;  // units per head
-  const int h = live ? u / upr : 0, p0 = (u % upr) * kUnit;
-  float Dv[8];
+  const int t_begin = blockIdx.y * steps_per_block, t_end = min(t_begin + steps_per_block, a.len);
+  const int64_t row = units;  // in units
+  const int h = u / (kP / kUnit), p0 = (u % (kP / kUnit)) * kUnit;
+  float Dv[8], acc[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) Dv[e] = !a.D ? 0.f : (a.d_has_p ? __ldg(a.D + h * a.headdim + p0 + e) : __ldg(a.D + h));
-  float acc[8];
+  for (int e = 0; e < 8; ++e) Dv[e] = !a.D ? 0.f : (a.d_has_p ? __ldg(a.D + h * kP + p0 + e) : __ldg(a.D + h)), acc[e] = 0.f;
+  const uint4 *gy = reinterpret_cast<const uint4*>(a.gY), *z = reinterpret_cast<const uint4*>(a.z), *X = reinterpret_cast<const uint4*>(a.X);
+  const uint4 *yp = reinterpret_cast<const uint4*>(a.y_plain), *dx = reinterpret_cast<const uint4*>(a.dx);
+  uint4 *dX = reinterpret_cast<uint4*>(a.dX), *dz = reinterpret_cast<uint4*>(a.dz);
+  auto unpack = [](const uint4& r, float (&f)[8]) {
+    Vec16<T> v;
+    v.raw = r;
+    v.unpack(f);
+  };
+  for (int t0 = t_begin; t0 < t_end; t0 += U) {
+    uint4 xr[U], dr[U], gr[U], zr[U], yr[U];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-  const T* gy = reinterpret_cast<const T*>(a.gY);
-  const T* z = reinterpret_cast<const T*>(a.z);
-  const T* X = reinterpret_cast<const T*>(a.X);
-  const T* yp = reinterpret_cast<const T*>(a.y_plain);
-  const T* dy = reinterpret_cast<const T*>(a.dy);
-  const T* dxr = reinterpret_cast<const T*>(a.dx_rev);
-  T* dX = reinterpret_cast<T*>(a.dX);
-  T* dz = reinterpret_cast<T*>(a.dz);
-  if (live) {
-#pragma unroll 2
-    for (int t = t_begin; t < t_end; ++t) {
-      const int64_t off = (int64_t)u * kUnit;
-      const int64_t at_v = ((int64_t)b * a.len_valid + t) * row + off;       // tensors of the caller (unpadded)
-      const int64_t at_p = ((int64_t)b * a.len + t) * row + off;             // padded work tensors
-      const int64_t rt_p = ((int64_t)b * a.len + (a.len - 1 - t)) * row + off;
-      Vec16<T> vx, vdy, vdx;
-      float x[8], d[8], g[8];
-      vx.load_stream(X + at_v);
-      vdy.load_stream(dy + at_p);
-      vdx.load_stream(dxr + rt_p);
-      vx.unpack(x);
-      vdy.unpack(d);
-      vdx.unpack(g);
+    for (int k = 0; k < U; ++k) {
+      const int64_t at = ((int64_t)b * a.len + min(t0 + k, t_end - 1)) * row + u;
+      xr[k] = __ldcs(X + at), dr[k] = __ldcs(dx + at), gr[k] = __ldcs(gy + at);
+      if (z) zr[k] = __ldcs(z + at), yr[k] = __ldcs(yp + at);
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (t0 + k >= t_end) break;
+      const int64_t at = ((int64_t)b * a.len + t0 + k) * row + u;
+      float x[8], g[8], o[8];
+      unpack(xr[k], x), unpack(gr[k], g), unpack(dr[k], o);
+      Vec16<T> v;
+      if (z) {
+        float zv[8], y[8], dzo[8];
+        unpack(zr[k], zv), unpack(yr[k], y);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float s = sigmoid_fast(zv[e]);
+          dzo[e] = g[e] * fmaf(Dv[e], x[e], y[e]) * (s * (1.f + zv[e] * (1.f - s)));
+          g[e] *= zv[e] * s;
+        }
+        v.pack(dzo);
+        if (live) __stcs(dz + at, v.raw);
+        v.pack(g), v.unpack(g);  // dy as the scan passes read it
+      }
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        acc[e] = fmaf(d[e], x[e], acc[e]);
-        g[e] = fmaf(Dv[e], d[e], g[e]);
+        acc[e] = fmaf(g[e], x[e], acc[e]);
+        o[e] = fmaf(Dv[e], g[e], o[e]);
       }
-      Vec16<T> o;
-      o.pack(g);
-      o.store_stream(dX + at_v);
-      if (z) {
-        Vec16<T> vg, vz, vy;
-        float gg[8], zv[8], y[8];
-        vg.load_stream(gy + at_v);
-        vz.load_stream(z + at_v);
-        vy.load_stream(yp + at_p);
-        vg.unpack(gg);
-        vz.unpack(zv);
-        vy.unpack(y);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) gg[e] *= fmaf(Dv[e], x[e], y[e]) * silu_grad_fast(zv[e]);
-        o.pack(gg);
-        o.store_stream(dz + at_v);
-      }
+      v.pack(o);
+      if (live) __stcs(dX + at, v.raw);
     }
   }
   if (!a.dD) return;
   if (a.d_has_p) {
     if (live) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) atomicAdd(a.dD + h * a.headdim + p0 + e, acc[e]);
+      for (int e = 0; e < 8; ++e) atomicAdd(a.dD + h * kP + p0 + e, acc[e]);
     }
-  } else {
-    // the units of one head are `upr` neighbouring lanes (headdim 64: 8 lanes): fold them, one atomic per head and warp
+  } else {  // the eight units of a head are neighbouring lanes
     float s = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) s += acc[e];
     if (!live) s = 0.f;
-    for (int off = 1; off < upr && off < 32; off <<= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (live && (u % upr == 0 || upr > 32)) atomicAdd(a.dD + h, s);
+    s = group_sum<8, 1>(s);
+    if (live && u % (kP / kUnit) == 0) atomicAdd(a.dD + h, s);
   }
 }
 
-// out[b, t, g, :] = sum over the heads h of group g of  w[b, t, h] * y[b, ts, h, :],  ts = t or len - 1 - t;  rows of 128 states
-template <typename T, typename TO>
-__global__ void __launch_bounds__(256) ssd_bwd_group_sum_kernel(const T* __restrict__ y, const float* __restrict__ w, TO* __restrict__ out, int batch,
-                                                                int len, int len_out, int heads, int groups, int nstate, int reversed) {
-  const int upr = nstate / kUnit;
-  const int64_t total = (int64_t)batch * len_out * groups * upr;
-  const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (idx >= total) return;
-  const int u = (int)(idx % upr);
-  const int g = (int)((idx / upr) % groups);
-  const int t = (int)((idx / ((int64_t)upr * groups)) % len_out);
-  const int b = (int)(idx / ((int64_t)upr * groups * len_out));
-  const int rep = heads / groups;
-  const int ts = reversed ? len - 1 - t : t;
-  float acc[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-  for (int r = 0; r < rep; ++r) {
-    const int h = g * rep + r;
-    Vec16<T> v;
-    float f[8];
-    v.load_stream(y + (((int64_t)b * len + ts) * heads + h) * nstate + (int64_t)u * kUnit);
-    v.unpack(f);
-    const float wt = w ? __ldg(w + ((int64_t)b * len + t) * heads + h) : 1.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = fmaf(wt, f[e], acc[e]);
-  }
-  TO* dst = out + (((int64_t)b * len_out + t) * groups + g) * nstate + (int64_t)u * kUnit;
-  if constexpr (std::is_same<TO, float>::value) {
-    *reinterpret_cast<float4*>(dst) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
-  } else {
-    Vec16<TO> o;
-    o.pack(acc);
-    o.store(dst);
-  }
-}
-
-// dst[r, h, :] = src[r, h / rep, :] for rows r = (batch, step): the rows of a B / C group handed to each of its heads
-__global__ void __launch_bounds__(256) ssd_bwd_spread_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int64_t rows, int heads, int rep,
-                                                             int units) {
-  const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (idx >= rows * heads * units) return;
-  const int u = (int)(idx % units);
-  const int h = (int)((idx / units) % heads);
-  const int64_t r = idx / ((int64_t)units * heads);
-  dst[idx] = __ldg(src + (r * (heads / rep) + h / rep) * units + u);
-}
-
-// one warp per (batch, chunk c >= 1, head): out[b, c, h] = <fwd[b, c, h, :], adj[b, nchunks - c, h, :]>; out[b, 0, h] = 0
+// One CTA per (batch, chunk, eight heads).  The per-step values are read as they lie in memory (heads innermost) and transposed through
+// shared memory; then a warp per head forms the product <state, adjoint> at the chunk's left boundary (fp32, 8192 terms each)
+// and the running sum of qd - u over the chunk's 256 steps, eight of them per lane.
+constexpr int kStepHeads = 8, kStepLd = kQ + 4;
 template <typename T>
-__global__ void __launch_bounds__(128) ssd_state_dot_kernel(const T* __restrict__ fwd, const T* __restrict__ adj, float* __restrict__ out, int batch,
-                                                            int nchunks, int heads, int elems) {
-  const int warp = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= batch * nchunks * heads) return;
-  const int h = warp % heads, c = (warp / heads) % nchunks, b = warp / (heads * nchunks);
-  float s = 0.f;
-  if (c > 0) {
-    const T* pa = fwd + (((int64_t)b * nchunks + c) * heads + h) * elems;
-    const T* pb = adj + (((int64_t)b * nchunks + (nchunks - c)) * heads + h) * elems;
-#pragma unroll 4
-    for (int i = lane * kUnit; i < elems; i += 32 * kUnit) {
-      Vec16<T> va, vb;
-      float fa[8], fb[8];
-      va.load_stream(pa + i);
-      vb.load_stream(pb + i);
-      va.unpack(fa);
-      vb.unpack(fb);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) s = fmaf(fa[e], fb[e], s);
+__global__ void __launch_bounds__(kQ) ssd_bwd_steps_kernel(const ssm_ssd_steps_args a, int nchunks) {
+  __shared__ __align__(16) float sPre[kStepHeads][kStepLd], sQ[kStepHeads][kStepLd], sR[kStepHeads][kStepLd];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h0 = blockIdx.x * kStepHeads, c = blockIdx.y, b = blockIdx.z, nh = min(kStepHeads, a.heads - h0);
+  const int t0 = c * kQ, steps = min(kQ, a.len - t0);
+  const T* dt = reinterpret_cast<const T*>(a.dt);
+  for (int i = tid; i < kQ * kStepHeads; i += kQ) {
+    const int t = i / kStepHeads, hh = i % kStepHeads;
+    float pre = 0.f, q = 0.f, r = 0.f;
+    if (t < steps && hh < nh) {
+      const int64_t at = ((int64_t)b * a.len + t0 + t) * a.heads + h0 + hh;
+      pre = to_f<T>(dt[at]) + (a.dt_bias ? __ldg(a.dt_bias + h0 + hh) : 0.f);
+      q = __ldg(a.qd + at), r = q - __ldg(a.u + at);
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    sPre[hh][t] = pre, sQ[hh][t] = q, sR[hh][t] = r;
   }
-  if (lane == 0) out[warp] = s;
+  __syncthreads();
+  if (warp < nh) {
+    const int h = h0 + warp;
+    const float Ah = __ldg(a.A + h);
+    float start = 0.f;
+    if (c > 0) {
+      const float4* s = reinterpret_cast<const float4*>(a.state_f32 + (((int64_t)b * nchunks + c) * a.heads + h) * (kP * kN));
+      const float4* g = reinterpret_cast<const float4*>(a.adjoint_f32 + (((int64_t)b * nchunks + c - 1) * a.heads + h) * (kP * kN));
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+      for (int i = lane; i < kP * kN / 4; i += 32) {
+        const float4 x = __ldcs(s + i), y = __ldcs(g + i);
+        acc.x = fmaf(x.x, y.x, acc.x), acc.y = fmaf(x.y, y.y, acc.y), acc.z = fmaf(x.z, y.z, acc.z), acc.w = fmaf(x.w, y.w, acc.w);
+      }
+      start = warp_sum((acc.x + acc.y) + (acc.z + acc.w)) * ex2_approx(__ldg(a.ws_cum + (((int64_t)b * a.heads + h) * nchunks + c) * kQ));
+    } else if (a.start0) {
+      start = __ldg(a.start0 + b * a.heads + h);
+    }
+    float r[8], run = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) r[k] = sR[warp][lane * 8 + k], run += r[k];
+    float incl = run;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const float o = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += o;
+    }
+    float da = start + (incl - run), dA = 0.f, db = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int t = lane * 8 + k;
+      const float pre = sPre[warp][t], delta = a.dt_softplus ? softplus_f(pre) : pre;
+      float d = (delta > 0.f ? sQ[warp][t] / delta : 0.f) + Ah * da;
+      if (a.dt_softplus) d *= sigmoid_f(pre);
+      if (t < steps) dA = fmaf(delta, da, dA), db += d;
+      sR[warp][t] = d;
+      da += r[k];
+    }
+    dA = warp_sum(dA), db = warp_sum(db);
+    if (lane == 0) {
+      atomicAdd(a.dA + h, dA);
+      if (a.ddt_bias) atomicAdd(a.ddt_bias + h, db);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < steps * kStepHeads; i += kQ) {
+    const int t = i / kStepHeads, hh = i % kStepHeads;
+    if (hh < nh) reinterpret_cast<T*>(a.ddt)[((int64_t)b * a.len + t0 + t) * a.heads + h0 + hh] = from_f<T>(sR[hh][t]);
+  }
 }
 
-static int bwd_common_checks(const ssm_ssd_bwd_args* a, const char* what) {
+static int bwd_common_checks(const ssm_ssd_bwd_args* a) {
   SSM_REQUIRE(a != nullptr, SSM_ERR_NULL, "ssd backward: args is NULL");
-  SSM_REQUIRE(a->batch >= 0 && a->len >= 0 && a->len_valid >= 0 && a->len_valid <= a->len && a->heads >= 1 && a->headdim >= kUnit &&
-                  a->headdim % kUnit == 0,
-              SSM_ERR_SHAPE, "ssd backward: bad shape");
+  SSM_REQUIRE(a->batch >= 0 && a->len >= 0 && a->heads >= 1 && a->headdim == kP, SSM_ERR_SHAPE, "ssd backward: bad shape");
   SSM_REQUIRE(a->io_dtype == SSM_BF16 || a->io_dtype == SSM_F16, SSM_ERR_DTYPE, "ssd backward: operands must be bf16 or fp16");
-  SSM_REQUIRE((int64_t)a->batch <= 65535, SSM_ERR_TOO_LARGE, "ssd backward: batch too large for one launch");
-  (void)what;
+  SSM_REQUIRE(a->batch <= 65535, SSM_ERR_TOO_LARGE, "ssd backward: batch too large for one launch");
   return SSM_OK;
-}
-
-__global__ void __launch_bounds__(128) ssd_state_dot_f32_kernel(const float* __restrict__ fwd, const float* __restrict__ adj, float* __restrict__ out,
-                                                                int batch, int nchunks, int heads, int elems) {
-  const int warp = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= batch * nchunks * heads) return;
-  const int h = warp % heads, c = (warp / heads) % nchunks, b = warp / (heads * nchunks);
-  float s = 0.f;
-  if (c > 0) {
-    const float4* pa = reinterpret_cast<const float4*>(fwd + (((int64_t)b * nchunks + c) * heads + h) * elems);
-    const float4* pb = reinterpret_cast<const float4*>(adj + (((int64_t)b * nchunks + (nchunks - c)) * heads + h) * elems);
-    float s4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int i = lane; i < elems / 4; i += 32) {
-      const float4 x = __ldcs(pa + i), y = __ldcs(pb + i);
-      s4[0] = fmaf(x.x, y.x, s4[0]), s4[1] = fmaf(x.y, y.y, s4[1]), s4[2] = fmaf(x.z, y.z, s4[2]), s4[3] = fmaf(x.w, y.w, s4[3]);
-    }
-    s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  }
-  if (lane == 0) out[warp] = s;
 }
 
 }  // namespace ssmb
 
 using namespace ssmb;
 
-constexpr int kStepsPerBlock = 64;
-
 extern "C" int ssm_ssd_bwd_gate(const ssm_ssd_bwd_args* a, ssm_stream_t stream) {
-  if (int rc = bwd_common_checks(a, "gate")) return rc;
+  if (int rc = bwd_common_checks(a)) return rc;
   if (a->batch == 0 || a->len == 0) return SSM_OK;
-  SSM_REQUIRE(a->gY && a->dy && a->dy_rev, SSM_ERR_NULL, "ssd_bwd_gate: missing tensor");
-  SSM_REQUIRE(aligned_to(a->gY, 16) && aligned_to(a->dy, 16) && aligned_to(a->dy_rev, 16) && (!a->z || aligned_to(a->z, 16)), SSM_ERR_ALIGN,
-              "ssd_bwd_gate: tensors must be 16-byte aligned");
-  const int units = a->heads * a->headdim / kUnit;
-  const dim3 grid((units + 255) / 256, (a->len + kStepsPerBlock - 1) / kStepsPerBlock, a->batch);
-  SSM_REQUIRE(grid.y <= 65535, SSM_ERR_TOO_LARGE, "ssd_bwd_gate: sequence too long for one launch");
+  SSM_REQUIRE(a->gY && a->z && a->dy, SSM_ERR_NULL, "ssd_bwd_gate: missing tensor");
+  SSM_REQUIRE(aligned_to(a->gY, 16) && aligned_to(a->dy, 16) && aligned_to(a->z, 16), SSM_ERR_ALIGN, "ssd_bwd_gate: tensors must be 16-byte aligned");
+  const int64_t units = (int64_t)a->batch * a->len * a->heads * kP / kUnit, grid = (units + 1023) / 1024;
+  SSM_REQUIRE(grid < (1ll << 31), SSM_ERR_TOO_LARGE, "ssd_bwd_gate: too large for one launch");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (a->io_dtype == SSM_BF16) ssd_bwd_gate_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*a, kStepsPerBlock);
-  else ssd_bwd_gate_kernel<__half><<<grid, 256, 0, st>>>(*a, kStepsPerBlock);
+  if (a->io_dtype == SSM_BF16) ssd_bwd_gate_kernel<__nv_bfloat16><<<(unsigned)grid, 256, 0, st>>>(*a, units);
+  else ssd_bwd_gate_kernel<__half><<<(unsigned)grid, 256, 0, st>>>(*a, units);
   return launch_status("ssd_bwd_gate_kernel");
 }
 
 extern "C" int ssm_ssd_bwd_finish(const ssm_ssd_bwd_args* a, ssm_stream_t stream) {
-  if (int rc = bwd_common_checks(a, "finish")) return rc;
-  if (a->batch == 0 || a->len_valid == 0) return SSM_OK;
-  SSM_REQUIRE(a->X && a->dy && a->dx_rev && a->dX, SSM_ERR_NULL, "ssd_bwd_finish: missing tensor");
-  SSM_REQUIRE(!a->z || (a->gY && a->y_plain && a->dz), SSM_ERR_NULL, "ssd_bwd_finish: a gate needs gY, y_plain and dz");
-  SSM_REQUIRE(aligned_to(a->X, 16) && aligned_to(a->dy, 16) && aligned_to(a->dx_rev, 16) && aligned_to(a->dX, 16) && (!a->z || aligned_to(a->z, 16)) &&
-                  (!a->gY || aligned_to(a->gY, 16)) && (!a->y_plain || aligned_to(a->y_plain, 16)) && (!a->dz || aligned_to(a->dz, 16)),
+  if (int rc = bwd_common_checks(a)) return rc;
+  if (a->batch == 0 || a->len == 0) return SSM_OK;
+  SSM_REQUIRE(a->X && a->gY && a->dx && a->dX && (!a->z || (a->y_plain && a->dz)), SSM_ERR_NULL, "ssd_bwd_finish: missing tensor");
+  SSM_REQUIRE(aligned_to(a->X, 16) && aligned_to(a->gY, 16) && aligned_to(a->dx, 16) && aligned_to(a->dX, 16) && aligned_to(a->z, 16) && aligned_to(a->y_plain, 16) &&
+                  aligned_to(a->dz, 16),
               SSM_ERR_ALIGN, "ssd_bwd_finish: tensors must be 16-byte aligned");
-  const int units = a->heads * a->headdim / kUnit;
-  const dim3 grid((units + 255) / 256, (a->len_valid + kStepsPerBlock - 1) / kStepsPerBlock, a->batch);
-  SSM_REQUIRE(grid.y <= 65535, SSM_ERR_TOO_LARGE, "ssd_bwd_finish: sequence too long for one launch");
+  // steps per CTA: long enough that dD costs few additions, short enough to fill the GPU a few times
+  const int units = a->heads * kP / kUnit, gx = (units + 255) / 256;
+  int spb = 64;
+  while (spb > 8 && (int64_t)gx * a->batch * ((a->len + spb - 1) / spb) < 4ll * sm_count()) spb /= 2;
+  while ((a->len + spb - 1) / spb > 65535) spb *= 2;
+  const dim3 grid(gx, (a->len + spb - 1) / spb, a->batch);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (a->io_dtype == SSM_BF16) ssd_bwd_finish_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*a, kStepsPerBlock);
-  else ssd_bwd_finish_kernel<__half><<<grid, 256, 0, st>>>(*a, kStepsPerBlock);
+  if (a->io_dtype == SSM_BF16) ssd_bwd_finish_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*a, spb);
+  else ssd_bwd_finish_kernel<__half><<<grid, 256, 0, st>>>(*a, spb);
   return launch_status("ssd_bwd_finish_kernel");
 }
 
-extern "C" int ssm_time_flip(const void* src, void* dst, int32_t batch, int32_t len, int32_t len_valid, int64_t row_bytes, ssm_stream_t stream) {
-  SSM_REQUIRE(batch >= 0 && len >= 0 && len_valid >= 0 && len_valid <= len && row_bytes >= 0, SSM_ERR_SHAPE, "time_flip: bad shape");
-  if (batch == 0 || len == 0 || row_bytes == 0) return SSM_OK;
-  SSM_REQUIRE(src && dst, SSM_ERR_NULL, "time_flip: missing tensor");
-  SSM_REQUIRE(row_bytes % 16 == 0 && aligned_to(src, 16) && aligned_to(dst, 16), SSM_ERR_ALIGN, "time_flip: rows must be whole 16-byte units");
-  SSM_REQUIRE(batch <= 65535 && row_bytes / 16 < (1ll << 31), SSM_ERR_TOO_LARGE, "time_flip: too large for one launch");
-  const int units = (int)(row_bytes / 16);
-  const int spb = units >= 256 ? 16 : 64;
-  const dim3 grid((units + 255) / 256, (len + spb - 1) / spb, batch);
-  SSM_REQUIRE(grid.y <= 65535, SSM_ERR_TOO_LARGE, "time_flip: sequence too long for one launch");
-  time_flip_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<const uint4*>(src), reinterpret_cast<uint4*>(dst), len, len_valid,
-                                                                            units, spb);
-  return launch_status("time_flip_kernel");
-}
-
-extern "C" int ssm_ssd_bwd_group_sum(const void* y, const float* weight, void* out, int32_t batch, int32_t len, int32_t len_out, int32_t heads,
-                                     int32_t groups, int32_t nstate, int32_t reversed, int32_t io_dtype, int32_t out_dtype, ssm_stream_t stream) {
-  SSM_REQUIRE(batch >= 0 && len >= 0 && len_out >= 0 && len_out <= len && heads >= 1 && groups >= 1 && heads % groups == 0 && nstate >= kUnit &&
-                  nstate % kUnit == 0,
-              SSM_ERR_SHAPE, "ssd_bwd_group_sum: bad shape");
-  SSM_REQUIRE(io_dtype == SSM_BF16 || io_dtype == SSM_F16, SSM_ERR_DTYPE, "ssd_bwd_group_sum: rows must be bf16 or fp16");
-  SSM_REQUIRE(out_dtype == io_dtype || out_dtype == SSM_F32, SSM_ERR_DTYPE, "ssd_bwd_group_sum: the sum is written in the rows' dtype or fp32");
-  if (batch == 0 || len_out == 0) return SSM_OK;
-  SSM_REQUIRE(y && out, SSM_ERR_NULL, "ssd_bwd_group_sum: missing tensor");
-  SSM_REQUIRE(aligned_to(y, 16) && aligned_to(out, 16), SSM_ERR_ALIGN, "ssd_bwd_group_sum: tensors must be 16-byte aligned");
-  const int64_t total = (int64_t)batch * len_out * groups * (nstate / kUnit);
-  SSM_REQUIRE((total + 255) / 256 < (1ll << 31), SSM_ERR_TOO_LARGE, "ssd_bwd_group_sum: too large for one launch");
-  const unsigned grid = (unsigned)((total + 255) / 256);
+extern "C" int ssm_ssd_bwd_steps(const ssm_ssd_steps_args* a, ssm_stream_t stream) {
+  SSM_REQUIRE(a != nullptr, SSM_ERR_NULL, "ssd_bwd_steps: args is NULL");
+  SSM_REQUIRE(a->batch >= 0 && a->len >= 0 && a->heads >= 1, SSM_ERR_SHAPE, "ssd_bwd_steps: bad shape");
+  SSM_REQUIRE(a->io_dtype == SSM_BF16 || a->io_dtype == SSM_F16, SSM_ERR_DTYPE, "ssd_bwd_steps: dt must be bf16 or fp16");
+  if (a->batch == 0 || a->len == 0) return SSM_OK;
+  SSM_REQUIRE(a->dt && a->A && a->u && a->qd && a->ws_cum && a->state_f32 && a->adjoint_f32 && a->ddt && a->dA, SSM_ERR_NULL, "ssd_bwd_steps: missing tensor");
+  SSM_REQUIRE(aligned_to(a->state_f32, 16) && aligned_to(a->adjoint_f32, 16), SSM_ERR_ALIGN, "ssd_bwd_steps: states must be 16-byte aligned");
+  const int64_t nchunks = (a->len + kQ - 1) / kQ;
+  SSM_REQUIRE(nchunks <= 65535 && a->batch <= 65535, SSM_ERR_TOO_LARGE, "ssd_bwd_steps: too large for one launch");
+  const dim3 grid((a->heads + kStepHeads - 1) / kStepHeads, (unsigned)nchunks, a->batch);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-#define SSM_GS(T, TO) \
-  ssd_bwd_group_sum_kernel<T, TO><<<grid, 256, 0, st>>>(reinterpret_cast<const T*>(y), weight, reinterpret_cast<TO*>(out), batch, len, len_out, heads, \
-                                                        groups, nstate, reversed)
-  if (io_dtype == SSM_BF16) {
-    if (out_dtype == SSM_F32) SSM_GS(__nv_bfloat16, float);
-    else SSM_GS(__nv_bfloat16, __nv_bfloat16);
-  } else {
-    if (out_dtype == SSM_F32) SSM_GS(__half, float);
-    else SSM_GS(__half, __half);
-  }
-#undef SSM_GS
-  return launch_status("ssd_bwd_group_sum_kernel");
-}
-
-extern "C" int ssm_ssd_bwd_spread(const void* src, void* dst, int64_t rows, int32_t heads, int32_t groups, int64_t row_bytes, ssm_stream_t stream) {
-  SSM_REQUIRE(rows >= 0 && heads >= 1 && groups >= 1 && heads % groups == 0 && row_bytes >= 0, SSM_ERR_SHAPE, "ssd_bwd_spread: bad shape");
-  if (rows == 0 || row_bytes == 0) return SSM_OK;
-  SSM_REQUIRE(src && dst, SSM_ERR_NULL, "ssd_bwd_spread: missing tensor");
-  SSM_REQUIRE(row_bytes % 16 == 0 && aligned_to(src, 16) && aligned_to(dst, 16), SSM_ERR_ALIGN, "ssd_bwd_spread: rows must be whole 16-byte units");
-  const int64_t total = rows * heads * (row_bytes / 16);
-  SSM_REQUIRE((total + 255) / 256 < (1ll << 31), SSM_ERR_TOO_LARGE, "ssd_bwd_spread: too large for one launch");
-  ssd_bwd_spread_kernel<<<(unsigned)((total + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const uint4*>(src), reinterpret_cast<uint4*>(dst), rows, heads, heads / groups, (int)(row_bytes / 16));
-  return launch_status("ssd_bwd_spread_kernel");
-}
-
-extern "C" int ssm_ssd_state_dot(const void* fwd_states, const void* adj_states, float* out, int32_t batch, int32_t nchunks, int32_t heads, int32_t elems,
-                                 int32_t io_dtype, ssm_stream_t stream) {
-  SSM_REQUIRE(batch >= 0 && nchunks >= 0 && heads >= 1 && elems >= 0 && elems % (32 * kUnit) == 0, SSM_ERR_SHAPE, "ssd_state_dot: bad shape");
-  SSM_REQUIRE(io_dtype == SSM_BF16 || io_dtype == SSM_F16 || io_dtype == SSM_F32, SSM_ERR_DTYPE, "ssd_state_dot: states must be bf16, fp16 or fp32");
-  if (batch == 0 || nchunks == 0) return SSM_OK;
-  SSM_REQUIRE(fwd_states && adj_states && out, SSM_ERR_NULL, "ssd_state_dot: missing tensor");
-  SSM_REQUIRE(aligned_to(fwd_states, 16) && aligned_to(adj_states, 16), SSM_ERR_ALIGN, "ssd_state_dot: tensors must be 16-byte aligned");
-  const int64_t warps = (int64_t)batch * nchunks * heads;
-  SSM_REQUIRE(warps < (1ll << 28), SSM_ERR_TOO_LARGE, "ssd_state_dot: too large for one launch");
-  const unsigned grid = (unsigned)((warps * 32 + 127) / 128);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (io_dtype == SSM_F32)
-    ssd_state_dot_f32_kernel<<<grid, 128, 0, st>>>(reinterpret_cast<const float*>(fwd_states), reinterpret_cast<const float*>(adj_states), out, batch, nchunks,
-                                                   heads, elems);
-  else if (io_dtype == SSM_BF16)
-    ssd_state_dot_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(fwd_states),
-                                                              reinterpret_cast<const __nv_bfloat16*>(adj_states), out, batch, nchunks, heads, elems);
-  else
-    ssd_state_dot_kernel<__half><<<grid, 128, 0, st>>>(reinterpret_cast<const __half*>(fwd_states), reinterpret_cast<const __half*>(adj_states), out, batch,
-                                                       nchunks, heads, elems);
-  return launch_status("ssd_state_dot_kernel");
+  if (a->io_dtype == SSM_BF16) ssd_bwd_steps_kernel<__nv_bfloat16><<<grid, kQ, 0, st>>>(*a, (int)nchunks);
+  else ssd_bwd_steps_kernel<__half><<<grid, kQ, 0, st>>>(*a, (int)nchunks);
+  return launch_status("ssd_bwd_steps_kernel");
 }

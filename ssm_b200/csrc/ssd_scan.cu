@@ -20,19 +20,9 @@
 //
 // Exponent differences are always formed before exp2 (never exp2(c_i) / exp2(c_j)), so long
 // sequences stay finite.  Every wait on an mbarrier is bounded and reports through the status word.
-#include <cuda.h>
-
-#include <type_traits>
-
-#include "common.cuh"
-#include "tc05.cuh"
+#include "ssd_common.cuh"
 
 namespace ssmb {
-
-constexpr int kQ = 256;    // chunk length
-constexpr int kP = 64;     // head dimension
-constexpr int kN = 128;    // state dimension
-constexpr int kBlk = 128;  // rows per scan CTA
 
 // floats of the shard summary (final state, then total log-decay), rounded up to whole 256-byte lines
 __host__ __device__ inline int64_t ssd_summary_floats_padded(int batch, int heads) {
@@ -61,10 +51,7 @@ __global__ void __launch_bounds__(kQ) ssd_cumsum_kernel(const ssm_ssd_args a, in
     const int t = chunk_begin(a, c) + tid;
     if (t < chunk_limit(a, c)) {
       const int64_t at = ((int64_t)b * a.len + t) * a.heads + h0;
-      if (a.dt_mode & 1) {  // fp32 step sizes, already activated
-        const float* p = reinterpret_cast<const float*>(a.dt) + at;
-        for (int hh = 0; hh < nh; ++hh) sD[hh * kCumLd + tid] = __ldg(p + hh);
-      } else {
+      {
         const T* p = reinterpret_cast<const T*>(a.dt) + at;
         if (nh == kCumHeads && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
 #pragma unroll
@@ -120,9 +107,8 @@ __global__ void __launch_bounds__(kQ) ssd_cumsum_kernel(const ssm_ssd_args a, in
       acc += d[k] * Ah;
       const float c2 = acc * kLog2e;
       oc[k] = c2;                      // running decay exponent, base 2
-      // the same with delta folded in: exp2(x - odt[j]) = exp2(x - c2_j) * delta_j  (delta 0 -> +inf -> weight 0);
-      // dt_mode & 2: the inputs enter with unit weight, only the decay uses delta
-      od[k] = (a.dt_mode & 2) ? c2 : c2 - lg2_approx(d[k]);
+      // the same with delta folded in: exp2(x - odt[j]) = exp2(x - c2_j) * delta_j  (delta 0 -> +inf -> weight 0)
+      od[k] = c2 - lg2_approx(d[k]);
     }
     reinterpret_cast<float4*>(ocum)[0] = make_float4(oc[0], oc[1], oc[2], oc[3]);
     reinterpret_cast<float4*>(ocum)[1] = make_float4(oc[4], oc[5], oc[6], oc[7]);
@@ -176,7 +162,10 @@ constexpr int kStateComputeThreads = 256;
 constexpr int kStateThreads = kStateComputeThreads + 64;
 constexpr int kStateCopyWarp = 8, kStateMmaWarp = 9;
 
-template <typename T, int HPC>
+// REV: the adjoint recurrence.  The chunks are walked from the last to the first with dy, C and B in the places of x, B and C; the
+// local sum is taken to a chunk's first step, sum_i exp2(c_i - c_0) C_i dy_i^T, and what is handed out is the adjoint that enters a
+// chunk from the right (the adjoint state at the next chunk's first step; the decay of that step belongs to the walk).
+template <typename T, int HPC, bool REV>
 __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_kernel(const ssm_ssd_args a, const __grid_constant__ StateMaps maps, int nchunks) {
   using M = StateSmem<HPC>;
   constexpr int kStep = M::kStep, NS = M::NSTAGE;
@@ -224,24 +213,27 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
 
   const int64_t vrow0 = (((int64_t)b * a.heads + h0) * nchunks + c_off) * kQ;  // exponent vectors of head h0 (next head: + nchunks * kQ)
   const int nst = SPC * nwalk;
+  auto chunk_of = [&](int c) { return REV ? nwalk - 1 - c : c; };  // c-th chunk of the walk
   // stage s = steps [s * 64, s * 64 + 64), issued by one thread: two boxes of B, one box of x per head, and with a
   // chunk's first stage the exponent vectors of its heads.  Steps beyond the sequence read as zero.
   auto copy_stage = [&](int s) {
     const uint32_t base = tc::smem_u32(smraw + (s % NS) * M::STAGE);
     const uint32_t full = tc::smem_u32(&mbar_full[s % NS]);
     const bool first = s % SPC == 0;
-    tc::mbar_expect_tx(full, M::STAGE + (first ? HPC * kQ * 4 + M::LAST_BYTES : 0));
-    tc::tma_load_4d(base, &maps.b, full, 0, g, t_off + s * kStep, b);
-    tc::tma_load_4d(base + M::BLK_BYTES, &maps.b, full, 64, g, t_off + s * kStep, b);
+    const int t = t_off + chunk_of(s / SPC) * kQ + (s % SPC) * kStep;
+    tc::mbar_expect_tx(full, M::STAGE + (first ? HPC * kQ * 4 + (REV ? 0 : M::LAST_BYTES) : 0));
+    tc::tma_load_4d(base, &maps.b, full, 0, g, t, b);
+    tc::tma_load_4d(base + M::BLK_BYTES, &maps.b, full, 64, g, t, b);
 #pragma unroll
     for (int hh = 0; hh < HPC; ++hh)
-      tc::tma_load_4d(base + M::A_BYTES + hh * M::BLK_BYTES, &maps.x, full, 0, a.x_heads ? (h0 + hh) % a.x_heads : h0 + hh, t_off + s * kStep, b);
+      tc::tma_load_4d(base + M::A_BYTES + hh * M::BLK_BYTES, &maps.x, full, 0, h0 + hh, t, b);
     if (first) {
       const int c = s / SPC;
 #pragma unroll
       for (int hh = 0; hh < HPC; ++hh) {
-        tc::bulk_load(tc::smem_u32(sVec + ((c % M::NVEC) * HPC + hh) * kQ), a.ws_dt + vrow0 + ((int64_t)hh * nchunks + c) * kQ, kQ * 4, full);
-        tc::bulk_load(tc::smem_u32(sLast + ((c % M::NVEC) * HPC + hh) * 4), a.ws_cum + vrow0 + ((int64_t)hh * nchunks + c) * kQ + kQ - 4, 16, full);
+        const int64_t at = vrow0 + ((int64_t)hh * nchunks + chunk_of(c)) * kQ;
+        tc::bulk_load(tc::smem_u32(sVec + ((c % M::NVEC) * HPC + hh) * kQ), (REV ? a.ws_cum : a.ws_dt) + at, kQ * 4, full);
+        if (!REV) tc::bulk_load(tc::smem_u32(sLast + ((c % M::NVEC) * HPC + hh) * 4), a.ws_cum + at + kQ - 4, 16, full);
       }
     }
   };
@@ -299,7 +291,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
   auto emit_state_in = [&](int c) {
 #pragma unroll
     for (int hh = 0; hh < HPC; ++hh) {
-      T* blk = sin + (((int64_t)b * nchunks + c_off + c) * a.heads + h0 + hh) * (int64_t)(kP * kN);
+      T* blk = sin + (((int64_t)b * nchunks + c_off + chunk_of(c)) * a.heads + h0 + hh) * (int64_t)(kP * kN);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         Vec16<T> o;
@@ -307,7 +299,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
         *reinterpret_cast<uint4*>(blk + ((size_t)(wg * 4 + q) * kN + n) * 8) = o.raw;
       }
       if (a.ws_state_in_f32) {  // the same tile unrounded (the backward pass forms <adjoint state, state> from it)
-        float* blk32 = a.ws_state_in_f32 + (((int64_t)b * nchunks + c_off + c) * a.heads + h0 + hh) * (int64_t)(kP * kN);
+        float* blk32 = a.ws_state_in_f32 + (((int64_t)b * nchunks + c_off + chunk_of(c)) * a.heads + h0 + hh) * (int64_t)(kP * kN);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           float4* dst = reinterpret_cast<float4*>(blk32 + ((size_t)(wg * 4 + q) * kN + n) * 8);
@@ -321,6 +313,9 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
   float clast[HPC], clast_prev[HPC], ctot[HPC];
 #pragma unroll
   for (int hh = 0; hh < HPC; ++hh) clast[hh] = 0.f, clast_prev[hh] = 0.f, ctot[hh] = 0.f;
+  float cfirst[HPC];  // REV: the running exponent at the current chunk's first step
+#pragma unroll
+  for (int hh = 0; hh < HPC; ++hh) cfirst[hh] = 0.f;
   // fold chunk c's finished accumulators into the running states
   auto fold_chunk = [&](int c, const float (&cl)[HPC]) -> bool {
     const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&mbar_acc[c & 1]), (c >> 1) & 1));
@@ -353,10 +348,16 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
 #pragma unroll
       for (int hh = 0; hh < HPC; ++hh) {
         clast_prev[hh] = clast[hh];
-        clast[hh] = sLast[((c % M::NVEC) * HPC + hh) * 4 + 3];
+        if (REV) {  // from the first step of the chunk to its right, which was walked before, down to this one's
+          const float* v = sVec + ((c % M::NVEC) * HPC + hh) * kQ;
+          clast[hh] = v[kQ - 1] - v[0] + cfirst[hh];
+          cfirst[hh] = v[0];
+        } else {
+          clast[hh] = sLast[((c % M::NVEC) * HPC + hh) * 4 + 3];
+        }
         // exponent (base 2) of the decay from the start of the sequence to the start of this chunk: what a state
         // that arrives later (phase 2 of a sequence shard) is multiplied by before it joins this chunk's state
-        if (tid == 0 && !packed) a.ws_state[ssd_summary_floats_padded(a.batch, a.heads) + ((int64_t)b * a.heads + h0 + hh) * nchunks + c] = ctot[hh];
+        if (tid == 0 && !packed && !REV) a.ws_state[ssd_summary_floats_padded(a.batch, a.heads) + ((int64_t)b * a.heads + h0 + hh) * nchunks + c] = ctot[hh];
         ctot[hh] += clast[hh];
       }
     }
@@ -370,7 +371,7 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
 #pragma unroll
       for (int k = 0; k < M::BLK_BYTES / 16 / 256; ++k) {
         const int u = tid + 256 * k;  // 16-byte unit of this head's tile; 8 units per step
-        const float w = ex2_approx(c_last - vcp[u >> 3]);  // 0 for steps beyond the sequence
+        const float w = REV ? ex2_approx(vcp[u >> 3] - cfirst[hh]) : ex2_approx(c_last - vcp[u >> 3]);  // 0 for steps beyond the sequence
         unsigned char* px = base + M::A_BYTES + hh * M::BLK_BYTES + (size_t)u * 16;
         Vec16<T> v;
         v.raw = *reinterpret_cast<const uint4*>(px);
@@ -501,12 +502,6 @@ constexpr int kScanThreads = 512;
 constexpr int kScanWG = kScanThreads / 128;  // warpgroups: each owns every kScanWG-th 32-step column chunk of the mask and kP / kScanWG output columns
 constexpr int kEC = kP / kScanWG;             // epilogue columns per thread
 constexpr int kEU = kEC / 8;                  // ... in 16-byte units
-// Thread that issues the bulk copies (TMA): lane 0 of the warp with the least mask work (rows 0..31 of the block, odd
-// chunks), so that its issue time hides behind the other warps' mask stage; thread 0 issues the MMAs.
-constexpr int kCopyThread = 128;
-// Issues the per-head MMAs: lane 0 of the warp with the least mask work (rows 0..31 of the block, last column slice).
-constexpr int kMmaWarp = 12;
-
 // tensor maps of one call: x (box of 128 or 256 steps), z and y (boxes of 128 rows); rank 4 (p, head, step, batch)
 struct ScanMaps {
   CUtensorMap x0, x1, z, y;
@@ -516,12 +511,20 @@ struct ScanMaps {
 // Body for row block MB (0: rows 0..127, steps 0..127; 1: rows 128..255, steps 0..255).  XSKIP: the skip term D x is added
 // in the epilogue (a weight per channel, or the row sums of the backward pass are wanted), which carries each thread's x row
 // from one iteration to the next; without it a weight per head rides on the diagonal of the masked operand.
-template <typename T, int MB, bool XSKIP>
+// REV: the adjoint pass, dx_j = dt_j (sum_{i >= j} exp2(c_i - c_j) (B_j . C_i) dy_i + exp2(off - c_j) G B_j), with B, C and dy in the places of C, B
+// and x, and G the adjoint that enters the chunk from the right (off: the decay of the chunk and of the step after it).  It is the
+// mirror image in time: columns at or after the row's step, the long block is rows 0..127.
+template <typename T, int MB, bool XSKIP, bool REV>
 __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanMaps& maps, int nchunks, int hpc, int nparts, unsigned char* smraw,
                                               uint64_t* mbar, uint32_t* tmem_slot) {
   using M = ScanSmem<T>;
   constexpr int KJ = (MB + 1) * kBlk;  // steps that can reach this block's rows
   constexpr int NCH = KJ / (32 * kScanWG);  // 32-step column chunks per thread (the warpgroups interleave chunks)
+  constexpr int ROW0 = (REV ? 1 - MB : MB) * kBlk;  // first row and first column of the block within the chunk
+  constexpr int COL0 = REV ? ROW0 : 0;
+  constexpr int VLEN = REV ? kQ : KJ;               // exponents of the chunk that are needed
+  constexpr int kCopyThread = REV ? 224 : 128;      // lane 0 of a warp with little mask work (fewest unmasked columns)
+  constexpr int kMmaWarp = REV ? 3 : 12;
   unsigned char* sC = smraw;
   unsigned char* sBA = sC + M::C_BYTES;
   unsigned char* sX = sBA + M::B_BYTES;        // two buffers
@@ -552,12 +555,13 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   const int t0 = chunk_begin(a, c);
   // rows of this block that exist; a ragged block of a packed sequence stores its rows by hand (what follows them belongs to
   // the next sequence), everything else leaves through TMA, which cuts at the end of the tensor
-  const int t_live = chunk_limit(a, c) - t0 - MB * kBlk;
+  const int t_live = chunk_limit(a, c) - t0 - ROW0;
   const bool ragged = a.seq_table != nullptr && t_live < kBlk;
   if (ragged && t_live <= 0) return;  // the whole CTA: nothing has been issued yet
   const int i_loc = (warp & 3) * 32 + lane;    // row within the block = TMEM lane
-  const int i_chunk = MB * kBlk + i_loc;       // row within the chunk
-  const int rc = MB * 4 + (warp & 3);          // this warp's rows as a 32-step chunk index
+  const int i_chunk = ROW0 + i_loc;            // row within the chunk
+  const int rc = (ROW0 - COL0) / 32 + (warp & 3);  // this warp's rows as a 32-step chunk index, counted like the columns
+  auto reached = [&](int cc) { return REV ? cc >= rc : cc <= rc; };  // column chunks that reach this warp's rows
   constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
   const bool has_z = a.z != nullptr;
   const CUtensorMap* mapx = MB ? &maps.x1 : &maps.x0;
@@ -568,26 +572,26 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     tc::mbar_expect_tx(mb_cb, M::C_BYTES + KJ * kN * 2);
 #pragma unroll
     for (int nb2 = 0; nb2 < 2; ++nb2) {
-      tc::tma_load_4d(tc::smem_u32(sC + nb2 * (kBlk * 128)), &maps.c, mb_cb, nb2 * 64, g, t0 + MB * kBlk, b);
+      tc::tma_load_4d(tc::smem_u32(sC + nb2 * (kBlk * 128)), &maps.c, mb_cb, nb2 * 64, g, t0 + ROW0, b);
 #pragma unroll
       for (int jb2 = 0; jb2 <= MB; ++jb2)
-        tc::tma_load_4d(tc::smem_u32(sBA + nb2 * (KJ * 128) + jb2 * (kBlk * 128)), &maps.bm, mb_cb, nb2 * 64, g, t0 + jb2 * kBlk, b);
+        tc::tma_load_4d(tc::smem_u32(sBA + nb2 * (KJ * 128) + jb2 * (kBlk * 128)), &maps.bm, mb_cb, nb2 * 64, g, t0 + COL0 + jb2 * kBlk, b);
     }
   }
 
   // One head's operands, by bulk copies issued from one thread: x rows through the tensor map (128-byte rows, swizzled),
   // the incoming state and the two exponent vectors as contiguous pieces.  Steps beyond the sequence read as zero.
-  constexpr uint32_t kOperandBytes = KJ * kP * 2 + M::S_BYTES + 2 * KJ * 4;
+  constexpr uint32_t kOperandBytes = KJ * kP * 2 + M::S_BYTES + 2 * VLEN * 4;
   auto prefetch = [&](int h, int buf) {
     const uint32_t full = mb_full(buf);
     tc::mbar_expect_tx(full, kOperandBytes);
-    tc::tma_load_4d(tc::smem_u32(sX + buf * M::X_BYTES), mapx, full, 0, a.x_heads ? h % a.x_heads : h, t0, b);
+    tc::tma_load_4d(tc::smem_u32(sX + buf * M::X_BYTES), mapx, full, 0, h, t0 + COL0, b);
     const T* ss = reinterpret_cast<const T*>(a.ws_state_in) + (((int64_t)b * nchunks + c) * a.heads + h) * (int64_t)(kP * kN);
     tc::bulk_load(tc::smem_u32(sS + buf * M::S_BYTES), ss, M::S_BYTES, full);
     const int64_t voff = (((int64_t)b * a.heads + h) * nchunks + c) * kQ;
     float* dV = sVec + buf * (2 * kQ);
-    tc::bulk_load(tc::smem_u32(dV), a.ws_cum + voff, KJ * 4, full);
-    tc::bulk_load(tc::smem_u32(dV + kQ), a.ws_dt + voff, KJ * 4, full);
+    tc::bulk_load(tc::smem_u32(dV), a.ws_cum + voff, VLEN * 4, full);
+    tc::bulk_load(tc::smem_u32(dV + kQ), a.ws_dt + voff, VLEN * 4, full);
   };
   // slot of (row, 16-byte chunk) in a tile of 128-byte rows written / read by TMA with the 128-byte swizzle
   auto swz = [&](unsigned char* tile, int row, int chunk) { return tile + ((size_t)row * 8 + (chunk ^ (row & 7))) * 16; };
@@ -622,7 +626,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
 #pragma unroll
   for (int k = 0; k < NCH; ++k) {
     const int cc = wg + kScanWG * k;
-    if (ok && cc <= rc) {
+    if (ok && reached(cc)) {
       tc::tmem_ld32(tmem + lane_base + cc * 32, vG[k]);
     } else {
 #pragma unroll
@@ -633,7 +637,6 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   // A skip weight per head (not per channel) rides on the diagonal of the masked operand: (G o L + D I) X = Y_intra + D x.
   // The row sums for the backward pass want y without the skip term, so that mode keeps the explicit form.
   const bool fold_d = !XSKIP && a.D;
-  const bool pair_reuse = (a.dt_mode & 4) && !a.D && !a.row_scale;  // nothing per head may ride on the mask
   constexpr bool skip_explicit = XSKIP;
 
   // epilogue of head h from accumulator pair `buf`: y = Y_intra + exp2(c_i) Y_inter (+ D x where it is not folded), gated by
@@ -694,13 +697,13 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
       *reinterpret_cast<uint4*>(swz(sZ, i_loc, wg * kEU + q)) = o.raw;
     }
     if (dots && has_z) {
-      const int t = t0 + MB * kBlk + i_loc;
+      const int t = t0 + ROW0 + i_loc;
       // the threads of a row (column slices) add to one zero-initialised word: the sum does not depend on their order
       if (t < a.len) atomicAdd(a.row_dots + ((int64_t)b * a.len + t) * a.heads + h, dot);
     }
     tc::fence_async_smem();  // the staged rows leave through a bulk store
   };
-  const int t_blk = t0 + MB * kBlk;  // first step of this block's rows
+  const int t_blk = t0 + ROW0;  // first step of this block's rows
   auto store_rows = [&](int h) {     // the staged rows of a ragged block, 16 bytes a thread
     for (int u = tid; u < t_live * 8; u += kScanThreads)
       *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.Y) + (((int64_t)b * a.len + t_blk + (u >> 3)) * a.heads + h) * kP + (u & 7) * 8) =
@@ -722,31 +725,30 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     const float* vc = sVec + buf * (2 * kQ);
     const float* vcp = vc + kQ;
     const float Dfold = fold_d ? __ldg(a.D + h) : 0.f;
-    float ct = vc[i_chunk];
-    if (a.row_scale) {
-      // optional weight of this thread's row, folded into the row exponent: it scales the mask before rounding and the
-      // carried-state term alike
-      const int t_row = t0 + MB * kBlk + i_loc;
-      ct += lg2_approx(t_row < a.len ? __ldg(a.row_scale + ((int64_t)b * a.len + t_row) * a.heads + h) : 1.f);
+    // exponents of the decay mask, weight = exp2(re - col(j)), and of the carried state's row weight, exp2(ct)
+    float re, ct;
+    if constexpr (REV) {
+      const float next = c + 1 < nchunks ? __ldg(a.ws_cum + (((int64_t)b * a.heads + h) * nchunks + c + 1) * kQ) : 0.f;
+      re = -vcp[i_chunk], ct = vc[kQ - 1] + next + re;
+    } else {
+      re = ct = vc[i_chunk];
     }
+    auto col = [&](int j) { return REV ? -vc[COL0 + j] : vcp[j]; };
     // The weight exp2(c_i - c'_j) of a 32-step chunk factors as exp2(c_i - r) * exp2(r - c'_j) with r = c at the
     // chunk's first step (row factor <= 1 for causal rows, column factor bounded by the decay inside the chunk).
     // Each lane forms one column factor per chunk, each thread one row factor per chunk: 2 ex2 per 32 elements
     // instead of 32.  Chunks whose internal decay exceeds 2^60 keep the exact per-element form.
-    // dt_mode & 4: heads 2 i and 2 i + 1 have the same step sizes and decay, so the masked operand the even head left in
-    // tensor memory serves the odd head as it is (its MMAs have completed and only read it)
-    const bool reuse = pair_reuse && (h & 1) && hi > 0;
     float arow[NCH];
     bool fast[NCH];
 #pragma unroll
     for (int k = 0; k < NCH; ++k) {
       const int cc = wg + kScanWG * k;
       arow[k] = 0.f, fast[k] = false;
-      if (cc <= rc && !reuse) {
-        const float r = vc[cc * 32];
-        fast[k] = r - vc[cc * 32 + 31] < 60.f;  // same for every lane
-        arow[k] = ex2_approx(ct - r);
-        sW[k * 32 + lane] = ex2_approx(r - vcp[cc * 32 + lane]);
+      if (reached(cc)) {
+        const float first = vc[COL0 + cc * 32], r = REV ? -first : first;
+        fast[k] = first - vc[COL0 + cc * 32 + 31] < 60.f;  // same for every lane
+        arow[k] = ex2_approx(re - r);
+        sW[k * 32 + lane] = ex2_approx(r - col(cc * 32 + lane));
       }
     }
     // MMAs of the previous head: the masked tile, the other buffer and its accumulators are free / ready
@@ -780,7 +782,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
         tc::bulk_commit();
       }
       if (hi + 2 < nh) {  // the tiles of the head after next on their way into the L2: one iteration alone does not cover the latency
-        tc::tma_prefetch_4d(mapx, 0, a.x_heads ? (h + 2) % a.x_heads : h + 2, t0, b);
+        tc::tma_prefetch_4d(mapx, 0, h + 2, t0 + COL0, b);
         if (has_z) tc::tma_prefetch_4d(&maps.z, 0, h + 2, t_blk, b);
         tc::bulk_prefetch(reinterpret_cast<const T*>(a.ws_state_in) + (((int64_t)b * nchunks + c) * a.heads + h + 2) * (int64_t)(kP * kN), M::S_BYTES);
       }
@@ -788,15 +790,14 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
 
     if (ragged && hi >= 2) store_rows(h - 2);  // read before the mid-iteration barrier, overwritten after it
     // ---- decay mask: G (registers) x the factors formed above -> the A operand in tensor memory
-    if (!reuse) {
 #pragma unroll
     for (int k = 0; k < NCH; ++k) {
-      const int cc = wg + kScanWG * k;  // chunk of 32 steps: fully causal (cc < rc), diagonal (cc == rc) or empty (cc > rc) for this warp's rows
+      const int cc = wg + kScanWG * k;  // chunk of 32 steps: whole, diagonal (cc == rc) or empty for this warp's rows
       const int jb = cc * 32;
       // the masked row goes to tensor memory as the A operand: 32 steps = 16 columns of two 16-bit values
       const uint32_t dst = tmem + lane_base + cc * 16;
       uint32_t packed[16];
-      if (cc > rc) {
+      if (!reached(cc)) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) packed[q] = 0u;
         tc::tmem_st16(dst, packed);
@@ -831,10 +832,10 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
 #pragma unroll
           for (int e = 0; e < 8; e += 2) {
             float2 w = __fmul2_rn(__fmul2_rn(make_float2(vG[k][q + e], vG[k][q + e + 1]), bp[e / 2]), a2);
-            if (q + e > lane) w.x = 0.f;
-            if (q + e + 1 > lane) w.y = 0.f;
-            if (q + e == lane) w.x += Dfold;
-            if (q + e + 1 == lane) w.y += Dfold;
+            if (REV ? q + e < lane : q + e > lane) w.x = 0.f;
+            if (REV ? q + e + 1 < lane : q + e + 1 > lane) w.y = 0.f;
+            if (!REV && q + e == lane) w.x += Dfold;
+            if (!REV && q + e + 1 == lane) w.y += Dfold;
             f[e] = w.x, f[e + 1] = w.y;
           }
           Vec16<T> o;
@@ -844,16 +845,13 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
       } else {
 #pragma unroll
         for (int q = 0; q < 32; q += 8) {
-          const float4 c0 = *reinterpret_cast<const float4*>(vcp + jb + q);
-          const float4 c1 = *reinterpret_cast<const float4*>(vcp + jb + q + 4);
-          const float cj[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            float w = ex2_approx(ct - cj[e]);
-            if (diag && q + e > lane) w = 0.f;
+            float w = ex2_approx(re - col(jb + q + e));
+            if (diag && (REV ? q + e < lane : q + e > lane)) w = 0.f;
             f[e] = vG[k][q + e] * w;
-            if (diag && q + e == lane) f[e] += Dfold;
+            if (!REV && diag && q + e == lane) f[e] += Dfold;
           }
           Vec16<T> o;
           o.pack(f);
@@ -863,7 +861,6 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
       tc::tmem_st16(dst, packed);
     }
     tc::tmem_wait_st();
-    }
     // this row of x (for D x in the epilogue one iteration later)
     uint4 xr[kXR];
 #pragma unroll
@@ -934,7 +931,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   if (fail && tid == 0 && a.status) *(volatile int32_t*)a.status = 2;
 }
 
-template <typename T, bool XSKIP>
+template <typename T, bool XSKIP, bool REV>
 __global__ void __launch_bounds__(kScanThreads, 1)
     ssd_scan_kernel(const ssm_ssd_args a, const __grid_constant__ ScanMaps maps, int nchunks, int hpc, int nparts) {
   extern __shared__ unsigned char smdyn[];
@@ -947,51 +944,22 @@ __global__ void __launch_bounds__(kScanThreads, 1)
     for (int i = 0; i < 8; ++i) tc::mbar_init(tc::smem_u32(&mbar[i]), 1);
   }
   __syncthreads();  // barriers and the TMEM address are set up before anyone arms or polls them
-  // the heavier blocks (rows 128..255) are scheduled first
-  if ((int)blockIdx.x < (int)(gridDim.x >> 1)) ssd_scan_body<T, 1, XSKIP>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
-  else ssd_scan_body<T, 0, XSKIP>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
+  // the heavier blocks (rows 128..255; REV: rows 0..127) are scheduled first
+  if ((int)blockIdx.x < (int)(gridDim.x >> 1)) ssd_scan_body<T, 1, XSKIP, REV>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
+  else ssd_scan_body<T, 0, XSKIP, REV>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem_slot, 512);
 }
 
-// ---- tensor maps (driver entry point fetched through the runtime; no link-time dependency on the driver) -------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-// (batch, len, outer, inner) tensor of 16-bit elements seen as rank 4 (inner, outer, step, batch);
-// box = 64 inner elements of one outer index x `rows` steps
-static int encode_rows_map(CUtensorMap* m, const void* base, const ssm_ssd_args& a, int rows, int inner = kP, int outer = -1) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return ::ssmb::fail(SSM_ERR_DEVICE, "ssd_scan: cuTensorMapEncodeTiled is not available from this driver");
-  if (outer < 0) outer = a.heads;
-  const cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)outer, (cuuint64_t)a.len, (cuuint64_t)a.batch};
-  const cuuint64_t strides[3] = {(cuuint64_t)inner * 2, (cuuint64_t)outer * inner * 2, (cuuint64_t)a.len * outer * inner * 2};
-  const cuuint32_t box[4] = {(cuuint32_t)kP, 1, (cuuint32_t)rows, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUtensorMapDataType dt = a.io_dtype == SSM_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  const CUresult rc = fn(m, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (rc != CUDA_SUCCESS) return ::ssmb::fail(SSM_ERR_DEVICE, "ssd_scan: cuTensorMapEncodeTiled rejected the tensor");
-  return SSM_OK;
-}
-
-template <typename T, int HPC>
+template <typename T, int HPC, bool REV>
 static int ssd_state_launch(const ssm_ssd_args& a, int nchunks, cudaStream_t st) {
   StateMaps maps;
-  if (int rc = encode_rows_map(&maps.b, a.Bm, a, StateSmem<HPC>::kStep, a.bc_width ? a.bc_width : kN, a.groups)) return rc;
-  if (int rc = encode_rows_map(&maps.x, a.X, a, StateSmem<HPC>::kStep, kP, a.x_heads ? a.x_heads : a.heads)) return rc;
+  if (int rc = encode_rows_map(&maps.b, a.Bm, a.batch, a.len, a.groups, kN, StateSmem<HPC>::kStep, a.io_dtype)) return rc;
+  if (int rc = encode_rows_map(&maps.x, a.X, a.batch, a.len, a.heads, kP, StateSmem<HPC>::kStep, a.io_dtype)) return rc;
   const size_t smem = StateSmem<HPC>::ALLOC;
-  cudaFuncSetAttribute(ssd_state_kernel<T, HPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  ssd_state_kernel<T, HPC><<<dim3(a.heads / HPC, a.num_seqs ? a.num_seqs : a.batch), kStateThreads, smem, st>>>(a, maps, nchunks);
+  cudaFuncSetAttribute(ssd_state_kernel<T, HPC, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  ssd_state_kernel<T, HPC, REV><<<dim3(a.heads / HPC, a.num_seqs ? a.num_seqs : a.batch), kStateThreads, smem, st>>>(a, maps, nchunks);
   return launch_status("ssd_state_kernel");
 }
 
@@ -1024,6 +992,24 @@ __global__ void __launch_bounds__(32) ssd_wait_selftest_kernel(int32_t* status, 
   if (!ok && threadIdx.x == 0 && status) *(volatile int32_t*)status = 3;
 }
 
+template <typename T, bool REV>
+static int ssd_state_dispatch(const ssm_ssd_args& a, int hpc, int nchunks, cudaStream_t st) {
+  switch (hpc) {
+    case 1: return ssd_state_launch<T, 1, REV>(a, nchunks, st);
+    case 2: return ssd_state_launch<T, 2, REV>(a, nchunks, st);
+    case 3: return ssd_state_launch<T, 3, REV>(a, nchunks, st);
+    default: return ssd_state_launch<T, 4, REV>(a, nchunks, st);
+  }
+}
+
+template <typename T, bool XSKIP, bool REV>
+static int ssd_scan_launch(const ssm_ssd_args& a, const ScanMaps& maps, unsigned ctas, int nchunks, int hpc, int nparts, cudaStream_t st) {
+  const size_t smem = ScanSmem<T>::ALLOC;
+  cudaFuncSetAttribute(ssd_scan_kernel<T, XSKIP, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  ssd_scan_kernel<T, XSKIP, REV><<<ctas, kScanThreads, smem, st>>>(a, maps, nchunks, hpc, nparts);
+  return launch_status("ssd_scan_kernel");
+}
+
 template <typename T>
 static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
   const int nchunks = a.num_seqs ? a.num_chunks : (a.len + kQ - 1) / kQ;
@@ -1049,7 +1035,7 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
     }
   }
   const int nparts = a.heads / hpc;
-  if (a.phase != 2) {
+  if (a.phase != 2 && !a.reverse) {
     ssd_cumsum_kernel<T><<<dim3((a.heads + kCumHeads - 1) / kCumHeads, nchunks, a.batch), kQ, 0, st>>>(a, nchunks);
     if (int rc = launch_status("ssd_cumsum_kernel")) return rc;
   }
@@ -1063,14 +1049,7 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
     // between one and two (batch, head) pairs per SM: two heads per CTA would leave almost half of the SMs idle; one head per
     // CTA, two CTAs per SM (they fit) keeps every SM busy and halves what the longest SM has to walk
     if ((int64_t)walks * a.heads > sm_count && (int64_t)walks * a.heads <= 2 * (int64_t)sm_count) shpc = 1;
-    int rc;
-    switch (shpc) {
-      case 1: rc = ssd_state_launch<T, 1>(a, nchunks, st); break;
-      case 2: rc = ssd_state_launch<T, 2>(a, nchunks, st); break;
-      case 3: rc = ssd_state_launch<T, 3>(a, nchunks, st); break;
-      default: rc = ssd_state_launch<T, 4>(a, nchunks, st); break;
-    }
-    if (rc) return rc;
+    if (int rc = a.reverse ? ssd_state_dispatch<T, true>(a, shpc, nchunks, st) : ssd_state_dispatch<T, false>(a, shpc, nchunks, st)) return rc;
   } else if (a.initial_states) {
     const int64_t units = (int64_t)a.batch * a.heads * (kP * kN / 8);
     ssd_fold_init_kernel<T><<<dim3((unsigned)((units + 255) / 256), (nchunks + 1 + kFoldChunks - 1) / kFoldChunks), 256, 0, st>>>(a, nchunks);
@@ -1081,25 +1060,16 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
   }
   if (a.phase != 1) {
     ScanMaps maps;
-    const int xh = a.x_heads ? a.x_heads : a.heads;  // input heads stored
-    if (int rc = encode_rows_map(&maps.x0, a.X, a, kBlk, kP, xh)) return rc;
-    if (int rc = encode_rows_map(&maps.x1, a.X, a, kQ, kP, xh)) return rc;
-    if (int rc = encode_rows_map(&maps.z, a.z ? a.z : a.Y, a, kBlk)) return rc;
-    if (int rc = encode_rows_map(&maps.y, a.Y, a, kBlk)) return rc;
-    // narrower stored rows (bc_width 64): the copies of the upper 64 states start outside the tensor and bring zeros
-    const int bcw = a.bc_width ? a.bc_width : kN;
-    if (int rc = encode_rows_map(&maps.c, a.Cm, a, kBlk, bcw, a.groups)) return rc;
-    if (int rc = encode_rows_map(&maps.bm, a.Bm, a, kBlk, bcw, a.groups)) return rc;
-    const size_t smem = ScanSmem<T>::ALLOC;
+    if (int rc = encode_rows_map(&maps.x0, a.X, a.batch, a.len, a.heads, kP, kBlk, a.io_dtype)) return rc;
+    if (int rc = encode_rows_map(&maps.x1, a.X, a.batch, a.len, a.heads, kP, kQ, a.io_dtype)) return rc;
+    if (int rc = encode_rows_map(&maps.z, a.z ? a.z : a.Y, a.batch, a.len, a.heads, kP, kBlk, a.io_dtype)) return rc;
+    if (int rc = encode_rows_map(&maps.y, a.Y, a.batch, a.len, a.heads, kP, kBlk, a.io_dtype)) return rc;
+    if (int rc = encode_rows_map(&maps.c, a.Cm, a.batch, a.len, a.groups, kN, kBlk, a.io_dtype)) return rc;
+    if (int rc = encode_rows_map(&maps.bm, a.Bm, a.batch, a.len, a.groups, kN, kBlk, a.io_dtype)) return rc;
     const unsigned ctas = 2u * nparts * a.batch * nchunks;
-    if (a.D && (a.d_has_p || a.row_dots)) {
-      cudaFuncSetAttribute(ssd_scan_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      ssd_scan_kernel<T, true><<<ctas, kScanThreads, smem, st>>>(a, maps, nchunks, hpc, nparts);
-    } else {
-      cudaFuncSetAttribute(ssd_scan_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      ssd_scan_kernel<T, false><<<ctas, kScanThreads, smem, st>>>(a, maps, nchunks, hpc, nparts);
-    }
-    if (int rc = launch_status("ssd_scan_kernel")) return rc;
+    if (a.reverse) return ssd_scan_launch<T, false, true>(a, maps, ctas, nchunks, hpc, nparts, st);
+    if (a.D && (a.d_has_p || a.row_dots)) return ssd_scan_launch<T, true, false>(a, maps, ctas, nchunks, hpc, nparts, st);
+    return ssd_scan_launch<T, false, false>(a, maps, ctas, nchunks, hpc, nparts, st);
   }
   return SSM_OK;
 }
@@ -1159,9 +1129,7 @@ extern "C" int ssm_ssd_fwd(const ssm_ssd_args* a, ssm_stream_t stream) {
               "ssd_scan: the tensor-core path is built for headdim 64, d_state 128, chunk 256, bf16 / fp16");
   if (a->batch == 0 || a->len == 0) return SSM_OK;
   SSM_REQUIRE(a->phase >= 0 && a->phase <= 2, SSM_ERR_SHAPE, "ssd_scan: phase must be 0, 1 or 2");
-  SSM_REQUIRE(a->dt_mode >= 0 && a->dt_mode <= 7 && (a->dt_mode & 3) != 2, SSM_ERR_SHAPE, "ssd_scan: dt_mode must be 0, 1 or 3, optionally + 4");
-  SSM_REQUIRE(a->bc_width == 0 || a->bc_width == kN || a->bc_width == 64, SSM_ERR_SHAPE, "ssd_scan: bc_width must be 0, 64 or nstate");
-  SSM_REQUIRE(a->x_heads >= 0 && (a->x_heads == 0 || a->heads % a->x_heads == 0), SSM_ERR_SHAPE, "ssd_scan: x_heads must be 0 or divide heads");
+  SSM_REQUIRE(!a->reverse || (a->phase == 0 && !a->D && !a->num_seqs), SSM_ERR_UNSUPPORTED, "ssd_scan: the adjoint pass has no skip term, shards or packed sequences");
   SSM_REQUIRE(a->X && a->dt && a->A && a->Bm && a->Cm && (a->Y || a->phase == 1), SSM_ERR_NULL, "ssd_scan: missing tensor");
   SSM_REQUIRE(a->ws_dt && a->ws_cum && a->ws_state && a->ws_state_in, SSM_ERR_NULL, "ssd_scan: missing scratch");
   SSM_REQUIRE(aligned_to(a->X, 16) && aligned_to(a->Bm, 16) && aligned_to(a->Cm, 16) && (!a->Y || aligned_to(a->Y, 16)) && aligned_to(a->ws_state_in, 16) &&
@@ -1170,7 +1138,7 @@ extern "C" int ssm_ssd_fwd(const ssm_ssd_args* a, ssm_stream_t stream) {
   if (a->num_seqs) {
     SSM_REQUIRE(a->num_seqs > 0 && a->num_seqs <= 65535 && a->num_chunks > 0 && a->seq_table && a->batch == 1, SSM_ERR_SHAPE,
                 "ssd_scan: packed sequences need a batch of one and a table");
-    SSM_REQUIRE(a->phase != 2 && !a->initial_states && !a->row_dots && !a->row_scale, SSM_ERR_UNSUPPORTED, "ssd_scan: not built for packed sequences");
+    SSM_REQUIRE(a->phase != 2 && !a->initial_states && !a->row_dots, SSM_ERR_UNSUPPORTED, "ssd_scan: not built for packed sequences");
   }
   const int64_t nchunks = a->num_seqs ? a->num_chunks : (a->len + kQ - 1) / kQ;
   SSM_REQUIRE((a->num_seqs == 0) == (a->seq_table == nullptr), SSM_ERR_NULL, "ssd_scan: num_seqs without a table");

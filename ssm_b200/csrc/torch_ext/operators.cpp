@@ -676,10 +676,113 @@ std::tuple<Tensor, Tensor> ssd_run(const Tensor& X_, const Tensor& dt_, const Te
   return {Y, fin};
 }
 
-std::tuple<Tensor, Tensor> ssd_forward(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
-                                       const OptTensor& z, const OptTensor& dt_bias, bool softplus, const OptTensor& init, int64_t chunk) {
+// Differentiable call on the tensor cores; the backward runs in the dual form (see include/ssm_b200.h for its passes).
+struct SsdCall final : Call {
+  Tensor X_, dt_, A_, B_, C_;
+  OptTensor D_, z_, bias_, init_;
+  bool softplus;
+  int64_t chunk;
+
+  SsdCall(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D, const OptTensor& z,
+          const OptTensor& dt_bias, bool softplus_, const OptTensor& init, int64_t chunk_)
+      : X_(X), dt_(dt), A_(A), B_(B), C_(C), D_(D), z_(z), bias_(dt_bias), init_(init), softplus(softplus_), chunk(chunk_) {
+    for (const Tensor* t : {&X, &dt, &A, &B, &C}) input(*t);
+    input(D), input(z), input(dt_bias), input(init);
+  }
+  variable_list forward(bool) override {
+    auto [Y, fin] = ssd_run(X_, dt_, A_, B_, C_, D_, z_, bias_, softplus, init_, chunk, nullptr, true);
+    return {Y, fin};
+  }
+
+  variable_list backward(const variable_list& grads) override {
+    c10::cuda::CUDAGuard guard(X_.device());
+    const int64_t nb = X_.size(0), nl = X_.size(1), nh = X_.size(2), np = X_.size(3), ng = B_.size(2), nn = B_.size(3), nchunks = (nl + chunk - 1) / chunk;
+    const auto f32 = X_.options().dtype(at::kFloat).requires_grad(false);
+    Tensor X = X_.detach().contiguous(), dt = like(dt_, X), B = like(B_, X), C = like(C_, X), A = f32c(A_);
+    OptTensor D = f32c(D_), bias = f32c(bias_), init = f32c(init_), z;
+    if (z_.has_value()) z = like(*z_, X);
+    Tensor gy = grads[0].defined() ? like(grads[0], X) : at::zeros_like(X);
+    OptTensor gfin;
+    if (grads.size() > 1 && grads[1].defined()) gfin = f32c(grads[1]);
+    const bool init_grad = init_.has_value() && init_->requires_grad();
+    const int io = dtype_code(X, "ssd_scan");
+    ssm_stream_t stream = stream_of(X);
+
+    Tensor u, qd, dB, dC, dA, dD, dbias;
+    ZeroPool pool;
+    pool.add(u, {nb, nl, nh}), pool.add(qd, {nb, nl, nh}), pool.add(dB, {nb, nl, ng, nn}), pool.add(dC, {nb, nl, ng, nn}), pool.add(dA, {nh});
+    if (D.has_value()) pool.add(dD, D->sizes());
+    if (bias.has_value()) pool.add(dbias, {nh});
+    pool.make(f32);
+    Tensor dX = at::empty_like(X), ddt = at::empty_like(dt), dz, dinit, start0;
+
+    ssm_ssd_bwd_args e{};
+    e.batch = (int)nb, e.len = (int)nl, e.heads = (int)nh, e.headdim = (int)np, e.io_dtype = io, e.d_has_p = D.has_value() && D->dim() == 2;
+    e.gY = gy.data_ptr(), e.z = ptr(z), e.X = X.data_ptr(), e.D = fptr(D), e.dX = dX.data_ptr(), e.dD = out_ptr(dD);
+    Tensor dy = gy;
+    if (z.has_value()) {
+      dy = at::empty_like(X), dz = at::empty_like(X);
+      e.dy = dy.data_ptr(), e.dz = dz.data_ptr();
+      run(ssm_ssd_bwd_gate(&e, stream));
+    }
+    // forward again without skip and gate, then the adjoint pass on the same exponents
+    const int64_t vec = nb * nh * nchunks * chunk * 4, fin_bytes = ssm_ssd_state_scratch_bytes((int)nb, (int)nl, (int)nh);
+    const auto bytes = X.options().dtype(at::kByte);
+    Tensor ws = at::empty({ssm_ssd_scratch_bytes((int)nb, (int)nl, (int)nh)}, bytes), ws_r = at::empty({ws.numel() - 2 * vec}, bytes);
+    Tensor st32 = at::empty({nb, nchunks, nh, np * nn}, f32), ad32 = at::empty({nb, nchunks, nh, np * nn}, f32), y = at::empty_like(X), dx = at::empty_like(X), gstate;
+    char *base = reinterpret_cast<char*>(ws.data_ptr()), *base_r = reinterpret_cast<char*>(ws_r.data_ptr());
+    ssm_ssd_args a{};
+    a.batch = (int)nb, a.len = (int)nl, a.heads = (int)nh, a.headdim = (int)np, a.nstate = (int)nn, a.groups = (int)ng, a.chunk_size = (int)chunk, a.io_dtype = io;
+    a.dt_softplus = softplus, a.dt = dt.data_ptr(), a.A = A.data_ptr<float>(), a.dt_bias = fptr(bias);
+    a.ws_dt = reinterpret_cast<float*>(base), a.ws_cum = reinterpret_cast<float*>(base + vec);
+    a.status = ssd_status(X.get_device()).data_ptr<int32_t>();
+    ssm_ssd_args f = a;
+    f.X = X.data_ptr(), f.Bm = B.data_ptr(), f.Cm = C.data_ptr(), f.z = dy.data_ptr(), f.initial_states = fptr(init), f.Y = y.data_ptr();
+    f.ws_state = reinterpret_cast<float*>(base + 2 * vec), f.ws_state_in = base + 2 * vec + fin_bytes;
+    f.row_dots = u.data_ptr<float>(), f.ws_state_in_f32 = st32.data_ptr<float>();
+    run(ssm_ssd_fwd(&f, stream));
+    ssm_ssd_args r = a;
+    r.reverse = 1, r.X = dy.data_ptr(), r.Bm = C.data_ptr(), r.Cm = B.data_ptr(), r.z = X.data_ptr(), r.initial_states = fptr(gfin), r.Y = dx.data_ptr();
+    r.ws_state = reinterpret_cast<float*>(base_r), r.ws_state_in = base_r + fin_bytes;
+    r.row_dots = qd.data_ptr<float>(), r.ws_state_in_f32 = ad32.data_ptr<float>();
+    if (init.has_value()) gstate = at::empty({nb, nh, np, nn}, f32), r.final_states = gstate.data_ptr<float>();
+    run(ssm_ssd_fwd(&r, stream));
+
+    ssm_ssd_bc_args g{};
+    g.batch = (int)nb, g.len = (int)nl, g.heads = (int)nh, g.groups = (int)ng, g.io_dtype = io;
+    g.X = X.data_ptr(), g.dy = dy.data_ptr(), g.Bm = B.data_ptr(), g.Cm = C.data_ptr(), g.ws_dt = a.ws_dt, g.ws_cum = a.ws_cum;
+    g.state_in = f.ws_state_in, g.adjoint_in = r.ws_state_in, g.dB = out_ptr(dB), g.dC = out_ptr(dC), g.status = a.status;
+    run(ssm_ssd_bwd_bc(&g, stream));
+    e.y_plain = y.data_ptr(), e.dx = dx.data_ptr();
+    run(ssm_ssd_bwd_finish(&e, stream));
+    if (init.has_value()) {  // the state before the first step: one decay further
+      Tensor c0 = ws.narrow(0, vec, vec).view(at::kFloat).view({nb, nh, nchunks * chunk}).select(2, 0);
+      dinit = gstate * at::exp2(c0).unsqueeze(-1).unsqueeze(-1);
+      start0 = (dinit * *init).sum({-2, -1}).contiguous();
+    }
+    ssm_ssd_steps_args s{};
+    s.batch = (int)nb, s.len = (int)nl, s.heads = (int)nh, s.io_dtype = io, s.dt_softplus = softplus;
+    s.dt = dt.data_ptr(), s.dt_bias = fptr(bias), s.A = A.data_ptr<float>(), s.u = u.data_ptr<float>(), s.qd = qd.data_ptr<float>(), s.ws_cum = a.ws_cum;
+    s.state_f32 = st32.data_ptr<float>(), s.adjoint_f32 = ad32.data_ptr<float>(), s.start0 = start0.defined() ? start0.data_ptr<float>() : nullptr;
+    s.ddt = ddt.data_ptr(), s.dA = out_ptr(dA), s.ddt_bias = out_ptr(dbias);
+    run(ssm_ssd_bwd_steps(&s, stream));
+
+    auto to = [](const Tensor& grad, const Tensor& t) { return cast(grad, t.scalar_type()); };
+    variable_list res = {dX, to(ddt, dt_), to(dA, A_), to(dB, B_), to(dC, C_)};
+    if (D_.has_value()) res.push_back(to(dD, *D_));
+    if (z_.has_value()) res.push_back(to(dz, *z_));
+    if (bias_.has_value()) res.push_back(to(dbias, *bias_));
+    if (init_.has_value()) res.push_back(init_grad ? to(dinit, *init_) : Tensor());
+    return res;
+  }
+};
+
+std::tuple<Tensor, Tensor> ssd_scan(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
+                                    const OptTensor& z, const OptTensor& dt_bias, bool softplus, const OptTensor& init, int64_t chunk) {
   ValueErrors scope;
-  return ssd_run(X, dt, A, B, C, D, z, dt_bias, softplus, init, chunk, nullptr, true);
+  ssd_check(X, dt, A, B, C, D, z, dt_bias, init);
+  variable_list r = invoke_call(c10::make_intrusive<SsdCall>(X, dt, A, B, C, D, z, dt_bias, softplus, init, chunk));
+  return {r[0], r[1]};
 }
 
 // Packed sequences.  reset: Y restarts at every boundary; without it Y is the scan through all of them.  -> (Y, last state, states)
@@ -708,7 +811,7 @@ void bind_operators(py::module& m) {
   ops.def("fused_layer_norm", &fused_layer_norm);
   ops.def("mamba1_step", &mamba1_step);
   ops.def("mamba2_step", &mamba2_step);
-  ops.def("ssd_forward", &ssd_forward);
+  ops.def("ssd_scan", &ssd_scan);
   ops.def("ssd_packed", &ssd_packed);
   ops.def("ssd_status", &ssd_status);
   ops.def("ssd_poll", &ssd_poll);

@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <cstdio>
+#include <type_traits>
 
 #include "../../include/ssm_b200.h"
 
@@ -128,15 +129,37 @@ struct Vec16 {
   __device__ __forceinline__ void load_stream(const T* p) { raw = __ldcs(reinterpret_cast<const uint4*>(p)); }
   __device__ __forceinline__ void store(T* p) const { *reinterpret_cast<uint4*>(p) = raw; }
   __device__ __forceinline__ void store_stream(T* p) const { __stcs(reinterpret_cast<uint4*>(p), raw); }
+  // 16-bit elements two at a time: a shift and a mask (or one convert) per 32-bit word in, one packed convert per word out; element
+  // by element the compiler spends a byte permute more on each
   __device__ __forceinline__ void unpack(float (&f)[N]) const {
-    const T* e = reinterpret_cast<const T*>(&raw);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-    for (int i = 0; i < N; ++i) f[i] = to_f<T>(e[i]);
+    for (int i = 0; i < 4; ++i) {
+      if constexpr (std::is_same<T, float>::value) {
+        f[i] = __uint_as_float(w[i]);
+      } else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        f[2 * i] = __uint_as_float(w[i] << 16), f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      } else {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        f[2 * i] = v.x, f[2 * i + 1] = v.y;
+      }
+    }
   }
   __device__ __forceinline__ void pack(const float (&f)[N]) {
-    T* e = reinterpret_cast<T*>(&raw);
+    uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < N; ++i) e[i] = from_f<T>(f[i]);
+    for (int i = 0; i < 4; ++i) {
+      if constexpr (std::is_same<T, float>::value) {
+        w[i] = __float_as_uint(f[i]);
+      } else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&v);
+      } else {
+        const __half2 v = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&v);
+      }
+    }
+    raw = make_uint4(w[0], w[1], w[2], w[3]);
   }
 };
 

@@ -67,7 +67,10 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
   const int b = blockIdx.y;
   const int d0 = blockIdx.x * ROWS;
   const int N = a.nstate, L = a.len, D = a.dim;
-  const int r = lane / LPR, sg = lane % LPR;
+  // Rows in the low lane bits: the eight lanes of a quarter warp share their states, so the 16-byte reads of B and C (most of the
+  // kernel's shared-memory traffic) are broadcasts of one group instead of two rows' worth of four.  8 x 1536 rows, 4096 steps,
+  // 16 states: 1641 -> 1583 us; 2 x 2048 rows, 1024 steps, 64 states: 1458 -> 1135 us.
+  const int r = lane % RPW, sg = lane / RPW;
   const int drow0 = d0 + warp * RPW;
   const int d_raw = drow0 + r;
   const bool row_ok = d_raw < D;
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
           }
         }
         if (gz) {  // dz = dout * silu'(z) * (sum_n C h + D u)
-          reduce_scatter<LPR, 1, TB>(p, lane);
+          reduce_scatter<LPR, RPW, TB>(p, lane);
           constexpr int PER = TB / LPR;
 #pragma unroll
           for (int i = 0; i < PER; ++i) {
@@ -340,8 +343,7 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
         for (int j = 0; j < NS / 2; ++j) hc[j] = hs[0][j];
         if (SHARED) {
           // lanes -> staging area: group (output o, row slot) holds the four steps' products
-          constexpr int ROT = LPR <= 8 ? 8 / LPR : 0;
-          const int slot = (r + ROT * sg) & (RPW - 1);
+          const int slot = (r + (RPW >= 8 ? 0 : sg)) & (RPW - 1);
 #pragma unroll
           for (int j = 0; j < NS; ++j) {
             const int o = sg * NS + j;
@@ -402,8 +404,8 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
           }
         }
       }
-      reduce_scatter<LPR, 1, TB>(s1, lane);
-      reduce_scatter<LPR, 1, TB>(s2, lane);
+      reduce_scatter<LPR, RPW, TB>(s1, lane);
+      reduce_scatter<LPR, RPW, TB>(s2, lane);
       constexpr int PER = TB / LPR;
 #pragma unroll
       __syncwarp();  // every lane has read this batch's u / dy before they are overwritten
@@ -475,8 +477,8 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
     }
   }
 
-  dDacc = group_sum<LPR, 1>(dDacc);
-  dBiasAcc = group_sum<LPR, 1>(dBiasAcc);
+  dDacc = group_sum<LPR, RPW>(dDacc);
+  dBiasAcc = group_sum<LPR, RPW>(dBiasAcc);
   if (g.dinitial_state && row_ok) {  // what the adjoint carries past step 0 is the gradient of the state before it
 #pragma unroll
     for (int j = 0; j < NS; j += 2) {

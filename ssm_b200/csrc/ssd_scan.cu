@@ -124,7 +124,9 @@ __global__ void __launch_bounds__(kQ) ssd_cumsum_kernel(const ssm_ssd_args a, in
 //   A operand = B^T, MN-major;  B operand = w x of the CTA's heads side by side, MN-major;  M = 128 (n), N = 64 per head (p),
 //   K = 64 per stage.  (Units that are neighbours along M / N are 128 bytes apart, so the tensor core's reads of one K slice
 //   fall on different banks; with units 2 KB apart the MMAs ran 4-5x slower.)
-// Eight compute warps scale the x rows of a landed stage in place and keep the running state in registers (thread = state n,
+// Eight compute warps scale the x rows of the landed stages in place, four of them the even and four the odd stages (a stage costs a
+// warp a fixed chain of waits, shared-memory round trips and fences, whatever the number of rows: half as many stages per warp,
+// each with twice the rows; sixteen warps on four groups were slower), and keep the running state in registers (thread = state n,
 // 32 of the 64 columns p):  state <- exp2(c_last) * state + S_c ;  the state BEFORE each chunk goes out in the operand dtype,
 // in the operand order of the scan kernel (MN-major units [p/8][n][8]).  The per-chunk local states never touch global memory.
 // A ninth warp issues the copies (a buffer is refilled once the MMAs that read it have completed: tcgen05.commit -> mbarrier),
@@ -133,20 +135,17 @@ __global__ void __launch_bounds__(kQ) ssd_cumsum_kernel(const ssm_ssd_args a, in
 // HPC heads of one B / C group per CTA share the B^T tile of every stage (the grid is sized to about one CTA per SM).
 // Tiles are rows of 128 bytes (64 elements along M / N) written by TMA with the 128-byte swizzle, 64 steps each:
 // B^T as two blocks (states 0..63, 64..127), then one x block per head; blocks are 8 KB apart.
-template <int HPC>
+template <int HPC, int NST>
 struct StateSmem {
   static constexpr int kStep = 64;                            // steps per stage
   static constexpr int BLK_BYTES = kStep * 128;               // 8 KB: 64 steps x 64 elements
   static constexpr int A_BYTES = 2 * BLK_BYTES;               // 16 KB
   static constexpr int STAGE = A_BYTES + HPC * BLK_BYTES;
-  // one head per CTA: four stages (100 KB), so that two CTAs share an SM when there are more heads than SMs
-  static constexpr int NSTAGE = HPC == 1 ? 4 : (HPC == 2 ? 6 : (HPC == 3 ? 5 : 4));
-  static constexpr int VEC_BYTES = HPC * kQ * 4;              // c - log2(delta) of a chunk, per head
-  // The copies run up to NSTAGE stages ahead of the MMAs, so a chunk's vectors may arrive while the chunk before last is still
-  // being scaled: three buffers (NSTAGE <= 6 stages = one and a half chunks).
-  static constexpr int NVEC = 3;
-  static constexpr int LAST_BYTES = HPC * 16;                 // the last four running exponents of a chunk, per head
-  static constexpr int TOTAL = NSTAGE * STAGE + NVEC * (VEC_BYTES + LAST_BYTES);
+  static constexpr int NSTAGE = NST;
+  // exponents that come with a stage, per head: those of its steps, the chunk's first four (REV) and its last four
+  static constexpr int kVec = kStep + 8;
+  static constexpr int VEC_BYTES = HPC * kVec * 4;
+  static constexpr int TOTAL = NSTAGE * (STAGE + VEC_BYTES);
   static constexpr int ALLOC = TOTAL + 1024;
 };
 
@@ -159,25 +158,27 @@ struct StateMaps {
 // from role to role through mbarriers only (landed -> scaled -> multiplied -> free), so no warp waits for another role's
 // instruction issue.
 constexpr int kStateComputeThreads = 256;
+constexpr int kStateGroupThreads = kStateComputeThreads / 2;  // one group scales the even stages, the other the odd ones
 constexpr int kStateThreads = kStateComputeThreads + 64;
 constexpr int kStateCopyWarp = 8, kStateMmaWarp = 9;
 
 // REV: the adjoint recurrence.  The chunks are walked from the last to the first with dy, C and B in the places of x, B and C; the
 // local sum is taken to a chunk's first step, sum_i exp2(c_i - c_0) C_i dy_i^T, and what is handed out is the adjoint that enters a
 // chunk from the right (the adjoint state at the next chunk's first step; the decay of that step belongs to the walk).
-template <typename T, int HPC, bool REV>
-__global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_kernel(const ssm_ssd_args a, const __grid_constant__ StateMaps maps, int nchunks) {
-  using M = StateSmem<HPC>;
+template <typename T, int HPC, int NST, bool REV>
+__global__ void __launch_bounds__(kStateThreads, 1) ssd_state_kernel(const ssm_ssd_args a, const __grid_constant__ StateMaps maps, int nchunks) {
+  using M = StateSmem<HPC, NST>;
   constexpr int kStep = M::kStep, NS = M::NSTAGE;
   constexpr int SPC = kQ / kStep;  // stages per chunk
   extern __shared__ unsigned char smdyn[];
   unsigned char* smraw = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smdyn) + 1023) & ~(uintptr_t)1023);
-  float* sVec = reinterpret_cast<float*>(smraw + NS * M::STAGE);  // [NVEC][HPC][kQ]
-  float* sLast = sVec + M::NVEC * HPC * kQ;                       // [NVEC][HPC][4]: c at the chunk's last four steps
+  float* sVec = reinterpret_cast<float*>(smraw + NS * M::STAGE);  // [NS][HPC][kVec]
+  static_assert(SPC % 2 == 0 && NS >= 2, "a group's stages are the same parts of every chunk");
   __shared__ __align__(8) uint64_t mbar_full[NS];   // a stage's copies have landed
-  __shared__ __align__(8) uint64_t mbar_scaled[NS]; // every compute warp has scaled its part of a stage's x rows
+  __shared__ __align__(8) uint64_t mbar_scaled[NS]; // every warp of the stage's group has scaled its part of the x rows
   __shared__ __align__(8) uint64_t mbar_free[NS];   // the MMAs that read a stage's buffer have completed
   __shared__ __align__(8) uint64_t mbar_acc[2];     // a chunk's accumulators are complete
+  __shared__ __align__(8) uint64_t mbar_read[2];    // every compute warp has read them
   __shared__ uint32_t tmem_slot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wg = tid >> 7;
@@ -200,11 +201,13 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
   if (tid == 0) {
     for (int i = 0; i < NS; ++i) {
       tc::mbar_init(tc::smem_u32(&mbar_full[i]), 1);
-      tc::mbar_init(tc::smem_u32(&mbar_scaled[i]), kStateComputeThreads / 32);
+      tc::mbar_init(tc::smem_u32(&mbar_scaled[i]), kStateGroupThreads / 32);
       tc::mbar_init(tc::smem_u32(&mbar_free[i]), 1);
     }
     tc::mbar_init(tc::smem_u32(&mbar_acc[0]), 1);
     tc::mbar_init(tc::smem_u32(&mbar_acc[1]), 1);
+    tc::mbar_init(tc::smem_u32(&mbar_read[0]), kStateComputeThreads / 32);
+    tc::mbar_init(tc::smem_u32(&mbar_read[1]), kStateComputeThreads / 32);
   }
   __syncthreads();  // TMEM address and barriers are set up
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
@@ -214,27 +217,24 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
   const int64_t vrow0 = (((int64_t)b * a.heads + h0) * nchunks + c_off) * kQ;  // exponent vectors of head h0 (next head: + nchunks * kQ)
   const int nst = SPC * nwalk;
   auto chunk_of = [&](int c) { return REV ? nwalk - 1 - c : c; };  // c-th chunk of the walk
-  // stage s = steps [s * 64, s * 64 + 64), issued by one thread: two boxes of B, one box of x per head, and with a
-  // chunk's first stage the exponent vectors of its heads.  Steps beyond the sequence read as zero.
+  // stage s = steps [s * 64, s * 64 + 64), issued by one thread: two boxes of B, one box of x per head, and the exponents.
+  // Steps beyond the sequence read as zero.
   auto copy_stage = [&](int s) {
     const uint32_t base = tc::smem_u32(smraw + (s % NS) * M::STAGE);
     const uint32_t full = tc::smem_u32(&mbar_full[s % NS]);
-    const bool first = s % SPC == 0;
-    const int t = t_off + chunk_of(s / SPC) * kQ + (s % SPC) * kStep;
-    tc::mbar_expect_tx(full, M::STAGE + (first ? HPC * kQ * 4 + (REV ? 0 : M::LAST_BYTES) : 0));
+    const int c = chunk_of(s / SPC), part = s % SPC;
+    const int t = t_off + c * kQ + part * kStep;
+    tc::mbar_expect_tx(full, M::STAGE + HPC * (kStep * 4 + (REV ? 32 : 16)));
     tc::tma_load_4d(base, &maps.b, full, 0, g, t, b);
     tc::tma_load_4d(base + M::BLK_BYTES, &maps.b, full, 64, g, t, b);
 #pragma unroll
-    for (int hh = 0; hh < HPC; ++hh)
+    for (int hh = 0; hh < HPC; ++hh) {
       tc::tma_load_4d(base + M::A_BYTES + hh * M::BLK_BYTES, &maps.x, full, 0, h0 + hh, t, b);
-    if (first) {
-      const int c = s / SPC;
-#pragma unroll
-      for (int hh = 0; hh < HPC; ++hh) {
-        const int64_t at = vrow0 + ((int64_t)hh * nchunks + chunk_of(c)) * kQ;
-        tc::bulk_load(tc::smem_u32(sVec + ((c % M::NVEC) * HPC + hh) * kQ), (REV ? a.ws_cum : a.ws_dt) + at, kQ * 4, full);
-        if (!REV) tc::bulk_load(tc::smem_u32(sLast + ((c % M::NVEC) * HPC + hh) * 4), a.ws_cum + at + kQ - 4, 16, full);
-      }
+      const int64_t at = vrow0 + ((int64_t)hh * nchunks + c) * kQ;
+      const uint32_t dv = tc::smem_u32(sVec + ((s % NS) * HPC + hh) * M::kVec);
+      tc::bulk_load(dv, (REV ? a.ws_cum : a.ws_dt) + at + part * kStep, kStep * 4, full);
+      if (REV) tc::bulk_load(dv + kStep * 4, a.ws_cum + at, 16, full);
+      tc::bulk_load(dv + kStep * 4 + 16, a.ws_cum + at + kQ - 4, 16, full);
     }
   };
   int fail = 0;
@@ -253,14 +253,23 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
     }
   } else if (role == kStateMmaWarp) {
     // ---- MMAs: S_c (+)= B^T (w x) over the 64 steps of a stage, as soon as the eight compute warps have scaled it ----
+    float ctot[HPC];
+#pragma unroll
+    for (int hh = 0; hh < HPC; ++hh) ctot[hh] = 0.f;
 #pragma unroll 1
     for (int s = 0; s < nst; ++s) {
       const int c = s / SPC, part = s % SPC;
-      const bool okm = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&mbar_scaled[s % NS]), (s / NS) & 1));
+      bool okm = true;
+      // the accumulators of the chunk before last have been read
+      if (part == 0 && c >= 2) okm = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&mbar_read[c & 1]), ((c - 2) >> 1) & 1));
+      okm = okm && __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&mbar_scaled[s % NS]), (s / NS) & 1));
       if (!okm) {
         fail = 1;
         break;
       }
+      float last[HPC];  // read before the commit that lets the stage's buffer be refilled
+#pragma unroll
+      for (int hh = 0; hh < HPC; ++hh) last[hh] = sVec[((s % NS) * HPC + hh) * M::kVec + kStep + 7];
       tc::fence_after_sync();
       if (tc::elect_one()) {
         // M = 128 states = two 64-element blocks, N = 64 HPC = one block per head; blocks 8 KB apart, 8 steps 1 KB apart
@@ -275,6 +284,21 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
         if (part == SPC - 1) tc::commit(tc::smem_u32(&mbar_acc[c & 1]));
       }
       __syncwarp();
+      if (!REV && part == 0) {
+#pragma unroll
+        for (int hh = 0; hh < HPC; ++hh) {
+          // exponent (base 2) of the decay from the start of the sequence to the start of this chunk: what a state
+          // that arrives later (phase 2 of a sequence shard) is multiplied by before it joins this chunk's state
+          if (lane == 0 && !packed) a.ws_state[ssd_summary_floats_padded(a.batch, a.heads) + ((int64_t)b * a.heads + h0 + hh) * nchunks + c] = ctot[hh];
+          ctot[hh] += last[hh];
+        }
+      }
+    }
+    // the shard's total log-decay (natural log) follows the states in the scratch: together they are what a sequence shard sends to
+    // the other ranks
+    if (!REV && !fail && lane == 0) {
+#pragma unroll
+      for (int hh = 0; hh < HPC; ++hh) a.ws_state[(int64_t)n_states * a.heads * kP * kN + (int64_t)sb * a.heads + h0 + hh] = ctot[hh] * kLn2;
     }
   } else {
   // ======== compute warps ========================================================================================
@@ -310,9 +334,9 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
     }
   };
   // last exponent of the current / previous chunk per head (the decay across the chunk is exp2 of it)
-  float clast[HPC], clast_prev[HPC], ctot[HPC];
+  float clast[HPC], clast_prev[HPC];
 #pragma unroll
-  for (int hh = 0; hh < HPC; ++hh) clast[hh] = 0.f, clast_prev[hh] = 0.f, ctot[hh] = 0.f;
+  for (int hh = 0; hh < HPC; ++hh) clast[hh] = 0.f, clast_prev[hh] = 0.f;
   float cfirst[HPC];  // REV: the running exponent at the current chunk's first step
 #pragma unroll
   for (int hh = 0; hh < HPC; ++hh) cfirst[hh] = 0.f;
@@ -330,68 +354,82 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
         for (int i = 0; i < 32; ++i) st[hh][i] = fmaf(decay, st[hh][i], v[i]);
       }
     }
+    tc::fence_before_sync();
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(tc::smem_u32(&mbar_read[c & 1]));  // also by a warp whose wait ran out
     return ok;
   };
 
+  const int gtid = tid & (kStateGroupThreads - 1);
 #pragma unroll 1
-  for (int s = 0; s < nst; ++s) {
+  for (int s = wg; s < nst; s += 2) {  // a warp's group is its half of the columns, too
     const int c = s / SPC, part = s % SPC;
-    if (part == 0 && c == 0) emit_state_in(0);
-    // ---- one stage into a chunk its predecessor's MMAs have surely finished: fold them, hand out the states
-    // ---- before this chunk (its accumulators are the other pair, so the stage already issued is not disturbed)
-    if (part == 1 && c >= 1) {
-      if (!fail) fail = !fold_chunk(c - 1, clast_prev);
-      emit_state_in(c);
-    }
+    if (s == wg) emit_state_in(0);
     if (!fail) fail = !__all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&mbar_full[s % NS]), (s / NS) & 1));  // this stage's copies
-    if (part == 0) {  // a new chunk begins: its last exponent arrived with the stage
+    const float* vs = sVec + (s % NS) * HPC * M::kVec;
+    if (part < 2) {  // this group's first stage of a chunk
 #pragma unroll
       for (int hh = 0; hh < HPC; ++hh) {
+        const float* edge = vs + hh * M::kVec + kStep;  // c at the chunk's first four and last four steps
         clast_prev[hh] = clast[hh];
+        clast[hh] = edge[7];
         if (REV) {  // from the first step of the chunk to its right, which was walked before, down to this one's
-          const float* v = sVec + ((c % M::NVEC) * HPC + hh) * kQ;
-          clast[hh] = v[kQ - 1] - v[0] + cfirst[hh];
-          cfirst[hh] = v[0];
-        } else {
-          clast[hh] = sLast[((c % M::NVEC) * HPC + hh) * 4 + 3];
+          clast[hh] += cfirst[hh] - edge[0];
+          cfirst[hh] = edge[0];
         }
-        // exponent (base 2) of the decay from the start of the sequence to the start of this chunk: what a state
-        // that arrives later (phase 2 of a sequence shard) is multiplied by before it joins this chunk's state
-        if (tid == 0 && !packed && !REV) a.ws_state[ssd_summary_floats_padded(a.batch, a.heads) + ((int64_t)b * a.heads + h0 + hh) * nchunks + c] = ctot[hh];
-        ctot[hh] += clast[hh];
       }
     }
 
-    // ---- scale the x rows in place: w_j x_j (a row is one step, whatever the swizzle does inside it) ------------
-    unsigned char* base = smraw + (s % NS) * M::STAGE;
+    // ---- scale the x rows in place: w_j x_j (a row is one step, whatever the swizzle does inside it).  Every load of a head (or
+    // of two) before its first store: the compiler cannot tell that the units are distinct, and one after the other would put a
+    // shared-memory round trip per unit on the critical path of the stage
+    unsigned char* xs = smraw + (s % NS) * M::STAGE + M::A_BYTES;
+    constexpr int UPT = M::BLK_BYTES / 16 / kStateGroupThreads;  // 16-byte units of a head's tile per thread; 8 units per step
+    constexpr int HB = HPC == 2 ? 2 : 1;                         // heads at a time: what the registers allow
 #pragma unroll
-    for (int hh = 0; hh < HPC; ++hh) {
-      const float* vcp = sVec + ((c % M::NVEC) * HPC + hh) * kQ + part * kStep;
-      const float c_last = clast[hh];
+    for (int h2 = 0; h2 < HPC; h2 += HB) {
+      uint4 raw[HB][UPT];
+      float wt[HB][UPT];
 #pragma unroll
-      for (int k = 0; k < M::BLK_BYTES / 16 / 256; ++k) {
-        const int u = tid + 256 * k;  // 16-byte unit of this head's tile; 8 units per step
-        const float w = REV ? ex2_approx(vcp[u >> 3] - cfirst[hh]) : ex2_approx(c_last - vcp[u >> 3]);  // 0 for steps beyond the sequence
-        unsigned char* px = base + M::A_BYTES + hh * M::BLK_BYTES + (size_t)u * 16;
-        Vec16<T> v;
-        v.raw = *reinterpret_cast<const uint4*>(px);
-        float f[8];
-        v.unpack(f);
+      for (int hh = h2; hh < h2 + HB && hh < HPC; ++hh) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] *= w;
-        v.pack(f);
-        if (packed && w == 0.f) v.raw = make_uint4(0, 0, 0, 0);  // what follows is another sequence
-        *reinterpret_cast<uint4*>(px) = v.raw;
+        for (int k = 0; k < UPT; ++k) {
+          const int u = gtid + kStateGroupThreads * k;
+          wt[hh - h2][k] = vs[hh * M::kVec + (u >> 3)];
+          raw[hh - h2][k] = *reinterpret_cast<const uint4*>(xs + hh * M::BLK_BYTES + (size_t)u * 16);
+        }
+      }
+#pragma unroll
+      for (int hh = h2; hh < h2 + HB && hh < HPC; ++hh) {
+#pragma unroll
+        for (int k = 0; k < UPT; ++k) {
+          const float e = wt[hh - h2][k];
+          const float w = ex2_approx(REV ? e - cfirst[hh] : clast[hh] - e);  // 0 for steps beyond the sequence
+          Vec16<T> v;
+          v.raw = raw[hh - h2][k];
+          float f[8];
+          v.unpack(f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[i] *= w;
+          v.pack(f);
+          if (packed && w == 0.f) v.raw = make_uint4(0, 0, 0, 0);  // what follows is another sequence
+          *reinterpret_cast<uint4*>(xs + hh * M::BLK_BYTES + (size_t)(gtid + kStateGroupThreads * k) * 16) = v.raw;
+        }
       }
     }
-    // the scaled rows become visible to the tensor cores' reads; the accumulator reads of an earlier fold precede the MMAs
-    // that will overwrite that pair.  A warp whose wait ran out still arrives, so that the others do not wait for it.
+    // the scaled rows become visible to the tensor cores' reads.  A warp whose wait ran out still arrives, so that the others do
+    // not wait for it.
     tc::fence_async_smem();
-    tc::fence_before_sync();
     __syncwarp();
     if (lane == 0) tc::mbar_arrive(tc::smem_u32(&mbar_scaled[s % NS]));
+    // ---- its second stage is on its way, and the MMAs of the chunk before are surely finished: fold them, hand out the states
+    // ---- before this chunk
+    if (part >= 2 && c >= 1) {
+      if (!fold_chunk(c - 1, clast_prev)) fail = 1;
+      emit_state_in(c);
+    }
   }
-  if (nwalk > 0 && !fail) fail = !fold_chunk(nwalk - 1, clast);
+  if (nwalk > 0 && !fold_chunk(nwalk - 1, clast)) fail = 1;
   // final states in fp32, (p, n) order: to the caller, and kept in scratch for a later phase 2
   if (!fail) {
 #pragma unroll
@@ -402,9 +440,6 @@ __global__ void __launch_bounds__(kStateThreads, HPC == 1 ? 2 : 1) ssd_state_ker
         if (a.final_states) a.final_states[off + (int64_t)i * kN] = st[hh][i];
         a.ws_state[off + (int64_t)i * kN] = st[hh][i];
       }
-      // the shard's total log-decay (natural log) follows the states in the scratch: together they are what a
-      // sequence shard sends to the other ranks
-      if (tid == 0) a.ws_state[(int64_t)n_states * a.heads * kP * kN + (int64_t)sb * a.heads + h0 + hh] = ctot[hh] * kLn2;
     }
   }
   }  // compute warps
@@ -952,14 +987,14 @@ __global__ void __launch_bounds__(kScanThreads, 1)
   if (warp == 0) tc::tmem_dealloc(tmem_slot, 512);
 }
 
-template <typename T, int HPC, bool REV>
+template <typename T, int HPC, int NST, bool REV>
 static int ssd_state_launch(const ssm_ssd_args& a, int nchunks, cudaStream_t st) {
   StateMaps maps;
-  if (int rc = encode_rows_map(&maps.b, a.Bm, a.batch, a.len, a.groups, kN, StateSmem<HPC>::kStep, a.io_dtype)) return rc;
-  if (int rc = encode_rows_map(&maps.x, a.X, a.batch, a.len, a.heads, kP, StateSmem<HPC>::kStep, a.io_dtype)) return rc;
-  const size_t smem = StateSmem<HPC>::ALLOC;
-  cudaFuncSetAttribute(ssd_state_kernel<T, HPC, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  ssd_state_kernel<T, HPC, REV><<<dim3(a.heads / HPC, a.num_seqs ? a.num_seqs : a.batch), kStateThreads, smem, st>>>(a, maps, nchunks);
+  using M = StateSmem<HPC, NST>;
+  if (int rc = encode_rows_map(&maps.b, a.Bm, a.batch, a.len, a.groups, kN, M::kStep, a.io_dtype)) return rc;
+  if (int rc = encode_rows_map(&maps.x, a.X, a.batch, a.len, a.heads, kP, M::kStep, a.io_dtype)) return rc;
+  cudaFuncSetAttribute(ssd_state_kernel<T, HPC, NST, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::ALLOC);
+  ssd_state_kernel<T, HPC, NST, REV><<<dim3(a.heads / HPC, a.num_seqs ? a.num_seqs : a.batch), kStateThreads, M::ALLOC, st>>>(a, maps, nchunks);
   return launch_status("ssd_state_kernel");
 }
 
@@ -995,10 +1030,12 @@ __global__ void __launch_bounds__(32) ssd_wait_selftest_kernel(int32_t* status, 
 template <typename T, bool REV>
 static int ssd_state_dispatch(const ssm_ssd_args& a, int hpc, int nchunks, cudaStream_t st) {
   switch (hpc) {
-    case 1: return ssd_state_launch<T, 1, REV>(a, nchunks, st);
-    case 2: return ssd_state_launch<T, 2, REV>(a, nchunks, st);
-    case 3: return ssd_state_launch<T, 3, REV>(a, nchunks, st);
-    default: return ssd_state_launch<T, 4, REV>(a, nchunks, st);
+    // as many stages as fit: the ring's round trip (a copy's 2300 cycles, the waits and fences of three roles) is what bounds the walk.
+    // 96 walks of 4001 steps: 39 us with four stages and eight warps per stage, 38 with four per stage, 32 with eight stages
+    case 1: return ssd_state_launch<T, 1, 8, REV>(a, nchunks, st);
+    case 2: return ssd_state_launch<T, 2, 6, REV>(a, nchunks, st);
+    case 3: return ssd_state_launch<T, 3, 5, REV>(a, nchunks, st);
+    default: return ssd_state_launch<T, 4, 4, REV>(a, nchunks, st);
   }
 }
 
@@ -1040,15 +1077,15 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
     if (int rc = launch_status("ssd_cumsum_kernel")) return rc;
   }
   if (a.phase != 2) {
-    // heads per CTA of the sequential state kernel: enough to bring the grid down to about one CTA per SM
-    // (its CTAs all run for the whole sequence, so a second, partial wave would double the time), at most 4,
-    // and a divisor of the heads of one B / C group
+    // heads per CTA of the sequential state kernel: enough to bring the grid down to about one CTA per SM (its CTAs all run
+    // for the whole sequence, so a second, partial wave would double the time), at most 4, and a divisor of the heads of one
+    // B / C group.  Packed sequences differ in length, so their walks spread over the SMs by themselves as long as there are
+    // many; two heads share a B tile, four make the longest walk longer (24 sequences of 16384 steps, 48 heads: 104 us with
+    // four, 65 with two, 68-80 with one).
+    const int most = a.num_seqs ? 2 : 4;
     int shpc = (int)(((int64_t)walks * a.heads + sm_count - 1) / sm_count);
-    shpc = shpc < 1 ? 1 : (shpc > 4 ? 4 : shpc);
+    shpc = shpc < 1 ? 1 : (shpc > most ? most : shpc);
     while (hpg % shpc != 0) --shpc;
-    // between one and two (batch, head) pairs per SM: two heads per CTA would leave almost half of the SMs idle; one head per
-    // CTA, two CTAs per SM (they fit) keeps every SM busy and halves what the longest SM has to walk
-    if ((int64_t)walks * a.heads > sm_count && (int64_t)walks * a.heads <= 2 * (int64_t)sm_count) shpc = 1;
     if (int rc = a.reverse ? ssd_state_dispatch<T, true>(a, shpc, nchunks, st) : ssd_state_dispatch<T, false>(a, shpc, nchunks, st)) return rc;
   } else if (a.initial_states) {
     const int64_t units = (int64_t)a.batch * a.heads * (kP * kN / 8);

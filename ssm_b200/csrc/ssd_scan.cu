@@ -22,6 +22,8 @@
 // sequences stay finite.  Every wait on an mbarrier is bounded and reports through the status word.
 #include "ssd_common.cuh"
 
+#include <algorithm>
+
 namespace ssmb {
 
 // floats of the shard summary (final state, then total log-decay), rounded up to whole 256-byte lines
@@ -749,7 +751,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   uint4 xr_prev[kXR];
 #pragma unroll
   for (int q = 0; q < kXR; ++q) xr_prev[q] = make_uint4(0, 0, 0, 0);
-  int fail = 0;
+  int fail = ok ? 0 : 1;
 #pragma unroll 1
   for (int hi = 0; hi < nh; ++hi) {
     const int h = h0 + hi, buf = hi & 1;
@@ -1047,30 +1049,46 @@ static int ssd_scan_launch(const ssm_ssd_args& a, const ScanMaps& maps, unsigned
   return launch_status("ssd_scan_kernel");
 }
 
+// Heads per scan CTA: a divisor of the heads of one B / C group, so that a CTA's heads share their G.  One CTA runs per SM; the
+// long row blocks go first, then the short ones, each to the first SM that is free.  A long block costs 2 + d and a short one
+// 3 + 0.85 d head times (C / B tiles, G, pipeline fill; fitted to d = 8, 12, 16, 24 on 64 + 64 pieces).  Taken is the d with the
+// earliest end.  Counting whole waves of equal blocks instead chose d = 8 for 76 chunks of 48 heads: 143 us against 122 with 24.
+static int scan_heads_per_cta(int hpg, int64_t longs, int64_t shorts) {
+  const int64_t sms = sm_count();
+  double best = 1e300;
+  int heads = 1;
+  for (int d = 1; d <= hpg && d <= 32; ++d) {
+    if (hpg % d) continue;
+    const double lng = 2.0 + d, shrt = 3.0 + 0.85 * d;
+    const int64_t n = shorts * (hpg / d), q = longs * (hpg / d) / sms, r = longs * (hpg / d) % sms;  // r SMs run q + 1 long blocks, the others q
+    // how many short blocks can have ended by t
+    auto room = [&](double t) {
+      auto fit = [&](double from) { return t < from ? (int64_t)0 : (int64_t)((t - from) / shrt + 1e-9); };
+      return r * fit((q + 1) * lng) + (sms - r) * fit(q * lng);
+    };
+    for (int64_t more = 0; more < (r ? 2 : 1); ++more) {  // the last short block follows q or q + 1 long ones
+      int64_t lo = 0, hi = n + 1;                        // the fewest short blocks on one SM that make room for all of them
+      while (lo < hi) {
+        const int64_t mid = (lo + hi) / 2;
+        if (room((q + more) * lng + mid * shrt) >= n) hi = mid;
+        else lo = mid + 1;
+      }
+      double end = (q + more) * lng + lo * shrt;
+      if (r && end < (q + 1) * lng) end = (q + 1) * lng;
+      if (end < best) best = end, heads = d;
+    }
+  }
+  return heads;
+}
+
 template <typename T>
 static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
   const int nchunks = a.num_seqs ? a.num_chunks : (a.len + kQ - 1) / kQ;
   const int walks = a.num_seqs ? a.num_seqs : a.batch;  // sequences that the state kernel walks
-  // heads per scan CTA (a divisor of the heads of one B / C group, so that a CTA's heads share their G): every CTA
-  // pays a prologue (C / B tiles, G) of about two heads' worth of time, and the grid runs in whole waves of one CTA
-  // per SM; take the divisor with the least (waves x (prologue + heads)).
   const int hpg = a.heads / a.groups;
-  int sm_count = 148;
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-  }
-  int hpc = 1;
-  {
-    double best = 1e300;
-    for (int d = 1; d <= hpg && d <= 32; ++d) {
-      if (hpg % d) continue;
-      const int64_t ctas = 2ll * a.batch * nchunks * (a.heads / d);
-      const double cost = (double)((ctas + sm_count - 1) / sm_count) * (2.0 + d);
-      if (cost < best) best = cost, hpc = d;
-    }
-  }
+  // (of packed sequences about every second one ends in a chunk without a long block)
+  const int64_t blocks = (int64_t)a.batch * nchunks;
+  const int hpc = scan_heads_per_cta(hpg, (a.num_seqs ? std::max<int64_t>(blocks - a.num_seqs / 2, 0) : blocks) * a.groups, blocks * a.groups);
   const int nparts = a.heads / hpc;
   if (a.phase != 2 && !a.reverse) {
     ssd_cumsum_kernel<T><<<dim3((a.heads + kCumHeads - 1) / kCumHeads, nchunks, a.batch), kQ, 0, st>>>(a, nchunks);
@@ -1083,7 +1101,7 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
     // many; two heads share a B tile, four make the longest walk longer (24 sequences of 16384 steps, 48 heads: 104 us with
     // four, 65 with two, 68-80 with one).
     const int most = a.num_seqs ? 2 : 4;
-    int shpc = (int)(((int64_t)walks * a.heads + sm_count - 1) / sm_count);
+    int shpc = (int)(((int64_t)walks * a.heads + sm_count() - 1) / sm_count());
     shpc = shpc < 1 ? 1 : (shpc > most ? most : shpc);
     while (hpg % shpc != 0) --shpc;
     if (int rc = a.reverse ? ssd_state_dispatch<T, true>(a, shpc, nchunks, st) : ssd_state_dispatch<T, false>(a, shpc, nchunks, st)) return rc;

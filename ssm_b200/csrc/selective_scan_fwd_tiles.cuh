@@ -1,5 +1,4 @@
-// Mamba-1 selective scan, forward: the fast path for vectorisable inputs whose rows share B / C
-// (one B / C group per CTA, 16-byte aligned rows, d_state <= 32).
+// Mamba-1 selective scan, forward: the fast path for inputs whose rows share B / C (one B / C group per CTA, d_state <= 32).
 //
 // A CTA owns 32 channel rows of one batch element.  LANE = ROW and WARP = STATE GROUP: warp g
 // keeps states 4g .. 4g+3 of all 32 rows in registers, time is walked sequentially in tiles of
@@ -18,6 +17,11 @@
 // Global -> shared copies of u / delta / z (cp.async, 16 bytes) run a tile ahead into double-buffered raw tiles; the
 // raw u / z of a tile stay valid until its epilogue, where the skip term D*u and the gate silu(z) are applied.  The
 // small B / C tiles travel through registers (one 16-byte chunk per thread, fetched a tile ahead).  Per (row, state, step): one ex2.approx and four packed-fp32 issue slots.
+//
+// RAG: rows that do not start on 16-byte boundaries (a length that is no multiple of 16 bytes), or B / C that do not.  The copies
+// stay 16 bytes wide: each row is fetched from the boundary before its first element, with one chunk more per tile, and read at its
+// own offset by threads that hold one step each (lane = step, so the stores of a row are as contiguous as they can be); B and C
+// travel through registers element by element.  512 rows of 2001 steps, fp32: 402 us in the general kernel, 52 here.
 #pragma once
 
 #include "scan_common.cuh"
@@ -26,18 +30,20 @@ namespace ssmb {
 
 constexpr int kTileRows = 32;  // rows per CTA (one per lane)
 
-template <typename T, int NG>
+template <typename T, int NG, bool RAG>
 struct FwdTiles {
   static constexpr int NP = 4 * NG;     // padded state count
   static constexpr int TL = kScanCkpt;  // one tile = one checkpoint interval
   static constexpr int TLP = TL + 4;
   static constexpr int V = 16 / (int)sizeof(T);
   static constexpr int NT = NG * 32;
+  static constexpr int RP = TL + (RAG ? V : 0);   // pitch of a raw row: one chunk more where rows start anywhere
+  static constexpr int BCP = NP + (RAG ? 4 : 0);  // pitch of a step of B / C: padded where the lanes that write it hold one step each
   // bytes
-  static constexpr int RAW_ROWS = 3 * kTileRows * TL * (int)sizeof(T);  // u, delta, z of one tile
+  static constexpr int RAW_ROWS = 3 * kTileRows * RP * (int)sizeof(T);  // u, delta, z of one tile
   static constexpr int DD = kTileRows * TL * 16;                        // (dl, dl, du, du) per (row, step)
   static constexpr int PART = NG * kTileRows * TLP * 4;                 // partial sums [group][row][TLP]
-  static constexpr int BC_F32 = 2 * TL * NP * 4;                        // B and C as fp32 [TL][NP]
+  static constexpr int BC_F32 = 2 * TL * BCP * 4;                       // B and C as fp32 [TL][BCP]
   static constexpr size_t kBytes = BC_F32 + 2 * RAW_ROWS + DD + PART;
   static_assert(kBytes <= 227 * 1024, "shared memory budget");
 };
@@ -57,19 +63,19 @@ struct FwdStepOps {  // everything of one step that does not depend on the state
 // parallel (for calls whose rows alone cannot fill the machine): pass 1 integrates every segment from a zero state (segment 0:
 // from the initial state) and leaves its end state and decay product exp(A sum delta) in `split`; after the serial combine
 // (scan_split_combine_kernel) pass 2 replays every segment from its true incoming state and produces the outputs.
-template <typename T, int NG, int MODE>
+template <typename T, int NG, int MODE, bool RAG>
 __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kernel(const ssm_scan_fwd_args a, const ScanFlags fl, int seg_tiles) {
-  using M = FwdTiles<T, NG>;
-  constexpr int NP = M::NP, TL = M::TL, TLP = M::TLP, V = M::V, NT = M::NT;
+  using M = FwdTiles<T, NG, RAG>;
+  constexpr int NP = M::NP, TL = M::TL, TLP = M::TLP, V = M::V, NT = M::NT, RP = M::RP, BCP = M::BCP;
   constexpr int CH = TL / V;  // 16-byte chunks per row and tile
   constexpr int ROWS = kTileRows;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, grp = tid >> 5;
-  float* sB = reinterpret_cast<float*>(smem_raw);  // [TL][NP]
-  float* sC = sB + TL * NP;
+  float* sB = reinterpret_cast<float*>(smem_raw);  // [TL][BCP]
+  float* sC = sB + TL * BCP;
   unsigned char* rbase = smem_raw + M::BC_F32;
-  T* rawrows = reinterpret_cast<T*>(rbase);                                     // [2 buffers][u | delta | z][ROWS][TL]
+  T* rawrows = reinterpret_cast<T*>(rbase);                                     // [2 buffers][u | delta | z][ROWS][RP]
   float4* sDD = reinterpret_cast<float4*>(rbase + 2 * M::RAW_ROWS);             // [ROWS][TL], swizzled
   float* sP = reinterpret_cast<float*>(rbase + 2 * M::RAW_ROWS + M::DD);        // [NG][ROWS][TLP]
 
@@ -121,13 +127,15 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
   // ---- tile ahead with a plain vector load and written to the fp32 [step][state] tiles when its tile starts
   const int bc_esz = a.bc_dtype == SSM_F32 ? 4 : 2;
   const int bc_per = 16 / bc_esz;                                 // steps per chunk
-  constexpr int kBcSlots = (2 * NP * (TL / 4) + NT - 1) / NT;     // enough for fp32 coefficients
+  constexpr int kBcSlots = RAG ? 1 : (2 * NP * (TL / 4) + NT - 1) / NT;  // enough for fp32 coefficients
+  constexpr int kBcOne = RAG ? 2 * NP * TL / NT : 1;                     // RAG: one element (of step `lane`) per slot
+  uint32_t bcone[kBcOne];  // raw bits, converted when they are stored: all of a tile's loads are in flight together
   uint4 bcreg[kBcSlots];
   const char* bc_src[kBcSlots];  // this thread's chunk of tile 0 (NULL: no chunk in this slot)
   float* bc_dst[kBcSlots];
   int bc_tt[kBcSlots];
 #pragma unroll
-  for (int s_ = 0; s_ < kBcSlots; ++s_) {
+  for (int s_ = 0; s_ < kBcSlots && !RAG; ++s_) {
     const int c = tid + s_ * NT;
     const int per_op = N * (TL / bc_per);  // chunks of B (then the same number for C); within each: state fastest
     bc_src[s_] = nullptr, bc_dst[s_] = sB, bc_tt[s_] = 0;
@@ -140,7 +148,31 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
                          : reinterpret_cast<const char*>(a.Bm) + (boff + (int64_t)n * a.b_sn + tt) * bc_esz;
     }
   }
+  // RAG: slot s_ of this thread is state (s_ * NG + grp) % NP of B (first half) or C, at step `lane` of the tile; NULL beyond the end
+  auto bc_one = [&](int s_, int t) -> const void* {
+    const int row = s_ * NG + grp, n = row % NP;
+    if (n >= N || t >= L) return nullptr;
+    return row < NP ? reinterpret_cast<const char*>(a.Bm) + (boff + (int64_t)n * a.b_sn + (int64_t)t * a.b_st) * bc_esz
+                    : reinterpret_cast<const char*>(a.Cm) + (coff + (int64_t)n * a.c_sn + (int64_t)t * a.c_st) * bc_esz;
+  };
   auto bc_fetch = [&](int k) {
+    if constexpr (RAG) {
+      const int t = k * TL + lane;
+      if (a.bc_dtype == SSM_F32) {
+#pragma unroll
+        for (int s_ = 0; s_ < kBcOne; ++s_) {
+          const void* src = bc_one(s_, t);
+          bcone[s_] = src ? __ldg(reinterpret_cast<const uint32_t*>(src)) : 0u;
+        }
+      } else {
+#pragma unroll
+        for (int s_ = 0; s_ < kBcOne; ++s_) {
+          const void* src = bc_one(s_, t);
+          bcone[s_] = src ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(src)) : 0u;
+        }
+      }
+      return;
+    }
 #pragma unroll
     for (int s_ = 0; s_ < kBcSlots; ++s_) {
       bcreg[s_] = make_uint4(0u, 0u, 0u, 0u);
@@ -148,6 +180,17 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
     }
   };
   auto bc_store = [&]() {
+    if constexpr (RAG) {
+#pragma unroll
+      for (int s_ = 0; s_ < kBcOne; ++s_) {
+        const int row = s_ * NG + grp;
+        const uint32_t v = bcone[s_];
+        (row < NP ? sB : sC)[lane * BCP + row % NP] = a.bc_dtype == SSM_F32    ? __uint_as_float(v)
+                                                      : a.bc_dtype == SSM_BF16 ? __uint_as_float(v << 16)
+                                                                               : __half2float(__ushort_as_half((unsigned short)v));
+      }
+      return;
+    }
 #pragma unroll
     for (int s_ = 0; s_ < kBcSlots; ++s_) {
       if (bc_src[s_]) {
@@ -168,14 +211,29 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
       }
     }
   };
-  if (N < NP) {  // padded states read as zero for the whole launch
+  if (!RAG && N < NP) {  // padded states read as zero for the whole launch
     for (int i = tid; i < 2 * TL * NP; i += NT) sB[i] = 0.f;
   }
 
   // one 16-byte chunk of u / delta / z per (row, chunk) and thread; out-of-range steps are zero-filled
   auto fill_raw = [&](int k) {
     const int t0 = k * TL;
-    T* rr = rawrows + (k & 1) * (3 * ROWS * TL);
+    T* rr = rawrows + (k & 1) * (3 * ROWS * RP);
+    if constexpr (RAG) {
+      for (int c = tid; c < ROWS * (CH + 1); c += NT) {
+        const int r_ = c / (CH + 1), j = c % (CH + 1);
+        const int64_t off = (int64_t)b * a.row_sb + (int64_t)min(d0 + r_, D - 1) * a.row_sd;  // bases are 16-byte aligned
+        const int64_t first = (off + t0) / V * V + j * V;                                      // this chunk's first element
+        const int n = (int)min((int64_t)V, max((int64_t)0, off + L - first)) * (int)sizeof(T);  // nothing beyond the row is read
+        const int64_t src = n > 0 ? first : 0;
+        T* dst = rr + r_ * RP + j * V;
+        cp_async16n(dst, gu + src, n);
+        cp_async16n(dst + ROWS * RP, gdl + src, n);
+        if (has_z) cp_async16n(dst + 2 * ROWS * RP, gz + src, n);
+      }
+      cp_async_commit();
+      return;
+    }
     for (int c = tid; c < ROWS * CH; c += NT) {
       const int r_ = c / CH, ch = c % CH;
       const int dd = min(d0 + r_, D - 1);
@@ -189,6 +247,9 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
     cp_async_commit();
   };
 
+  // RAG: elements between the boundary that a row is fetched from and its first element
+  auto row_shift = [&](int rr) { return (int)(((int64_t)b * a.row_sb + (int64_t)min(d0 + rr, D - 1) * a.row_sd) % V); };
+
   if (k_begin < k_end) {
     fill_raw(k_begin);
     bc_fetch(k_begin);
@@ -200,12 +261,22 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
     __syncthreads();  // raw tile k has landed for every thread; the other raw buffer, the fp32 tiles and the partials are free
     if (k + 1 < k_end) fill_raw(k + 1);
 
-    const T* rawU = rawrows + (k & 1) * (3 * ROWS * TL);
-    const T* rawD = rawU + ROWS * TL;
-    const T* rawZ = rawD + ROWS * TL;
+    const T* rawU = rawrows + (k & 1) * (3 * ROWS * RP);
+    const T* rawD = rawU + ROWS * RP;
+    const T* rawZ = rawD + ROWS * RP;
 
     // ---- delta (bias, softplus) and delta*u as fp32 operand pairs ---------------------------
-    {
+    if constexpr (RAG) {
+#pragma unroll 4
+      for (int rr = grp; rr < ROWS; rr += NG) {
+        const int at = rr * RP + row_shift(rr) + lane;
+        float x = to_f<T>(rawD[at]) + (a.dt_bias ? __ldg(a.dt_bias + min(d0 + rr, D - 1)) : 0.f);
+        if (a.delta_softplus) x = sizeof(T) == 2 ? softplus_half_io(x) : softplus_fast(x);
+        if (t0 + lane >= L) x = 0.f;  // (u reads as zero there)
+        const float xu = x * to_f<T>(rawU[at]);
+        sDD[dd_slot(rr, lane)] = make_float4(x, x, xu, xu);
+      }
+    } else {
       const bool tail = t0 + TL > L;
       for (int c = tid; c < ROWS * CH; c += NT) {
         const int rr = c / CH, ch = c % CH;
@@ -259,8 +330,8 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
       auto prepare = [&](int tt) {
         FwdStepOps o;
         const float4 dd4 = sDD[dd_slot(lane, tt)];
-        const float4 b4 = *reinterpret_cast<const float4*>(pB + tt * NP);
-        const float4 c4 = *reinterpret_cast<const float4*>(pC + tt * NP);
+        const float4 b4 = *reinterpret_cast<const float4*>(pB + tt * BCP);
+        const float4 c4 = *reinterpret_cast<const float4*>(pC + tt * BCP);
         const float2 dl2 = make_float2(dd4.x, dd4.y), du2 = make_float2(dd4.z, dd4.w);
         const float2 e0 = __fmul2_rn(dl2, A2[0]), e1 = __fmul2_rn(dl2, A2[1]);
         o.da0 = make_float2(ex2_approx(e0.x), ex2_approx(e0.y));
@@ -299,6 +370,19 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
     if (MODE == 1) continue;  // pass 1 of a split call produces no output
 
     // ---- epilogue: add the state groups' partial sums, skip term, gate, store ---------------------
+    if constexpr (RAG) {
+#pragma unroll 4
+      for (int rr = grp; rr < ROWS; rr += NG) {
+        const int dd = min(d0 + rr, D - 1), at = rr * RP + row_shift(rr) + lane;
+        float y = 0.f;
+#pragma unroll
+        for (int s = 0; s < NG; ++s) y += sP[(s * ROWS + rr) * TLP + lane];
+        y = fmaf(a.D ? __ldg(a.D + dd) : 0.f, to_f<T>(rawU[at]), y);
+        if (has_z) y *= silu_fast(to_f<T>(rawZ[at]));
+        if (d0 + rr < D && t0 + lane < L) gout[(int64_t)b * a.row_sb + (int64_t)dd * a.row_sd + t0 + lane] = from_f<T>(y);
+      }
+      continue;
+    }
     for (int c = tid; c < ROWS * CH; c += NT) {
       const int rr = c / CH, ch = c % CH;
       const int dd = d0 + rr;
@@ -386,22 +470,22 @@ static inline int fwd_split_segments(int batch, int dim, int len) {
   return want < 2 ? 1 : (int)want;
 }
 
-template <typename T, int NG>
+template <typename T, int NG, bool RAG>
 static int launch_fwd_tiles(const ssm_scan_fwd_args& a, const ScanFlags& fl, cudaStream_t st) {
-  using M = FwdTiles<T, NG>;
+  using M = FwdTiles<T, NG, RAG>;
   const int ntiles = (a.len + kScanCkpt - 1) / kScanCkpt;
   const int nseg = a.split_scratch && a.split_segments > 1 ? a.split_segments : 1;
   const unsigned gx = (a.dim + kTileRows - 1) / kTileRows;
   if (nseg <= 1) {
-    auto kern = scan_fwd_tiles_kernel<T, NG, 0>;
+    auto kern = scan_fwd_tiles_kernel<T, NG, 0, RAG>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kBytes);
     kern<<<dim3(gx, a.batch), NG * 32, M::kBytes, st>>>(a, fl, ntiles);
     return launch_status("scan_fwd_tiles_kernel");
   }
   const int seg_tiles = (ntiles + nseg - 1) / nseg;
   const int used = (ntiles + seg_tiles - 1) / seg_tiles;  // segments that hold at least one tile
-  auto k1 = scan_fwd_tiles_kernel<T, NG, 1>;
-  auto k2 = scan_fwd_tiles_kernel<T, NG, 2>;
+  auto k1 = scan_fwd_tiles_kernel<T, NG, 1, RAG>;
+  auto k2 = scan_fwd_tiles_kernel<T, NG, 2, RAG>;
   cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kBytes);
   cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kBytes);
   k1<<<dim3(gx, a.batch, used), NG * 32, M::kBytes, st>>>(a, fl, seg_tiles);
@@ -413,19 +497,26 @@ static int launch_fwd_tiles(const ssm_scan_fwd_args& a, const ScanFlags& fl, cud
   return launch_status("scan_fwd_tiles_kernel<final>");
 }
 
-// True when the tile kernel covers this call: vectorisable rows and coefficients and a CTA's 32 rows inside one
-// B / C group.
+// The tile kernel covers a call whose CTAs' 32 rows lie inside one B / C group: as whole vectors, or (rows that start anywhere, B / C
+// of any strides) in its RAG form, which needs aligned base pointers for the copies' boundaries.
+static inline bool fwd_tiles_vec(const ssm_scan_fwd_args& a, const ScanFlags& fl) { return fl.io_vec && fl.bc_vec && a.b_st == 1 && a.c_st == 1; }
 static inline bool fwd_tiles_ok(const ssm_scan_fwd_args& a, const ScanFlags& fl) {
-  return fl.io_vec && fl.bc_vec && a.b_st == 1 && a.c_st == 1 && (fl.rows_per_group % kTileRows == 0) && a.len > 0 && a.nstate <= 32;
+  return fl.rows_per_group % kTileRows == 0 && a.len > 0 && a.nstate <= 32 &&
+         (fwd_tiles_vec(a, fl) || (aligned_to(a.u, 16) && aligned_to(a.delta, 16) && (!a.z || aligned_to(a.z, 16))));
+}
+
+template <typename T, bool RAG>
+static int dispatch_fwd_groups(const ssm_scan_fwd_args& a, const ScanFlags& fl, cudaStream_t st) {
+  const int ng = (a.nstate + 3) / 4;
+  if (ng <= 1) return launch_fwd_tiles<T, 1, RAG>(a, fl, st);
+  if (ng <= 2) return launch_fwd_tiles<T, 2, RAG>(a, fl, st);
+  if (ng <= 4) return launch_fwd_tiles<T, 4, RAG>(a, fl, st);
+  return launch_fwd_tiles<T, 8, RAG>(a, fl, st);
 }
 
 template <typename T>
 static int dispatch_fwd_tiles(const ssm_scan_fwd_args& a, const ScanFlags& fl, cudaStream_t st) {
-  const int ng = (a.nstate + 3) / 4;
-  if (ng <= 1) return launch_fwd_tiles<T, 1>(a, fl, st);
-  if (ng <= 2) return launch_fwd_tiles<T, 2>(a, fl, st);
-  if (ng <= 4) return launch_fwd_tiles<T, 4>(a, fl, st);
-  return launch_fwd_tiles<T, 8>(a, fl, st);
+  return fwd_tiles_vec(a, fl) ? dispatch_fwd_groups<T, false>(a, fl, st) : dispatch_fwd_groups<T, true>(a, fl, st);
 }
 
 }  // namespace ssmb

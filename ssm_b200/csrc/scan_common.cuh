@@ -36,6 +36,8 @@ struct ScanFlags {
   int bc_vec;      // B and C: unit time stride and every (b, g, n) row 16-byte aligned
   int shared_bc;   // all rows of a CTA belong to one B/C group
   int rows_per_group;
+  int io_pieces;   // the bases of the row tensors are 16-byte aligned: ragged rows are fetched in 16-byte pieces (backward)
+  int bc_pieces;   // B and C: unit time stride and aligned bases
 };
 
 // ---- cp.async -----------------------------------------------------------------------------
@@ -78,6 +80,38 @@ __device__ __forceinline__ void fill_rows_raw(T* __restrict__ raw, const T* __re
   }
 }
 
+// The same for rows that start anywhere in memory whose base is 16-byte aligned: 16-byte pieces from the boundary before each row's
+// first element of the tile, one piece more per row (pitch TL + 16 bytes); the row is read at its offset from that boundary, which is
+// row_shift for every tile (TL is a multiple of 16 bytes).  Nothing beyond the row's end is read; what follows it reads as zero.
+template <typename T>
+__device__ __forceinline__ int row_shift(int64_t row_start) { return (int)row_start & (16 / (int)sizeof(T) - 1); }
+template <typename T, int RPW, int TL>
+__device__ __forceinline__ void fill_rows_pieces(T* __restrict__ raw, const T* __restrict__ g, int b, int D, int L, int drow0, int t0, int lane, int64_t sb,
+                                                 int64_t sd) {
+  constexpr int V = 16 / sizeof(T), CH = TL / V + 1;
+  for (int c = lane; c < RPW * CH; c += 32) {
+    const int rr = c / CH, j = c % CH;
+    const int64_t off = (int64_t)b * sb + (int64_t)min(drow0 + rr, D - 1) * sd;
+    const int64_t first = ((off + t0) & ~(int64_t)(V - 1)) + j * V;
+    const int n = (int)min((int64_t)V, max((int64_t)0, off + L - first)) * (int)sizeof(T);
+    cp_async16n(raw + rr * (TL + V) + j * V, g + (n > 0 ? first : 0), n);
+  }
+}
+// ... and for a (N x TL) tile of B or C in the source type; `start`: element offset of state 0 at step 0 from the aligned base
+template <int TL>
+__device__ __forceinline__ void fill_bc_pieces(void* __restrict__ raw, const void* __restrict__ base, int dtype, int64_t start, int64_t sn, int N, int t0, int L,
+                                               int tid, int nthreads) {
+  const int esz = dtype == SSM_F32 ? 4 : 2, per = 16 / esz, CH = TL / per + 1;
+  char* dst = reinterpret_cast<char*>(raw);
+  const char* src = reinterpret_cast<const char*>(base);
+  for (int c = tid; c < N * CH; c += nthreads) {
+    const int n = c / CH, j = c % CH;
+    const int64_t off = start + n * sn, first = ((off + t0) & ~(int64_t)(per - 1)) + j * per;
+    const int bytes = (int)min((int64_t)per, max((int64_t)0, off + L - first)) * esz;
+    cp_async16n(dst + (n * (TL + per) + j * per) * esz, src + (bytes > 0 ? first : 0) * esz, bytes);
+  }
+}
+
 // One (N x TL) tile of B or C for the CTA.  vec: raw bytes in the source dtype, [n][TL].
 // Otherwise the elements are converted while loading and stored as fp32 [n][TL].
 template <int TL>
@@ -110,9 +144,11 @@ __device__ __forceinline__ float raw_bc_at(const void* raw, int idx, int dtype) 
   return __half2float(reinterpret_cast<const __half*>(raw)[idx]);
 }
 
-// raw [n][TL] -> fp32 [TL][NP]; states >= N are written as zero.
-template <int TL, int NP>
-__device__ __forceinline__ void convert_bc(float* __restrict__ dst, const void* __restrict__ raw, int dtype, int N, int tid, int nthreads) {
+// raw [n][pitch] -> fp32 [TL][NP]; states >= N are written as zero.  PIECES with `per` > 0 (a power of two, elements per
+// piece): what fill_bc_pieces fetched, state n at its shift.
+template <int TL, int NP, bool PIECES = false>
+__device__ __forceinline__ void convert_bc(float* __restrict__ dst, const void* __restrict__ raw, int dtype, int N, int tid, int nthreads, int per = 0,
+                                           int64_t start = 0, int64_t sn = 0) {
   constexpr int NQ = NP / 4;
   for (int i = tid; i < NQ * TL; i += nthreads) {
     const int nq = i % NQ, tt = i / NQ;
@@ -120,7 +156,8 @@ __device__ __forceinline__ void convert_bc(float* __restrict__ dst, const void* 
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int n = nq * 4 + k;
-      v[k] = n < N ? raw_bc_at(raw, n * TL + tt, dtype) : 0.f;
+      const int at = PIECES ? n * (TL + per) + ((int)(start + n * sn) & max(per - 1, 0)) + tt : n * TL + tt;
+      v[k] = n < N ? raw_bc_at(raw, at, dtype) : 0.f;
     }
     *reinterpret_cast<float4*>(dst + tt * NP + nq * 4) = make_float4(v[0], v[1], v[2], v[3]);
   }

@@ -24,6 +24,7 @@ extern "C" int ssm_selective_scan_bwd(const ssm_scan_bwd_args* g, ssm_stream_t s
   SSM_REQUIRE(g->dout && g->du && g->ddelta && g->dA && g->dB && g->dC, SSM_ERR_NULL, "selective_scan_backward: missing pointer");
   SSM_REQUIRE(!a->z == !g->dz, SSM_ERR_NULL, "selective_scan_backward: dz must be given exactly when z is");
   fl.io_vec = fl.io_vec && aligned_to(g->dout, 16) && aligned_to(g->du, 16) && aligned_to(g->ddelta, 16) && (!g->dz || aligned_to(g->dz, 16));
+  fl.io_pieces = fl.io_pieces && aligned_to(g->dout, 16);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   switch (a->io_dtype) {
     case SSM_F32: return dispatch_bwd<float>(*g, fl, st);

@@ -16,7 +16,7 @@
 
 namespace ssmb {
 
-template <typename T, int NS, int LPR, bool SHARED>
+template <typename T, int NS, int LPR, bool SHARED, bool PIECES>
 struct BwdShape : ScanShape<NS, LPR> {
   using S = ScanShape<NS, LPR>;
   static constexpr int NW = (S::NP > 128 || S::RPW > 16) ? 2 : kScanWarps;  // warps per CTA
@@ -30,16 +30,19 @@ struct BwdShape : ScanShape<NS, LPR> {
   static constexpr int WARP_STAGE = SHARED ? 2 * S::NP * S::RPW * 4 : 0;  // dB / dC products of 4 steps: [2 * NP][RPW][4]
   static constexpr int WARP_WORK = WARP_ROWS + WARP_HIST + WARP_STAGE;
   // bytes
-  static constexpr int BC_RAW_BYTES = SHARED ? 2 * S::NP * TL * 4 : 0;
-  static constexpr int WARP_RAW_BYTES = 4 * S::RPW * TL * (int)sizeof(T);
+  static constexpr int RP = TL + (PIECES ? 16 / (int)sizeof(T) : 0);  // pitch of a raw row: rows that start anywhere take one 16-byte piece more
+  static constexpr int BC_RAW_BYTES = SHARED ? 2 * S::NP * (TL + (PIECES ? 4 : 0)) * 4 : 0;
+  static constexpr int WARP_RAW_BYTES = 4 * S::RPW * RP * (int)sizeof(T);
   static constexpr size_t kBytes = sizeof(float) * (BC_WORK + NW * WARP_WORK) + BC_RAW_BYTES + NW * WARP_RAW_BYTES;
   static_assert(kBytes <= 227 * 1024, "shared memory budget");
   static constexpr size_t bytes() { return kBytes; }
 };
 
-template <typename T, int NS, int LPR, bool SHARED>
-__global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShape<T, NS, LPR, SHARED>::NW == 4 ? 3 : 1) scan_bwd_kernel(const ssm_scan_bwd_args g, const ScanFlags fl) {
-  using S = BwdShape<T, NS, LPR, SHARED>;
+// PIECES: ragged rows or coefficients (see fill_rows_pieces); an instance of its own, because the offsets cost the aligned form 5-10 %
+template <typename T, int NS, int LPR, bool SHARED, bool PIECES>
+__global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32, BwdShape<T, NS, LPR, SHARED, PIECES>::NW == 4 ? 3 : 1)
+    scan_bwd_kernel(const ssm_scan_bwd_args g, const ScanFlags fl) {
+  using S = BwdShape<T, NS, LPR, SHARED, PIECES>;
   constexpr int NP = S::NP, RPW = S::RPW, ROWS = S::ROWS, TB = S::TB, TL = S::TL, TLP = S::TLP, NW = S::NW;
   constexpr int V = 16 / sizeof(T);
   constexpr int NT = NW * 32;
@@ -60,9 +63,9 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
   char* rawB = rawbase;
   char* rawC = rawbase + S::BC_RAW_BYTES / 2;
   T* rawU = reinterpret_cast<T*>(rawbase + S::BC_RAW_BYTES + warp * S::WARP_RAW_BYTES);
-  T* rawD = rawU + RPW * TL;
-  T* rawZ = rawD + RPW * TL;
-  T* rawO = rawZ + RPW * TL;
+  T* rawD = rawU + RPW * S::RP;
+  T* rawZ = rawD + RPW * S::RP;
+  T* rawO = rawZ + RPW * S::RP;
 
   const int b = blockIdx.y;
   const int d0 = blockIdx.x * ROWS;
@@ -108,17 +111,31 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
   const char* Bbase = reinterpret_cast<const char*>(a.Bm) + boff * bcsz;
   const char* Cbase = reinterpret_cast<const char*>(a.Cm) + coff * bcsz;
   const bool io_vec = fl.io_vec != 0, bc_vec = fl.bc_vec != 0;
-  const int raw_bc_dtype = bc_vec ? a.bc_dtype : SSM_F32;
+  // ragged rows and coefficients: the same asynchronous copies in 16-byte pieces, read at the row's own offset.  (With scalar loads
+  // between two barriers the tile's DRAM latency was exposed: 2 x 1024 rows, fp16, 3999 steps 2364 us against 1008 for 4000.)
+  const bool io_pieces = PIECES && !io_vec && fl.io_pieces, bc_pieces = PIECES && SHARED && !bc_vec && fl.bc_pieces;
+  const int raw_bc_dtype = bc_vec || bc_pieces ? a.bc_dtype : SSM_F32;
+  const int bc_per = bc_pieces ? 16 / bcsz : 0;
 
   const int ntiles = (L + TL - 1) / TL;
   const float Dv = a.D ? __ldg(a.D + d) : 0.f;
 
   auto fill_raw = [&](int t0) {
-    fill_rows_raw<T, RPW, TL>(rawU, gu, b, D, L, drow0, t0, io_vec, lane, a.row_sb, a.row_sd);
-    fill_rows_raw<T, RPW, TL>(rawD, gdl, b, D, L, drow0, t0, io_vec, lane, a.row_sb, a.row_sd);
-    fill_rows_raw<T, RPW, TL>(rawO, gdo, b, D, L, drow0, t0, io_vec, lane, a.row_sb, a.row_sd);
-    if (gz) fill_rows_raw<T, RPW, TL>(rawZ, gz, b, D, L, drow0, t0, io_vec, lane, a.row_sb, a.row_sd);
-    if (SHARED) {
+    if (io_pieces) {
+      fill_rows_pieces<T, RPW, TL>(rawU, gu, b, D, L, drow0, t0, lane, a.row_sb, a.row_sd);
+      fill_rows_pieces<T, RPW, TL>(rawD, gdl, b, D, L, drow0, t0, lane, a.row_sb, a.row_sd);
+      fill_rows_pieces<T, RPW, TL>(rawO, gdo, b, D, L, drow0, t0, lane, a.row_sb, a.row_sd);
+      if (gz) fill_rows_pieces<T, RPW, TL>(rawZ, gz, b, D, L, drow0, t0, lane, a.row_sb, a.row_sd);
+    } else {
+      fill_rows_raw<T, RPW, TL>(rawU, gu, b, D, L, drow0, t0, io_vec, lane, a.row_sb, a.row_sd);
+      fill_rows_raw<T, RPW, TL>(rawD, gdl, b, D, L, drow0, t0, io_vec, lane, a.row_sb, a.row_sd);
+      fill_rows_raw<T, RPW, TL>(rawO, gdo, b, D, L, drow0, t0, io_vec, lane, a.row_sb, a.row_sd);
+      if (gz) fill_rows_raw<T, RPW, TL>(rawZ, gz, b, D, L, drow0, t0, io_vec, lane, a.row_sb, a.row_sd);
+    }
+    if (bc_pieces) {
+      fill_bc_pieces<TL>(rawB, a.Bm, a.bc_dtype, boff, a.b_sn, N, t0, L, tid, NT);
+      fill_bc_pieces<TL>(rawC, a.Cm, a.bc_dtype, coff, a.c_sn, N, t0, L, tid, NT);
+    } else if (SHARED) {
       fill_bc_raw<TL>(rawB, Bbase, a.bc_dtype, a.b_sn, a.b_st, N, t0, L, bc_vec, tid, NT);
       fill_bc_raw<TL>(rawC, Cbase, a.bc_dtype, a.c_sn, a.c_st, N, t0, L, bc_vec, tid, NT);
     }
@@ -154,15 +171,24 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
         const int t = t0 + ch * V;
         float fu[V], fd[V], fz[V], fo[V], fdy[V], fzf[V];
         Vec16<T> v;
-        v.raw = *reinterpret_cast<const uint4*>(rawU + rr * TL + ch * V);
-        v.unpack(fu);
-        v.raw = *reinterpret_cast<const uint4*>(rawD + rr * TL + ch * V);
-        v.unpack(fd);
-        v.raw = *reinterpret_cast<const uint4*>(rawO + rr * TL + ch * V);
-        v.unpack(fo);
-        if (gz) {
-          v.raw = *reinterpret_cast<const uint4*>(rawZ + rr * TL + ch * V);
-          v.unpack(fz);
+        const int at = rr * (io_pieces ? S::RP : TL) + ch * V + (io_pieces ? row_shift<T>((int64_t)b * a.row_sb + (int64_t)dd * a.row_sd) : 0);
+        if (io_pieces) {
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            fu[i] = to_f<T>(rawU[at + i]), fd[i] = to_f<T>(rawD[at + i]), fo[i] = to_f<T>(rawO[at + i]);
+            if (gz) fz[i] = to_f<T>(rawZ[at + i]);
+          }
+        } else {
+          v.raw = *reinterpret_cast<const uint4*>(rawU + at);
+          v.unpack(fu);
+          v.raw = *reinterpret_cast<const uint4*>(rawD + at);
+          v.unpack(fd);
+          v.raw = *reinterpret_cast<const uint4*>(rawO + at);
+          v.unpack(fo);
+          if (gz) {
+            v.raw = *reinterpret_cast<const uint4*>(rawZ + at);
+            v.unpack(fz);
+          }
         }
         const float bias = a.dt_bias ? __ldg(a.dt_bias + dd) : 0.f;
 #pragma unroll
@@ -191,8 +217,8 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
       }
     }
     if (SHARED) {
-      convert_bc<TL, NP>(sB, rawB, raw_bc_dtype, N, tid, NT);
-      convert_bc<TL, NP>(sC, rawC, raw_bc_dtype, N, tid, NT);
+      convert_bc<TL, NP, PIECES>(sB, rawB, raw_bc_dtype, N, tid, NT, bc_per, boff, a.b_sn);
+      convert_bc<TL, NP, PIECES>(sC, rawC, raw_bc_dtype, N, tid, NT, bc_per, coff, a.c_sn);
     }
     __syncthreads();
     if (k > 0) fill_raw(t0 - TL);  // next (earlier) tile; overlaps the work below
@@ -503,7 +529,7 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED>::NW * 32, BwdShap
 
 template <typename T, int NS, int LPR>
 static int launch_bwd(const ssm_scan_bwd_args& g, ScanFlags fl, cudaStream_t st) {
-  using S1 = BwdShape<T, NS, LPR, false>;
+  using S1 = BwdShape<T, NS, LPR, false, false>;
   // the CTA-wide B / C / dB / dC tiles of more than 128 states do not fit next to the state
   // history; such rows read B / C from global memory and accumulate dB / dC there directly
   constexpr bool kCanShare = NS * LPR <= 128;
@@ -512,16 +538,18 @@ static int launch_bwd(const ssm_scan_bwd_args& g, ScanFlags fl, cudaStream_t st)
   dim3 grid((a.dim + S1::ROWS - 1) / S1::ROWS, a.batch);
   if constexpr (kCanShare) {
     if (fl.shared_bc) {
-      const size_t smem = BwdShape<T, NS, LPR, true>::bytes();
-      auto kern = scan_bwd_kernel<T, NS, LPR, true>;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      kern<<<grid, S1::NW * 32, smem, st>>>(g, fl);
-      return launch_status("scan_bwd_kernel");
+      auto launch = [&](auto kern, size_t smem) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kern<<<grid, S1::NW * 32, smem, st>>>(g, fl);
+        return launch_status("scan_bwd_kernel");
+      };
+      if ((!fl.io_vec && fl.io_pieces) || (!fl.bc_vec && fl.bc_pieces)) return launch(scan_bwd_kernel<T, NS, LPR, true, true>, BwdShape<T, NS, LPR, true, true>::bytes());
+      return launch(scan_bwd_kernel<T, NS, LPR, true, false>, BwdShape<T, NS, LPR, true, false>::bytes());
     }
   }
   {
-    const size_t smem = BwdShape<T, NS, LPR, false>::bytes();
-    auto kern = scan_bwd_kernel<T, NS, LPR, false>;
+    const size_t smem = S1::bytes();
+    auto kern = scan_bwd_kernel<T, NS, LPR, false, false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kern<<<grid, S1::NW * 32, smem, st>>>(g, fl);
   }

@@ -35,6 +35,8 @@ int ssmb::scan_validate(const ssm_scan_fwd_args* a, ScanFlags* fl, int rows_per_
     return st == 1 && aligned_to(p, 16) && sb % bv == 0 && sg % bv == 0 && sn % bv == 0;
   };
   fl->bc_vec = ok(a->Bm, a->b_sb, a->b_sg, a->b_sn, a->b_st) && ok(a->Cm, a->c_sb, a->c_sg, a->c_sn, a->c_st) && (a->len % bv == 0);
+  fl->io_pieces = aligned_to(a->u, 16) && aligned_to(a->delta, 16) && (!a->z || aligned_to(a->z, 16));
+  fl->bc_pieces = a->b_st == 1 && a->c_st == 1 && aligned_to(a->Bm, 16) && aligned_to(a->Cm, 16);
   fl->rows_per_group = a->dim / a->bc_groups;
   fl->shared_bc = (fl->rows_per_group % rows_per_cta == 0);
   return SSM_OK;

@@ -157,7 +157,15 @@ struct ScanCall final : Call {
     params.add(dA, {c.nd, c.nn});
     if (c.D.has_value()) params.add(dD, {c.nd});
     if (c.bias.has_value()) params.add(db, {c.nd});
-    coeffs.add(dB, c.B.t.sizes()), coeffs.add(dC, c.C.t.sizes());
+    // rows of dB and dC on 16-byte boundaries, so that the kernel's additions go out four steps at a time whatever the length
+    const int64_t lp = (c.nl + 3) / 4 * 4;
+    auto row_pitch = [&](const auto& k) { return k.st == 1 && k.t.dim() == 4 && k.t.size(3) == c.nl && k.sn == c.nl ? lp : c.nl; };
+    auto grad_shape = [&](const auto& k) {
+      std::vector<int64_t> shape = k.t.sizes().vec();
+      if (row_pitch(k) != c.nl) shape.back() = lp;
+      return shape;
+    };
+    coeffs.add(dB, grad_shape(c.B)), coeffs.add(dC, grad_shape(c.C));
     params.make(f32), coeffs.make(f32);
     if (init_grad) {  // an empty sequence hands the gradient of the last state straight to the initial state
       if (c.nl == 0) dinit = gl.has_value() ? gl->clone() : at::zeros({c.nb, c.nd, c.nn}, f32);
@@ -169,11 +177,16 @@ struct ScanCall final : Call {
     g.dout = go.data_ptr(), g.dlast_state = fptr(gl);
     g.du = du.data_ptr(), g.ddelta = dd.data_ptr(), g.dz = dz.defined() ? dz.data_ptr() : nullptr;
     g.dA = out_ptr(dA), g.dB = out_ptr(dB), g.dC = out_ptr(dC), g.dD = out_ptr(dD), g.ddt_bias = out_ptr(db);
-    g.db_sb = c.B.sb, g.db_sg = c.B.sg, g.db_sn = c.B.sn, g.db_st = c.B.st;
-    g.dc_sb = c.C.sb, g.dc_sg = c.C.sg, g.dc_sn = c.C.sn, g.dc_st = c.C.st;
+    auto scaled = [&](const auto& k, int64_t stride) { return row_pitch(k) != c.nl ? stride / c.nl * lp : stride; };
+    g.db_sb = scaled(c.B, c.B.sb), g.db_sg = scaled(c.B, c.B.sg), g.db_sn = scaled(c.B, c.B.sn), g.db_st = c.B.st;
+    g.dc_sb = scaled(c.C, c.C.sb), g.dc_sg = scaled(c.C, c.C.sg), g.dc_sn = scaled(c.C, c.C.sn), g.dc_st = c.C.st;
     g.dinitial_state = out_ptr(dinit);
     run(ssm_selective_scan_bwd(&g, stream_of(c.u)));
-    auto fold = [](Tensor grad, at::IntArrayRef shape, at::ScalarType t) {
+    auto fold = [&](Tensor grad, at::IntArrayRef shape, at::ScalarType t) {
+      if (grad.dim() == 4 && grad.size(3) != shape.back()) {
+        grad = grad.narrow(3, 0, shape.back());
+        if (t == at::kFloat || grad.sizes() != shape) grad = grad.contiguous();
+      }
       if (grad.sizes() != shape)  // the coefficient had been regrouped: sum the repeats back
         grad = grad.view({shape[0], shape[1], grad.size(1) / shape[1], shape[2], shape[3]}).sum(2);
       return cast(grad, t);

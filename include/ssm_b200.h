@@ -104,6 +104,8 @@ typedef struct {
 
 int ssm_scan_checkpoint_interval(void);
 int ssm_scan_split_segments(int32_t batch, int32_t dim, int32_t len, int32_t nstate);
+/* the same for the backward (its fwd.split_scratch / split_segments; d_state <= 32) */
+int ssm_scan_bwd_split_segments(int32_t batch, int32_t dim, int32_t len, int32_t nstate);
 int ssm_selective_scan_fwd(const ssm_scan_fwd_args* args, ssm_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------

@@ -148,6 +148,7 @@ ENTRY_POINTS = {
     "ssm_b200_launch_count": (C.c_int64, []),
     "ssm_scan_checkpoint_interval": (C.c_int, []),
     "ssm_scan_split_segments": (C.c_int, [i32, i32, i32, i32]),
+    "ssm_scan_bwd_split_segments": (C.c_int, [i32, i32, i32, i32]),
     "ssm_selective_scan_fwd": (C.c_int, [C.POINTER(ScanFwdArgs), vp]),
     "ssm_selective_scan_bwd": (C.c_int, [C.POINTER(ScanBwdArgs), vp]),
     "ssm_mamba1_decode_supported": (C.c_int, [i32] * 7),

@@ -2,6 +2,8 @@
 // instantiated per element type in selective_scan_bwd_*.cu.
 #include "scan_common.cuh"
 
+#include <algorithm>
+
 namespace ssmb {
 template <typename T>
 int dispatch_bwd(const ssm_scan_bwd_args& a, const ScanFlags& fl, cudaStream_t st);
@@ -12,6 +14,18 @@ int scan_validate(const ssm_scan_fwd_args* a, ScanFlags* fl, int rows_per_cta);
 }  // namespace ssmb
 
 using namespace ssmb;
+
+// Segments of a call cut in time: enough to offer every SM the three CTAs that it holds, each at least two tiles long.  A warp alone
+// on its scheduler takes about 500 cycles a step, three take 730 for three, and the pass that finds the segments' adjoints adds
+// about a fifth.  1 = no split.
+extern "C" int ssm_scan_bwd_split_segments(int32_t batch, int32_t dim, int32_t len, int32_t nstate) {
+  if (batch <= 0 || dim <= 0 || len <= 0 || nstate < 1 || nstate > 32) return 1;
+  const int rows = nstate <= 8 ? 64 : nstate <= 16 ? 32 : 16;  // of a CTA
+  const int64_t ctas = (int64_t)batch * ((dim + rows - 1) / rows);
+  const int tiles = (len + kScanCkpt - 1) / kScanCkpt;
+  const int64_t want = std::min<int64_t>(3ll * sm_count() / ctas, tiles / 2);
+  return want < 2 ? 1 : (int)std::min<int64_t>(want, 65535);
+}
 
 extern "C" int ssm_selective_scan_bwd(const ssm_scan_bwd_args* g, ssm_stream_t stream) {
   SSM_REQUIRE(g != nullptr, SSM_ERR_NULL, "selective_scan_backward: args is NULL");

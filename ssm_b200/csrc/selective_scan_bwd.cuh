@@ -38,10 +38,14 @@ struct BwdShape : ScanShape<NS, LPR> {
   static constexpr size_t bytes() { return kBytes; }
 };
 
+// A call whose rows alone cannot fill the machine is cut in time into gridDim.z segments of `seg_tiles` tiles.  The states need
+// nothing for it (every tile starts from its checkpoint); the adjoint that enters a segment from the right does.  CARRY: the pass
+// that finds it, the recurrence G alone from zero at every segment's end (the last one's: the gradient of the last state), which
+// leaves what the segment hands to the left and its decay product exp(A sum delta) for scan_bwd_combine_kernel.
 // PIECES: ragged rows or coefficients (see fill_rows_pieces); an instance of its own, because the offsets cost the aligned form 5-10 %
-template <typename T, int NS, int LPR, bool SHARED, bool PIECES>
+template <typename T, int NS, int LPR, bool SHARED, bool PIECES, bool CARRY>
 __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32, BwdShape<T, NS, LPR, SHARED, PIECES>::NW == 4 ? 3 : 1)
-    scan_bwd_kernel(const ssm_scan_bwd_args g, const ScanFlags fl) {
+    scan_bwd_kernel(const ssm_scan_bwd_args g, const ScanFlags fl, int seg_tiles) {
   using S = BwdShape<T, NS, LPR, SHARED, PIECES>;
   constexpr int NP = S::NP, RPW = S::RPW, ROWS = S::ROWS, TB = S::TB, TL = S::TL, TLP = S::TLP, NW = S::NW;
   constexpr int V = 16 / sizeof(T);
@@ -88,6 +92,13 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
   T* __restrict__ gdd = reinterpret_cast<T*>(g.ddelta);
   T* __restrict__ gdz = reinterpret_cast<T*>(g.dz);
 
+  const int seg = blockIdx.z, nseg = gridDim.z;
+  // split scratch: [2][batch][dim][nseg][N]: the adjoint a segment hands to the left (after the combine: the one that enters it from
+  // the right), then its decay product
+  float* split_g = nseg > 1 ? a.split_scratch + (row * nseg + seg) * N : nullptr;
+  float* split_p = nseg > 1 ? split_g + (int64_t)a.batch * D * nseg * N : nullptr;
+  float sumdl = 0.f;  // CARRY: sum of this row's delta over the segment
+
   // per-lane state as pairs of adjacent states for the packed-fp32 (f32x2) pipe
   float2 A2[NS / 2], carry[NS / 2], dAacc[NS / 2];
 #pragma unroll
@@ -95,8 +106,13 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
     const int n = sg * NS + j;
     A2[j / 2].x = n < N ? __ldg(a.A + (int64_t)d * N + n) * kLog2e : 0.f;
     A2[j / 2].y = n + 1 < N ? __ldg(a.A + (int64_t)d * N + n + 1) * kLog2e : 0.f;
-    carry[j / 2].x = (n < N && g.dlast_state) ? __ldg(g.dlast_state + row * N + n) : 0.f;
-    carry[j / 2].y = (n + 1 < N && g.dlast_state) ? __ldg(g.dlast_state + row * N + n + 1) : 0.f;
+    if (seg == nseg - 1) {
+      carry[j / 2].x = (n < N && g.dlast_state) ? __ldg(g.dlast_state + row * N + n) : 0.f;
+      carry[j / 2].y = (n + 1 < N && g.dlast_state) ? __ldg(g.dlast_state + row * N + n + 1) : 0.f;
+    } else {
+      carry[j / 2].x = !CARRY && n < N ? split_g[n] : 0.f;
+      carry[j / 2].y = !CARRY && n + 1 < N ? split_g[n + 1] : 0.f;
+    }
     dAacc[j / 2] = make_float2(0.f, 0.f);
   }
   float dDacc = 0.f, dBiasAcc = 0.f;  // this lane's share of the row's dD / ddt_bias
@@ -118,6 +134,7 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
   const int bc_per = bc_pieces ? 16 / bcsz : 0;
 
   const int ntiles = (L + TL - 1) / TL;
+  const int k_begin = seg * seg_tiles, k_end = min(ntiles, k_begin + seg_tiles);
   const float Dv = a.D ? __ldg(a.D + d) : 0.f;
 
   auto fill_raw = [&](int t0) {
@@ -152,12 +169,12 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
       hck[j / 2].y = (sg * NS + j + 1) < N ? __ldg(ck + sg * NS + j + 1) : 0.f;
     }
   };
-  if (ntiles > 0) {
-    fill_raw((ntiles - 1) * TL);
-    load_checkpoint(ntiles - 1);
+  if (k_begin < k_end) {
+    fill_raw((k_end - 1) * TL);
+    if (!CARRY) load_checkpoint(k_end - 1);
   }
 
-  for (int k = ntiles - 1; k >= 0; --k) {
+  for (int k = k_end - 1; k >= k_begin; --k) {
     const int t0 = k * TL;
     cp_async_wait_all();
     __syncthreads();  // raw tile k landed; previous tile's working arrays consumed, dB / dC flushed
@@ -221,7 +238,7 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
       convert_bc<TL, NP, PIECES>(sC, rawC, raw_bc_dtype, N, tid, NT, bc_per, coff, a.c_sn);
     }
     __syncthreads();
-    if (k > 0) fill_raw(t0 - TL);  // next (earlier) tile; overlaps the work below
+    if (k > k_begin) fill_raw(t0 - TL);  // next (earlier) tile; overlaps the work below
 
     const float* rDl = sDl + r * TLP;
     float* rU = sU + r * TLP;
@@ -254,12 +271,40 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
       }
     };
 
+    if constexpr (CARRY) {
+      __syncwarp();
+#pragma unroll 1
+      for (int tt = TL - 4; tt >= 0; tt -= 4) {
+        const float4 dl4 = *reinterpret_cast<const float4*>(rDl + tt), dy4 = *reinterpret_cast<const float4*>(rDy + tt);
+        const float dl[4] = {dl4.x, dl4.y, dl4.z, dl4.w}, dy[4] = {dy4.x, dy4.y, dy4.z, dy4.w};
+        sumdl += (dl4.x + dl4.y) + (dl4.z + dl4.w);
+        float2 da[4][NS / 2], cd[4][NS / 2];  // decays and C dy: what does not depend on the adjoint
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float cv[NS];
+          load_bc(sC, Cbase, a.c_sn, a.c_st, tt + i, cv);
+#pragma unroll
+          for (int j = 0; j < NS; j += 2) {
+            const float2 e = __fmul2_rn(make_float2(dl[i], dl[i]), A2[j / 2]);
+            da[i][j / 2] = make_float2(ex2_approx(e.x), ex2_approx(e.y));
+            cd[i][j / 2] = __fmul2_rn(make_float2(cv[j], cv[j + 1]), make_float2(dy[i], dy[i]));
+          }
+        }
+#pragma unroll
+        for (int i = 3; i >= 0; --i) {
+#pragma unroll
+          for (int j = 0; j < NS / 2; ++j) carry[j] = __fmul2_rn(da[i][j], __fadd2_rn(cd[i][j], carry[j]));
+        }
+      }
+      continue;
+    }
+
     // ---- rebuild the tile's states from the checkpoint -----------------------------------------
     {
       float2 h[NS / 2];
 #pragma unroll
       for (int j = 0; j < NS / 2; ++j) h[j] = hck[j];
-      if (k > 0) load_checkpoint(k - 1);  // for the next (earlier) tile: its latency hides behind this tile's work
+      if (k > k_begin) load_checkpoint(k - 1);  // for the next (earlier) tile: its latency hides behind this tile's work
       hist_store(0, h);
 #pragma unroll 2
       for (int tb0 = 0; tb0 < TL; tb0 += TB) {
@@ -503,9 +548,20 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
     }
   }
 
+  if constexpr (CARRY) {
+    if (row_ok) {
+#pragma unroll
+      for (int j = 0; j < NS; j += 2) {
+        const int n = sg * NS + j;
+        if (n < N) split_g[n] = carry[j / 2].x, split_p[n] = ex2_approx(sumdl * A2[j / 2].x);
+        if (n + 1 < N) split_g[n + 1] = carry[j / 2].y, split_p[n + 1] = ex2_approx(sumdl * A2[j / 2].y);
+      }
+    }
+    return;
+  }
   dDacc = group_sum<LPR, RPW>(dDacc);
   dBiasAcc = group_sum<LPR, RPW>(dBiasAcc);
-  if (g.dinitial_state && row_ok) {  // what the adjoint carries past step 0 is the gradient of the state before it
+  if (g.dinitial_state && row_ok && seg == 0) {  // what the adjoint carries past step 0 is the gradient of the state before it
 #pragma unroll
     for (int j = 0; j < NS; j += 2) {
       const int n = sg * NS + j;
@@ -527,6 +583,22 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
   }
 }
 
+// Serial pass over the segments, last to first: split_g[s] <- adjoint entering segment s from the right.  One thread per (row, state).
+static __global__ void __launch_bounds__(128) scan_bwd_combine_kernel(float* __restrict__ split, int64_t rows_states, int nstate, int nseg) {
+  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (i >= rows_states) return;
+  const int64_t row = i / nstate;
+  float* gs = split + row * nseg * nstate + i % nstate;
+  const float* ps = gs + rows_states * nseg;
+  float in = 0.f;  // the last segment started from the gradient of the last state already, and its replay reads that again
+  for (int s = nseg - 1; s >= 0; --s) {
+    const float local = gs[(int64_t)s * nstate];
+    const float p = ps[(int64_t)s * nstate];
+    gs[(int64_t)s * nstate] = in;
+    in = s == nseg - 1 ? local : fmaf(p, in, local);
+  }
+}
+
 template <typename T, int NS, int LPR>
 static int launch_bwd(const ssm_scan_bwd_args& g, ScanFlags fl, cudaStream_t st) {
   using S1 = BwdShape<T, NS, LPR, false, false>;
@@ -538,20 +610,38 @@ static int launch_bwd(const ssm_scan_bwd_args& g, ScanFlags fl, cudaStream_t st)
   dim3 grid((a.dim + S1::ROWS - 1) / S1::ROWS, a.batch);
   if constexpr (kCanShare) {
     if (fl.shared_bc) {
+      const int ntiles = (a.len + kScanCkpt - 1) / kScanCkpt;
+      const int nseg = a.split_scratch && a.split_segments > 1 ? a.split_segments : 1;
+      const int seg_tiles = (ntiles + nseg - 1) / nseg, used = (ntiles + seg_tiles - 1) / seg_tiles;  // segments that hold a tile
+      grid.z = used;
       auto launch = [&](auto kern, size_t smem) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, S1::NW * 32, smem, st>>>(g, fl);
+        kern<<<grid, S1::NW * 32, smem, st>>>(g, fl, seg_tiles);
         return launch_status("scan_bwd_kernel");
       };
-      if ((!fl.io_vec && fl.io_pieces) || (!fl.bc_vec && fl.bc_pieces)) return launch(scan_bwd_kernel<T, NS, LPR, true, true>, BwdShape<T, NS, LPR, true, true>::bytes());
-      return launch(scan_bwd_kernel<T, NS, LPR, true, false>, BwdShape<T, NS, LPR, true, false>::bytes());
+      const bool pieces = (!fl.io_vec && fl.io_pieces) || (!fl.bc_vec && fl.bc_pieces);
+      using P0 = BwdShape<T, NS, LPR, true, false>;
+      using P1 = BwdShape<T, NS, LPR, true, true>;
+      if constexpr (NS * LPR <= 32) {
+        if (used > 1) {
+          const int rc = pieces ? launch(scan_bwd_kernel<T, NS, LPR, true, true, true>, P1::bytes()) : launch(scan_bwd_kernel<T, NS, LPR, true, false, true>, P0::bytes());
+          if (rc) return rc;
+          const int64_t rs = (int64_t)a.batch * a.dim * a.nstate;
+          scan_bwd_combine_kernel<<<(unsigned)((rs + 127) / 128), 128, 0, st>>>(a.split_scratch, rs, a.nstate, used);
+          if (int rc2 = launch_status("scan_bwd_combine_kernel")) return rc2;
+        }
+      } else {
+        SSM_REQUIRE(used == 1, SSM_ERR_UNSUPPORTED, "selective_scan_backward: calls of more than 32 states are not cut in time");
+      }
+      if (pieces) return launch(scan_bwd_kernel<T, NS, LPR, true, true, false>, P1::bytes());
+      return launch(scan_bwd_kernel<T, NS, LPR, true, false, false>, P0::bytes());
     }
   }
   {
     const size_t smem = S1::bytes();
-    auto kern = scan_bwd_kernel<T, NS, LPR, false, false>;
+    auto kern = scan_bwd_kernel<T, NS, LPR, false, false, false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<grid, S1::NW * 32, smem, st>>>(g, fl);
+    kern<<<grid, S1::NW * 32, smem, st>>>(g, fl, (a.len + kScanCkpt - 1) / kScanCkpt);
   }
   return launch_status("scan_bwd_kernel");
 }

@@ -181,6 +181,12 @@ struct ScanCall final : Call {
     g.db_sb = scaled(c.B, c.B.sb), g.db_sg = scaled(c.B, c.B.sg), g.db_sn = scaled(c.B, c.B.sn), g.db_st = c.B.st;
     g.dc_sb = scaled(c.C, c.C.sb), g.dc_sg = scaled(c.C, c.C.sg), g.dc_sn = scaled(c.C, c.C.sn), g.dc_st = c.C.st;
     g.dinitial_state = out_ptr(dinit);
+    const int nseg = ssm_scan_bwd_split_segments((int)c.nb, (int)c.nd, (int)c.nl, (int)c.nn);
+    Tensor split;
+    if (nseg > 1) {
+      split = at::empty({2 * c.nb * c.nd * nseg * c.nn}, f32);
+      g.fwd.split_scratch = split.data_ptr<float>(), g.fwd.split_segments = nseg;
+    }
     run(ssm_selective_scan_bwd(&g, stream_of(c.u)));
     auto fold = [&](Tensor grad, at::IntArrayRef shape, at::ScalarType t) {
       if (grad.dim() == 4 && grad.size(3) != shape.back()) {

@@ -1,5 +1,5 @@
-"""Selective scan on rows that do not start on 16-byte boundaries, against the fp32 oracle: lengths around the tile of 32 steps and the
-vector widths, a call that is cut in time, padded state counts, several B / C groups, and B / C with a stride over time."""
+"""Selective scan on ragged rows and on calls that are cut in time, against the fp32 oracle: lengths around the tile of 32 steps and the
+vector widths, whole vectors, padded state counts, several B / C groups, gradients of the first and last states across the cuts."""
 
 from __future__ import annotations
 
@@ -13,19 +13,20 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("nb,dim,length,n,groups", [(2, 64, 1, 16, 1), (1, 32, 31, 16, 1), (2, 96, 33, 5, 1), (1, 64, 301, 16, 2), (3, 64, 95, 32, 1), (1, 32, 67, 3, 1)])
-def test_ragged_rows(nb, dim, length, n, groups, dtype):
+@pytest.mark.parametrize("nb,dim,length,n,groups", [(2, 64, 1, 16, 1), (1, 32, 31, 16, 1), (2, 96, 33, 5, 1), (1, 64, 301, 16, 2), (3, 64, 95, 32, 1), (1, 32, 67, 3, 1),
+                                                    (1, 32, 64, 16, 1), (2, 32, 416, 16, 1), (1, 64, 1000, 8, 1), (1, 32, 129, 32, 1)])
+def test_scan_edges(nb, dim, length, n, groups, dtype):
     g = torch.Generator().manual_seed(length)
     r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
     u, delta, z = (r(nb, dim, length).to(dtype) for _ in range(3))
     A, D, bias = -torch.exp(r(dim, n) * 0.5), r(dim), r(dim) * 0.3 - 1.0
     B, C = (r(nb, groups, n, length).to(dtype) for _ in range(2))
-    go = r(nb, dim, length).to(dtype)
+    init, go, gl = r(nb, dim, n), r(nb, dim, length).to(dtype), r(nb, dim, n)
 
     def both(fn, dev, cast):
-        t = [x.to(dev).to(cast(x)).requires_grad_() for x in (u, delta, A, B, C, D, z, bias)]
-        out, last = fn(t[0], t[1], t[2], t[3], t[4], D=t[5], z=t[6], dt_bias=t[7], softplus=True, return_last_state=True)
-        return [out, last, *torch.autograd.grad(out, t, go.to(dev).to(out.dtype))]
+        t = [x.to(dev).to(cast(x)).requires_grad_() for x in (u, delta, A, B, C, D, z, bias, init)]
+        out, last = fn(t[0], t[1], t[2], t[3], t[4], D=t[5], z=t[6], dt_bias=t[7], softplus=True, return_last_state=True, initial_state=t[8])
+        return [out, last, *torch.autograd.grad((out, last), t, (go.to(dev).to(out.dtype), gl.to(dev).to(last.dtype)))]
 
     got = both(ops.selective_scan, "cuda", lambda x: x.dtype)
     want = both(oracle.selective_scan, "cpu", lambda x: torch.float32)

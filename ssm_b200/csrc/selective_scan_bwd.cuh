@@ -591,11 +591,18 @@ static __global__ void __launch_bounds__(128) scan_bwd_combine_kernel(float* __r
   float* gs = split + row * nseg * nstate + i % nstate;
   const float* ps = gs + rows_states * nseg;
   float in = 0.f;  // the last segment started from the gradient of the last state already, and its replay reads that again
-  for (int s = nseg - 1; s >= 0; --s) {
-    const float local = gs[(int64_t)s * nstate];
-    const float p = ps[(int64_t)s * nstate];
-    gs[(int64_t)s * nstate] = in;
-    in = s == nseg - 1 ? local : fmaf(p, in, local);
+  for (int s0 = nseg - 1; s0 >= 0; s0 -= 8) {  // loads first, as in the forward's
+    float local[8], p[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int64_t at = (int64_t)max(s0 - k, 0) * nstate;
+      local[k] = gs[at], p[k] = ps[at];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (s0 - k >= 0) gs[(int64_t)(s0 - k) * nstate] = in;
+      in = s0 - k == nseg - 1 ? local[k] : fmaf(p[k], in, local[k]);
+    }
   }
 }
 

@@ -116,10 +116,11 @@ __global__ void __launch_bounds__(256) ssd_bwd_finish_kernel(const ssm_ssd_bwd_a
   }
 }
 
-// One CTA per (batch, chunk, eight heads).  The per-step values are read as they lie in memory (heads innermost) and transposed through
-// shared memory; then a warp per head forms the product <state, adjoint> at the chunk's left boundary (fp32, 8192 terms each)
-// and the running sum of qd - u over the chunk's 256 steps, eight of them per lane.
-constexpr int kStepHeads = 8, kStepLd = kQ + 4;
+// One CTA per (batch, chunk, four heads).  The per-step values are read as they lie in memory (heads innermost) and transposed through
+// shared memory; two warps per head form the product <state, adjoint> at the chunk's left boundary (fp32, 8192 terms; what the kernel
+// spends its time on: a warp per head and eight heads per CTA left too few loads in flight, 43 us against 28 for 2 x 4001 steps, 48 heads),
+// then one of them the running sum of qd - u over the chunk's 256 steps, eight of them per lane.
+constexpr int kStepHeads = 4, kStepLd = kQ + 4;
 template <typename T>
 __global__ void __launch_bounds__(kQ) ssd_bwd_steps_kernel(const ssm_ssd_steps_args a, int nchunks) {
   __shared__ __align__(16) float sPre[kStepHeads][kStepLd], sQ[kStepHeads][kStepLd], sR[kStepHeads][kStepLd];
@@ -137,24 +138,28 @@ __global__ void __launch_bounds__(kQ) ssd_bwd_steps_kernel(const ssm_ssd_steps_a
     }
     sPre[hh][t] = pre, sQ[hh][t] = q, sR[hh][t] = r;
   }
+  static_assert(kQ / 32 == 2 * kStepHeads, "two warps per head");
+  __shared__ float sDot[2 * kStepHeads];
+  if (warp % kStepHeads < nh && c > 0) {
+    const int h = h0 + warp % kStepHeads, part = warp / kStepHeads * (kP * kN / 8);
+    const float4* s = reinterpret_cast<const float4*>(a.state_f32 + (((int64_t)b * nchunks + c) * a.heads + h) * (kP * kN)) + part;
+    const float4* g = reinterpret_cast<const float4*>(a.adjoint_f32 + (((int64_t)b * nchunks + c - 1) * a.heads + h) * (kP * kN)) + part;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int i = lane; i < kP * kN / 8; i += 32) {
+      const float4 x = __ldcs(s + i), y = __ldcs(g + i);
+      acc.x = fmaf(x.x, y.x, acc.x), acc.y = fmaf(x.y, y.y, acc.y), acc.z = fmaf(x.z, y.z, acc.z), acc.w = fmaf(x.w, y.w, acc.w);
+    }
+    const float dot = warp_sum((acc.x + acc.y) + (acc.z + acc.w));
+    if (lane == 0) sDot[warp] = dot;
+  }
   __syncthreads();
   if (warp < nh) {
     const int h = h0 + warp;
     const float Ah = __ldg(a.A + h);
     float start = 0.f;
-    if (c > 0) {
-      const float4* s = reinterpret_cast<const float4*>(a.state_f32 + (((int64_t)b * nchunks + c) * a.heads + h) * (kP * kN));
-      const float4* g = reinterpret_cast<const float4*>(a.adjoint_f32 + (((int64_t)b * nchunks + c - 1) * a.heads + h) * (kP * kN));
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-      for (int i = lane; i < kP * kN / 4; i += 32) {
-        const float4 x = __ldcs(s + i), y = __ldcs(g + i);
-        acc.x = fmaf(x.x, y.x, acc.x), acc.y = fmaf(x.y, y.y, acc.y), acc.z = fmaf(x.z, y.z, acc.z), acc.w = fmaf(x.w, y.w, acc.w);
-      }
-      start = warp_sum((acc.x + acc.y) + (acc.z + acc.w)) * ex2_approx(__ldg(a.ws_cum + (((int64_t)b * a.heads + h) * nchunks + c) * kQ));
-    } else if (a.start0) {
-      start = __ldg(a.start0 + b * a.heads + h);
-    }
+    if (c > 0) start = (sDot[warp] + sDot[warp + kStepHeads]) * ex2_approx(__ldg(a.ws_cum + (((int64_t)b * a.heads + h) * nchunks + c) * kQ));
+    else if (a.start0) start = __ldg(a.start0 + b * a.heads + h);
     float r[8], run = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) r[k] = sR[warp][lane * 8 + k], run += r[k];

@@ -167,7 +167,10 @@ constexpr int kStateCopyWarp = 8, kStateMmaWarp = 9;
 // REV: the adjoint recurrence.  The chunks are walked from the last to the first with dy, C and B in the places of x, B and C; the
 // local sum is taken to a chunk's first step, sum_i exp2(c_i - c_0) C_i dy_i^T, and what is handed out is the adjoint that enters a
 // chunk from the right (the adjoint state at the next chunk's first step; the decay of that step belongs to the walk).
-template <typename T, int HPC, int NST, bool REV>
+// PACKED: the walk covers one of several sequences that follow one another along the time axis.  Rows behind its end belong to the next
+// one and must not reach the sums in any form (0 x Inf is NaN): K slices of 16 steps beyond the end are not multiplied, and the
+// rows of the slice in which it ends are overwritten with zeros, in x and in B.
+template <typename T, int HPC, int NST, bool REV, bool PACKED>
 __global__ void __launch_bounds__(kStateThreads, 1) ssd_state_kernel(const ssm_ssd_args a, const __grid_constant__ StateMaps maps, int nchunks) {
   using M = StateSmem<HPC, NST>;
   constexpr int kStep = M::kStep, NS = M::NSTAGE;
@@ -188,7 +191,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) ssd_state_kernel(const ssm_s
   const int g = h0 / (a.heads / a.groups);
   // b: batch element of the operands; sb: whose state this is (the packed sequence, or b); the walk covers chunks c_off ..
   // c_off + nwalk, whose first step is t_off
-  const bool packed = a.seq_table != nullptr;
+  constexpr bool packed = PACKED;
   const int sb = blockIdx.y, b = packed ? 0 : sb;
   const int* seq_first = packed ? a.seq_table + 2 * a.num_chunks + sb : nullptr;
   const int c_off = packed ? __ldg(seq_first) : 0;
@@ -218,6 +221,8 @@ __global__ void __launch_bounds__(kStateThreads, 1) ssd_state_kernel(const ssm_s
 
   const int64_t vrow0 = (((int64_t)b * a.heads + h0) * nchunks + c_off) * kQ;  // exponent vectors of head h0 (next head: + nchunks * kQ)
   const int nst = SPC * nwalk;
+  // steps of the sequence from the first step of a stage on (packed sequences only; the first stage of a chunk has at least one)
+  auto steps_left = [&](int c, int part) { return __ldg(a.seq_table + 2 * (c_off + c) + 1) - (t_off + c * kQ + part * kStep); };
   auto chunk_of = [&](int c) { return REV ? nwalk - 1 - c : c; };  // c-th chunk of the walk
   // stage s = steps [s * 64, s * 64 + 64), issued by one thread: two boxes of B, one box of x per head, and the exponents.
   // Steps beyond the sequence read as zero.
@@ -279,9 +284,10 @@ __global__ void __launch_bounds__(kStateThreads, 1) ssd_state_kernel(const ssm_s
         constexpr uint32_t idesc = tc::instr_desc(kN, HPC * kP, fmt, 1, 1);
         const uint64_t da0 = tc::smem_desc_sw128(tc::smem_u32(base), M::BLK_BYTES, 1024);
         const uint64_t db0 = tc::smem_desc_sw128(tc::smem_u32(base + M::A_BYTES), M::BLK_BYTES, 1024);
+        const int live = packed && c == nwalk - 1 ? steps_left(c, part) : kStep;
 #pragma unroll
         for (int kk = 0; kk < kStep / 16; ++kk)  // 16 steps = 16 rows of 128 bytes
-          tc::mma_ss(tmem + (c & 1) * HPC * 64, da0 + (uint64_t)(kk * (2048 >> 4)), db0 + (uint64_t)(kk * (2048 >> 4)), idesc, part > 0 || kk > 0);
+          if (kk * 16 < live) tc::mma_ss(tmem + (c & 1) * HPC * 64, da0 + (uint64_t)(kk * (2048 >> 4)), db0 + (uint64_t)(kk * (2048 >> 4)), idesc, part > 0 || kk > 0);
         tc::commit(tc::smem_u32(&mbar_free[s % NS]));
         if (part == SPC - 1) tc::commit(tc::smem_u32(&mbar_acc[c & 1]));
       }
@@ -414,9 +420,16 @@ __global__ void __launch_bounds__(kStateThreads, 1) ssd_state_kernel(const ssm_s
 #pragma unroll
           for (int i = 0; i < 8; ++i) f[i] *= w;
           v.pack(f);
-          if (packed && w == 0.f) v.raw = make_uint4(0, 0, 0, 0);  // what follows is another sequence
           *reinterpret_cast<uint4*>(xs + hh * M::BLK_BYTES + (size_t)(gtid + kStateGroupThreads * k) * 16) = v.raw;
         }
+      }
+    }
+    if (packed && c == nwalk - 1) {  // the last chunk: zeros behind the sequence, by the threads that have scaled these units of x
+      const int live = steps_left(c, part);
+      if (live > 0 && live < kStep && (gtid >> 3) >= (live & 15)) {
+#pragma unroll
+        for (int blk = 0; blk < 2 + HPC; ++blk)
+          *reinterpret_cast<uint4*>(smraw + (s % NS) * M::STAGE + blk * M::BLK_BYTES + (size_t)(gtid + kStateGroupThreads * (live >> 4)) * 16) = make_uint4(0, 0, 0, 0);
       }
     }
     // the scaled rows become visible to the tensor cores' reads.  A warp whose wait ran out still arrives, so that the others do
@@ -551,7 +564,10 @@ struct ScanMaps {
 // REV: the adjoint pass, dx_j = dt_j (sum_{i >= j} exp2(c_i - c_j) (B_j . C_i) dy_i + exp2(off - c_j) G B_j), with B, C and dy in the places of C, B
 // and x, and G the adjoint that enters the chunk from the right (off: the decay of the chunk and of the step after it).  It is the
 // mirror image in time: columns at or after the row's step, the long block is rows 0..127.
-template <typename T, int MB, bool XSKIP, bool REV>
+// PACKED: several sequences along the time axis; rows behind the end of a chunk's sequence belong to the next one.  Their columns of the
+// mask are zero, but 0 x Inf is NaN: K slices of 16 steps beyond the end are not multiplied, and the x rows of the slice in
+// which it ends are overwritten with zeros.
+template <typename T, int MB, bool XSKIP, bool REV, bool PACKED>
 __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanMaps& maps, int nchunks, int hpc, int nparts, unsigned char* smraw,
                                               uint64_t* mbar, uint32_t* tmem_slot) {
   using M = ScanSmem<T>;
@@ -589,12 +605,13 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   const int h0 = part * hpc;
   const int nh = min(hpc, a.heads - h0);
   const int g = h0 / (a.heads / a.groups);
-  const int t0 = chunk_begin(a, c);
+  const int t0 = PACKED ? chunk_begin(a, c) : c * kQ;
   // rows of this block that exist; a ragged block of a packed sequence stores its rows by hand (what follows them belongs to
   // the next sequence), everything else leaves through TMA, which cuts at the end of the tensor
-  const int t_live = chunk_limit(a, c) - t0 - ROW0;
-  const bool ragged = a.seq_table != nullptr && t_live < kBlk;
+  const int t_live = PACKED ? chunk_limit(a, c) - t0 - ROW0 : kBlk;
+  const bool ragged = PACKED && t_live < kBlk;
   if (ragged && t_live <= 0) return;  // the whole CTA: nothing has been issued yet
+  const int k_live = ragged ? t_live + ROW0 - COL0 : KJ;  // columns that belong to the sequence
   const int i_loc = (warp & 3) * 32 + lane;    // row within the block = TMEM lane
   const int i_chunk = ROW0 + i_loc;            // row within the chunk
   const int rc = (ROW0 - COL0) / 32 + (warp & 3);  // this warp's rows as a 32-step chunk index, counted like the columns
@@ -756,6 +773,10 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   for (int hi = 0; hi < nh; ++hi) {
     const int h = h0 + hi, buf = hi & 1;
     ok = !fail && tc::mbar_wait(mb_full(buf), (hi >> 1) & 1);  // this head's operands (no more waiting once a wait ran out)
+    if (ragged && tid < (-k_live & 15) * 8) {  // x rows of the next sequence in the last K slice
+      *reinterpret_cast<uint4*>(sX + buf * M::X_BYTES + (size_t)(k_live * 8 + tid) * 16) = make_uint4(0, 0, 0, 0);
+      tc::fence_async_smem();
+    }
     // ---- factors of the decay mask, formed before the CTA-wide barrier below so that their latency (shared-memory reads, ex2,
     // the exchange of the column factors through sW) overlaps the wait for the slowest warp; the barrier also orders the
     // writes to sW before the reads of the other lanes
@@ -885,9 +906,8 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            float w = ex2_approx(re - col(jb + q + e));
-            if (diag && (REV ? q + e < lane : q + e > lane)) w = 0.f;
-            f[e] = vG[k][q + e] * w;
+            const bool cut = diag && (REV ? q + e < lane : q + e > lane);  // selected and not multiplied by zero: G may be Inf there
+            f[e] = cut ? 0.f : vG[k][q + e] * ex2_approx(re - col(jb + q + e));
             if (!REV && diag && q + e == lane) f[e] += Dfold;
           }
           Vec16<T> o;
@@ -918,7 +938,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
       const uint32_t dY = tmem + 256 + buf * 128;
 #pragma unroll
       for (int kk = 0; kk < KJ / 16; ++kk)  // 16 steps = 16 rows of 128 bytes of the x tile
-        tc::mma_ts(dY, tmem + kk * 8, dx0 + (uint64_t)(kk * (2048 >> 4)), idY, kk > 0);  // A: 16 steps = 8 columns of the masked rows
+        if (!PACKED || kk * 16 < k_live) tc::mma_ts(dY, tmem + kk * 8, dx0 + (uint64_t)(kk * (2048 >> 4)), idY, kk > 0);  // A: 16 steps = 8 columns of the masked rows
       tc::commit(mb_mma(buf));
     }
     // ---- the previous head's result, while the tensor cores work on this one ---------------------------------
@@ -968,7 +988,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   if (fail && tid == 0 && a.status) *(volatile int32_t*)a.status = 2;
 }
 
-template <typename T, bool XSKIP, bool REV>
+template <typename T, bool XSKIP, bool REV, bool PACKED>
 __global__ void __launch_bounds__(kScanThreads, 1)
     ssd_scan_kernel(const ssm_ssd_args a, const __grid_constant__ ScanMaps maps, int nchunks, int hpc, int nparts) {
   extern __shared__ unsigned char smdyn[];
@@ -982,21 +1002,21 @@ __global__ void __launch_bounds__(kScanThreads, 1)
   }
   __syncthreads();  // barriers and the TMEM address are set up before anyone arms or polls them
   // the heavier blocks (rows 128..255; REV: rows 0..127) are scheduled first
-  if ((int)blockIdx.x < (int)(gridDim.x >> 1)) ssd_scan_body<T, 1, XSKIP, REV>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
-  else ssd_scan_body<T, 0, XSKIP, REV>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
+  if ((int)blockIdx.x < (int)(gridDim.x >> 1)) ssd_scan_body<T, 1, XSKIP, REV, PACKED>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
+  else ssd_scan_body<T, 0, XSKIP, REV, PACKED>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem_slot, 512);
 }
 
-template <typename T, int HPC, int NST, bool REV>
+template <typename T, int HPC, int NST, bool REV, bool PACKED>
 static int ssd_state_launch(const ssm_ssd_args& a, int nchunks, cudaStream_t st) {
   StateMaps maps;
   using M = StateSmem<HPC, NST>;
   if (int rc = encode_rows_map(&maps.b, a.Bm, a.batch, a.len, a.groups, kN, M::kStep, a.io_dtype)) return rc;
   if (int rc = encode_rows_map(&maps.x, a.X, a.batch, a.len, a.heads, kP, M::kStep, a.io_dtype)) return rc;
-  cudaFuncSetAttribute(ssd_state_kernel<T, HPC, NST, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::ALLOC);
-  ssd_state_kernel<T, HPC, NST, REV><<<dim3(a.heads / HPC, a.num_seqs ? a.num_seqs : a.batch), kStateThreads, M::ALLOC, st>>>(a, maps, nchunks);
+  cudaFuncSetAttribute(ssd_state_kernel<T, HPC, NST, REV, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::ALLOC);
+  ssd_state_kernel<T, HPC, NST, REV, PACKED><<<dim3(a.heads / HPC, a.num_seqs ? a.num_seqs : a.batch), kStateThreads, M::ALLOC, st>>>(a, maps, nchunks);
   return launch_status("ssd_state_kernel");
 }
 
@@ -1029,23 +1049,23 @@ __global__ void __launch_bounds__(32) ssd_wait_selftest_kernel(int32_t* status, 
   if (!ok && threadIdx.x == 0 && status) *(volatile int32_t*)status = 3;
 }
 
-template <typename T, bool REV>
+template <typename T, bool REV, bool PACKED>
 static int ssd_state_dispatch(const ssm_ssd_args& a, int hpc, int nchunks, cudaStream_t st) {
-  switch (hpc) {
-    // as many stages as fit: the ring's round trip (a copy's 2300 cycles, the waits and fences of three roles) is what bounds the walk.
-    // 96 walks of 4001 steps: 39 us with four stages and eight warps per stage, 38 with four per stage, 32 with eight stages
-    case 1: return ssd_state_launch<T, 1, 8, REV>(a, nchunks, st);
-    case 2: return ssd_state_launch<T, 2, 6, REV>(a, nchunks, st);
-    case 3: return ssd_state_launch<T, 3, 5, REV>(a, nchunks, st);
-    default: return ssd_state_launch<T, 4, 4, REV>(a, nchunks, st);
+  // as many stages as fit: the ring's round trip (a copy's 2300 cycles, the waits and fences of three roles) is what bounds the walk.
+  // 96 walks of 4001 steps: 39 us with four stages and eight warps per stage, 38 with four per stage, 32 with eight stages
+  if (hpc == 1) return ssd_state_launch<T, 1, 8, REV, PACKED>(a, nchunks, st);
+  if (PACKED || hpc == 2) return ssd_state_launch<T, 2, 6, REV, PACKED>(a, nchunks, st);  // packed sequences: at most two
+  if constexpr (!PACKED) {
+    if (hpc == 3) return ssd_state_launch<T, 3, 5, REV, false>(a, nchunks, st);
+    return ssd_state_launch<T, 4, 4, REV, false>(a, nchunks, st);
   }
 }
 
-template <typename T, bool XSKIP, bool REV>
+template <typename T, bool XSKIP, bool REV, bool PACKED>
 static int ssd_scan_launch(const ssm_ssd_args& a, const ScanMaps& maps, unsigned ctas, int nchunks, int hpc, int nparts, cudaStream_t st) {
   const size_t smem = ScanSmem<T>::ALLOC;
-  cudaFuncSetAttribute(ssd_scan_kernel<T, XSKIP, REV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  ssd_scan_kernel<T, XSKIP, REV><<<ctas, kScanThreads, smem, st>>>(a, maps, nchunks, hpc, nparts);
+  cudaFuncSetAttribute(ssd_scan_kernel<T, XSKIP, REV, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  ssd_scan_kernel<T, XSKIP, REV, PACKED><<<ctas, kScanThreads, smem, st>>>(a, maps, nchunks, hpc, nparts);
   return launch_status("ssd_scan_kernel");
 }
 
@@ -1104,7 +1124,10 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
     int shpc = (int)(((int64_t)walks * a.heads + sm_count() - 1) / sm_count());
     shpc = shpc < 1 ? 1 : (shpc > most ? most : shpc);
     while (hpg % shpc != 0) --shpc;
-    if (int rc = a.reverse ? ssd_state_dispatch<T, true>(a, shpc, nchunks, st) : ssd_state_dispatch<T, false>(a, shpc, nchunks, st)) return rc;
+    const int rc = a.reverse    ? ssd_state_dispatch<T, true, false>(a, shpc, nchunks, st)
+                   : a.num_seqs ? ssd_state_dispatch<T, false, true>(a, shpc, nchunks, st)
+                                : ssd_state_dispatch<T, false, false>(a, shpc, nchunks, st);
+    if (rc) return rc;
   } else if (a.initial_states) {
     const int64_t units = (int64_t)a.batch * a.heads * (kP * kN / 8);
     ssd_fold_init_kernel<T><<<dim3((unsigned)((units + 255) / 256), (nchunks + 1 + kFoldChunks - 1) / kFoldChunks), 256, 0, st>>>(a, nchunks);
@@ -1122,9 +1145,13 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
     if (int rc = encode_rows_map(&maps.c, a.Cm, a.batch, a.len, a.groups, kN, kBlk, a.io_dtype)) return rc;
     if (int rc = encode_rows_map(&maps.bm, a.Bm, a.batch, a.len, a.groups, kN, kBlk, a.io_dtype)) return rc;
     const unsigned ctas = 2u * nparts * a.batch * nchunks;
-    if (a.reverse) return ssd_scan_launch<T, false, true>(a, maps, ctas, nchunks, hpc, nparts, st);
-    if (a.D && (a.d_has_p || a.row_dots)) return ssd_scan_launch<T, true, false>(a, maps, ctas, nchunks, hpc, nparts, st);
-    return ssd_scan_launch<T, false, false>(a, maps, ctas, nchunks, hpc, nparts, st);
+    if (a.reverse) return ssd_scan_launch<T, false, true, false>(a, maps, ctas, nchunks, hpc, nparts, st);
+    const bool xskip = a.D && (a.d_has_p || a.row_dots);
+    if (a.num_seqs)
+      return xskip ? ssd_scan_launch<T, true, false, true>(a, maps, ctas, nchunks, hpc, nparts, st)
+                   : ssd_scan_launch<T, false, false, true>(a, maps, ctas, nchunks, hpc, nparts, st);
+    return xskip ? ssd_scan_launch<T, true, false, false>(a, maps, ctas, nchunks, hpc, nparts, st)
+                 : ssd_scan_launch<T, false, false, false>(a, maps, ctas, nchunks, hpc, nparts, st);
   }
   return SSM_OK;
 }

@@ -244,6 +244,8 @@ Tensor state_step_heads(const Tensor& state, const Tensor& x, const Tensor& dt, 
           "B and C must have shape (B, G, N) with G dividing H.");
   same_device(state, {&x, &dt, &A, &B, &C});
   need_cuda(state, {&D, &z, &dt_bias});
+  SSM_ARG((!D.has_value() || D->numel() == nh) && (!dt_bias.has_value() || dt_bias->numel() == nh), "D and dt_bias must have shape (H,).");
+  if (z.has_value()) SSM_ARG(z->numel() == x.numel(), "z must have shape (B, H, P).");
   SSM_ARG(state.scalar_type() == at::kFloat && state.is_contiguous(), "state must be a contiguous float32 tensor.");
   c10::cuda::CUDAGuard guard(state.device());
   Tensor xs = x.detach().contiguous(), dts = like(dt, xs), Bt = B.detach().contiguous(), Ct = C.detach().contiguous();
@@ -401,6 +403,7 @@ Tensor dw_causal_conv_update(const Tensor& conv_state, const Tensor& x, const Te
   SSM_ARG(w2.dim() == 2 && w2.size(0) == x.size(1) && w2.size(1) == conv_state.size(2), "weight must have shape (C, K).");
   same_device(conv_state, {&x, &weight});
   need_cuda(conv_state, {&bias});
+  if (bias.has_value()) SSM_ARG(bias->numel() == x.size(1), "bias must have shape (C,).");
   SSM_ARG(conv_state.scalar_type() == at::kFloat && conv_state.is_contiguous(), "conv_state must be a contiguous float32 tensor.");
   const bool silu = is_silu(activation);
   c10::cuda::CUDAGuard guard(x.device());
@@ -498,6 +501,8 @@ py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tenso
   ValueErrors scope;
   at::NoGradGuard no_grad;
   SSM_ARG(tok.dim() == 2 && tok.is_cuda(), "mamba1_step: tok must be a (B, d_model) CUDA tensor.");
+  same_device(tok, {&conv_state, &ssm_state, &in_x, &in_z, &conv_w, &x_proj, &dt_proj, &dt_bias, &A, &D, &out_proj});
+  need_cuda(tok, {&residual, &conv_b, &norm_w});
   const int64_t nb = tok.size(0), dm = tok.size(1), di = in_x.size(0), n = ssm_state.size(-1), r = dt_proj.size(1), k = conv_w.size(-1);
   const auto T = tok.scalar_type();
   const bool half = T == at::kBFloat16 || T == at::kHalf;
@@ -507,7 +512,8 @@ py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tenso
   fused = fused && in_x.sizes() == in_z.sizes() && in_x.size(1) == dm && conv_w.size(0) == di && x_proj.size(0) == r + 2 * n && x_proj.size(1) == di &&
           dt_proj.size(0) == di && out_proj.size(0) == dm && out_proj.size(1) == di && conv_state.dim() == 3 && conv_state.size(0) == nb && conv_state.size(1) == di &&
           conv_state.size(2) == k && ssm_state.dim() == 3 && ssm_state.size(0) == nb && ssm_state.size(1) == di && A.dim() == 2 && A.size(0) == di && A.size(1) == n &&
-          D.numel() == di && dt_bias.numel() == di && (!residual.has_value() || residual->numel() == nb * dm) &&
+          D.numel() == di && dt_bias.numel() == di && conv_w.numel() == di * k && (!conv_b.has_value() || conv_b->numel() == di) &&
+          (!norm_w.has_value() || norm_w->numel() == dm) && (!residual.has_value() || residual->numel() == nb * dm) &&
           ssm_mamba1_decode_supported((int)nb, (int)dm, (int)di, (int)n, (int)r, (int)k, dtype_code(tok, "mamba1_step"));
   if (fused) {
     c10::cuda::CUDAGuard guard(tok.device());
@@ -549,6 +555,8 @@ Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B
   ValueErrors scope;
   at::NoGradGuard no_grad;
   SSM_ARG(tok.dim() == 2 && tok.is_cuda() && ssm_state.dim() == 4, "mamba2_step: tok must be a (B, d_model) CUDA tensor and the state (B, H, P, N).");
+  same_device(tok, {&conv_x, &conv_B, &conv_C, &ssm_state, &in_z, &in_x, &in_B, &in_C, &in_dt, &wx, &wB, &wC, &dt_bias, &A, &D, &norm_w, &out_proj});
+  need_cuda(tok, {&bx, &bB, &bC});
   const int64_t nb = tok.size(0), dm = tok.size(1), nh = ssm_state.size(1), hp = ssm_state.size(2), n = ssm_state.size(3), di = nh * hp;
   SSM_ARG(in_B.size(0) % n == 0, "mamba2_step: in_B must have groups * d_state rows.");
   const int64_t g = in_B.size(0) / n, k = wx.size(-1);
@@ -559,7 +567,8 @@ Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B
   for (const Tensor* w : {&in_z, &in_x, &in_B, &in_C, &in_dt, &wx, &wB, &wC, &norm_w, &out_proj}) fused = fused && plain(*w, T);
   for (const Tensor* w : {&in_z, &in_x, &in_B, &in_C, &in_dt}) fused = fused && w->dim() == 2 && w->size(1) == dm;
   fused = fused && in_x.size(0) == di && in_z.size(0) == di && in_C.size(0) == g * n && in_dt.size(0) == nh && wx.numel() == di * k && wB.numel() == g * n * k &&
-          wC.numel() == g * n * k && conv_x.numel() == nb * di * k && conv_B.numel() == nb * g * n * k && conv_C.numel() == nb * g * n * k &&
+          wC.numel() == g * n * k && (!bx.has_value() || bx->numel() == di) && (!bB.has_value() || bB->numel() == g * n) &&
+          (!bC.has_value() || bC->numel() == g * n) && conv_x.numel() == nb * di * k && conv_B.numel() == nb * g * n * k && conv_C.numel() == nb * g * n * k &&
           ssm_state.size(0) == nb && dt_bias.numel() == nh && A.numel() == nh && D.numel() == nh && norm_w.numel() == di && out_proj.dim() == 2 &&
           out_proj.size(0) == dm && out_proj.size(1) == di &&
           ssm_mamba2_decode_supported((int)nb, (int)dm, (int)nh, (int)hp, (int)n, (int)g, (int)k, dtype_code(tok, "mamba2_step"));

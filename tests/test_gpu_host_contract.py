@@ -1,0 +1,45 @@
+"""The host side of the operators: what they refuse, what they hold up, and what they do when a launch is refused."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nb", [1, 17])  # one launch, and the projections as separate calls
+@pytest.mark.parametrize("which", ["in_x", "conv_w", "conv_b", "x_proj", "dt_proj", "dt_bias", "A_log", "D", "out_proj", "conv_state", "ssm_state", "residual", "norm_w"])
+def test_mamba1_step_refuses_host_tensors(which, nb):
+    from ssm_b200 import ops
+    from ssm_b200.mixer import Mamba1Block
+
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    conv, state = block.allocate_inference_cache(nb)
+    t = {**block._parameters, "conv_state": conv, "ssm_state": state, "residual": torch.zeros(nb, 64, device="cuda"), "norm_w": block.norm_w}
+    t[which] = t[which].detach().cpu()
+    with torch.no_grad(), pytest.raises((RuntimeError, ValueError)):
+        ops.mamba1_step(torch.zeros(nb, 64, device="cuda", dtype=torch.bfloat16), t["residual"], t["conv_state"], t["ssm_state"], t, t["norm_w"])
+
+
+@pytest.mark.parametrize("nb", [1, 17])
+def test_decode_steps_refuse_short_vectors(nb):
+    from ssm_b200 import ops
+    from ssm_b200.mixer import Mamba1Block, Mamba2Block
+
+    tok = torch.zeros(nb, 64, device="cuda", dtype=torch.bfloat16)
+    b1, b2 = Mamba1Block(64, device="cuda", dtype=torch.bfloat16), Mamba2Block(64, device="cuda", dtype=torch.bfloat16)
+    c1, (win, s2) = b1.allocate_inference_cache(nb), b2.allocate_inference_cache(nb)
+    w1, w2 = dict(b1._parameters), dict(b2._parameters)
+    norm = b1.norm_w.detach()
+    with torch.no_grad():
+        for key in ("conv_b", "dt_bias", "D"):
+            with pytest.raises((RuntimeError, ValueError)):
+                ops.mamba1_step(tok, None, *c1, dict(w1, **{key: w1[key].detach()[:16].clone()}), norm)
+        with pytest.raises((RuntimeError, ValueError)):
+            ops.mamba1_step(tok, None, *c1, w1, norm[:16].clone())
+        for key in ("conv_x_b", "conv_B_b", "conv_C_b", "dt_bias", "D", "norm_w"):
+            with pytest.raises((RuntimeError, ValueError)):
+                ops.mamba2_step(tok, win, s2, dict(w2, **{key: w2[key].detach()[:1].clone()}))
+        with pytest.raises((RuntimeError, ValueError)):
+            ops.mamba2_step(tok, [t.cpu() for t in win], s2, w2)

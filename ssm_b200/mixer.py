@@ -131,6 +131,14 @@ class Mamba1Block(nn.Module):
 
         return ops
 
+    _STEP_WEIGHTS = ("in_x", "in_z", "conv_w", "conv_b", "x_proj", "dt_proj", "dt_bias", "A_log", "D", "out_proj", "norm_w")
+
+    def _step_weights(self) -> dict:
+        """The weights as a decode step takes them.  The parameter table saves nn.Module's attribute look-up per weight and step; with a
+        weight that is not in it (parametrised, pruned, replaced by a plain tensor) all are read as attributes."""
+        p = self._parameters
+        return p if all(n in p for n in self._STEP_WEIGHTS) else {n: getattr(self, n) for n in self._STEP_WEIGHTS}
+
     def _weights(self) -> dict:
         return dict(in_x=self.in_x, in_z=self.in_z, conv_w=self.conv_w, conv_b=self.conv_b, x_proj=self.x_proj, dt_proj=self.dt_proj,
                     dt_bias=self.dt_bias, A=-torch.exp(self.A_log), D=self.D, out_proj=self.out_proj, norm_w=self.norm_w)
@@ -147,7 +155,7 @@ class Mamba1Block(nn.Module):
 
     def mixer_step(self, tok: Tensor, cache) -> Tensor:
         """The mixer alone on one token: tok (B, d_model) -> (B, d_model); ``cache`` from `allocate_inference_cache`."""
-        return mamba1_mixer_step(self._namespace(), self._parameters, dict(d_state=self.d_state, dt_rank=self.dt_rank), tok, cache[0], cache[1])
+        return mamba1_mixer_step(self._namespace(), self._step_weights(), dict(d_state=self.d_state, dt_rank=self.dt_rank), tok, cache[0], cache[1])
 
     def allocate_inference_cache(self, batch_size: int, dtype: Optional[torch.dtype] = None):
         """(conv_state (B, d_inner, K), ssm_state (B, d_inner, N)), both fp32 and zero-filled."""
@@ -162,11 +170,11 @@ class Mamba1Block(nn.Module):
             raise ValueError("step expects inputs of shape (B, 1, d_model)")
         ops = self._namespace()
         if _native_step(ops, hidden, "mamba1_step"):
-            p = self._parameters
+            p = self._step_weights()
             out, res = ops.mamba1_step(hidden[:, 0], residual, conv_state, ssm_state, p, p["norm_w"], self.eps)
             return out.unsqueeze(1), res.unsqueeze(1)
         cfg = dict(d_state=self.d_state, dt_rank=self.dt_rank)
-        out = mamba1_mixer_step(ops, self._parameters, cfg, hidden[:, 0], conv_state, ssm_state).unsqueeze(1)
+        out = mamba1_mixer_step(ops, self._step_weights(), cfg, hidden[:, 0], conv_state, ssm_state).unsqueeze(1)
         res1 = None if residual is None else residual
         return ops.fused_layer_norm(out, self.norm_w, None, residual=res1, is_rms=True, eps=self.eps, prenorm=True,
                                     residual_in_fp32=True, return_residual=True)

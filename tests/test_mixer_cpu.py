@@ -55,6 +55,29 @@ def test_step_reproduces_forward_token_by_token():
             torch.testing.assert_close(rt, r[:, t:t + 1], rtol=1e-5, atol=1e-6)
 
 
+def test_step_reads_weights_that_are_no_plain_parameters():
+    """A parametrised or pruned weight is no entry of the parameter table; the step takes what the attribute gives, as forward does."""
+    import torch.nn.utils.parametrize as parametrize
+    from torch.nn.utils import prune
+
+    class Half(torch.nn.Module):
+        def forward(self, w):
+            return 0.5 * w
+
+    torch.manual_seed(2)
+    m = Mamba1Block(24, d_state=4, d_conv=3, expand=2, ops=orc)
+    parametrize.register_parametrization(m, "out_proj", Half())
+    prune.random_unstructured(m, "in_x", amount=0.5)
+    hidden, residual = torch.randn(2, 3, 24), torch.randn(2, 3, 24)
+    with torch.no_grad():
+        y, r = m(hidden, residual)
+        cache = m.allocate_inference_cache(2)
+        for t in range(3):
+            yt, rt = m.step(hidden[:, t:t + 1], residual[:, t:t + 1], *cache)
+            torch.testing.assert_close(yt, y[:, t:t + 1], rtol=1e-5, atol=1e-6)
+            torch.testing.assert_close(rt, r[:, t:t + 1], rtol=1e-5, atol=1e-6)
+
+
 def test_constructor_rejects_bad_arguments():
     import pytest
 

@@ -71,7 +71,9 @@ variable_list invoke_call(const c10::intrusive_ptr<Call>& call) {
 
 Tensor cast(const Tensor& grad, at::ScalarType t) { return grad.scalar_type() == t ? grad : grad.to(t); }
 
-// Several fp32 buffers that the kernels add into, zeroed by one launch; each starts on a 256-byte line.
+// Several fp32 buffers that the kernels add into, zeroed by one launch; each starts on a 256-byte line.  They share one piece of memory,
+// which lives as long as any of them, and autograd keeps a gradient it is given without a copy: gradients go into one pool only
+// with others of their size class, and never with work buffers.
 struct ZeroPool {
   std::vector<std::pair<Tensor*, std::vector<int64_t>>> want;
   int64_t total = 0;
@@ -304,13 +306,13 @@ struct ChunkCall final : Call {
     const auto f32 = c.X.options().dtype(at::kFloat);
     Tensor gy = like(grads[0], c.X);
     Tensor dX = at::empty_like(c.X), ddt, dA, dB, dC, dD, dz, dI, hist;
-    ZeroPool pool;
+    ZeroPool params, per_row, per_step;
     int typed = 0;
     // per-token B / C / z: their gradients are written by the kernel in the tensor's own type (no zero-fill, no fp32 copy)
     auto own = [&](Tensor& grad, const OptTensor& t, Kind k, int bit) {
       if (!t.has_value()) return;
       if (k == Kind::BLHP) grad = at::empty_like(*t), typed |= bit;
-      else pool.add(grad, t->sizes());
+      else (k == Kind::HP ? params : k == Kind::BHP ? per_row : per_step).add(grad, t->sizes());
     };
     own(dB, c.B, c.kB, 1), own(dC, c.C, c.kC, 2), own(dz, c.z, c.kz, 4);
     Tensor scratch = at::empty({std::max<int64_t>(1, ssm_chunk_scan_bwd_scratch_floats((int)c.nb, (int)c.nl, (int)c.nh, (int)c.np, c.chunk))}, f32);
@@ -326,11 +328,11 @@ struct ChunkCall final : Call {
       fused = ssm_chunk_scan_bwd_fused(&g) != 0;
     }
     if (fused) ddt = at::empty({c.nb, c.nl, c.nh}, c.X.options()), typed |= 8;
-    else pool.add(ddt, {c.nb, c.nl, c.nh}), hist = at::empty({c.nb, std::max<int64_t>(c.nl, 1), c.nh, c.np}, f32);
-    pool.add(dA, c.A->sizes());
-    if (c.D.has_value()) pool.add(dD, c.D->sizes());
-    if (c.init.has_value()) pool.add(dI, c.init->sizes());
-    pool.make(f32);
+    else per_step.add(ddt, {c.nb, c.nl, c.nh}), hist = at::empty({c.nb, std::max<int64_t>(c.nl, 1), c.nh, c.np}, f32);
+    params.add(dA, c.A->sizes());
+    if (c.D.has_value()) params.add(dD, c.D->sizes());
+    if (c.init.has_value()) per_row.add(dI, c.init->sizes());
+    params.make(f32), per_row.make(f32), per_step.make(f32);
     set_bcz();
     g.fwd.typed_grads = typed, g.ddt = ddt.data_ptr(), g.history = out_ptr(hist);
     set_bc4(g.dA, grad_of(dA), c.kA), set_bc4(g.dD, grad_of(dD), c.kD), set_bc4(g.dinitial, grad_of(dI), Kind::BHP);
@@ -737,11 +739,14 @@ struct SsdCall final : Call {
     ssm_stream_t stream = stream_of(X);
 
     Tensor u, qd, dB, dC, dA, dD, dbias;
-    ZeroPool pool;
-    pool.add(u, {nb, nl, nh}), pool.add(qd, {nb, nl, nh}), pool.add(dB, {nb, nl, ng, nn}), pool.add(dC, {nb, nl, ng, nn}), pool.add(dA, {nh});
-    if (D.has_value()) pool.add(dD, D->sizes());
-    if (bias.has_value()) pool.add(dbias, {nh});
-    pool.make(f32);
+    ZeroPool work, coeffs, params;
+    work.add(u, {nb, nl, nh}), work.add(qd, {nb, nl, nh});
+    auto own = [&](const Tensor& t) -> ZeroPool& { return t.scalar_type() == at::kFloat ? coeffs : work; };  // in another type it is copied below
+    own(B_).add(dB, {nb, nl, ng, nn}), own(C_).add(dC, {nb, nl, ng, nn});
+    params.add(dA, {nh});
+    if (D.has_value()) params.add(dD, D->sizes());
+    if (bias.has_value()) params.add(dbias, {nh});
+    work.make(f32), coeffs.make(f32), params.make(f32);
     Tensor dX = at::empty_like(X), ddt = at::empty_like(dt), dz, dinit, start0;
 
     ssm_ssd_bwd_args e{};

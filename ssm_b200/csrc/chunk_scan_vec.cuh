@@ -1,6 +1,7 @@
-// Element-wise chunked recurrence on lanes of four neighbouring projections of one head: B, C (and z) of X's element type with the
-// projection axis contiguous, as models use the operator.  A scalar lane moves 2 or 4 bytes per instruction and is bound by
-// instruction issue; four projections make every load and store 8 or 16 bytes, 256 or 512 bytes per warp, in both element sizes.
+// Element-wise chunked recurrence on lanes of neighbouring projections of one head: B, C (and z) of X's element type with the projection
+// axis contiguous, as models use the operator.  A scalar lane moves 2 or 4 bytes per instruction and is bound by instruction
+// issue.  The forward takes 16 bytes of a row per lane, four fp32 or eight 16-bit projections, and 8 bytes where only those are
+// aligned; the backward, which keeps five rows of a step in registers, takes four projections in either element size.
 //
 // The sequence is cut into pieces of at most kPiece steps (whatever the caller's chunk size: the recurrence does not depend on
 // the cut), which is what puts enough independent walks in flight.  Forward: local states, carry over the pieces, replay.
@@ -15,43 +16,66 @@ namespace ssmb {
 
 constexpr int kPiece = 32;  // longest piece of the sequence
 
-template <typename T>
-struct Row4;
-template <>
-struct Row4<float> {
-  using Raw = uint4;
+// V consecutive elements of a row as one load or store of 8 or 16 bytes
+template <typename T, int V>
+struct RowRaw {
+  static_assert(V * sizeof(T) == 8 || V * sizeof(T) == 16, "one access");
+  using type = typename std::conditional<V * sizeof(T) == 16, uint4, uint2>::type;
 };
-template <>
-struct Row4<__nv_bfloat16> {
-  using Raw = uint2;
-};
-template <>
-struct Row4<__half> {
-  using Raw = uint2;
-};
-template <typename T>
-__device__ __forceinline__ typename Row4<T>::Raw ld4(const T* p) {
-  return __ldg(reinterpret_cast<const typename Row4<T>::Raw*>(p));
+template <typename T, int V>
+__device__ __forceinline__ typename RowRaw<T, V>::type ld_row(const T* p) {
+  return __ldg(reinterpret_cast<const typename RowRaw<T, V>::type*>(p));
 }
-template <typename T>
-__device__ __forceinline__ void unpack4(const typename Row4<T>::Raw& r, float (&f)[4]) {
-  const T* e = reinterpret_cast<const T*>(&r);
+// 16-bit elements word by word (see Vec16)
+template <typename T, int V>
+__device__ __forceinline__ void unpack_row(const typename RowRaw<T, V>::type& r, float (&f)[V]) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(&r);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) f[i] = to_f<T>(e[i]);
+  for (int i = 0; i < (int)sizeof(r) / 4; ++i) {
+    if constexpr (std::is_same<T, float>::value) {
+      f[i] = __uint_as_float(w[i]);
+    } else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      f[2 * i] = __uint_as_float(w[i] << 16), f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    } else {
+      const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+      f[2 * i] = v.x, f[2 * i + 1] = v.y;
+    }
+  }
 }
-template <typename T>
-__device__ __forceinline__ void store4(T* p, const float (&f)[4]) {
-  typename Row4<T>::Raw r;
-  T* e = reinterpret_cast<T*>(&r);
+template <typename T, int V>
+__device__ __forceinline__ void store_row(T* p, const float (&f)[V]) {
+  typename RowRaw<T, V>::type r;
+  uint32_t* w = reinterpret_cast<uint32_t*>(&r);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) e[i] = from_f<T>(f[i]);
-  *reinterpret_cast<typename Row4<T>::Raw*>(p) = r;
+  for (int i = 0; i < (int)sizeof(r) / 4; ++i) {
+    if constexpr (std::is_same<T, float>::value) {
+      w[i] = __float_as_uint(f[i]);
+    } else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      const __nv_bfloat162 v = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&v);
+    } else {
+      const __half2 v = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+  }
+  *reinterpret_cast<typename RowRaw<T, V>::type*>(p) = r;
 }
 __device__ __forceinline__ void load4f(const float* p, float (&f)[4]) {
   const float4 v = *reinterpret_cast<const float4*>(p);
   f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
 }
 __device__ __forceinline__ void store4f(float* p, const float (&f)[4]) { *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]); }
+
+template <int V>
+__device__ __forceinline__ void load_f32(const float* p, float (&f)[V]) {
+#pragma unroll
+  for (int i = 0; i < V; i += 4) load4f(p + i, *reinterpret_cast<float(*)[4]>(&f[i]));
+}
+template <int V>
+__device__ __forceinline__ void store_f32(float* p, const float (&f)[V]) {
+#pragma unroll
+  for (int i = 0; i < V; i += 4) store4f(p + i, *reinterpret_cast<const float(*)[4]>(&f[i]));
+}
 
 // Where a thread's piece lies: batch row b, first step t0, n valid steps, rows of X / dY / dX at `row`.
 struct Piece4 {
@@ -68,25 +92,27 @@ struct Piece4 {
 };
 
 // APPLY false: local end state and decay product of every piece.  APPLY true: the piece replayed from its incoming state, Y written.
-// The loads of eight steps go out before the first is used.
-template <typename T, bool APPLY>
-__global__ void __launch_bounds__(kChunkThreads) chunk_fwd4_kernel(const ssm_chunk_args a, int nchunks, int len) {
-  constexpr int U = 8;
-  using Raw = typename Row4<T>::Raw;
+// The loads of several steps go out before the first is used.  Bound by instruction issue.  bf16 with gate, us for all launches of
+// the forward at (8, 2048, 16, 64) and (4, 4096, 32, 64): lanes of four projections 79 and 133, of eight 62 and 99.
+template <typename T, int V, bool APPLY>
+__global__ void __launch_bounds__(kChunkThreads) chunk_fwd_row_kernel(const ssm_chunk_args a, int nchunks, int len) {
+  constexpr int U = 32 / V;
+  using Raw = typename RowRaw<T, V>::type;
   const int HP = a.heads * a.proj;
-  const int hp = (blockIdx.x * kChunkThreads + threadIdx.x) * 4;
+  const int hp = (blockIdx.x * kChunkThreads + threadIdx.x) * V;
   if (hp >= HP) return;
   const int h = hp / a.proj, q = hp % a.proj;
   const Piece4 pc(a, nchunks, len, blockIdx.z, blockIdx.y, hp);
   float* P = a.scratch + pc.slot;                                    // decay products
   float* S = a.scratch + (int64_t)a.batch * nchunks * HP + pc.slot;  // local end states, then incoming states
-  float Av[4], Dv[4], s[4] = {0.f, 0.f, 0.f, 0.f}, sumdt = 0.f;
+  float Av[V], Dv[V], s[V], sumdt = 0.f;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
+  for (int e = 0; e < V; ++e) {
+    s[e] = 0.f;
     Av[e] = bc4_load_f32(a.A, 0, 0, h, q + e) * kLog2e;
     Dv[e] = (APPLY && a.D.ptr) ? bc4_load_f32(a.D, 0, 0, h, q + e) : 0.f;
   }
-  if (APPLY) load4f(S, s);
+  if (APPLY) load_f32<V>(S, s);
   const T* px = reinterpret_cast<const T*>(a.X) + pc.row;
   const T* pdt = reinterpret_cast<const T*>(a.dt) + ((int64_t)pc.b * a.len + pc.t0) * a.heads + h;
   const T* pB = reinterpret_cast<const T*>(a.Bm.ptr) + bc4_off(a.Bm, pc.b, pc.t0, h, q);
@@ -100,43 +126,43 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_fwd4_kernel(const ssm_chu
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       const int kk = min(k + i, pc.n - 1);  // beyond the piece: a valid row, dropped below
-      xr[i] = ld4<T>(px + (int64_t)kk * HP);
-      br[i] = ld4<T>(pB + (int64_t)kk * a.Bm.st);
-      if (APPLY) cr[i] = ld4<T>(pC + (int64_t)kk * a.Cm.st);
-      if (has_z) zr[i] = ld4<T>(pz + (int64_t)kk * a.z.st);
+      xr[i] = ld_row<T, V>(px + (int64_t)kk * HP);
+      br[i] = ld_row<T, V>(pB + (int64_t)kk * a.Bm.st);
+      if (APPLY) cr[i] = ld_row<T, V>(pC + (int64_t)kk * a.Cm.st);
+      if (has_z) zr[i] = ld_row<T, V>(pz + (int64_t)kk * a.z.st);
       d[i] = to_f<T>(__ldg(pdt + (int64_t)kk * a.heads));
     }
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       if (k + i >= pc.n) break;
-      float x[4], bv[4];
-      unpack4<T>(xr[i], x), unpack4<T>(br[i], bv);
+      float x[V], bv[V];
+      unpack_row<T, V>(xr[i], x), unpack_row<T, V>(br[i], bv);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s[e] = fmaf(ex2_approx(d[i] * Av[e]), s[e], d[i] * bv[e] * x[e]);
+      for (int e = 0; e < V; ++e) s[e] = fmaf(ex2_approx(d[i] * Av[e]), s[e], d[i] * bv[e] * x[e]);
       sumdt += d[i];
       if (APPLY) {
-        float cv[4], y[4];
-        unpack4<T>(cr[i], cv);
+        float cv[V], y[V];
+        unpack_row<T, V>(cr[i], cv);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = fmaf(Dv[e], x[e], s[e] * cv[e]);
+        for (int e = 0; e < V; ++e) y[e] = fmaf(Dv[e], x[e], s[e] * cv[e]);
         if (has_z) {
-          float zv[4];
-          unpack4<T>(zr[i], zv);
+          float zv[V];
+          unpack_row<T, V>(zr[i], zv);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) y[e] *= silu_fast(zv[e]);
+          for (int e = 0; e < V; ++e) y[e] *= silu_fast(zv[e]);
         }
-        store4<T>(Y + (int64_t)(k + i) * HP, y);
+        store_row<T, V>(Y + (int64_t)(k + i) * HP, y);
       }
     }
   }
   if (APPLY) {
-    const float zero[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int k = pc.n; k < pc.rows; ++k) store4<T>(Y + (int64_t)k * HP, zero);
+    const float zero[V] = {};
+    for (int k = pc.n; k < pc.rows; ++k) store_row<T, V>(Y + (int64_t)k * HP, zero);
   } else {
-    float pr[4];
+    float pr[V];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) pr[e] = ex2_approx(sumdt * Av[e]);
-    store4f(P, pr), store4f(S, s);
+    for (int e = 0; e < V; ++e) pr[e] = ex2_approx(sumdt * Av[e]);
+    store_f32<V>(P, pr), store_f32<V>(S, s);
   }
 }
 
@@ -144,7 +170,7 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_fwd4_kernel(const ssm_chu
 template <typename T>
 __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_local4_kernel(const ssm_chunk_bwd_args g, float* __restrict__ R, int nchunks, int len) {
   constexpr int U = 8;
-  using Raw = typename Row4<T>::Raw;
+  using Raw = typename RowRaw<T, 4>::type;
   const ssm_chunk_args& a = g.fwd;
   const int HP = a.heads * a.proj;
   const int hp = (blockIdx.x * kChunkThreads + threadIdx.x) * 4;
@@ -165,18 +191,18 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_local4_kernel(const s
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       const int kk = max(k - 1 - i, 0);
-      gr[i] = ld4<T>(pdy + (int64_t)kk * HP);
-      cr[i] = ld4<T>(pC + (int64_t)kk * a.Cm.st);
-      if (has_z) zr[i] = ld4<T>(pz + (int64_t)kk * a.z.st);
+      gr[i] = ld_row<T, 4>(pdy + (int64_t)kk * HP);
+      cr[i] = ld_row<T, 4>(pC + (int64_t)kk * a.Cm.st);
+      if (has_z) zr[i] = ld_row<T, 4>(pz + (int64_t)kk * a.z.st);
       d[i] = to_f<T>(__ldg(pdt + (int64_t)kk * a.heads));
     }
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       if (k - 1 - i < 0) break;
       float dout[4], cv[4], zv[4];
-      unpack4<T>(gr[i], dout), unpack4<T>(cr[i], cv);
+      unpack_row<T, 4>(gr[i], dout), unpack_row<T, 4>(cr[i], cv);
       if (has_z) {
-        unpack4<T>(zr[i], zv);
+        unpack_row<T, 4>(zr[i], zv);
 #pragma unroll
         for (int e = 0; e < 4; ++e) dout[e] *= silu_fast(zv[e]);
       }
@@ -204,7 +230,7 @@ template <typename T>
 __global__ void __launch_bounds__(kChunkThreads, bwd4_ctas<T>()) chunk_bwd4_kernel(const ssm_chunk_bwd_args g, const float* __restrict__ S, const float* __restrict__ R,
                                                                       int nchunks, int len, int typed_dt) {
   constexpr int SUB = kBwdSub, NG = kPiece / SUB, UF = kBwdSweep;
-  using Raw = typename Row4<T>::Raw;
+  using Raw = typename RowRaw<T, 4>::type;
   __shared__ float4 entry[NG][kChunkThreads];  // the state that enters each group of steps
   const ssm_chunk_args& a = g.fwd;
   const int HP = a.heads * a.proj;
@@ -243,14 +269,14 @@ __global__ void __launch_bounds__(kChunkThreads, bwd4_ctas<T>()) chunk_bwd4_kern
 #pragma unroll
       for (int i = 0; i < UF; ++i) {
         const bool in = k + i < min(pc.n, sweep);
-        xr[i] = in ? ld4<T>(px + (int64_t)(k + i) * HP) : zero_raw;
-        br[i] = in ? ld4<T>(pB + (int64_t)(k + i) * a.Bm.st) : zero_raw;
+        xr[i] = in ? ld_row<T, 4>(px + (int64_t)(k + i) * HP) : zero_raw;
+        br[i] = in ? ld_row<T, 4>(pB + (int64_t)(k + i) * a.Bm.st) : zero_raw;
         d[i] = in ? to_f<T>(__ldg(pdt + (int64_t)(k + i) * a.heads)) : 0.f;
       }
 #pragma unroll
       for (int i = 0; i < UF; ++i) {
         float x[4], bv[4];
-        unpack4<T>(xr[i], x), unpack4<T>(br[i], bv);
+        unpack_row<T, 4>(xr[i], x), unpack_row<T, 4>(br[i], bv);
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[e] = fmaf(ex2_approx(d[i] * Av[e]), s[e], d[i] * bv[e] * x[e]);
         if ((i + 1) % SUB == 0 && k + i < sweep) entry[(k + i + 1) / SUB][threadIdx.x] = make_float4(s[0], s[1], s[2], s[3]);
@@ -263,11 +289,11 @@ __global__ void __launch_bounds__(kChunkThreads, bwd4_ctas<T>()) chunk_bwd4_kern
 #pragma unroll
       for (int i = 0; i < SUB; ++i) {
         const bool in = k0 + i >= 0 && k0 + i < pc.n;
-        nx[i] = in ? ld4<T>(px + (int64_t)(k0 + i) * HP) : zero_raw;
-        nbr[i] = in ? ld4<T>(pB + (int64_t)(k0 + i) * a.Bm.st) : zero_raw;
-        nc[i] = in ? ld4<T>(pC + (int64_t)(k0 + i) * a.Cm.st) : zero_raw;
-        ng[i] = in ? ld4<T>(pdy + (int64_t)(k0 + i) * HP) : zero_raw;
-        nz[i] = in && has_z ? ld4<T>(pz + (int64_t)(k0 + i) * a.z.st) : zero_raw;
+        nx[i] = in ? ld_row<T, 4>(px + (int64_t)(k0 + i) * HP) : zero_raw;
+        nbr[i] = in ? ld_row<T, 4>(pB + (int64_t)(k0 + i) * a.Bm.st) : zero_raw;
+        nc[i] = in ? ld_row<T, 4>(pC + (int64_t)(k0 + i) * a.Cm.st) : zero_raw;
+        ng[i] = in ? ld_row<T, 4>(pdy + (int64_t)(k0 + i) * HP) : zero_raw;
+        nz[i] = in && has_z ? ld_row<T, 4>(pz + (int64_t)(k0 + i) * a.z.st) : zero_raw;
         nd[i] = in ? to_f<T>(__ldg(pdt + (int64_t)(k0 + i) * a.heads)) : 0.f;
       }
     };
@@ -287,7 +313,7 @@ __global__ void __launch_bounds__(kChunkThreads, bwd4_ctas<T>()) chunk_bwd4_kern
 #pragma unroll
       for (int i = 0; i < SUB; ++i) {
         float x[4], bv[4];
-        unpack4<T>(xr[i], x), unpack4<T>(br[i], bv);
+        unpack_row<T, 4>(xr[i], x), unpack_row<T, 4>(br[i], bv);
 #pragma unroll
         for (int e = 0; e < 4; ++e) st[i + 1][e] = fmaf(ex2_approx(d[i] * Av[e]), st[i][e], d[i] * bv[e] * x[e]);
       }
@@ -295,17 +321,17 @@ __global__ void __launch_bounds__(kChunkThreads, bwd4_ctas<T>()) chunk_bwd4_kern
       for (int i = SUB - 1; i >= 0; --i) {
         const int k = k0 + i;
         float x[4], bv[4], cv[4], dy[4], dxo[4], dbo[4], dco[4], ddt = 0.f;
-        unpack4<T>(xr[i], x), unpack4<T>(br[i], bv), unpack4<T>(cr[i], cv), unpack4<T>(gr[i], dy);
+        unpack_row<T, 4>(xr[i], x), unpack_row<T, 4>(br[i], bv), unpack_row<T, 4>(cr[i], cv), unpack_row<T, 4>(gr[i], dy);
         if (has_z) {
           float zv[4], dzo[4];
-          unpack4<T>(zr[i], zv);
+          unpack_row<T, 4>(zr[i], zv);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float sg = sigmoid_fast(zv[e]);
             dzo[e] = dy[e] * fmaf(Dv[e], x[e], st[i + 1][e] * cv[e]) * sg * (1.f + zv[e] * (1.f - sg));
             dy[e] *= zv[e] * sg;
           }
-          if (active && k < pc.rows) store4<T>(dZ + (int64_t)k * g.dz.st, dzo);
+          if (active && k < pc.rows) store_row<T, 4>(dZ + (int64_t)k * g.dz.st, dzo);
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -321,9 +347,9 @@ __global__ void __launch_bounds__(kChunkThreads, bwd4_ctas<T>()) chunk_bwd4_kern
           dD[e] = fmaf(dy[e], x[e], dD[e]);
         }
         if (active && k < pc.rows) {
-          store4<T>(dC + (int64_t)k * g.dC.st, dco);
-          store4<T>(dB + (int64_t)k * g.dB.st, dbo);
-          store4<T>(dX + (int64_t)k * HP, dxo);
+          store_row<T, 4>(dC + (int64_t)k * g.dC.st, dco);
+          store_row<T, 4>(dB + (int64_t)k * g.dB.st, dbo);
+          store_row<T, 4>(dX + (int64_t)k * HP, dxo);
         }
         for (int o = 1; o < share; o <<= 1) ddt += __shfl_xor_sync(0xffffffffu, ddt, o);
         if (active && k < pc.rows && (threadIdx.x & (share - 1)) == 0) {

@@ -14,7 +14,7 @@
 //             (g_t = C_t dy_t + exp(dt_{t+1} A) g_{t+1} is a linear recurrence too), and one
 //             final pass per chunk replays the states and walks back through them producing every
 //             gradient.
-// The usual layouts run on lanes of four projections (chunk_scan_vec.cuh); the kernels of this
+// The usual layouts run on lanes of several projections (chunk_scan_vec.cuh); the kernels of this
 // file take any broadcast.
 // Every thread keeps raw pointers that advance by one time stride per step, and the loads of
 // eight steps are issued before the first of them is used, so that enough bytes are in flight.
@@ -431,13 +431,13 @@ static int chunk_fwd_len(int chunk_size, int len) {
   return piece < chunk_size ? piece : chunk_size;
 }
 
-// The layouts that the four-projection kernels read: the projection axis contiguous, every row a multiple of four elements and
+// The layouts that the kernels on lanes of `v` projections read: the projection axis contiguous, every row a multiple of `v` elements and
 // aligned to them; B, C, z of X's element type.
-static bool chunk_vec_ok(const ssm_chunk_args& a, int piece) {
-  if (a.proj % 4 != 0 || a.scratch == nullptr || a.par_dtype != a.io_dtype || piece > kPiece) return false;
-  const size_t al = 4 * dtype_size(a.io_dtype);
-  auto rows4 = [&](const ssm_bcast4& p) { return p.sq == 1 && p.sb % 4 == 0 && p.st % 4 == 0 && p.sh % 4 == 0 && aligned_to(p.ptr, al); };
-  if (!rows4(a.Bm) || !rows4(a.Cm) || (a.z.ptr && !rows4(a.z))) return false;
+static bool chunk_vec_ok(const ssm_chunk_args& a, int piece, int v) {
+  if (a.proj % v != 0 || a.scratch == nullptr || a.par_dtype != a.io_dtype || piece > kPiece) return false;
+  const size_t al = v * dtype_size(a.io_dtype);
+  auto rows = [&](const ssm_bcast4& p) { return p.sq == 1 && p.sb % v == 0 && p.st % v == 0 && p.sh % v == 0 && aligned_to(p.ptr, al); };
+  if (!rows(a.Bm) || !rows(a.Cm) || (a.z.ptr && !rows(a.z))) return false;
   return aligned_to(a.X, al) && aligned_to(a.Y, al) && aligned_to(a.scratch, 16);
 }
 
@@ -452,16 +452,20 @@ static int chunk_fwd_t(const ssm_chunk_args& a, cudaStream_t st, int chunk_len, 
     return launch_status("chunk_fwd_kernel<serial>");
   }
   SSM_REQUIRE(nchunks <= 65535, SSM_ERR_TOO_LARGE, "ssd_chunk_scan: more than 65535 chunks");
-  const bool vec = std::is_same<T, PT>::value && chunk_vec_ok(a, chunk_len);
-  const unsigned gv = (HP / 4 + kChunkThreads - 1) / kChunkThreads;
-  if (vec) chunk_fwd4_kernel<T, false><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  else chunk_fwd_kernel<T, PT, 1><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  // projections per lane: what makes 16 bytes, else (16-bit rows on 8-byte boundaries) four, else one
+  constexpr int kWide = 16 / sizeof(T);
+  const int v = !std::is_same<T, PT>::value ? 1 : chunk_vec_ok(a, chunk_len, kWide) ? kWide : chunk_vec_ok(a, chunk_len, 4) ? 4 : 1;
+  const dim3 grid((HP / v + kChunkThreads - 1) / kChunkThreads, nchunks, a.batch);
+  if (v == kWide) chunk_fwd_row_kernel<T, kWide, false><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  else if (v == 4) chunk_fwd_row_kernel<T, 4, false><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  else chunk_fwd_kernel<T, PT, 1><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
   if (int rc = launch_status("chunk_fwd_kernel<local>")) return rc;
   chunk_carry_kernel<<<dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), kCarryLanes * kCarryGroups, 0, st>>>(a, nchunks);
   if (int rc = launch_status("chunk_carry_kernel")) return rc;
   if (through_phase2_only) return SSM_OK;
-  if (vec) chunk_fwd4_kernel<T, true><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  else chunk_fwd_kernel<T, PT, 3><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  if (v == kWide) chunk_fwd_row_kernel<T, kWide, true><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  else if (v == 4) chunk_fwd_row_kernel<T, 4, true><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  else chunk_fwd_kernel<T, PT, 3><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
   return launch_status("chunk_fwd_kernel<apply>");
 }
 
@@ -482,7 +486,7 @@ static bool chunk_bwd_vec_ok(const ssm_chunk_bwd_args& g, int piece, int nchunks
   const int share = a.proj / 4, need = 3 | (a.z.ptr ? 4 : 0);
   ssm_chunk_args f = a;
   f.scratch = g.scratch, f.Y = g.dX;  // only their alignment is looked at
-  if (!chunk_vec_ok(f, piece) || nchunks <= 1 || nchunks > 65535 || (a.typed_grads & need) != need || share > 32 || (share & (share - 1)) != 0) return false;
+  if (!chunk_vec_ok(f, piece, 4) || nchunks <= 1 || nchunks > 65535 || (a.typed_grads & need) != need || share > 32 || (share & (share - 1)) != 0) return false;
   auto rows4 = [&](const ssm_bcast4& p) { return p.sq == 1 && p.sb % 4 == 0 && p.st % 4 == 0 && p.sh % 4 == 0 && aligned_to(p.ptr, al); };
   return rows4(g.dB) && rows4(g.dC) && (!a.z.ptr || rows4(g.dz)) && aligned_to(g.dY, al);
 }

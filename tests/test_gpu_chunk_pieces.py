@@ -43,3 +43,29 @@ def test_gradients_match_oracle(nl, nh, p, gate, per_head, lens, dtype):
         assert a.dtype == ins[k].dtype
         # ddt is a sum over the head's projections of terms of both signs
         close(a, b, **tol, what=f"d{k}", reduced=k in ("A", "D", "dt"))
+
+
+# storage offsets in elements: 0 and 8 leave 16-bit rows on 16-byte boundaries (eight projections per lane), 4 on 8-byte ones (four), 1
+# on none (one); projections that are no multiple of eight go the same ways
+@pytest.mark.parametrize("offset", [0, 8, 4, 1])
+@pytest.mark.parametrize("nl,nh,p,gate,lens,dtype", [(33, 3, 64, True, None, torch.bfloat16), (257, 5, 8, False, [257, 0, 31], torch.float16),
+                                                     (100, 2, 24, True, [99, 100, 1], torch.bfloat16), (64, 4, 12, True, None, torch.float16), (96, 2, 20, True, [7, 96, 33], torch.float32)])
+def test_forward_on_every_lane_width(nl, nh, p, gate, lens, dtype, offset):
+    from ssm_b200 import ops
+
+    nb = 3
+    gen = torch.Generator().manual_seed(nl + p)
+    rnd = lambda *s: torch.randn(*s, generator=gen)  # noqa: E731
+
+    def at(t):  # contiguous, `offset` elements into its allocation
+        buf = torch.empty(t.numel() + offset, dtype=t.dtype, device="cuda")
+        return buf[offset:].view(t.shape).copy_(t)
+
+    X, B, C = (rnd(nb, nl, nh, p).to(dtype) for _ in range(3))
+    z = rnd(nb, nl, nh, p).to(dtype) if gate else None
+    dt, A, D, init = F.softplus(rnd(nb, nl, nh) - 2).to(dtype), -torch.exp(rnd(nh, p) * 0.5), rnd(nh, p), rnd(nb, nh, p)
+    meta = None if lens is None else {"seq_lens": torch.tensor(lens)}
+    with torch.no_grad():
+        y = ops.ssd_chunk_scan(at(X), at(dt), A.cuda(), at(B), at(C), 64, D=D.cuda(), z=None if z is None else at(z), seq_meta=meta, initial_states=init.cuda())
+        yo = orc.ssd_chunk_scan(X.float(), dt.float(), A, B.float(), C.float(), 64, D=D, z=None if z is None else z.float(), seq_meta=meta, initial_states=init)
+    close(y, yo, **(FP32_TOL if dtype == torch.float32 else HALF_TOL), what="y")

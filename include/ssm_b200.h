@@ -23,7 +23,9 @@
 extern "C" {
 #endif
 
-#define SSM_B200_ABI_VERSION 3
+/* Raised with every change of a struct's layout, of an entry point's signature or of the set of entry points.
+ * 4: entry points and fields of the earlier SSD backward removed; log(-A) in the state step; packed sequences, decode steps. */
+#define SSM_B200_ABI_VERSION 4
 
 /* element types of activation tensors.  SSM_F64 selects the double-precision variants of the five operators (forward and
  * backward; written for gradient checking as in upstream's tests/ops/test_backend_gradients.py:1172-1612, not for speed): with
@@ -246,7 +248,6 @@ typedef struct {
   float* scratch; /* nullable: ssm_chunk_scan_bwd_scratch_floats() floats; with it the chunks run in parallel, without it one thread
                      per (batch, head, proj) walks the whole sequence */
   float* fwd_scratch; /* nullable: the scratch that the forward call with the same arguments left behind */
-  float* scratch_fwd; /* set inside the call */
 } ssm_chunk_bwd_args;
 
 int64_t ssm_chunk_scan_bwd_scratch_floats(int32_t batch, int32_t len, int32_t heads, int32_t proj, int32_t chunk_size);

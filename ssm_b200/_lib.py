@@ -13,7 +13,7 @@ from pathlib import Path
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libssm_b200.so"
 
 F32, BF16, F16 = 0, 1, 2
-ABI_VERSION = 3  # SSM_B200_ABI_VERSION of include/ssm_b200.h this binding mirrors
+ABI_VERSION = 4  # SSM_B200_ABI_VERSION of include/ssm_b200.h this binding mirrors
 i32, i64, vp, fp = C.c_int32, C.c_int64, C.c_void_p, C.c_void_p
 
 
@@ -82,7 +82,7 @@ class ChunkBwdArgs(C.Structure):
         ("fwd", ChunkArgs),
         ("dY", vp), ("dX", vp), ("ddt", fp),
         ("dA", Bcast4), ("dB", Bcast4), ("dC", Bcast4), ("dD", Bcast4), ("dz", Bcast4), ("dinitial", Bcast4),
-        ("history", fp), ("scratch", fp), ("fwd_scratch", fp), ("scratch_fwd", fp),
+        ("history", fp), ("scratch", fp), ("fwd_scratch", fp),
     ]
 
 

@@ -262,14 +262,14 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_local_kernel(const ss
 }
 
 // reverse phase 2: over the pieces from the right; R[c] <- adjoint entering piece c from piece c + 1
-__global__ void __launch_bounds__(kCarryLanes * kCarryGroups) chunk_bwd_carry_kernel(const ssm_chunk_bwd_args g, int nchunks) {
+__global__ void __launch_bounds__(kCarryLanes * kCarryGroups) chunk_bwd_carry_kernel(const ssm_chunk_bwd_args g, const float* __restrict__ P_all, int nchunks) {
   const ssm_chunk_args& a = g.fwd;
   const int HP = a.heads * a.proj;
   const int hp_raw = blockIdx.x * kCarryLanes + threadIdx.x % kCarryLanes;
   const bool live = hp_raw < HP;
   const int hp = live ? hp_raw : HP - 1;
   const int b = blockIdx.z;
-  const float* P = g.scratch_fwd + (int64_t)b * nchunks * HP + hp;
+  const float* P = P_all + (int64_t)b * nchunks * HP + hp;
   float* R = g.scratch + 2 * (int64_t)a.batch * nchunks * HP + (int64_t)b * nchunks * HP + hp;
   const float carry = carry_pieces<true>(P, R, nchunks, HP, 0.f, live);
   if (live && threadIdx.x < kCarryLanes && g.dinitial.ptr) {
@@ -288,10 +288,10 @@ __device__ __forceinline__ void add_reduced(float* dst, float v, bool whole_warp
   }
 }
 
-// final pass: MODE 0 = one thread walks the whole sequence (no scratch); MODE 1 = one chunk per blockIdx.y, states and
-// adjoints entering the chunk taken from the scratch.
+// final pass: MODE 0 = one thread walks the whole sequence (no scratch); MODE 1 = one chunk per blockIdx.y, the states entering the
+// chunks taken from S, the adjoints from the scratch.
 template <typename T, typename PT, int MODE>
-__global__ void __launch_bounds__(kChunkThreads) chunk_bwd_kernel(const ssm_chunk_bwd_args g, int nchunks) {
+__global__ void __launch_bounds__(kChunkThreads) chunk_bwd_kernel(const ssm_chunk_bwd_args g, const float* __restrict__ S, int nchunks) {
   const ssm_chunk_args& a = g.fwd;
   Lane<T> ln;
   if (!ln.init(a)) return;
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_kernel(const ssm_chun
     s0 = a.initial.ptr ? bc4_load_f32(a.initial, ln.b, 0, ln.h, ln.q) : 0.f;
     carry = 0.f;
   } else {
-    s0 = g.scratch_fwd[(int64_t)a.batch * nchunks * ln.HP + slot];
+    s0 = S[slot];
     carry = g.scratch[2 * (int64_t)a.batch * nchunks * ln.HP + slot];
   }
   const Stream<T> sx = ln.x(a, t0), sdt = ln.dt(a, t0);
@@ -502,34 +502,35 @@ static int chunk_bwd_t(const ssm_chunk_bwd_args& g_in, cudaStream_t st) {
   const bool vec = std::is_same<T, PT>::value && chunk_bwd_vec_ok(g, a.chunk_size, nchunks);
   SSM_REQUIRE(vec || (g.history && !(a.typed_grads & 8)), SSM_ERR_UNSUPPORTED, "ssd_chunk_scan_backward: this call needs a history and an fp32 ddt");
   if (!g.scratch || nchunks <= 1 || nchunks > 65535) {
-    chunk_bwd_kernel<T, PT, 0><<<dim3(gx, 1, a.batch), kChunkThreads, 0, st>>>(g, 1);
+    chunk_bwd_kernel<T, PT, 0><<<dim3(gx, 1, a.batch), kChunkThreads, 0, st>>>(g, nullptr, 1);
     return launch_status("chunk_bwd_kernel<serial>");
   }
   // states entering every piece and the pieces' decay products: left by the forward call, or formed again (its phases 1 and 2 on
   // this call's scratch; no final state, no Y)
+  const float* P = g.scratch;
   if (g.fwd_scratch && chunk_fwd_len(g_in.fwd.chunk_size, a.len) == a.chunk_size) {
-    g.scratch_fwd = g.fwd_scratch;
+    P = g.fwd_scratch;
   } else {
     ssm_chunk_args f = a;
     f.scratch = g.scratch, f.final_state = nullptr;
     if (int rc = chunk_fwd_t<T, PT>(f, st, a.chunk_size, true)) return rc;
-    g.scratch_fwd = g.scratch;
   }
+  const float* S = P + (int64_t)a.batch * nchunks * HP;
   float* R = g.scratch + 2 * (int64_t)a.batch * nchunks * HP;
   const unsigned gv = (HP / 4 + kChunkThreads - 1) / kChunkThreads;
   if (vec) chunk_bwd_local4_kernel<T><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(g, R, nchunks, a.chunk_size);
   else chunk_bwd_local_kernel<T, PT><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
   if (int rc = launch_status("chunk_bwd_local_kernel")) return rc;
-  chunk_bwd_carry_kernel<<<dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), kCarryLanes * kCarryGroups, 0, st>>>(g, nchunks);
+  chunk_bwd_carry_kernel<<<dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), kCarryLanes * kCarryGroups, 0, st>>>(g, P, nchunks);
   if (int rc = launch_status("chunk_bwd_carry_kernel")) return rc;
   if (vec) {
     const int64_t items = (int64_t)a.batch * nchunks, slots = (int64_t)bwd4_ctas<T>() * sm_count() / gv;  // one wave of CTAs, each looping over pieces
     const int64_t rounds = (items + (slots < 1 ? 1 : slots) - 1) / (slots < 1 ? 1 : slots);
     const unsigned gy = (unsigned)((items + rounds - 1) / rounds);  // as many CTAs as the longest of them makes worthwhile
-    chunk_bwd4_kernel<T><<<dim3(gv, gy), kChunkThreads, 0, st>>>(g, g.scratch_fwd + items * HP, R, nchunks, a.chunk_size, (a.typed_grads & 8) != 0);
+    chunk_bwd4_kernel<T><<<dim3(gv, gy), kChunkThreads, 0, st>>>(g, S, R, nchunks, a.chunk_size, (a.typed_grads & 8) != 0);
     return launch_status("chunk_bwd4_kernel");
   }
-  chunk_bwd_kernel<T, PT, 1><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
+  chunk_bwd_kernel<T, PT, 1><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, S, nchunks);
   return launch_status("chunk_bwd_kernel");
 }
 

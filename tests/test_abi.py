@@ -29,7 +29,7 @@ def test_library_exports_every_declared_symbol():
     for name in names:
         assert hasattr(lib, name), f"{name} is declared in the header but not exported"
         assert name in _lib.ENTRY_POINTS, f"{name} has no ctypes prototype"
-    assert lib.ssm_b200_abi_version() == 3
+    assert lib.ssm_b200_abi_version() == 4
     assert lib.ssm_scan_checkpoint_interval() == 32
 
 
@@ -89,3 +89,15 @@ def test_missing_library_is_a_loud_error(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "nope.so")
     with pytest.raises(RuntimeError, match="no CPU or PyTorch fallback"):
         _lib.load()
+
+
+def test_abi_version_stands_for_this_header():
+    """The version is what a binding checks, so it has to move with the interface.  When this fails: raise SSM_B200_ABI_VERSION (and
+    ABI_VERSION in _lib.py) unless it already is above the last released one, then record the digest printed here."""
+    import hashlib
+
+    text = re.sub(r"/\*.*?\*/", "", HEADER.read_text(), flags=re.S)
+    version = int(re.search(r"#define SSM_B200_ABI_VERSION (\d+)", text).group(1))
+    # structs, enums and prototypes without comments and spacing
+    digest = hashlib.sha256("".join("".join(ln.split()) for ln in text.splitlines() if not ln.lstrip().startswith("#")).encode()).hexdigest()[:16]
+    assert (version, digest) == (4, "e96543baf59aa5b9")

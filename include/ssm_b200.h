@@ -237,7 +237,8 @@ int ssm_chunk_scan_fwd(const ssm_chunk_args* args, ssm_stream_t stream);
  * (b, t, h, q) a distinct element) that the call WRITES, every element of it, zeros beyond a row's length included: no zero-fill
  * by the caller, no fp32 copy to convert afterwards.
  * ssm_chunk_scan_bwd_fused(args) tells whether a call with these arguments (typed_grads bits 0 - 2, layouts, pointers of the
- * gradients of B, C, z) keeps its states in registers: it then needs no history, and bit 3 may be set. */
+ * gradients of B, C, z) keeps its states in registers: it then needs no history, and bit 3 may be set.  Such a call reads
+ * `scratch` and `fwd_scratch` in 16-byte pieces: set them before asking. */
 typedef struct {
   ssm_chunk_args fwd;
   const void* dY;

@@ -488,7 +488,7 @@ static bool chunk_bwd_vec_ok(const ssm_chunk_bwd_args& g, int piece, int nchunks
   f.scratch = g.scratch, f.Y = g.dX;  // only their alignment is looked at
   if (!chunk_vec_ok(f, piece, 4) || nchunks <= 1 || nchunks > 65535 || (a.typed_grads & need) != need || share > 32 || (share & (share - 1)) != 0) return false;
   auto rows4 = [&](const ssm_bcast4& p) { return p.sq == 1 && p.sb % 4 == 0 && p.st % 4 == 0 && p.sh % 4 == 0 && aligned_to(p.ptr, al); };
-  return rows4(g.dB) && rows4(g.dC) && (!a.z.ptr || rows4(g.dz)) && aligned_to(g.dY, al);
+  return rows4(g.dB) && rows4(g.dC) && (!a.z.ptr || rows4(g.dz)) && aligned_to(g.dY, al) && aligned_to(g.fwd_scratch, 16);
 }
 
 template <typename T, typename PT>

@@ -101,3 +101,28 @@ def test_abi_version_stands_for_this_header():
     # structs, enums and prototypes without comments and spacing
     digest = hashlib.sha256("".join("".join(ln.split()) for ln in text.splitlines() if not ln.lstrip().startswith("#")).encode()).hexdigest()[:16]
     assert (version, digest) == (4, "e96543baf59aa5b9")
+
+
+def test_fused_chunk_backward_looks_at_every_pointer_it_reads_in_pieces():
+    """Host logic only: no pointer is followed."""
+    from ssm_b200 import _lib
+
+    lib = _lib.load()
+
+    def fused(**moved):
+        g = _lib.ChunkBwdArgs()
+        f = g.fwd
+        f.batch, f.len, f.heads, f.proj, f.chunk_size, f.io_dtype, f.par_dtype, f.typed_grads = 2, 100, 4, 64, 64, _lib.BF16, _lib.BF16, 7
+        at = {k: 1 << 20 for k in ("X", "dt", "A", "Bm", "Cm", "z", "dY", "dX", "dB", "dC", "dz", "scratch", "fwd_scratch")}
+        at.update({k: (1 << 20) + v for k, v in moved.items()})
+        f.X, f.dt, g.dY, g.dX, g.scratch, g.fwd_scratch = (at[k] for k in ("X", "dt", "dY", "dX", "scratch", "fwd_scratch"))
+        for where, name in ((f, "Bm"), (f, "Cm"), (f, "z"), (g, "dB"), (g, "dC"), (g, "dz")):
+            p = getattr(where, name)
+            p.ptr, p.sb, p.st, p.sh, p.sq = at[name], 100 * 256, 256, 64, 1
+        return lib.ssm_chunk_scan_bwd_fused(ctypes.byref(g))
+
+    assert fused() == 1 and fused(fwd_scratch=-(1 << 20)) == 1  # a missing fwd_scratch is formed again
+    for name in ("X", "Bm", "Cm", "z", "dY", "dX", "dB", "dC", "dz"):
+        assert fused(**{name: 4}) == 0 and fused(**{name: 8}) == 1, name
+    for name in ("scratch", "fwd_scratch"):
+        assert fused(**{name: 8}) == 0 and fused(**{name: 16}) == 1, name

@@ -646,9 +646,14 @@ SsdShape ssd_check(const Tensor& X, const Tensor& dt, const Tensor& A, const Ten
   return s;
 }
 
-// Boundaries of packed sequences as host integers (one read of cu_seqlens), checked.
+// Boundaries of packed sequences as host integers (one read of cu_seqlens), checked.  Called from Python; other threads of the
+// interpreter run while this one waits for the device.
 std::vector<int64_t> seq_bounds(const Tensor& cu, int64_t len) {
-  Tensor host = cu.to(at::kCPU, at::kLong).contiguous();
+  Tensor host;
+  {
+    py::gil_scoped_release unlocked;
+    host = cu.to(at::kCPU, at::kLong).contiguous();
+  }
   std::vector<int64_t> v(host.data_ptr<int64_t>(), host.data_ptr<int64_t>() + host.numel());
   bool ok = v.size() >= 2 && v.front() == 0 && v.back() == len;
   for (size_t i = 1; i < v.size(); ++i) ok = ok && v[i] >= v[i - 1];

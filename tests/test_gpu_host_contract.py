@@ -2,6 +2,9 @@
 
 from __future__ import annotations
 
+import threading
+import time
+
 import pytest
 import torch
 
@@ -43,3 +46,33 @@ def test_decode_steps_refuse_short_vectors(nb):
                 ops.mamba2_step(tok, win, s2, dict(w2, **{key: w2[key].detach()[:1].clone()}))
         with pytest.raises((RuntimeError, ValueError)):
             ops.mamba2_step(tok, [t.cpu() for t in win], s2, w2)
+
+
+def test_packed_scan_waits_without_the_interpreter_lock():
+    from ssm_b200 import ops
+
+    X = torch.randn(1, 600, 2, 64, device="cuda").bfloat16()
+    dt, B, A = torch.rand(1, 600, 2, device="cuda").bfloat16(), torch.randn(1, 600, 1, 128, device="cuda").bfloat16(), -torch.ones(2, device="cuda")
+    cu = torch.tensor([0, 300, 600], device="cuda")
+    ops.ssd_scan(X, dt, A, B, B, 256, cu_seqlens=cu)
+    torch.cuda.synchronize()
+    beats, stop = [], threading.Event()
+
+    def beat():
+        while not stop.is_set():
+            beats.append(time.perf_counter())
+            time.sleep(0.002)
+
+    th = threading.Thread(target=beat)
+    th.start()
+    try:
+        torch.cuda._sleep(600_000_000)  # about 0.3 s of device time ahead of the read of cu_seqlens
+        t0 = time.perf_counter()
+        ops.ssd_scan(X, dt, A, B, B, 256, cu_seqlens=cu)
+        t1 = time.perf_counter()
+    finally:
+        stop.set()
+        th.join()
+    assert t1 - t0 > 0.1, "the call was meant to wait"
+    during = [b for b in beats if t0 < b < t1]
+    assert len(during) > 0.1 * (t1 - t0) / 0.002, f"{len(during)} beats of another thread in {t1 - t0:.3f} s"

@@ -27,7 +27,10 @@ struct Call : torch::CustomClassHolder {
   void input(const OptTensor& t) {
     if (t.has_value() && t->defined()) inputs.push_back(*t);
   }
+  // A call without a node would drop tangents in silence, so they are looked for first.
   bool needs_grad() const {
+    for (const Tensor& t : inputs)
+      TORCH_CHECK_NOT_IMPLEMENTED(!t._fw_grad(0).defined(), "ssm_b200 operators have no forward-mode derivative");
     if (!at::GradMode::is_enabled()) return false;
     for (const Tensor& t : inputs)
       if (t.requires_grad()) return true;

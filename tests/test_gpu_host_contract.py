@@ -76,3 +76,28 @@ def test_packed_scan_waits_without_the_interpreter_lock():
     assert t1 - t0 > 0.1, "the call was meant to wait"
     during = [b for b in beats if t0 < b < t1]
     assert len(during) > 0.1 * (t1 - t0) / 0.002, f"{len(during)} beats of another thread in {t1 - t0:.3f} s"
+
+
+@pytest.mark.parametrize("op", ["scan", "chunk", "conv", "norm", "ssd"])
+def test_forward_mode_is_refused(op):
+    """No operator has a forward-mode rule: a tangent is an error and never dropped."""
+    import torch.autograd.forward_ad as fwd
+
+    from ssm_b200 import ops
+
+    mk = lambda *s: torch.randn(*s, device="cuda")  # noqa: E731
+    with fwd.dual_level():
+        dual = lambda *s: fwd.make_dual(mk(*s), mk(*s))  # noqa: E731
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            if op == "scan":
+                ops.selective_scan(dual(1, 8, 40), mk(1, 8, 40), -torch.rand(8, 16, device="cuda"), mk(1, 1, 16, 40), mk(1, 1, 16, 40))
+            elif op == "chunk":
+                ops.ssd_chunk_scan(dual(1, 40, 2, 8), torch.rand(1, 40, 2, device="cuda"), -torch.rand(2, 8, device="cuda"), mk(1, 40, 2, 8), mk(1, 40, 2, 8), 32)
+            elif op == "conv":
+                ops.dw_causal_conv(mk(1, 8, 40), dual(8, 4))
+            elif op == "norm":
+                ops.fused_layer_norm(mk(1, 3, 64), dual(64), None)
+            else:
+                X = fwd.make_dual(mk(1, 256, 2, 64).bfloat16(), mk(1, 256, 2, 64).bfloat16())
+                B = mk(1, 256, 1, 128).bfloat16()
+                ops.ssd_scan(X, torch.rand(1, 256, 2, device="cuda").bfloat16(), -torch.ones(2, device="cuda"), B, B, 256)

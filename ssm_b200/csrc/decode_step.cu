@@ -448,8 +448,10 @@ static int dec_launch(K kernel, const A& a, const DecSplits& sp, int sms, size_t
   void* params[] = {&arg, &s};
   const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(sms), dim3(kDecThreads), params, smem, st);
   if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here; the next launch starts clean
     set_error("%s: %s", name, cudaGetErrorString(e));
-    return (int)e;
+    // a CTA per SM of the device, but the context may have fewer to give (green contexts, partitions): the separate calls serve it
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported ? SSM_ERR_UNSUPPORTED : (int)e;
   }
   return launch_status(name);
 }

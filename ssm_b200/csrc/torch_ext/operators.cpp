@@ -498,6 +498,14 @@ bool plain(const Tensor& t, at::ScalarType type) {
 }
 bool plain(const OptTensor& t, at::ScalarType type) { return !t.has_value() || plain(*t, type); }
 
+// The outcome of a one-launch step: false when the kernel cannot run here (too few SMs for all of its CTAs at once).  Nothing has been
+// launched then and the states are untouched, so the separate calls can serve the step.
+bool launched(int rc) {
+  if (rc == SSM_ERR_UNSUPPORTED) return false;
+  run(rc);
+  return true;
+}
+
 // Up to 16 sequences: one launch (ssm_mamba1_decode).  More: library GEMMs around the conv and state kernels.  With norm_w the
 // residual add and RMSNorm behind the mixer are included and the result is (normed, residual stream in fp32).
 py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tensor& conv_state, const Tensor& ssm_state, const Tensor& in_x, const Tensor& in_z,
@@ -536,9 +544,10 @@ py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tenso
       a.residual_out = res.data_ptr(), a.resout_dtype = SSM_F32;
       if (residual.has_value()) a.residual = residual->data_ptr(), a.res_dtype = dtype_code(*residual, "mamba1_step residual");
     }
-    run(ssm_mamba1_decode(&a, stream_of(tok)));
-    if (norm_w.has_value()) return py::make_tuple(out, res);
-    return py::cast(out);
+    if (launched(ssm_mamba1_decode(&a, stream_of(tok)))) {
+      if (norm_w.has_value()) return py::make_tuple(out, res);
+      return py::cast(out);
+    }
   }
   Tensor x = at::matmul(tok, in_x.t()), z = at::matmul(tok, in_z.t());
   Tensor u = dw_causal_conv_update(conv_state, x, conv_w, conv_b, "silu");
@@ -589,8 +598,7 @@ Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B
     a.dt_bias = dt_bias.data_ptr<float>(), a.A = A.data_ptr<float>(), a.D = D.data_ptr<float>(), a.norm_w = norm_w.data_ptr(), a.out_proj = out_proj.data_ptr();
     a.conv_state_x = conv_x.data_ptr<float>(), a.conv_state_B = conv_B.data_ptr<float>(), a.conv_state_C = conv_C.data_ptr<float>();
     a.ssm_state = ssm_state.data_ptr<float>(), a.out = out.data_ptr(), a.scratch = scratch.data_ptr();
-    run(ssm_mamba2_decode(&a, stream_of(tok)));
-    return out;
+    if (launched(ssm_mamba2_decode(&a, stream_of(tok)))) return out;
   }
   Tensor z = at::matmul(tok, in_z.t());
   Tensor x = dw_causal_conv_update(conv_x, at::matmul(tok, in_x.t()), wx, bx, "silu");

@@ -101,3 +101,43 @@ def test_forward_mode_is_refused(op):
                 X = fwd.make_dual(mk(1, 256, 2, 64).bfloat16(), mk(1, 256, 2, 64).bfloat16())
                 B = mk(1, 256, 1, 128).bfloat16()
                 ops.ssd_scan(X, torch.rand(1, 256, 2, device="cuda").bfloat16(), -torch.ones(2, device="cuda"), B, B, 256)
+
+
+_REFUSED_STEP = """
+import sys, torch
+from ssm_b200.mixer import Mamba1Block, Mamba2Block
+torch.manual_seed(0)
+b1, b2 = Mamba1Block(64, device="cuda", dtype=torch.bfloat16), Mamba2Block(64, device="cuda", dtype=torch.bfloat16)
+c1, c2 = b1.allocate_inference_cache(3), b2.allocate_inference_cache(3)
+outs = []
+with torch.no_grad():
+    for _ in range(2):
+        tok, res = torch.randn(3, 64, device="cuda").bfloat16(), torch.randn(3, 1, 64, device="cuda")
+        outs += [*b1.step(tok[:, None], res, *c1), b1.mixer_step(tok, c1), b2.mixer_step(tok, c2)]
+torch.save([t.float().cpu() for t in (*outs, *c1, *c2[0], c2[1])], sys.argv[1])
+"""
+
+
+def test_steps_run_when_the_one_launch_kernel_cannot(tmp_path):
+    """The library's decode entry points are replaced by ones that answer "unsupported"; the step goes through the separate calls."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    from tests.gpu_util import close
+
+    (tmp_path / "refuse.c").write_text('#include <stdio.h>\nint ssm_mamba1_decode(void* a, void* s) { fputs("refused1\\n", stderr); return -5; }\n'
+                                       'int ssm_mamba2_decode(void* a, void* s) { fputs("refused2\\n", stderr); return -5; }\n')
+    (tmp_path / "step.py").write_text(_REFUSED_STEP)
+    subprocess.run(["gcc", "-shared", "-fPIC", str(tmp_path / "refuse.c"), "-o", str(tmp_path / "refuse.so")], check=True)
+    root = str(Path(__file__).resolve().parent.parent)
+    got = {}
+    for name, preload in (("one", ""), ("separate", str(tmp_path / "refuse.so"))):
+        env = dict(os.environ, PYTHONPATH=root, **({"LD_PRELOAD": preload} if preload else {}))
+        r = subprocess.run([sys.executable, str(tmp_path / "step.py"), str(tmp_path / name)], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        got[name] = torch.load(tmp_path / name)
+        assert r.stderr.count("refused1") == (4 if preload else 0) and r.stderr.count("refused2") == (2 if preload else 0)
+    for i, (a, b) in enumerate(zip(got["one"], got["separate"])):
+        close(a, b, rtol=2e-2, atol=2e-2, what=str(i))

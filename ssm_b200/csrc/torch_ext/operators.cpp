@@ -840,8 +840,32 @@ std::tuple<Tensor, Tensor, Tensor> ssd_packed(const Tensor& X, const Tensor& dt,
                                               const Tensor& cu_seqlens, bool reset) {
   ValueErrors scope;
   const std::vector<int64_t> cu = seq_bounds(cu_seqlens, X.size(1));
-  auto [Y, states] = ssd_run(X, dt, A, B, C, D, z, dt_bias, softplus, c10::nullopt, chunk, &cu, reset);
-  Tensor last;
+  // One set of launches takes up to 65535 sequences and chunks (a grid axis each); beyond that, groups of sequences one after the other.
+  constexpr int64_t kMost = 65535;
+  const int64_t nseq = (int64_t)cu.size() - 1;
+  std::vector<Tensor> Ys, all;
+  for (int64_t s0 = 0, s1; s0 < nseq; s0 = s1) {
+    int64_t chunks = 0;
+    for (s1 = s0; s1 < nseq && s1 - s0 < kMost; ++s1) {
+      const int64_t more = (cu[s1 + 1] - cu[s1] + chunk - 1) / chunk;
+      if (s1 > s0 && chunks + more > kMost) break;
+      chunks += more;
+    }
+    const bool whole = s1 - s0 == nseq;
+    const int64_t t0 = cu[s0], len = cu[s1] - t0;
+    if (len == 0) {  // nothing but empty sequences
+      all.push_back(at::zeros({s1 - s0, X.size(2), X.size(3), B.size(3)}, X.options().dtype(at::kFloat)));
+      continue;
+    }
+    auto rows = [&](const Tensor& t) { return whole ? t : t.narrow(1, t0, len); };
+    std::vector<int64_t> part(cu.begin() + s0, cu.begin() + s1 + 1);
+    for (int64_t& v : part) v -= t0;
+    auto [y, st] = ssd_run(rows(X), rows(dt), A, rows(B), rows(C), D, z.has_value() ? OptTensor(rows(*z)) : z, dt_bias, softplus, c10::nullopt, chunk, &part, reset);
+    if (reset) Ys.push_back(y);
+    all.push_back(st);
+  }
+  Tensor Y, last, states = all.size() == 1 ? all[0] : at::cat(all);
+  if (reset) Y = Ys.size() == 1 ? Ys[0] : at::cat(Ys, 1);
   if (reset) last = states.slice(0, states.size(0) - 1).clone();
   else std::tie(Y, last) = ssd_run(X, dt, A, B, C, D, z, dt_bias, softplus, init, chunk, nullptr, true);
   return {Y, last, states};

@@ -45,3 +45,30 @@ def test_packed_sequences_match_oracle(lens, nh, ng, dtype, per_channel, reset):
     else:
         yo, so = orc.ssd_scan(X, dt, A, B, C, 256, D=D, z=z, dt_bias=bias, dt_softplus=True, return_final_states=True)
         close(Y, yo, **SSD_TOL, what="Y", reduced=True), close(last, so, **SSD_TOL, what="last state", reduced=True)
+
+
+@pytest.mark.parametrize("empty", [0, 66000])  # sequences of no step in front: a group of nothing else
+def test_more_sequences_than_one_grid_takes(empty):
+    """65536 chunks and more go in groups; each sequence as when it is scanned alone."""
+    from ssm_b200 import ops
+
+    ones, tail = 65700, 300
+    nl = ones + tail
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    X, z, dt = r(1, nl, 1, 64).bfloat16(), r(1, nl, 1, 64).bfloat16(), (torch.rand(1, nl, 1, generator=g, device="cuda") + 0.1).bfloat16()
+    B, C, A, D = r(1, nl, 1, 128).bfloat16() / 11, r(1, nl, 1, 128).bfloat16() / 11, -torch.ones(1, device="cuda"), r(1)
+    cu = torch.cat([torch.zeros(empty, dtype=torch.long), torch.arange(ones + 1), torch.tensor([nl])]).cuda()
+    with torch.no_grad():
+        Y, states = ops.ssd_scan(X, dt, A, B, C, 256, D=D, z=z, cu_seqlens=cu, return_varlen_states=True, check_status=True)
+        yt, st = ops.ssd_scan(X[:, ones:], dt[:, ones:], A, B[:, ones:], C[:, ones:], 256, D=D, z=z[:, ones:], return_final_states=True)
+    assert states.shape[0] == empty + ones + 1 and not states[:empty].any()
+    close(Y[:, ones:], yt, **SSD_TOL, what="Y of the last", reduced=True), close(states[-1], st[0], **SSD_TOL, what="state of the last", reduced=True)
+    # one step from zero: S = dt x B^T, y = (dt B . C + D) x silu(z)
+    x, b, c, d = X[0, :ones, 0].float(), B[0, :ones, 0].float(), C[0, :ones, 0].float(), dt[0, :ones].float()
+    zz = z[0, :ones, 0].float()
+    want = ((b * c).sum(-1, keepdim=True) * d + D) * x * torch.nn.functional.silu(zz)
+    close(Y[0, :ones, 0], want, **SSD_TOL, what="Y", reduced=True)
+    for a in range(0, ones, 10000):
+        e = min(a + 10000, ones)
+        close(states[empty + a:empty + e, 0], (d[a:e] * x[a:e])[:, :, None] * b[a:e, None, :], **SSD_TOL, what="states", reduced=True)

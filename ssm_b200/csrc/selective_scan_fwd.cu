@@ -46,7 +46,7 @@ extern "C" int ssm_scan_checkpoint_interval(void) { return kScanCkpt; }
 
 extern "C" int ssm_scan_split_segments(int32_t batch, int32_t dim, int32_t len, int32_t nstate) {
   if (batch <= 0 || dim <= 0 || len <= 0 || nstate > 32) return 1;  // the split lives in the tile kernel (d_state <= 32)
-  return ssmb::fwd_split_segments(batch, dim, len);
+  return ssmb::fwd_split_segments(batch, dim, len, nstate);
 }
 
 extern "C" int ssm_selective_scan_fwd(const ssm_scan_fwd_args* a, ssm_stream_t stream) {

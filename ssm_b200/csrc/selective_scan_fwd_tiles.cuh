@@ -466,25 +466,32 @@ static __global__ void __launch_bounds__(128) scan_split_combine_kernel(float* _
   }
 }
 
-// Segments of a call cut in time; 1 = no split.  A segment runs its tiles one after the other; CTAs that share an SM slow each other
-// down by what was measured for two and three of them, and a segment has at least two tiles.  Taken is the count with the least time
-// of a pass, if the two passes and the stitching between them are worth it.  (A fixed four tiles and two CTAs per SM before: 2 x 1024
-// rows of 4000 steps 147 us against 126, 512 rows of 256 steps 16.5 against 11.)
-static inline int fwd_split_segments(int batch, int dim, int len) {
+// Segments of a call cut in time; 1 = no split.  A segment runs its tiles one after the other and has at least two.  CTAs that share an
+// SM slow each other down by kShare[how many], which depends on the warps of a CTA (four states each): one or two warps hardly
+// fill an SM's issue slots, eight leave nothing to share, so that only one segment per SM pays.  Taken is the count with the least time
+// of a pass, if both passes and the stitching between them (kCut and three tiles' worth of prologues) take less than no cut.
+// Measured, us of all kernels, against no cut and the best of twelve counts: 16 states, 1 x 512 rows of 2048 steps 31 (132, 31), 2 x 1024
+// of 4000 132 (202, 125), 1 x 3200 of 4096 200 (231, 192), 3 x 640 of 350 27 (37, 27), 1 x 4096 of 512 28 (28, 28; 43 when cut in two);
+// 32 states, 1 x 512 of 2048 47 (155, 47), 2 x 256 of 5000 96 (368, 96), 1 x 4480 of 8192 624 (624, 624; 1115 when cut in three).
+static inline int fwd_split_segments(int batch, int dim, int len, int nstate) {
   const int sms = sm_count();
   const int64_t ctas = (int64_t)batch * ((dim + kTileRows - 1) / kTileRows);
   const int tiles = (len + kScanCkpt - 1) / kScanCkpt;
   if (ctas >= sms) return 1;
-  constexpr double kShare[4] = {0.0, 1.0, 1.1, 1.55};
+  struct Cost {
+    double kShare[4], kCut, kFixed;
+  };
+  static constexpr Cost few{{0.0, 1.0, 1.1, 1.55}, 1.65, 1.0}, four{{0.0, 1.0, 1.55, 2.2}, 1.7, 3.0}, eight{{0.0, 1.0, 2.35, 3.5}, 2.0, 3.0};
+  const Cost& cost = nstate <= 8 ? few : nstate <= 16 ? four : eight;
   double best = 1e300;
   int segs = 1;
   for (int per = 2; per < tiles; ++per) {  // tiles per segment
     const int64_t used = (tiles + per - 1) / per, share = (ctas * used + sms - 1) / sms;
     if (share > 3) continue;
-    if (per * kShare[share] < best) best = per * kShare[share], segs = (int)used;
+    if (per * cost.kShare[share] < best) best = per * cost.kShare[share], segs = (int)used;
     if (share == 1) break;  // longer segments only get slower
   }
-  return 1.65 * best + 1.0 < tiles ? segs : 1;  // the first pass, without outputs, costs about two thirds of the second
+  return cost.kCut * best + cost.kFixed < tiles ? segs : 1;
 }
 
 template <typename T, int NG, bool RAG>

@@ -126,3 +126,19 @@ def test_fused_chunk_backward_looks_at_every_pointer_it_reads_in_pieces():
         assert fused(**{name: 4}) == 0 and fused(**{name: 8}) == 1, name
     for name in ("scratch", "fwd_scratch"):
         assert fused(**{name: 8}) == 0 and fused(**{name: 16}) == 1, name
+
+
+# the rule for 148 SMs (which it assumes where there is no device): calls that a cut was measured to slow down stay whole, those that
+# it speeds up are cut into the counts that were measured best or close to it
+@pytest.mark.parametrize("batch,dim,length,nstate,segments", [
+    (1, 4096, 512, 16, 1), (1, 4096, 1024, 16, 1), (1, 4480, 8192, 16, 1), (1, 512, 2048, 16, 16), (1, 1024, 3000, 16, 9), (2, 256, 5000, 16, 27), (3, 640, 350, 16, 6),
+    (1, 4096, 512, 32, 1), (1, 3200, 4096, 32, 1), (1, 4480, 8192, 24, 1), (2, 1536, 1500, 32, 1), (1, 2048, 1024, 32, 1), (1, 512, 2048, 32, 8), (2, 256, 5000, 24, 9),
+    (1, 1024, 3000, 8, 9), (1, 768, 200, 4, 4), (1, 8192, 512, 16, 1), (1, 512, 2048, 33, 1)])
+def test_segments_of_a_selective_scan(batch, dim, length, nstate, segments):
+    import torch
+
+    from ssm_b200 import _lib
+
+    if torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("stated for 148 SMs")
+    assert _lib.load().ssm_scan_split_segments(batch, dim, length, nstate) == segments

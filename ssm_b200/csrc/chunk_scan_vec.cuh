@@ -6,7 +6,7 @@
 // The sequence is cut into pieces of at most kPiece steps (whatever the caller's chunk size: the recurrence does not depend on
 // the cut), which is what puts enough independent walks in flight.  Forward: local states, carry over the pieces, replay.
 // Backward: the states that enter the pieces are kept from the forward pass (1/32 of X in fp32), so it starts with the local
-// adjoints; the final pass then keeps the states of kSub steps in registers while it walks them back, instead of writing
+// adjoints; the final pass then keeps the states of kBwdSub steps in registers while it walks them back, instead of writing
 // an fp32 history of the whole sequence and reading it again.
 #pragma once
 
@@ -218,8 +218,8 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_local4_kernel(const s
 // of the group to its left are under way.  CTAs keep their projections and loop over pieces, so that the sums over batch and
 // time (dA, dD) cost one addition per CTA and lane instead of one per piece (additions to one word are served one after the
 // other, about 40 ns each).  Bound by latency: X, B (twice, the second time from the L2), C, z, dY in, dX, dB, dC, dz out, 302 MB
-// in 115 us at (8, 2048, 16, 64) bf16.  The scalar pass with an fp32 history took 196 us; groups of 16 steps without requests
-// ahead 163, of 8 131, of 4 123, of 2 with requests ahead 115.
+// in 110 us at (8, 2048, 16, 64) bf16.  The scalar pass with an fp32 history took 196 us; groups of 16 steps without requests
+// ahead 163, of 8 131, of 4 123, of 2 with requests ahead 115, with rows converted word by word 110.
 constexpr int kBwdSub = 2;    // steps of a group
 constexpr int kBwdSweep = 8;  // steps per batch of loads of the forward sweep
 template <typename T>

@@ -126,7 +126,6 @@ struct Vec16 {
   static constexpr int N = 16 / sizeof(T);
   uint4 raw;
   __device__ __forceinline__ void load(const T* p) { raw = __ldg(reinterpret_cast<const uint4*>(p)); }
-  __device__ __forceinline__ void load_stream(const T* p) { raw = __ldcs(reinterpret_cast<const uint4*>(p)); }
   __device__ __forceinline__ void store(T* p) const { *reinterpret_cast<uint4*>(p) = raw; }
   __device__ __forceinline__ void store_stream(T* p) const { __stcs(reinterpret_cast<uint4*>(p), raw); }
   // 16-bit elements two at a time: a shift and a mask (or one convert) per 32-bit word in, one packed convert per word out; element
@@ -176,7 +175,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float exp_fast(float x) { return ex2_approx(x * kLog2e); }
 // torch.nn.functional.softplus with its defaults: identity above 20, log1p(exp(x)) below.
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }

@@ -635,14 +635,15 @@ __device__ __forceinline__ float2 silu_grad2(float2 p) {
 // accumulators are pairs of channels for the packed-fp32 instructions, the taps exist once, and the eight steps of a batch of loads run
 // without any check unless they touch an end of the tile.  Bound by instructions (about 13 per element; the kernel above
 // takes 31), hence four CTAs per SM and a tile length that fills whole waves (conv_cl_tile).
-// (4, 4093, 2560) bf16, 251 MB: 154 us with the kernel above, 76 us with this one (3.3 TB/s; two channels per thread and six CTAs
+// (4, 4093, 2560) bf16, 251 MB: 154 us with the kernel above, 73 us with this one (3.4 TB/s; two channels per thread and six CTAs
 // more per SM: 91).  Narrow tensors, NT = 512: (2, 16384, 128) bf16 72 -> 18 us.
 template <typename T, int V, int NT>
 __global__ void __launch_bounds__(NT, V == 4 ? 512 / NT : 768 / NT) conv_cl_bwd4_kernel(const ssm_conv_bwd_args g, int tile) {
   const ssm_conv_args& a = g.fwd;
   constexpr int U = 32 / (V * (int)sizeof(T) / 2);  // steps per batch of loads: 64 bytes of x and of dy a thread
   constexpr int P = V / 2;
-  using Raw = typename std::conditional<V * sizeof(T) == 16, uint4, typename std::conditional<V * sizeof(T) == 8, uint2, uint32_t>::type>::type;
+  static_assert(V == 4, "a thread's channels are one load of 8 or 16 bytes");
+  using Raw = typename std::conditional<V * sizeof(T) == 16, uint4, uint2>::type;
   const int C = a.channels, L = a.len, nvec = C / V;
   const int64_t item = (int64_t)blockIdx.x * NT + threadIdx.x;  // channel groups fastest, then time tiles
   const int c0 = (int)(item % nvec) * V;

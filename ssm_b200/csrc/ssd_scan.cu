@@ -522,27 +522,27 @@ __global__ void __launch_bounds__(256) ssd_fold_init_kernel(const ssm_ssd_args a
 }
 
 // ---------------------------------------------------------------------------------------------
-// chunk scan: one CTA (256 threads) per (batch, chunk, 128-row block m, part of the heads of one
+// chunk scan: one CTA (512 threads) per (batch, chunk, 128-row block m, part of the heads of one
 // B / C group).  Heads of a group share B and C, so  G = C_m B^T  (128 x 128 (m+1), causal: only
 // steps before the block's last row) is formed ONCE per CTA; every thread then keeps its part of
-// G (one row, half of the steps) in registers while the CTA walks its heads:
+// G (one row, a quarter of the steps) in registers while the CTA walks its heads:
 //   per head:  G times the head's decay mask exp2(c_i - c_j) delta_j [j <= i], packed as the A
-//              operand (overwrites the dead B tile);  Y_intra = (G o L) X  and  Y_inter = C_m S_in
-//              accumulate in TMEM while the previous head's result is read back, gated and staged.
-//   Copies (cp.async, whole 128 / 256-byte rows per group of lanes) run one head ahead into the
-//   other half of a double buffer: x, the incoming state, the exponent vectors; z goes through
-//   the same 16 KB staging tile that carries y back out, so that every global access of the
-//   head loop touches whole 128-byte lines.
+//              operand (in tensor memory, over the dead G columns);  Y_intra = (G o L) X  and
+//              Y_inter = C_m S_in accumulate in TMEM while the previous head's result is read
+//              back, gated and staged.
+//   Copies (TMA and bulk copies issued by one thread) run one head ahead into the other half of a
+//   double buffer: x, the incoming state, the exponent vectors; z has two buffers of its own over
+//   the dead B tile; y is staged in a 16 KB tile and leaves by a TMA store.
 //   TMEM columns: G [0,256); per buffer b: Y_intra [256+128b, +64), Y_inter [320+128b, +64).
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 struct ScanSmem {
   static constexpr int C_BYTES = kBlk * kN * 2;     // C rows of the block: two blocks (states 0..63, 64..127) of [i][128 B], swizzled   32 KB
-  static constexpr int B_BYTES = kQ * kN * 2;       // B rows likewise, [j][128 B] per block; later the masked tile, K-major [j/8][i][8]  64 KB
+  static constexpr int B_BYTES = kQ * kN * 2;       // B rows likewise, [j][128 B] per block; later the gate tiles of two heads  64 KB
   static constexpr int X_BYTES = kQ * kP * 2;       // x rows [j][64 p], 128-byte rows, TMA 128-byte swizzle  32 KB (x2)
   static constexpr int S_BYTES = kP * kN * 2;       // incoming state, MN-major [p/8][n][8]                 16 KB (x2)
   static constexpr int VEC_BYTES = 2 * kQ * 4;      // c and c - log2(delta) of the chunk                     2 KB (x2)
-  static constexpr int Z_BYTES = kBlk * kP * 2;     // z in / y out of one head: [row][64 p], same swizzle    16 KB
+  static constexpr int Z_BYTES = kBlk * kP * 2;     // y of one head on its way out: [row][64 p], same swizzle  16 KB
   static constexpr int W_BYTES = 1024 * 4;          // per warp: the column factors of its mask chunks (16 warps x 64)          4 KB
   static constexpr int TOTAL = C_BYTES + B_BYTES + 2 * (X_BYTES + S_BYTES + VEC_BYTES) + Z_BYTES + W_BYTES;
   static constexpr int ALLOC = TOTAL + 1024;        // the tiles TMA swizzles must start on 1024-byte boundaries
@@ -752,7 +752,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     }
     if (dots && has_z) {
       const int t = t0 + ROW0 + i_loc;
-      // the threads of a row (column slices) add to one zero-initialised word: the sum does not depend on their order
+      // the four threads of a row (column slices) add to one zero-initialised word, in any order: its last bits vary from run to run
       if (t < a.len) atomicAdd(a.row_dots + ((int64_t)b * a.len + t) * a.heads + h, dot);
     }
     tc::fence_async_smem();  // the staged rows leave through a bulk store
@@ -1072,7 +1072,10 @@ static int ssd_scan_launch(const ssm_ssd_args& a, const ScanMaps& maps, unsigned
 // Heads per scan CTA: a divisor of the heads of one B / C group, so that a CTA's heads share their G.  One CTA runs per SM; the
 // long row blocks go first, then the short ones, each to the first SM that is free.  A long block costs 2 + d and a short one
 // 3 + 0.85 d head times (C / B tiles, G, pipeline fill; fitted to d = 8, 12, 16, 24 on 64 + 64 pieces).  Taken is the d with the
-// earliest end.  Counting whole waves of equal blocks instead chose d = 8 for 76 chunks of 48 heads: 143 us against 122 with 24.
+// earliest end: within 2 % of the best divisor in ten dense shapes of both types from 1 x 300 steps of 80 heads (14.8 us) to 8 x 8192 of
+// 48 (387).  Of packed sequences the number of long blocks is a guess, good while they are longer than a chunk (24 in 16384 steps, 48
+// heads: 127 us, the best) and up to 15 % off when they are not (200 in 16384: 192 against 167 with 24; 64 in 4096, 8 heads: 26
+// against 16 with 4).  Counting whole waves of equal blocks instead chose d = 8 for 76 chunks of 48 heads: 143 us against 122 with 24.
 static int scan_heads_per_cta(int hpg, int64_t longs, int64_t shorts) {
   const int64_t sms = sm_count();
   double best = 1e300;
@@ -1118,8 +1121,10 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
     // heads per CTA of the sequential state kernel: enough to bring the grid down to about one CTA per SM (its CTAs all run
     // for the whole sequence, so a second, partial wave would double the time), at most 4, and a divisor of the heads of one
     // B / C group.  Packed sequences differ in length, so their walks spread over the SMs by themselves as long as there are
-    // many; two heads share a B tile, four make the longest walk longer (24 sequences of 16384 steps, 48 heads: 104 us with
-    // four, 65 with two, 68-80 with one).
+    // many; two heads share a B tile, four make the longest walk longer.  us with one / two / three / four heads, 48 heads unless
+    // stated: 24 sequences in 16384 steps 77 / 57 / 57 / 72, 2 in 16384 72 / 86 / 128 / 269 (one is taken), 64 in 16384 137 / 98 / 92 / 101,
+    // 200 in 16384 353 / 244 / 214 / 228, 64 in 65536 225 / 165 / 153 / 200, 8 in 4096 with 24 heads 18.5 / 22.5 / 31 / 50, 32 short ones and one
+    // of 14336 steps 148 / 151 / 203 / 405.
     const int most = a.num_seqs ? 2 : 4;
     int shpc = (int)(((int64_t)walks * a.heads + sm_count() - 1) / sm_count());
     shpc = shpc < 1 ? 1 : (shpc > most ? most : shpc);

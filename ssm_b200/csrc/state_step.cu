@@ -419,9 +419,7 @@ static int step_stream_launch(const ssm_step_args& a, int sms, cudaStream_t st) 
 }
 template <typename T, typename BT>
 static int step_fwd_fast_n(const ssm_step_args& a, cudaStream_t st) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const int64_t rows = (int64_t)a.batch * a.dim;
   if (rows * a.nstate / 512 >= (int64_t)2 * sms * kStreamCtasPerSm * (kStreamThreads / 32) && rows < (1ll << 30)) {
     switch (a.nstate) {

@@ -642,8 +642,8 @@ __global__ void __launch_bounds__(NT, V == 4 ? 512 / NT : 768 / NT) conv_cl_bwd4
   const ssm_conv_args& a = g.fwd;
   constexpr int U = 32 / (V * (int)sizeof(T) / 2);  // steps per batch of loads: 64 bytes of x and of dy a thread
   constexpr int P = V / 2;
-  static_assert(V == 4, "a thread's channels are one load of 8 or 16 bytes");
-  using Raw = typename std::conditional<V * sizeof(T) == 16, uint4, uint2>::type;
+  static_assert(V * sizeof(T) == 8, "a thread's channels of a step are one load of 8 bytes");
+  using Raw = uint2;
   const int C = a.channels, L = a.len, nvec = C / V;
   const int64_t item = (int64_t)blockIdx.x * NT + threadIdx.x;  // channel groups fastest, then time tiles
   const int c0 = (int)(item % nvec) * V;

@@ -37,7 +37,9 @@ struct Call : torch::CustomClassHolder {
     return false;
   }
   virtual variable_list forward(bool train) = 0;
-  virtual variable_list backward(const variable_list& grads) = 0;  // one gradient (or an undefined tensor) per input
+  // One gradient (or an undefined tensor) per input.  An incoming gradient is undefined where nothing flowed back to that output, and all
+  // of them can be (a node downstream that returns none).
+  virtual variable_list backward(const variable_list& grads) = 0;
 };
 
 struct CallFn : torch::autograd::Function<CallFn> {
@@ -307,7 +309,7 @@ struct ChunkCall final : Call {
   variable_list backward(const variable_list& grads) override {
     c10::cuda::CUDAGuard guard(c.X.device());
     const auto f32 = c.X.options().dtype(at::kFloat);
-    Tensor gy = like(grads[0], c.X);
+    Tensor gy = grads[0].defined() ? like(grads[0], c.X) : at::zeros_like(c.X);
     Tensor dX = at::empty_like(c.X), ddt, dA, dB, dC, dD, dz, dI, hist;
     ZeroPool params, per_row, per_step;
     int typed = 0;
@@ -379,7 +381,7 @@ struct ConvCall final : Call {
   }
   variable_list backward(const variable_list& grads) override {
     c10::cuda::CUDAGuard guard(c.x.device());
-    Tensor go = rows_like(grads[0], c.x), dx = at::empty_like(c.x), dw, db;
+    Tensor go = grads[0].defined() ? rows_like(grads[0], c.x) : at::zeros_like(c.x), dx = at::empty_like(c.x), dw, db;
     ZeroPool pool;
     pool.add(dw, {c.nc, c.k});
     if (c.b.has_value()) pool.add(db, {c.nc});

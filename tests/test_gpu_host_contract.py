@@ -141,3 +141,39 @@ def test_steps_run_when_the_one_launch_kernel_cannot(tmp_path):
         assert r.stderr.count("refused1") == (4 if preload else 0) and r.stderr.count("refused2") == (2 if preload else 0)
     for i, (a, b) in enumerate(zip(got["one"], got["separate"])):
         close(a, b, rtol=2e-2, atol=2e-2, what=str(i))
+
+
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, t):
+        return t.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+@pytest.mark.parametrize("op", ["scan", "chunk", "conv", "norm", "ssd"])
+def test_a_node_that_returns_no_gradient_is_zero_upstream(op):
+    from ssm_b200 import ops
+
+    mk = lambda *s: torch.randn(*s, device="cuda", requires_grad=True)  # noqa: E731
+    A = -torch.rand(8, 16, device="cuda")
+    if op == "scan":
+        x = mk(1, 8, 40)
+        y = ops.selective_scan(x, mk(1, 8, 40), A, mk(1, 1, 16, 40), mk(1, 1, 16, 40))
+    elif op == "chunk":
+        x = mk(1, 40, 2, 8)
+        y = ops.ssd_chunk_scan(x, torch.rand(1, 40, 2, device="cuda"), -torch.rand(2, 8, device="cuda"), mk(1, 40, 2, 8), mk(1, 40, 2, 8), 32)
+    elif op == "conv":
+        x = mk(1, 8, 40)
+        y = ops.dw_causal_conv(x, mk(8, 4))
+    elif op == "norm":
+        x = mk(1, 3, 64)
+        y = ops.fused_layer_norm(x, mk(64), None)
+    else:
+        x = torch.randn(1, 256, 2, 64, device="cuda").bfloat16().requires_grad_()
+        B = torch.randn(1, 256, 1, 128, device="cuda").bfloat16()
+        y = ops.ssd_scan(x, torch.rand(1, 256, 2, device="cuda").bfloat16(), -torch.ones(2, device="cuda"), B, B, 256)
+    _NoGradient.apply(y).sum().backward()
+    assert x.grad is None or not x.grad.any()

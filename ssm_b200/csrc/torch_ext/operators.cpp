@@ -706,8 +706,10 @@ std::tuple<Tensor, Tensor> ssd_run(const Tensor& X_, const Tensor& dt_, const Te
   } else {
     bytes = ssm_ssd_scratch_bytes((int)s.nb, (int)s.nl, (int)s.nh), state_bytes = ssm_ssd_state_scratch_bytes((int)s.nb, (int)s.nl, (int)s.nh);
   }
-  Tensor Y, fin = at::empty({walks, s.nh, s.np, s.nn}, f32);
+  Tensor Y, fin;
   if (want_y) Y = at::empty_like(X);
+  if (s.nl == 0) return {Y, init.has_value() ? init->clone() : at::zeros({walks, s.nh, s.np, s.nn}, f32)};  // no step: the state stays what it was
+  fin = at::empty({walks, s.nh, s.np, s.nn}, f32);
   Tensor ws = at::empty({bytes}, X.options().dtype(at::kByte));
   const int64_t vec = s.nh * nchunks * chunk * 4;
   char* base = reinterpret_cast<char*>(ws.data_ptr());
@@ -755,6 +757,14 @@ struct SsdCall final : Call {
     const bool init_grad = init_.has_value() && init_->requires_grad();
     const int io = dtype_code(X, "ssd_scan");
     ssm_stream_t stream = stream_of(X);
+    if (nl == 0) {  // the gradient of the final state is that of the initial one; everything else is empty or zero
+      variable_list none;
+      for (const Tensor* t : {&X_, &dt_, &A_, &B_, &C_}) none.push_back(at::zeros_like(*t));
+      for (const OptTensor* t : {&D_, &z_, &bias_})
+        if (t->has_value()) none.push_back(at::zeros_like(**t));
+      if (init_.has_value()) none.push_back(!init_grad ? Tensor() : gfin.has_value() ? cast(gfin->clone(), init_->scalar_type()) : at::zeros_like(*init_));
+      return none;
+    }
 
     Tensor u, qd, dB, dC, dA, dD, dbias;
     ZeroPool work, coeffs, params;

@@ -188,3 +188,22 @@ def test_a_wait_that_runs_out_is_reported_and_the_device_stays_usable():
     Yg = ops.ssd_scan(t["X"], t["dt"], t["A"], t["B"], t["C"], 256, dt_softplus=True, check_status=True)
     Yo = orc.ssd_scan(t["X"].cpu(), t["dt"].cpu(), t["A"].cpu(), t["B"].cpu(), t["C"].cpu(), 256, dt_softplus=True)
     close(Yg, Yo, **SSD_TOL, what="Y after the reported failure", reduced=True)
+
+
+@pytest.mark.parametrize("with_init", [False, True])
+def test_a_sequence_of_no_steps_keeps_its_state(with_init):
+    from ssm_b200 import ops
+
+    m = lambda *s: torch.randn(*s, device="cuda").bfloat16().requires_grad_()  # noqa: E731
+    X, z, dt, B, C = m(2, 0, 4, 64), m(2, 0, 4, 64), m(2, 0, 4), m(2, 0, 1, 128), m(2, 0, 1, 128)
+    A, D = (-torch.ones(4, device="cuda")).requires_grad_(), torch.ones(4, device="cuda", requires_grad=True)
+    init = torch.randn(2, 4, 64, 128, device="cuda", requires_grad=True) if with_init else None
+    used = torch.full((2, 4, 64, 128), 7.0, device="cuda")  # memory that the call is likely to be given
+    del used
+    Y, final = ops.ssd_scan(X, dt, A, B, C, 256, D=D, z=z, initial_states=init, return_final_states=True)
+    assert Y.shape == X.shape and torch.equal(final, init if with_init else torch.zeros_like(final))
+    leaves = [X, dt, A, B, C, D, z] + ([init] if with_init else [])
+    grads = torch.autograd.grad((final * 3).sum() + Y.float().sum(), leaves)
+    assert all(g.shape == t.shape and g.dtype == t.dtype for g, t in zip(grads, leaves)) and not grads[2].any() and not grads[5].any()
+    if with_init:
+        assert torch.equal(grads[-1], torch.full_like(init, 3.0))

@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) ssd_state_kernel(const ssm_s
   const int c_off = packed ? __ldg(seq_first) : 0;
   const int nwalk = packed ? __ldg(seq_first + 1) - c_off : nchunks;
   const int t_off = packed && nwalk > 0 ? __ldg(a.seq_table + 2 * c_off) : 0;
+  const int walk_len = packed && nwalk > 0 ? __ldg(a.seq_table + 2 * c_off + 1) - t_off : 0;
   const int n_states = packed ? a.num_seqs : a.batch;  // batch extent of the states
   const int n = (warp & 3) * 32 + lane;  // this thread's state index = TMEM lane
   constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) ssd_state_kernel(const ssm_s
   const int64_t vrow0 = (((int64_t)b * a.heads + h0) * nchunks + c_off) * kQ;  // exponent vectors of head h0 (next head: + nchunks * kQ)
   const int nst = SPC * nwalk;
   // steps of the sequence from the first step of a stage on (packed sequences only; the first stage of a chunk has at least one)
-  auto steps_left = [&](int c, int part) { return __ldg(a.seq_table + 2 * (c_off + c) + 1) - (t_off + c * kQ + part * kStep); };
+  auto steps_left = [&](int c, int part) { return walk_len - c * kQ - part * kStep; };
   auto chunk_of = [&](int c) { return REV ? nwalk - 1 - c : c; };  // c-th chunk of the walk
   // stage s = steps [s * 64, s * 64 + 64), issued by one thread: two boxes of B, one box of x per head, and the exponents.
   // Steps beyond the sequence read as zero.
@@ -565,8 +566,9 @@ struct ScanMaps {
 // and x, and G the adjoint that enters the chunk from the right (off: the decay of the chunk and of the step after it).  It is the
 // mirror image in time: columns at or after the row's step, the long block is rows 0..127.
 // PACKED: several sequences along the time axis; rows behind the end of a chunk's sequence belong to the next one.  Their columns of the
-// mask are zero, but 0 x Inf is NaN: K slices of 16 steps beyond the end are not multiplied, and the x rows of the slice in
-// which it ends are overwritten with zeros.
+// mask are zero, but 0 x Inf is NaN: the x rows under them are overwritten with zeros.  Kernel us without / with that, 24 sequences in
+// 16384 steps of 48 heads 121 / 123, 4 in 6344 of 28 heads 39.3 / 39.8 (by all warps in front of the mask 124 and 42; with an instance of
+// the body for ragged blocks, which the instruction cache does not hold beside the other two, 131 and 49).
 template <typename T, int MB, bool XSKIP, bool REV, bool PACKED>
 __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanMaps& maps, int nchunks, int hpc, int nparts, unsigned char* smraw,
                                               uint64_t* mbar, uint32_t* tmem_slot) {
@@ -773,10 +775,6 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   for (int hi = 0; hi < nh; ++hi) {
     const int h = h0 + hi, buf = hi & 1;
     ok = !fail && tc::mbar_wait(mb_full(buf), (hi >> 1) & 1);  // this head's operands (no more waiting once a wait ran out)
-    if (ragged && tid < (-k_live & 15) * 8) {  // x rows of the next sequence in the last K slice
-      *reinterpret_cast<uint4*>(sX + buf * M::X_BYTES + (size_t)(k_live * 8 + tid) * 16) = make_uint4(0, 0, 0, 0);
-      tc::fence_async_smem();
-    }
     // ---- factors of the decay mask, formed before the CTA-wide barrier below so that their latency (shared-memory reads, ex2,
     // the exchange of the column factors through sW) overlaps the wait for the slowest warp; the barrier also orders the
     // writes to sW before the reads of the other lanes
@@ -906,8 +904,8 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const bool cut = diag && (REV ? q + e < lane : q + e > lane);  // selected and not multiplied by zero: G may be Inf there
-            f[e] = cut ? 0.f : vG[k][q + e] * ex2_approx(re - col(jb + q + e));
+            f[e] = vG[k][q + e] * ex2_approx(re - col(jb + q + e));
+            if (diag && (REV ? q + e < lane : q + e > lane)) f[e] = 0.f;  // after the product: G may be Inf there
             if (!REV && diag && q + e == lane) f[e] += Dfold;
           }
           Vec16<T> o;
@@ -924,7 +922,11 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     for (int q = 0; q < kXR; ++q)
       xr[q] = XSKIP ? *reinterpret_cast<const uint4*>(swz(sX + buf * M::X_BYTES, i_chunk, wg * kEU + q)) : make_uint4(0, 0, 0, 0);
 
-
+    if (ragged && (warp == 13 || warp == 14)) {  // x rows of the next sequence, by two of the warps that have had the least mask work
+#pragma unroll 1
+      for (int u = k_live * 8 + tid - 13 * 32; u < KJ * 8; u += 64) *reinterpret_cast<uint4*>(sX + buf * M::X_BYTES + (size_t)u * 16) = make_uint4(0, 0, 0, 0);
+      tc::fence_async_smem();
+    }
     if (tid == kCopyThread && hi >= 2) tc::bulk_wait_read();  // the staging tile may be overwritten by the epilogue below
     tc::fence_before_sync();
     __syncthreads();
@@ -938,7 +940,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
       const uint32_t dY = tmem + 256 + buf * 128;
 #pragma unroll
       for (int kk = 0; kk < KJ / 16; ++kk)  // 16 steps = 16 rows of 128 bytes of the x tile
-        if (!PACKED || kk * 16 < k_live) tc::mma_ts(dY, tmem + kk * 8, dx0 + (uint64_t)(kk * (2048 >> 4)), idY, kk > 0);  // A: 16 steps = 8 columns of the masked rows
+        tc::mma_ts(dY, tmem + kk * 8, dx0 + (uint64_t)(kk * (2048 >> 4)), idY, kk > 0);  // A: 16 steps = 8 columns of the masked rows
       tc::commit(mb_mma(buf));
     }
     // ---- the previous head's result, while the tensor cores work on this one ---------------------------------

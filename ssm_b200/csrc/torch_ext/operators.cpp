@@ -829,6 +829,11 @@ struct SsdCall final : Call {
     run(ssm_ssd_bwd_steps(&s, stream));
 
     auto to = [](const Tensor& grad, const Tensor& t) { return cast(grad, t.scalar_type()); };
+    if (const auto type = B_.scalar_type(); type != at::kFloat && type == C_.scalar_type()) {  // neighbours at the end of the pool: one conversion
+      const int64_t n = dB.numel();
+      Tensor both = work.all.narrow(0, work.all.numel() - 2 * n, 2 * n).to(type);
+      dB = both.narrow(0, 0, n).view(dB.sizes()), dC = both.narrow(0, n, n).view(dC.sizes());
+    }
     variable_list res = {dX, to(ddt, dt_), to(dA, A_), to(dB, B_), to(dC, C_)};
     if (D_.has_value()) res.push_back(to(dD, *D_));
     if (z_.has_value()) res.push_back(to(dz, *z_));

@@ -433,6 +433,8 @@ def dw_causal_conv_update(conv_state: Tensor, x: Tensor, weight: Tensor, bias: O
 
 
 class _NormCtx:
+    """Operands of a norm call for direct use of the C ABI: the allocation-free backward has no operator of its own."""
+
     def __init__(self, x, weight, bias, residual, is_rms, eps, prenorm):
         if x.ndim != 3:
             raise ValueError("x must have shape (B, L, D).")

@@ -10,11 +10,11 @@ pytestmark = pytest.mark.gpu
 
 def _check(out, leaves, small):
     grads = dict(zip(leaves, torch.autograd.grad(out.float().sum(), list(leaves.values()))))
-    budget = sum(-(-grads[k].numel() // 64) * 256 for k in small)  # every small one on 256-byte lines of its own
+    room = sum(-(-grads[k].numel() // 64) * 256 for k in small)  # every small one on 256-byte lines of its own
     for k in small:
-        assert grads[k].untyped_storage().nbytes() <= budget, (k, grads[k].untyped_storage().nbytes())
+        assert grads[k].untyped_storage().nbytes() <= room, (k, grads[k].untyped_storage().nbytes())
     for k, g in grads.items():  # any gradient: at most a few others of its own size
-        assert g.untyped_storage().nbytes() <= 4 * max(g.numel() * g.element_size(), 256) + budget, k
+        assert g.untyped_storage().nbytes() <= 4 * max(g.numel() * g.element_size(), 256) + room, k
     return grads
 
 

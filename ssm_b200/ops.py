@@ -41,6 +41,34 @@ def _native():
     return _ops
 
 
+class _Traced(torch.autograd.Function):
+    """One call inside ``torch.jit.trace``: a Python node of the traced graph, which makes the call again whenever the graph runs.
+    (The allocations of a compiled call would be recorded without its launches.)  Its backward is that of the call inside."""
+
+    @staticmethod
+    def forward(ctx, name, *args):
+        with torch.enable_grad():
+            ctx.leaves = [a.detach().requires_grad_(a.requires_grad) if isinstance(a, Tensor) else a for a in args]
+            out = getattr(_native(), name)(*ctx.leaves)
+        ctx.outs = out if isinstance(out, tuple) else (out,)
+        res = tuple(t.detach() for t in ctx.outs)
+        return res if isinstance(out, tuple) else res[0]
+
+    @staticmethod
+    def backward(ctx, *grads):
+        live = [a for a in ctx.leaves if isinstance(a, Tensor) and a.requires_grad]
+        pairs = [(o, g) for o, g in zip(ctx.outs, grads) if g is not None and o.requires_grad]
+        got = iter(torch.autograd.grad([o for o, _ in pairs], live, [g for _, g in pairs], retain_graph=True, allow_unused=True))
+        return (None, *(next(got) if isinstance(a, Tensor) and a.requires_grad else None for a in ctx.leaves))
+
+
+def _run(name: str, *args):
+    """A differentiable call of the compiled operator surface."""
+    if torch._C._get_tracing_state() is None:
+        return getattr(_native(), name)(*args)
+    return _Traced.apply(name, *args)
+
+
 def _code(t: Tensor, what: str) -> int:
     try:
         return _CODES[t.dtype]
@@ -173,7 +201,7 @@ def selective_scan(
     if u.dtype == torch.float64:  # double-precision kernels, meant for gradient checks (ops_f64.py)
         from . import ops_f64
         return ops_f64.selective_scan(u, delta, A, B, C, D, z, dt_bias, softplus, return_last_state, initial_state)
-    return _native().selective_scan(u, delta, A, B, C, D, z, dt_bias, softplus, return_last_state, initial_state, keep_state_fp32)
+    return _run("selective_scan", u, delta, A, B, C, D, z, dt_bias, softplus, return_last_state, initial_state, keep_state_fp32)
 
 
 # =========================================================================================
@@ -398,7 +426,7 @@ def ssd_chunk_scan(
             raise ValueError("seq_meta must provide cu_seqlens or seq_lens.")
         cu = None if cu is None else torch.as_tensor(cu)
         lens = None if lens is None or cu is not None else torch.as_tensor(lens)
-    return _native().ssd_chunk_scan(X, dt, A, B, C, int(chunk_size), D, z, lens, cu, initial_states)
+    return _run("ssd_chunk_scan", X, dt, A, B, C, int(chunk_size), D, z, lens, cu, initial_states)
 
 
 # =========================================================================================
@@ -416,7 +444,7 @@ def dw_causal_conv(x: Tensor, weight: Tensor, bias: Optional[Tensor] = None, act
             raise ValueError("dw_causal_conv in float64 takes no halo.")
         from . import ops_f64
         return ops_f64.dw_causal_conv(x, weight, bias, activation)
-    return _native().dw_causal_conv(x, weight, bias, str(activation), halo)
+    return _run("dw_causal_conv", x, weight, bias, str(activation), halo)
 
 
 def dw_causal_conv_update(conv_state: Tensor, x: Tensor, weight: Tensor, bias: Optional[Tensor] = None,
@@ -479,7 +507,7 @@ def fused_layer_norm(
     if x.dtype == torch.float64:
         from . import ops_f64
         return ops_f64.fused_layer_norm(x, weight, bias, residual, is_rms, eps, prenorm, residual_in_fp32, return_residual)
-    return _native().fused_layer_norm(x, weight, bias, residual, is_rms, float(eps), prenorm, residual_in_fp32, return_residual)
+    return _run("fused_layer_norm", x, weight, bias, residual, is_rms, float(eps), prenorm, residual_in_fp32, return_residual)
 
 
 # =========================================================================================
@@ -629,7 +657,7 @@ def _ssd_call(X, dt, A, B, C_, D, z, dt_bias, dt_softplus, init, chunk_size, che
     """``(Y, final_states)`` of one dense scan."""
     _need_cuda(X)
     if dual and X.ndim == 4 and B.ndim == 4 and ssd_tensor_core_supported(X, B, chunk_size):
-        out = _native().ssd_scan(X, dt, A, B, C_, D, z, dt_bias, dt_softplus, init, int(chunk_size))
+        out = _run("ssd_scan", X, dt, A, B, C_, D, z, dt_bias, dt_softplus, init, int(chunk_size))
     else:
         out = _SsdFn.apply(X, dt, A, B, C_, D, z, dt_bias, dt_softplus, init, int(chunk_size))
     if check_status:
@@ -688,8 +716,8 @@ def ssd_scan(
         raise ValueError("initial_states cannot be combined with sequences that restart at cu_seqlens.")
     grads = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (X, dt, A, B, C, D, z, dt_bias, initial_states))
     if not grads and X.shape[1] > 0 and ssd_tensor_core_supported(X, B, chunk_size):  # all sequences in one set of launches
-        Y, final, varlen = _native().ssd_packed(X, dt, A, B, C, D, z, dt_bias, dt_softplus, initial_states, int(chunk_size), torch.as_tensor(cu_seqlens),
-                                                seq_reset)
+        Y, final, varlen = _run("ssd_packed", X, dt, A, B, C, D, z, dt_bias, dt_softplus, initial_states, int(chunk_size), torch.as_tensor(cu_seqlens),
+                                seq_reset)
         if check_status:
             ssd_check_status(X.device)
         out = (Y,) + ((final,) if return_final_states else ()) + ((varlen,) if return_varlen_states else ())

@@ -23,7 +23,7 @@ def test_nonfinite_neighbours_do_not_leak(first, steep, bad, dtype):
     r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
     X, z, dt = r(1, nl, nh, 64).to(dtype), r(1, nl, nh, 64).to(dtype), r(1, nl, nh).to(dtype)
     B, C = (r(1, nl, ng, 128) / 128 ** 0.5).to(dtype), (r(1, nl, ng, 128) / 128 ** 0.5).to(dtype)
-    A, D = -torch.exp(r(nh)) * (40.0 if steep else 1.0), r(nh)
+    A, D = -torch.exp(r(nh)) * (40.0 if steep else 1.0), r(nh, 64) if first % 4 == 1 else r(nh)  # a skip weight per channel is another instance
     cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda()
     clean = [t.cuda() for t in (X, dt, A, B, C)]
     kw = dict(D=D.cuda(), z=z.cuda(), dt_softplus=True, cu_seqlens=cu, return_final_states=True, return_varlen_states=True, check_status=True)

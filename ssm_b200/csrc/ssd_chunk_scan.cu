@@ -491,6 +491,23 @@ static bool chunk_bwd_vec_ok(const ssm_chunk_bwd_args& g, int piece, int nchunks
   return rows4(g.dB) && rows4(g.dC) && (!a.z.ptr || rows4(g.dz)) && aligned_to(g.dY, al) && aligned_to(g.fwd_scratch, 16);
 }
 
+// The rows that the local adjoint reads (dY, C, z), as chunk_vec_ok.
+static bool chunk_bwd_wide_ok(const ssm_chunk_bwd_args& g, int v) {
+  const ssm_chunk_args& a = g.fwd;
+  const size_t al = v * dtype_size(a.io_dtype);
+  auto rows = [&](const ssm_bcast4& p) { return p.sq == 1 && p.sb % v == 0 && p.st % v == 0 && p.sh % v == 0 && aligned_to(p.ptr, al); };
+  return a.proj % v == 0 && rows(a.Cm) && (!a.z.ptr || rows(a.z)) && aligned_to(g.dY, al);
+}
+
+// Every row tensor of the call is contiguous like X, and a row's byte offset fits 32 bits.
+static bool chunk_same_layout(const ssm_chunk_bwd_args& g) {
+  const ssm_chunk_args& a = g.fwd;
+  const int64_t HP = (int64_t)a.heads * a.proj, total = (int64_t)a.batch * a.len * HP;
+  auto like_x = [&](const ssm_bcast4& p) { return p.sq == 1 && p.sh == a.proj && p.st == HP && p.sb == a.len * HP; };
+  return total * dtype_size(a.io_dtype) < ((int64_t)1 << 32) && like_x(a.Bm) && like_x(a.Cm) && like_x(g.dB) && like_x(g.dC) &&
+         (!a.z.ptr || (like_x(a.z) && like_x(g.dz)));
+}
+
 template <typename T, typename PT>
 static int chunk_bwd_t(const ssm_chunk_bwd_args& g_in, cudaStream_t st) {
   ssm_chunk_bwd_args g = g_in;
@@ -518,8 +535,12 @@ static int chunk_bwd_t(const ssm_chunk_bwd_args& g_in, cudaStream_t st) {
   const float* S = P + (int64_t)a.batch * nchunks * HP;
   float* R = g.scratch + 2 * (int64_t)a.batch * nchunks * HP;
   const unsigned gv = (HP / 4 + kChunkThreads - 1) / kChunkThreads;
-  if (vec) chunk_bwd_local4_kernel<T><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(g, R, nchunks, a.chunk_size);
-  else chunk_bwd_local_kernel<T, PT><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
+  if (vec && chunk_bwd_wide_ok(g, 16 / (int)sizeof(T))) {
+    chunk_bwd_local_row_kernel<T, 16 / (int)sizeof(T)><<<dim3((HP / (16 / (int)sizeof(T)) + kChunkThreads - 1) / kChunkThreads, nchunks, a.batch), kChunkThreads, 0, st>>>(
+        g, R, nchunks, a.chunk_size);
+  } else if (vec) {
+    chunk_bwd_local_row_kernel<T, 4><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(g, R, nchunks, a.chunk_size);
+  } else chunk_bwd_local_kernel<T, PT><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
   if (int rc = launch_status("chunk_bwd_local_kernel")) return rc;
   chunk_bwd_carry_kernel<<<dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), kCarryLanes * kCarryGroups, 0, st>>>(g, P, nchunks);
   if (int rc = launch_status("chunk_bwd_carry_kernel")) return rc;
@@ -527,7 +548,8 @@ static int chunk_bwd_t(const ssm_chunk_bwd_args& g_in, cudaStream_t st) {
     const int64_t items = (int64_t)a.batch * nchunks, slots = (int64_t)bwd4_ctas<T>() * sm_count() / gv;  // one wave of CTAs, each looping over pieces
     const int64_t rounds = (items + (slots < 1 ? 1 : slots) - 1) / (slots < 1 ? 1 : slots);
     const unsigned gy = (unsigned)((items + rounds - 1) / rounds);  // as many CTAs as the longest of them makes worthwhile
-    chunk_bwd4_kernel<T><<<dim3(gv, gy), kChunkThreads, 0, st>>>(g, S, R, nchunks, a.chunk_size, (a.typed_grads & 8) != 0);
+    if (chunk_same_layout(g)) chunk_bwd4_kernel<T, true><<<dim3(gv, gy), kChunkThreads, 0, st>>>(g, S, R, nchunks, a.chunk_size, (a.typed_grads & 8) != 0);
+    else chunk_bwd4_kernel<T, false><<<dim3(gv, gy), kChunkThreads, 0, st>>>(g, S, R, nchunks, a.chunk_size, (a.typed_grads & 8) != 0);
     return launch_status("chunk_bwd4_kernel");
   }
   chunk_bwd_kernel<T, PT, 1><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, S, nchunks);

@@ -481,6 +481,124 @@ __global__ void __launch_bounds__(kConvThreads, 3) conv_cl_fwd_kernel(const ssm_
   }
 }
 
+// 16-bit or fp32 elements of a piece of 8 or 16 bytes as pairs of channels, word by word (see Vec16), and back
+template <typename T, int V>
+__device__ __forceinline__ void unpack_cl(const uint32_t* w, float2 (&f)[V / 2]) {
+#pragma unroll
+  for (int i = 0; i < V / 2; ++i) {
+    if constexpr (std::is_same<T, float>::value) f[i] = make_float2(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
+    else if constexpr (std::is_same<T, __nv_bfloat16>::value) f[i] = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+    else f[i] = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+  }
+}
+template <typename T, int V>
+__device__ __forceinline__ void pack_cl(const float2 (&f)[V / 2], uint32_t* w) {
+#pragma unroll
+  for (int i = 0; i < V / 2; ++i) {
+    if constexpr (std::is_same<T, float>::value) {
+      w[2 * i] = __float_as_uint(f[i].x), w[2 * i + 1] = __float_as_uint(f[i].y);
+    } else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      const __nv_bfloat162 v = __floats2bfloat162_rn(f[i].x, f[i].y);
+      w[i] = *reinterpret_cast<const uint32_t*>(&v);
+    } else {
+      const __half2 v = __floats2half2_rn(f[i].x, f[i].y);
+      w[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+  }
+}
+template <bool HALF>
+__device__ __forceinline__ float2 silu2(float2 p) {
+  if constexpr (HALF) {  // see silu_half_io
+    const float2 h = __fmul2_rn(p, make_float2(0.5f, 0.5f));
+    float2 t;
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t.x) : "f"(h.x));
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t.y) : "f"(h.y));
+    return __ffma2_rn(h, t, h);
+  } else {
+    return make_float2(silu_fast(p.x), silu_fast(p.y));
+  }
+}
+
+// The same for the width that state-space models use (4) and channels in whole 16-byte groups: the taps exist once, the window is
+// the batch of rows itself (the steps of a batch are unrolled and nothing moves from step to step), the rows of the next batch are under
+// way while this one is formed, and no step is guarded but those of a tile's last batch.  Bound by HBM.
+template <typename T, bool SILU>
+__global__ void __launch_bounds__(kConvThreads, 4) conv_cl_fwd4_kernel(const ssm_conv_args a, int tile) {
+  constexpr int V = 16 / sizeof(T), P = V / 2;
+  constexpr int U = 4;  // steps per batch of loads
+  const int C = a.channels, L = a.len, nvec = C / V;
+  const int64_t item = (int64_t)blockIdx.x * kConvThreads + threadIdx.x;  // channel groups fastest, then time tiles
+  const int c0 = (int)(item % nvec) * V;
+  const int64_t ts64 = item / nvec * tile;
+  if (ts64 >= L) return;
+  const int ts = (int)ts64, te = min(L, ts + tile), b = blockIdx.z;
+  const T* __restrict__ x = reinterpret_cast<const T*>(a.x) + (int64_t)b * L * C + c0;
+  T* __restrict__ y = reinterpret_cast<T*>(a.y) + (int64_t)b * L * C + c0;
+  uint4 nxt[U];
+  auto request = [&](int t) {  // beyond the sequence: its last row, dropped
+#pragma unroll
+    for (int j = 0; j < U; ++j) nxt[j] = __ldcs(reinterpret_cast<const uint4*>(x + (int64_t)min(t + j, L - 1) * C));
+  };
+  request(ts);
+  float2 win[U + 3][P];  // win[j]: x of step t + j - 3
+  if (ts >= 3) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const uint4 r = __ldcs(reinterpret_cast<const uint4*>(x + (int64_t)(ts - 3 + j) * C));
+      unpack_cl<T, V>(reinterpret_cast<const uint32_t*>(&r), win[j]);
+    }
+  } else {  // (tiles are multiples of eight steps: the sequence's first)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const float* h = a.halo + ((int64_t)b * C + c0 + 2 * p) * 3 + j;
+        win[j][p] = a.halo ? make_float2(__ldg(h), __ldg(h + 3)) : make_float2(0.f, 0.f);
+      }
+    }
+  }
+  float2 w[4][P], bias[P];  // w[m]: the tap of x[t - m]
+  {
+    float wf[V * 4], bf[V];
+    load_param_vec<V * 4>(a.weight, (int64_t)c0 * 4, a.param_dtype, wf);
+    if (a.bias) load_param_vec<V>(a.bias, c0, a.param_dtype, bf);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      bias[p] = a.bias ? make_float2(bf[2 * p], bf[2 * p + 1]) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) w[m][p] = make_float2(wf[8 * p + 3 - m], wf[8 * p + 7 - m]);
+    }
+  }
+#pragma unroll 1
+  for (int t = ts; t < te; t += U) {
+#pragma unroll
+    for (int j = 0; j < U; ++j) unpack_cl<T, V>(reinterpret_cast<const uint32_t*>(&nxt[j]), win[j + 3]);
+    if (t + U < te) request(t + U);
+    T* out = y + (int64_t)t * C;
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      if (t + j >= te) break;
+      float2 o[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        float2 acc = __ffma2_rn(w[0][p], win[j + 3][p], bias[p]);
+#pragma unroll
+        for (int m = 1; m < 4; ++m) acc = __ffma2_rn(w[m][p], win[j + 3 - m][p], acc);
+        o[p] = SILU ? silu2<sizeof(T) == 2>(acc) : acc;
+      }
+      uint4 r;
+      pack_cl<T, V>(o, reinterpret_cast<uint32_t*>(&r));
+      __stcs(reinterpret_cast<uint4*>(out), r);
+      out += C;
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+      for (int p = 0; p < P; ++p) win[j][p] = win[U + j][p];
+    }
+  }
+}
+
 // channels-last backward.  Walk s over [ts, te + K - 1): dpre[s] needs x[s-(K-1) .. s];
 // dx[t = s-(K-1)] = sum_q w[q] dpre[s - q] (w in stored order) needs dpre[s-(K-1) .. s].
 // Four channels per thread keep both windows, both tap orders and the weight-gradient
@@ -637,10 +755,15 @@ __device__ __forceinline__ float2 silu_grad2(float2 p) {
 // takes 31), hence four CTAs per SM and a tile length that fills whole waves (conv_cl_tile).
 // (4, 4093, 2560) bf16, 251 MB: 154 us with the kernel above, 73 us with this one (3.4 TB/s; two channels per thread and six CTAs
 // more per SM: 91).  Narrow tensors, NT = 512: (2, 16384, 128) bf16 72 -> 18 us.
-template <typename T, int V, int NT>
-__global__ void __launch_bounds__(NT, V == 4 ? 512 / NT : 768 / NT) conv_cl_bwd4_kernel(const ssm_conv_bwd_args g, int tile) {
+constexpr int kConvRing = 4, kConvBatch = 4;  // batches of the ring, steps of a batch
+constexpr size_t conv_ring_bytes(int threads) { return (size_t)kConvRing * kConvBatch * 2 * 8 * threads; }
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+template <typename T, int V, int NT, bool SILU>
+__global__ void __launch_bounds__(NT, 512 / NT) conv_cl_bwd4_kernel(const ssm_conv_bwd_args g, int tile) {
   const ssm_conv_args& a = g.fwd;
-  constexpr int U = 32 / (V * (int)sizeof(T) / 2);  // steps per batch of loads: 64 bytes of x and of dy a thread
+  constexpr int U = kConvBatch;
   constexpr int P = V / 2;
   static_assert(V * sizeof(T) == 8, "a thread's channels of a step are one load of 8 bytes");
   using Raw = uint2;
@@ -666,74 +789,95 @@ __global__ void __launch_bounds__(NT, V == 4 ? 512 / NT : 768 / NT) conv_cl_bwd4
       for (int m = 0; m < 4; ++m) w[m][p] = make_float2(wf[8 * p + 3 - m], wf[8 * p + 7 - m]), dw[m][p] = make_float2(0.f, 0.f);
     }
   }
-  float2 xh[3][P], dh[3][P];  // x[s - 1 - m], dpre[s - 1 - m]
+  // rows travel through a ring of batches in shared memory, each thread's own 8 bytes of x and of dy: no barrier, and twelve steps
+  // are under way without a register
+  extern __shared__ __align__(16) unsigned char conv_ring[];
+  Raw* ring = reinterpret_cast<Raw*>(conv_ring) + threadIdx.x;  // [stage][step][x | dy][NT]
+  auto request = [&](int s, int stage) {
+    if (s < te + 3) {
+      const T *px = x + (int64_t)min(s, L - 1) * C, *pg = dy + (int64_t)min(s, L - 1) * C;
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const int t = ts - 1 - m;
+      for (int j = 0; j < U; ++j) {
+        cp_async8(ring + ((stage * U + j) * 2) * NT, px), cp_async8(ring + ((stage * U + j) * 2 + 1) * NT, pg);
+        if (s + j + 1 < L) px += C, pg += C;  // beyond the sequence: its last row, dropped
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+#pragma unroll
+  for (int q = 0; q < kConvRing - 1; ++q) request(ts + q * U, q);
+  float2 win[U + 3][P], dwin[U + 3][P];  // x and the pre-activation gradient of step s + j - 3
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int t = ts - 3 + j;
+    if (t >= 0) {
+      const Raw r = __ldcs(reinterpret_cast<const Raw*>(x + (int64_t)t * C));
+      unpack_cl<T, V>(reinterpret_cast<const uint32_t*>(&r), win[j]);
+    }
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      float f[2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        f[q] = 0.f;
-        if (t >= 0) f[q] = to_f<T>(x[(int64_t)t * C + 2 * p + q]);
-        else if (a.halo) f[q] = __ldg(a.halo + ((int64_t)b * C + c0 + 2 * p + q) * 3 + 3 + t);
+      if (t < 0) {
+        const float* h = a.halo + ((int64_t)b * C + c0 + 2 * p) * 3 + 3 + t;
+        win[j][p] = a.halo ? make_float2(__ldg(h), __ldg(h + 3)) : make_float2(0.f, 0.f);
       }
-      xh[m][p] = make_float2(f[0], f[1]), dh[m][p] = make_float2(0.f, 0.f);
+      dwin[j][p] = make_float2(0.f, 0.f);
     }
   }
-  auto step = [&](auto inner, int s, const Raw& xr, const Raw& gr) {
+  // a batch of steps; not inner: those that touch an end of the tile (each position's parameter gradient is counted by the tile
+  // that owns it, each dx written by the tile that owns it) or lie beyond the sequence
+  auto batch = [&](auto inner, int s0) {
     constexpr bool kInner = decltype(inner)::value;
-    float xf[V], gf[V];
-    const T *ex = reinterpret_cast<const T*>(&xr), *eg = reinterpret_cast<const T*>(&gr);
+    T* to = dx + (int64_t)(s0 - 3) * C;
 #pragma unroll
-    for (int i = 0; i < V; ++i) xf[i] = kInner || s < L ? to_f<T>(ex[i]) : 0.f, gf[i] = kInner || s < L ? to_f<T>(eg[i]) : 0.f;
-    Raw ow;
-    T* out = reinterpret_cast<T*>(&ow);
+    for (int j = 0; j < U; ++j) {
+      const int s = s0 + j;
 #pragma unroll
-    for (int p = 0; p < P; ++p) {
-      const float2 cur = make_float2(xf[2 * p], xf[2 * p + 1]);
-      float2 pre = __ffma2_rn(w[0][p], cur, bias[p]);
+      for (int p = 0; p < P; ++p) {
+        if (!kInner && s >= L) win[j + 3][p] = dwin[j + 3][p] = make_float2(0.f, 0.f);
+        float2 pre = __ffma2_rn(w[0][p], win[j + 3][p], bias[p]);
 #pragma unroll
-      for (int m = 1; m < 4; ++m) pre = __ffma2_rn(w[m][p], xh[m - 1][p], pre);
-      float2 dp = make_float2(gf[2 * p], gf[2 * p + 1]);
-      if (a.silu) dp = __fmul2_rn(dp, silu_grad2<sizeof(T) == 2>(pre));
-      if (kInner || s < te) {  // each position's parameter gradient is counted by the tile that owns it
-        db[p] = __fadd2_rn(db[p], dp);
-        dw[0][p] = __ffma2_rn(dp, cur, dw[0][p]);
+        for (int m = 1; m < 4; ++m) pre = __ffma2_rn(w[m][p], win[j + 3 - m][p], pre);
+        float2& dp = dwin[j + 3][p];
+        if (SILU) dp = __fmul2_rn(dp, silu_grad2<sizeof(T) == 2>(pre));
+        if (kInner || s < te) {
+          db[p] = __fadd2_rn(db[p], dp);
 #pragma unroll
-        for (int m = 1; m < 4; ++m) dw[m][p] = __ffma2_rn(dp, xh[m - 1][p], dw[m][p]);
+          for (int m = 0; m < 4; ++m) dw[m][p] = __ffma2_rn(dp, win[j + 3 - m][p], dw[m][p]);
+        }
       }
-      // dx[s - 3] = w[3] dpre[s] + w[2] dpre[s - 1] + w[1] dpre[s - 2] + w[0] dpre[s - 3]
-      float2 o = __fmul2_rn(w[3][p], dp);
+      if (kInner || (s - 3 >= ts && s - 3 < te)) {  // dx[s - 3] = w[3] dpre[s] + w[2] dpre[s - 1] + w[1] dpre[s - 2] + w[0] dpre[s - 3]
+        float2 o[P];
 #pragma unroll
-      for (int m = 0; m < 3; ++m) o = __ffma2_rn(w[2 - m][p], dh[m][p], o);
-      out[2 * p] = from_f<T>(o.x), out[2 * p + 1] = from_f<T>(o.y);
-      xh[2][p] = xh[1][p], xh[1][p] = xh[0][p], xh[0][p] = cur;
-      dh[2][p] = dh[1][p], dh[1][p] = dh[0][p], dh[0][p] = dp;
+        for (int p = 0; p < P; ++p) {
+          o[p] = __fmul2_rn(w[3][p], dwin[j + 3][p]);
+#pragma unroll
+          for (int m = 0; m < 3; ++m) o[p] = __ffma2_rn(w[m][p], dwin[j + m][p], o[p]);
+        }
+        Raw r;
+        pack_cl<T, V>(o, reinterpret_cast<uint32_t*>(&r));
+        __stcs(reinterpret_cast<Raw*>(to), r);
+      }
+      to += C;
     }
-    if (kInner || (s - 3 >= ts && s - 3 < te)) __stcs(reinterpret_cast<Raw*>(dx + (int64_t)(s - 3) * C), ow);
   };
+  int stage = 0;
+#pragma unroll 1
   for (int s0 = ts; s0 < te + 3; s0 += U) {
-    Raw xr[U], gr[U];
-    if (s0 >= ts + 3 && s0 + U <= te) {
-      const T *px = x + (int64_t)s0 * C, *pg = dy + (int64_t)s0 * C;
+    request(s0 + (kConvRing - 1) * U, stage == 0 ? kConvRing - 1 : stage - 1);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kConvRing - 1) : "memory");
 #pragma unroll
-      for (int j = 0; j < U; ++j) {
-        xr[j] = __ldcs(reinterpret_cast<const Raw*>(px)), gr[j] = __ldcs(reinterpret_cast<const Raw*>(pg));
-        px += C, pg += C;
-      }
+    for (int j = 0; j < U; ++j) {
+      const Raw xr = ring[((stage * U + j) * 2) * NT], gr = ring[((stage * U + j) * 2 + 1) * NT];
+      unpack_cl<T, V>(reinterpret_cast<const uint32_t*>(&xr), win[j + 3]);
+      unpack_cl<T, V>(reinterpret_cast<const uint32_t*>(&gr), dwin[j + 3]);
+    }
+    stage = stage == kConvRing - 1 ? 0 : stage + 1;
+    if (s0 >= ts + 3 && s0 + U <= te) batch(std::true_type{}, s0);
+    else batch(std::false_type{}, s0);
 #pragma unroll
-      for (int j = 0; j < U; ++j) step(std::true_type{}, s0 + j, xr[j], gr[j]);
-    } else {
+    for (int j = 0; j < 3; ++j) {
 #pragma unroll
-      for (int j = 0; j < U; ++j) {
-        const int sc = min(s0 + j, L - 1);  // beyond the sequence: its last row, dropped
-        xr[j] = __ldcs(reinterpret_cast<const Raw*>(x + (int64_t)sc * C));
-        gr[j] = __ldcs(reinterpret_cast<const Raw*>(dy + (int64_t)sc * C));
-      }
-#pragma unroll
-      for (int j = 0; j < U; ++j) step(std::false_type{}, s0 + j, xr[j], gr[j]);
+      for (int p = 0; p < P; ++p) win[j][p] = win[U + j][p], dwin[j][p] = dwin[U + j][p];
     }
   }
   auto comp = [](const float2 (&v)[P], int i) { return i & 1 ? v[i / 2].y : v[i / 2].x; };
@@ -842,6 +986,13 @@ static int conv_fwd_launch(const ssm_conv_args& a, cudaStream_t st) {
     else conv_cf_fwd_kernel<T, KM, kRowRagged><<<grid, kConvThreads, 0, st>>>(a);
   } else {
     const int vec = (a.channels % V == 0) && aligned_to(a.x, 16) && aligned_to(a.y, 16);
+    if (a.width == 4 && vec && aligned_to(a.weight, 16) && aligned_to(a.bias, 16)) {
+      const int tile = conv_cl_tile(a, V, kConvThreads, 4, 12, 128);
+      const dim3 grid((unsigned)conv_cl_ctas(a, V, kConvThreads, tile), 1, a.batch);
+      if (a.silu) conv_cl_fwd4_kernel<T, true><<<grid, kConvThreads, 0, st>>>(a, tile);
+      else conv_cl_fwd4_kernel<T, false><<<grid, kConvThreads, 0, st>>>(a, tile);
+      return launch_status("dw_causal_conv_fwd");
+    }
     const int tile = conv_cl_tile(a, V, kConvThreads, 3, 12, 128);
     conv_cl_fwd_kernel<T, KM><<<dim3((unsigned)conv_cl_ctas(a, V, kConvThreads, tile), 1, a.batch), kConvThreads, 0, st>>>(a, vec, tile);
   }
@@ -861,15 +1012,19 @@ static int conv_bwd_launch(const ssm_conv_bwd_args& g, cudaStream_t st) {
     const size_t gb = V * sizeof(T);
     const int vec = (a.channels % V == 0) && aligned_to(a.x, gb) && aligned_to(g.dy, gb) && aligned_to(g.dx, gb);
     if (a.width == 4 && vec && aligned_to(a.weight, 16) && aligned_to(a.bias, 16)) {
-      constexpr int VB = 8 / sizeof(T), kPerSm = VB == 4 ? 512 : 768;  // channels and resident threads per SM
+      constexpr int VB = 8 / sizeof(T), kPerSm = 512;  // channels and resident threads per SM
       // up to 512 channels: CTAs of 512 threads, each holding all channels at several time tiles
       constexpr int kWide = 512;
+      auto launch = [&](auto kern, int threads, int tile) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)conv_ring_bytes(threads));
+        kern<<<dim3((unsigned)conv_cl_ctas(a, VB, threads, tile), 1, a.batch), threads, conv_ring_bytes(threads), st>>>(g, tile);
+      };
       if (a.channels <= kWide) {
         const int tile = conv_cl_tile(a, VB, kWide, kPerSm / kWide, 16, 256);
-        conv_cl_bwd4_kernel<T, VB, kWide><<<dim3((unsigned)conv_cl_ctas(a, VB, kWide, tile), 1, a.batch), kWide, 0, st>>>(g, tile);
+        launch(a.silu ? conv_cl_bwd4_kernel<T, VB, kWide, true> : conv_cl_bwd4_kernel<T, VB, kWide, false>, kWide, tile);
       } else {
         const int tile = conv_cl_tile(a, VB, kConvThreads, kPerSm / kConvThreads, 16, 256);
-        conv_cl_bwd4_kernel<T, VB, kConvThreads><<<dim3((unsigned)conv_cl_ctas(a, VB, kConvThreads, tile), 1, a.batch), kConvThreads, 0, st>>>(g, tile);
+        launch(a.silu ? conv_cl_bwd4_kernel<T, VB, kConvThreads, true> : conv_cl_bwd4_kernel<T, VB, kConvThreads, false>, kConvThreads, tile);
       }
     } else {
       conv_cl_bwd_kernel<T, KM><<<conv_cl_grid(a, V), kConvThreads, 0, st>>>(g, vec);

@@ -55,7 +55,7 @@ def _stale(target: Path, deps: list[Path]) -> bool:
 def build_library(force: bool = False, verbose: bool = False) -> Path:
     nvcc = _nvcc()
     OBJ.mkdir(parents=True, exist_ok=True)
-    headers = sorted(CSRC.glob("*.cuh")) + sorted((PKG.parent / "include").glob("*.h"))
+    headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + sorted((PKG.parent / "include").glob("*.h"))
 
     def compile_one(src: Path) -> Path:
         obj = OBJ / (src.stem + ".o")
@@ -88,7 +88,7 @@ def build_extension(force: bool = False, verbose: bool = False) -> Path:
     import torch
     from torch.utils.cpp_extension import include_paths, library_paths
 
-    headers = [PKG.parent / "include" / "ssm_b200.h", *EXT_SRC.glob("*.h")]
+    headers = [PKG.parent / "include" / "ssm_b200.h", *EXT_SRC.glob("*.h"), *CSRC.glob("*.h")]
     srcs = sorted(EXT_SRC.glob("*.cpp"))
     if not (force or _stale(EXT, [*srcs, *headers, LIB])):
         return EXT

@@ -46,6 +46,27 @@ inline int launch_status(const char* kernel) {
   return SSM_OK;
 }
 
+// Launch that may begin while the kernel before it on the stream drains.  The kernel calls pdl_wait() before it touches memory, then
+// pdl_trigger(): in that order, so that whatever starts early behind it finds everything before it finished.
+template <typename... P, typename... A>
+inline int launch_overlapped(const char* name, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    count_launch();
+    set_error("%s: %s", name, cudaGetErrorString(e));
+    return (int)e;
+  }
+  return launch_status(name);
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // SMs of the current device (148 on a B200)
 inline int sm_count() {
   int dev = 0, n = 148;

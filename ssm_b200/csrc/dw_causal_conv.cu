@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "decode_parts.h"
 
 namespace ssmb {
 
@@ -911,30 +912,77 @@ __global__ void __launch_bounds__(NT, 512 / NT) conv_cl_bwd4_kernel(const ssm_co
   }
 }
 
-// decode-time update: one thread per (batch, channel)
-template <typename T>
-__global__ void __launch_bounds__(256) conv_update_kernel(const ssm_conv_update_args a) {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= (int64_t)a.batch * a.channels) return;
-  const int c = (int)(i % a.channels), K = a.width;
-  float* cs = a.conv_state + i * K;
-  const float xn = to_f<T>(reinterpret_cast<const T*>(a.x)[i]);
-  float acc = a.bias ? load_dyn(a.bias, c, a.param_dtype) : 0.f;
-  if (K == 4 && aligned_to_dev(cs)) {
-    float4 v = *reinterpret_cast<float4*>(cs);
-    v = make_float4(v.y, v.z, v.w, xn);
-    *reinterpret_cast<float4*>(cs) = v;
-    float w[4];
+// Decode-time update of up to three windows.  A thread takes one channel of U sequences: its weights once, and U states in flight (one
+// state per thread kept too few bytes under way: (256, 5120) 11.3 us, 84 MB/ms of 42 MB).
+struct ConvUpdates {
+  ssm_conv_update_args a[3];
+  int blocks_end[3];  // thread blocks of the windows so far
+};
+template <typename T, int U>
+__global__ void __launch_bounds__(256) conv_update_kernel(const __grid_constant__ ConvUpdates all) {
+  pdl_wait();
+  pdl_trigger();
+  const int which = (int)blockIdx.x >= all.blocks_end[0] ? (int)blockIdx.x >= all.blocks_end[1] ? 2 : 1 : 0;
+  const ssm_conv_update_args& a = all.a[which];
+  const int64_t i = (int64_t)(blockIdx.x - (which ? all.blocks_end[which - 1] : 0)) * 256 + threadIdx.x;
+  const int C = a.channels, K = a.width;
+  const int c = (int)(i % C), b0 = (int)(i / C) * U;
+  if (b0 >= a.batch) return;
+  const float bias = a.bias ? load_dyn(a.bias, c, a.param_dtype) : 0.f;
+  if (K == 4 && aligned_to_dev(a.conv_state)) {
+    float4 v[U];
+    float xn[U], w[4];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t at = (int64_t)min(b0 + u, a.batch - 1) * C + c;
+      v[u] = *reinterpret_cast<const float4*>(a.conv_state + at * 4);
+      xn[u] = to_f<T>(reinterpret_cast<const T*>(a.x)[at]);
+    }
     load_param_vec<4>(a.weight, (int64_t)c * 4, a.param_dtype, w);
-    acc = fmaf(v.x, w[0], fmaf(v.y, w[1], fmaf(v.z, w[2], fmaf(v.w, w[3], acc))));
-  } else {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (b0 + u >= a.batch) break;
+      const int64_t at = (int64_t)(b0 + u) * C + c;
+      const float4 n = make_float4(v[u].y, v[u].z, v[u].w, xn[u]);
+      *reinterpret_cast<float4*>(a.conv_state + at * 4) = n;
+      const float acc = fmaf(n.x, w[0], fmaf(n.y, w[1], fmaf(n.z, w[2], fmaf(n.w, w[3], bias))));
+      reinterpret_cast<T*>(a.out)[at] = from_f<T>(a.silu ? silu_fast(acc) : acc);
+    }
+    return;
+  }
+  for (int b = b0; b < min(b0 + U, a.batch); ++b) {
+    const int64_t at = (int64_t)b * C + c;
+    float* cs = a.conv_state + at * K;
+    const float xn = to_f<T>(reinterpret_cast<const T*>(a.x)[at]);
+    float acc = bias;
     for (int j = 0; j < K; ++j) {
       const float v = j + 1 < K ? cs[j + 1] : xn;
       cs[j] = v;
       acc = fmaf(v, load_dyn(a.weight, (int64_t)c * K + j, a.param_dtype), acc);
     }
+    reinterpret_cast<T*>(a.out)[at] = from_f<T>(a.silu ? silu_fast(acc) : acc);
   }
-  reinterpret_cast<T*>(a.out)[i] = from_f<T>(a.silu ? silu_fast(acc) : acc);
+}
+
+template <typename T, int U>
+static int conv_update_launch(const ssm_conv_update_args* a, int n, cudaStream_t st) {
+  ConvUpdates all{};
+  int blocks = 0;
+  for (int i = 0; i < 3; ++i) {
+    if (i < n) {
+      all.a[i] = a[i];
+      blocks += (int)(((int64_t)((a[i].batch + U - 1) / U) * a[i].channels + 255) / 256);
+    }
+    all.blocks_end[i] = i < n - 1 ? blocks : INT32_MAX;
+  }
+  return launch_overlapped("conv_update_kernel", conv_update_kernel<T, U>, dim3(blocks), dim3(256), 0, st, all);
+}
+template <typename T>
+static int conv_update_t(const ssm_conv_update_args* a, int n, cudaStream_t st) {
+  int64_t items = 0;
+  for (int i = 0; i < n; ++i) items += (int64_t)a[i].batch * a[i].channels;
+  // four sequences per thread once that still gives every SM a thousand threads
+  return items >= (int64_t)sm_count() * 4096 ? conv_update_launch<T, 4>(a, n, st) : conv_update_launch<T, 1>(a, n, st);
 }
 
 static int conv_validate(const ssm_conv_args* a) {
@@ -1078,21 +1126,29 @@ extern "C" int ssm_dw_causal_conv_bwd(const ssm_conv_bwd_args* g, ssm_stream_t s
   }
 }
 
-extern "C" int ssm_dw_causal_conv_update(const ssm_conv_update_args* a, ssm_stream_t stream) {
+static int conv_update_check(const ssm_conv_update_args* a) {
   SSM_REQUIRE(a != nullptr, SSM_ERR_NULL, "dw_causal_conv_update: args is NULL");
   SSM_REQUIRE(a->batch >= 0 && a->channels >= 0 && a->width >= 1, SSM_ERR_SHAPE, "dw_causal_conv_update: bad shape");
   SSM_REQUIRE(valid_dtype(a->io_dtype), SSM_ERR_DTYPE, "dw_causal_conv_update: unknown dtype");
-  const int64_t n = (int64_t)a->batch * a->channels;
-  if (n == 0) return SSM_OK;
+  if ((int64_t)a->batch * a->channels == 0) return SSM_OK;
   SSM_REQUIRE(a->conv_state && a->x && a->weight && a->out, SSM_ERR_NULL, "dw_causal_conv_update: missing pointer");
   SSM_REQUIRE(valid_dtype(a->param_dtype), SSM_ERR_DTYPE, "dw_causal_conv_update: unknown parameter dtype");
   SSM_REQUIRE(a->width != 4 || aligned_to(a->weight, 4 * dtype_size(a->param_dtype)), SSM_ERR_ALIGN, "dw_causal_conv_update: weight must be aligned to four elements");
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const unsigned grid = (unsigned)((n + 255) / 256);
-  switch (a->io_dtype) {
-    case SSM_F32: conv_update_kernel<float><<<grid, 256, 0, st>>>(*a); break;
-    case SSM_BF16: conv_update_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*a); break;
-    default: conv_update_kernel<__half><<<grid, 256, 0, st>>>(*a); break;
-  }
-  return launch_status("conv_update_kernel");
+  return SSM_OK;
 }
+
+extern "C" int ssmb_conv_update_many(const ssm_conv_update_args* a, int32_t n, void* stream) {
+  SSM_REQUIRE(n >= 1 && n <= 3, SSM_ERR_UNSUPPORTED, "dw_causal_conv_update: one to three windows");
+  for (int i = 0; i < n; ++i) {
+    if (int rc = conv_update_check(a + i)) return rc;
+    if ((int64_t)a[i].batch * a[i].channels == 0) return SSM_OK;  // (the windows share the batch)
+  }
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  switch (a->io_dtype) {
+    case SSM_F32: return conv_update_t<float>(a, n, st);
+    case SSM_BF16: return conv_update_t<__nv_bfloat16>(a, n, st);
+    default: return conv_update_t<__half>(a, n, st);
+  }
+}
+
+extern "C" int ssm_dw_causal_conv_update(const ssm_conv_update_args* a, ssm_stream_t stream) { return ssmb_conv_update_many(a, 1, stream); }

@@ -6,6 +6,7 @@
 
 #include <utility>
 
+#include "../decode_parts.h"
 #include "operands.h"
 
 namespace ssm_ext {
@@ -495,6 +496,9 @@ py::object fused_layer_norm(const Tensor& x, const Tensor& weight, const OptTens
 // ---------------------------------------------------------------------------------------------
 // one decode token through a whole mixer (no gradients)
 // ---------------------------------------------------------------------------------------------
+Tensor ssd_status(int64_t device);
+void ssd_poll(int64_t device);
+
 bool plain(const Tensor& t, at::ScalarType type) {
   return t.scalar_type() == type && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
 }
@@ -508,7 +512,119 @@ bool launched(int rc) {
   return true;
 }
 
-// Up to 16 sequences: one launch (ssm_mamba1_decode).  More: library GEMMs around the conv and state kernels.  With norm_w the
+// A step of up to 256 sequences as five to seven launches of this library on one piece of scratch, each starting while the one before it
+// drains.  The callers have checked types, sizes and alignment.
+struct Parts {
+  Tensor scratch;
+  char* at;
+  int io;
+  int32_t* status;
+  ssm_stream_t st;
+  Parts(const Tensor& tok, int64_t elements, int pieces)
+      : scratch(at::empty({(elements + 64 * pieces) * 2}, tok.options().dtype(at::kByte))), at(static_cast<char*>(scratch.data_ptr())), io(dtype_code(tok, "decode step")),
+        status(ssd_status(tok.get_device()).data_ptr<int32_t>()), st(stream_of(tok)) {}
+  char* take(int64_t elements) {  // 16-bit elements, from a 128-byte line
+    char* p = at;
+    at += (elements + 63) / 64 * 128;
+    return p;
+  }
+  // out_i = x w_i^T, x (nb, k) with ldx elements from row to row
+  void product(int64_t nb, const void* x, int64_t k, int64_t ldx, bool weights_ahead, std::initializer_list<std::pair<const Tensor*, void*>> mats) const {
+    ssmb_rows_gemm_args a{};
+    a.batch = (int)nb, a.k = (int)k, a.ldx = ldx, a.io_dtype = io, a.x = x, a.status = status, a.weights_ahead = weights_ahead;
+    for (const auto& m : mats) {
+      a.w[a.mats] = m.first->data_ptr(), a.rows[a.mats] = (int)m.first->size(0), a.out[a.mats] = m.second, a.ldo[a.mats] = m.first->size(0);
+      ++a.mats;
+    }
+    run(ssmb_rows_gemm(&a, st));
+  }
+};
+Tensor rows_of(void* p, int64_t rows, int64_t cols, int64_t ld, const Tensor& like) { return at::from_blob(p, {rows, cols}, {ld, 1}, like.options()); }
+// The library's product of many token rows with one large matrix keeps more of the GPU busy than the kernel of Parts (256 rows, 2560 x 5120: 10.6
+// us against 16.2; 128 rows 10.1 against 11.3; 256 rows, 768 x 1536 4.5 against 5.8, but 10 us more of host time).
+bool library_product(int64_t nb, const Tensor& w) { return nb > 128 && w.size(0) >= 1024 && w.size(1) >= 2048; }
+
+py::object mamba1_parts(const Tensor& tok, const OptTensor& residual, const Tensor& conv_state, const Tensor& ssm_state, const Tensor& in_x, const Tensor& in_z,
+                        const Tensor& conv_w, const OptTensor& conv_b, const Tensor& x_proj, const Tensor& dt_proj, const Tensor& dt_bias, const Tensor& A, bool a_log,
+                        const Tensor& D, const Tensor& out_proj, const OptTensor& norm_w, double eps) {
+  c10::cuda::CUDAGuard guard(tok.device());
+  ssd_poll(tok.get_device());
+  const int64_t nb = tok.size(0), dm = tok.size(1), di = in_x.size(0), n = ssm_state.size(-1), r = dt_proj.size(1), xw = r + 2 * n;
+  Parts p(tok, nb * (5 * di + xw + dm), 7);
+  char *x = p.take(nb * di), *z = p.take(nb * di), *u = p.take(nb * di), *xd = p.take(nb * xw), *dt = p.take(nb * di), *y = p.take(nb * di), *o = p.take(nb * dm);
+  Tensor out = at::empty_like(tok), res;
+  p.product(nb, tok.data_ptr(), dm, dm, false, {{&in_x, x}, {&in_z, z}});
+  ssm_conv_update_args c{};
+  c.batch = (int)nb, c.channels = (int)di, c.width = (int)conv_w.size(-1), c.io_dtype = c.param_dtype = p.io, c.silu = 1;
+  c.conv_state = conv_state.data_ptr<float>(), c.x = x, c.weight = conv_w.data_ptr(), c.bias = ptr(conv_b), c.out = u;
+  run(ssmb_conv_update_many(&c, 1, p.st));
+  p.product(nb, u, di, di, true, {{&x_proj, xd}});
+  if (ssmb_rows_gemm_supported((int)nb, (int)r, xw, p.io)) {
+    p.product(nb, xd, r, xw, true, {{&dt_proj, dt}});
+  } else {  // rows of dt_proj that do not start on 16-byte boundaries
+    Tensor to = rows_of(dt, nb, di, di, tok);
+    at::mm_out(to, rows_of(xd, nb, r, xw, tok), dt_proj.t());
+  }
+  ssm_step_args s{};
+  s.batch = (int)nb, s.dim = (int)di, s.nstate = (int)n, s.io_dtype = s.bc_dtype = p.io, s.bc_groups = 1, s.dt_softplus = 1, s.a_log = a_log;
+  s.state = ssm_state.data_ptr<float>(), s.x = u, s.dt = dt, s.z = z, s.A = A.data_ptr<float>(), s.D = D.data_ptr<float>(), s.dt_bias = dt_bias.data_ptr<float>();
+  s.Bm = xd + r * 2, s.Cm = xd + (r + n) * 2, s.b_sb = s.c_sb = xw, s.b_sn = s.c_sn = 1, s.out = y;
+  run(ssm_selective_state_step(&s, p.st));
+  void* mixed = norm_w.has_value() ? (void*)o : out.data_ptr();
+  if (library_product(nb, out_proj)) {
+    Tensor to = norm_w.has_value() ? rows_of(o, nb, dm, dm, tok) : out;
+    at::mm_out(to, rows_of(y, nb, di, di, tok), out_proj.t());
+  } else {
+    p.product(nb, y, di, di, true, {{&out_proj, mixed}});
+  }
+  if (!norm_w.has_value()) return py::cast(out);
+  res = at::empty({nb, dm}, tok.options().dtype(at::kFloat));
+  ssm_norm_args a{};
+  a.rows = nb, a.hidden = (int)dm, a.io_dtype = a.param_dtype = p.io, a.is_rms = 1, a.prenorm = 1, a.eps = (float)eps;
+  a.x = o, a.weight = norm_w->data_ptr(), a.y = out.data_ptr(), a.residual_out = res.data_ptr(), a.resout_dtype = SSM_F32;
+  if (residual.has_value()) a.residual = residual->data_ptr(), a.res_dtype = dtype_code(*residual, "mamba1_step residual");
+  run(ssm_fused_add_norm_fwd(&a, p.st));
+  return py::make_tuple(out, res);
+}
+
+Tensor mamba2_parts(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B, const Tensor& conv_C, const Tensor& ssm_state, const Tensor& in_z, const Tensor& in_x,
+                    const Tensor& in_B, const Tensor& in_C, const Tensor& in_dt, const Tensor& wx, const OptTensor& bx, const Tensor& wB, const OptTensor& bB,
+                    const Tensor& wC, const OptTensor& bC, const Tensor& dt_bias, const Tensor& A, bool a_log, const Tensor& D, const Tensor& norm_w,
+                    const Tensor& out_proj, double eps) {
+  c10::cuda::CUDAGuard guard(tok.device());
+  ssd_poll(tok.get_device());
+  const int64_t nb = tok.size(0), dm = tok.size(1), nh = ssm_state.size(1), n = ssm_state.size(3), di = in_x.size(0), gn = in_B.size(0);
+  Parts p(tok, nb * (5 * di + 4 * gn + nh), 10);
+  char *x = p.take(nb * di), *z = p.take(nb * di), *u = p.take(nb * di), *y = p.take(nb * di), *yn = p.take(nb * di), *B = p.take(nb * gn), *C = p.take(nb * gn),
+       *uB = p.take(nb * gn), *uC = p.take(nb * gn), *dt = p.take(nb * nh);
+  Tensor out = at::empty_like(tok);
+  p.product(nb, tok.data_ptr(), dm, dm, false, {{&in_x, x}, {&in_z, z}, {&in_B, B}, {&in_C, C}, {&in_dt, dt}});
+  ssm_conv_update_args c[3] = {};
+  const Tensor* states[3] = {&conv_x, &conv_B, &conv_C};
+  const Tensor* weights[3] = {&wx, &wB, &wC};
+  const OptTensor* biases[3] = {&bx, &bB, &bC};
+  const char* from[3] = {x, B, C};
+  char* to[3] = {u, uB, uC};
+  for (int i = 0; i < 3; ++i) {
+    c[i].batch = (int)nb, c[i].channels = (int)(i ? gn : di), c[i].width = (int)wx.size(-1), c[i].io_dtype = c[i].param_dtype = p.io, c[i].silu = 1;
+    c[i].conv_state = states[i]->data_ptr<float>(), c[i].x = from[i], c[i].weight = weights[i]->data_ptr(), c[i].bias = ptr(*biases[i]), c[i].out = to[i];
+  }
+  run(ssmb_conv_update_many(c, 3, p.st));
+  ssm_step_args s{};
+  s.batch = (int)nb, s.dim = (int)di, s.nstate = (int)n, s.io_dtype = s.bc_dtype = p.io, s.bc_groups = (int)(gn / n), s.dt_softplus = 1, s.param_heads = (int)nh, s.a_log = a_log;
+  s.state = ssm_state.data_ptr<float>(), s.x = u, s.dt = dt, s.z = z, s.A = A.data_ptr<float>(), s.D = D.data_ptr<float>(), s.dt_bias = dt_bias.data_ptr<float>();
+  s.Bm = uB, s.Cm = uC, s.b_sb = s.c_sb = gn, s.b_sg = s.c_sg = n, s.b_sn = s.c_sn = 1, s.out = y;
+  run(ssm_selective_state_step(&s, p.st));
+  ssm_norm_args a{};
+  a.rows = nb, a.hidden = (int)di, a.io_dtype = a.param_dtype = p.io, a.is_rms = 1, a.prenorm = 1, a.eps = (float)eps;
+  a.x = y, a.weight = norm_w.data_ptr(), a.y = yn;
+  run(ssm_fused_add_norm_fwd(&a, p.st));
+  if (library_product(nb, out_proj)) at::mm_out(out, rows_of(yn, nb, di, di, tok), out_proj.t());
+  else p.product(nb, yn, di, di, true, {{&out_proj, out.data_ptr()}});
+  return out;
+}
+
+// Up to 16 sequences: one launch (ssm_mamba1_decode).  Up to 256: the launches above.  More, or other types and layouts: library GEMMs around the conv and state kernels.  With norm_w the
 // residual add and RMSNorm behind the mixer are included and the result is (normed, residual stream in fp32).
 py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tensor& conv_state, const Tensor& ssm_state, const Tensor& in_x, const Tensor& in_z,
                        const Tensor& conv_w, const OptTensor& conv_b, const Tensor& x_proj, const Tensor& dt_proj, const Tensor& dt_bias, const Tensor& A,
@@ -528,9 +644,8 @@ py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tenso
           dt_proj.size(0) == di && out_proj.size(0) == dm && out_proj.size(1) == di && conv_state.dim() == 3 && conv_state.size(0) == nb && conv_state.size(1) == di &&
           conv_state.size(2) == k && ssm_state.dim() == 3 && ssm_state.size(0) == nb && ssm_state.size(1) == di && A.dim() == 2 && A.size(0) == di && A.size(1) == n &&
           D.numel() == di && dt_bias.numel() == di && conv_w.numel() == di * k && (!conv_b.has_value() || conv_b->numel() == di) &&
-          (!norm_w.has_value() || norm_w->numel() == dm) && (!residual.has_value() || residual->numel() == nb * dm) &&
-          ssm_mamba1_decode_supported((int)nb, (int)dm, (int)di, (int)n, (int)r, (int)k, dtype_code(tok, "mamba1_step"));
-  if (fused) {
+          (!norm_w.has_value() || norm_w->numel() == dm) && (!residual.has_value() || residual->numel() == nb * dm) && nb > 0;
+  if (fused && ssm_mamba1_decode_supported((int)nb, (int)dm, (int)di, (int)n, (int)r, (int)k, dtype_code(tok, "mamba1_step"))) {
     c10::cuda::CUDAGuard guard(tok.device());
     Tensor out = at::empty_like(tok), res;
     Tensor scratch = at::empty({ssm_mamba1_decode_scratch_bytes((int)nb, (int)dm, (int)di, (int)n, (int)r)}, tok.options().dtype(at::kByte));
@@ -551,6 +666,8 @@ py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tenso
       return py::cast(out);
     }
   }
+  if (fused && dm % 8 == 0 && di % 8 == 0 && nb <= SSMB_GEMM_MAX_ROWS)
+    return mamba1_parts(tok, residual, conv_state, ssm_state, in_x, in_z, conv_w, conv_b, x_proj, dt_proj, dt_bias, A, a_log, D, out_proj, norm_w, eps);
   Tensor x = at::matmul(tok, in_x.t()), z = at::matmul(tok, in_z.t());
   Tensor u = dw_causal_conv_update(conv_state, x, conv_w, conv_b, "silu");
   Tensor xd = at::matmul(u, x_proj.t());
@@ -586,9 +703,8 @@ Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B
           wC.numel() == g * n * k && (!bx.has_value() || bx->numel() == di) && (!bB.has_value() || bB->numel() == g * n) &&
           (!bC.has_value() || bC->numel() == g * n) && conv_x.numel() == nb * di * k && conv_B.numel() == nb * g * n * k && conv_C.numel() == nb * g * n * k &&
           ssm_state.size(0) == nb && dt_bias.numel() == nh && A.numel() == nh && D.numel() == nh && norm_w.numel() == di && out_proj.dim() == 2 &&
-          out_proj.size(0) == dm && out_proj.size(1) == di &&
-          ssm_mamba2_decode_supported((int)nb, (int)dm, (int)nh, (int)hp, (int)n, (int)g, (int)k, dtype_code(tok, "mamba2_step"));
-  if (fused) {
+          out_proj.size(0) == dm && out_proj.size(1) == di && nb > 0;
+  if (fused && ssm_mamba2_decode_supported((int)nb, (int)dm, (int)nh, (int)hp, (int)n, (int)g, (int)k, dtype_code(tok, "mamba2_step"))) {
     c10::cuda::CUDAGuard guard(tok.device());
     Tensor out = at::empty_like(tok);
     Tensor scratch = at::empty({ssm_mamba2_decode_scratch_bytes((int)nb, (int)nh, (int)g)}, tok.options().dtype(at::kByte));
@@ -602,6 +718,8 @@ Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B
     a.ssm_state = ssm_state.data_ptr<float>(), a.out = out.data_ptr(), a.scratch = scratch.data_ptr();
     if (launched(ssm_mamba2_decode(&a, stream_of(tok)))) return out;
   }
+  if (fused && dm % 8 == 0 && di % 8 == 0 && nb <= SSMB_GEMM_MAX_ROWS)
+    return mamba2_parts(tok, conv_x, conv_B, conv_C, ssm_state, in_z, in_x, in_B, in_C, in_dt, wx, bx, wB, bB, wC, bC, dt_bias, A, a_log, D, norm_w, out_proj, eps);
   Tensor z = at::matmul(tok, in_z.t());
   Tensor x = dw_causal_conv_update(conv_x, at::matmul(tok, in_x.t()), wx, bx, "silu");
   Tensor Bm = dw_causal_conv_update(conv_B, at::matmul(tok, in_B.t()), wB, bB, "silu").view({nb, g, n});

@@ -1,4 +1,5 @@
-// Mamba-1 selective scan, backward, for sm_100a.
+// Mamba-1 selective scan, backward, for sm_100a.  (Calls of 5 to 16 states whose rows share B and C: selective_scan_bwd_pairs.cuh, for
+// which this kernel finds the adjoints that enter the segments of a call cut in time.)
 //
 // Same lane layout and tile staging as the forward kernel (scan_common.cuh).  Time is walked
 // in reverse in tiles of one checkpoint interval: the tile's states are rebuilt from the
@@ -12,7 +13,7 @@
 // group over the warp's rows and adds it to global memory with one vector reduction.
 #pragma once
 
-#include "scan_common.cuh"
+#include "selective_scan_bwd_pairs.cuh"
 
 namespace ssmb {
 
@@ -75,8 +76,8 @@ __global__ void __launch_bounds__(BwdShape<T, NS, LPR, SHARED, PIECES>::NW * 32,
   const int d0 = blockIdx.x * ROWS;
   const int N = a.nstate, L = a.len, D = a.dim;
   // Rows in the low lane bits: the eight lanes of a quarter warp share their states, so the 16-byte reads of B and C (most of the
-  // kernel's shared-memory traffic) are broadcasts of one group instead of two rows' worth of four.  8 x 1536 rows, 4096 steps,
-  // 16 states: 1641 -> 1583 us; 2 x 2048 rows, 1024 steps, 64 states: 1458 -> 1135 us.
+  // kernel's shared-memory traffic) are broadcasts of one group instead of two rows' worth of four.  2 x 2048 rows, 1024 steps,
+  // 64 states: 1458 -> 1135 us.
   const int r = lane % RPW, sg = lane / RPW;
   const int drow0 = d0 + warp * RPW;
   const int d_raw = drow0 + r;
@@ -640,8 +641,22 @@ static int launch_bwd(const ssm_scan_bwd_args& g, ScanFlags fl, cudaStream_t st)
       } else {
         SSM_REQUIRE(used == 1, SSM_ERR_UNSUPPORTED, "selective_scan_backward: calls of more than 32 states are not cut in time");
       }
-      if (pieces) return launch(scan_bwd_kernel<T, NS, LPR, true, true, false>, P1::bytes());
-      return launch(scan_bwd_kernel<T, NS, LPR, true, false, false>, P0::bytes());
+      // Two rows per lane where shared memory leaves two such CTAs per SM or more.  With one (fp32, 8 states): 690 us against 659 at 4 x 2048 rows
+      // of 2048 steps; with 4 states a row has too few lanes for the sums over states to cost anything: 554 against 432.
+      if constexpr (NS == 4 && (LPR == 4 || (LPR == 2 && sizeof(T) == 2))) {
+        using Q0 = BwdPairs<T, LPR, false>;
+        using Q1 = BwdPairs<T, LPR, true>;
+        static_assert(Q0::ROWS == S1::ROWS, "the same rows per CTA");
+        auto pairs = [&](auto kern, size_t smem) {
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          kern<<<grid, Q0::NW * 64, smem, st>>>(g, fl, seg_tiles, sm_count());
+          return launch_status("scan_bwd_pairs_kernel");
+        };
+        return pieces ? pairs(scan_bwd_pairs_kernel<T, LPR, true>, Q1::kBytes) : pairs(scan_bwd_pairs_kernel<T, LPR, false>, Q0::kBytes);
+      } else {
+        if (pieces) return launch(scan_bwd_kernel<T, NS, LPR, true, true, false>, P1::bytes());
+        return launch(scan_bwd_kernel<T, NS, LPR, true, false, false>, P0::bytes());
+      }
     }
   }
   {

@@ -2,6 +2,9 @@
 // passes call the backward entry points.  Everything between a Python call and its kernel launches happens here, once per
 // call and without Python: a small operator is bound by exactly this work (a Python implementation of the same steps, with
 // a ctypes struct per call and torch.autograd.Function, took 40 to 90 us a call; these take 6 to 15 us).
+#include <ATen/SavedTensorHooks.h>
+#include <ATen/TracerMode.h>
+#include <ATen/autocast_mode.h>
 #include <torch/csrc/autograd/custom_function.h>
 
 #include <utility>
@@ -969,6 +972,138 @@ std::tuple<Tensor, Tensor> ssd_scan(const Tensor& X, const Tensor& dt, const Ten
   return {r[0], r[1]};
 }
 
+// ---------------------------------------------------------------------------------------------
+// whole mixers
+// ---------------------------------------------------------------------------------------------
+// A mixer of a short sequence is bound by the host: as separate calls its projections and operators were two dozen autograd nodes, 0.95 ms
+// of host time per training step for 0.12 ms of device time (d_model 256, 256 steps).  The calls below are the same products and
+// operators behind one node; products that add into a gradient do so in their epilogue instead of a pass of their own.
+//
+// They stand for the composed form only where nothing can tell the difference: no tracing, autocast or saved-tensor hooks, plain types.
+bool composed_only(const Tensor& x, std::initializer_list<const Tensor*> weights) {
+  if (at::tracer::impl::is_dispatch_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || at::SavedTensorDefaultHooks::get_hooks().has_value()) return true;
+  if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || !io_dtype_ok(x)) return true;
+  for (const Tensor* w : weights)
+    if (w->scalar_type() != x.scalar_type() || w->dim() != 2 || w->device() != x.device()) return true;
+  return false;
+}
+
+struct Mamba1MixerCall final : Call {
+  Tensor hidden, in_x, in_z, conv_w, x_proj, dt_proj, dt_bias, A_in, D, out_proj;
+  OptTensor conv_b;
+  bool a_log;
+  int64_t nb, nl, dm, di, n, r;
+  std::vector<bool> need;
+  // of the forward pass, for the backward
+  Tensor h2, u2, xd, y2, A;
+  c10::intrusive_ptr<ConvCall> conv;
+  c10::intrusive_ptr<ScanCall> scan;
+
+  Mamba1MixerCall(const Tensor& hidden_, const Tensor& in_x_, const Tensor& in_z_, const Tensor& conv_w_, const OptTensor& conv_b_, const Tensor& x_proj_,
+                  const Tensor& dt_proj_, const Tensor& dt_bias_, const Tensor& A_, bool a_log_, const Tensor& D_, const Tensor& out_proj_)
+      : hidden(hidden_), in_x(in_x_), in_z(in_z_), conv_w(conv_w_), x_proj(x_proj_), dt_proj(dt_proj_), dt_bias(dt_bias_), A_in(A_), D(D_), out_proj(out_proj_),
+        conv_b(conv_b_), a_log(a_log_) {
+    for (const Tensor* t : {&hidden, &in_x, &in_z, &conv_w}) input(*t);
+    input(conv_b);
+    for (const Tensor* t : {&x_proj, &dt_proj, &dt_bias, &A_in, &D, &out_proj}) input(*t);
+    for (const Tensor& t : inputs) need.push_back(t.requires_grad());
+    nb = hidden.size(0), nl = hidden.size(1), dm = hidden.size(2), di = in_x.size(0), r = dt_proj.size(1), n = (x_proj.size(0) - r) / 2;
+  }
+  Tensor rows(const Tensor& m) const { return m.view({m.size(0), nb, nl}).permute({1, 0, 2}); }                    // (C, B L) -> (B, C, L)
+  Tensor flat(const Tensor& t) const { return t.permute({1, 0, 2}).reshape({t.size(1), nb * nl}); }                // and back
+
+  variable_list forward(bool train) override {
+    c10::cuda::CUDAGuard guard(hidden.device());
+    Tensor h = hidden.detach().reshape({nb * nl, dm});
+    Tensor x = at::mm(in_x.detach(), h.t()), z = at::mm(in_z.detach(), h.t());
+    auto cv = c10::make_intrusive<ConvCall>(rows(x), conv_w.detach(), conv_b.has_value() ? OptTensor(conv_b->detach()) : conv_b, "silu", OptTensor());
+    Tensor u = cv->forward(train)[0], uf = flat(u);
+    Tensor xdbl = at::mm(x_proj.detach(), uf), delta = at::mm(dt_proj.detach(), xdbl.narrow(0, 0, r));
+    auto coeff = [&](int64_t from) { return xdbl.narrow(0, from, n).view({n, nb, nl}).permute({1, 0, 2}).unsqueeze(1); };  // (B, 1, N, L)
+    Tensor Av = a_log ? at::exp(A_in.detach()).neg_() : A_in.detach();
+    auto sc = c10::make_intrusive<ScanCall>(u, rows(delta), Av, coeff(r), coeff(r + n), OptTensor(D.detach()), OptTensor(rows(z)), OptTensor(dt_bias.detach()), true, false,
+                                            OptTensor(), false);
+    Tensor yf = flat(sc->forward(train)[0]);
+    Tensor out = at::mm(yf.t(), out_proj.detach().t()).view({nb, nl, dm});
+    if (train) {
+      sc->t_B = sc->t_C = at::kFloat;  // their gradients are converted where they are copied
+      h2 = h, u2 = uf, xd = xdbl, y2 = yf, A = Av, conv = cv, scan = sc;
+    }
+    return {out};
+  }
+
+  variable_list backward(const variable_list& grads) override {
+    c10::cuda::CUDAGuard guard(hidden.device());
+    const bool has_b = conv_b.has_value();
+    if (!grads[0].defined()) return variable_list(10 + has_b);
+    enum { kHidden, kInX, kInZ, kConvW };
+    const int kXProj = 4 + has_b, kDtProj = kXProj + 1, kDtBias = kXProj + 2, kA = kXProj + 3, kD = kXProj + 4, kOut = kXProj + 5;
+    variable_list res(kOut + 1);
+    Tensor g = cast(grads[0], h2.scalar_type()).reshape({nb * nl, dm});
+    if (need[kOut]) res[kOut] = at::mm(g.t(), y2.t());
+    bool any = false;  // anything behind the out projection
+    for (int i = 0; i < kOut; ++i) any = any || need[i];
+    if (!any) return res;
+    Tensor dy = at::mm(out_proj.detach().t(), g.t());
+    variable_list s = scan->backward({rows(dy)});  // u, delta, A, B, C, D, z, dt_bias
+    Tensor du = flat(s[0]), dd = flat(s[1]), dz = flat(s[6]);
+    if (need[kA]) res[kA] = cast(a_log ? s[2].mul_(A) : s[2], A_in.scalar_type());
+    if (need[kD]) res[kD] = cast(s[5], D.scalar_type());
+    if (need[kDtBias]) res[kDtBias] = cast(s[7], dt_bias.scalar_type());
+    if (need[kDtProj]) res[kDtProj] = at::mm(dd, xd.narrow(0, 0, r).t());
+    Tensor dxd = at::empty_like(xd), low = dxd.narrow(0, 0, r);
+    at::mm_out(low, dt_proj.detach().t(), dd);
+    dxd.narrow(0, r, n).view({n, nb, nl}).copy_(s[3].squeeze(1).permute({1, 0, 2}));
+    dxd.narrow(0, r + n, n).view({n, nb, nl}).copy_(s[4].squeeze(1).permute({1, 0, 2}));
+    if (need[kXProj]) res[kXProj] = at::mm(dxd, u2.t());
+    if (!(need[kHidden] || need[kInX] || need[kInZ] || need[kConvW] || (has_b && need[4]))) return res;
+    du.addmm_(x_proj.detach().t(), dxd);
+    variable_list c = conv->backward({rows(du)});
+    Tensor dx = flat(c[0]);
+    if (need[kConvW]) res[kConvW] = c[1];
+    if (has_b && need[4]) res[4] = c[2];
+    if (need[kInX]) res[kInX] = at::mm(dx, h2);
+    if (need[kInZ]) res[kInZ] = at::mm(dz, h2);
+    if (need[kHidden]) {
+      Tensor dh = at::mm(dx.t(), in_x.detach());
+      dh.addmm_(dz.t(), in_z.detach());
+      res[kHidden] = dh.view(hidden.sizes());
+    }
+    return res;
+  }
+};
+
+// hidden (B, L, d_model) through a Mamba-1 mixer; None where the composed form has to serve.
+py::object mamba1_mixer(const Tensor& hidden, const Tensor& in_x, const Tensor& in_z, const Tensor& conv_w, const OptTensor& conv_b, const Tensor& x_proj,
+                        const Tensor& dt_proj, const Tensor& dt_bias, const Tensor& A, bool a_log, const Tensor& D, const Tensor& out_proj) {
+  ValueErrors scope;
+  if (composed_only(hidden, {&in_x, &in_z, &x_proj, &dt_proj, &out_proj})) return py::none();
+  const int64_t dm = hidden.size(2), di = in_x.size(0), r = dt_proj.size(1), rest = x_proj.size(0) - r;
+  if (in_x.size(1) != dm || in_z.sizes() != in_x.sizes() || x_proj.size(1) != di || dt_proj.size(0) != di || out_proj.size(0) != dm || out_proj.size(1) != di ||
+      r < 1 || rest < 2 || rest % 2 != 0 || A.dim() != 2 || A.size(0) != di || A.size(1) != rest / 2 || conv_w.size(0) != di)
+    return py::none();
+  return py::cast(invoke_call(c10::make_intrusive<Mamba1MixerCall>(hidden, in_x, in_z, conv_w, conv_b, x_proj, dt_proj, dt_bias, A, a_log, D, out_proj))[0]);
+}
+
+// u (B, L, d_model), normed, through a Mamba-2 mixer on the tensor-core scan, without gradients; None where the composed form has to serve.
+py::object mamba2_mixer(const Tensor& u, const Tensor& in_z, const Tensor& in_x, const Tensor& in_B, const Tensor& in_C, const Tensor& in_dt, const Tensor& wx,
+                        const OptTensor& bx, const Tensor& wB, const OptTensor& bB, const Tensor& wC, const OptTensor& bC, const Tensor& dt_bias, const Tensor& A_log,
+                        const Tensor& D, const Tensor& norm_w, const Tensor& out_proj, int64_t nh, int64_t hp, int64_t n, int64_t g, int64_t chunk, double eps) {
+  ValueErrors scope;
+  if (at::GradMode::is_enabled() || composed_only(u, {&in_z, &in_x, &in_B, &in_C, &in_dt, &out_proj})) return py::none();
+  const int64_t nb = u.size(0), nl = u.size(1), dm = u.size(2), di = nh * hp;
+  if (!ssm_ssd_supported((int)hp, (int)n, (int)chunk, dtype_code(u, "mamba2_mixer")) || in_x.size(0) != di || in_x.size(1) != dm) return py::none();
+  c10::cuda::CUDAGuard guard(u.device());
+  Tensor u2 = u.reshape({nb * nl, dm});
+  auto proj = [&](const Tensor& w) { return at::mm(u2, w.t()).view({nb, nl, w.size(0)}); };
+  auto conv = [&](const Tensor& t, const Tensor& w, const OptTensor& b) { return invoke_call(c10::make_intrusive<ConvCall>(t, w, b, "silu", OptTensor()))[0]; };
+  Tensor x = conv(proj(in_x), wx, bx).view({nb, nl, nh, hp}), B = conv(proj(in_B), wB, bB).view({nb, nl, g, n}), C = conv(proj(in_C), wC, bC).view({nb, nl, g, n});
+  Tensor z = proj(in_z).view({nb, nl, nh, hp}), dt = proj(in_dt);
+  Tensor y = std::get<0>(ssd_scan(x, dt, at::exp(A_log).neg_(), B, C, D, z, dt_bias, true, OptTensor(), chunk));
+  y = invoke_call(c10::make_intrusive<NormCall>(y.view({nb, nl, di}), norm_w, OptTensor(), OptTensor(), true, eps, true, false, true))[0];
+  return py::cast(at::mm(y.view({nb * nl, di}), out_proj.t()).view({nb, nl, dm}));
+}
+
 // Packed sequences.  reset: Y restarts at every boundary; without it Y is the scan through all of them.  -> (Y, last state, states)
 std::tuple<Tensor, Tensor, Tensor> ssd_packed(const Tensor& X, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
                                               const OptTensor& z, const OptTensor& dt_bias, bool softplus, const OptTensor& init, int64_t chunk,
@@ -1019,6 +1154,8 @@ void bind_operators(py::module& m) {
   ops.def("fused_layer_norm", &fused_layer_norm);
   ops.def("mamba1_step", &mamba1_step);
   ops.def("mamba2_step", &mamba2_step);
+  ops.def("mamba1_mixer", &mamba1_mixer);
+  ops.def("mamba2_mixer", &mamba2_mixer);
   ops.def("ssd_scan", &ssd_scan);
   ops.def("ssd_packed", &ssd_packed);
   ops.def("ssd_status", &ssd_status);

@@ -29,8 +29,12 @@ def mamba1_mixer_forward(ops: Any, w: dict, cfg: dict, hidden: Tensor) -> Tensor
     """The Mamba-1 mixer alone: hidden (B, L, d_model) -> (B, L, d_model), before any residual add or norm.
 
     ``w``: in_x, in_z (d_inner, d_model); conv_w (d_inner, K), conv_b; x_proj (R + 2N, d_inner);
-    dt_proj (d_inner, R); dt_bias, A (d_inner, N), D (fp32); out_proj (d_model, d_inner).
+    dt_proj (d_inner, R); dt_bias, A (d_inner, N) or A_log, D (fp32); out_proj (d_model, d_inner).
     """
+    if hidden.is_cuda and hasattr(ops, "mamba1_mixer"):  # one call where the operators need not be composed
+        out = ops.mamba1_mixer(hidden, w)
+        if out is not None:
+            return out
     n, r = cfg["d_state"], cfg["dt_rank"]
     nb, nl, dm = hidden.shape
     di = w["in_x"].shape[0]
@@ -48,7 +52,8 @@ def mamba1_mixer_forward(ops: Any, w: dict, cfg: dict, hidden: Tensor) -> Tensor
     delta = rows(torch.matmul(w["dt_proj"], dt_low))                   # (B, Di, L) view
     Bg = Bm.view(n, nb, nl).permute(1, 0, 2).unsqueeze(1)              # (B, 1, N, L)
     Cg = Cm.view(n, nb, nl).permute(1, 0, 2).unsqueeze(1)
-    y = ops.selective_scan(u, delta, w["A"], Bg, Cg, D=w["D"], z=z, dt_bias=w["dt_bias"], softplus=True)
+    A = w["A"] if "A" in w else -torch.exp(w["A_log"])
+    y = ops.selective_scan(u, delta, A, Bg, Cg, D=w["D"], z=z, dt_bias=w["dt_bias"], softplus=True)
     y2 = y.permute(1, 0, 2).reshape(di, nb * nl)
     return torch.matmul(y2.t(), w["out_proj"].t()).view(nb, nl, dm)     # (B, L, d_model)
 
@@ -134,24 +139,20 @@ class Mamba1Block(nn.Module):
     _STEP_WEIGHTS = ("in_x", "in_z", "conv_w", "conv_b", "x_proj", "dt_proj", "dt_bias", "A_log", "D", "out_proj", "norm_w")
 
     def _step_weights(self) -> dict:
-        """The weights as a decode step takes them.  The parameter table saves nn.Module's attribute look-up per weight and step; with a
+        """The weights as the mixer's functions take them.  The parameter table saves nn.Module's attribute look-up per weight and step; with a
         weight that is not in it (parametrised, pruned, replaced by a plain tensor) all are read as attributes."""
         p = self._parameters
         return p if all(n in p for n in self._STEP_WEIGHTS) else {n: getattr(self, n) for n in self._STEP_WEIGHTS}
-
-    def _weights(self) -> dict:
-        return dict(in_x=self.in_x, in_z=self.in_z, conv_w=self.conv_w, conv_b=self.conv_b, x_proj=self.x_proj, dt_proj=self.dt_proj,
-                    dt_bias=self.dt_bias, A=-torch.exp(self.A_log), D=self.D, out_proj=self.out_proj, norm_w=self.norm_w)
 
     def forward(self, hidden: Tensor, residual: Optional[Tensor] = None):
         if hidden.ndim != 3 or hidden.shape[-1] != self.d_model:
             raise ValueError("hidden_states must have shape (B, L, d_model).")
         cfg = dict(d_state=self.d_state, dt_rank=self.dt_rank, eps=self.eps)
-        return mamba1_block_forward(self._namespace(), self._weights(), cfg, hidden, residual)
+        return mamba1_block_forward(self._namespace(), self._step_weights(), cfg, hidden, residual)
 
     def mixer_forward(self, u: Tensor) -> Tensor:
         """The mixer alone (no residual add, no norm): u (B, L, d_model) -> (B, L, d_model)."""
-        return mamba1_mixer_forward(self._namespace(), self._weights(), dict(d_state=self.d_state, dt_rank=self.dt_rank), u)
+        return mamba1_mixer_forward(self._namespace(), self._step_weights(), dict(d_state=self.d_state, dt_rank=self.dt_rank), u)
 
     def mixer_step(self, tok: Tensor, cache) -> Tensor:
         """The mixer alone on one token: tok (B, d_model) -> (B, d_model); ``cache`` from `allocate_inference_cache`."""
@@ -200,6 +201,10 @@ def mamba2_block_forward(ops: Any, w: dict, cfg: dict, hidden: Tensor, residual:
 
 def mamba2_mixer_forward(ops: Any, w: dict, cfg: dict, u: Tensor, group=None, sharded: bool = False) -> Tensor:
     """The Mamba-2 mixer alone on normed activations u (B, L, d_model) -> (B, L, d_model); see `mamba2_block_forward`."""
+    if not sharded and u.is_cuda and hasattr(ops, "mamba2_mixer") and not torch.is_grad_enabled():
+        out = ops.mamba2_mixer(u, w, cfg)
+        if out is not None:
+            return out
     nb, nl, dm = u.shape
     nh, hp, n, g = cfg["heads"], cfg["headdim"], cfg["d_state"], cfg["groups"]
     eps = cfg.get("eps", 1e-5)
@@ -313,18 +318,25 @@ class Mamba2Block(nn.Module):
 
         return ops
 
+    _WEIGHTS = ("pre_norm_w", "in_z", "in_x", "in_B", "in_C", "in_dt", "conv_x", "conv_B", "conv_C", "conv_x_b", "conv_B_b", "conv_C_b", "dt_bias", "A_log",
+                "D", "norm_w", "out_proj")
+
+    def _weights(self) -> dict:
+        """As Mamba1Block._step_weights."""
+        p = self._parameters
+        return p if all(n in p for n in self._WEIGHTS) else {n: getattr(self, n) for n in self._WEIGHTS}
+
     def _cfg(self) -> dict:
         return dict(heads=self.heads, headdim=self.headdim, d_state=self.d_state, groups=self.ngroups, chunk_size=self.chunk_size, eps=self.eps)
 
     def forward(self, hidden: Tensor, residual: Optional[Tensor] = None, sharded: bool = False, group=None):
         if hidden.ndim != 3 or hidden.shape[-1] != self.d_model:
             raise ValueError("hidden_states must have shape (B, L, d_model).")
-        w = {k: v for k, v in self.named_parameters()}
-        return mamba2_block_forward(self._namespace(), w, self._cfg(), hidden, residual, group=group, sharded=sharded)
+        return mamba2_block_forward(self._namespace(), self._weights(), self._cfg(), hidden, residual, group=group, sharded=sharded)
 
     def mixer_forward(self, u: Tensor, sharded: bool = False, group=None) -> Tensor:
         """The mixer alone on normed activations: u (B, L, d_model) -> (B, L, d_model)."""
-        return mamba2_mixer_forward(self._namespace(), {k: v for k, v in self.named_parameters()}, self._cfg(), u, group=group, sharded=sharded)
+        return mamba2_mixer_forward(self._namespace(), self._weights(), self._cfg(), u, group=group, sharded=sharded)
 
     def allocate_inference_cache(self, batch_size: int, dtype: Optional[torch.dtype] = None):
         """((conv windows of x, B, C: (B, C_i, K)), ssm_state (B, H, P, N)), all fp32 and zero-filled."""

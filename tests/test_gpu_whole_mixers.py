@@ -1,0 +1,105 @@
+"""Mixers behind one call against the same operators composed one by one: outputs, every gradient, any subset of inputs that takes one, and
+the modes in which the composed form has to serve."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from ssm_b200 import ops
+from ssm_b200.mixer import Mamba1Block, Mamba2Block
+
+pytestmark = pytest.mark.gpu
+
+# the composed form, which torch has to record node by node
+composed = lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t)  # noqa: E731
+
+
+def _near(a, b, dtype, what):
+    # 16-bit chains that differ where a gradient is added in a product's epilogue instead of after a rounding of its own
+    tol = 1e-4 if dtype == torch.float32 else 2e-2
+    assert a.dtype == b.dtype and a.shape == b.shape, what
+    assert (a.double() - b.double()).norm() <= tol * b.double().norm() + 1e-6, what
+
+
+@pytest.mark.parametrize("nb,nl,dm,dtype", [(2, 40, 96, torch.bfloat16), (1, 1, 64, torch.float16), (3, 77, 64, torch.float32), (2, 300, 256, torch.bfloat16)])
+def test_mamba1_matches_composed_operators(nb, nl, dm, dtype):
+    torch.manual_seed(nl)
+    block = Mamba1Block(dm, device="cuda", dtype=dtype)
+    hidden = torch.randn(nb, nl, dm, device="cuda").to(dtype).requires_grad_()
+    res = torch.randn(nb, nl, dm, device="cuda").requires_grad_()
+    go, gr = torch.randn(nb, nl, dm, device="cuda").to(dtype), torch.randn(nb, nl, dm, device="cuda")
+    names = ["hidden", "residual", *(n for n, _ in block.named_parameters())]
+
+    def run():
+        out, new = block(hidden, res)
+        return out, new, torch.autograd.grad((out, new), [hidden, res, *block.parameters()], (go, gr))
+
+    assert ops.mamba1_mixer(hidden, block._step_weights()) is not None
+    got = run()
+    with composed():
+        assert ops.mamba1_mixer(hidden, block._step_weights()) is None
+        want = run()
+    with torch.no_grad():
+        plain = block(hidden, res)
+    _near(got[0], want[0], dtype, "out"), _near(got[1], want[1], dtype, "residual"), _near(plain[0], want[0], dtype, "out without gradients")
+    for n, a, b in zip(names, got[2], want[2]):
+        _near(a, b, dtype, n)
+
+
+@pytest.mark.parametrize("live", [["hidden"], ["out_proj"], ["in_z", "conv_b"], ["A_log", "dt_proj"], ["x_proj"], ["hidden", "in_x", "conv_w", "D", "dt_bias"]])
+def test_mamba1_gradients_of_a_subset(live):
+    torch.manual_seed(0)
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    hidden = torch.randn(2, 33, 64, device="cuda").bfloat16().requires_grad_("hidden" in live)
+    for n, p in block.named_parameters():
+        p.requires_grad_(n in live)
+    go = torch.randn(2, 33, 64, device="cuda").bfloat16()
+    leaves = [hidden if n == "hidden" else getattr(block, n) for n in live]
+    got = torch.autograd.grad(block.mixer_forward(hidden), leaves, go)
+    with composed():
+        want = torch.autograd.grad(block.mixer_forward(hidden), leaves, go)
+    for n, a, b in zip(live, got, want):
+        _near(a, b, torch.bfloat16, n)
+
+
+def test_mamba1_edits_in_place_are_seen_and_a_graph_can_be_walked_twice():
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    hidden = torch.randn(1, 20, 64, device="cuda").bfloat16().requires_grad_()
+    out = block.mixer_forward(hidden)
+    a = torch.autograd.grad(out.sum(), [hidden, block.in_x], retain_graph=True)
+    b = torch.autograd.grad(out.sum(), [hidden, block.in_x], retain_graph=True)
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    with torch.no_grad():
+        block.out_proj.mul_(2.0)
+    with pytest.raises(RuntimeError, match="modified in place"):
+        torch.autograd.grad(out.sum(), hidden)
+
+
+def test_mamba1_modes_that_compose():
+    block = Mamba1Block(64, device="cuda", dtype=torch.float32)
+    hidden = torch.randn(1, 20, 64, device="cuda")
+    with torch.autocast("cuda", torch.bfloat16):
+        assert ops.mamba1_mixer(hidden, block._step_weights()) is None
+        assert block.mixer_forward(hidden).dtype == torch.bfloat16
+    assert ops.mamba1_mixer(hidden.bfloat16(), block._step_weights()) is None  # other types than the weights'
+    assert ops.mamba1_mixer(hidden[:, :0], block._step_weights()) is None
+    half = Mamba1Block(64, device="cuda", dtype=torch.bfloat16).requires_grad_(False)
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda t: half.mixer_forward(t), hidden.bfloat16(), check_trace=False)
+        _near(traced(hidden.bfloat16() * 2), half.mixer_forward(hidden.bfloat16() * 2), torch.bfloat16, "traced")
+
+
+@pytest.mark.parametrize("nb,nl,dm,groups,dtype", [(2, 300, 128, 1, torch.bfloat16), (1, 1, 64, 1, torch.float16), (1, 513, 256, 2, torch.bfloat16)])
+def test_mamba2_matches_composed_operators(nb, nl, dm, groups, dtype):
+    torch.manual_seed(nl)
+    block = Mamba2Block(dm, ngroups=groups, device="cuda", dtype=dtype)
+    hidden, res = torch.randn(nb, nl, dm, device="cuda").to(dtype), torch.randn(nb, nl, dm, device="cuda")
+    with torch.no_grad():
+        assert ops.mamba2_mixer(hidden, block._weights(), block._cfg()) is not None
+        got = block(hidden, res)
+        with composed():
+            assert ops.mamba2_mixer(hidden, block._weights(), block._cfg()) is None
+            want = block(hidden, res)
+    assert ops.mamba2_mixer(hidden, block._weights(), block._cfg()) is None  # gradients enabled
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])

@@ -118,6 +118,8 @@ struct Piece4 {
 // Lanes of four projections instead of eight take 19.3 and 32.0 us.
 template <typename T, int V, bool APPLY>
 __global__ void __launch_bounds__(kChunkThreads) chunk_fwd_row_kernel(const ssm_chunk_args a, int nchunks, int len) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int U = 32 / V, P2 = V / 2;
   using Raw = typename RowRaw<T, V>::type;
   const int HP = a.heads * a.proj;
@@ -207,6 +209,8 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_fwd_row_kernel(const ssm_
 // 29.0 with them; lanes of four projections 25.6.
 template <typename T, int V>
 __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_local_row_kernel(const ssm_chunk_bwd_args g, float* __restrict__ R, int nchunks, int len) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int U = 32 / V, P2 = V / 2;
   using Raw = typename RowRaw<T, V>::type;
   const ssm_chunk_args& a = g.fwd;
@@ -279,6 +283,8 @@ constexpr int bwd4_ctas() {  // resident CTAs per SM: what the registers of the 
 template <typename T, bool SAME>
 __global__ void __launch_bounds__(kChunkThreads, bwd4_ctas<T>()) chunk_bwd4_kernel(const ssm_chunk_bwd_args g, const float* __restrict__ S, const float* __restrict__ R,
                                                                       int nchunks, int len, int typed_dt) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int SUB = kBwdSub, NG = kPiece / SUB, UF = kBwdSweep;
   static_assert(SUB == 2, "the sums of a group's two steps share their shuffles");
   using Raw = typename RowRaw<T, 4>::type;

@@ -48,6 +48,8 @@ inline int launch_status(const char* kernel) {
 
 // Launch that may begin while the kernel before it on the stream drains.  The kernel calls pdl_wait() before it touches memory, then
 // pdl_trigger(): in that order, so that whatever starts early behind it finds everything before it finished.
+// For chains of short kernels: a cut selective scan of 512 rows (three launches) 34.6 -> 31.1 us.  Not for the state-space-dual scan, whose
+// kernels fill an SM's shared memory each (forward and backward of 2 x 4001 steps 524 us, 564 so).
 template <typename... P, typename... A>
 inline int launch_overlapped(const char* name, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchAttribute attr[1];

@@ -241,6 +241,8 @@ __device__ __forceinline__ void norm_stats(const ssm_norm_args& a, int gt, int n
 // RES = false: the call has no residual (its registers are then free, which raises the number of rows in flight).
 template <typename T, int G, int MC = kNormFwdChunks, bool RES = true>
 __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK) norm_fwd_kernel(const ssm_norm_args a) {
+  pdl_wait();
+  pdl_trigger();
   using Cfg = NormCfg<T, G>;
   constexpr int V = Cfg::V;
   constexpr int kNormFwdChunks = MC;
@@ -336,6 +338,8 @@ constexpr int norm_bwd_min_ctas() {
 }
 template <typename T, int G, int MC>
 __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_min_ctas<G, MC>()) norm_bwd_kernel(const ssm_norm_bwd_args g) {
+  pdl_wait();
+  pdl_trigger();
   using Cfg = NormCfg<T, G>;
   constexpr int V = Cfg::V;
   constexpr bool kSmemAcc = G <= 128;
@@ -497,6 +501,8 @@ __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_min_ctas<G, MC>
 constexpr int kFoldLanes = 32;
 __global__ void __launch_bounds__(32 * kFoldLanes) norm_fold_kernel(const float* __restrict__ partial, int nctas, int hidden,
                                                                    void* __restrict__ dweight, void* __restrict__ dbias, int dtype) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float sw[kFoldLanes][33], sb[kFoldLanes][33];
   const int cx = threadIdx.x & 31, ky = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + cx;
@@ -618,9 +624,11 @@ template <typename T, int G, int MC = kNormFwdChunks>
 static int norm_fwd_launch(const ssm_norm_args& a, cudaStream_t st) {
   using Cfg = NormCfg<T, G>;
   const unsigned grid = (unsigned)((a.rows + Cfg::RPC - 1) / Cfg::RPC);
-  if (a.residual) norm_fwd_kernel<T, G, MC, true><<<grid, Cfg::BLOCK, 0, st>>>(a);
-  else norm_fwd_kernel<T, G, MC, false><<<grid, Cfg::BLOCK, 0, st>>>(a);
-  return launch_status("norm_fwd_kernel");
+  return launch_overlapped("norm_fwd_kernel", a.residual ? norm_fwd_kernel<T, G, MC, true> : norm_fwd_kernel<T, G, MC, false>, dim3(grid), dim3(Cfg::BLOCK), 0, st, a);
+}
+static int norm_fold(const ssm_norm_bwd_args& g, int parts, cudaStream_t st) {
+  return launch_overlapped("norm_fold_kernel", norm_fold_kernel, dim3((g.fwd.hidden + 31) / 32), dim3(32 * kFoldLanes), 0, st, g.partial, parts, g.fwd.hidden, g.dweight, g.dbias,
+                           g.fwd.dparam_dtype);
 }
 template <typename T, int G, int MC>
 static int norm_bwd_launch(const ssm_norm_bwd_args& g, cudaStream_t st, int max_ctas = kNormBwdMaxCtas) {
@@ -634,10 +642,8 @@ static int norm_bwd_launch(const ssm_norm_bwd_args& g, cudaStream_t st, int max_
   int nctas = norm_bwd_ctas(g.fwd, Cfg::RPC);
   if (nctas > max_ctas) nctas = max_ctas;
   if (nctas > resident) nctas = resident;
-  norm_bwd_kernel<T, G, MC><<<nctas, Cfg::BLOCK, 0, st>>>(g);
-  if (int rc = launch_status("norm_bwd_kernel")) return rc;
-  norm_fold_kernel<<<(g.fwd.hidden + 31) / 32, 32 * kFoldLanes, 0, st>>>(g.partial, nctas, g.fwd.hidden, g.dweight, g.dbias, g.fwd.dparam_dtype);
-  return launch_status("norm_fold_kernel");
+  if (int rc = launch_overlapped("norm_bwd_kernel", norm_bwd_kernel<T, G, MC>, dim3(nctas), dim3(Cfg::BLOCK), 0, st, g)) return rc;
+  return norm_fold(g, nctas, st);
 }
 
 // rows of up to 128 chunks go to one warp each (1 .. 4 chunks per lane), wider ones to 128 or 512 threads
@@ -683,8 +689,7 @@ static int norm_bwd_scalar(const ssm_norm_bwd_args& g, cudaStream_t st) {
   cudaMemsetAsync(g.partial, 0, sizeof(float) * 2 * hidden, st);
   norm_scalar_kernel<T, true><<<(unsigned)g.fwd.rows, 128, 0, st>>>(g);
   if (int rc = launch_status("norm_scalar_kernel")) return rc;
-  norm_fold_kernel<<<(hidden + 31) / 32, 32 * kFoldLanes, 0, st>>>(g.partial, 1, hidden, g.dweight, g.dbias, g.fwd.dparam_dtype);
-  return launch_status("norm_fold_kernel");
+  return norm_fold(g, 1, st);
 }
 template <typename T>
 static int norm_bwd_t(const ssm_norm_bwd_args& g, cudaStream_t st) {

@@ -65,6 +65,8 @@ struct FwdStepOps {  // everything of one step that does not depend on the state
 // (scan_split_combine_kernel) pass 2 replays every segment from its true incoming state and produces the outputs.
 template <typename T, int NG, int MODE, bool RAG>
 __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kernel(const ssm_scan_fwd_args a, const ScanFlags fl, int seg_tiles) {
+  pdl_wait();
+  pdl_trigger();
   using M = FwdTiles<T, NG, RAG>;
   constexpr int NP = M::NP, TL = M::TL, TLP = M::TLP, V = M::V, NT = M::NT, RP = M::RP, BCP = M::BCP;
   constexpr int CH = TL / V;  // 16-byte chunks per row and tile
@@ -442,6 +444,8 @@ __global__ void __launch_bounds__(NG * 32, NG <= 4 ? 3 : 1) scan_fwd_tiles_kerne
 
 // Serial pass over the segments of a split call: split_h[s] <- state entering segment s.  One thread per (row, state).
 static __global__ void __launch_bounds__(128) scan_split_combine_kernel(float* __restrict__ split, int64_t rows_states, int nstate, int nseg) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
   if (i >= rows_states) return;
   const int64_t row = i / nstate;
@@ -503,8 +507,7 @@ static int launch_fwd_tiles(const ssm_scan_fwd_args& a, const ScanFlags& fl, cud
   if (nseg <= 1) {
     auto kern = scan_fwd_tiles_kernel<T, NG, 0, RAG>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kBytes);
-    kern<<<dim3(gx, a.batch), NG * 32, M::kBytes, st>>>(a, fl, ntiles);
-    return launch_status("scan_fwd_tiles_kernel");
+    return launch_overlapped("scan_fwd_tiles_kernel", kern, dim3(gx, a.batch), dim3(NG * 32), M::kBytes, st, a, fl, ntiles);
   }
   const int seg_tiles = (ntiles + nseg - 1) / nseg;
   const int used = (ntiles + seg_tiles - 1) / seg_tiles;  // segments that hold at least one tile
@@ -512,13 +515,11 @@ static int launch_fwd_tiles(const ssm_scan_fwd_args& a, const ScanFlags& fl, cud
   auto k2 = scan_fwd_tiles_kernel<T, NG, 2, RAG>;
   cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kBytes);
   cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kBytes);
-  k1<<<dim3(gx, a.batch, used), NG * 32, M::kBytes, st>>>(a, fl, seg_tiles);
-  if (int rc = launch_status("scan_fwd_tiles_kernel<local>")) return rc;
+  if (int rc = launch_overlapped("scan_fwd_tiles_kernel<local>", k1, dim3(gx, a.batch, used), dim3(NG * 32), M::kBytes, st, a, fl, seg_tiles)) return rc;
   const int64_t rs = (int64_t)a.batch * a.dim * a.nstate;
-  scan_split_combine_kernel<<<(unsigned)((rs + 127) / 128), 128, 0, st>>>(a.split_scratch, rs, a.nstate, used);
-  if (int rc = launch_status("scan_split_combine_kernel")) return rc;
-  k2<<<dim3(gx, a.batch, used), NG * 32, M::kBytes, st>>>(a, fl, seg_tiles);
-  return launch_status("scan_fwd_tiles_kernel<final>");
+  if (int rc = launch_overlapped("scan_split_combine_kernel", scan_split_combine_kernel, dim3((unsigned)((rs + 127) / 128)), dim3(128), 0, st, a.split_scratch, rs, a.nstate, used))
+    return rc;
+  return launch_overlapped("scan_fwd_tiles_kernel<final>", k2, dim3(gx, a.batch, used), dim3(NG * 32), M::kBytes, st, a, fl, seg_tiles);
 }
 
 // The tile kernel covers a call whose CTAs' 32 rows lie inside one B / C group: as whole vectors, or (rows that start anywhere, B / C

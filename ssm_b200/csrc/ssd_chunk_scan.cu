@@ -204,6 +204,8 @@ __device__ __forceinline__ float carry_pieces(const float* __restrict__ P, float
 
 // phase 2: S[c] <- state entering piece c
 __global__ void __launch_bounds__(kCarryLanes * kCarryGroups) chunk_carry_kernel(const ssm_chunk_args a, int nchunks) {
+  pdl_wait();
+  pdl_trigger();
   const int HP = a.heads * a.proj;
   const int hp_raw = blockIdx.x * kCarryLanes + threadIdx.x % kCarryLanes;
   const bool live = hp_raw < HP;
@@ -263,6 +265,8 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_bwd_local_kernel(const ss
 
 // reverse phase 2: over the pieces from the right; R[c] <- adjoint entering piece c from piece c + 1
 __global__ void __launch_bounds__(kCarryLanes * kCarryGroups) chunk_bwd_carry_kernel(const ssm_chunk_bwd_args g, const float* __restrict__ P_all, int nchunks) {
+  pdl_wait();
+  pdl_trigger();
   const ssm_chunk_args& a = g.fwd;
   const int HP = a.heads * a.proj;
   const int hp_raw = blockIdx.x * kCarryLanes + threadIdx.x % kCarryLanes;
@@ -456,16 +460,18 @@ static int chunk_fwd_t(const ssm_chunk_args& a, cudaStream_t st, int chunk_len, 
   constexpr int kWide = 16 / sizeof(T);
   const int v = !std::is_same<T, PT>::value ? 1 : chunk_vec_ok(a, chunk_len, kWide) ? kWide : chunk_vec_ok(a, chunk_len, 4) ? 4 : 1;
   const dim3 grid((HP / v + kChunkThreads - 1) / kChunkThreads, nchunks, a.batch);
-  if (v == kWide) chunk_fwd_row_kernel<T, kWide, false><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  else if (v == 4) chunk_fwd_row_kernel<T, 4, false><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  else chunk_fwd_kernel<T, PT, 1><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  if (int rc = launch_status("chunk_fwd_kernel<local>")) return rc;
-  chunk_carry_kernel<<<dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), kCarryLanes * kCarryGroups, 0, st>>>(a, nchunks);
-  if (int rc = launch_status("chunk_carry_kernel")) return rc;
+  const dim3 block(kChunkThreads);
+  int rc;
+  if (v == kWide) rc = launch_overlapped("chunk_fwd_row_kernel<local>", chunk_fwd_row_kernel<T, kWide, false>, grid, block, 0, st, a, nchunks, chunk_len);
+  else if (v == 4) rc = launch_overlapped("chunk_fwd_row_kernel<local>", chunk_fwd_row_kernel<T, 4, false>, grid, block, 0, st, a, nchunks, chunk_len);
+  else chunk_fwd_kernel<T, PT, 1><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len), rc = launch_status("chunk_fwd_kernel<local>");
+  if (rc) return rc;
+  rc = launch_overlapped("chunk_carry_kernel", chunk_carry_kernel, dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), dim3(kCarryLanes * kCarryGroups), 0, st, a, nchunks);
+  if (rc) return rc;
   if (through_phase2_only) return SSM_OK;
-  if (v == kWide) chunk_fwd_row_kernel<T, kWide, true><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  else if (v == 4) chunk_fwd_row_kernel<T, 4, true><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
-  else chunk_fwd_kernel<T, PT, 3><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
+  if (v == kWide) return launch_overlapped("chunk_fwd_row_kernel<apply>", chunk_fwd_row_kernel<T, kWide, true>, grid, block, 0, st, a, nchunks, chunk_len);
+  if (v == 4) return launch_overlapped("chunk_fwd_row_kernel<apply>", chunk_fwd_row_kernel<T, 4, true>, grid, block, 0, st, a, nchunks, chunk_len);
+  chunk_fwd_kernel<T, PT, 3><<<grid, kChunkThreads, 0, st>>>(a, nchunks, chunk_len);
   return launch_status("chunk_fwd_kernel<apply>");
 }
 
@@ -535,22 +541,27 @@ static int chunk_bwd_t(const ssm_chunk_bwd_args& g_in, cudaStream_t st) {
   const float* S = P + (int64_t)a.batch * nchunks * HP;
   float* R = g.scratch + 2 * (int64_t)a.batch * nchunks * HP;
   const unsigned gv = (HP / 4 + kChunkThreads - 1) / kChunkThreads;
-  if (vec && chunk_bwd_wide_ok(g, 16 / (int)sizeof(T))) {
-    chunk_bwd_local_row_kernel<T, 16 / (int)sizeof(T)><<<dim3((HP / (16 / (int)sizeof(T)) + kChunkThreads - 1) / kChunkThreads, nchunks, a.batch), kChunkThreads, 0, st>>>(
-        g, R, nchunks, a.chunk_size);
+  constexpr int kWide = 16 / sizeof(T);
+  int rc;
+  if (vec && chunk_bwd_wide_ok(g, kWide)) {
+    rc = launch_overlapped("chunk_bwd_local_row_kernel", chunk_bwd_local_row_kernel<T, kWide>, dim3((HP / kWide + kChunkThreads - 1) / kChunkThreads, nchunks, a.batch),
+                           dim3(kChunkThreads), 0, st, g, R, nchunks, a.chunk_size);
   } else if (vec) {
-    chunk_bwd_local_row_kernel<T, 4><<<dim3(gv, nchunks, a.batch), kChunkThreads, 0, st>>>(g, R, nchunks, a.chunk_size);
-  } else chunk_bwd_local_kernel<T, PT><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
-  if (int rc = launch_status("chunk_bwd_local_kernel")) return rc;
-  chunk_bwd_carry_kernel<<<dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), kCarryLanes * kCarryGroups, 0, st>>>(g, P, nchunks);
-  if (int rc = launch_status("chunk_bwd_carry_kernel")) return rc;
+    rc = launch_overlapped("chunk_bwd_local_row_kernel", chunk_bwd_local_row_kernel<T, 4>, dim3(gv, nchunks, a.batch), dim3(kChunkThreads), 0, st, g, R, nchunks, a.chunk_size);
+  } else {
+    chunk_bwd_local_kernel<T, PT><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, nchunks);
+    rc = launch_status("chunk_bwd_local_kernel");
+  }
+  if (rc) return rc;
+  rc = launch_overlapped("chunk_bwd_carry_kernel", chunk_bwd_carry_kernel, dim3((HP + kCarryLanes - 1) / kCarryLanes, 1, a.batch), dim3(kCarryLanes * kCarryGroups), 0, st, g, P,
+                         nchunks);
+  if (rc) return rc;
   if (vec) {
     const int64_t items = (int64_t)a.batch * nchunks, slots = (int64_t)bwd4_ctas<T>() * sm_count() / gv;  // one wave of CTAs, each looping over pieces
     const int64_t rounds = (items + (slots < 1 ? 1 : slots) - 1) / (slots < 1 ? 1 : slots);
     const unsigned gy = (unsigned)((items + rounds - 1) / rounds);  // as many CTAs as the longest of them makes worthwhile
-    if (chunk_same_layout(g)) chunk_bwd4_kernel<T, true><<<dim3(gv, gy), kChunkThreads, 0, st>>>(g, S, R, nchunks, a.chunk_size, (a.typed_grads & 8) != 0);
-    else chunk_bwd4_kernel<T, false><<<dim3(gv, gy), kChunkThreads, 0, st>>>(g, S, R, nchunks, a.chunk_size, (a.typed_grads & 8) != 0);
-    return launch_status("chunk_bwd4_kernel");
+    return launch_overlapped("chunk_bwd4_kernel", chunk_same_layout(g) ? chunk_bwd4_kernel<T, true> : chunk_bwd4_kernel<T, false>, dim3(gv, gy), dim3(kChunkThreads), 0, st, g, S, R,
+                             nchunks, a.chunk_size, (int)((a.typed_grads & 8) != 0));
   }
   chunk_bwd_kernel<T, PT, 1><<<dim3(gx, nchunks, a.batch), kChunkThreads, 0, st>>>(g, S, nchunks);
   return launch_status("chunk_bwd_kernel");

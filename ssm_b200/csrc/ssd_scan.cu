@@ -20,6 +20,7 @@
 //
 // Exponent differences are always formed before exp2 (never exp2(c_i) / exp2(c_j)), so long
 // sequences stay finite.  Every wait on an mbarrier is bounded and reports through the status word.
+#include "seq_table.h"
 #include "ssd_common.cuh"
 
 #include <algorithm>
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(kQ) ssd_cumsum_kernel(const ssm_ssd_args a, in
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h0 = blockIdx.x * kCumHeads, c = blockIdx.y, b = blockIdx.z;
   const int nh = min(kCumHeads, a.heads - h0);
+  if (a.seq_table && chunk_begin(a, c) >= chunk_limit(a, c)) return;  // no chunk: the table has room to spare
   {
     const int t = chunk_begin(a, c) + tid;
     if (t < chunk_limit(a, c)) {
@@ -612,7 +614,6 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   // the next sequence), everything else leaves through TMA, which cuts at the end of the tensor
   const int t_live = PACKED ? chunk_limit(a, c) - t0 - ROW0 : kBlk;
   const bool ragged = PACKED && t_live < kBlk;
-  if (ragged && t_live <= 0) return;  // the whole CTA: nothing has been issued yet
   const int k_live = ragged ? t_live + ROW0 - COL0 : KJ;  // columns that belong to the sequence
   const int i_loc = (warp & 3) * 32 + lane;    // row within the block = TMEM lane
   const int i_chunk = ROW0 + i_loc;            // row within the chunk
@@ -998,17 +999,62 @@ __global__ void __launch_bounds__(kScanThreads, 1)
   __shared__ __align__(8) uint64_t mbar[8];
   __shared__ uint32_t tmem_slot;
   const int warp = threadIdx.x >> 5;
+  const bool long_block = (int)blockIdx.x < (int)(gridDim.x >> 1);
+  if constexpr (PACKED) {  // no rows: the sequence ends before them, or the table has room to spare
+    const int c = (int)blockIdx.x % (int)(gridDim.x >> 1) / nparts % nchunks;
+    if (chunk_limit(a, c) - chunk_begin(a, c) <= (long_block ? kBlk : 0)) return;
+  }
   if (warp == 0) tc::tmem_alloc(tc::smem_u32(&tmem_slot), 512);
   if (threadIdx.x == 0) {
     for (int i = 0; i < 8; ++i) tc::mbar_init(tc::smem_u32(&mbar[i]), 1);
   }
   __syncthreads();  // barriers and the TMEM address are set up before anyone arms or polls them
   // the heavier blocks (rows 128..255; REV: rows 0..127) are scheduled first
-  if ((int)blockIdx.x < (int)(gridDim.x >> 1)) ssd_scan_body<T, 1, XSKIP, REV, PACKED>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
+  if (long_block) ssd_scan_body<T, 1, XSKIP, REV, PACKED>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
   else ssd_scan_body<T, 0, XSKIP, REV, PACKED>(a, maps, nchunks, hpc, nparts, smraw, mbar, &tmem_slot);
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem_slot, 512);
+}
+
+// One CTA: sequences are taken kTableThreads at a time, a thread counting the chunks of one, a warp writing them out.
+constexpr int kTableThreads = 1024;
+__global__ void __launch_bounds__(kTableThreads) seq_table_kernel(const void* __restrict__ cu, int wide, int num_seqs, int len, int num_chunks, int* __restrict__ table) {
+  __shared__ int from[kTableThreads], to[kTableThreads], at[kTableThreads], warp_sum[32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  auto bound = [&](int i) {
+    const int64_t v = wide ? __ldg(reinterpret_cast<const long long*>(cu) + i) : (int64_t)__ldg(reinterpret_cast<const int*>(cu) + i);
+    return (int)min(max(v, (int64_t)0), (int64_t)len);
+  };
+  int* first = table + 2 * num_chunks;
+  int base = 0;  // chunks of the sequences so far
+  for (int s0 = 0; s0 < num_seqs; s0 += kTableThreads) {
+    const int s = s0 + tid, b = s < num_seqs ? bound(s) : 0, e = s < num_seqs ? bound(s + 1) : 0;
+    const int n = e > b ? (e - b + kQ - 1) / kQ : 0;
+    int sum = n;  // inclusive prefix over the warp, then over the warps
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, sum, off);
+      if (lane >= off) sum += v;
+    }
+    if (lane == 31) warp_sum[warp] = sum;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) before += warp_sum[w];
+      total += warp_sum[w];
+    }
+    from[tid] = b, to[tid] = e, at[tid] = min(base + before + sum - n, num_chunks);
+    if (s < num_seqs) first[s] = at[tid];
+    __syncthreads();
+    for (int q = warp; q < kTableThreads && s0 + q < num_seqs; q += 32) {
+      for (int c = lane; from[q] + c * kQ < to[q] && at[q] + c < num_chunks; c += 32) table[2 * (at[q] + c)] = from[q] + c * kQ, table[2 * (at[q] + c) + 1] = to[q];
+    }
+    base = min(base + total, num_chunks);
+    __syncthreads();
+  }
+  if (tid == 0) first[num_seqs] = base;
+  for (int c = base + tid; c < num_chunks; c += kTableThreads) table[2 * c] = table[2 * c + 1] = len;
 }
 
 template <typename T, int HPC, int NST, bool REV, bool PACKED>
@@ -1111,8 +1157,9 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
   const int nchunks = a.num_seqs ? a.num_chunks : (a.len + kQ - 1) / kQ;
   const int walks = a.num_seqs ? a.num_seqs : a.batch;  // sequences that the state kernel walks
   const int hpg = a.heads / a.groups;
-  // (of packed sequences about every second one ends in a chunk without a long block)
-  const int64_t blocks = (int64_t)a.batch * nchunks;
+  // (of packed sequences about every second one ends in a chunk without a long block, and a table with room to spare holds half a chunk per
+  // sequence more than there are)
+  const int64_t blocks = a.num_seqs ? std::min<int64_t>(nchunks, a.len / kQ + (a.num_seqs + 1) / 2) : (int64_t)a.batch * nchunks;
   const int hpc = scan_heads_per_cta(hpg, (a.num_seqs ? std::max<int64_t>(blocks - a.num_seqs / 2, 0) : blocks) * a.groups, blocks * a.groups);
   const int nparts = a.heads / hpc;
   if (a.phase != 2 && !a.reverse) {
@@ -1201,6 +1248,13 @@ extern "C" int ssm_ssd_fold_shards(const float* gathered, int32_t world, int32_t
   ssd_fold_shards_kernel<<<(unsigned)((total + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       gathered, rank, ssm_ssd_shard_summary_floats(batch, heads), batch * heads, kP * kN, initial_states, incoming);
   return launch_status("ssd_fold_shards_kernel");
+}
+
+extern "C" int ssmb_seq_table(const void* cu, int32_t wide, int32_t num_seqs, int32_t len, int32_t num_chunks, int32_t* table, void* stream) {
+  SSM_REQUIRE(cu && table, SSM_ERR_NULL, "seq_table: missing tensor");
+  SSM_REQUIRE(num_seqs >= 1 && len >= 0 && num_chunks >= 0, SSM_ERR_SHAPE, "seq_table: bad shape");
+  seq_table_kernel<<<1, kTableThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(cu, wide, num_seqs, len, num_chunks, table);
+  return launch_status("seq_table_kernel");
 }
 
 extern "C" int ssm_ssd_wait_selftest(int32_t* status, int32_t probes, ssm_stream_t stream) {

@@ -8,7 +8,9 @@
 // gradient of its own columns in registers across all rows its CTA visits, the CTA writes
 // one partial row, and a second small kernel folds the partials -- no atomics, bitwise
 // reproducible.
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -314,183 +316,247 @@ __device__ __forceinline__ void group_allsum2(float& a, float& b, float2 (*scrat
   }
 }
 
-// A row's pieces of everything the backward pass reads, in flight: x, the residual, dy, and the gradient arriving through the
-// x + residual output.
-template <int MC>
-struct NormBwdRaw {
-  NormRowRaw<MC> in;
-  uint4 dy[MC], ga[MC], gb[MC];
-};
-
-// MC = 16-byte chunks of a row per thread.  A row of up to 32 * MC chunks is owned by ONE warp (G = 32); wider rows take 128 or
-// 512 threads.  The time of a row is a chain of latencies, so:
-//  * every load of a row is issued before the first use (requesting the next row ahead as well costs more CTAs per SM than it
-//    hides: 123 us against 107 then);
-//  * a row needs two rounds of sums, two values each: {sum s, sum w dy}, then {sum (s - mean)^2, sum w dy (s - mean)}, from which
-//    the standard deviation and both correction terms follow (one round for RMSNorm);
-//  * with 128-thread CTAs the running weight / bias gradients of a thread's columns live in shared-memory slots of its own, four
-//    to a 16-byte access (same additions in the same order), which leaves the registers to the loads in flight.
-// 16376 rows of 1600 bf16 columns, fp32 residual and its gradient, 471 MB: 157 us with one barrier pair per value and sum, now
-// 101 us (4.7 TB/s).
-template <int G, int MC>
-constexpr int norm_bwd_min_ctas() {
-  return G <= 128 ? (MC <= 1 ? 5 : (MC == 2 ? 4 : (MC == 3 ? 3 : 2))) : 1;
+// Backward.  A row is split into granules of four elements, MG to a thread: granule k of thread t is k * G + t, so that every access
+// of a warp is contiguous in 16-bit and 32-bit tensors alike (8 elements a thread read fp32 rows in half sectors: twice the L2 traffic).
+// The time of a row is a chain of latencies (loads, two rounds of sums, stores), so the rows travel through a ring in shared
+// memory: each thread copies its own granules of x, dy, the residual and the gradient arriving through the x + residual output
+// (asynchronous copies, no barrier) and has its next row under way while it works on this one.  What a row still needs at its end is
+// read there again, which leaves the registers to the running weight / bias gradients of the thread's columns.  Packed fp32 arithmetic.
+//  * A row of up to 32 * 8 granules (fp32: 32 * 4) is owned by ONE warp (G = 32), four rows to a CTA; wider rows take 128 or 512 threads.
+//  * Two rounds of sums, two values each: {sum s, sum w dy}, then {sum (s - mean)^2, sum w dy (s - mean)}, from which the standard
+//    deviation and both correction terms follow (one round for RMSNorm).
+// 16376 rows of 1600 bf16 columns, fp32 residual and its gradient, 471 MB: 104 us with the loads in registers, scalar arithmetic and 16
+// bytes of x per access (63 instructions per element), 69 us so (28; 6.3 TB/s).
+//  * STREAM: a residual stream of fp32, in and out, known at compile time, and FULL granules that every thread has: with run-time types
+//    and every granule guarded the loads of a row could not be put together (54 instructions per element, 104 us).
+template <typename T, int G, int MG>
+constexpr int norm_bwd_ctas_per_sm() {
+  if (G > 128) return 1;
+  return MG <= 4 ? 4 : (MG <= 6 ? 3 : 2);
 }
-template <typename T, int G, int MC>
-__global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_min_ctas<G, MC>()) norm_bwd_kernel(const ssm_norm_bwd_args g) {
+__host__ __device__ constexpr int dtype_bytes(int dtype) { return dtype == SSM_F32 ? 4 : 2; }
+// four elements of a shared-memory slot as fp32 pairs
+template <typename T>
+__device__ __forceinline__ void granule(const unsigned char* p, float2 (&f)[2]) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    f[0] = make_float2(v.x, v.y), f[1] = make_float2(v.z, v.w);
+  } else if constexpr (std::is_same<T, __half>::value) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    f[0] = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), f[1] = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+  } else {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    f[0] = make_float2(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u));
+    f[1] = make_float2(__uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+  }
+}
+__device__ __forceinline__ void granule_dyn(const unsigned char* p, int dtype, float2 (&f)[2]) {
+  if (dtype == SSM_F32) granule<float>(p, f);
+  else if (dtype == SSM_BF16) granule<__nv_bfloat16>(p, f);
+  else granule<__half>(p, f);
+}
+template <typename T>
+__device__ __forceinline__ void granule_store(T* p, const float2 (&f)[2]) {
+  if constexpr (sizeof(T) == 4) {
+    __stcs(reinterpret_cast<float4*>(p), make_float4(f[0].x, f[0].y, f[1].x, f[1].y));
+  } else if constexpr (std::is_same<T, __half>::value) {
+    const __half2 a = __float22half2_rn(f[0]), b = __float22half2_rn(f[1]);
+    __stcs(reinterpret_cast<uint2*>(p), make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b)));
+  } else {
+    const __nv_bfloat162 a = __float22bfloat162_rn(f[0]), b = __float22bfloat162_rn(f[1]);
+    __stcs(reinterpret_cast<uint2*>(p), make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b)));
+  }
+}
+__device__ __forceinline__ void granule_store_dyn(void* base, int64_t i, int dtype, const float2 (&f)[2]) {
+  if (dtype == SSM_F32) granule_store(reinterpret_cast<float*>(base) + i, f);
+  else if (dtype == SSM_BF16) granule_store(reinterpret_cast<__nv_bfloat16*>(base) + i, f);
+  else granule_store(reinterpret_cast<__half*>(base) + i, f);
+}
+__device__ __forceinline__ void granule_copy(uint32_t dst, const char* src, bool wide) {
+  if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
+template <typename T, int G, int MG, int FULL, int ST, bool STREAM>
+__global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_ctas_per_sm<T, G, MG>()) norm_bwd_kernel(const ssm_norm_bwd_args g) {
   pdl_wait();
   pdl_trigger();
   using Cfg = NormCfg<T, G>;
-  constexpr int V = Cfg::V;
-  constexpr bool kSmemAcc = G <= 128;
-  constexpr int kAccRegs = kSmemAcc ? 1 : MC;
-  constexpr int kAccRow = MC * (V / 4) * G;  // float4 slots of one gradient: [chunk][quarter][thread]
+  constexpr int BLOCK = Cfg::BLOCK, RPC = Cfg::RPC, E = 4 * (int)sizeof(T);
+  constexpr bool HOLD = G == 32 || MG <= 6;  // w dy stays in registers between the rounds of sums
+  constexpr bool HOLD_W = MG <= 4;      // the weights of the thread's columns too
+  constexpr int MH = HOLD ? MG : 1, MW = HOLD_W ? MG : 1;
   const ssm_norm_args& a = g.fwd;
+  extern __shared__ __align__(16) unsigned char norm_ring[];
   __shared__ float2 scratch[2][16];
-  __shared__ float4 acc_all[kSmemAcc ? Cfg::RPC * 2 * kAccRow : 1];  // [row slot][weight | bias]
-  const int gt = threadIdx.x % G, slot = threadIdx.x / G;
-  float4* acc = acc_all + (kSmemAcc ? slot * 2 * kAccRow : 0);
-  const int nchunk = a.hidden / V;
+  const int tid = threadIdx.x, gt = tid % G, slot = tid / G;
+  const int ngran = a.hidden / 4;
   const float inv = 1.f / (float)a.hidden;
-  float dw[kAccRegs][V], db[kAccRegs][V];
+  const bool has_r = STREAM || (a.residual && a.prenorm), has_g = STREAM || g.dresidual_out != nullptr;
+  const int rtype = STREAM ? SSM_F32 : a.res_dtype, gtype = STREAM ? SSM_F32 : a.resout_dtype;
+  const int re = has_r ? 4 * dtype_bytes(rtype) : 0, ge = has_g ? 4 * dtype_bytes(gtype) : 0;  // bytes per granule
+  // a stage: x, dy, residual, gradient of the x + residual output, each [granule][thread]
+  const int stage_bytes = MG * BLOCK * (2 * E + re + ge);
+  unsigned char* const sx = norm_ring + tid * E;
+  unsigned char* const sr = norm_ring + 2 * MG * BLOCK * E + tid * re;
+  unsigned char* const sg = norm_ring + MG * BLOCK * (2 * E + re) + tid * ge;
+  const uint32_t ux = (uint32_t)__cvta_generic_to_shared(sx), ur = (uint32_t)__cvta_generic_to_shared(sr), ug = (uint32_t)__cvta_generic_to_shared(sg);
+  const int64_t step = (int64_t)gridDim.x * RPC;
+  auto issue = [&](int64_t row, int at) {
+    if (row < a.rows) {
+      const char* px = reinterpret_cast<const char*>(a.x) + (row * a.hidden + gt * 4) * sizeof(T);
+      const char* pd = reinterpret_cast<const char*>(g.dy) + (row * a.hidden + gt * 4) * sizeof(T);
+      const char* pr = reinterpret_cast<const char*>(a.residual) + (row * ngran + gt) * re;
+      const char* pg = reinterpret_cast<const char*>(g.dresidual_out) + (row * ngran + gt) * ge;
 #pragma unroll
-  for (int c = 0; c < MC; ++c) {
-    if constexpr (kSmemAcc) {
-#pragma unroll
-      for (int q = 0; q < V / 4; ++q) acc[(c * (V / 4) + q) * G + gt] = acc[kAccRow + (c * (V / 4) + q) * G + gt] = make_float4(0.f, 0.f, 0.f, 0.f);
-    } else {
-#pragma unroll
-      for (int i = 0; i < V; ++i) dw[c][i] = 0.f, db[c][i] = 0.f;
+      for (int k = 0; k < MG; ++k) {
+        if (k < FULL || k * G + gt < ngran) {
+          granule_copy(ux + at + k * BLOCK * E, px + k * G * E, E == 16);
+          granule_copy(ux + at + (MG + k) * BLOCK * E, pd + k * G * E, E == 16);
+          if (has_r) granule_copy(ur + at + k * BLOCK * re, pr + k * G * re, re == 16);
+          if (has_g) granule_copy(ug + at + k * BLOCK * ge, pg + k * G * ge, ge == 16);
+        }
+      }
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const float2 zero = make_float2(0.f, 0.f);
+  float2 dw[MG][2], db[MG][2];
+#pragma unroll
+  for (int k = 0; k < MG; ++k) dw[k][0] = dw[k][1] = db[k][0] = db[k][1] = zero;
+  float wh[MW][4];
+  if (HOLD_W) {
+#pragma unroll
+    for (int k = 0; k < MG; ++k) load_param_vec<4>(a.weight, min(k * G + gt, ngran - 1) * 4, a.param_dtype, wh[HOLD_W ? k : 0]);
   }
-  // the weights of this thread's columns are re-read from L1 for every row instead of occupying registers
-  auto load_w = [&](int c, float (&wv)[V]) {
-    load_param_vec<V>(a.weight, min(c * G + gt, nchunk - 1) * V, a.param_dtype, wv);  // beyond the row: dropped (dy is zero there)
-  };
-  auto issue = [&](int64_t row, NormBwdRaw<MC>& raw) {
-    norm_issue_row<T, G, MC>(a, row, gt, nchunk, raw.in);
-    io_issue_row<T, G, MC>(g.dy, row * a.hidden, gt, nchunk, raw.dy);
-    if (g.dresidual_out) dyn_issue_row<V, G, MC>(g.dresidual_out, row * a.hidden, gt, nchunk, a.resout_dtype, raw.ga, raw.gb);
-  };
-  const int64_t npass = (a.rows + Cfg::RPC - 1) / Cfg::RPC;
-  int turn = 0;
-  for (int64_t pass = blockIdx.x; pass < npass; pass += gridDim.x) {
-    const int64_t row = pass * Cfg::RPC + slot;
-    const bool live = row < a.rows;  // dead warps of the last pass (G == 32) work on the last row again and drop the result
-    float s[MC][V], r[MC][V], dy[MC][V];
-    NormBwdRaw<MC> raw;
-    issue(live ? row : a.rows - 1, raw);
-    norm_convert_row<T, G, MC>(a, gt, nchunk, raw.in, s, r);
+  auto load_wdy = [&](int k, int at, float2 (&wdy)[2]) {
+    float w[4];
+    float2 dy[2];
+    if (HOLD_W) {
 #pragma unroll
-    for (int c = 0; c < MC; ++c) {
-      if (live && c * G + gt < nchunk) {
-        Vec16<T> v;
-        v.raw = raw.dy[c];
-        v.unpack(dy[c]);
-        // the gradient through x + residual takes the place of the residual values, dead once the row sum is formed
-        if (g.dresidual_out) dyn_convert<V>(a.resout_dtype, raw.ga[c], raw.gb[c], r[c]);
-      } else {
+      for (int i = 0; i < 4; ++i) w[i] = wh[HOLD_W ? k : 0][i];
+    } else {
+      load_param_vec<4>(a.weight, (k * G + gt) * 4, a.param_dtype, w);
+    }
+    granule<T>(sx + at + (MG + k) * BLOCK * E, dy);
+    wdy[0] = __fmul2_rn(make_float2(w[0], w[1]), dy[0]), wdy[1] = __fmul2_rn(make_float2(w[2], w[3]), dy[1]);
+  };
+  int turn = 0, at = 0;
+  int64_t row = (int64_t)blockIdx.x * RPC + slot;  // the same for all threads of a group, and a group of more than a warp is the CTA
+  if (ST == 2) issue(row, 0);
+  for (; row < a.rows; row += step) {
+    if (ST == 2) {
+      issue(row + step, at ^ stage_bytes);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      issue(row, 0);
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    float2 s[MG][2], wdyh[MH][2];
+    float2 m2 = zero, e2 = zero;
 #pragma unroll
-        for (int i = 0; i < V; ++i) dy[c][i] = 0.f;
+    for (int k = 0; k < MG; ++k) {
+      s[k][0] = s[k][1] = zero;
+      if (HOLD) wdyh[HOLD ? k : 0][0] = wdyh[HOLD ? k : 0][1] = zero;
+      if (k < FULL || k * G + gt < ngran) {
+        granule<T>(sx + at + k * BLOCK * E, s[k]);
+        if (has_r) {
+          float2 r[2];
+          granule_dyn(sr + at + k * BLOCK * re, rtype, r);
+          s[k][0] = __fadd2_rn(s[k][0], r[0]), s[k][1] = __fadd2_rn(s[k][1], r[1]);
+        }
+        if (HOLD || !a.is_rms) {
+          float2 wdy[2];
+          load_wdy(k, at, wdy);
+          m2 = __fadd2_rn(m2, __fadd2_rn(s[k][0], s[k][1])), e2 = __fadd2_rn(e2, __fadd2_rn(wdy[0], wdy[1]));
+          if (HOLD) wdyh[HOLD ? k : 0][0] = wdy[0], wdyh[HOLD ? k : 0][1] = wdy[1];
+        }
       }
     }
     float mean = 0.f, c2 = 0.f;
     if (!a.is_rms) {
-#pragma unroll
-      for (int c = 0; c < MC; ++c) {
-        float wv[V];
-        load_w(c, wv);
-#pragma unroll
-        for (int i = 0; i < V; ++i) mean += s[c][i], c2 = fmaf(dy[c][i], wv[i], c2);
-      }
+      mean = m2.x + m2.y, c2 = e2.x + e2.y;
       group_allsum2<G>(mean, c2, scratch, turn);
       mean *= inv, c2 *= inv;
     }
-    float q = 0.f, c1 = 0.f;
+    const float2 nmean = make_float2(-mean, -mean);
+    float2 q2 = zero, d2 = zero;
 #pragma unroll
-    for (int c = 0; c < MC; ++c) {
-      float wv[V];
-      load_w(c, wv);
-      if (c * G + gt < nchunk) {
+    for (int k = 0; k < MG; ++k) {
+      if (k < FULL || k * G + gt < ngran) {
+        float2 wdy[2];
+        if (!HOLD) load_wdy(k, at, wdy);
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          s[c][i] -= mean;
-          q = fmaf(s[c][i], s[c][i], q);
-          c1 = fmaf(dy[c][i] * wv[i], s[c][i], c1);
+        for (int i = 0; i < 2; ++i) {
+          s[k][i] = __fadd2_rn(s[k][i], nmean);
+          q2 = __ffma2_rn(s[k][i], s[k][i], q2);
+          d2 = __ffma2_rn(HOLD ? wdyh[HOLD ? k : 0][i] : wdy[i], s[k][i], d2);
         }
       }
     }
+    float q = q2.x + q2.y, c1 = d2.x + d2.y;
     group_allsum2<G>(q, c1, scratch, turn);
     const float rstd = rsqrtf(q * inv + a.eps);
-    c1 *= inv * rstd;
+    // ds = rstd (w dy - xhat c1 - c2), xhat = rstd (s - mean), c1 = mean of w dy xhat, c2 = mean of w dy
+    const float sc = -(c1 * inv * rstd) * rstd * rstd, off = -c2 * rstd;
+    const float2 rs = make_float2(rstd, rstd), sc2 = make_float2(sc, sc), off2 = make_float2(off, off);
+    const int64_t col = row * a.hidden + gt * 4;
 #pragma unroll
-    for (int c = 0; c < MC; ++c) {
-      const int ch = c * G + gt;
-      if (live && ch < nchunk) {
+    for (int k = 0; k < MG; ++k) {
+      if (k < FULL || k * G + gt < ngran) {
+        float2 dy[2], wdyl[2], ds[2];
+        granule<T>(sx + at + (MG + k) * BLOCK * E, dy);
+        if (!HOLD) load_wdy(k, at, wdyl);
 #pragma unroll
-        for (int i = 0; i < V; ++i) s[c][i] *= rstd;  // xhat
-        if constexpr (kSmemAcc) {
-#pragma unroll
-          for (int k = 0; k < V / 4; ++k) {
-            float4* pw = acc + (c * (V / 4) + k) * G + gt;
-            float4* pb = pw + kAccRow;
-            float4 w4 = *pw, b4 = *pb;
-            const float *d = &dy[c][4 * k], *x = &s[c][4 * k];
-            w4.x = fmaf(d[0], x[0], w4.x), w4.y = fmaf(d[1], x[1], w4.y), w4.z = fmaf(d[2], x[2], w4.z), w4.w = fmaf(d[3], x[3], w4.w);
-            b4.x += d[0], b4.y += d[1], b4.z += d[2], b4.w += d[3];
-            *pw = w4;
-            if (g.dbias) *pb = b4;
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < V; ++i) dw[c][i] = fmaf(dy[c][i], s[c][i], dw[c][i]), db[c][i] += dy[c][i];
+        for (int i = 0; i < 2; ++i) {
+          dw[k][i] = __ffma2_rn(dy[i], __fmul2_rn(s[k][i], rs), dw[k][i]);
+          db[k][i] = __fadd2_rn(db[k][i], dy[i]);
+          ds[i] = __ffma2_rn(s[k][i], sc2, __ffma2_rn(HOLD ? wdyh[HOLD ? k : 0][i] : wdyl[i], rs, off2));
         }
-        float dsv[V], wv[V];
-        load_w(c, wv);
+        if (has_g) {  // the gradient arriving through the x + residual output reaches x and residual unchanged
+          float2 ga[2];
+          granule_dyn(sg + at + k * BLOCK * ge, gtype, ga);
 #pragma unroll
-        for (int i = 0; i < V; ++i) dsv[i] = (dy[c][i] * wv[i] - s[c][i] * c1 - c2) * rstd;
-        const int64_t off = row * a.hidden + (int64_t)ch * V;
-        if (g.dresidual_out) {  // gradient arriving through the x + residual output reaches x and residual unchanged
-#pragma unroll
-          for (int i = 0; i < V; ++i) dsv[i] += r[c][i], dy[c][i] += r[c][i];
+          for (int i = 0; i < 2; ++i) ds[i] = __fadd2_rn(ds[i], ga[i]), dy[i] = __fadd2_rn(dy[i], ga[i]);
         }
-        Vec16<T> v;
-        v.pack(dsv);
-        v.store_stream(reinterpret_cast<T*>(g.dx) + off);
-        if (g.dresidual) {
-          if (a.prenorm) store_dyn_vec<V>(g.dresidual, off, a.res_dtype, dsv);
-          else store_dyn_vec<V>(g.dresidual, off, a.res_dtype, dy[c]);
+        granule_store(reinterpret_cast<T*>(g.dx) + col + k * G * 4, ds);
+        if (STREAM || g.dresidual) {
+          if (STREAM || a.prenorm) granule_store_dyn(g.dresidual, col + k * G * 4, rtype, ds);
+          else granule_store_dyn(g.dresidual, col + k * G * 4, rtype, dy);
         }
       }
     }
+    if (ST == 2) at ^= stage_bytes;
   }
-  // fold the RPC row slots of this CTA, then write the CTA's partial rows
-  if constexpr (Cfg::RPC > 1) __syncthreads();
+  // fold the RPC row slots of this CTA (over the ring), then write the CTA's partial rows
+  float4* const acc = reinterpret_cast<float4*>(norm_ring);
+  if constexpr (RPC > 1) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < MG; ++k) {
+      acc[(2 * k) * BLOCK + tid] = make_float4(dw[k][0].x, dw[k][0].y, dw[k][1].x, dw[k][1].y);
+      acc[(2 * k + 1) * BLOCK + tid] = make_float4(db[k][0].x, db[k][0].y, db[k][1].x, db[k][1].y);
+    }
+    __syncthreads();
+  }
   if (slot == 0) {
-    float* pw = g.partial + (int64_t)blockIdx.x * 2 * a.hidden;
-    float* pb = pw + a.hidden;
+    float* pw = g.partial + (int64_t)blockIdx.x * 2 * a.hidden + gt * 4;
 #pragma unroll
-    for (int c = 0; c < MC; ++c) {
-      const int ch = c * G + gt;
-      if (ch < nchunk) {
+    for (int k = 0; k < MG; ++k) {
+      if (k < FULL || k * G + gt < ngran) {
+        float4 tw = make_float4(dw[k][0].x, dw[k][0].y, dw[k][1].x, dw[k][1].y);
+        float4 tb = make_float4(db[k][0].x, db[k][0].y, db[k][1].x, db[k][1].y);
+        if constexpr (RPC > 1) {
 #pragma unroll
-        for (int k = 0; k < V / 4; ++k) {
-          float4 tw, tb;
-          if constexpr (kSmemAcc) {
-            tw = tb = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int q = 0; q < Cfg::RPC; ++q) {
-              const float4 x = acc_all[q * 2 * kAccRow + (c * (V / 4) + k) * G + gt], y = acc_all[(q * 2 + 1) * kAccRow + (c * (V / 4) + k) * G + gt];
-              tw.x += x.x, tw.y += x.y, tw.z += x.z, tw.w += x.w;
-              tb.x += y.x, tb.y += y.y, tb.z += y.z, tb.w += y.w;
-            }
-          } else {
-            tw = make_float4(dw[c][4 * k], dw[c][4 * k + 1], dw[c][4 * k + 2], dw[c][4 * k + 3]);
-            tb = make_float4(db[c][4 * k], db[c][4 * k + 1], db[c][4 * k + 2], db[c][4 * k + 3]);
+          for (int o = 1; o < RPC; ++o) {
+            const float4 x = acc[(2 * k) * BLOCK + o * G + gt], y = acc[(2 * k + 1) * BLOCK + o * G + gt];
+            tw.x += x.x, tw.y += x.y, tw.z += x.z, tw.w += x.w;
+            tb.x += y.x, tb.y += y.y, tb.z += y.z, tb.w += y.w;
           }
-          *reinterpret_cast<float4*>(pw + ch * V + 4 * k) = tw;
-          *reinterpret_cast<float4*>(pb + ch * V + 4 * k) = tb;
         }
+        *reinterpret_cast<float4*>(pw + k * G * 4) = tw;
+        *reinterpret_cast<float4*>(pw + a.hidden + k * G * 4) = tb;
       }
     }
   }
@@ -503,24 +569,21 @@ __global__ void __launch_bounds__(32 * kFoldLanes) norm_fold_kernel(const float*
                                                                    void* __restrict__ dweight, void* __restrict__ dbias, int dtype) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float sw[kFoldLanes][33], sb[kFoldLanes][33];
+  __shared__ float sums[kFoldLanes][33];
   const int cx = threadIdx.x & 31, ky = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + cx;
-  float tw = 0.f, tb = 0.f;
+  const float* __restrict__ p = partial + blockIdx.y * hidden + col;  // y: 0 the weight's gradient, 1 the bias's
+  float t = 0.f;
   if (col < hidden) {
-#pragma unroll 4
-    for (int k = ky; k < nctas; k += kFoldLanes) {
-      tw += __ldg(partial + (int64_t)k * 2 * hidden + col);
-      tb += __ldg(partial + (int64_t)k * 2 * hidden + hidden + col);
-    }
+#pragma unroll 8
+    for (int k = ky; k < nctas; k += kFoldLanes) t += __ldg(p + (int64_t)k * 2 * hidden);
   }
-  sw[ky][cx] = tw, sb[ky][cx] = tb;
+  sums[ky][cx] = t;
   __syncthreads();
   if (ky == 0 && col < hidden) {
 #pragma unroll
-    for (int k = 1; k < kFoldLanes; ++k) tw += sw[k][cx], tb += sb[k][cx];
-    store_dyn(dweight, col, dtype, tw);
-    if (dbias) store_dyn(dbias, col, dtype, tb);
+    for (int k = 1; k < kFoldLanes; ++k) t += sums[k][cx];
+    store_dyn(blockIdx.y ? dbias : dweight, col, dtype, t);
   }
 }
 
@@ -627,39 +690,58 @@ static int norm_fwd_launch(const ssm_norm_args& a, cudaStream_t st) {
   return launch_overlapped("norm_fwd_kernel", a.residual ? norm_fwd_kernel<T, G, MC, true> : norm_fwd_kernel<T, G, MC, false>, dim3(grid), dim3(Cfg::BLOCK), 0, st, a);
 }
 static int norm_fold(const ssm_norm_bwd_args& g, int parts, cudaStream_t st) {
-  return launch_overlapped("norm_fold_kernel", norm_fold_kernel, dim3((g.fwd.hidden + 31) / 32), dim3(32 * kFoldLanes), 0, st, g.partial, parts, g.fwd.hidden, g.dweight, g.dbias,
+  return launch_overlapped("norm_fold_kernel", norm_fold_kernel, dim3((g.fwd.hidden + 31) / 32, g.dbias ? 2 : 1), dim3(32 * kFoldLanes), 0, st, g.partial, parts, g.fwd.hidden, g.dweight, g.dbias,
                            g.fwd.dparam_dtype);
 }
-template <typename T, int G, int MC>
-static int norm_bwd_launch(const ssm_norm_bwd_args& g, cudaStream_t st, int max_ctas = kNormBwdMaxCtas) {
+constexpr size_t kNormRing = 200 * 1024;
+template <typename T, int G, int MG, int FULL>
+static int norm_bwd_launch(const ssm_norm_bwd_args& g, cudaStream_t st, int max_ctas) {
   using Cfg = NormCfg<T, G>;
+  const ssm_norm_args& a = g.fwd;
+  const int element = 2 * (int)sizeof(T) + (a.residual && a.prenorm ? dtype_bytes(a.res_dtype) : 0) + (g.dresidual_out ? dtype_bytes(a.resout_dtype) : 0);
+  const size_t stage = (size_t)MG * 4 * Cfg::BLOCK * element, fold = Cfg::RPC > 1 ? (size_t)MG * Cfg::BLOCK * 32 : 0;
+  const bool two = 2 * stage <= kNormRing;  // else (512 threads of the most granules) one row at a time
+  const size_t smem = std::max(two ? 2 * stage : stage, fold);
+  constexpr int ONE = G == 512 && MG * sizeof(T) == 16 ? 1 : 2;
+  // the middle of a network: a residual stream of fp32, in and out
+  const bool stream = a.prenorm && a.residual && g.dresidual && g.dresidual_out && a.res_dtype == SSM_F32 && a.resout_dtype == SSM_F32;
+  auto kern = stream ? (two ? norm_bwd_kernel<T, G, MG, FULL, 2, true> : norm_bwd_kernel<T, G, MG, FULL, ONE, true>)
+                     : (two ? norm_bwd_kernel<T, G, MG, FULL, 2, false> : norm_bwd_kernel<T, G, MG, FULL, ONE, false>);
+  static_assert(ONE == 1 || 2 * MG * 4 * Cfg::BLOCK * (2 * sizeof(T) + 8) <= kNormRing, "two rows fit");
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   // persistent grid: exactly one resident wave (a second, partial wave would double the time)
-  static const int resident = [] {
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, norm_bwd_kernel<T, G, MC>, Cfg::BLOCK, 0);
-    return (per_sm < 1 ? 1 : per_sm) * sm_count();
-  }();
-  int nctas = norm_bwd_ctas(g.fwd, Cfg::RPC);
-  if (nctas > max_ctas) nctas = max_ctas;
-  if (nctas > resident) nctas = resident;
-  if (int rc = launch_overlapped("norm_bwd_kernel", norm_bwd_kernel<T, G, MC>, dim3(nctas), dim3(Cfg::BLOCK), 0, st, g)) return rc;
+  const int resident = std::min<int>(norm_bwd_ctas_per_sm<T, G, MG>(), (int)(228 * 1024 / (smem + 2048))) * sm_count();
+  const int nctas = std::min(std::min(norm_bwd_ctas(a, Cfg::RPC), max_ctas), resident);
+  if (int rc = launch_overlapped("norm_bwd_kernel", kern, dim3(nctas), dim3(Cfg::BLOCK), smem, st, g)) return rc;
   return norm_fold(g, nctas, st);
 }
 
-// rows of up to 128 chunks go to one warp each (1 .. 4 chunks per lane), wider ones to 128 or 512 threads
+// As few granules of four columns per thread as the row needs: what a thread does not hold leaves room for more rows in flight
+// (2560 columns of 16 bits: five, three CTAs per SM), and the number of them that all threads have (FULL) is known.  A warp owns a row while its lanes can hold it.
 template <typename T>
 static int norm_bwd_dispatch(const ssm_norm_bwd_args& g, cudaStream_t st, int max_ctas) {
-  const int V = 16 / (int)sizeof(T);
-  const int nchunk = g.fwd.hidden / V;
-  if (nchunk <= 32) return norm_bwd_launch<T, 32, 1>(g, st, max_ctas);
-  if (nchunk <= 64) return norm_bwd_launch<T, 32, 2>(g, st, max_ctas);
-  if (nchunk <= 96) return norm_bwd_launch<T, 32, 3>(g, st, max_ctas);
-  if (nchunk <= 128) return norm_bwd_launch<T, 32, 4>(g, st, max_ctas);
-  if (nchunk <= 256) return norm_bwd_launch<T, 128, 2>(g, st, max_ctas);
-  if (nchunk <= 384) return norm_bwd_launch<T, 128, 3>(g, st, max_ctas);  // e.g. 2560 columns of 16 bits: three CTAs per SM, not two
-  if (nchunk <= 512) return norm_bwd_launch<T, 128, 4>(g, st, max_ctas);
-  if (nchunk <= 1024) return norm_bwd_launch<T, 512, 2>(g, st, max_ctas);
-  return norm_bwd_launch<T, 512, 4>(g, st, max_ctas);
+  const int n = g.fwd.hidden / 4;
+  if (n <= 32) return norm_bwd_launch<T, 32, 1, 0>(g, st, max_ctas);
+  if (n <= 64) return norm_bwd_launch<T, 32, 2, 1>(g, st, max_ctas);
+  if (n <= 96) return norm_bwd_launch<T, 32, 3, 2>(g, st, max_ctas);
+  if (n <= 128) return norm_bwd_launch<T, 32, 4, 3>(g, st, max_ctas);
+  if constexpr (sizeof(T) == 4) {
+    if (n <= 256) return norm_bwd_launch<T, 128, 2, 1>(g, st, max_ctas);
+    if (n <= 384) return norm_bwd_launch<T, 128, 3, 2>(g, st, max_ctas);
+    if (n <= 512) return norm_bwd_launch<T, 128, 4, 3>(g, st, max_ctas);
+    if (n <= 1024) return norm_bwd_launch<T, 512, 2, 1>(g, st, max_ctas);
+    return norm_bwd_launch<T, 512, 4, 2>(g, st, max_ctas);
+  } else {
+    if (n <= 192) return norm_bwd_launch<T, 32, 6, 4>(g, st, max_ctas);
+    if (n <= 256) return norm_bwd_launch<T, 32, 8, 6>(g, st, max_ctas);
+    if (n <= 384) return norm_bwd_launch<T, 128, 3, 2>(g, st, max_ctas);
+    if (n <= 512) return norm_bwd_launch<T, 128, 4, 3>(g, st, max_ctas);
+    if (n <= 640) return norm_bwd_launch<T, 128, 5, 4>(g, st, max_ctas);
+    if (n <= 768) return norm_bwd_launch<T, 128, 6, 5>(g, st, max_ctas);
+    if (n <= 1024) return norm_bwd_launch<T, 128, 8, 6>(g, st, max_ctas);
+    if (n <= 2048) return norm_bwd_launch<T, 512, 4, 2>(g, st, max_ctas);
+    return norm_bwd_launch<T, 512, 8, 4>(g, st, max_ctas);
+  }
 }
 
 template <typename T>

@@ -304,12 +304,14 @@ __device__ __forceinline__ void group_allsum2(float& a, float& b, float2 (*scrat
     b += __shfl_xor_sync(0xffffffffu, b, off);
   }
   if constexpr (G > 32) {
+    const int first = G == 64 ? threadIdx.x >> 6 << 1 : 0;  // two groups of two warps to a CTA, each with a barrier of its own
     if ((threadIdx.x & 31) == 0) scratch[turn][threadIdx.x >> 5] = make_float2(a, b);
-    __syncthreads();
+    if constexpr (G == 64) asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (first >> 1)) : "memory");
+    else __syncthreads();
     a = 0.f, b = 0.f;
 #pragma unroll
     for (int w = 0; w < G / 32; ++w) {
-      const float2 v = scratch[turn][w];
+      const float2 v = scratch[turn][first + w];
       a += v.x, b += v.y;
     }
     turn ^= 1;
@@ -322,7 +324,8 @@ __device__ __forceinline__ void group_allsum2(float& a, float& b, float2 (*scrat
 // memory: each thread copies its own granules of x, dy, the residual and the gradient arriving through the x + residual output
 // (asynchronous copies, no barrier) and has its next row under way while it works on this one.  What a row still needs at its end is
 // read there again, which leaves the registers to the running weight / bias gradients of the thread's columns.  Packed fp32 arithmetic.
-//  * A row of up to 32 * 8 granules (fp32: 32 * 4) is owned by ONE warp (G = 32), four rows to a CTA; wider rows take 128 or 512 threads.
+//  * A row of up to 32 * 4 granules is owned by ONE warp (G = 32), four rows to a CTA; wider rows take 64 to 512 threads, four granules
+//    each if they can (eight leave no room for what a row keeps in registers: 4096 bf16 columns, fp32 residual, 336 us; four of 256 threads: 173).
 //  * Two rounds of sums, two values each: {sum s, sum w dy}, then {sum (s - mean)^2, sum w dy (s - mean)}, from which the standard
 //    deviation and both correction terms follow (one round for RMSNorm).
 // 16376 rows of 1600 bf16 columns, fp32 residual and its gradient, 471 MB: 104 us with the loads in registers, scalar arithmetic and 16
@@ -331,7 +334,7 @@ __device__ __forceinline__ void group_allsum2(float& a, float& b, float2 (*scrat
 //    and every granule guarded the loads of a row could not be put together (54 instructions per element, 104 us).
 template <typename T, int G, int MG>
 constexpr int norm_bwd_ctas_per_sm() {
-  if (G > 128) return 1;
+  if (G > 128) return G == 256 ? 2 : 1;
   return MG <= 4 ? 4 : (MG <= 6 ? 3 : 2);
 }
 __host__ __device__ constexpr int dtype_bytes(int dtype) { return dtype == SSM_F32 ? 4 : 2; }
@@ -383,7 +386,7 @@ __global__ void __launch_bounds__(NormCfg<T, G>::BLOCK, norm_bwd_ctas_per_sm<T, 
   pdl_trigger();
   using Cfg = NormCfg<T, G>;
   constexpr int BLOCK = Cfg::BLOCK, RPC = Cfg::RPC, E = 4 * (int)sizeof(T);
-  constexpr bool HOLD = G == 32 || MG <= 6;  // w dy stays in registers between the rounds of sums
+  constexpr bool HOLD = MG <= 6;  // w dy stays in registers between the rounds of sums
   constexpr bool HOLD_W = MG <= 4;      // the weights of the thread's columns too
   constexpr int MH = HOLD ? MG : 1, MW = HOLD_W ? MG : 1;
   const ssm_norm_args& a = g.fwd;
@@ -732,13 +735,13 @@ static int norm_bwd_dispatch(const ssm_norm_bwd_args& g, cudaStream_t st, int ma
     if (n <= 1024) return norm_bwd_launch<T, 512, 2, 1>(g, st, max_ctas);
     return norm_bwd_launch<T, 512, 4, 2>(g, st, max_ctas);
   } else {
-    if (n <= 192) return norm_bwd_launch<T, 32, 6, 4>(g, st, max_ctas);
-    if (n <= 256) return norm_bwd_launch<T, 32, 8, 6>(g, st, max_ctas);
+    if (n <= 192) return norm_bwd_launch<T, 64, 3, 2>(g, st, max_ctas);
+    if (n <= 256) return norm_bwd_launch<T, 64, 4, 3>(g, st, max_ctas);
     if (n <= 384) return norm_bwd_launch<T, 128, 3, 2>(g, st, max_ctas);
     if (n <= 512) return norm_bwd_launch<T, 128, 4, 3>(g, st, max_ctas);
     if (n <= 640) return norm_bwd_launch<T, 128, 5, 4>(g, st, max_ctas);
     if (n <= 768) return norm_bwd_launch<T, 128, 6, 5>(g, st, max_ctas);
-    if (n <= 1024) return norm_bwd_launch<T, 128, 8, 6>(g, st, max_ctas);
+    if (n <= 1024) return norm_bwd_launch<T, 256, 4, 3>(g, st, max_ctas);
     if (n <= 2048) return norm_bwd_launch<T, 512, 4, 2>(g, st, max_ctas);
     return norm_bwd_launch<T, 512, 8, 4>(g, st, max_ctas);
   }

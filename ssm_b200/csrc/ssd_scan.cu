@@ -15,8 +15,8 @@
 //   ssd_scan_kernel     per (batch, chunk, 128-row block, part of a head group):  G = C B^T once (TMEM -> registers), then per
 //                       head the decay mask exp2(c_i - c_j) delta_j [j <= i] (+ D on the diagonal) written back to TMEM
 //                       (tcgen05.st) as the A operand of Y_intra = (G o L) X, plus  Y_inter = C S_in;
-//                       y = Y_intra + exp2(c_i) Y_inter, gated, stored by TMA.  Sixteen warps form masks and epilogues; an
-//                       elected lane of the warp with the least mask work issues the MMAs, one thread the copies.
+//                       y = Y_intra + exp2(c_i) Y_inter, gated, stored by TMA.  Sixteen warps form masks and epilogues, one
+//                       issues the MMAs and the copies.
 //
 // Exponent differences are always formed before exp2 (never exp2(c_i) / exp2(c_j)), so long
 // sequences stay finite.  Every wait on an mbarrier is bounded and reports through the status word.
@@ -533,10 +533,17 @@ __global__ void __launch_bounds__(256) ssd_fold_init_kernel(const ssm_ssd_args a
 //              operand (in tensor memory, over the dead G columns);  Y_intra = (G o L) X  and
 //              Y_inter = C_m S_in accumulate in TMEM while the previous head's result is read
 //              back, gated and staged.
-//   Copies (TMA and bulk copies issued by one thread) run one head ahead into the other half of a
-//   double buffer: x, the incoming state, the exponent vectors; z has two buffers of its own over
-//   the dead B tile; y is staged in a 16 KB tile and leaves by a TMA store.
-//   TMEM columns: G [0,256); per buffer b: Y_intra [256+128b, +64), Y_inter [320+128b, +64).
+//   Copies (TMA and bulk copies issued by one warp, the MMAs too) run one head ahead into the other half of a
+//   double buffer: x, the incoming state, the exponent vectors; z and the y that leaves by a TMA store have two
+//   tiles each over the dead B tile.
+//   TMEM columns: G [0,256), later the masked operands of two heads [128b, +128); per buffer b: Y_intra [256+128b, +64),
+//   Y_inter [320+128b, +64).
+// No CTA-wide barrier per head: the warps pass mbarriers (operands landed, operand written, MMAs done, epilogue done, y read), so
+// that one warp's mask runs beside another's epilogue.  Before, two CTA-wide barriers per head kept the warps in step, the cut on the
+// diagonal cost its four warps 128 compares and adds a head, and all waited for them.  8 x 8192 steps of 48 heads, gate and D: 390 us,
+// now 347; 24 packed sequences in 16384 steps 125, now 107; 2 x 4001 steps 63, now 56.5, adjoint 62.5, now 57.
+// Tried: column factors formed once per CTA by idle warps (353, 113, 57); operands two heads ahead with y stored from registers in sectors of
+// 32 bytes (401, 103, 76: the row-strided stores); the issuing done by a seventeenth warp without the register split (spills).
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 struct ScanSmem {
@@ -545,14 +552,20 @@ struct ScanSmem {
   static constexpr int X_BYTES = kQ * kP * 2;       // x rows [j][64 p], 128-byte rows, TMA 128-byte swizzle  32 KB (x2)
   static constexpr int S_BYTES = kP * kN * 2;       // incoming state, MN-major [p/8][n][8]                 16 KB (x2)
   static constexpr int VEC_BYTES = 2 * kQ * 4;      // c and c - log2(delta) of the chunk                     2 KB (x2)
-  static constexpr int Z_BYTES = kBlk * kP * 2;     // y of one head on its way out: [row][64 p], same swizzle  16 KB
+  static constexpr int Z_BYTES = kBlk * kP * 2;     // gate rows of a head, or y on its way out: [row][64 p], same swizzle; 4 x 16 KB over the B tile
+  static_assert(4 * Z_BYTES <= B_BYTES, "two gate tiles and two of y fit over the B tile");
   static constexpr int W_BYTES = 1024 * 4;          // per warp: the column factors of its mask chunks (16 warps x 64)          4 KB
-  static constexpr int TOTAL = C_BYTES + B_BYTES + 2 * (X_BYTES + S_BYTES + VEC_BYTES) + Z_BYTES + W_BYTES;
+  static constexpr int TOTAL = C_BYTES + B_BYTES + 2 * (X_BYTES + S_BYTES + VEC_BYTES) + W_BYTES;
   static constexpr int ALLOC = TOTAL + 1024;        // the tiles TMA swizzles must start on 1024-byte boundaries
 };
 
-constexpr int kScanThreads = 512;
-constexpr int kScanWG = kScanThreads / 128;  // warpgroups: each owns every kScanWG-th 32-step column chunk of the mask and kP / kScanWG output columns
+constexpr int kScanCompute = 512;                // threads of the mask and the epilogue
+// ... and a warpgroup whose first warp issues the copies and the MMAs.  Launched with 96 registers a thread (640 x 96 = 61440): the
+// issuing group keeps 32, the others take 112 (128 x 32 + 512 x 112 = 61440).
+constexpr int kScanThreads = kScanCompute + 128;
+constexpr int kScanIssueRegs = 32, kScanComputeRegs = 112;
+static_assert(128 * kScanIssueRegs + kScanCompute * kScanComputeRegs <= kScanThreads * 96, "the split draws on what the block was launched with");
+constexpr int kScanWG = kScanCompute / 128;  // warpgroups: each owns every kScanWG-th 32-step column chunk of the mask and kP / kScanWG output columns
 constexpr int kEC = kP / kScanWG;             // epilogue columns per thread
 constexpr int kEU = kEC / 8;                  // ... in 16-byte units
 // tensor maps of one call: x (box of 128 or 256 steps), z and y (boxes of 128 rows); rank 4 (p, head, step, batch)
@@ -580,28 +593,28 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   constexpr int ROW0 = (REV ? 1 - MB : MB) * kBlk;  // first row and first column of the block within the chunk
   constexpr int COL0 = REV ? ROW0 : 0;
   constexpr int VLEN = REV ? kQ : KJ;               // exponents of the chunk that are needed
-  constexpr int kCopyThread = REV ? 224 : 128;      // lane 0 of a warp with little mask work (fewest unmasked columns)
-  constexpr int kMmaWarp = REV ? 3 : 12;
   unsigned char* sC = smraw;
   unsigned char* sBA = sC + M::C_BYTES;
   unsigned char* sX = sBA + M::B_BYTES;        // two buffers
   unsigned char* sS = sX + 2 * M::X_BYTES;     // two buffers
   float* sVec = reinterpret_cast<float*>(sS + 2 * M::S_BYTES);  // two buffers of [c | c - log2 delta]
-  unsigned char* sZ = reinterpret_cast<unsigned char*>(sVec) + 2 * M::VEC_BYTES;
-  // mbar: 0 G done; 1 + b MMAs of a head into accumulator pair b done; 3 + b operands of buffer b landed; 5, 7 gate tiles landed;
-  // 6 C and B tiles landed
-  const uint32_t mb_g = tc::smem_u32(&mbar[0]);
-  auto mb_z = [&](int bf) { return tc::smem_u32(&mbar[bf ? 7 : 5]); };  // gate tile of buffer bf landed
-  auto mb_mma = [&](int bf) { return tc::smem_u32(&mbar[1 + bf]); };
-  auto mb_full = [&](int bf) { return tc::smem_u32(&mbar[3 + bf]); };
+  // mbar: 0 G done; 1 C and B tiles landed; per buffer b of a head: 2 + b its MMAs done; 4 + b its operands landed; 6 + b masked operand
+  // written; 8 + b epilogue done; 10 + b its y has been read from the staging tile; 12 + b its gate rows landed
+  const uint32_t mb_g = tc::smem_u32(&mbar[0]), mb_cb = tc::smem_u32(&mbar[1]);
+  auto mb_mma = [&](int bf) { return tc::smem_u32(&mbar[2 + bf]); };
+  auto mb_full = [&](int bf) { return tc::smem_u32(&mbar[4 + bf]); };
+  auto mb_mask = [&](int bf) { return tc::smem_u32(&mbar[6 + bf]); };
+  auto mb_epi = [&](int bf) { return tc::smem_u32(&mbar[8 + bf]); };
+  auto mb_out = [&](int bf) { return tc::smem_u32(&mbar[10 + bf]); };
+  auto mb_z = [&](int bf) { return tc::smem_u32(&mbar[12 + bf]); };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wg = tid >> 7;                     // column chunks wg, wg + kScanWG, ... in the mask stage; column slice in the epilogue
-  float* sW = reinterpret_cast<float*>(sZ + M::Z_BYTES) + warp * (NCH * 32);  // this warp's column factors
-  // The gate rows of a head get buffers of their own, over the B tile (dead once G is formed: the masked operand lives in
-  // tensor memory): head h's tile is requested at the top of its own iteration and read by its epilogue one iteration later,
-  // instead of waiting, in the shared staging tile, for the previous head's y to be stored first.
+  float* sW = sVec + 2 * (M::VEC_BYTES / 4) + (warp & 15) * (NCH * 32);  // this warp's column factors
+  // The gate rows of a head and its y on the way out have two buffers each, over the B tile (dead once G is formed: the masked
+  // operand lives in tensor memory).
   auto sZin = [&](int bf) { return sBA + bf * M::Z_BYTES; };
+  auto sY = [&](int bf) { return sBA + (2 + bf) * M::Z_BYTES; };
   const int half_grid = gridDim.x >> 1;
   const int rem = (int)blockIdx.x % half_grid;
   const int part = rem % nparts, bc = rem / nparts;
@@ -624,8 +637,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   const CUtensorMap* mapx = MB ? &maps.x1 : &maps.x0;
 
   // ---- C rows of the block, B rows of the reachable steps, by TMA: per half of the states one block of 128-byte rows
-  const uint32_t mb_cb = tc::smem_u32(&mbar[6]);
-  if (tid == kCopyThread) {
+  if (tid == kScanCompute) {
     tc::mbar_expect_tx(mb_cb, M::C_BYTES + KJ * kN * 2);
 #pragma unroll
     for (int nb2 = 0; nb2 < 2; ++nb2) {
@@ -653,33 +665,128 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   // slot of (row, 16-byte chunk) in a tile of 128-byte rows written / read by TMA with the 128-byte swizzle
   auto swz = [&](unsigned char* tile, int row, int chunk) { return tile + ((size_t)row * 8 + (chunk ^ (row & 7))) * 16; };
 
-  if (tid == kCopyThread) prefetch(h0, 0);
+  if (tid == kScanCompute) prefetch(h0, 0);
 
-  bool ok = __all_sync(0xffffffffu, tc::mbar_wait(mb_cb, 0));  // C and B have landed
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-  const bool mma_warp = __shfl_sync(0xffffffffu, warp, 0) == kMmaWarp;  // the same in every lane, and visibly so
+  const bool issuer = __shfl_sync(0xffffffffu, warp, 0) == kScanCompute / 32;  // the same in every lane, and visibly so
+  auto wait = [&](uint32_t bar, int n) { return (bool)__all_sync(0xffffffffu, tc::mbar_test(bar, n & 1) || tc::mbar_wait(bar, n & 1)); };  // the n-th completion; warp-uniform
+  const int t_blk = t0 + ROW0;  // first step of this block's rows
 
   // ---- G = C_m B^T ------------------------------------------------------------------------------------
   // K-major operands in 128-byte-swizzled rows: 16 states = 32 bytes further along the row, 64 states = the next block
-  if (tid == 0 && ok) {
-    const uint64_t dc0 = tc::smem_desc_sw128(tc::smem_u32(sC), 16, 1024);
-    const uint64_t db0 = tc::smem_desc_sw128(tc::smem_u32(sBA), 16, 1024);
-    constexpr uint32_t idG = tc::instr_desc(kBlk, KJ, fmt, 0, 0);
+  const uint64_t dc0 = tc::smem_desc_sw128(tc::smem_u32(sC), 16, 1024);
+  bool ok = true;
+  if (issuer) {
+    ok = wait(mb_cb, 0);
+    if (ok && tc::elect_one()) {
+      const uint64_t db0 = tc::smem_desc_sw128(tc::smem_u32(sBA), 16, 1024);
+      constexpr uint32_t idG = tc::instr_desc(kBlk, KJ, fmt, 0, 0);
 #pragma unroll
-    for (int kk = 0; kk < kN / 16; ++kk)
-      tc::mma_ss(tmem, dc0 + (uint64_t)(((kk >> 2) * (kBlk * 128) + (kk & 3) * 32) >> 4), db0 + (uint64_t)(((kk >> 2) * (KJ * 128) + (kk & 3) * 32) >> 4), idG,
-                 kk > 0);
-    tc::commit(mb_g);
+      for (int kk = 0; kk < kN / 16; ++kk)
+        tc::mma_ss(tmem, dc0 + (uint64_t)(((kk >> 2) * (kBlk * 128) + (kk & 3) * 32) >> 4), db0 + (uint64_t)(((kk >> 2) * (KJ * 128) + (kk & 3) * 32) >> 4), idG,
+                   kk > 0);
+      tc::commit(mb_g);
+    }
+    __syncwarp();
   }
-  ok = __all_sync(0xffffffffu, ok && tc::mbar_wait(mb_g, 0));  // warp-uniform
+  ok = wait(mb_g, 0) && ok;
   tc::fence_after_sync();
 
+  // ======== copies and MMAs: one warp, which the others never wait for but through what it issues ====================
+  if (wg == kScanWG) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kScanIssueRegs));
+    __syncthreads();  // G has been read: its columns and the B tile are free
+    if (!issuer) return;
+    int fail = ok ? 0 : 1;
+#pragma unroll 1
+    for (int hi = 0; hi < nh && !fail; ++hi) {
+      const int h = h0 + hi, buf = hi & 1;
+      // the other buffer's tiles are free once the MMAs of the head before are done (its exponents were read before those began)
+      if (hi >= 1 && !wait(mb_mma(buf ^ 1), (hi - 1) >> 1)) {
+        fail = 1;
+        break;
+      }
+      if (hi + 1 < nh && lane == 0) prefetch(h + 1, buf ^ 1);
+      __syncwarp();
+      // accumulators, gate tile and staged y of this buffer: the epilogue of the head before last
+      if ((hi >= 2 && !wait(mb_epi(buf), (hi - 2) >> 1)) || !wait(mb_full(buf), hi >> 1)) {
+        fail = 1;
+        break;
+      }
+      tc::fence_after_sync();
+      if (tc::elect_one()) {
+        // Y_inter = C_m S_in needs nothing of the mask: issued first, it runs on the tensor cores while the mask is formed
+        const uint64_t ds0 = tc::smem_desc(tc::smem_u32(sS + buf * M::S_BYTES), 128, kN * 16);
+        constexpr uint32_t idS = tc::instr_desc(kBlk, kP, fmt, 0, 1);
+        const uint32_t dS = tmem + 256 + buf * 128 + 64;
+#pragma unroll
+        for (int kk = 0; kk < kN / 16; ++kk)
+          tc::mma_ss(dS, dc0 + (uint64_t)(((kk >> 2) * (kBlk * 128) + (kk & 3) * 32) >> 4), ds0 + (uint64_t)(kk * (256 >> 4)), idS, kk > 0);
+      }
+      __syncwarp();
+      if (lane == 0) {
+        if (has_z) {
+          tc::mbar_expect_tx(mb_z(buf), M::Z_BYTES);
+          tc::tma_load_4d(tc::smem_u32(sZin(buf)), &maps.z, mb_z(buf), 0, h, t_blk, b);
+        }
+        if (hi >= 2 && !ragged) {
+          tc::tma_store_4d(&maps.y, tc::smem_u32(sY(buf)), 0, h - 2, t_blk, b);
+          tc::bulk_commit();
+        }
+        if (hi + 2 < nh) {  // the tiles of the head after next on their way into the L2: one iteration alone does not cover the latency
+          tc::tma_prefetch_4d(mapx, 0, h + 2, t0 + COL0, b);
+          if (has_z) tc::tma_prefetch_4d(&maps.z, 0, h + 2, t_blk, b);
+          tc::bulk_prefetch(reinterpret_cast<const T*>(a.ws_state_in) + (((int64_t)b * nchunks + c) * a.heads + h + 2) * (int64_t)(kP * kN), M::S_BYTES);
+        }
+      }
+      __syncwarp();
+      if (!wait(mb_mask(buf), hi >> 1)) {
+        fail = 1;
+        break;
+      }
+      tc::fence_after_sync();
+      // ---- Y_intra = (G o L) X  for this head; the commit also covers the Y_inter MMAs issued above
+      if (tc::elect_one()) {
+        // descriptors differ from instruction to instruction only in the start address (16-byte units, low bits)
+        const uint64_t dx0 = tc::smem_desc_sw128(tc::smem_u32(sX + buf * M::X_BYTES), 16, 1024);
+        constexpr uint32_t idY = tc::instr_desc(kBlk, kP, fmt, 0, 1);
+        const uint32_t dY = tmem + 256 + buf * 128, dA = tmem + buf * 128;
+#pragma unroll
+        for (int kk = 0; kk < KJ / 16; ++kk)  // 16 steps = 16 rows of 128 bytes of the x tile
+          tc::mma_ts(dY, dA + kk * 8, dx0 + (uint64_t)(kk * (2048 >> 4)), idY, kk > 0);  // A: 16 steps = 8 columns of the masked rows
+        tc::commit(mb_mma(buf));
+      }
+      __syncwarp();
+      if (hi >= 2 && !ragged && lane == 0) {  // (the store's reads queue behind this iteration's copies: never in front of the MMAs)
+        tc::bulk_wait_read();
+        tc::mbar_arrive(mb_out(buf));
+      }
+      __syncwarp();
+    }
+    for (int hi = max(nh - 2, 0); hi < nh && !fail && !ragged; ++hi) {
+      if (!wait(mb_epi(hi & 1), hi >> 1)) {
+        fail = 1;
+      } else if (lane == 0) {
+        tc::tma_store_4d(&maps.y, tc::smem_u32(sY(hi & 1)), 0, h0 + hi, t_blk, b);
+        tc::bulk_commit();
+      }
+    }
+    if (lane == 0) {
+      tc::bulk_wait_all();  // the staging tiles must outlive the stores that read them
+      if (fail && a.status) *(volatile int32_t*)a.status = 2;
+    }
+    return;
+  }
+
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kScanComputeRegs));
+
   // This thread's part of G stays in registers for all heads: row i_loc, chunks wg, wg + kScanWG, ...
-  float vG[NCH][32];
+  const bool fold_d = !XSKIP && !REV && a.D;  // see below
+  float vG[NCH][32], gdiag = 0.f;
 #pragma unroll
   for (int k = 0; k < NCH; ++k) {
     const int cc = wg + kScanWG * k;
@@ -689,11 +796,20 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
 #pragma unroll
       for (int e = 0; e < 32; ++e) vG[k][e] = 0.f;
     }
+    if (cc == rc) {  // the chunk of this warp's own rows: steps after the row are cut
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        if (e == lane) gdiag = vG[k][e];
+        if (REV ? e < lane : (fold_d ? e >= lane : e > lane)) vG[k][e] = 0.f;
+      }
+    }
   }
+  tc::fence_before_sync();
+  __syncthreads();  // every part of G has been read: the masked operands take its columns, the gate tiles and y the B tile
+  tc::fence_after_sync();
 
   // A skip weight per head (not per channel) rides on the diagonal of the masked operand: (G o L + D I) X = Y_intra + D x.
   // The row sums for the backward pass want y without the skip term, so that mode keeps the explicit form.
-  const bool fold_d = !XSKIP && a.D;
   constexpr bool skip_explicit = XSKIP;
 
   // epilogue of head h from accumulator pair `buf`: y = Y_intra + exp2(c_i) Y_inter (+ D x where it is not folded), gated by
@@ -703,8 +819,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     const float escale = ex2_approx(ct);
     const float2 es2 = make_float2(escale, escale);
     float yi[kEC], ys[kEC];
-    tc::tmem_ld16(tmem + lane_base + 256 + buf * 128 + wg * kEC, yi);
-    tc::tmem_ld16(tmem + lane_base + 320 + buf * 128 + wg * kEC, ys);
+    tc::tmem_ld16_pair(tmem + lane_base + 256 + buf * 128 + wg * kEC, tmem + lane_base + 320 + buf * 128 + wg * kEC, yi, ys);
     const float Dh = (skip_explicit && !a.d_has_p) ? __ldg(a.D + h) : 0.f;
     const bool dots = a.row_dots != nullptr;
     float dot = 0.f;  // row_dots: this thread's 16 columns of  sum_p y[p] z[p]  (y before the skip term and unrounded)
@@ -751,7 +866,7 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
       for (int e = 0; e < 4; ++e) f[2 * e] = f2[e].x, f[2 * e + 1] = f2[e].y;
       Vec16<T> o;
       o.pack(f);
-      *reinterpret_cast<uint4*>(swz(sZ, i_loc, wg * kEU + q)) = o.raw;
+      *reinterpret_cast<uint4*>(swz(sY(buf), i_loc, wg * kEU + q)) = o.raw;
     }
     if (dots && has_z) {
       const int t = t0 + ROW0 + i_loc;
@@ -760,11 +875,10 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
     }
     tc::fence_async_smem();  // the staged rows leave through a bulk store
   };
-  const int t_blk = t0 + ROW0;  // first step of this block's rows
-  auto store_rows = [&](int h) {     // the staged rows of a ragged block, 16 bytes a thread
-    for (int u = tid; u < t_live * 8; u += kScanThreads)
+  auto store_rows = [&](int h, int buf) {  // the staged rows of a ragged block, 16 bytes a thread
+    for (int u = tid; u < t_live * 8; u += kScanCompute)
       *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.Y) + (((int64_t)b * a.len + t_blk + (u >> 3)) * a.heads + h) * kP + (u & 7) * 8) =
-          *reinterpret_cast<const uint4*>(swz(sZ, u >> 3, u & 7));
+          *reinterpret_cast<const uint4*>(swz(sY(buf), u >> 3, u & 7));
   };
 
   float ct_prev = 0.f;   // the previous head's row exponent and x row, carried into its (deferred) epilogue
@@ -772,223 +886,163 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
 #pragma unroll
   for (int q = 0; q < kXR; ++q) xr_prev[q] = make_uint4(0, 0, 0, 0);
   int fail = ok ? 0 : 1;
+  // No CTA-wide barrier in the loop: a warp tells the issuing warp when its rows of the masked operand are written and when its
+  // epilogue is done, and waits only for what it reads next.  With two masked operands a warp's mask needs the MMAs of the head before last,
+  // and its epilogue those of the head before, which have had a whole mask to run.
 #pragma unroll 1
-  for (int hi = 0; hi < nh; ++hi) {
+  for (int hi = 0; hi <= nh && !fail; ++hi) {
     const int h = h0 + hi, buf = hi & 1;
-    ok = !fail && tc::mbar_wait(mb_full(buf), (hi >> 1) & 1);  // this head's operands (no more waiting once a wait ran out)
-    // ---- factors of the decay mask, formed before the CTA-wide barrier below so that their latency (shared-memory reads, ex2,
-    // the exchange of the column factors through sW) overlaps the wait for the slowest warp; the barrier also orders the
-    // writes to sW before the reads of the other lanes
-    const float* vc = sVec + buf * (2 * kQ);
-    const float* vcp = vc + kQ;
-    const float Dfold = fold_d ? __ldg(a.D + h) : 0.f;
-    // exponents of the decay mask, weight = exp2(re - col(j)), and of the carried state's row weight, exp2(ct)
-    float re, ct;
-    if constexpr (REV) {
-      const float next = c + 1 < nchunks ? __ldg(a.ws_cum + (((int64_t)b * a.heads + h) * nchunks + c + 1) * kQ) : 0.f;
-      re = -vcp[i_chunk], ct = vc[kQ - 1] + next + re;
-    } else {
-      re = ct = vc[i_chunk];
-    }
-    auto col = [&](int j) { return REV ? -vc[COL0 + j] : vcp[j]; };
-    // The weight exp2(c_i - c'_j) of a 32-step chunk factors as exp2(c_i - r) * exp2(r - c'_j) with r = c at the
-    // chunk's first step (row factor <= 1 for causal rows, column factor bounded by the decay inside the chunk).
-    // Each lane forms one column factor per chunk, each thread one row factor per chunk: 2 ex2 per 32 elements
-    // instead of 32.  Chunks whose internal decay exceeds 2^60 keep the exact per-element form.
-    float arow[NCH];
-    bool fast[NCH];
-#pragma unroll
-    for (int k = 0; k < NCH; ++k) {
-      const int cc = wg + kScanWG * k;
-      arow[k] = 0.f, fast[k] = false;
-      if (reached(cc)) {
-        const float first = vc[COL0 + cc * 32], r = REV ? -first : first;
-        fast[k] = first - vc[COL0 + cc * 32 + 31] < 60.f;  // same for every lane
-        arow[k] = ex2_approx(re - r);
-        sW[k * 32 + lane] = ex2_approx(r - col(cc * 32 + lane));
-      }
-    }
-    // MMAs of the previous head: the masked tile, the other buffer and its accumulators are free / ready
-    if (hi > 0) ok = tc::mbar_wait(mb_mma(buf ^ 1), ((hi - 1) >> 1) & 1) && ok;
-    tc::fence_after_sync();
-    tc::fence_before_sync();     // the accumulator reads of the previous epilogue precede the MMAs issued below
-    ok = __syncthreads_and(ok);  // the staged y of the head before last is complete; the outcome of the waits is CTA-wide
-    if (!ok) {
-      fail = 1;
-      break;
-    }
-    if (mma_warp && tc::elect_one()) {
-      // Y_inter = C_m S_in needs nothing of the mask: issued first, it runs on the tensor cores while the mask is formed
-      tc::fence_after_sync();
-      const uint64_t dc0 = tc::smem_desc_sw128(tc::smem_u32(sC), 16, 1024);
-      const uint64_t ds0 = tc::smem_desc(tc::smem_u32(sS + buf * M::S_BYTES), 128, kN * 16);
-      constexpr uint32_t idS = tc::instr_desc(kBlk, kP, fmt, 0, 1);
-      const uint32_t dS = tmem + 256 + buf * 128 + 64;
-#pragma unroll
-      for (int kk = 0; kk < kN / 16; ++kk)
-        tc::mma_ss(dS, dc0 + (uint64_t)(((kk >> 2) * (kBlk * 128) + (kk & 3) * 32) >> 4), ds0 + (uint64_t)(kk * (256 >> 4)), idS, kk > 0);
-    }
-    if (tid == kCopyThread) {
-      if (hi + 1 < nh) prefetch(h + 1, buf ^ 1);
-      if (has_z) {  // its buffer was last read by the epilogue of head h - 2, one iteration ago
-        tc::mbar_expect_tx(mb_z(buf), M::Z_BYTES);
-        tc::tma_load_4d(tc::smem_u32(sZin(buf)), &maps.z, mb_z(buf), 0, h, t_blk, b);
-      }
-      if (hi >= 2 && !ragged) {  // staged by the epilogue of the previous iteration; its reads are awaited after the mask, below
-        tc::tma_store_4d(&maps.y, tc::smem_u32(sZ), 0, h - 2, t_blk, b);
-        tc::bulk_commit();
-      }
-      if (hi + 2 < nh) {  // the tiles of the head after next on their way into the L2: one iteration alone does not cover the latency
-        tc::tma_prefetch_4d(mapx, 0, h + 2, t0 + COL0, b);
-        if (has_z) tc::tma_prefetch_4d(&maps.z, 0, h + 2, t_blk, b);
-        tc::bulk_prefetch(reinterpret_cast<const T*>(a.ws_state_in) + (((int64_t)b * nchunks + c) * a.heads + h + 2) * (int64_t)(kP * kN), M::S_BYTES);
-      }
-    }
-
-    if (ragged && hi >= 2) store_rows(h - 2);  // read before the mid-iteration barrier, overwritten after it
-    // ---- decay mask: G (registers) x the factors formed above -> the A operand in tensor memory
-#pragma unroll
-    for (int k = 0; k < NCH; ++k) {
-      const int cc = wg + kScanWG * k;  // chunk of 32 steps: whole, diagonal (cc == rc) or empty for this warp's rows
-      const int jb = cc * 32;
-      // the masked row goes to tensor memory as the A operand: 32 steps = 16 columns of two 16-bit values
-      const uint32_t dst = tmem + lane_base + cc * 16;
-      uint32_t packed[16];
-      if (!reached(cc)) {
-#pragma unroll
-        for (int q = 0; q < 16; ++q) packed[q] = 0u;
-        tc::tmem_st16(dst, packed);
-        continue;
-      }
-      const bool diag = cc == rc;
-      if (fast[k] && !diag) {  // the common case: every step of the chunk precedes every row of this warp, nothing to cut
-        const float2 a2 = make_float2(arow[k], arow[k]);
-#pragma unroll
-        for (int q = 0; q < 32; q += 8) {
-          const float4 b0 = *reinterpret_cast<const float4*>(sW + k * 32 + q);
-          const float4 b1 = *reinterpret_cast<const float4*>(sW + k * 32 + q + 4);
-          const float2 bp[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
-          float f[8];
-#pragma unroll
-          for (int e = 0; e < 8; e += 2) {
-            const float2 w = __fmul2_rn(__fmul2_rn(make_float2(vG[k][q + e], vG[k][q + e + 1]), bp[e / 2]), a2);
-            f[e] = w.x, f[e + 1] = w.y;
-          }
-          Vec16<T> o;
-          o.pack(f);
-          packed[q / 2] = o.raw.x, packed[q / 2 + 1] = o.raw.y, packed[q / 2 + 2] = o.raw.z, packed[q / 2 + 3] = o.raw.w;
-        }
-      } else if (fast[k]) {  // the chunk of this warp's own rows: steps after the row are cut
-        const float2 a2 = make_float2(arow[k], arow[k]);
-#pragma unroll
-        for (int q = 0; q < 32; q += 8) {
-          const float4 b0 = *reinterpret_cast<const float4*>(sW + k * 32 + q);
-          const float4 b1 = *reinterpret_cast<const float4*>(sW + k * 32 + q + 4);
-          const float2 bp[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
-          float f[8];
-#pragma unroll
-          for (int e = 0; e < 8; e += 2) {
-            float2 w = __fmul2_rn(__fmul2_rn(make_float2(vG[k][q + e], vG[k][q + e + 1]), bp[e / 2]), a2);
-            if (REV ? q + e < lane : q + e > lane) w.x = 0.f;
-            if (REV ? q + e + 1 < lane : q + e + 1 > lane) w.y = 0.f;
-            if (!REV && q + e == lane) w.x += Dfold;
-            if (!REV && q + e + 1 == lane) w.y += Dfold;
-            f[e] = w.x, f[e + 1] = w.y;
-          }
-          Vec16<T> o;
-          o.pack(f);
-          packed[q / 2] = o.raw.x, packed[q / 2 + 1] = o.raw.y, packed[q / 2 + 2] = o.raw.z, packed[q / 2 + 3] = o.raw.w;
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 32; q += 8) {
-          float f[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            f[e] = vG[k][q + e] * ex2_approx(re - col(jb + q + e));
-            if (diag && (REV ? q + e < lane : q + e > lane)) f[e] = 0.f;  // after the product: G may be Inf there
-            if (!REV && diag && q + e == lane) f[e] += Dfold;
-          }
-          Vec16<T> o;
-          o.pack(f);
-          packed[q / 2] = o.raw.x, packed[q / 2 + 1] = o.raw.y, packed[q / 2 + 2] = o.raw.z, packed[q / 2 + 3] = o.raw.w;
-        }
-      }
-      tc::tmem_st16(dst, packed);
-    }
-    tc::tmem_wait_st();
-    // this row of x (for D x in the epilogue one iteration later)
+    float ct = 0.f;
     uint4 xr[kXR];
 #pragma unroll
-    for (int q = 0; q < kXR; ++q)
-      xr[q] = XSKIP ? *reinterpret_cast<const uint4*>(swz(sX + buf * M::X_BYTES, i_chunk, wg * kEU + q)) : make_uint4(0, 0, 0, 0);
-
-    if (ragged && (warp == 13 || warp == 14)) {  // x rows of the next sequence, by two of the warps that have had the least mask work
-#pragma unroll 1
-      for (int u = k_live * 8 + tid - 13 * 32; u < KJ * 8; u += 64) *reinterpret_cast<uint4*>(sX + buf * M::X_BYTES + (size_t)u * 16) = make_uint4(0, 0, 0, 0);
-      tc::fence_async_smem();
-    }
-    if (tid == kCopyThread && hi >= 2) tc::bulk_wait_read();  // the staging tile may be overwritten by the epilogue below
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-
-    // ---- Y_intra = (G o L) X  for this head; the commit also covers the Y_inter MMAs issued above --------------
-    if (mma_warp && tc::elect_one()) {
-      // descriptors differ from instruction to instruction only in the start address (16-byte units, low bits)
-      const uint64_t dx0 = tc::smem_desc_sw128(tc::smem_u32(sX + buf * M::X_BYTES), 16, 1024);
-      constexpr uint32_t idY = tc::instr_desc(kBlk, kP, fmt, 0, 1);
-      const uint32_t dY = tmem + 256 + buf * 128;
+    for (int q = 0; q < kXR; ++q) xr[q] = make_uint4(0, 0, 0, 0);
+    if (hi < nh) {
+      if (!wait(mb_full(buf), hi >> 1)) {  // this head's operands
+        fail = 1;
+        break;
+      }
+      const float* vc = sVec + buf * (2 * kQ);
+      const float* vcp = vc + kQ;
+      const float Dfold = fold_d ? __ldg(a.D + h) : 0.f;
+      // exponents of the decay mask, weight = exp2(re - col(j)), and of the carried state's row weight, exp2(ct)
+      float re;
+      if constexpr (REV) {
+        const float next = c + 1 < nchunks ? __ldg(a.ws_cum + (((int64_t)b * a.heads + h) * nchunks + c + 1) * kQ) : 0.f;
+        re = -vcp[i_chunk], ct = vc[kQ - 1] + next + re;
+      } else {
+        re = ct = vc[i_chunk];
+      }
+      auto col = [&](int j) { return REV ? -vc[COL0 + j] : vcp[j]; };
+      // The weight exp2(c_i - c'_j) of a 32-step chunk factors as exp2(c_i - r) * exp2(r - c'_j) with r = c at the
+      // chunk's first step (row factor <= 1 for causal rows, column factor bounded by the decay inside the chunk).
+      // Each lane forms one column factor per chunk, each thread one row factor per chunk: 2 ex2 per 32 elements
+      // instead of 32.  Chunks whose internal decay exceeds 2^60 keep the exact per-element form.
+      float arow[NCH], bdiag = 0.f;
+      bool fast[NCH];
 #pragma unroll
-      for (int kk = 0; kk < KJ / 16; ++kk)  // 16 steps = 16 rows of 128 bytes of the x tile
-        tc::mma_ts(dY, tmem + kk * 8, dx0 + (uint64_t)(kk * (2048 >> 4)), idY, kk > 0);  // A: 16 steps = 8 columns of the masked rows
-      tc::commit(mb_mma(buf));
+      for (int k = 0; k < NCH; ++k) {
+        const int cc = wg + kScanWG * k;
+        arow[k] = 0.f, fast[k] = false;
+        if (reached(cc)) {
+          const float first = vc[COL0 + cc * 32], r = REV ? -first : first;
+          fast[k] = first - vc[COL0 + cc * 32 + 31] < 60.f;  // same for every lane
+          arow[k] = ex2_approx(re - r);
+          const float bcol = ex2_approx(r - col(cc * 32 + lane));
+          sW[k * 32 + lane] = bcol;
+          // on the diagonal the steps after a row are cut by a zero in its G, which needs finite factors (a step size may be anything)
+          if (cc == rc) bdiag = bcol, fast[k] = __all_sync(0xffffffffu, fast[k] && fabsf(bcol) < __int_as_float(0x7f800000));
+        }
+      }
+      __syncwarp();  // the column factors are read by other lanes
+      if (ragged && hi >= 2) {  // before this head's mask is reported, and thereby before the staging tile is written again
+        if (!wait(mb_epi(buf), (hi - 2) >> 1)) {
+          fail = 1;
+          break;
+        }
+        store_rows(h - 2, buf);
+      }
+      // ---- decay mask: G (registers) x the factors formed above -> the A operand in tensor memory
+#pragma unroll
+      for (int k = 0; k < NCH; ++k) {
+        const int cc = wg + kScanWG * k;  // chunk of 32 steps: whole, diagonal (cc == rc) or empty for this warp's rows
+        const int jb = cc * 32;
+        // the masked row goes to tensor memory as the A operand: 32 steps = 16 columns of two 16-bit values
+        const uint32_t dst = tmem + lane_base + buf * 128 + cc * 16;
+        uint32_t packed[16];
+        if (!reached(cc)) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) packed[q] = 0u;
+          tc::tmem_st16(dst, packed);
+          continue;
+        }
+        const bool diag = cc == rc;
+        if (fast[k]) {
+          const float2 a2 = make_float2(arow[k], arow[k]);
+#pragma unroll
+          for (int q = 0; q < 32; q += 8) {
+            const float4 b0 = *reinterpret_cast<const float4*>(sW + k * 32 + q);
+            const float4 b1 = *reinterpret_cast<const float4*>(sW + k * 32 + q + 4);
+            const float2 bp[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+              const float2 w = __fmul2_rn(__fmul2_rn(make_float2(vG[k][q + e], vG[k][q + e + 1]), bp[e / 2]), a2);
+              f[e] = w.x, f[e + 1] = w.y;
+            }
+            Vec16<T> o;
+            o.pack(f);
+            packed[q / 2] = o.raw.x, packed[q / 2 + 1] = o.raw.y, packed[q / 2 + 2] = o.raw.z, packed[q / 2 + 3] = o.raw.w;
+          }
+          if (diag && fold_d) {  // the diagonal with its D, formed once per row and merged into the word that has been left zero there
+            Vec16<T> d;
+            const float one[8] = {fmaf(gdiag * bdiag, arow[k], Dfold), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            d.pack(one);
+            const uint32_t word = lane & 1 ? d.raw.x << 16 : d.raw.x & 0xffffu;
+            const int at = lane >> 1;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) packed[q] |= q == at ? word : 0u;
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 32; q += 8) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              f[e] = vG[k][q + e] * ex2_approx(re - col(jb + q + e));
+              if (diag && (REV ? q + e < lane : q + e > lane)) f[e] = 0.f;  // after the product: G may be Inf there
+              if (diag && fold_d && q + e == lane) f[e] = fmaf(gdiag, ex2_approx(re - col(jb + q + e)), Dfold);
+            }
+            Vec16<T> o;
+            o.pack(f);
+            packed[q / 2] = o.raw.x, packed[q / 2 + 1] = o.raw.y, packed[q / 2 + 2] = o.raw.z, packed[q / 2 + 3] = o.raw.w;
+          }
+        }
+        tc::tmem_st16(dst, packed);
+      }
+      tc::tmem_wait_st();
+      if constexpr (XSKIP) {  // this row of x (for D x in the epilogue one iteration later)
+#pragma unroll
+        for (int q = 0; q < kXR; ++q) xr[q] = *reinterpret_cast<const uint4*>(swz(sX + buf * M::X_BYTES, i_chunk, wg * kEU + q));
+      }
+      if (ragged && (warp == 13 || warp == 14)) {  // x rows of the next sequence, by two of the warps that have had the least mask work
+#pragma unroll 1
+        for (int u = k_live * 8 + tid - 13 * 32; u < KJ * 8; u += 64) *reinterpret_cast<uint4*>(sX + buf * M::X_BYTES + (size_t)u * 16) = make_uint4(0, 0, 0, 0);
+        tc::fence_async_smem();
+      }
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(mb_mask(buf));
     }
     // ---- the previous head's result, while the tensor cores work on this one ---------------------------------
     if (hi > 0) {
-      if (has_z) ok = tc::mbar_wait(mb_z(buf ^ 1), ((hi - 1) >> 1) & 1);
-      if (ok) epilogue(h - 1, buf ^ 1, ct_prev, xr_prev);
-      else fail = 1;  // becomes CTA-wide at the next iteration's barrier (or right after the loop)
+      const int ob = buf ^ 1, hp = hi - 1;
+      // its MMAs, its gate rows, and the staging tile: y of two heads ago has left it (a barrier that has completed no phase passes
+      // parity 1).  Mostly complete by now: the probes overlap.
+      const uint32_t par = (hp >> 1) & 1, zb = has_z ? mb_z(ob) : mb_mma(ob), yb = ragged ? mb_mma(ob) : mb_out(ob), yp = ragged ? par : par ^ 1;
+      const uint32_t t0 = tc::mbar_test(mb_mma(ob), par), t1 = tc::mbar_test(zb, par), t2 = tc::mbar_test(yb, yp);
+      bool there = (t0 & t1 & t2) != 0;
+      if (!there) there = tc::mbar_wait(mb_mma(ob), par) && tc::mbar_wait(zb, par) && tc::mbar_wait(yb, yp);
+      if (!__all_sync(0xffffffffu, there)) {
+        fail = 1;
+        break;
+      }
+      tc::fence_after_sync();
+      epilogue(h - 1, ob, ct_prev, xr_prev);
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(mb_epi(ob));
     }
     ct_prev = ct;
 #pragma unroll
     for (int q = 0; q < kXR; ++q) xr_prev[q] = xr[q];
   }
-  // leave the loop together: a thread that saw a wait run out above still reaches the same barriers
-  fail = __syncthreads_or(fail);
-  if (!fail && nh > 0) {
-    const int last = nh - 1, buf = last & 1;
-    ok = tc::mbar_wait(mb_mma(buf), (last >> 1) & 1);
-    tc::fence_after_sync();
-    ok = __syncthreads_and(ok);
-    if (ok) {
-      if (ragged) {
-        if (nh >= 2) store_rows(h0 + last - 1);
-      } else if (tid == kCopyThread && nh >= 2) {
-        tc::tma_store_4d(&maps.y, tc::smem_u32(sZ), 0, h0 + last - 1, t_blk, b);
-        tc::bulk_commit();
-        tc::bulk_wait_read();
-      }
-      if (has_z) ok = tc::mbar_wait(mb_z(buf), (last >> 1) & 1);
-      ok = __syncthreads_and(ok);  // also orders thread 0's wait on the store's reads before everyone's writes
-      if (ok) {
-        epilogue(h0 + last, buf, ct_prev, xr_prev);
-        __syncthreads();
-        if (ragged) {
-          store_rows(h0 + last);
-        } else if (tid == kCopyThread) {
-          tc::tma_store_4d(&maps.y, tc::smem_u32(sZ), 0, h0 + last, t_blk, b);
-          tc::bulk_commit();
-        }
-      } else {
-        fail = 1;
-      }
-    } else {
-      fail = 1;
+  if (ragged) {
+    for (int hi = max(nh - 2, 0); hi < nh && !fail; ++hi) {
+      if (wait(mb_epi(hi & 1), hi >> 1)) store_rows(h0 + hi, hi & 1);
+      else fail = 1;
     }
   }
-  if (tid == kCopyThread) tc::bulk_wait_all();  // the staging tile must outlive the stores that read it
-  if (fail && tid == 0 && a.status) *(volatile int32_t*)a.status = 2;
+  if (fail && lane == 0 && a.status) *(volatile int32_t*)a.status = 2;
 }
 
 template <typename T, bool XSKIP, bool REV, bool PACKED>
@@ -996,7 +1050,7 @@ __global__ void __launch_bounds__(kScanThreads, 1)
     ssd_scan_kernel(const ssm_ssd_args a, const __grid_constant__ ScanMaps maps, int nchunks, int hpc, int nparts) {
   extern __shared__ unsigned char smdyn[];
   unsigned char* smraw = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smdyn) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t mbar[8];
+  __shared__ __align__(8) uint64_t mbar[14];
   __shared__ uint32_t tmem_slot;
   const int warp = threadIdx.x >> 5;
   const bool long_block = (int)blockIdx.x < (int)(gridDim.x >> 1);
@@ -1006,7 +1060,7 @@ __global__ void __launch_bounds__(kScanThreads, 1)
   }
   if (warp == 0) tc::tmem_alloc(tc::smem_u32(&tmem_slot), 512);
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 8; ++i) tc::mbar_init(tc::smem_u32(&mbar[i]), 1);
+    for (int i = 0; i < 14; ++i) tc::mbar_init(tc::smem_u32(&mbar[i]), i >= 6 && i < 10 ? kScanCompute / 32 : 1);
   }
   __syncthreads();  // barriers and the TMEM address are set up before anyone arms or polls them
   // the heavier blocks (rows 128..255; REV: rows 0..127) are scheduled first
@@ -1121,7 +1175,7 @@ static int ssd_scan_launch(const ssm_ssd_args& a, const ScanMaps& maps, unsigned
 // long row blocks go first, then the short ones, each to the first SM that is free.  A long block costs 2 + d and a short one
 // 3 + 0.85 d head times (C / B tiles, G, pipeline fill; fitted to d = 8, 12, 16, 24 on 64 + 64 pieces).  Taken is the d with the
 // earliest end: within 2 % of the best divisor in ten dense shapes of both types from 1 x 300 steps of 80 heads (14.8 us) to 8 x 8192 of
-// 48 (387).  Of packed sequences the number of long blocks is a guess, good while they are longer than a chunk (24 in 16384 steps, 48
+// 48 (387; figures of a form 8-14 % slower).  Of packed sequences the number of long blocks is a guess, good while they are longer than a chunk (24 in 16384 steps, 48
 // heads: 127 us, the best) and up to 15 % off when they are not (200 in 16384: 192 against 167 with 24; 64 in 4096, 8 heads: 26
 // against 16 with 4).  Counting whole waves of equal blocks instead chose d = 8 for 76 chunks of 48 heads: 143 us against 122 with 24.
 static int scan_heads_per_cta(int hpg, int64_t longs, int64_t shorts) {

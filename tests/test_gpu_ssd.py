@@ -59,6 +59,38 @@ def test_tensor_core_ssd_matches_oracle(nb, nl, nh, ng, dtype):
     close(Sg, So, **SSD_TOL, what="final state", reduced=True)
 
 
+@pytest.mark.parametrize("nh", [1, 2, 3, 5])
+@pytest.mark.parametrize("gate,skip", [(True, True), (False, True), (True, False)])
+def test_few_heads_per_block(nh, gate, skip):
+    """One to five heads pass through the two buffers of a block; the skip weight rides on the diagonal of the mask."""
+    from ssm_b200 import ops
+
+    t = _inputs(2, 333, nh, 1, torch.bfloat16, seed=nh, with_init=False)
+    if not gate:
+        t["z"] = None
+    if not skip:
+        t["D"] = None
+    yo, so = orc.ssd_scan(**{k: v.float() if torch.is_tensor(v) else v for k, v in t.items()}, dt_softplus=True, return_final_states=True)
+    y, sg = ops.ssd_scan(**{k: v.cuda() if torch.is_tensor(v) else v for k, v in t.items()}, dt_softplus=True, return_final_states=True)
+    close(y, yo, **SSD_TOL, what="y", reduced=True)
+    close(sg, so, **SSD_TOL, what="state", reduced=True)
+
+
+def test_a_nonfinite_step_size_does_not_reach_earlier_steps():
+    """Rows before it in the same 32 steps keep their values (running exponents are formed eight steps at a time: from its eight on)."""
+    from ssm_b200 import ops
+
+    t = {k: v.cuda() if torch.is_tensor(v) else v for k, v in _inputs(1, 256, 2, 1, torch.bfloat16, seed=7, with_init=False).items()}
+    want = ops.ssd_scan(**t, dt_softplus=True)
+    for bad in (float("inf"), float("nan")):
+        for at in (77, 140, 255):
+            dt = t["dt"].clone()
+            dt[0, at, 1] = bad
+            got = ops.ssd_scan(**{**t, "dt": dt}, dt_softplus=True)
+            close(got[:, : at // 8 * 8], want[:, : at // 8 * 8], **SSD_TOL, what=f"{bad} at {at}", reduced=True)
+            assert torch.equal(got[:, :, 0], want[:, :, 0])
+
+
 def test_tensor_core_ssd_without_optionals_and_matrix_D():
     from ssm_b200 import ops
 

@@ -22,6 +22,8 @@
 //   Mamba-2 d_model  768   16.7  19.2  23.8   against  33.4  37.8  38.2  37.8   45.1
 //   Mamba-2 d_model 2560   31.6  45.6  63.7   against  56.2  75.9  77.0  89.1  115.6
 // Without a graph the separate calls take 70 to 100 us of host time.
+// 17 to 256 sequences take a few overlapped launches instead, with products of their own (decode_parts.h): a Mamba-1 step of 256 sequences at
+// d_model 2560 97 us, against 110 with library GEMMs.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -48,6 +48,28 @@ struct Call : torch::CustomClassHolder {
   virtual variable_list backward(const variable_list& grads) = 0;
 };
 
+// Gradients that a graph is recorded through (create_graph).  The kernels' backward passes have no derivative of their own, so the values are
+// right, but differentiated again they would be constants: that raises.  They hang on all they depend on, because the engine walks only
+// paths that lead to what it is asked for.
+struct OnceFn : torch::autograd::Function<OnceFn> {
+  static variable_list forward(AutogradContext*, const variable_list& values, at::TensorList sources) {
+    (void)sources;
+    return values;
+  }
+  static variable_list backward(AutogradContext*, const variable_list&) {
+    TORCH_CHECK(false, "ssm_b200 operators are differentiable once: a gradient formed with create_graph=True cannot be differentiated through them");
+  }
+};
+variable_list differentiable_once(const variable_list& grads, const variable_list& sources) {
+  variable_list values, res;
+  for (const Tensor& t : grads)
+    if (t.defined()) values.push_back(t.detach());
+  if (!values.empty()) values = OnceFn::apply(values, at::TensorList(sources));
+  size_t next = 0;
+  for (const Tensor& t : grads) res.push_back(t.defined() ? values[next++] : Tensor());
+  return res;
+}
+
 struct CallFn : torch::autograd::Function<CallFn> {
   static variable_list forward(AutogradContext* ctx, const c10::intrusive_ptr<Call>& call, at::TensorList inputs) {
     for (const Tensor& t : inputs)
@@ -67,7 +89,19 @@ struct CallFn : torch::autograd::Function<CallFn> {
                              std::to_string(kept.first._version()) + ", expected " + std::to_string(kept.second) + ")");
     }
     ValueErrors scope;
-    variable_list res = call->backward(grads);
+    const bool recorded = at::GradMode::is_enabled();
+    variable_list res;
+    {
+      at::NoGradGuard values_only;
+      res = call->backward(grads);
+    }
+    if (recorded) {
+      variable_list sources;
+      for (const auto& kept : call->guarded) sources.push_back(kept.first);
+      for (const Tensor& g : grads)
+        if (g.defined()) sources.push_back(g);
+      res = differentiable_once(res, sources);
+    }
     res.insert(res.begin(), Tensor());  // the slot of `call`
     return res;
   }

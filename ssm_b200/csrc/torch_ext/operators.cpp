@@ -6,6 +6,7 @@
 #include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/autocast_mode.h>
+#include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/custom_function.h>
 
 #include <utility>
@@ -24,30 +25,6 @@ using torch::autograd::variable_list;
 // ---------------------------------------------------------------------------------------------
 // one differentiable call
 // ---------------------------------------------------------------------------------------------
-// The operands of a call, kept by its autograd node.  `guarded` holds the tensors that the backward pass reads again with
-// their version counters at the time of the forward pass: an in-place edit in between is an error, as for any saved tensor.
-struct Call : torch::CustomClassHolder {
-  std::vector<std::pair<Tensor, uint32_t>> guarded;
-  variable_list inputs;  // the defined tensor arguments, in the order backward() answers for them
-  void input(const Tensor& t) { inputs.push_back(t); }
-  void input(const OptTensor& t) {
-    if (t.has_value() && t->defined()) inputs.push_back(*t);
-  }
-  // A call without a node would drop tangents in silence, so they are looked for first.
-  bool needs_grad() const {
-    for (const Tensor& t : inputs)
-      TORCH_CHECK_NOT_IMPLEMENTED(!t._fw_grad(0).defined(), "ssm_b200 operators have no forward-mode derivative");
-    if (!at::GradMode::is_enabled()) return false;
-    for (const Tensor& t : inputs)
-      if (t.requires_grad()) return true;
-    return false;
-  }
-  virtual variable_list forward(bool train) = 0;
-  // One gradient (or an undefined tensor) per input.  An incoming gradient is undefined where nothing flowed back to that output, and all
-  // of them can be (a node downstream that returns none).
-  virtual variable_list backward(const variable_list& grads) = 0;
-};
-
 // Gradients that a graph is recorded through (create_graph).  The kernels' backward passes have no derivative of their own, so the values are
 // right, but differentiated again they would be constants: that raises.  They hang on all they depend on, because the engine walks only
 // paths that lead to what it is asked for.
@@ -70,6 +47,42 @@ variable_list differentiable_once(const variable_list& grads, const variable_lis
   return res;
 }
 
+// The operands of a call, kept by its autograd node.  `guarded` holds the tensors that the backward pass reads again with
+// their version counters at the time of the forward pass: an in-place edit in between is an error, as for any saved tensor.
+struct Call : torch::CustomClassHolder {
+  std::vector<std::pair<Tensor, uint32_t>> guarded;
+  variable_list inputs;  // the defined tensor arguments, in the order backward() answers for them
+  void input(const Tensor& t) { inputs.push_back(t); }
+  void input(const OptTensor& t) {
+    if (t.has_value() && t->defined()) inputs.push_back(*t);
+  }
+  // A call without a node would drop tangents in silence, so they are looked for first.
+  bool needs_grad() const {
+    for (const Tensor& t : inputs)
+      TORCH_CHECK_NOT_IMPLEMENTED(!t._fw_grad(0).defined(), "ssm_b200 operators have no forward-mode derivative");
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor& t : inputs)
+      if (t.requires_grad()) return true;
+    return false;
+  }
+  virtual variable_list forward(bool train) = 0;
+  // One gradient (or an undefined tensor) per input.  An incoming gradient is undefined where nothing flowed back to that output, and all
+  // of them can be (a node downstream that returns none).
+  virtual variable_list backward(const variable_list& grads) = 0;
+  // The same where a graph is recorded through the gradients.
+  virtual variable_list backward_recorded(const variable_list& grads) {
+    variable_list res, sources;
+    {
+      at::NoGradGuard values_only;
+      res = backward(grads);
+    }
+    for (const auto& kept : guarded) sources.push_back(kept.first);
+    for (const Tensor& g : grads)
+      if (g.defined()) sources.push_back(g);
+    return differentiable_once(res, sources);
+  }
+};
+
 struct CallFn : torch::autograd::Function<CallFn> {
   static variable_list forward(AutogradContext* ctx, const c10::intrusive_ptr<Call>& call, at::TensorList inputs) {
     for (const Tensor& t : inputs)
@@ -89,19 +102,7 @@ struct CallFn : torch::autograd::Function<CallFn> {
                              std::to_string(kept.first._version()) + ", expected " + std::to_string(kept.second) + ")");
     }
     ValueErrors scope;
-    const bool recorded = at::GradMode::is_enabled();
-    variable_list res;
-    {
-      at::NoGradGuard values_only;
-      res = call->backward(grads);
-    }
-    if (recorded) {
-      variable_list sources;
-      for (const auto& kept : call->guarded) sources.push_back(kept.first);
-      for (const Tensor& g : grads)
-        if (g.defined()) sources.push_back(g);
-      res = differentiable_once(res, sources);
-    }
+    variable_list res = at::GradMode::is_enabled() ? call->backward_recorded(grads) : call->backward(grads);
     res.insert(res.begin(), Tensor());  // the slot of `call`
     return res;
   }
@@ -1054,24 +1055,50 @@ struct Mamba1MixerCall final : Call {
   Tensor rows(const Tensor& m) const { return m.view({m.size(0), nb, nl}).permute({1, 0, 2}); }                    // (C, B L) -> (B, C, L)
   Tensor flat(const Tensor& t) const { return t.permute({1, 0, 2}).reshape({t.size(1), nb * nl}); }                // and back
 
-  variable_list forward(bool train) override {
-    c10::cuda::CUDAGuard guard(hidden.device());
-    Tensor h = hidden.detach().reshape({nb * nl, dm});
-    Tensor x = at::mm(in_x.detach(), h.t()), z = at::mm(in_z.detach(), h.t());
-    auto cv = c10::make_intrusive<ConvCall>(rows(x), conv_w.detach(), conv_b.has_value() ? OptTensor(conv_b->detach()) : conv_b, "silu", OptTensor());
-    Tensor u = cv->forward(train)[0], uf = flat(u);
-    Tensor xdbl = at::mm(x_proj.detach(), uf), delta = at::mm(dt_proj.detach(), xdbl.narrow(0, 0, r));
+  // keep: for backward().  Else autograd records the parts wherever it records.
+  Tensor evaluate(bool keep) {
+    Tensor h = hidden.reshape({nb * nl, dm});
+    Tensor x = at::mm(in_x, h.t()), z = at::mm(in_z, h.t());
+    auto cv = c10::make_intrusive<ConvCall>(rows(x), conv_w, conv_b, "silu", OptTensor());
+    Tensor u = (keep ? cv->forward(true) : invoke_call(cv))[0], uf = flat(u);
+    Tensor xdbl = at::mm(x_proj, uf), delta = at::mm(dt_proj, xdbl.narrow(0, 0, r));
     auto coeff = [&](int64_t from) { return xdbl.narrow(0, from, n).view({n, nb, nl}).permute({1, 0, 2}).unsqueeze(1); };  // (B, 1, N, L)
-    Tensor Av = a_log ? at::exp(A_in.detach()).neg_() : A_in.detach();
-    auto sc = c10::make_intrusive<ScanCall>(u, rows(delta), Av, coeff(r), coeff(r + n), OptTensor(D.detach()), OptTensor(rows(z)), OptTensor(dt_bias.detach()), true, false,
-                                            OptTensor(), false);
-    Tensor yf = flat(sc->forward(train)[0]);
-    Tensor out = at::mm(yf.t(), out_proj.detach().t()).view({nb, nl, dm});
-    if (train) {
+    Tensor Av = a_log ? at::exp(A_in).neg() : A_in;
+    auto sc = c10::make_intrusive<ScanCall>(u, rows(delta), Av, coeff(r), coeff(r + n), OptTensor(D), OptTensor(rows(z)), OptTensor(dt_bias), true, false, OptTensor(), false);
+    Tensor yf = flat((keep ? sc->forward(true) : invoke_call(sc))[0]);
+    if (keep) {
+      cv->inputs.clear(), sc->inputs.clear();
       sc->t_B = sc->t_C = at::kFloat;  // their gradients are converted where they are copied
       h2 = h, u2 = uf, xd = xdbl, y2 = yf, A = Av, conv = cv, scan = sc;
     }
-    return {out};
+    return at::mm(yf.t(), out_proj.t()).view({nb, nl, dm});
+  }
+
+  variable_list forward(bool train) override {
+    c10::cuda::CUDAGuard guard(hidden.device());
+    return {evaluate(train)};
+  }
+
+  // What can be differentiated twice (the products) has to be: the composed form again, for autograd to record.  Its inputs are aliases, so
+  // that hooks on the real ones see one gradient each.
+  variable_list backward_recorded(const variable_list& grads) override {
+    if (!grads[0].defined()) return Call::backward_recorded(grads);
+    c10::cuda::CUDAGuard guard(hidden.device());
+    variable_list asked;
+    auto alias = [&](const Tensor& t) {
+      if (!t.requires_grad()) return t;
+      asked.push_back(at::alias(t));
+      return asked.back();
+    };
+    const Tensor a_hidden = alias(hidden), a_in_x = alias(in_x), a_in_z = alias(in_z), a_conv_w = alias(conv_w);
+    const OptTensor a_conv_b = conv_b.has_value() ? OptTensor(alias(*conv_b)) : conv_b;
+    const Tensor a_x_proj = alias(x_proj), a_dt_proj = alias(dt_proj), a_dt_bias = alias(dt_bias), a_A = alias(A_in), a_D = alias(D), a_out_proj = alias(out_proj);
+    Tensor out = c10::make_intrusive<Mamba1MixerCall>(a_hidden, a_in_x, a_in_z, a_conv_w, a_conv_b, a_x_proj, a_dt_proj, a_dt_bias, a_A, a_log, a_D, a_out_proj)->evaluate(false);
+    const variable_list got = torch::autograd::grad({out}, asked, {cast(grads[0], out.scalar_type())}, true, true, true);
+    variable_list res;
+    size_t next = 0;
+    for (bool wanted : need) res.push_back(wanted ? got[next++] : Tensor());
+    return res;
   }
 
   variable_list backward(const variable_list& grads) override {

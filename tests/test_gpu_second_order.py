@@ -8,6 +8,7 @@ import torch
 import torch.nn.functional as F
 
 from ssm_b200 import ops
+from ssm_b200.mixer import Mamba1Block
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +48,37 @@ def test_a_gradient_that_is_not_asked_for_stays_absent():
     y = ops.dw_causal_conv(x, w, None, "silu").square().sum()
     y.backward(create_graph=True)
     assert x.grad.requires_grad and w.grad is None
+
+
+def _mixer_second_order(block, hidden, go, penalised):
+    out = block.mixer_forward(hidden)
+    (g,) = torch.autograd.grad(out, penalised, go, create_graph=True)
+    wrt = [hidden, go, *block.parameters()]
+    return g, torch.autograd.grad(g.square().sum(), wrt, allow_unused=True)
+
+
+def test_a_penalty_on_the_out_projections_gradient_reaches_everything_in_front_of_it():
+    """The product is differentiated twice, the operators before it once: as exact as in the composed form."""
+    torch.manual_seed(0)
+    block = Mamba1Block(64, device="cuda", dtype=torch.float32)
+    hidden, go = torch.randn(2, 33, 64, device="cuda").requires_grad_(), torch.randn(2, 33, 64, device="cuda").requires_grad_()
+    calls = []
+    hook = block.out_proj.register_hook(lambda g: calls.append(1))
+    g, got = _mixer_second_order(block, hidden, go, block.out_proj)
+    assert len(calls) == 1
+    hook.remove()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t):  # the composed form
+        gc, want = _mixer_second_order(block, hidden, go, block.out_proj)
+    torch.testing.assert_close(g, gc, rtol=1e-4, atol=1e-4)
+    for name, a, b in zip(["hidden", "go", *(n for n, _ in block.named_parameters())], got, want):
+        assert (a is None) == (b is None), name
+        if b is not None:
+            assert (a - b).norm() <= 1e-4 * b.norm(), name
+    assert got[0] is not None and got[1] is not None
+
+
+def test_a_penalty_on_a_gradient_behind_the_scan_raises():
+    block = Mamba1Block(64, device="cuda", dtype=torch.float32)
+    hidden, go = torch.randn(2, 33, 64, device="cuda").requires_grad_(), torch.randn(2, 33, 64, device="cuda").requires_grad_()
+    with pytest.raises(RuntimeError, match="differentiable once"):
+        _mixer_second_order(block, hidden, go, block.in_x)

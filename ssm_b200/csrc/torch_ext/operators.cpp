@@ -8,6 +8,8 @@
 #include <ATen/autocast_mode.h>
 #include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/graph_task.h>
+#include <torch/csrc/autograd/saved_variable.h>
 
 #include <utility>
 
@@ -69,7 +71,10 @@ struct Call : torch::CustomClassHolder {
   // One gradient (or an undefined tensor) per input.  An incoming gradient is undefined where nothing flowed back to that output, and all
   // of them can be (a node downstream that returns none).
   virtual variable_list backward(const variable_list& grads) = 0;
-  // The same where a graph is recorded through the gradients.
+  // Whether backward() may run again after a walk that does not retain the graph.  A whole mixer's tensors go with that walk, as those of the
+  // products that it stands for would.
+  virtual bool survives_its_walk() const { return true; }
+  // backward() where a graph is recorded through the gradients.
   virtual variable_list backward_recorded(const variable_list& grads) {
     variable_list res, sources;
     {
@@ -92,7 +97,9 @@ struct CallFn : torch::autograd::Function<CallFn> {
     return call->forward(true);
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
-    auto holder = ctx->saved_data["call"].toCapsule();
+    const auto saved = ctx->saved_data.find("call");
+    TORCH_CHECK(saved != ctx->saved_data.end(), torch::autograd::ERR_BACKWARD_TWICE);
+    auto holder = saved->second.toCapsule();
     Call* call = static_cast<Call*>(holder.get());
     for (const auto& kept : call->guarded) {
       if (kept.first._version() == kept.second) continue;
@@ -102,7 +109,9 @@ struct CallFn : torch::autograd::Function<CallFn> {
                              std::to_string(kept.first._version()) + ", expected " + std::to_string(kept.second) + ")");
     }
     ValueErrors scope;
+    const bool last_walk = !call->survives_its_walk() && !torch::autograd::get_current_graph_task_keep_graph();
     variable_list res = at::GradMode::is_enabled() ? call->backward_recorded(grads) : call->backward(grads);
+    if (last_walk) ctx->saved_data.clear();
     res.insert(res.begin(), Tensor());  // the slot of `call`
     return res;
   }
@@ -1054,6 +1063,8 @@ struct Mamba1MixerCall final : Call {
   }
   Tensor rows(const Tensor& m) const { return m.view({m.size(0), nb, nl}).permute({1, 0, 2}); }                    // (C, B L) -> (B, C, L)
   Tensor flat(const Tensor& t) const { return t.permute({1, 0, 2}).reshape({t.size(1), nb * nl}); }                // and back
+
+  bool survives_its_walk() const override { return false; }
 
   // keep: for backward().  Else autograd records the parts wherever it records.
   Tensor evaluate(bool keep) {

@@ -3,6 +3,8 @@ the modes in which the composed form has to serve."""
 
 from __future__ import annotations
 
+import contextlib
+
 import pytest
 import torch
 
@@ -74,6 +76,20 @@ def test_mamba1_edits_in_place_are_seen_and_a_graph_can_be_walked_twice():
         block.out_proj.mul_(2.0)
     with pytest.raises(RuntimeError, match="modified in place"):
         torch.autograd.grad(out.sum(), hidden)
+
+
+@pytest.mark.parametrize("whole", [True, False])
+def test_mamba1_graph_is_walked_once_unless_it_is_retained(whole):
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    hidden = torch.randn(1, 20, 64, device="cuda").bfloat16().requires_grad_()
+    with contextlib.nullcontext() if whole else composed():
+        out = block.mixer_forward(hidden).float().sum()
+        out.backward(retain_graph=True)
+        out.backward()
+        grad = hidden.grad.clone()
+        with pytest.raises(RuntimeError, match="backward through the graph a second time"):
+            out.backward()
+    assert torch.equal(hidden.grad, grad)
 
 
 def test_mamba1_modes_that_compose():

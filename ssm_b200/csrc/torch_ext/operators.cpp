@@ -50,9 +50,10 @@ variable_list differentiable_once(const variable_list& grads, const variable_lis
 }
 
 // The operands of a call, kept by its autograd node.  `guarded` holds the tensors that the backward pass reads again with
-// their version counters at the time of the forward pass: an in-place edit in between is an error, as for any saved tensor.
+// their version counters at the time of the forward pass: an in-place edit in between is an error, as for any saved tensor.  `unread` holds the
+// others, which may be edited.
 struct Call : torch::CustomClassHolder {
-  std::vector<std::pair<Tensor, uint32_t>> guarded;
+  std::vector<std::pair<Tensor, uint32_t>> guarded, unread;
   variable_list inputs;  // the defined tensor arguments, in the order backward() answers for them
   void input(const Tensor& t) { inputs.push_back(t); }
   void input(const OptTensor& t) {
@@ -67,6 +68,7 @@ struct Call : torch::CustomClassHolder {
       if (t.requires_grad()) return true;
     return false;
   }
+  virtual bool reads(size_t) const { return true; }  // whether backward() reads this input again
   virtual variable_list forward(bool train) = 0;
   // One gradient (or an undefined tensor) per input.  An incoming gradient is undefined where nothing flowed back to that output, and all
   // of them can be (a node downstream that returns none).
@@ -82,6 +84,7 @@ struct Call : torch::CustomClassHolder {
       res = backward(grads);
     }
     for (const auto& kept : guarded) sources.push_back(kept.first);
+    for (const auto& kept : unread) sources.push_back(kept.first);
     for (const Tensor& g : grads)
       if (g.defined()) sources.push_back(g);
     return differentiable_once(res, sources);
@@ -90,8 +93,8 @@ struct Call : torch::CustomClassHolder {
 
 struct CallFn : torch::autograd::Function<CallFn> {
   static variable_list forward(AutogradContext* ctx, const c10::intrusive_ptr<Call>& call, at::TensorList inputs) {
-    for (const Tensor& t : inputs)
-      if (!t.is_inference()) call->guarded.emplace_back(t, t._version());
+    for (size_t i = 0; i < inputs.size(); ++i)
+      if (!inputs[i].is_inference()) (call->reads(i) ? call->guarded : call->unread).emplace_back(inputs[i], inputs[i]._version());
     ctx->saved_data["call"] = c10::IValue::make_capsule(call);
     ctx->set_materialize_grads(false);
     return call->forward(true);
@@ -1045,7 +1048,10 @@ struct Mamba1MixerCall final : Call {
   OptTensor conv_b;
   bool a_log;
   int64_t nb, nl, dm, di, n, r;
+  enum { kHidden, kInX, kInZ, kConvW, kConvB };
+  int kXProj, kDtProj, kDtBias, kA, kD, kOut;  // the inputs behind the conv's bias, if it has one
   std::vector<bool> need;
+  bool conv_live, scan_live;  // parts that a gradient flows back through
   // of the forward pass, for the backward
   Tensor h2, u2, xd, y2, A;
   c10::intrusive_ptr<ConvCall> conv;
@@ -1059,12 +1065,26 @@ struct Mamba1MixerCall final : Call {
     input(conv_b);
     for (const Tensor* t : {&x_proj, &dt_proj, &dt_bias, &A_in, &D, &out_proj}) input(*t);
     for (const Tensor& t : inputs) need.push_back(t.requires_grad());
+    kXProj = kConvB + conv_b.has_value(), kDtProj = kXProj + 1, kDtBias = kXProj + 2, kA = kXProj + 3, kD = kXProj + 4, kOut = kXProj + 5;
+    conv_live = need[kHidden] || need[kInX] || need[kConvW] || (conv_b.has_value() && need[kConvB]);
+    scan_live = conv_live || need[kInZ];
+    for (int i = kXProj; i < kOut; ++i) scan_live = scan_live || need[i];
     nb = hidden.size(0), nl = hidden.size(1), dm = hidden.size(2), di = in_x.size(0), r = dt_proj.size(1), n = (x_proj.size(0) - r) / 2;
   }
   Tensor rows(const Tensor& m) const { return m.view({m.size(0), nb, nl}).permute({1, 0, 2}); }                    // (C, B L) -> (B, C, L)
   Tensor flat(const Tensor& t) const { return t.permute({1, 0, 2}).reshape({t.size(1), nb * nl}); }                // and back
 
   bool survives_its_walk() const override { return false; }
+  // What the products and operators would keep one by one: a factor of a product where the other factor takes a gradient, all inputs of an
+  // operator, A as it is formed (not its logarithm).
+  bool reads(size_t input) const override {
+    const int i = (int)input;
+    if (i == kHidden) return need[kInX] || need[kInZ];
+    if (i == kInX || i == kInZ) return need[kHidden];
+    if (i <= kXProj) return conv_live;  // conv_w, conv_b, x_proj
+    if (i == kDtProj) return conv_live || need[kXProj];
+    return scan_live && !(i == kA && a_log);
+  }
 
   // keep: for backward().  Else autograd records the parts wherever it records.
   Tensor evaluate(bool keep) {
@@ -1093,12 +1113,16 @@ struct Mamba1MixerCall final : Call {
   // What can be differentiated twice (the products) has to be: the composed form again, for autograd to record.  Its inputs are aliases, so
   // that hooks on the real ones see one gradient each.
   variable_list backward_recorded(const variable_list& grads) override {
-    if (!grads[0].defined()) return Call::backward_recorded(grads);
+    bool edited = false;
+    for (const auto& kept : unread) edited = edited || kept.first._version() != kept.second;
+    if (edited || !grads[0].defined()) return Call::backward_recorded(grads);
     c10::cuda::CUDAGuard guard(hidden.device());
     variable_list asked;
+    size_t at_input = 0;
     auto alias = [&](const Tensor& t) {
-      if (!t.requires_grad()) return t;
+      if (!need[at_input++]) return t.detach();
       asked.push_back(at::alias(t));
+      if (!asked.back().requires_grad()) asked.back().requires_grad_();  // switched off since
       return asked.back();
     };
     const Tensor a_hidden = alias(hidden), a_in_x = alias(in_x), a_in_z = alias(in_z), a_conv_w = alias(conv_w);
@@ -1115,15 +1139,11 @@ struct Mamba1MixerCall final : Call {
   variable_list backward(const variable_list& grads) override {
     c10::cuda::CUDAGuard guard(hidden.device());
     const bool has_b = conv_b.has_value();
-    if (!grads[0].defined()) return variable_list(10 + has_b);
-    enum { kHidden, kInX, kInZ, kConvW };
-    const int kXProj = 4 + has_b, kDtProj = kXProj + 1, kDtBias = kXProj + 2, kA = kXProj + 3, kD = kXProj + 4, kOut = kXProj + 5;
     variable_list res(kOut + 1);
+    if (!grads[0].defined()) return res;
     Tensor g = cast(grads[0], h2.scalar_type()).reshape({nb * nl, dm});
     if (need[kOut]) res[kOut] = at::mm(g.t(), y2.t());
-    bool any = false;  // anything behind the out projection
-    for (int i = 0; i < kOut; ++i) any = any || need[i];
-    if (!any) return res;
+    if (!scan_live) return res;
     Tensor dy = at::mm(out_proj.detach().t(), g.t());
     variable_list s = scan->backward({rows(dy)});  // u, delta, A, B, C, D, z, dt_bias
     Tensor du = flat(s[0]), dd = flat(s[1]), dz = flat(s[6]);
@@ -1136,12 +1156,12 @@ struct Mamba1MixerCall final : Call {
     dxd.narrow(0, r, n).view({n, nb, nl}).copy_(s[3].squeeze(1).permute({1, 0, 2}));
     dxd.narrow(0, r + n, n).view({n, nb, nl}).copy_(s[4].squeeze(1).permute({1, 0, 2}));
     if (need[kXProj]) res[kXProj] = at::mm(dxd, u2.t());
-    if (!(need[kHidden] || need[kInX] || need[kInZ] || need[kConvW] || (has_b && need[4]))) return res;
+    if (!(need[kHidden] || need[kInX] || need[kInZ] || need[kConvW] || (has_b && need[kConvB]))) return res;
     du.addmm_(x_proj.detach().t(), dxd);
     variable_list c = conv->backward({rows(du)});
     Tensor dx = flat(c[0]);
     if (need[kConvW]) res[kConvW] = c[1];
-    if (has_b && need[4]) res[4] = c[2];
+    if (has_b && need[kConvB]) res[4] = c[2];
     if (need[kInX]) res[kInX] = at::mm(dx, h2);
     if (need[kInZ]) res[kInZ] = at::mm(dz, h2);
     if (need[kHidden]) {

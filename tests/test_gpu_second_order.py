@@ -82,3 +82,18 @@ def test_a_penalty_on_a_gradient_behind_the_scan_raises():
     hidden, go = torch.randn(2, 33, 64, device="cuda").requires_grad_(), torch.randn(2, 33, 64, device="cuda").requires_grad_()
     with pytest.raises(RuntimeError, match="differentiable once"):
         _mixer_second_order(block, hidden, go, block.in_x)
+
+
+def test_a_mixers_gradient_after_an_edit_of_what_it_does_not_read_raises_when_differentiated():
+    """Its composed form cannot be formed again then."""
+    block = Mamba1Block(64, device="cuda", dtype=torch.float32)
+    hidden, go = torch.randn(2, 33, 64, device="cuda").requires_grad_(), torch.randn(2, 33, 64, device="cuda")
+    out = block.mixer_forward(hidden)
+    (want,) = torch.autograd.grad(out, block.out_proj, go, retain_graph=True)
+    with torch.no_grad():
+        block.A_log.mul_(0.5)
+    (g,) = torch.autograd.grad(out, block.out_proj, go, create_graph=True)
+    torch.testing.assert_close(g.detach(), want, rtol=1e-4, atol=1e-4)
+    for wrt in (hidden, block.in_x):
+        with pytest.raises(RuntimeError, match="differentiable once"):
+            torch.autograd.grad(g.square().sum(), wrt, retain_graph=True)

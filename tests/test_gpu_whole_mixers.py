@@ -4,6 +4,7 @@ the modes in which the composed form has to serve."""
 from __future__ import annotations
 
 import contextlib
+import types
 
 import pytest
 import torch
@@ -90,6 +91,47 @@ def test_mamba1_graph_is_walked_once_unless_it_is_retained(whole):
         with pytest.raises(RuntimeError, match="backward through the graph a second time"):
             out.backward()
     assert torch.equal(hidden.grad, grad)
+
+
+# parameters without a gradient; what is edited between forward and backward; whether the backward reads it
+@pytest.mark.parametrize("frozen,edited,read", [
+    (["in_x", "in_z"], "hidden", False), (["in_x"], "hidden", True), ([], "A_log", False), ([], "in_x", True), (["hidden"], "in_x", False), (["hidden"], "x_proj", True),
+    (["hidden", "in_x", "conv_w", "conv_b"], "x_proj", False), (["hidden", "in_x", "conv_w", "conv_b", "x_proj"], "dt_proj", False), ([], "out_proj", True), ([], "dt_bias", True)])
+def test_mamba1_inputs_that_the_backward_does_not_read_may_be_edited(frozen, edited, read):
+    torch.manual_seed(1)
+    block = Mamba1Block(64, device="cuda", dtype=torch.float32)
+    leaf = torch.randn(1, 20, 64, device="cuda").requires_grad_("hidden" not in frozen)
+    for n, p in block.named_parameters():
+        p.requires_grad_(n not in frozen)
+    live = [p for p in [leaf, *block.parameters()] if p.requires_grad and p is not block.norm_w]
+
+    def run():
+        hidden = leaf * 1.0
+        out = block.mixer_forward(hidden)
+        with torch.no_grad():
+            (hidden if edited == "hidden" else getattr(block, edited)).mul_(1.0)
+        return torch.autograd.grad(out.square().sum(), live)
+
+    results = []
+    for namespace in (ops, types.SimpleNamespace(**{n: getattr(ops, n) for n in ops.__all__})):  # the second without whole mixers
+        block._ops = namespace
+        if read:
+            with pytest.raises(RuntimeError, match="modified in place|modified by an inplace"):
+                run()
+        else:
+            results.append(run())
+    for a, b in zip(*results):
+        _near(a, b, torch.float32, edited)
+
+
+def test_mamba1_in_place_residual_trains():
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    block.in_x.requires_grad_(False), block.in_z.requires_grad_(False)
+    leaf = torch.randn(1, 20, 64, device="cuda").bfloat16().requires_grad_()
+    h = leaf * 1.0
+    h += block.mixer_forward(h)
+    h.float().sum().backward()
+    assert leaf.grad.isfinite().all() and block.out_proj.grad is not None
 
 
 def test_mamba1_modes_that_compose():

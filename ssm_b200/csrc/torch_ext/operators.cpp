@@ -1052,7 +1052,7 @@ struct Mamba1MixerCall final : Call {
   int kXProj, kDtProj, kDtBias, kA, kD, kOut;  // the inputs behind the conv's bias, if it has one
   std::vector<bool> need;
   bool conv_live, scan_live;  // parts that a gradient flows back through
-  // of the forward pass, for the backward
+  // of the forward pass, what the backward reads
   Tensor h2, u2, xd, y2, A;
   c10::intrusive_ptr<ConvCall> conv;
   c10::intrusive_ptr<ScanCall> scan;
@@ -1096,24 +1096,41 @@ struct Mamba1MixerCall final : Call {
     auto coeff = [&](int64_t from) { return xdbl.narrow(0, from, n).view({n, nb, nl}).permute({1, 0, 2}).unsqueeze(1); };  // (B, 1, N, L)
     Tensor Av = a_log ? at::exp(A_in).neg() : A_in;
     auto sc = c10::make_intrusive<ScanCall>(u, rows(delta), Av, coeff(r), coeff(r + n), OptTensor(D), OptTensor(rows(z)), OptTensor(dt_bias), true, false, OptTensor(), false);
-    Tensor yf = flat((keep ? sc->forward(true) : invoke_call(sc))[0]);
+    Tensor yf = flat((keep ? sc->forward(scan_live) : invoke_call(sc))[0]);
     if (keep) {
       cv->inputs.clear(), sc->inputs.clear();
       sc->t_B = sc->t_C = at::kFloat;  // their gradients are converted where they are copied
-      h2 = h, u2 = uf, xd = xdbl, y2 = yf, A = Av, conv = cv, scan = sc;
+      if (need[kInX] || need[kInZ]) h2 = h;
+      if (need[kDtProj]) xd = xdbl;
+      if (need[kXProj]) u2 = uf;
+      if (need[kOut]) y2 = yf;
+      if (need[kA]) A = Av;
+      if (conv_live) conv = cv;
+      if (scan_live) scan = sc;
     }
     return at::mm(yf.t(), out_proj.t()).view({nb, nl, dm});
   }
 
   variable_list forward(bool train) override {
-    c10::cuda::CUDAGuard guard(hidden.device());
-    return {evaluate(train)};
+    c10::cuda::CUDAGuard guard(out_proj.device());
+    Tensor out = evaluate(train);
+    if (train && !reads(kHidden)) {  // its values are not needed again; what hangs on its graph is an alias without any
+      for (size_t i = 0; i < unread.size(); ++i)
+        if (unread[i].first.is_same(hidden)) unread.erase(unread.begin() + i--);
+      if (need[kHidden]) {
+        at::AutoGradMode record(true);
+        const Tensor none = hidden.narrow(0, 0, 0).clone();
+        unread.emplace_back(none, none._version());
+      }
+      hidden = Tensor();
+    }
+    return {out};
   }
 
   // What can be differentiated twice (the products) has to be: the composed form again, for autograd to record.  Its inputs are aliases, so
   // that hooks on the real ones see one gradient each.
   variable_list backward_recorded(const variable_list& grads) override {
-    bool edited = false;
+    bool edited = !hidden.defined();
     for (const auto& kept : unread) edited = edited || kept.first._version() != kept.second;
     if (edited || !grads[0].defined()) return Call::backward_recorded(grads);
     c10::cuda::CUDAGuard guard(hidden.device());
@@ -1136,38 +1153,54 @@ struct Mamba1MixerCall final : Call {
     return res;
   }
 
+  // Each tensor goes with its last use, on the walk that ends the graph those of the forward pass too.
   variable_list backward(const variable_list& grads) override {
-    c10::cuda::CUDAGuard guard(hidden.device());
-    const bool has_b = conv_b.has_value();
+    c10::cuda::CUDAGuard guard(out_proj.device());
+    const bool ends = !torch::autograd::get_current_graph_task_keep_graph();
+    auto drop = [&](auto& kept) {
+      if (ends) kept = std::decay_t<decltype(kept)>();
+    };
     variable_list res(kOut + 1);
     if (!grads[0].defined()) return res;
-    Tensor g = cast(grads[0], h2.scalar_type()).reshape({nb * nl, dm});
+    Tensor g = cast(grads[0], out_proj.scalar_type()).reshape({nb * nl, dm});
     if (need[kOut]) res[kOut] = at::mm(g.t(), y2.t());
+    drop(y2);
     if (!scan_live) return res;
-    Tensor dy = at::mm(out_proj.detach().t(), g.t());
-    variable_list s = scan->backward({rows(dy)});  // u, delta, A, B, C, D, z, dt_bias
+    variable_list s = scan->backward({rows(at::mm(out_proj.detach().t(), g.t()))});  // u, delta, A, B, C, D, z, dt_bias
+    drop(scan);
     Tensor du = flat(s[0]), dd = flat(s[1]), dz = flat(s[6]);
+    s[0] = s[1] = s[6] = g = Tensor();
     if (need[kA]) res[kA] = cast(a_log ? s[2].mul_(A) : s[2], A_in.scalar_type());
     if (need[kD]) res[kD] = cast(s[5], D.scalar_type());
     if (need[kDtBias]) res[kDtBias] = cast(s[7], dt_bias.scalar_type());
+    if (need[kInZ]) res[kInZ] = at::mm(dz, h2);
+    if (!need[kHidden]) dz = Tensor();
     if (need[kDtProj]) res[kDtProj] = at::mm(dd, xd.narrow(0, 0, r).t());
-    Tensor dxd = at::empty_like(xd), low = dxd.narrow(0, 0, r);
+    drop(xd);
+    if (!(conv_live || need[kXProj])) return res;
+    Tensor dxd = at::empty({r + 2 * n, nb * nl}, du.options()), low = dxd.narrow(0, 0, r);
     at::mm_out(low, dt_proj.detach().t(), dd);
+    dd = Tensor();
     dxd.narrow(0, r, n).view({n, nb, nl}).copy_(s[3].squeeze(1).permute({1, 0, 2}));
     dxd.narrow(0, r + n, n).view({n, nb, nl}).copy_(s[4].squeeze(1).permute({1, 0, 2}));
+    s.clear();
     if (need[kXProj]) res[kXProj] = at::mm(dxd, u2.t());
-    if (!(need[kHidden] || need[kInX] || need[kInZ] || need[kConvW] || (has_b && need[kConvB]))) return res;
+    drop(u2);
+    if (!conv_live) return res;
     du.addmm_(x_proj.detach().t(), dxd);
     variable_list c = conv->backward({rows(du)});
-    Tensor dx = flat(c[0]);
+    drop(conv);
+    du = dxd = Tensor();
     if (need[kConvW]) res[kConvW] = c[1];
-    if (has_b && need[kConvB]) res[4] = c[2];
+    if (conv_b.has_value() && need[kConvB]) res[kConvB] = c[2];
+    Tensor dx = flat(c[0]);
+    c.clear();
     if (need[kInX]) res[kInX] = at::mm(dx, h2);
-    if (need[kInZ]) res[kInZ] = at::mm(dz, h2);
+    drop(h2);
     if (need[kHidden]) {
       Tensor dh = at::mm(dx.t(), in_x.detach());
       dh.addmm_(dz.t(), in_z.detach());
-      res[kHidden] = dh.view(hidden.sizes());
+      res[kHidden] = dh.view({nb, nl, dm});
     }
     return res;
   }

@@ -134,6 +134,36 @@ def test_mamba1_in_place_residual_trains():
     assert leaf.grad.isfinite().all() and block.out_proj.grad is not None
 
 
+@pytest.mark.parametrize("frozen", [[], ["out_proj"], ["in_x", "in_z"], ["x_proj", "dt_proj"], ["but out_proj"]])
+def test_mamba1_keeps_no_more_than_composed_operators(frozen):
+    """Bytes held after the forward pass, at the worst in the backward, and after it while the loss is alive."""
+    block = Mamba1Block(256, device="cuda", dtype=torch.bfloat16)
+    for n, p in block.named_parameters():
+        p.requires_grad_(n == "out_proj" if frozen == ["but out_proj"] else n not in frozen)
+
+    def run(namespace):
+        block._ops = namespace
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        leaf = torch.randn(8, 1024, 256, device="cuda").bfloat16().requires_grad_(frozen != ["but out_proj"])
+        loss = block.mixer_forward(leaf * 1.0).float().sum()
+        kept = torch.cuda.memory_allocated() - before
+        torch.cuda.reset_peak_memory_stats()
+        loss.backward()
+        peak, left = torch.cuda.max_memory_allocated() - before, torch.cuda.memory_allocated() - before
+        for p in block.parameters():
+            p.grad = None
+        assert loss.isfinite()
+        return kept, peak, left
+
+    whole, apart = ops, types.SimpleNamespace(**{n: getattr(ops, n) for n in ops.__all__})
+    run(whole), run(apart)  # library workspaces
+    got, want = run(whole), run(apart)
+    gradient = 8 * 1024 * 256 * 2  # the incoming one, which autograd holds while the node runs
+    for what, a, b in zip(("kept", "peak", "left"), got, want):
+        assert a <= b + 65536 + (gradient if what == "peak" else 0), (what, got, want)  # (small tensors round up to blocks of their own)
+
+
 def test_mamba1_modes_that_compose():
     block = Mamba1Block(64, device="cuda", dtype=torch.float32)
     hidden = torch.randn(1, 20, 64, device="cuda")

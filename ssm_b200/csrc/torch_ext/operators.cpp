@@ -1075,6 +1075,8 @@ struct Mamba1MixerCall final : Call {
   Tensor flat(const Tensor& t) const { return t.permute({1, 0, 2}).reshape({t.size(1), nb * nl}); }                // and back
 
   bool survives_its_walk() const override { return false; }
+  // The products are formed in the types of the forward pass, also where the backward runs inside autocast.
+  using NoAutocast = c10::impl::ExcludeDispatchKeyGuard;
   // What the products and operators would keep one by one: a factor of a product where the other factor takes a gradient, all inputs of an
   // operator, A as it is formed (not its logarithm).
   bool reads(size_t input) const override {
@@ -1133,6 +1135,7 @@ struct Mamba1MixerCall final : Call {
     bool edited = !hidden.defined();
     for (const auto& kept : unread) edited = edited || kept.first._version() != kept.second;
     if (edited || !grads[0].defined()) return Call::backward_recorded(grads);
+    NoAutocast plain_types(c10::autocast_dispatch_keyset);
     c10::cuda::CUDAGuard guard(hidden.device());
     variable_list asked;
     size_t at_input = 0;
@@ -1156,6 +1159,7 @@ struct Mamba1MixerCall final : Call {
   // Each tensor goes with its last use, on the walk that ends the graph those of the forward pass too.
   variable_list backward(const variable_list& grads) override {
     c10::cuda::CUDAGuard guard(out_proj.device());
+    NoAutocast plain_types(c10::autocast_dispatch_keyset);
     const bool ends = !torch::autograd::get_current_graph_task_keep_graph();
     auto drop = [&](auto& kept) {
       if (ends) kept = std::decay_t<decltype(kept)>();

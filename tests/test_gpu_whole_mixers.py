@@ -164,6 +164,23 @@ def test_mamba1_keeps_no_more_than_composed_operators(frozen):
         assert a <= b + 65536 + (gradient if what == "peak" else 0), (what, got, want)  # (small tensors round up to blocks of their own)
 
 
+@pytest.mark.parametrize("create_graph", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_mamba1_backward_inside_autocast(dtype, create_graph):
+    """The forward pass ran outside: the gradients are those of its types."""
+    torch.manual_seed(2)
+    block = Mamba1Block(64, device="cuda", dtype=dtype)
+    hidden = torch.randn(2, 33, 64, device="cuda").to(dtype).requires_grad_()
+    go = torch.randn(2, 33, 64, device="cuda").to(dtype)
+    leaves = [hidden, *(p for n, p in block.named_parameters() if n != "norm_w")]
+    want = torch.autograd.grad(block.mixer_forward(hidden), leaves, go)
+    out = block.mixer_forward(hidden)
+    with torch.autocast("cuda", torch.float16):
+        got = torch.autograd.grad(out, leaves, go, create_graph=create_graph)
+    for a, b in zip(got, want):
+        _near(a.detach(), b, dtype, "gradient")
+
+
 def test_mamba1_modes_that_compose():
     block = Mamba1Block(64, device="cuda", dtype=torch.float32)
     hidden = torch.randn(1, 20, 64, device="cuda")

@@ -596,6 +596,20 @@ Tensor rows_of(void* p, int64_t rows, int64_t cols, int64_t ld, const Tensor& li
 // us against 16.2; 128 rows 10.1 against 11.3; 256 rows, 768 x 1536 4.5 against 5.8, but 10 us more of host time).
 bool library_product(int64_t nb, const Tensor& w) { return nb > 128 && w.size(0) >= 1024 && w.size(1) >= 2048; }
 
+// What the separate calls refuse, or answer in another type, goes to them: shapes that agree in their number of elements only, tangents, autocast
+// to another type.
+bool by_parts(const Tensor& tok, std::initializer_list<std::pair<const Tensor*, std::initializer_list<int64_t>>> shapes, std::initializer_list<const OptTensor*> tangents) {
+  if (tok.size(1) % 8 != 0 || tok.size(0) > SSMB_GEMM_MAX_ROWS) return false;
+  if (at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) != tok.scalar_type()) return false;
+  for (const auto& [t, shape] : shapes)
+    if (t->sizes() != at::IntArrayRef(shape)) return false;
+  for (const OptTensor* t : tangents)
+    if (t->has_value() && (*t)->_fw_grad(0).defined()) return false;
+  return true;
+}
+// conv weights (C, K), or (C, 1, K)
+bool conv_weight(const Tensor& w, int64_t c, int64_t k) { return w.size(0) == c && w.size(-1) == k && (w.dim() == 2 || (w.dim() == 3 && w.size(1) == 1)); }
+
 py::object mamba1_parts(const Tensor& tok, const OptTensor& residual, const Tensor& conv_state, const Tensor& ssm_state, const Tensor& in_x, const Tensor& in_z,
                         const Tensor& conv_w, const OptTensor& conv_b, const Tensor& x_proj, const Tensor& dt_proj, const Tensor& dt_bias, const Tensor& A, bool a_log,
                         const Tensor& D, const Tensor& out_proj, const OptTensor& norm_w, double eps) {
@@ -718,7 +732,7 @@ py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tenso
       return py::cast(out);
     }
   }
-  if (fused && dm % 8 == 0 && di % 8 == 0 && nb <= SSMB_GEMM_MAX_ROWS)
+  if (fused && di % 8 == 0 && conv_weight(conv_w, di, k) && by_parts(tok, {{&D, {di}}, {&dt_bias, {di}}, {norm_w.has_value() ? &*norm_w : &D, {norm_w.has_value() ? dm : di}}}, {&residual, &norm_w}))
     return mamba1_parts(tok, residual, conv_state, ssm_state, in_x, in_z, conv_w, conv_b, x_proj, dt_proj, dt_bias, A, a_log, D, out_proj, norm_w, eps);
   Tensor x = at::matmul(tok, in_x.t()), z = at::matmul(tok, in_z.t());
   Tensor u = dw_causal_conv_update(conv_state, x, conv_w, conv_b, "silu");
@@ -745,6 +759,7 @@ Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B
   const int64_t nb = tok.size(0), dm = tok.size(1), nh = ssm_state.size(1), hp = ssm_state.size(2), n = ssm_state.size(3), di = nh * hp;
   SSM_ARG(in_B.size(0) % n == 0, "mamba2_step: in_B must have groups * d_state rows.");
   const int64_t g = in_B.size(0) / n, k = wx.size(-1);
+  SSM_ARG(g > 0 && nh % g == 0, "B and C must have shape (B, G, N) with G dividing H.");  // before any window is written
   const auto T = tok.scalar_type();
   bool fused = (T == at::kBFloat16 || T == at::kHalf) && plain(tok, T) && plain(dt_bias, at::kFloat) && plain(A, at::kFloat) && plain(D, at::kFloat) &&
                plain(bx, T) && plain(bB, T) && plain(bC, T);
@@ -770,7 +785,8 @@ Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B
     a.ssm_state = ssm_state.data_ptr<float>(), a.out = out.data_ptr(), a.scratch = scratch.data_ptr();
     if (launched(ssm_mamba2_decode(&a, stream_of(tok)))) return out;
   }
-  if (fused && dm % 8 == 0 && di % 8 == 0 && nb <= SSMB_GEMM_MAX_ROWS)
+  if (fused && di % 8 == 0 && conv_weight(wx, di, k) && conv_weight(wB, g * n, k) && conv_weight(wC, g * n, k) &&
+      by_parts(tok, {{&conv_x, {nb, di, k}}, {&conv_B, {nb, g * n, k}}, {&conv_C, {nb, g * n, k}}, {&A, {nh}}, {&norm_w, {di}}}, {}))
     return mamba2_parts(tok, conv_x, conv_B, conv_C, ssm_state, in_z, in_x, in_B, in_C, in_dt, wx, bx, wB, bB, wC, bC, dt_bias, A, a_log, D, norm_w, out_proj, eps);
   Tensor z = at::matmul(tok, in_z.t());
   Tensor x = dw_causal_conv_update(conv_x, at::matmul(tok, in_x.t()), wx, bx, "silu");

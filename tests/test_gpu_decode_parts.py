@@ -128,3 +128,75 @@ def test_state_step_by_channels_matches_oracle(n, nd, groups, gate, a_dtype):
     yo = orc.selective_state_step(state, x, dt, A, B, C, D=D, z=z, dt_bias=bias, softplus=True)
     tol = dict(rtol=1e-4, atol=1e-4) if a_dtype == torch.float32 else dict(rtol=2e-2, atol=1e-2)
     close(y, yo, **tol, what="y"), close(sg, state, rtol=1e-4, atol=1e-4, what="state")
+
+
+@pytest.mark.parametrize("nb", [3, 20, 300])
+def test_groups_that_cut_through_a_head_are_refused_before_anything_is_written(nb):
+    from ssm_b200 import ops
+    from ssm_b200.mixer import Mamba2Block
+
+    w = dict(Mamba2Block(96, device="cuda", dtype=torch.bfloat16)._weights())  # three heads, here with two groups of states
+    for k, shape in {"in_B": (256, 96), "in_C": (256, 96), "conv_B": (256, 4), "conv_C": (256, 4), "conv_B_b": (256,), "conv_C_b": (256,)}.items():
+        w[k] = torch.randn(*shape, device="cuda").bfloat16()
+    windows = [torch.zeros(nb, c, 4, device="cuda") for c in (192, 256, 256)]
+    state = torch.zeros(nb, 3, 64, 128, device="cuda")
+    with torch.no_grad(), pytest.raises(ValueError, match="G dividing H"):
+        ops.mamba2_step(torch.randn(nb, 96, device="cuda").bfloat16(), tuple(windows), state, w)
+    assert not any(t.any() for t in (*windows, state))
+
+
+def test_windows_of_another_shape_are_refused():
+    from ssm_b200 import ops
+    from ssm_b200.mixer import Mamba2Block
+
+    block = Mamba2Block(64, device="cuda", dtype=torch.bfloat16)
+    (wx, wB, wC), state = block.allocate_inference_cache(20)
+    with torch.no_grad(), pytest.raises(ValueError, match="conv_state must be"):
+        ops.mamba2_step(torch.randn(20, 64, device="cuda").bfloat16(), (wx.view(20, 4, -1), wB, wC), state, block._weights())
+
+
+def test_a_step_inside_autocast_to_another_type_answers_in_that_type():
+    from ssm_b200.mixer import Mamba1Block
+
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    tok, cache = torch.randn(20, 64, device="cuda").bfloat16(), block.allocate_inference_cache(20)
+    with torch.no_grad(), torch.autocast("cuda", torch.float16):
+        assert block.mixer_step(tok, cache).dtype == torch.float16
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        assert block.mixer_step(tok, cache).dtype == torch.bfloat16
+
+
+def test_a_tangent_of_the_residual_is_refused():
+    import torch.autograd.forward_ad as fwd
+    from ssm_b200.mixer import Mamba1Block
+
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    hidden, res, cache = torch.randn(20, 1, 64, device="cuda").bfloat16(), torch.randn(20, 1, 64, device="cuda"), block.allocate_inference_cache(20)
+    with torch.no_grad(), fwd.dual_level(), pytest.raises(NotImplementedError, match="forward-mode"):
+        block.step(hidden, fwd.make_dual(res, torch.ones_like(res)), *cache)
+
+
+# the launches of a step that is captured: overlapped kernels, clusters and, at 256 sequences of a wide model, one of the library's products
+@pytest.mark.parametrize("cls,nb,dm", [("Mamba1Block", 20, 320), ("Mamba1Block", 256, 2048), ("Mamba2Block", 130, 256)])
+def test_captured_steps_match_plain_ones(cls, nb, dm):
+    from ssm_b200 import mixer
+
+    torch.manual_seed(0)
+    block = getattr(mixer, cls)(dm, device="cuda", dtype=torch.bfloat16)
+    flat = lambda cache: [cache[0], cache[1]] if cls == "Mamba1Block" else [*cache[0], cache[1]]  # noqa: E731
+    toks = [torch.randn(nb, dm, device="cuda").bfloat16() for _ in range(3)]
+    plain, captured = block.allocate_inference_cache(nb), block.allocate_inference_cache(nb)
+    with torch.no_grad():
+        want = [block.mixer_step(t, plain) for t in toks]
+        tok = toks[0].clone()
+        block.mixer_step(tok, block.allocate_inference_cache(nb))  # library handles and workspaces
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = block.mixer_step(tok, captured)
+        for t, w in zip(toks, want):
+            tok.copy_(t)
+            graph.replay()
+            assert torch.equal(out, w)
+    for a, b in zip(flat(plain), flat(captured)):
+        assert torch.equal(a, b)
+    del graph

@@ -1263,9 +1263,12 @@ std::tuple<Tensor, Tensor, Tensor> ssd_packed(const Tensor& X, const Tensor& dt,
                                               const Tensor& cu_seqlens, bool reset) {
   ValueErrors scope;
   // Boundaries on the device: the kernels are enqueued behind a table formed there, and the copy that the boundaries are checked on is awaited
-  // only then, so that the device does not stand idle while the host reads them (24 sequences in 16384 steps of 48 heads: 35 us).
-  const int64_t chunk_slots = cu_seqlens.dim() == 1 && cu_seqlens.numel() >= 2 ? X.size(1) / chunk + cu_seqlens.numel() - 1 : 1 << 30;
-  if (reset && cu_seqlens.is_cuda() && cu_seqlens.get_device() == X.get_device() && chunk_slots <= 65535 && X.size(1) > 0 && X.size(1) < (1 << 30)) {
+  // only then, so that the device does not stand idle while the host reads them (35 us for 24 sequences in 16384 steps of 48 heads, 20 us at 4 to
+  // 512 sequences in 512 to 16384).  The table has room for a chunk per sequence, 18 KB of scratch per head even where the sequence is
+  // empty (boundaries padded to a fixed number: 1024 entries, 48 heads 0.9 GB): with more than four sequences to a chunk, and more than
+  // 64, the host counts the chunks.
+  const int64_t seqs = cu_seqlens.dim() == 1 ? cu_seqlens.numel() - 1 : 0, whole_chunks = X.size(1) / chunk, chunk_slots = whole_chunks + seqs;
+  if (reset && seqs >= 1 && seqs <= std::max<int64_t>(64, 4 * whole_chunks) && cu_seqlens.is_cuda() && cu_seqlens.get_device() == X.get_device() && chunk_slots <= 65535 && X.size(1) > 0 && X.size(1) < (1 << 30)) {
     c10::cuda::CUDAGuard guard(X.device());
     const Tensor bounds = cu_seqlens.scalar_type() == at::kInt ? cu_seqlens.contiguous() : cu_seqlens.to(at::kLong).contiguous();
     Tensor host = at::empty(bounds.sizes(), bounds.options().device(at::kCPU).pinned_memory(true));

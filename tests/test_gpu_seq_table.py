@@ -44,3 +44,24 @@ def test_what_does_not_rise_from_zero_to_the_end_is_refused(cu):
     torch.cuda.synchronize()
     with torch.no_grad():
         assert ops.ssd_scan(X, dt, A, B, C, cu_seqlens=torch.tensor([0, 600], device="cuda")).isfinite().all()
+
+
+# padding to a fixed number of sequences: empty ones behind the last
+@pytest.mark.parametrize("entries", [64, 1024])
+def test_padded_boundaries_on_the_device_take_little_more_than_on_the_host(entries):
+    nl, nh = 4096, 16
+    X, dt, A, B, C = _inputs(nl, nh, 1)
+    cu = torch.tensor([0, 1000] + [nl] * (entries - 1), dtype=torch.int32)
+
+    def peak(c):
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        with torch.no_grad():
+            out = ops.ssd_scan(X, dt, A, B, C, dt_softplus=True, cu_seqlens=c, return_varlen_states=True)
+        return torch.cuda.max_memory_allocated() - before, out
+
+    (host, want), (device, got) = peak(cu), peak(cu.cuda())
+    assert device <= host + 64 * nh * 19 * 1024
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)

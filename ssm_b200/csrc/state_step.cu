@@ -307,23 +307,22 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamCtasPerSm) step_stream_
   }
 }
 
-// Four consecutive B or C values as raw words, and as two pairs of fp32
+// Four consecutive 16-bit B or C values as raw words, and as two pairs of fp32
 template <typename BT>
 struct Bc4 {
-  using Raw = typename std::conditional<sizeof(BT) == 4, uint4, uint2>::type;
-  Raw raw;
-  __device__ __forceinline__ void load(const void* base, int64_t off) { raw = __ldg(reinterpret_cast<const Raw*>(reinterpret_cast<const BT*>(base) + off)); }
+  uint2 raw;
+  __device__ __forceinline__ void load(const void* base, int64_t off) { raw = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const BT*>(base) + off)); }
   __device__ __forceinline__ float2 pair(int i) const {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(&raw);
-    if constexpr (sizeof(BT) == 4) return make_float2(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
-    else if constexpr (std::is_same<BT, __nv_bfloat16>::value) return make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-    else return __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+    const uint32_t w = i ? raw.y : raw.x;
+    if constexpr (std::is_same<BT, __nv_bfloat16>::value) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    else return __half22float2(*reinterpret_cast<const __half2*>(&w));
   }
 };
 
-// step_stream_kernel for parameters per channel: a warp keeps its 512 / N channels and walks over sequences, so that A (and its
-// exponential, where log(-A) is given), D and the bias are formed once and no index is divided.  (256, 5120) x 16 states took
-// 37 instructions per state in the kernel above, 35 us.
+// step_stream_kernel for parameters per channel and 16-bit operands: a warp keeps its 512 / N channels and walks over sequences, so that A (and
+// its exponential, where log(-A) is given), D and the bias are formed once and no index is divided.  bf16, us of steps back to back against
+// the kernel above: (256, 5120) x 16 26.1 and 28.9, (128, 5120) x 16 12.4 and 14.5, (256, 1024) x 64 19.8 and 22.9, (1024, 5120) x 16 116 and
+// 120.  With fp32 operands it was the slower one: (256, 5120) x 16 36.6 and 30.2, (256, 512) x 128 26.0 and 22.3.
 template <typename T, typename BT, int N>
 __global__ void __launch_bounds__(kStreamThreads, kStreamCtasPerSm) step_channels_kernel(const ssm_step_args a) {
   constexpr int kPiece = 512, RPW = kPiece / N, LPR = N / 16;
@@ -524,10 +523,12 @@ template <typename T, typename BT, int N>
 static int step_stream_launch(const ssm_step_args& a, int sms, cudaStream_t st) {
   const int grid = sms * kStreamCtasPerSm;
   if (a.param_heads > 0) return launch_overlapped("step_stream_kernel", step_stream_kernel<T, BT, N, true>, dim3(grid), dim3(kStreamThreads), 0, st, a);
-  // whole pieces of channels per sequence, and warps that the channels' pieces do not leave idle
-  const int per_seq = a.dim / (512 / N), warps = grid * (kStreamThreads / 32);
-  if (a.dim % (512 / N) == 0 && a.batch >= 2 * (warps / per_seq) && (warps / per_seq) * per_seq * 8 >= 7 * warps)
-    return launch_overlapped("step_channels_kernel", step_channels_kernel<T, BT, N>, dim3(grid), dim3(kStreamThreads), 0, st, a);
+  if constexpr (sizeof(T) == 2 && sizeof(BT) == 2) {
+    // whole pieces of channels per sequence, and warps that the channels' pieces do not leave idle
+    const int per_seq = a.dim / (512 / N), warps = grid * (kStreamThreads / 32);
+    if (a.dim % (512 / N) == 0 && a.batch >= 2 * (warps / per_seq) && (warps / per_seq) * per_seq * 8 >= 7 * warps)
+      return launch_overlapped("step_channels_kernel", step_channels_kernel<T, BT, N>, dim3(grid), dim3(kStreamThreads), 0, st, a);
+  }
   return launch_overlapped("step_stream_kernel", step_stream_kernel<T, BT, N, false>, dim3(grid), dim3(kStreamThreads), 0, st, a);
 }
 template <typename T, typename BT>

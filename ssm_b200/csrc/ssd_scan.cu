@@ -24,6 +24,7 @@
 #include "ssd_common.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace ssmb {
 
@@ -1172,19 +1173,18 @@ static int ssd_scan_launch(const ssm_ssd_args& a, const ScanMaps& maps, unsigned
 }
 
 // Heads per scan CTA: a divisor of the heads of one B / C group, so that a CTA's heads share their G.  One CTA runs per SM; the
-// long row blocks go first, then the short ones, each to the first SM that is free.  A long block costs 2 + d and a short one
-// 3 + 0.85 d head times (C / B tiles, G, pipeline fill; fitted to d = 8, 12, 16, 24 on 64 + 64 pieces).  Taken is the d with the
-// earliest end: within 2 % of the best divisor in ten dense shapes of both types from 1 x 300 steps of 80 heads (14.8 us) to 8 x 8192 of
-// 48 (387; figures of a form 8-14 % slower).  Of packed sequences the number of long blocks is a guess, good while they are longer than a chunk (24 in 16384 steps, 48
-// heads: 127 us, the best) and up to 15 % off when they are not (200 in 16384: 192 against 167 with 24; 64 in 4096, 8 heads: 26
-// against 16 with 4).  Counting whole waves of equal blocks instead chose d = 8 for 76 chunks of 48 heads: 143 us against 122 with 24.
+// long row blocks go first, then the short ones, each to the first SM that is free.  A long block costs 3 + d and a short one
+// 1.9 + 0.82 d head times (C / B tiles, G, pipeline fill; fitted to all divisors of 13 dense shapes, rms 2.3 %).  Taken is the d with the
+// earliest end: within 3 % of the best divisor in those shapes, from 1 x 178 steps of 20 heads (8.2 us) over 3 x 777 of 40 in two groups (22.3;
+// 25.6 with the next one) to 8 x 8192 of 48 (343), and in seven packed ones from 64 sequences in 512 steps of 8 heads (13.8; 19.0 with half as
+// many) to 24 in 16384 of 48 (105); of those 64 sequences in 16384 are 3 % off.
 static int scan_heads_per_cta(int hpg, int64_t longs, int64_t shorts) {
   const int64_t sms = sm_count();
   double best = 1e300;
   int heads = 1;
   for (int d = 1; d <= hpg && d <= 32; ++d) {
     if (hpg % d) continue;
-    const double lng = 2.0 + d, shrt = 3.0 + 0.85 * d;
+    const double lng = 3.0 + d, shrt = 1.9 + 0.82 * d;
     const int64_t n = shorts * (hpg / d), q = longs * (hpg / d) / sms, r = longs * (hpg / d) % sms;  // r SMs run q + 1 long blocks, the others q
     // how many short blocks can have ended by t
     auto room = [&](double t) {
@@ -1211,10 +1211,12 @@ static int ssd_launch(const ssm_ssd_args& a, cudaStream_t st) {
   const int nchunks = a.num_seqs ? a.num_chunks : (a.len + kQ - 1) / kQ;
   const int walks = a.num_seqs ? a.num_seqs : a.batch;  // sequences that the state kernel walks
   const int hpg = a.heads / a.groups;
-  // (of packed sequences about every second one ends in a chunk without a long block, and a table with room to spare holds half a chunk per
-  // sequence more than there are)
-  const int64_t blocks = a.num_seqs ? std::min<int64_t>(nchunks, a.len / kQ + (a.num_seqs + 1) / 2) : (int64_t)a.batch * nchunks;
-  const int hpc = scan_heads_per_cta(hpg, (a.num_seqs ? std::max<int64_t>(blocks - a.num_seqs / 2, 0) : blocks) * a.groups, blocks * a.groups);
+  int64_t shorts = (int64_t)a.batch * nchunks, longs = shorts;
+  if (a.num_seqs) {  // as many as sequences have that are cut at random: where they are cut is not known here
+    const double mean = (double)a.len / a.num_seqs, chunks = a.num_seqs / (1.0 - std::exp(-kQ / mean));
+    shorts = std::min<int64_t>(nchunks, std::llround(chunks)), longs = std::min<int64_t>(shorts, std::llround(chunks * std::exp(-kBlk / mean)));
+  }
+  const int hpc = scan_heads_per_cta(hpg, longs * a.groups, shorts * a.groups);
   const int nparts = a.heads / hpc;
   if (a.phase != 2 && !a.reverse) {
     ssd_cumsum_kernel<T><<<dim3((a.heads + kCumHeads - 1) / kCumHeads, nchunks, a.batch), kQ, 0, st>>>(a, nchunks);

@@ -819,17 +819,19 @@ __device__ __forceinline__ void ssd_scan_body(const ssm_ssd_args& a, const ScanM
   auto epilogue = [&](int h, int buf, float ct, const uint4 (&xr)[kXR]) {
     const float escale = ex2_approx(ct);
     const float2 es2 = make_float2(escale, escale);
-    float yi[kEC], ys[kEC];
-    tc::tmem_ld16_pair(tmem + lane_base + 256 + buf * 128 + wg * kEC, tmem + lane_base + 320 + buf * 128 + wg * kEC, yi, ys);
     const float Dh = (skip_explicit && !a.d_has_p) ? __ldg(a.D + h) : 0.f;
     const bool dots = a.row_dots != nullptr;
     float dot = 0.f;  // row_dots: this thread's 16 columns of  sum_p y[p] z[p]  (y before the skip term and unrounded)
 #pragma unroll
     for (int q = 0; q < kEU; ++q) {
+      // eight columns at a time: sixteen left too few registers, and the instance with a skip weight per channel spilled 130 bytes (1 x 1024 steps of
+      // 24 heads 11.8 us, 10.1 so; mirrored 2 x 4001 of 48 55.0 and 52.6; the others equal)
       float2 f2[4];
+      float yi[8], ys[8];
+      tc::tmem_ld8_pair(tmem + lane_base + 256 + buf * 128 + wg * kEC + q * 8, tmem + lane_base + 320 + buf * 128 + wg * kEC + q * 8, yi, ys);
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        f2[e] = __ffma2_rn(es2, make_float2(ys[q * 8 + 2 * e], ys[q * 8 + 2 * e + 1]), make_float2(yi[q * 8 + 2 * e], yi[q * 8 + 2 * e + 1]));
+        f2[e] = __ffma2_rn(es2, make_float2(ys[2 * e], ys[2 * e + 1]), make_float2(yi[2 * e], yi[2 * e + 1]));
       float zv[8];
       if (has_z) {
         Vec16<T> zz;

@@ -214,23 +214,19 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Two of them under one wait.
-__device__ __forceinline__ void tmem_ld16_pair(uint32_t taddr0, uint32_t taddr1, float (&v)[16], float (&w)[16]) {
-  uint32_t r[16], q[16];  // early-clobber: the second address is read after the first load has been issued
+// Eight columns of two accumulators under one wait.
+__device__ __forceinline__ void tmem_ld8_pair(uint32_t taddr0, uint32_t taddr1, float (&v)[8], float (&w)[8]) {
+  uint32_t r[8], q[8];  // early-clobber: the second address is read after the first load has been issued
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n\t"
       "tcgen05.wait::ld.sync.aligned;\n"
-      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "=&r"(r[8]), "=&r"(r[9]),
-        "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]), "=&r"(q[0]), "=&r"(q[1]), "=&r"(q[2]),
-        "=&r"(q[3]), "=&r"(q[4]), "=&r"(q[5]), "=&r"(q[6]), "=&r"(q[7]), "=&r"(q[8]), "=&r"(q[9]), "=&r"(q[10]), "=&r"(q[11]), "=&r"(q[12]),
-        "=&r"(q[13]), "=&r"(q[14]), "=&r"(q[15])
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "=&r"(q[0]), "=&r"(q[1]), "=&r"(q[2]), "=&r"(q[3]),
+        "=&r"(q[4]), "=&r"(q[5]), "=&r"(q[6]), "=&r"(q[7])
       : "r"(taddr0), "r"(taddr1)
       : "memory");
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]), w[i] = __uint_as_float(q[i]);
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]), w[i] = __uint_as_float(q[i]);
 }
 
 // 32 lanes x 32 consecutive fp32 columns -> 32 registers per thread (thread = TMEM lane).

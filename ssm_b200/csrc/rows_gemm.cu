@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
       }
       pdl_wait();
       const uint32_t stage0 = tc::smem_u32(base);
-      int st = 0, parity = 1, kc = kb0 * kGemmK;
+      int st = 0, parity = 1, kc = kb0 * kGemmK, issued = 0;
       for (int i = 0; i < kb1 - kb0; ++i, kc += kGemmK) {
         const uint32_t at = stage0 + st * stage_bytes, bar = full + 8 * st;
         if (i >= ahead) {
@@ -90,7 +90,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
         }
         tma_load_2d(at + kGemmWBytes, &maps.x, bar, kc, tok0);
         if (++st == g.stages) st = 0, parity ^= 1;
+        issued = i + 1;
       }
+      // no copy is under way when the block ends, also where a wait has run out
+      for (int i = max(0, issued - g.stages); i < issued; ++i)
+        if (!tc::mbar_wait(full + 8 * (i % g.stages), (i / g.stages) & 1)) ran_out();
     }
     __syncwarp();
   } else if (warp == 1) {

@@ -258,7 +258,10 @@ extern "C" int ssmb_rows_gemm(const ssmb_rows_gemm_args* a, void* stream) {
   if (int rc = encode_matrix(&maps.x, a->x, a->batch, a->k, a->ldx, g.n, a->io_dtype)) return rc;
   const size_t stage = kGemmWBytes + (size_t)g.n * kGemmK * 2, part = (size_t)g.n * kGemmRows * 4;
   const int steps = (g.nkb + g.splits - 1) / g.splits;
-  g.stages = (int)((tiles * tok_tiles * g.splits > sms ? kGemmSmem / 2 : kGemmSmem) / stage);  // more CTAs than SMs: two of them on an SM
+  // more CTAs than SMs: half the ring, so that two of them share an SM, where the accumulator tile that lies over the ring leaves room for it (up to
+  // 208 token rows; 3 KB per CTA for the alignment, the barriers and the system)
+  const bool two = tiles * tok_tiles * g.splits > sms && 2 * ((part > kGemmSmem / 2 ? part : kGemmSmem / 2) + 3 * 1024) <= 228 * 1024;
+  g.stages = (int)((two ? kGemmSmem / 2 : kGemmSmem) / stage);
   g.stages = g.stages > kGemmMaxStages ? kGemmMaxStages : g.stages < 2 ? 2 : g.stages;
   g.stages = g.stages > steps ? steps : g.stages;
   size_t smem = g.stages * stage;

@@ -23,7 +23,9 @@ typedef struct {
   void* out[SSMB_GEMM_MATS];
   int64_t ldo[SSMB_GEMM_MATS];
   int32_t* status;
-  int32_t weights_ahead, reserved0;
+  int32_t weights_ahead;
+  int32_t plan_rows, plan_splits; /* token rows of a CTA (a multiple of 16) and CTAs that share its columns (1, 2, 4, 8); 0: chosen */
+  int32_t reserved0;
 } ssmb_rows_gemm_args;
 int ssmb_rows_gemm_supported(int32_t batch, int32_t k, int64_t ldx, int32_t io_dtype);
 int ssmb_rows_gemm(const ssmb_rows_gemm_args* args, void* stream);

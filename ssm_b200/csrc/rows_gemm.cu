@@ -9,6 +9,8 @@
 // distributed shared memory: no workspace, no second launch, and the order of the sum is fixed.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "decode_parts.h"
 #include "ssd_common.cuh"
 
@@ -207,22 +209,50 @@ static int gemm_launch(const GemmMaps& maps, const GemmShape& g, dim3 grid, size
   return launch_status("rows_gemm_kernel");
 }
 
-// Token rows of a CTA and CTAs that share its columns.
+// Clusters of the kernel that run at once.  A cluster lies within one GPC: 74 of two, 33 of four, 15 of eight CTAs on 148 SMs.
+static int gemm_clusters(int splits) {
+  static std::atomic<int> known[64][4];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return sm_count() / splits;
+  std::atomic<int>& n = known[dev][splits == 2 ? 1 : splits == 4 ? 2 : 3];
+  if (n == 0) {
+    auto kern = rows_gemm_kernel<__nv_bfloat16>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(splits), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kGemmSmem, cfg.attrs = attr, cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) != cudaSuccess || fit < 1) cudaGetLastError(), fit = sm_count() / splits;
+    n = fit;
+  }
+  return n;
+}
+
+// Token rows of a CTA and CTAs that share its columns: the least estimated time.  Operands at what one SM and all of them together read (from
+// the L2: token tiles share the weights), the accumulator's way out per token row, and the exchange of partial sums.  Clusters that do not
+// run at once take a second round that is as long as the first (2048 rows of 4096 columns, 17 to 128 sequences: 10.8 to 14.4 us in 16 clusters
+// of eight, 6.6 to 8.5 in clusters of four) and are not considered.  Against all plans of 203 products of 17 to 256 rows with 320 to 10576 weight rows
+// and 48 to 5120 columns: median 0.2 % above the best, nine in ten within 7 %, the worst 16 % (64 rows, 320 x 640: 4.0 us against 3.4).
 struct GemmPlan {
   int n, splits;
 };
+constexpr double kSmRate = 115e3, kAllRate = 11e6;                               // bytes per us
+constexpr double kReadOut = 0.008, kExchange = 0.6, kExchangePerRow = 0.011;  // us
 static GemmPlan gemm_plan(int tiles, int batch, int nkb, int sms) {
   GemmPlan best{16, 1};
-  double cost = 1e300;
-  for (int p = 1; p <= 8; p *= 2) {
-    const int n = ((batch + p - 1) / p + 15) / 16 * 16, toks = (batch + n - 1) / n;
-    for (int s = 1; s <= 8 && s <= nkb; s *= 2) {
-      const int ctas = tiles * toks * s, steps = (nkb + s - 1) / s;
-      const double bytes = (double)steps * (kGemmWBytes + n * kGemmK * 2.0), per_sm = ctas > sms ? (double)((ctas + sms - 1) / sms) : 1.0;
-      double c = bytes / 115e3;
-      if (c < ctas * bytes / 9e6) c = ctas * bytes / 9e6;
-      c = c * 1.0 + (per_sm > 1.0 ? (per_sm - 1.0) * bytes / 115e3 : 0.0) + n * 0.008 + (s > 1 ? 0.6 + n * 0.011 : 0.0);
-      if (c < cost) cost = c, best = GemmPlan{n, s};
+  double least = 1e300;
+  for (int s = 1; s <= 8 && s <= nkb; s *= 2) {
+    const int clusters = s > 1 ? gemm_clusters(s) : 0, steps = (nkb + s - 1) / s;
+    for (int p = 1; p <= 8; p *= 2) {
+      const int n = ((batch + p - 1) / p + 15) / 16 * 16, toks = (batch + n - 1) / n, ctas = tiles * toks * s;
+      if (s > 1 && tiles * toks > clusters) continue;
+      const double bytes = (double)steps * (kGemmWBytes + n * kGemmK * 2.0), rounds = (ctas + sms - 1) / sms;
+      double t = bytes / kSmRate;
+      if (t < ctas * bytes / kAllRate) t = ctas * bytes / kAllRate;
+      t += (rounds - 1) * bytes / kSmRate + n * kReadOut + (s > 1 ? kExchange + n * kExchangePerRow : 0.0);
+      if (t < least) least = t, best = GemmPlan{n, s};
     }
   }
   return best;
@@ -252,7 +282,14 @@ extern "C" int ssmb_rows_gemm(const ssmb_rows_gemm_args* a, void* stream) {
     g.rows[i] = a->rows[i], g.tiles_end[i] = tiles, g.out[i] = a->out[i], g.ldo[i] = a->ldo[i];
   }
   const int sms = sm_count();
-  const GemmPlan plan = gemm_plan(tiles, a->batch, g.nkb, sms);
+  GemmPlan plan;
+  if (a->plan_rows) {
+    plan = GemmPlan{a->plan_rows, a->plan_splits};
+    SSM_REQUIRE(plan.n >= 16 && plan.n <= SSMB_GEMM_MAX_ROWS && plan.n % 16 == 0 && (plan.splits == 1 || plan.splits == 2 || plan.splits == 4 || plan.splits == 8) &&
+                    plan.splits <= g.nkb, SSM_ERR_UNSUPPORTED, "rows_gemm: unsupported plan");
+  } else {
+    plan = gemm_plan(tiles, a->batch, g.nkb, sms);
+  }
   g.n = plan.n, g.splits = plan.splits;
   const int tok_tiles = (a->batch + g.n - 1) / g.n;
   if (int rc = encode_matrix(&maps.x, a->x, a->batch, a->k, a->ldx, g.n, a->io_dtype)) return rc;

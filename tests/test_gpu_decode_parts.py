@@ -19,15 +19,34 @@ pytestmark = pytest.mark.gpu
 class _GemmArgs(ctypes.Structure):
     _fields_ = [("batch", ctypes.c_int32), ("k", ctypes.c_int32), ("mats", ctypes.c_int32), ("io_dtype", ctypes.c_int32), ("ldx", ctypes.c_int64),
                 ("x", ctypes.c_void_p), ("w", ctypes.c_void_p * 5), ("rows", ctypes.c_int32 * 5), ("out", ctypes.c_void_p * 5), ("ldo", ctypes.c_int64 * 5),
-                ("status", ctypes.c_void_p), ("weights_ahead", ctypes.c_int32), ("reserved0", ctypes.c_int32)]
+                ("status", ctypes.c_void_p), ("weights_ahead", ctypes.c_int32), ("plan_rows", ctypes.c_int32), ("plan_splits", ctypes.c_int32),
+                ("reserved0", ctypes.c_int32)]
 
 
-# one element of everything; whole tiles; token rows, weight rows and columns that end inside one; columns split over 2, 4 and 8 CTAs;
-# token rows in several CTAs; an output whose rows start on no 8-byte boundary (odd row counts); rows of x that lie apart
+# one element of everything; whole tiles; token rows, weight rows and columns that end inside one; an output whose rows start on no 8-byte
+# boundary (odd row counts); rows of x that lie apart; more CTAs than SMs
 @pytest.mark.parametrize("nb,k,rows,pad,dtype", [(1, 8, [1], 0, torch.bfloat16), (16, 64, [128], 0, torch.float16), (17, 72, [129, 5], 8, torch.bfloat16),
                                                  (33, 200, [300, 20, 7], 0, torch.float16), (255, 128, [128, 130], 24, torch.bfloat16), (256, 2112, [200], 0, torch.bfloat16),
-                                                 (64, 5120, [192], 0, torch.float16), (100, 768, [1536, 1536, 128, 128, 24], 0, torch.bfloat16), (256, 160, [5120], 32, torch.bfloat16)])
+                                                 (64, 5120, [192], 0, torch.float16), (100, 768, [1536, 1536, 128, 128, 24], 0, torch.bfloat16), (256, 160, [5120], 32, torch.bfloat16), (200, 128, [19300], 0, torch.float16)])
 def test_rows_product_matches_double_precision(nb, k, rows, pad, dtype):
+    _check_product(nb, k, rows, pad, dtype)
+
+
+# every split over 2, 4 and 8 CTAs at 16 to 256 token rows of a CTA: one pass through the stages and several; columns that are no multiple of the
+# split; token rows that end inside a CTA's; two CTAs on an SM (more CTAs than SMs, up to 208 token rows) and one with the whole ring (more)
+@pytest.mark.parametrize("nb,k,rows,n,splits", [(17, 320, [130], 16, 2), (64, 5120, [2560], 64, 4), (128, 5120, [2560], 128, 2), (128, 2112, [200, 7], 64, 8), (255, 1032, [300], 256, 4),
+                                                (256, 5120, [256], 256, 8), (100, 520, [129], 112, 8), (200, 640, [19200], 208, 1), (250, 640, [19200], 256, 1), (256, 640, [9600], 128, 4)])
+def test_rows_product_of_every_split_matches_double_precision(nb, k, rows, n, splits):
+    _check_product(nb, k, rows, 0, torch.bfloat16, n, splits)
+
+
+@pytest.mark.parametrize("n,splits", [(8, 1), (24, 1), (272, 1), (16, 3), (16, 16), (32, 4)])
+def test_plans_that_are_none_are_refused(n, splits):
+    with pytest.raises(AssertionError):
+        _check_product(32, 128, [128], 0, torch.bfloat16, n, splits)
+
+
+def _check_product(nb, k, rows, pad, dtype, n=0, splits=0):
     lib = _lib.load()
     lib.ssmb_rows_gemm.restype = ctypes.c_int
     gen = torch.Generator(device="cuda").manual_seed(nb + k)
@@ -36,7 +55,8 @@ def test_rows_product_matches_double_precision(nb, k, rows, pad, dtype):
     ws = [(rnd(r, k) / k ** 0.5).to(dtype) for r in rows]
     outs = [torch.full((nb, r + 3), 9.0, device="cuda", dtype=dtype) for r in rows]  # rows that lie apart: nothing beyond them is written
     status = torch.zeros(1, dtype=torch.int32).pin_memory()
-    a = _GemmArgs(batch=nb, k=k, mats=len(ws), io_dtype=1 if dtype == torch.bfloat16 else 2, ldx=k + pad, x=x.data_ptr(), status=status.data_ptr())
+    a = _GemmArgs(batch=nb, k=k, mats=len(ws), io_dtype=1 if dtype == torch.bfloat16 else 2, ldx=k + pad, x=x.data_ptr(), status=status.data_ptr(),
+                  plan_rows=n, plan_splits=splits)
     for i, (w, o) in enumerate(zip(ws, outs)):
         a.w[i], a.rows[i], a.out[i], a.ldo[i] = w.data_ptr(), w.shape[0], o.data_ptr(), o.stride(0)
     for ahead in (0, 1):

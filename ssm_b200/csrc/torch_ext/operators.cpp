@@ -1249,7 +1249,11 @@ py::object mamba2_mixer(const Tensor& u, const Tensor& in_z, const Tensor& in_x,
   c10::cuda::CUDAGuard guard(u.device());
   Tensor u2 = u.reshape({nb * nl, dm});
   auto proj = [&](const Tensor& w) { return at::mm(u2, w.t()).view({nb, nl, w.size(0)}); };
-  auto conv = [&](const Tensor& t, const Tensor& w, const OptTensor& b) { return invoke_call(c10::make_intrusive<ConvCall>(t, w, b, "silu", OptTensor()))[0]; };
+  auto conv = [&](const Tensor& t, const Tensor& w, const OptTensor& b) {
+    const bool square = nl == t.size(2);  // as many steps as channels: (B, L, C) would be taken for (B, C, L)
+    Tensor y = invoke_call(c10::make_intrusive<ConvCall>(square ? t.transpose(1, 2) : t, w, b, "silu", OptTensor()))[0];
+    return square ? y.transpose(1, 2).contiguous() : y;
+  };
   Tensor x = conv(proj(in_x), wx, bx).view({nb, nl, nh, hp}), B = conv(proj(in_B), wB, bB).view({nb, nl, g, n}), C = conv(proj(in_C), wC, bC).view({nb, nl, g, n});
   Tensor z = proj(in_z).view({nb, nl, nh, hp}), dt = proj(in_dt);
   Tensor y = std::get<0>(ssd_scan(x, dt, at::exp(A_log).neg_(), B, C, D, z, dt_bias, true, OptTensor(), chunk));

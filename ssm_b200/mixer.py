@@ -224,13 +224,14 @@ def mamba2_mixer_forward(ops: Any, w: dict, cfg: dict, u: Tensor, group=None, sh
         halos = posted.wait()
 
     def conv(t, name, halo):
-        if halo is None:
-            return ops.dw_causal_conv(t, w[name], w[name + "_b"], "silu")
-        return ops.dw_causal_conv(t, w[name], w[name + "_b"], "silu", halo=halo)
+        kw = {} if halo is None else {"halo": halo}
+        if t.shape[1] == t.shape[2]:  # as many steps as channels: (B, L, C) would be taken for (B, C, L)
+            return ops.dw_causal_conv(t.transpose(1, 2), w[name], w[name + "_b"], "silu", **kw).transpose(1, 2)
+        return ops.dw_causal_conv(t, w[name], w[name + "_b"], "silu", **kw)
 
-    x = conv(px, "conv_x", halos[0]).view(nb, nl, nh, hp)
-    Bm = conv(pB, "conv_B", halos[1]).view(nb, nl, g, n)
-    Cm = conv(pC, "conv_C", halos[2]).view(nb, nl, g, n)
+    x = conv(px, "conv_x", halos[0]).reshape(nb, nl, nh, hp)
+    Bm = conv(pB, "conv_B", halos[1]).reshape(nb, nl, g, n)
+    Cm = conv(pC, "conv_C", halos[2]).reshape(nb, nl, g, n)
     A = -torch.exp(w["A_log"])
     if sharded:
         from . import seqpar

@@ -208,3 +208,14 @@ def test_mamba2_matches_composed_operators(nb, nl, dm, groups, dtype):
             want = block(hidden, res)
     assert ops.mamba2_mixer(hidden, block._weights(), block._cfg()) is None  # gradients enabled
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("nl", [128, 256])  # as many steps as channels of B and C, of x
+def test_mamba2_of_as_many_steps_as_channels(nl, grad):
+    torch.manual_seed(4)
+    block = Mamba2Block(128, device="cuda", dtype=torch.bfloat16)
+    u = torch.randn(2, nl + 1, 128, device="cuda").bfloat16()
+    with torch.set_grad_enabled(grad):
+        got, want = block.mixer_forward(u[:, :nl]), block.mixer_forward(u)[:, :nl]
+    _near(got.detach(), want.detach(), torch.bfloat16, "out")

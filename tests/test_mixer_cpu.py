@@ -131,3 +131,15 @@ def test_mamba2_block_runs_on_the_oracle_and_matches_a_token_loop():
         ref = y @ m.out_proj.t()
     torch.testing.assert_close(res, r, rtol=1e-6, atol=1e-6)
     torch.testing.assert_close(out, ref, rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("nl", [16, 32])  # as many steps as channels of B and C, of x
+def test_mamba2_block_of_as_many_steps_as_channels(nl):
+    """What follows does not change what precedes: a longer sequence has the same first outputs."""
+    from ssm_b200.mixer import Mamba2Block
+
+    torch.manual_seed(3)
+    m = Mamba2Block(16, d_state=8, d_conv=3, expand=2, headdim=8, ngroups=2, chunk_size=4, ops=orc)
+    u = torch.randn(2, nl + 1, 16)
+    with torch.no_grad():
+        torch.testing.assert_close(m.mixer_forward(u[:, :nl]), m.mixer_forward(u)[:, :nl], rtol=1e-4, atol=1e-5)

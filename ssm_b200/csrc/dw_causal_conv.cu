@@ -751,11 +751,11 @@ __device__ __forceinline__ float2 silu_grad2(float2 p) {
 }
 
 // The same walk for the width that state-space models use (4) and channels in whole groups of four: taps, windows and
-// accumulators are pairs of channels for the packed-fp32 instructions, the taps exist once, and the eight steps of a batch of loads run
-// without any check unless they touch an end of the tile.  Bound by instructions (about 13 per element; the kernel above
-// takes 31), hence four CTAs per SM and a tile length that fills whole waves (conv_cl_tile).
-// (4, 4093, 2560) bf16, 251 MB: 154 us with the kernel above, 73 us with this one (3.4 TB/s; two channels per thread and six CTAs
-// more per SM: 91).  Narrow tensors, NT = 512: (2, 16384, 128) bf16 72 -> 18 us.
+// accumulators are pairs of channels for the packed-fp32 instructions, the taps exist once, rows travel through a ring in shared memory, and
+// the four steps of a batch run without any check unless they touch an end of the tile.  512 threads per SM, half of their issue slots
+// busy, and a tile length that fills whole waves (conv_cl_tile).
+// (4, 4093, 2560) bf16, 251 MB: 154 us with the kernel above, 63 us with this one (4.0 TB/s).  Narrow tensors, NT = 512: (2, 16384, 128) bf16
+// 72 -> 14 us.
 constexpr int kConvRing = 4, kConvBatch = 4;  // batches of the ring, steps of a batch
 constexpr size_t conv_ring_bytes(int threads) { return (size_t)kConvRing * kConvBatch * 2 * 8 * threads; }
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {

@@ -1,13 +1,11 @@
 // Residual add fused with LayerNorm / RMSNorm, forward and backward, sm_100a.
 //
-// HBM-bound: each row is read once into registers (x and residual as 16-byte vectors),
-// the mean and the centred variance are both computed from those registers (the two-pass
-// form of the specification, no E[x^2]-mean^2 cancellation), and y / residual_out are
-// written once.  A row is owned by a group of G threads (a warp, or 128 / 512 threads for
-// wide rows).  The backward kernel is persistent: every thread keeps the weight / bias
-// gradient of its own columns in registers across all rows its CTA visits, the CTA writes
-// one partial row, and a second small kernel folds the partials -- no atomics, bitwise
-// reproducible.
+// HBM-bound: each row is read once, the mean and the centred variance are both computed from what was read (the two-pass
+// form of the specification, no E[x^2]-mean^2 cancellation), and y / residual_out are written once.  Forward: a row is
+// owned by a warp or by 128 or 512 threads and lies in their registers, x and residual as 16-byte vectors.  Backward: a warp, or 64 to 512
+// threads, granules of four columns, the next row on its way into shared memory.  The backward kernel is persistent:
+// every thread keeps the weight / bias gradient of its own columns in registers across all rows its CTA visits, the CTA
+// writes one partial row, and a second small kernel folds the partials -- no atomics, bitwise reproducible.
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -17,43 +15,10 @@
 namespace ssmb {
 
 constexpr int kNormFwdChunks = 4;  // 16-byte chunks of x per thread, forward
-constexpr int kNormBwdChunks = 4;  // widest backward configuration: 512 threads x 4 chunks
+constexpr int kNormBwdChunks = 4;  // widest backward configuration: 512 threads x 4 chunks of 16 bytes
 constexpr int kNormBwdMaxCtas = 592;  // 4 per SM on a 148-SM part
 
-// V consecutive elements of run-time type -> fp32
-template <int V>
-__device__ __forceinline__ void load_dyn_vec(const void* base, int64_t i, int dtype, float (&f)[V]) {
-  if (dtype == SSM_F32) {
-    const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i);
-#pragma unroll
-    for (int k = 0; k < V / 4; ++k) {
-      const float4 v = __ldcs(p + k);
-      f[4 * k] = v.x, f[4 * k + 1] = v.y, f[4 * k + 2] = v.z, f[4 * k + 3] = v.w;
-    }
-  } else if constexpr (V == 8) {
-    const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + i));
-    if (dtype == SSM_BF16) {
-      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) f[k] = __bfloat162float(e[k]);
-    } else {
-      const __half* e = reinterpret_cast<const __half*>(&raw);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) f[k] = __half2float(e[k]);
-    }
-  } else {
-    const uint2 raw = __ldcs(reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(base) + i));
-    if (dtype == SSM_BF16) {
-      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) f[k] = __bfloat162float(e[k]);
-    } else {
-      const __half* e = reinterpret_cast<const __half*>(&raw);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) f[k] = __half2float(e[k]);
-    }
-  }
-}
+// fp32 -> V consecutive elements of run-time type
 template <int V>
 __device__ __forceinline__ void store_dyn_vec(void* base, int64_t i, int dtype, const float (&f)[V]) {
   if (dtype == SSM_F32) {

@@ -723,9 +723,9 @@ def ssd_scan(
             raise ValueError("return_varlen_states needs cu_seqlens.")
         Y, final = _ssd_call(X, dt, A, B, C, D, z, dt_bias, dt_softplus, initial_states, chunk_size, check_status, dual)
         return (Y, final) if return_final_states else Y
-    # packed sequences: every sequence is its own scan from a zero state (chunks counted from its first token); the boundaries are
-    # host integers (one read of cu_seqlens).  Without gradients the tensor-core kernels take them all at once, otherwise the
-    # scans are separate dense problems
+    # packed sequences: every sequence is its own scan from a zero state (chunks counted from its first token).  Without gradients the
+    # tensor-core kernels take them all at once (boundaries on the device are used where they lie and checked behind the launches); otherwise
+    # they are read by the host and the scans are separate dense problems
     if X.ndim != 4 or X.shape[0] != 1:
         raise ValueError("cu_seqlens needs a batch of one (sequences packed along L).")
     if initial_states is not None and seq_reset:

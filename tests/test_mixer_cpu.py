@@ -3,6 +3,7 @@ plain batch-major restatement of the same block, and its one-token `step` must r
 
 from __future__ import annotations
 
+import pytest
 import torch
 
 from oracle import ssm_oracle as orc
@@ -79,7 +80,6 @@ def test_step_reads_weights_that_are_no_plain_parameters():
 
 
 def test_constructor_rejects_bad_arguments():
-    import pytest
 
     with pytest.raises(ValueError):
         Mamba1Block(16, dt_rank="big", ops=orc)

@@ -598,13 +598,13 @@ bool library_product(int64_t nb, const Tensor& w) { return nb > 128 && w.size(0)
 
 // What the separate calls refuse, or answer in another type, goes to them: shapes that agree in their number of elements only, tangents, autocast
 // to another type.
-bool by_parts(const Tensor& tok, std::initializer_list<std::pair<const Tensor*, std::initializer_list<int64_t>>> shapes, std::initializer_list<const OptTensor*> tangents) {
+bool by_parts(const Tensor& tok, std::initializer_list<std::pair<const Tensor*, std::initializer_list<int64_t>>> shapes, std::initializer_list<const Tensor*> tangents) {
   if (tok.size(1) % 8 != 0 || tok.size(0) > SSMB_GEMM_MAX_ROWS) return false;
   if (at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) != tok.scalar_type()) return false;
   for (const auto& [t, shape] : shapes)
     if (t->sizes() != at::IntArrayRef(shape)) return false;
-  for (const OptTensor* t : tangents)
-    if (t->has_value() && (*t)->_fw_grad(0).defined()) return false;
+  for (const Tensor* t : tangents)
+    if (t && t->_fw_grad(0).defined()) return false;
   return true;
 }
 // conv weights (C, K), or (C, 1, K)
@@ -732,7 +732,9 @@ py::object mamba1_step(const Tensor& tok, const OptTensor& residual, const Tenso
       return py::cast(out);
     }
   }
-  if (fused && di % 8 == 0 && conv_weight(conv_w, di, k) && by_parts(tok, {{&D, {di}}, {&dt_bias, {di}}, {norm_w.has_value() ? &*norm_w : &D, {norm_w.has_value() ? dm : di}}}, {&residual, &norm_w}))
+  if (fused && di % 8 == 0 && conv_weight(conv_w, di, k) &&
+      by_parts(tok, {{&D, {di}}, {&dt_bias, {di}}, {norm_w.has_value() ? &*norm_w : &D, {norm_w.has_value() ? dm : di}}},
+               {residual.has_value() ? &*residual : nullptr, norm_w.has_value() ? &*norm_w : nullptr, &out_proj}))
     return mamba1_parts(tok, residual, conv_state, ssm_state, in_x, in_z, conv_w, conv_b, x_proj, dt_proj, dt_bias, A, a_log, D, out_proj, norm_w, eps);
   Tensor x = at::matmul(tok, in_x.t()), z = at::matmul(tok, in_z.t());
   Tensor u = dw_causal_conv_update(conv_state, x, conv_w, conv_b, "silu");
@@ -786,7 +788,7 @@ Tensor mamba2_step(const Tensor& tok, const Tensor& conv_x, const Tensor& conv_B
     if (launched(ssm_mamba2_decode(&a, stream_of(tok)))) return out;
   }
   if (fused && di % 8 == 0 && conv_weight(wx, di, k) && conv_weight(wB, g * n, k) && conv_weight(wC, g * n, k) &&
-      by_parts(tok, {{&conv_x, {nb, di, k}}, {&conv_B, {nb, g * n, k}}, {&conv_C, {nb, g * n, k}}, {&A, {nh}}, {&norm_w, {di}}}, {}))
+      by_parts(tok, {{&conv_x, {nb, di, k}}, {&conv_B, {nb, g * n, k}}, {&conv_C, {nb, g * n, k}}, {&A, {nh}}, {&norm_w, {di}}}, {&norm_w, &out_proj}))
     return mamba2_parts(tok, conv_x, conv_B, conv_C, ssm_state, in_z, in_x, in_B, in_C, in_dt, wx, bx, wB, bB, wC, bC, dt_bias, A, a_log, D, norm_w, out_proj, eps);
   Tensor z = at::matmul(tok, in_z.t());
   Tensor x = dw_causal_conv_update(conv_x, at::matmul(tok, in_x.t()), wx, bx, "silu");

@@ -220,3 +220,37 @@ def test_captured_steps_match_plain_ones(cls, nb, dm):
     for a, b in zip(flat(plain), flat(captured)):
         assert torch.equal(a, b)
     del graph
+
+
+@pytest.mark.parametrize("cls", ["Mamba1Block", "Mamba2Block"])
+def test_a_tangent_of_the_output_projection_goes_through_a_step(cls):
+    import torch.autograd.forward_ad as fwd
+    from ssm_b200 import mixer, ops
+
+    torch.manual_seed(3)
+    block = getattr(mixer, cls)(64, device="cuda", dtype=torch.bfloat16)
+    w = {n: p.detach() for n, p in block.named_parameters()}
+    other, tok = torch.randn_like(w["out_proj"]), torch.randn(20, 64, device="cuda").bfloat16()
+
+    def step(out_proj):
+        cache = block.allocate_inference_cache(20)
+        if cls == "Mamba1Block":
+            return ops.mamba1_step(tok, None, *cache, {**w, "out_proj": out_proj})
+        return ops.mamba2_step(tok, *cache, {**w, "out_proj": out_proj})
+
+    want = step(other)
+    with fwd.dual_level():
+        got = fwd.unpack_dual(step(fwd.make_dual(w["out_proj"], other))).tangent
+    assert got is not None and (got.double() - want.double()).norm() <= 1e-2 * want.double().norm()
+
+
+def test_a_tangent_of_the_gated_norm_is_refused():
+    import torch.autograd.forward_ad as fwd
+    from ssm_b200 import ops
+    from ssm_b200.mixer import Mamba2Block
+
+    block = Mamba2Block(64, device="cuda", dtype=torch.bfloat16)
+    w = {n: p.detach() for n, p in block.named_parameters()}
+    with fwd.dual_level(), pytest.raises(NotImplementedError, match="forward-mode"):
+        dual = {**w, "norm_w": fwd.make_dual(w["norm_w"], torch.ones_like(w["norm_w"]))}
+        ops.mamba2_step(torch.randn(20, 64, device="cuda").bfloat16(), *block.allocate_inference_cache(20), dual)

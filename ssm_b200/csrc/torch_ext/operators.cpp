@@ -1052,12 +1052,16 @@ std::tuple<Tensor, Tensor> ssd_scan(const Tensor& X, const Tensor& dt, const Ten
 // of host time per training step for 0.12 ms of device time (d_model 256, 256 steps).  The calls below are the same products and
 // operators behind one node; products that add into a gradient do so in their epilogue instead of a pass of their own.
 //
-// They stand for the composed form only where nothing can tell the difference: no tracing, autocast or saved-tensor hooks, plain types.
+// They stand for the composed form only where nothing can tell the difference: no tracing, autocast or saved-tensor hooks, plain types, no weight with a
+// tangent or of a transform (torch.func), which a product in front of or behind the operators may carry.
+bool transformed(const Tensor& t) {
+  return t._fw_grad(0).defined() || t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::FuncTorchBatched}));
+}
 bool composed_only(const Tensor& x, std::initializer_list<const Tensor*> weights) {
   if (at::tracer::impl::is_dispatch_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || at::SavedTensorDefaultHooks::get_hooks().has_value()) return true;
   if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || !io_dtype_ok(x)) return true;
   for (const Tensor* w : weights)
-    if (w->scalar_type() != x.scalar_type() || w->dim() != 2 || w->device() != x.device()) return true;
+    if (w->scalar_type() != x.scalar_type() || w->dim() != 2 || w->device() != x.device() || transformed(*w)) return true;
   return false;
 }
 

@@ -219,3 +219,40 @@ def test_mamba2_of_as_many_steps_as_channels(nl, grad):
     with torch.set_grad_enabled(grad):
         got, want = block.mixer_forward(u[:, :nl]), block.mixer_forward(u)[:, :nl]
     _near(got.detach(), want.detach(), torch.bfloat16, "out")
+
+
+def _other_out_proj(block):
+    """Weights without gradients and another output projection, in which a mixer is linear."""
+    w = {n: p.detach() for n, p in block.named_parameters()}
+    return w, torch.randn_like(w["out_proj"])
+
+
+@pytest.mark.parametrize("train", [False, True])
+def test_mamba1_tangent_of_the_output_projection(train):
+    import torch.autograd.forward_ad as fwd
+    from ssm_b200.mixer import mamba1_mixer_forward
+
+    torch.manual_seed(5)
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    w, other = _other_out_proj(block)
+    hidden = torch.randn(2, 33, 64, device="cuda").bfloat16().requires_grad_(train)
+    cfg = dict(d_state=block.d_state, dt_rank=block.dt_rank)
+    want = mamba1_mixer_forward(ops, {**w, "out_proj": other}, cfg, hidden)
+    with fwd.dual_level():
+        got = mamba1_mixer_forward(ops, {**w, "out_proj": fwd.make_dual(w["out_proj"], other)}, cfg, hidden)
+        _near(fwd.unpack_dual(got).tangent.detach(), want.detach(), torch.bfloat16, "tangent")
+
+
+def test_mamba1_transformed_output_projection():
+    """torch.func.grad over the last product's weight; the operators in front of it see plain tensors."""
+    from ssm_b200.mixer import mamba1_mixer_forward
+
+    torch.manual_seed(6)
+    block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
+    w, _ = _other_out_proj(block)
+    hidden, go = torch.randn(2, 33, 64, device="cuda").bfloat16(), torch.randn(2, 33, 64, device="cuda").bfloat16()
+    cfg = dict(d_state=block.d_state, dt_rank=block.dt_rank)
+    got = torch.func.grad(lambda o: (mamba1_mixer_forward(ops, {**w, "out_proj": o}, cfg, hidden) * go).sum())(w["out_proj"])
+    leaf = w["out_proj"].clone().requires_grad_()
+    (want,) = torch.autograd.grad(mamba1_mixer_forward(ops, {**w, "out_proj": leaf}, cfg, hidden), leaf, go)
+    _near(got, want, torch.bfloat16, "gradient")

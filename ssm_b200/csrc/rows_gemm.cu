@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
   extern __shared__ unsigned char gemm_raw[];
   __shared__ __align__(8) uint64_t bars[2 * kGemmMaxStages + 1];
   __shared__ uint32_t tmem_slot;
+  __shared__ int gave_up;  // a stage did not arrive in time
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_raw) + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = blockIdx.x % g.splits, tile = blockIdx.x / g.splits;
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
   if (tid == 0) {
     for (int s = 0; s < g.stages; ++s) tc::mbar_init(full + 8 * s, 1), tc::mbar_init(empty + 8 * s, 1);
     tc::mbar_init(done, 1);
+    gave_up = 0;
   }
   if (warp == 2) tc::tmem_alloc(tc::smem_u32(&tmem_slot), cols);
   tc::fence_before_sync();
@@ -69,6 +71,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
   auto ran_out = [&]() {
     if (g.status) *reinterpret_cast<volatile int32_t*>(g.status) = g.status_code;
   };
+  int issued = 0;  // stages that this thread has filled
   if (warp == 0) {
     if (tc::elect_one()) {
       // the first stages' weights go out ahead of the wait for the kernel before this one
@@ -79,7 +82,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
       }
       pdl_wait();
       const uint32_t stage0 = tc::smem_u32(base);
-      int st = 0, parity = 1, kc = kb0 * kGemmK, issued = 0;
+      int st = 0, parity = 1, kc = kb0 * kGemmK;
       for (int i = 0; i < kb1 - kb0; ++i, kc += kGemmK) {
         const uint32_t at = stage0 + st * stage_bytes, bar = full + 8 * st;
         if (i >= ahead) {
@@ -94,9 +97,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
         if (++st == g.stages) st = 0, parity ^= 1;
         issued = i + 1;
       }
-      // no copy is under way when the block ends, also where a wait has run out
-      for (int i = max(0, issued - g.stages); i < issued; ++i)
-        if (!tc::mbar_wait(full + 8 * (i % g.stages), (i / g.stages) & 1)) ran_out();
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
       for (int i = 0; i < kb1 - kb0; ++i) {
         if (!tc::mbar_wait(full + 8 * st, parity)) {
           ran_out();
+          gave_up = 1;
           break;
         }
         tc::fence_after_sync();
@@ -175,6 +176,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) rows_gemm_kernel(const __grid
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 2) tc::tmem_dealloc(tmem, cols);
+  // Where every stage was multiplied, no copy is under way by now.  Otherwise (a filling thread that gave up leaves the multiplying one without its next
+  // stage, too) the block ends once its copies have landed.
+  if (gave_up) {
+    for (int i = max(0, issued - g.stages); i < issued; ++i) tc::mbar_wait(full + 8 * (i % g.stages), (i / g.stages) & 1);
+  }
 }
 
 // (rows, k) matrix of 16-bit elements with `ld` elements from row to row; box = 64 columns x `box_rows` rows

@@ -1053,15 +1053,12 @@ std::tuple<Tensor, Tensor> ssd_scan(const Tensor& X, const Tensor& dt, const Ten
 // operators behind one node; products that add into a gradient do so in their epilogue instead of a pass of their own.
 //
 // They stand for the composed form only where nothing can tell the difference: no tracing, autocast or saved-tensor hooks, plain types, no weight with a
-// tangent or of a transform (torch.func), which a product in front of or behind the operators may carry.
-bool transformed(const Tensor& t) {
-  return t._fw_grad(0).defined() || t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::FuncTorchBatched}));
-}
+// tangent, which a product behind the operators carries.
 bool composed_only(const Tensor& x, std::initializer_list<const Tensor*> weights) {
   if (at::tracer::impl::is_dispatch_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || at::SavedTensorDefaultHooks::get_hooks().has_value()) return true;
   if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || !io_dtype_ok(x)) return true;
   for (const Tensor* w : weights)
-    if (w->scalar_type() != x.scalar_type() || w->dim() != 2 || w->device() != x.device() || transformed(*w)) return true;
+    if (w->scalar_type() != x.scalar_type() || w->dim() != 2 || w->device() != x.device() || w->_fw_grad(0).defined()) return true;
   return false;
 }
 

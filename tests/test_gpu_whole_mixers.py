@@ -243,16 +243,17 @@ def test_mamba1_tangent_of_the_output_projection(train):
         _near(fwd.unpack_dual(got).tangent.detach(), want.detach(), torch.bfloat16, "tangent")
 
 
-def test_mamba1_transformed_output_projection():
-    """torch.func.grad over the last product's weight; the operators in front of it see plain tensors."""
+@pytest.mark.parametrize("train", [False, True])
+def test_mamba1_batched_output_projection(train):
+    """torch.vmap over the last product's weight; the operators in front of it see plain tensors."""
     from ssm_b200.mixer import mamba1_mixer_forward
 
     torch.manual_seed(6)
     block = Mamba1Block(64, device="cuda", dtype=torch.bfloat16)
-    w, _ = _other_out_proj(block)
-    hidden, go = torch.randn(2, 33, 64, device="cuda").bfloat16(), torch.randn(2, 33, 64, device="cuda").bfloat16()
-    cfg = dict(d_state=block.d_state, dt_rank=block.dt_rank)
-    got = torch.func.grad(lambda o: (mamba1_mixer_forward(ops, {**w, "out_proj": o}, cfg, hidden) * go).sum())(w["out_proj"])
-    leaf = w["out_proj"].clone().requires_grad_()
-    (want,) = torch.autograd.grad(mamba1_mixer_forward(ops, {**w, "out_proj": leaf}, cfg, hidden), leaf, go)
-    _near(got, want, torch.bfloat16, "gradient")
+    w, other = _other_out_proj(block)
+    hidden, cfg = torch.randn(2, 33, 64, device="cuda").bfloat16(), dict(d_state=block.d_state, dt_rank=block.dt_rank)
+    both = torch.stack([w["out_proj"], other]).requires_grad_(train)
+    got = torch.vmap(lambda o: mamba1_mixer_forward(ops, {**w, "out_proj": o}, cfg, hidden))(both)
+    assert got.requires_grad == train
+    for a, o in zip(got, both):
+        _near(a.detach(), mamba1_mixer_forward(ops, {**w, "out_proj": o.detach()}, cfg, hidden), torch.bfloat16, "out")

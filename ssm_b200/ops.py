@@ -397,10 +397,16 @@ def mamba2_step(tok: Tensor, conv_states: tuple, ssm_state: Tensor, w: dict, eps
                                  w["out_proj"], eps)
 
 
+_PLAIN_TENSORS = (Tensor, torch.nn.Parameter)  # a subclass may answer torch's own functions in its own way
+
+
 def mamba1_mixer(hidden: Tensor, w: dict) -> Optional[Tensor]:
     """Extension: a whole Mamba-1 mixer behind one autograd node; ``hidden (B, L, d_model)``, ``w`` as for :func:`mamba1_step`.  ``None`` where
-    the operators have to be composed instead (tracing, autocast, saved-tensor hooks, mixed types)."""
+    the operators have to be composed instead (tracing, forward mode, autocast, saved-tensor hooks, mixed types, tensor subclasses)."""
     a_log = "A_log" in w
+    for t in (hidden, w["in_x"], w["in_z"], w["x_proj"], w["dt_proj"], w["A_log"] if a_log else w["A"], w["out_proj"]):
+        if type(t) not in _PLAIN_TENSORS:
+            return None
     return _native().mamba1_mixer(hidden, w["in_x"], w["in_z"], w["conv_w"], w["conv_b"], w["x_proj"], w["dt_proj"], w["dt_bias"], w["A_log"] if a_log else w["A"],
                                   a_log, w["D"], w["out_proj"])
 
@@ -408,6 +414,9 @@ def mamba1_mixer(hidden: Tensor, w: dict) -> Optional[Tensor]:
 def mamba2_mixer(u: Tensor, w: dict, cfg: dict) -> Optional[Tensor]:
     """Extension: a whole Mamba-2 mixer on the tensor-core scan, without gradients; ``None`` as for :func:`mamba1_mixer`, with gradients enabled
     and for shapes that the scan is not built for."""
+    for t in (u, w["in_z"], w["in_x"], w["in_B"], w["in_C"], w["in_dt"], w["A_log"], w["out_proj"]):
+        if type(t) not in _PLAIN_TENSORS:
+            return None
     return _native().mamba2_mixer(u, w["in_z"], w["in_x"], w["in_B"], w["in_C"], w["in_dt"], w["conv_x"], w["conv_x_b"], w["conv_B"], w["conv_B_b"], w["conv_C"],
                                   w["conv_C_b"], w["dt_bias"], w["A_log"], w["D"], w["norm_w"], w["out_proj"], cfg["heads"], cfg["headdim"], cfg["d_state"],
                                   cfg["groups"], cfg.get("chunk_size", 256), cfg.get("eps", 1e-5))

@@ -257,3 +257,34 @@ def test_mamba1_batched_output_projection(train):
     assert got.requires_grad == train
     for a, o in zip(got, both):
         _near(a.detach(), mamba1_mixer_forward(ops, {**w, "out_proj": o.detach()}, cfg, hidden), torch.bfloat16, "out")
+
+
+
+class _Doubled(torch.Tensor):
+    """A weight that stands for twice its values."""
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        plain = lambda t: t.as_subclass(torch.Tensor) if isinstance(t, cls) else t  # noqa: E731
+        if func is torch.Tensor.t:
+            return plain(args[0]).t().as_subclass(cls)
+        if func is torch.matmul:
+            return torch.matmul(*(2 * plain(t) if isinstance(t, cls) else t for t in args))
+        return func(*map(plain, args), **(kwargs or {}))
+
+
+@pytest.mark.parametrize("cls", [Mamba1Block, Mamba2Block])
+def test_weights_of_a_tensor_subclass(cls):
+    from ssm_b200 import mixer
+
+    torch.manual_seed(7)
+    block = cls(128, device="cuda", dtype=torch.bfloat16).requires_grad_(False)
+    w = dict(block.named_parameters())
+    hidden = torch.randn(2, 33, 128, device="cuda").bfloat16()
+    if cls is Mamba1Block:
+        run = lambda w: mixer.mamba1_mixer_forward(ops, w, dict(d_state=block.d_state, dt_rank=block.dt_rank), hidden)  # noqa: E731
+    else:
+        run = lambda w: mixer.mamba2_mixer_forward(ops, w, block._cfg(), hidden)  # noqa: E731
+    with torch.no_grad():
+        got = run({**w, "out_proj": w["out_proj"].detach().as_subclass(_Doubled)})
+        _near(got, 2 * run(w), torch.bfloat16, "out")

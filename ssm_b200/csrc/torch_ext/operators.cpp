@@ -592,8 +592,11 @@ struct Parts {
   }
 };
 Tensor rows_of(void* p, int64_t rows, int64_t cols, int64_t ld, const Tensor& like) { return at::from_blob(p, {rows, cols}, {ld, 1}, like.options()); }
-// The library's product of many token rows with one large matrix keeps more of the GPU busy than the kernel of Parts (256 rows, 2560 x 5120: 10.6
-// us against 16.2; 128 rows 10.1 against 11.3; 256 rows, 768 x 1536 4.5 against 5.8, but 10 us more of host time).
+// The library's product of many token rows with one large matrix keeps more of the GPU busy than the kernel of Parts (us of products back to back, own
+// and library: 2560 x 5120 at 256 rows 14.9 and 9.7, at 192 11.7 and 8.8, at 160 10.5 and 10.8, at 128 9.3 and 8.9; 1536 x 3072 at 256 8.1 and 6.7,
+// at 128 6.4 and 6.3; 768 x 1536 at 256 5.6 and 4.4, for which the host's 10 us more are too many).  The projections in front are one launch here for
+// two to five of the library's: 2 x (5120 x 2560) at 256 rows 19.2 and 16.6, at 192 15.1 and 15.5, at 128 11.5 and 13.1, at 32 8.5 and 14.8; 2 x
+// (3072 x 1536) at 256 8.7 and 10.0.
 bool library_product(int64_t nb, const Tensor& w) { return nb > 128 && w.size(0) >= 1024 && w.size(1) >= 2048; }
 
 // What the separate calls refuse, or answer in another type, goes to them: shapes that agree in their number of elements only, tangents, autocast

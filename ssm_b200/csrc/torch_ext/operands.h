@@ -70,7 +70,7 @@ inline Tensor like(const Tensor& t, const Tensor& ref) { return t.detach().to(re
 // buffer viewed as (B, D, L).  Anything else is copied to dense.
 inline Tensor rows(const Tensor& t) {
   Tensor d = t.detach();
-  if (d.is_contiguous()) return d;
+  if (d.is_contiguous()) return d.dim() == 3 ? d.as_strided(d.sizes(), {d.size(1) * d.size(2), d.size(2), 1}) : d;  // an extent of one may have any stride
   if (d.dim() == 3 && d.stride(2) == 1 && d.stride(0) == d.size(2) && d.stride(1) == d.size(0) * d.size(2)) return d;
   return d.contiguous();
 }

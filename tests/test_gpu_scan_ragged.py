@@ -34,3 +34,21 @@ def test_scan_edges(nb, dim, length, n, groups, dtype):
     for i, (a, b) in enumerate(zip(got, want)):
         b = b.reshape(a.shape).double()
         assert (a.cpu().double() - b).norm() <= tol * b.norm() + 1e-6, i
+
+
+@pytest.mark.parametrize("op", ["scan", "conv"])
+def test_one_row_of_any_stride(op):
+    """An extent of one may have any stride, also one shorter than a row."""
+    u = torch.randn(2, 40, 1, device="cuda").transpose(1, 2)  # (2, 1, 40) with strides (40, 1, 1)
+    if op == "conv":
+        w = torch.randn(1, 4, device="cuda")
+        run = lambda t: ops.dw_causal_conv(t, w)  # noqa: E731
+    else:
+        A, BC = -torch.rand(1, 4, device="cuda"), torch.randn(2, 1, 4, 40, device="cuda")
+        run = lambda t: ops.selective_scan(t, t.abs(), A, BC, BC)  # noqa: E731
+    a, b = u.clone(memory_format=torch.preserve_format).requires_grad_(), torch.empty(2, 1, 40, device="cuda").copy_(u).requires_grad_()
+    assert a.stride() == (40, 1, 1)
+    ya, yb = run(a), run(b)
+    assert torch.equal(ya, yb)
+    for x, y in zip(torch.autograd.grad(ya.sum(), a), torch.autograd.grad(yb.sum(), b)):
+        torch.testing.assert_close(x, y)
